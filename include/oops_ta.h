@@ -220,6 +220,40 @@ int oops_ta_layer_norm_backward(int dtype, int affine_dtype, int64_t rows, int32
                                 uint64_t workspace_bytes, void* stream);
 
 /*
+ * Passes of the triangle multiplicative update between its library GEMMs
+ * (oops/pair/triangle_multiplication/triangle_multiplication.py:45-141 in the reference).  Two layouts: token-major rows
+ * m = ((prefix * tokens) + i) * tokens + j with contiguous channels (16-byte accesses when channels, row strides and
+ * addresses allow), and channel-major planes (prefix * hidden, padded, padded), `padded` = a multiple of 8 not below
+ * `tokens`, whose padding rows and columns are written as zeros and never read back.  Everything is of type `dtype`.
+ *   pair_gate:     row m of `projections` (row stride ld) is [left gate | left value | right gate | right value | ...] of
+ *                  `hidden` channels each; left, right = mask[m] * sigmoid(gate) * value.  `mask` (of `dtype`, may be
+ *                  NULL) has one weight per row.  The reverse pass writes the gradients in the same column order.
+ *   channel_norm:  layer norm over the channels of channel-major `update` into token-major rows of `hidden` channels
+ *                  (contiguous), hidden <= 512; mean and rstd (f32 per row m) serve the reverse pass, whose parameter gradients
+ *                  (may be NULL) are summed in a fixed order through `workspace`.
+ *   output_gate:   out = values * sigmoid(gate) for contiguous (rows, channels) values; gate rows have stride gate_ld.
+ */
+int oops_ta_pair_gate_forward(int dtype, int32_t prefix, int32_t tokens, int32_t padded, int32_t hidden,
+                              const void* projections, int64_t ld, const void* mask, void* left, void* right, void* stream);
+int oops_ta_pair_gate_backward(int dtype, int32_t prefix, int32_t tokens, int32_t padded, int32_t hidden,
+                               const void* projections, int64_t ld, const void* mask, const void* dleft, const void* dright,
+                               void* dprojections, int64_t ld_d, void* stream);
+int oops_ta_channel_norm_forward(int dtype, int affine_dtype, int32_t prefix, int32_t tokens, int32_t padded, int32_t hidden,
+                                 const void* update, const void* weight, const void* bias, float eps, void* y, float* mean,
+                                 float* rstd, void* stream);
+uint64_t oops_ta_channel_norm_backward_workspace_bytes(int dtype, int32_t prefix, int32_t tokens, int32_t padded,
+                                                       int32_t hidden);
+int oops_ta_channel_norm_backward(int dtype, int affine_dtype, int32_t prefix, int32_t tokens, int32_t padded, int32_t hidden,
+                                  const void* dy, const void* update, const void* weight, const float* mean,
+                                  const float* rstd, void* dupdate, void* dweight, void* dbias, void* workspace,
+                                  uint64_t workspace_bytes, void* stream);
+int oops_ta_output_gate_forward(int dtype, int64_t rows, int32_t channels, const void* values, const void* gate,
+                                int64_t gate_ld, void* out, void* stream);
+int oops_ta_output_gate_backward(int dtype, int64_t rows, int32_t channels, const void* dout, const void* values,
+                                 const void* gate, int64_t gate_ld, void* dvalues, void* dgate, int64_t dgate_ld,
+                                 void* stream);
+
+/*
  * Pair validity of a packed ragged batch: for sample s with n_s tokens, out holds the samples' row-major n_s x n_s
  * squares one after the other, cell (i, j) = token i is valid and token j is valid (bytes 0 / 1).  `token_values` are
  * bytes (nonzero = valid), `token_offsets` the samples + 1 cumulative token counts (int64, device memory), `chunks`

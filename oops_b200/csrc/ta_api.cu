@@ -231,6 +231,85 @@ int oops_ta_layer_norm_backward(int dtype, int affine_dtype, int64_t rows, int32
   return status == OOPS_TA_UNSUPPORTED_DTYPE ? fail(status, "layer_norm dtype %d / parameter dtype %d", dtype, affine_dtype) : status;
 }
 
+int oops_ta_pair_gate_forward(int dtype, int32_t prefix, int32_t tokens, int32_t padded, int32_t hidden,
+                              const void* projections, int64_t ld, const void* mask, void* left, void* right, void* stream) {
+  if (!projections || !left || !right) return fail(OOPS_TA_INVALID_ARGUMENT, "projections, left or right is NULL");
+  const int status = check_device();
+  if (status) return status;
+  g_error[0] = 0;
+  return pair_gate_forward(dtype, prefix, tokens, padded, hidden, projections, ld, mask, left, right,
+                           reinterpret_cast<cudaStream_t>(stream));
+}
+
+int oops_ta_pair_gate_backward(int dtype, int32_t prefix, int32_t tokens, int32_t padded, int32_t hidden,
+                               const void* projections, int64_t ld, const void* mask, const void* dleft, const void* dright,
+                               void* dprojections, int64_t ld_d, void* stream) {
+  if (!projections || !dleft || !dright || !dprojections)
+    return fail(OOPS_TA_INVALID_ARGUMENT, "projections, dleft, dright or dprojections is NULL");
+  const int status = check_device();
+  if (status) return status;
+  g_error[0] = 0;
+  return pair_gate_backward(dtype, prefix, tokens, padded, hidden, projections, ld, mask, dleft, dright, dprojections, ld_d,
+                            reinterpret_cast<cudaStream_t>(stream));
+}
+
+int oops_ta_channel_norm_forward(int dtype, int affine_dtype, int32_t prefix, int32_t tokens, int32_t padded, int32_t hidden,
+                                 const void* update, const void* weight, const void* bias, float eps, void* y, float* mean,
+                                 float* rstd, void* stream) {
+  if (!update || !y || !mean || !rstd) return fail(OOPS_TA_INVALID_ARGUMENT, "update, y, mean or rstd is NULL");
+  if (hidden > channel_norm_max_width())
+    return fail(OOPS_TA_UNSUPPORTED_LAYOUT, "hidden %d above %d", hidden, channel_norm_max_width());
+  const int status = check_device();
+  if (status) return status;
+  g_error[0] = 0;
+  return channel_norm_forward(dtype, affine_dtype, prefix, tokens, padded, hidden, update, weight, bias, eps, y, mean, rstd,
+                              reinterpret_cast<cudaStream_t>(stream));
+}
+
+uint64_t oops_ta_channel_norm_backward_workspace_bytes(int dtype, int32_t prefix, int32_t tokens, int32_t padded,
+                                                       int32_t hidden) {
+  return channel_norm_backward_workspace_bytes(dtype, prefix, tokens, padded, hidden);
+}
+
+int oops_ta_channel_norm_backward(int dtype, int affine_dtype, int32_t prefix, int32_t tokens, int32_t padded, int32_t hidden,
+                                  const void* dy, const void* update, const void* weight, const float* mean,
+                                  const float* rstd, void* dupdate, void* dweight, void* dbias, void* workspace,
+                                  uint64_t workspace_bytes, void* stream) {
+  if (!dy || !update || !mean || !rstd || !dupdate)
+    return fail(OOPS_TA_INVALID_ARGUMENT, "dy, update, mean, rstd or dupdate is NULL");
+  if (hidden > channel_norm_max_width())
+    return fail(OOPS_TA_UNSUPPORTED_LAYOUT, "hidden %d above %d", hidden, channel_norm_max_width());
+  if ((dweight || dbias) &&
+      (!workspace || workspace_bytes < channel_norm_backward_workspace_bytes(dtype, prefix, tokens, padded, hidden)))
+    return fail(OOPS_TA_WORKSPACE_TOO_SMALL, "workspace too small for the parameter gradients");
+  const int status = check_device();
+  if (status) return status;
+  g_error[0] = 0;
+  return channel_norm_backward(dtype, affine_dtype, prefix, tokens, padded, hidden, dy, update, weight, mean, rstd, dupdate, dweight,
+                               dbias, reinterpret_cast<float*>(workspace), reinterpret_cast<cudaStream_t>(stream));
+}
+
+int oops_ta_output_gate_forward(int dtype, int64_t rows, int32_t channels, const void* values, const void* gate,
+                                int64_t gate_ld, void* out, void* stream) {
+  if (!values || !gate || !out) return fail(OOPS_TA_INVALID_ARGUMENT, "values, gate or out is NULL");
+  const int status = check_device();
+  if (status) return status;
+  g_error[0] = 0;
+  return output_gate_forward(dtype, rows, channels, values, gate, gate_ld, out, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int oops_ta_output_gate_backward(int dtype, int64_t rows, int32_t channels, const void* dout, const void* values,
+                                 const void* gate, int64_t gate_ld, void* dvalues, void* dgate, int64_t dgate_ld,
+                                 void* stream) {
+  if (!dout || !values || !gate || !dvalues || !dgate)
+    return fail(OOPS_TA_INVALID_ARGUMENT, "dout, values, gate, dvalues or dgate is NULL");
+  const int status = check_device();
+  if (status) return status;
+  g_error[0] = 0;
+  return output_gate_backward(dtype, rows, channels, dout, values, gate, gate_ld, dvalues, dgate, dgate_ld,
+                              reinterpret_cast<cudaStream_t>(stream));
+}
+
 int oops_ta_pair_mask_packed(const uint8_t* token_values, const int64_t* token_offsets, int32_t samples, int64_t chunks,
                              uint8_t* out, void* stream) {
   if (samples < 0 || chunks < 0) return fail(OOPS_TA_INVALID_ARGUMENT, "negative sample or chunk count");

@@ -61,6 +61,25 @@ int layer_norm_forward(int dtype, int affine_dtype, int64_t rows, int width, con
 int layer_norm_backward(int dtype, int affine_dtype, int64_t rows, int width, const void* dy, int64_t dy_stride, const void* x,
                         int64_t x_stride, const void* weight, const float* mean, const float* rstd, void* dx, int64_t dx_stride,
                         void* dweight, void* dbias, void* workspace, cudaStream_t stream);
+// Sums f32 partial rows of the two affine gradients in a fixed order (a NULL tensor is skipped).
+int reduce_parameter_parts(int affine_dtype, const float* dw_parts, const float* db_parts, int num_parts, int width, void* dweight,
+                           void* dbias, cudaStream_t stream);
+// Passes of the triangle multiplicative update between its GEMMs (include/oops_ta.h has the layouts).
+int channel_norm_max_width();
+int pair_gate_forward(int dtype, int prefix, int tokens, int padded, int hidden, const void* proj, int64_t ld, const void* mask,
+                      void* left, void* right, cudaStream_t stream);
+int pair_gate_backward(int dtype, int prefix, int tokens, int padded, int hidden, const void* proj, int64_t ld, const void* mask,
+                       const void* dleft, const void* dright, void* dproj, int64_t ld_d, cudaStream_t stream);
+int channel_norm_forward(int dtype, int affine_dtype, int prefix, int tokens, int padded, int hidden, const void* update,
+                         const void* weight, const void* bias, float eps, void* y, float* mean, float* rstd, cudaStream_t stream);
+uint64_t channel_norm_backward_workspace_bytes(int dtype, int prefix, int tokens, int padded, int hidden);
+int channel_norm_backward(int dtype, int affine_dtype, int prefix, int tokens, int padded, int hidden, const void* dy,
+                          const void* update, const void* weight, const float* mean, const float* rstd, void* dupdate,
+                          void* dweight, void* dbias, float* workspace, cudaStream_t stream);
+int output_gate_forward(int dtype, int64_t rows, int channels, const void* values, const void* gate, int64_t gate_ld, void* out,
+                        cudaStream_t stream);
+int output_gate_backward(int dtype, int64_t rows, int channels, const void* dout, const void* values, const void* gate,
+                         int64_t gate_ld, void* dvalues, void* dgate, int64_t dgate_ld, cudaStream_t stream);
 // Forward pass of the tcgen05 kernels with the gate applied in the epilogue: writes sigmoid(gate) * out to `gated`
 // and, when plain.ptr is not NULL, the ungated values to `plain`.
 int tensor_forward_gated(const oops_ta_problem& p, const oops_ta_pair& gate, const oops_ta_pair& gated,

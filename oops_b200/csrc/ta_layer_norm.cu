@@ -674,6 +674,17 @@ uint64_t layer_norm_backward_workspace_bytes(int64_t rows, int width) {
 
 int layer_norm_max_width() { return kLnMaxWidth; }
 
+int reduce_parameter_parts(int affine_dtype, const float* dw_parts, const float* db_parts, int num_parts, int width, void* dweight,
+                           void* dbias, cudaStream_t stream) {
+  return ln_dispatch(affine_dtype, affine_dtype, [&](auto, auto a) {
+    using A = decltype(a);
+    layer_norm_reduce_parts_kernel<A><<<dim3((width + 31) / 32, 2), 256, 0, stream>>>(
+        dw_parts, db_parts, num_parts, width, reinterpret_cast<A*>(dweight), reinterpret_cast<A*>(dbias));
+    count_launch();
+    return check_launch("parameter gradient reduction");
+  });
+}
+
 int layer_norm_forward(int dtype, int affine_dtype, int64_t rows, int width, const void* x, int64_t x_stride, const void* weight,
                        const void* bias, float eps, void* y, int64_t y_stride, float* mean, float* rstd, cudaStream_t stream) {
   if (rows == 0) return OOPS_TA_OK;
