@@ -20,9 +20,11 @@ from typing import Optional
 
 import torch
 from torch import Tensor
+from torch.autograd import forward_ad
 from torch.nn import functional as F
 
 from ...runtime import cabi, require_no_forward_mode, require_same_device, unsupported
+from ...runtime.native import native
 from ...runtime.nested_tensor import is_nested
 from ..triangle import function as _function
 from ..triangle.triangle_attention import (
@@ -53,69 +55,9 @@ def _check_gate_output(attention: Tensor, single: Tensor, gate_weight: Tensor, o
         raise ValueError("output_weight input channels must equal num_heads * head_size")
 
 
-def _pair_view(tensor: Tensor, heads: int, head_size: int, head_major: bool) -> Tensor:
-    """View ``(B, H, Q, D)`` (head-major) or ``(B, Q, H*D)`` (token-major) as the C ABI's ``(B, 1, Q, H, D)``."""
-    if head_major:
-        return tensor.permute(0, 2, 1, 3).unsqueeze(1)
-    return tensor.unflatten(-1, (heads, head_size)).unsqueeze(1)
-
-
 def _run_gate(attention5: Tensor, gate5: Tensor, out5: Tensor) -> None:
-    lib = cabi.library()
-    batch, rows, cols, heads, head_size = attention5.shape
-    a, g, o = cabi.pair_of(attention5), cabi.pair_of(gate5), cabi.pair_of(out5)
-    with torch.cuda.device(attention5.device):
-        status = lib.oops_ta_gate_forward(
-            cabi.DTYPE_CODE[attention5.dtype], batch, rows, cols, heads, head_size, cabi.byref(a), cabi.byref(g), cabi.byref(o),
-            torch.cuda.current_stream(attention5.device).cuda_stream,
-        )
-    if status:
-        raise RuntimeError(f"{_OPERATOR} gate kernel failed: {cabi.status_message(status)}")
-
-
-def _run_gate_backward(attention5: Tensor, gate5: Tensor, dout5: Tensor, dattention5: Optional[Tensor],
-                       dgate5: Optional[Tensor]) -> None:
-    lib = cabi.library()
-    batch, rows, cols, heads, head_size = attention5.shape
-    a, g, u = cabi.pair_of(attention5), cabi.pair_of(gate5), cabi.pair_of(dout5)
-    da, dg = cabi.pair_of(dattention5), cabi.pair_of(dgate5)
-    with torch.cuda.device(attention5.device):
-        status = lib.oops_ta_gate_backward(
-            cabi.DTYPE_CODE[attention5.dtype], batch, rows, cols, heads, head_size, cabi.byref(a), cabi.byref(g), cabi.byref(u),
-            cabi.byref(da), cabi.byref(dg), torch.cuda.current_stream(attention5.device).cuda_stream,
-        )
-    if status:
-        raise RuntimeError(f"{_OPERATOR} gate kernel failed: {cabi.status_message(status)}")
-
-
-class _SigmoidGate(torch.autograd.Function):
-    """``gated[b, q, h*D + d] = sigmoid(gate[b, q, h*D + d]) * attention[b, h, q, d]``."""
-
-    @staticmethod
-    def forward(ctx, attention: Tensor, gate: Tensor) -> Tensor:
-        batch, heads, length, head_size = attention.shape
-        attention, gate = _unit_inner(attention), gate.contiguous()
-        gated = torch.empty_like(gate)
-        _run_gate(_pair_view(attention, heads, head_size, True), _pair_view(gate, heads, head_size, False),
-                  _pair_view(gated, heads, head_size, False))
-        ctx.save_for_backward(attention, gate)
-        return gated
-
-    @staticmethod
-    def backward(ctx, grad_gated: Tensor):
-        attention, gate = ctx.saved_tensors
-        batch, heads, length, head_size = attention.shape
-        attention = _unit_inner(attention)
-        grad_gated = grad_gated.resolve_neg().to(gate.dtype).contiguous()
-        d_attention = torch.empty(attention.shape, dtype=attention.dtype, device=attention.device) if ctx.needs_input_grad[0] else None
-        d_gate = torch.empty_like(gate) if ctx.needs_input_grad[1] else None
-        _run_gate_backward(
-            _pair_view(attention, heads, head_size, True), _pair_view(gate, heads, head_size, False),
-            _pair_view(grad_gated, heads, head_size, False),
-            None if d_attention is None else _pair_view(d_attention, heads, head_size, True),
-            None if d_gate is None else _pair_view(d_gate, heads, head_size, False),
-        )
-        return d_attention, d_gate
+    """``out5 = sigmoid(gate5) * attention5`` on ``(B, R, C, H, D)`` views."""
+    native().run_gate(attention5, gate5, out5)
 
 
 def gate_attention_output(attention, single, gate_weight: Tensor, output_weight: Tensor):
@@ -155,7 +97,7 @@ def gate_attention_output(attention, single, gate_weight: Tensor, output_weight:
     attention4 = attention.reshape(-1, *attention.shape[-3:]) if len(lead) != 1 else attention
     single3 = single.reshape(-1, *single.shape[-2:]) if len(lead) != 1 else single
     gate = F.linear(single3, gate_weight.to(single3.dtype))
-    gated = _SigmoidGate.apply(attention4, gate)
+    gated = native().sigmoid_gate(attention4, gate)
     result = F.linear(gated, output_weight.to(gated.dtype))
     return result.reshape(*lead, *result.shape[-2:]) if len(lead) != 1 else result
 
@@ -163,66 +105,6 @@ def gate_attention_output(attention, single, gate_weight: Tensor, output_weight:
 # ----------------------------------------------------------------------------------------------
 # the gate fused into triangle attention
 # ----------------------------------------------------------------------------------------------
-
-
-class _GatedTriangleAttention(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, query, key, value, gate, mask, bias, scale, flags):
-        needs_grad = any(ctx.needs_input_grad[i] for i in (0, 1, 2, 3, 5))
-        gated, plain, lse = _run_forward_gated(query, key, value, gate, mask, bias, scale, flags, keep_plain=needs_grad)
-        ctx.set_materialize_grads(False)
-        if needs_grad:
-            ctx.save_for_backward(query, key, value, gate, mask, bias, plain, lse)
-            ctx.scale, ctx.flags = scale, flags
-        return gated
-
-    @staticmethod
-    def backward(ctx, grad_gated):
-        if grad_gated is None:
-            return (None,) * 8
-        query, key, value, gate, mask, bias, plain, lse = ctx.saved_tensors
-        geometry = _function.DenseGeometry()
-        query, key, value, plain, gate = (geometry.canonical_pair(t) for t in (query, key, value, plain, gate))
-        grad_gated = geometry.canonical_pair(grad_gated.resolve_neg().to(query.dtype))
-        need_q, need_k, need_v, need_g, need_b = (ctx.needs_input_grad[i] for i in (0, 1, 2, 3, 5))
-        # through the gate: d(attention) = d(gated) * sigmoid(gate), d(gate) = d(gated) * attention * s (1 - s)
-        d_plain = torch.empty_like(plain)
-        d_gate = torch.empty_like(gate) if need_g else None
-        _run_gate_backward(plain, gate, grad_gated, d_plain, d_gate)
-        dq = dk = dv = dbias = None
-        if need_q or need_k or need_v or (need_b and bias is not None):
-            dq, dk, dv, dbias = _function.run_backward(
-                geometry, d_plain, query, key, value, mask, bias, plain, lse.contiguous(), ctx.scale, ctx.flags,
-                (need_q, need_k, need_v, need_b),
-            )
-        return dq, dk, dv, d_gate, None, dbias, None, None
-
-
-def _run_forward_gated(query, key, value, gate, mask, bias, scale, flags, keep_plain):
-    lib = cabi.library()
-    device = query.device
-    gated = torch.empty(query.shape, dtype=query.dtype, device=device)
-    plain = torch.empty(query.shape, dtype=query.dtype, device=device) if keep_plain else None
-    batch, rows, cols, heads, _ = query.shape
-    lse = torch.empty(batch * rows * heads * cols, dtype=torch.float32, device=device) if keep_plain else None
-    with torch.cuda.device(device):
-        problem = cabi.make_problem(query, key, value, mask, bias, scale, flags)
-        status = lib.oops_ta_supported(cabi.byref(problem))
-        if status:
-            _function._raise_status(status, "gated forward")
-        nbytes = lib.oops_ta_forward_workspace_bytes(cabi.byref(problem))
-        scratch = _function._workspace(nbytes, device)
-        if scratch is not None:
-            problem.workspace, problem.workspace_bytes = scratch.data_ptr(), scratch.numel()
-        gate_pair, gated_pair, plain_pair = cabi.pair_of(gate), cabi.pair_of(gated), cabi.pair_of(plain)
-        status = lib.oops_ta_forward_gated(
-            cabi.byref(problem), cabi.byref(gate_pair), cabi.byref(gated_pair), cabi.byref(plain_pair),
-            None if lse is None else lse.data_ptr(), torch.cuda.current_stream(device).cuda_stream,
-        )
-        if status:
-            _function._raise_status(status, "gated forward")
-        _function._raise_if_device_failed("gated forward")
-    return gated, plain, lse
 
 
 def triangle_attention_gated(query: Tensor, key: Tensor, value: Tensor, gate: Tensor, mask: Optional[Tensor] = None,
@@ -234,6 +116,10 @@ def triangle_attention_gated(query: Tensor, key: Tensor, value: Tensor, gate: Te
     Dense rank-5 inputs; everything else as ``triangle_attention``.  Gradients flow to query, key, value, gate and bias.
     """
     operator = "triangle_attention_gated"
+    if not torch.compiler.is_compiling() and forward_ad._current_level < 0:
+        out = native().triangle_attention_gated(query, key, value, gate, mask, triangle_bias, scale, _flags())
+        if out is not None:
+            return out
     for operand in (query, key, value, gate, mask, triangle_bias):
         if operand is not None and is_nested(operand):
             raise unsupported(operator, "serves dense inputs only")
@@ -261,7 +147,7 @@ def triangle_attention_gated(query: Tensor, key: Tensor, value: Tensor, gate: Te
         if bias5.element_size() == 2 and cols % 8 != 0:
             bias5 = torch.nn.functional.pad(bias5, (0, -cols % 8))[..., :cols]
     scale = head_size**-0.5 if scale is None else float(scale)
-    return _GatedTriangleAttention.apply(q5, k5, v5, g5, mask3, bias5, scale, _flags())
+    return native().gated_attend(q5, k5, v5, g5, mask3, bias5, scale, _flags())
 
 
 __all__ = ["gate_attention_output", "triangle_attention_gated"]

@@ -14,8 +14,10 @@ from typing import Optional, Tuple
 
 import torch
 from torch import Tensor
+from torch.autograd import forward_ad
 
 from ...runtime import cabi, require_no_forward_mode, require_same_device, unsupported
+from ...runtime.native import native
 from ...runtime.nested_tensor import is_nested
 from . import function as _function
 from .function import DenseGeometry, NestedGeometry, checked_device_status
@@ -62,6 +64,10 @@ def triangle_attention(
         OOpsUnsupportedError: unsupported device, dtype, layout, empty size,
             launch limit, or forward-mode differentiation.
     """
+    if not torch.compiler.is_compiling() and forward_ad._current_level < 0:
+        out = native().triangle_attention(query, key, value, mask, triangle_bias, scale, _flags())
+        if out is not None:
+            return out
     operands = {"query": query, "key": key, "value": value, "mask": mask, "triangle_bias": triangle_bias}
     packed = {name for name, operand in operands.items() if operand is not None and is_nested(operand)}
     pair_names = {"query", "key", "value"}

@@ -1,16 +1,18 @@
-"""Builds liboops_ta_sm100.so in-tree with nvcc for sm_100a (no GPU needed).
+"""Builds liboops_ta_sm100.so in-tree with nvcc for sm_100a (no GPU needed), and the host layer _native.so with g++.
 
     python -m oops_b200.csrc.build [--force]
 
-The shared library lands in oops_b200/lib/.  It is a plain C-ABI library
-(include/oops_ta.h); nothing in it links against Python or PyTorch.
+Both land in oops_b200/lib/.  The first is a plain C-ABI library (include/oops_ta.h); nothing in it links against Python
+or PyTorch.  The second is the PyTorch extension over it (native.cpp).
 """
 
 from __future__ import annotations
 
+import importlib.util
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -18,6 +20,7 @@ CSRC = Path(__file__).resolve().parent
 ROOT = CSRC.parent.parent
 LIB_DIR = CSRC.parent / "lib"
 LIB_PATH = LIB_DIR / "liboops_ta_sm100.so"
+NATIVE_PATH = LIB_DIR / "_native.so"
 SOURCES = ("ta_api.cu", "ta_generic.cu", "ta_gate.cu", "ta_mask.cu", "ta_layer_norm.cu", "ta_pair_update.cu", "ta_tensor_sm100.cu", "ta_tensor_bwd_sm100.cu")
 NVCC_FLAGS = (
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -58,6 +61,25 @@ def _stale(target: Path, deps) -> bool:
     return any(Path(d).stat().st_mtime > stamp for d in deps)
 
 
+def _native_commands(obj: Path) -> tuple:
+    """Compile and link commands of the host layer; it finds the kernels' library beside itself."""
+    torch_dir = Path(importlib.util.find_spec("torch").origin).parent
+    cuda_home = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
+    includes = (torch_dir / "include", torch_dir / "include/torch/csrc/api/include", sysconfig.get_paths()["include"], cuda_home / "include")
+    compile_flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_native", "-I", str(ROOT / "include")]
+    compile_flags += [flag for path in includes for flag in ("-isystem", str(path))]
+    libraries = ["-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda"]
+    link_flags = ["-L", str(LIB_DIR), "-L", str(torch_dir / "lib"), f"-l:{LIB_PATH.name}", *libraries, "-Wl,-rpath,$ORIGIN"]
+    return (["g++", *compile_flags, "-c", str(CSRC / "native.cpp"), "-o", str(obj)],
+            ["g++", "-shared", str(obj), "-o", str(NATIVE_PATH), *link_flags])
+
+
+def _checked(cmd, what: str) -> None:
+    done = subprocess.run(cmd, capture_output=True, text=True)
+    if done.returncode != 0:
+        raise RuntimeError(f"{what} failed:\n{done.stdout}\n{done.stderr}")
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     LIB_DIR.mkdir(exist_ok=True)
     obj_dir = LIB_DIR / "obj"
@@ -82,13 +104,21 @@ def build(force: bool = False, verbose: bool = False) -> Path:
                 print(done.stderr)
         return obj
 
-    with ThreadPoolExecutor(max_workers=len(SOURCES)) as pool:
+    native_obj = obj_dir / "native.o"
+    compile_native, link_native = _native_commands(native_obj)
+
+    def compile_host():
+        if force or _stale(native_obj, [CSRC / "native.cpp", ROOT / "include" / "oops_ta.h"]):
+            _checked(compile_native, "g++ for native.cpp")
+
+    with ThreadPoolExecutor(max_workers=len(SOURCES) + 1) as pool:
+        host = pool.submit(compile_host)
         objects = list(pool.map(compile_one, SOURCES))
+        host.result()
     if force or _stale(LIB_PATH, objects):
-        cmd = [_nvcc(), "-shared", "-o", str(LIB_PATH), *map(str, objects), "-lcudart"]
-        done = subprocess.run(cmd, capture_output=True, text=True)
-        if done.returncode != 0:
-            raise RuntimeError(f"link failed:\n{done.stdout}\n{done.stderr}")
+        _checked([_nvcc(), "-shared", "-o", str(LIB_PATH), *map(str, objects), "-lcudart"], "link")
+    if force or _stale(NATIVE_PATH, [native_obj, LIB_PATH]):
+        _checked(link_native, "link of the host layer")
     return LIB_PATH
 
 

@@ -1,0 +1,913 @@
+// Host side of the operators: argument checks of the common case, autograd nodes, allocation and launches, in C++.
+//
+// The Python entry points hand their arguments to this module first.  A call it does not recognise as plain (another
+// device, tensor subclasses with their own dispatch, negated or conjugated views, shapes or types that do not fit) is
+// declined by returning None, and the Python code beside the entry point handles it or raises the documented error.
+// What it saves is host time: a Python autograd function with its ctypes structures cost 75 us per forward call and
+// 250 us per forward + reverse call, more than the kernels of calls below about 300 x 300 tokens take.
+// The kernels are reached through the C ABI only (include/oops_ta.h); PyTorch provides memory, streams and autograd.
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/extension.h>
+
+#include <atomic>
+#include <optional>
+#include <vector>
+
+#include "oops_ta.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::Function;
+using torch::autograd::variable_list;
+using MaybeTensor = std::optional<Tensor>;
+
+PyObject* g_unsupported_error = nullptr;  // OOpsUnsupportedError, set once at import
+std::atomic<bool> g_check_status{false};
+
+[[noreturn]] void raise_unsupported(const std::string& message) {
+  py::gil_scoped_acquire gil;
+  PyErr_SetString(g_unsupported_error ? g_unsupported_error : PyExc_NotImplementedError, message.c_str());
+  python_error error;
+  error.persist();
+  throw error;
+}
+
+void check_status(int status, const char* what) {
+  if (status == OOPS_TA_OK) return;
+  const char* detail = oops_ta_last_error();
+  std::string message = std::string(what) + " failed: " + oops_ta_status_string(status);
+  if (detail && *detail) message += std::string(": ") + detail;
+  TORCH_CHECK_VALUE(status != OOPS_TA_INVALID_ARGUMENT, message);
+  TORCH_CHECK(status != OOPS_TA_CUDA_ERROR && status != OOPS_TA_DEVICE_TIMEOUT && status != OOPS_TA_WORKSPACE_TOO_SMALL, message);
+  raise_unsupported(message);
+}
+
+// Inside `checked_device_status()` every pass ends with a synchronisation and a look at the device-side status word.
+void check_device(const char* what) {
+  if (!g_check_status.load(std::memory_order_relaxed)) return;
+  const int status = oops_ta_device_status(1);
+  TORCH_CHECK(status == OOPS_TA_OK, "triangle_attention ", what, ": a kernel recorded device status ", status, " (",
+              oops_ta_status_string(status), "); its results are undefined");
+}
+
+int dtype_code(at::ScalarType t) {
+  return t == at::kFloat ? OOPS_TA_F32 : t == at::kHalf ? OOPS_TA_F16 : t == at::kBFloat16 ? OOPS_TA_BF16 : -1;
+}
+
+void* current_stream(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+Tensor bytes_like(const Tensor& t, uint64_t count) {
+  return at::empty({int64_t(count)}, t.options().dtype(at::kByte).requires_grad(false));
+}
+
+Tensor floats_like(const Tensor& t, at::IntArrayRef sizes) {
+  return at::empty(sizes, t.options().dtype(at::kFloat).requires_grad(false));
+}
+
+bool requires_grad(const Tensor& t) { return t.defined() && t.requires_grad(); }
+bool requires_grad(const MaybeTensor& t) { return t.has_value() && t->defined() && t->requires_grad(); }
+
+void* data_of(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+void* data_of(const MaybeTensor& t) { return t.has_value() ? data_of(*t) : nullptr; }
+
+// No dispatch mode or transform is active that would have to see the operations of a call.
+bool plain_context() {
+  return !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
+         !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+}
+
+bool plain_tensor(const Tensor& t) {
+  static const c10::DispatchKeySet special({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched,
+                                            c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Functionalize,
+                                            c10::DispatchKey::ZeroTensor, c10::DispatchKey::Negative,
+                                            c10::DispatchKey::Conjugate});
+  return t.defined() && t.is_cuda() && t.layout() == at::kStrided && !t.key_set().has_any(special);
+}
+
+// ---------------------------------------------------------------------------------------------
+// triangle attention
+// ---------------------------------------------------------------------------------------------
+
+// One uniform problem (the tensors are (B, R, C, H, D) views), or a packed ragged batch: pair tensors (cells, P, H, D),
+// masks (cells, P), bias head-major (P, H, values) with a sample's block ordered (group, query, key).  `transposed`:
+// the packed cell order is column-major (the ending-node form).
+struct Geometry {
+  bool packed = false, transposed = false;
+  int64_t prefixes = 1;
+  std::vector<int64_t> lengths, groups, rows;  // tokens, bias groups and bias row strides of every sample
+
+  static Geometry decode(const std::vector<int64_t>& code) {
+    Geometry g;
+    if (code.empty()) return g;
+    g.packed = true;
+    g.prefixes = code[0];
+    g.transposed = code[1] != 0;
+    const int64_t count = code[2];
+    const bool has_bias = code[3] != 0;
+    auto at = code.begin() + 4;
+    g.lengths.assign(at, at + count);
+    if (has_bias) {
+      g.groups.assign(at + count, at + 2 * count);
+      g.rows.assign(at + 2 * count, at + 3 * count);
+    }
+    return g;
+  }
+  std::vector<int64_t> encode() const {
+    if (!packed) return {};
+    std::vector<int64_t> code{prefixes, transposed, int64_t(lengths.size()), !groups.empty()};
+    code.insert(code.end(), lengths.begin(), lengths.end());
+    code.insert(code.end(), groups.begin(), groups.end());
+    code.insert(code.end(), rows.begin(), rows.end());
+    return code;
+  }
+  size_t count() const { return packed ? lengths.size() : 1; }
+  int64_t lse_size(const Tensor& query) const {
+    if (!packed) return query.size(0) * query.size(1) * query.size(2) * query.size(3);
+    int64_t total = 0;
+    for (int64_t n : lengths) total += prefixes * n * n * query.size(2);
+    return total;
+  }
+};
+
+struct Sample {  // where a sample of a geometry starts
+  int64_t tokens = 0, cell = 0, bias = 0, lse = 0;
+};
+
+oops_ta_pair pair_of(const Geometry& g, const Sample& s, const Tensor& t) {
+  if (!t.defined()) return {nullptr, 0, 0, 0, 0};
+  char* base = static_cast<char*>(t.data_ptr());
+  if (!g.packed) return {base, t.stride(0), t.stride(1), t.stride(2), t.stride(3)};
+  const int64_t heads = t.size(2), dim = t.size(3), minor = g.prefixes * heads * dim, major = s.tokens * minor;
+  return {base + s.cell * minor * t.element_size(), heads * dim, g.transposed ? minor : major, g.transposed ? major : minor, dim};
+}
+
+void describe(oops_ta_problem& p, const Geometry& g, const Sample& s, size_t index, const Tensor& query, const Tensor& key,
+              const Tensor& value, const Tensor& mask, const Tensor& bias, double scale, int64_t flags) {
+  p.abi_version = OOPS_TA_ABI_VERSION;
+  p.flags = uint32_t(flags);
+  p.dtype = dtype_code(query.scalar_type());
+  p.batch = int32_t(g.packed ? g.prefixes : query.size(0));
+  p.rows = int32_t(g.packed ? s.tokens : query.size(1));
+  p.cols = int32_t(g.packed ? s.tokens : query.size(2));
+  p.heads = int32_t(query.size(-2));
+  p.head_dim = int32_t(query.size(-1));
+  p.scale = float(scale);
+  p.q = pair_of(g, s, query);
+  p.k = pair_of(g, s, key);
+  p.v = pair_of(g, s, value);
+  if (mask.defined()) {
+    if (!g.packed) {
+      p.mask = static_cast<const uint8_t*>(mask.data_ptr());
+      p.mask_sb = mask.stride(0);
+      p.mask_sr = mask.stride(1);
+      p.mask_sc = mask.stride(2);
+    } else {
+      p.mask = static_cast<const uint8_t*>(mask.data_ptr()) + s.cell * g.prefixes;
+      p.mask_sb = 1;
+      p.mask_sr = g.transposed ? g.prefixes : s.tokens * g.prefixes;
+      p.mask_sc = g.transposed ? s.tokens * g.prefixes : g.prefixes;
+    }
+  }
+  p.bias_dtype = p.dtype;
+  if (bias.defined()) {
+    p.bias_dtype = dtype_code(bias.scalar_type());
+    if (!g.packed) {
+      p.bias_groups = int32_t(bias.size(1));
+      p.bias = bias.data_ptr();
+      p.bias_sb = bias.stride(0);
+      p.bias_sg = bias.stride(1);
+      p.bias_sh = bias.stride(2);
+      p.bias_sq = bias.stride(3);
+      p.bias_sk = bias.stride(4);
+    } else {
+      const int64_t heads = bias.size(1), total = bias.size(2), row = g.rows[index];
+      p.bias_groups = int32_t(g.groups[index]);
+      p.bias = static_cast<char*>(bias.data_ptr()) + s.bias * bias.element_size();
+      p.bias_sb = heads * total;
+      p.bias_sg = s.tokens * row;
+      p.bias_sh = total;
+      p.bias_sq = row;
+      p.bias_sk = 1;
+    }
+  }
+}
+
+// Calls `body(problem, sample, index)` for every sample of the geometry.
+template <typename F>
+void for_each_sample(const Geometry& g, const Tensor& query, F&& body) {
+  Sample s;
+  for (size_t i = 0; i < g.count(); ++i) {
+    s.tokens = g.packed ? g.lengths[i] : 0;
+    body(s, i);
+    if (!g.packed) return;
+    s.cell += s.tokens * s.tokens;
+    s.lse += g.prefixes * s.tokens * s.tokens * query.size(2);
+    if (!g.groups.empty()) s.bias += g.groups[i] * s.tokens * g.rows[i];
+  }
+}
+
+Tensor result_like(const Tensor& t) {
+  Tensor out = at::empty_like(t);
+  if (out.size(-1) != 1 && out.stride(-1) != 1) out = at::empty(t.sizes(), t.options());
+  return out;
+}
+
+// `gate` and `plain` are undefined except for the gated form, whose result is the gated tensor.
+std::tuple<Tensor, Tensor> run_forward(const Geometry& g, const Tensor& query, const Tensor& key, const Tensor& value,
+                                       const Tensor& mask, const Tensor& bias, double scale, int64_t flags, bool want_lse,
+                                       const Tensor& gate = {}, const Tensor& plain = {}) {
+  const c10::cuda::CUDAGuard guard(query.device());
+  Tensor out = gate.defined() ? at::empty(query.sizes(), query.options()) : result_like(query);
+  Tensor lse = want_lse ? floats_like(query, {g.lse_size(query)}) : Tensor();
+  void* stream = current_stream(query);
+  for_each_sample(g, query, [&](const Sample& s, size_t i) {
+    oops_ta_problem problem{};
+    describe(problem, g, s, i, query, key, value, mask, bias, scale, flags);
+    check_status(oops_ta_supported(&problem), "triangle_attention forward");
+    Tensor scratch;
+    if (const uint64_t need = oops_ta_forward_workspace_bytes(&problem)) {
+      scratch = bytes_like(query, need);
+      problem.workspace = scratch.data_ptr();
+      problem.workspace_bytes = need;
+    }
+    const oops_ta_pair out_pair = pair_of(g, s, out);
+    float* lse_at = lse.defined() ? lse.data_ptr<float>() + s.lse : nullptr;
+    if (gate.defined()) {
+      const oops_ta_pair gate_pair = pair_of(g, s, gate), plain_pair = pair_of(g, s, plain);
+      check_status(oops_ta_forward_gated(&problem, &gate_pair, &out_pair, &plain_pair, lse_at, stream),
+                   "triangle_attention gated forward");
+    } else {
+      check_status(oops_ta_forward(&problem, &out_pair, lse_at, stream), "triangle_attention forward");
+    }
+  });
+  check_device(gate.defined() ? "gated forward" : "forward");
+  return {out, lse};
+}
+
+struct Gradients {
+  Tensor dq, dk, dv, dbias;
+};
+
+// `lent` is an optional caller-owned scratch buffer; `dbias_type` overrides the type of the bias gradient.
+Gradients run_backward(const Geometry& g, const Tensor& grad_out, const Tensor& query, const Tensor& key, const Tensor& value,
+                       const Tensor& mask, const Tensor& bias, const Tensor& out, const Tensor& lse, double scale, int64_t flags,
+                       bool need_q, bool need_k, bool need_v, bool need_b, const Tensor& lent = {},
+                       std::optional<at::ScalarType> dbias_type = std::nullopt) {
+  const c10::cuda::CUDAGuard guard(query.device());
+  Gradients grads;
+  if (need_q) grads.dq = result_like(query);
+  if (need_k) grads.dk = result_like(key);
+  if (need_v) grads.dv = result_like(value);
+  if (need_b && bias.defined()) grads.dbias = at::empty(bias.sizes(), bias.options().dtype(dbias_type.value_or(bias.scalar_type())));
+  void* stream = current_stream(query);
+  for_each_sample(g, query, [&](const Sample& s, size_t i) {
+    oops_ta_problem problem{};
+    describe(problem, g, s, i, query, key, value, mask, bias, scale, flags);
+    oops_ta_grads wanted{};
+    wanted.dq = pair_of(g, s, grads.dq);
+    wanted.dk = pair_of(g, s, grads.dk);
+    wanted.dv = pair_of(g, s, grads.dv);
+    if (grads.dbias.defined()) {
+      oops_ta_problem as_bias{};  // the gradient's own strides, through the same description
+      describe(as_bias, g, s, i, query, key, value, {}, grads.dbias, scale, flags);
+      wanted.dbias = const_cast<void*>(as_bias.bias);
+      wanted.dbias_sb = as_bias.bias_sb;
+      wanted.dbias_sg = as_bias.bias_sg;
+      wanted.dbias_sh = as_bias.bias_sh;
+      wanted.dbias_sq = as_bias.bias_sq;
+      wanted.dbias_sk = as_bias.bias_sk;
+    }
+    const uint64_t need = oops_ta_backward_workspace_bytes(&problem, &wanted);
+    Tensor scratch = lent;
+    if (need && !(lent.defined() && uint64_t(lent.numel()) >= need)) scratch = bytes_like(query, need);
+    if (scratch.defined()) {
+      problem.workspace = scratch.data_ptr();
+      problem.workspace_bytes = uint64_t(scratch.numel());
+    }
+    const oops_ta_pair out_pair = pair_of(g, s, out), dout_pair = pair_of(g, s, grad_out);
+    check_status(oops_ta_backward(&problem, &out_pair, &dout_pair, lse.data_ptr<float>() + s.lse, &wanted, stream),
+                 "triangle_attention backward");
+  });
+  check_device("backward");
+  return grads;
+}
+
+// Unit inner stride; 16-bit tensors additionally get 16-byte aligned rows, which the TMA kernels need.
+Tensor canonical_pair(const Geometry& g, const Tensor& t) {
+  if (g.packed || (t.size(-1) != 1 && t.stride(-1) != 1)) return t.contiguous();
+  if (t.element_size() == 2) {
+    bool aligned = reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+    for (int64_t d = 0; d + 1 < t.dim(); ++d) aligned = aligned && (t.size(d) <= 1 || (t.stride(d) > 0 && t.stride(d) % 8 == 0));
+    if (!aligned) return t.contiguous();
+  }
+  return t;
+}
+
+struct TriangleFunction : Function<TriangleFunction> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& query, const Tensor& key, const Tensor& value, const MaybeTensor& mask,
+                        const MaybeTensor& bias, double scale, const Geometry& g, int64_t flags) {
+    auto [out, lse] = run_forward(g, query, key, value, mask.value_or(Tensor()), bias.value_or(Tensor()), scale, flags, true);
+    ctx->set_materialize_grads(false);
+    ctx->save_for_backward({query, key, value, mask.value_or(Tensor()), bias.value_or(Tensor()), out, lse});
+    ctx->saved_data["scale"] = scale;
+    ctx->saved_data["geometry"] = g.encode();
+    ctx->saved_data["flags"] = flags;
+    return out;
+  }
+
+  static variable_list backward(AutogradContext* ctx, const variable_list& grad_outputs) {
+    variable_list result(8);
+    if (!grad_outputs[0].defined()) return result;
+    const variable_list saved = ctx->get_saved_variables();
+    const Geometry g = Geometry::decode(ctx->saved_data["geometry"].toIntVector());
+    // saved-tensor hooks may hand back copies with other strides; the views are rebuilt from what arrives
+    Tensor query = canonical_pair(g, saved[0]), key = canonical_pair(g, saved[1]), value = canonical_pair(g, saved[2]);
+    Tensor mask = saved[3], bias = saved[4], out = canonical_pair(g, saved[5]), lse = saved[6].contiguous();
+    Tensor grad_out = canonical_pair(g, grad_outputs[0].resolve_neg().to(query.scalar_type()));
+    if (g.packed && bias.defined()) bias = bias.contiguous();
+    if (g.packed && mask.defined()) mask = mask.contiguous();
+    // edges count the tensor arguments that were given
+    const size_t bias_edge = mask.defined() ? 4 : 3;
+    Gradients grads = run_backward(g, grad_out, query, key, value, mask, bias, out, lse, ctx->saved_data["scale"].toDouble(),
+                                   ctx->saved_data["flags"].toInt(), ctx->needs_input_grad(0), ctx->needs_input_grad(1),
+                                   ctx->needs_input_grad(2), bias.defined() && ctx->needs_input_grad(bias_edge));
+    result[0] = grads.dq;
+    result[1] = grads.dk;
+    result[2] = grads.dv;
+    result[4] = grads.dbias;
+    return result;
+  }
+};
+
+Tensor attend(const Tensor& query, const Tensor& key, const Tensor& value, const MaybeTensor& mask, const MaybeTensor& bias,
+              double scale, const Geometry& g, int64_t flags) {
+  if (at::GradMode::is_enabled() &&
+      (query.requires_grad() || key.requires_grad() || value.requires_grad() || requires_grad(bias)))
+    return TriangleFunction::apply(query, key, value, mask, bias, scale, g, flags);
+  return std::get<0>(run_forward(g, query, key, value, mask.value_or(Tensor()), bias.value_or(Tensor()), scale, flags, false));
+}
+
+// Folds the leading axes of (*lead, <keep axes>) into one batch axis.
+Tensor as_batch(const Tensor& t, int64_t keep) {
+  const int64_t lead = t.dim() - keep;
+  return lead == 1 ? t : lead == 0 ? t.unsqueeze(0) : t.flatten(0, lead - 1);
+}
+
+Tensor unit_inner(const Tensor& t) { return t.size(-1) == 1 || t.stride(-1) == 1 ? t : t.contiguous(); }
+
+bool broadcasts_to(at::IntArrayRef own, at::IntArrayRef want) {
+  if (own.size() > want.size()) return false;
+  for (size_t i = 1; i <= own.size(); ++i)
+    if (own[own.size() - i] != 1 && own[own.size() - i] != want[want.size() - i]) return false;
+  return true;
+}
+
+// Whether the operands of a dense call are what the kernels serve (the Python checks name what is not).
+bool dense_operands_fit(const Tensor& query, const Tensor& key, const Tensor& value, const MaybeTensor& mask, const MaybeTensor& bias) {
+  if (!plain_context() || !plain_tensor(query) || !plain_tensor(key) || !plain_tensor(value)) return false;
+  const auto type = query.scalar_type();
+  if (dtype_code(type) < 0 || key.scalar_type() != type || value.scalar_type() != type) return false;
+  if (query.dim() < 4 || key.sizes() != query.sizes() || value.sizes() != query.sizes()) return false;
+  if (query.numel() == 0 || query.size(-1) > 256) return false;
+  if (key.device() != query.device() || value.device() != query.device()) return false;
+  const at::IntArrayRef pair = query.sizes().slice(0, query.dim() - 2);
+  if (mask.has_value()) {
+    if (!plain_tensor(*mask) || mask->device() != query.device() || mask->scalar_type() != at::kBool) return false;
+    if (!broadcasts_to(mask->sizes(), pair)) return false;
+  }
+  if (bias.has_value()) {
+    const Tensor& b = *bias;
+    if (!plain_tensor(b) || b.device() != query.device() || (b.scalar_type() != type && b.scalar_type() != at::kFloat)) return false;
+    const int64_t lead = query.dim() - 4, rows = query.size(lead), cols = query.size(lead + 1), heads = query.size(lead + 2);
+    if (b.dim() != lead + 4 || b.sizes().slice(0, lead) != query.sizes().slice(0, lead)) return false;
+    if ((b.size(lead) != 1 && b.size(lead) != rows) || b.size(lead + 1) != heads || b.size(lead + 2) != cols || b.size(lead + 3) != cols)
+      return false;
+  }
+  return true;
+}
+
+// Contiguous bias; 16-bit biases get 16-byte aligned rows (the TMA kernels need them): the key axis is padded.
+Tensor aligned_bias(const Tensor& bias, int64_t cols) {
+  Tensor b = as_batch(bias, 4).contiguous();
+  if (b.element_size() == 2 && cols % 8 != 0) b = at::constant_pad_nd(b, {0, 8 - cols % 8}).narrow(-1, 0, cols);
+  return b;
+}
+
+std::optional<Tensor> dense_attention(const Tensor& query, const Tensor& key, const Tensor& value, const MaybeTensor& mask,
+                                      const MaybeTensor& bias, std::optional<double> scale, int64_t flags) {
+  if (!dense_operands_fit(query, key, value, mask, bias)) return std::nullopt;
+  const int64_t lead = query.dim() - 4;
+  const Tensor q5 = unit_inner(as_batch(query, 4));
+  // operands that are the same object stay the same object: the kernels then read one buffer
+  const Tensor k5 = key.is_same(query) ? q5 : unit_inner(as_batch(key, 4));
+  const Tensor v5 = value.is_same(query) ? q5 : value.is_same(key) ? k5 : unit_inner(as_batch(value, 4));
+  MaybeTensor mask3, bias5;
+  if (mask.has_value()) mask3 = as_batch(mask->expand(query.sizes().slice(0, query.dim() - 2)), 2);
+  if (bias.has_value()) bias5 = aligned_bias(*bias, query.size(-3));
+  const double factor = scale.has_value() ? *scale : 1.0 / std::sqrt(double(query.size(-1)));
+  const Tensor out = attend(q5, k5, v5, mask3, bias5, factor, Geometry(), flags);
+  if (lead == 1) return out;
+  return lead == 0 ? out.squeeze(0) : out.unflatten(0, query.sizes().slice(0, lead));
+}
+
+// ---------------------------------------------------------------------------------------------
+// the sigmoid gate
+// ---------------------------------------------------------------------------------------------
+
+oops_ta_pair dense_pair(const Tensor& t) { return pair_of(Geometry(), Sample(), t); }
+
+void run_gate(const Tensor& attention, const Tensor& gate, const Tensor& out) {
+  const c10::cuda::CUDAGuard guard(attention.device());
+  const oops_ta_pair a = dense_pair(attention), g = dense_pair(gate), o = dense_pair(out);
+  check_status(oops_ta_gate_forward(dtype_code(attention.scalar_type()), attention.size(0), attention.size(1), attention.size(2),
+                                    attention.size(3), attention.size(4), &a, &g, &o, current_stream(attention)),
+               "gate_attention_output gate kernel");
+}
+
+void run_gate_backward(const Tensor& attention, const Tensor& gate, const Tensor& dout, const Tensor& dattention, const Tensor& dgate) {
+  const c10::cuda::CUDAGuard guard(attention.device());
+  const oops_ta_pair a = dense_pair(attention), g = dense_pair(gate), u = dense_pair(dout), da = dense_pair(dattention),
+                     dg = dense_pair(dgate);
+  check_status(oops_ta_gate_backward(dtype_code(attention.scalar_type()), attention.size(0), attention.size(1), attention.size(2),
+                                     attention.size(3), attention.size(4), &a, &g, &u, &da, &dg, current_stream(attention)),
+               "gate_attention_output gate kernel");
+}
+
+// (B, H, Q, D) values as the C ABI's (B, 1, Q, H, D), and (B, Q, H * D) rows as the same.
+Tensor head_major(const Tensor& t) { return t.defined() ? t.permute({0, 2, 1, 3}).unsqueeze(1) : t; }
+Tensor token_major(const Tensor& t, int64_t heads, int64_t dim) {
+  return t.defined() ? t.view({t.size(0), 1, t.size(1), heads, dim}) : t;
+}
+
+// gated[b, q, h * D + d] = sigmoid(gate[b, q, h * D + d]) * attention[b, h, q, d]
+struct GateFunction : Function<GateFunction> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& attention_in, const Tensor& gate_in) {
+    const Tensor attention = unit_inner(attention_in.resolve_neg().resolve_conj()), gate = gate_in.contiguous();
+    const int64_t heads = attention.size(1), dim = attention.size(3);
+    Tensor gated = at::empty_like(gate);
+    run_gate(head_major(attention), token_major(gate, heads, dim), token_major(gated, heads, dim));
+    ctx->save_for_backward({attention, gate});
+    return gated;
+  }
+  static variable_list backward(AutogradContext* ctx, const variable_list& grad_outputs) {
+    const variable_list saved = ctx->get_saved_variables();
+    const Tensor attention = unit_inner(saved[0]), gate = saved[1].contiguous();
+    const int64_t heads = attention.size(1), dim = attention.size(3);
+    const Tensor dout = grad_outputs[0].resolve_neg().to(gate.scalar_type()).contiguous();
+    Tensor dattention, dgate;
+    if (ctx->needs_input_grad(0)) dattention = at::empty(attention.sizes(), attention.options());
+    if (ctx->needs_input_grad(1)) dgate = at::empty_like(gate);
+    run_gate_backward(head_major(attention), token_major(gate, heads, dim), token_major(dout, heads, dim), head_major(dattention),
+                      token_major(dgate, heads, dim));
+    return {dattention, dgate};
+  }
+};
+
+struct GatedTriangleFunction : Function<GatedTriangleFunction> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& query, const Tensor& key, const Tensor& value, const Tensor& gate,
+                        const MaybeTensor& mask, const MaybeTensor& bias, double scale, int64_t flags) {
+    Tensor plain = at::empty(query.sizes(), query.options());
+    auto [gated, lse] = run_forward(Geometry(), query, key, value, mask.value_or(Tensor()), bias.value_or(Tensor()), scale, flags, true,
+                                    gate, plain);
+    ctx->set_materialize_grads(false);
+    ctx->save_for_backward({query, key, value, gate, mask.value_or(Tensor()), bias.value_or(Tensor()), plain, lse});
+    ctx->saved_data["scale"] = scale;
+    ctx->saved_data["flags"] = flags;
+    return gated;
+  }
+  static variable_list backward(AutogradContext* ctx, const variable_list& grad_outputs) {
+    variable_list result(8);
+    if (!grad_outputs[0].defined()) return result;
+    const variable_list saved = ctx->get_saved_variables();
+    const Geometry g;
+    Tensor query = canonical_pair(g, saved[0]), key = canonical_pair(g, saved[1]), value = canonical_pair(g, saved[2]);
+    Tensor gate = canonical_pair(g, saved[3]), mask = saved[4], bias = saved[5], plain = canonical_pair(g, saved[6]);
+    Tensor grad_gated = canonical_pair(g, grad_outputs[0].resolve_neg().to(query.scalar_type()));
+    const bool need_q = ctx->needs_input_grad(0), need_k = ctx->needs_input_grad(1), need_v = ctx->needs_input_grad(2),
+               need_b = bias.defined() && ctx->needs_input_grad(mask.defined() ? 5 : 4);
+    // through the gate: d(attention) = d(gated) * sigmoid(gate), d(gate) = d(gated) * attention * s (1 - s)
+    Tensor dplain = at::empty_like(plain), dgate = ctx->needs_input_grad(3) ? at::empty_like(gate) : Tensor();
+    run_gate_backward(plain, gate, grad_gated, dplain, dgate);
+    result[3] = dgate;
+    if (need_q || need_k || need_v || need_b) {
+      Gradients grads = run_backward(g, dplain, query, key, value, mask, bias, plain, saved[7].contiguous(),
+                                     ctx->saved_data["scale"].toDouble(), ctx->saved_data["flags"].toInt(), need_q, need_k, need_v, need_b);
+      result[0] = grads.dq;
+      result[1] = grads.dk;
+      result[2] = grads.dv;
+      result[5] = grads.dbias;
+    }
+    return result;
+  }
+};
+
+Tensor gated_attend(const Tensor& query, const Tensor& key, const Tensor& value, const Tensor& gate, const MaybeTensor& mask,
+                    const MaybeTensor& bias, double scale, int64_t flags) {
+  if (at::GradMode::is_enabled() && (query.requires_grad() || key.requires_grad() || value.requires_grad() || gate.requires_grad() ||
+                                     requires_grad(bias)))
+    return GatedTriangleFunction::apply(query, key, value, gate, mask, bias, scale, flags);
+  return std::get<0>(run_forward(Geometry(), query, key, value, mask.value_or(Tensor()), bias.value_or(Tensor()), scale, flags, false, gate));
+}
+
+std::optional<Tensor> dense_gated_attention(const Tensor& query, const Tensor& key, const Tensor& value, const Tensor& gate_in,
+                                            const MaybeTensor& mask, const MaybeTensor& bias, std::optional<double> scale, int64_t flags) {
+  if (query.dim() != 5 || !dense_operands_fit(query, key, value, mask, bias) || !plain_tensor(gate_in)) return std::nullopt;
+  Tensor gate = gate_in;
+  if (gate.dim() == 4 && gate.size(-1) == query.size(-2) * query.size(-1)) gate = gate.unflatten(-1, query.sizes().slice(3, 2));
+  if (gate.sizes() != query.sizes() || gate.scalar_type() != query.scalar_type() || gate.device() != query.device()) return std::nullopt;
+  const Geometry g;
+  const Tensor q5 = canonical_pair(g, unit_inner(query));
+  const Tensor k5 = key.is_same(query) ? q5 : canonical_pair(g, unit_inner(key));
+  const Tensor v5 = value.is_same(query) ? q5 : value.is_same(key) ? k5 : canonical_pair(g, unit_inner(value));
+  MaybeTensor mask3, bias5;
+  if (mask.has_value()) mask3 = mask->expand(query.sizes().slice(0, 3));
+  if (bias.has_value()) bias5 = aligned_bias(*bias, query.size(2));
+  return gated_attend(q5, k5, v5, unit_inner(gate), mask3, bias5,
+                      scale.has_value() ? *scale : 1.0 / std::sqrt(double(query.size(-1))), flags);
+}
+
+// ---------------------------------------------------------------------------------------------
+// layer norm
+// ---------------------------------------------------------------------------------------------
+
+// `t` as (rows, width) with contiguous rows; a view when the layout allows it.
+Tensor rows_of(const Tensor& t, int64_t width) {
+  Tensor flat = t.reshape({-1, width});
+  if ((width > 1 && flat.stride(1) != 1) || (flat.size(0) > 1 && flat.stride(0) < width)) flat = flat.contiguous();
+  return flat;
+}
+
+struct Normed {
+  Tensor y, stats;  // stats: (2, rows) f32, mean and reciprocal standard deviation
+};
+
+Normed norm_forward(const Tensor& rows_in, const Tensor& weight, const Tensor& bias, double eps, bool keep_stats) {
+  const c10::cuda::CUDAGuard guard(rows_in.device());
+  const int64_t rows = rows_in.size(0), width = rows_in.size(1);
+  Normed n{at::empty({rows, width}, rows_in.options()), keep_stats ? floats_like(rows_in, {2, rows}) : Tensor()};
+  const auto affine = weight.defined() ? weight.scalar_type() : bias.defined() ? bias.scalar_type() : rows_in.scalar_type();
+  float* stats = keep_stats ? n.stats.data_ptr<float>() : nullptr;
+  const int status = oops_ta_layer_norm_forward(
+      dtype_code(rows_in.scalar_type()), dtype_code(affine), rows, int32_t(width), rows_in.data_ptr(), rows > 1 ? rows_in.stride(0) : width,
+      data_of(weight), data_of(bias), float(eps), n.y.data_ptr(), width, stats, stats ? stats + rows : nullptr, current_stream(rows_in));
+  if (status) raise_unsupported(std::string("layer_norm ") + oops_ta_status_string(status) + ": " + oops_ta_last_error());
+  return n;
+}
+
+struct NormGradients {
+  Tensor dx, dweight, dbias;
+};
+
+NormGradients norm_backward(const Tensor& dy, const Tensor& rows_in, const Tensor& weight, const Tensor& stats, at::ScalarType affine,
+                            bool need_x, bool need_w, bool need_b) {
+  const c10::cuda::CUDAGuard guard(rows_in.device());
+  const int64_t rows = rows_in.size(0), width = rows_in.size(1);
+  NormGradients grads;
+  if (need_x) grads.dx = at::empty({rows, width}, rows_in.options());
+  if (need_w) grads.dweight = at::empty({width}, rows_in.options().dtype(affine));
+  if (need_b) grads.dbias = at::empty({width}, rows_in.options().dtype(affine));
+  const uint64_t need = need_w || need_b ? oops_ta_layer_norm_backward_workspace_bytes(rows, int32_t(width)) : 0;
+  Tensor scratch = need ? bytes_like(rows_in, need) : Tensor();
+  const float* mean = stats.data_ptr<float>();
+  const int status = oops_ta_layer_norm_backward(
+      dtype_code(rows_in.scalar_type()), dtype_code(affine), rows, int32_t(width), dy.data_ptr(), rows > 1 ? dy.stride(0) : width,
+      rows_in.data_ptr(), rows > 1 ? rows_in.stride(0) : width, data_of(weight), mean, mean + rows, data_of(grads.dx), width,
+      data_of(grads.dweight), data_of(grads.dbias), data_of(scratch), need, current_stream(rows_in));
+  if (status) raise_unsupported(std::string("layer_norm ") + oops_ta_status_string(status) + ": " + oops_ta_last_error());
+  return grads;
+}
+
+struct LayerNormFunction : Function<LayerNormFunction> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const MaybeTensor& weight, const MaybeTensor& bias, double eps) {
+    const Tensor rows = rows_of(x, x.size(-1));
+    const Tensor w = weight.has_value() ? weight->contiguous() : Tensor(), b = bias.has_value() ? bias->contiguous() : Tensor();
+    Normed n = norm_forward(rows, w, b, eps, true);
+    ctx->save_for_backward({rows, w, n.stats});
+    ctx->saved_data["shape"] = x.sizes().vec();
+    ctx->saved_data["affine"] = int64_t(w.defined() ? w.scalar_type() : b.defined() ? b.scalar_type() : x.scalar_type());
+    ctx->saved_data["has_bias"] = b.defined();
+    return n.y.view(x.sizes());
+  }
+  static variable_list backward(AutogradContext* ctx, const variable_list& grad_outputs) {
+    const variable_list saved = ctx->get_saved_variables();
+    const Tensor rows = rows_of(saved[0], saved[0].size(-1));
+    const bool has_weight = saved[1].defined(), has_bias = ctx->saved_data["has_bias"].toBool();
+    const Tensor w = has_weight ? saved[1].contiguous() : Tensor();
+    const size_t bias_edge = has_weight ? 2 : 1;
+    NormGradients grads = norm_backward(rows_of(grad_outputs[0].resolve_neg(), rows.size(1)), rows, w, saved[2].contiguous(),
+                                        at::ScalarType(ctx->saved_data["affine"].toInt()), ctx->needs_input_grad(0),
+                                        has_weight && ctx->needs_input_grad(1), has_bias && ctx->needs_input_grad(bias_edge));
+    if (grads.dx.defined()) grads.dx = grads.dx.view(ctx->saved_data["shape"].toIntVector());
+    return {grads.dx, grads.dweight, grads.dbias, Tensor()};
+  }
+};
+
+bool norm_operands_fit(const Tensor& x, const MaybeTensor& weight, const MaybeTensor& bias, int64_t width) {
+  if (!plain_tensor(x) || dtype_code(x.scalar_type()) < 0 || x.dim() < 1 || x.size(-1) != width || width < 1 || width > 8192 || x.numel() == 0)
+    return false;
+  std::optional<at::ScalarType> affine;
+  for (const MaybeTensor* p : {&weight, &bias}) {
+    if (!p->has_value()) continue;
+    const Tensor& t = **p;
+    if (!plain_tensor(t) || t.device() != x.device() || t.dim() != 1 || t.size(0) != width) return false;
+    if (t.scalar_type() != x.scalar_type() && t.scalar_type() != at::kFloat) return false;
+    if (affine.has_value() && *affine != t.scalar_type()) return false;
+    affine = t.scalar_type();
+  }
+  return true;
+}
+
+std::optional<Tensor> layer_norm(const Tensor& x, int64_t width, const MaybeTensor& weight, const MaybeTensor& bias, double eps) {
+  if (!plain_context() || !norm_operands_fit(x, weight, bias, width)) return std::nullopt;
+  if (at::GradMode::is_enabled() && (x.requires_grad() || requires_grad(weight) || requires_grad(bias)))
+    return LayerNormFunction::apply(x, weight, bias, eps);
+  const Tensor w = weight.has_value() ? weight->contiguous() : Tensor(), b = bias.has_value() ? bias->contiguous() : Tensor();
+  return norm_forward(rows_of(x, width), w, b, eps, false).y.view(x.sizes());
+}
+
+// ---------------------------------------------------------------------------------------------
+// triangle multiplicative update
+// ---------------------------------------------------------------------------------------------
+
+struct UpdateShape {
+  int code;
+  int32_t prefix, tokens, padded, hidden;
+  int64_t cells() const { return int64_t(prefix) * tokens * tokens; }
+};
+
+// update[i, j] = sum_k left[i, k] right[j, k] (outgoing) or sum_k left[k, i] right[k, j], plane by plane
+Tensor contract(bool outgoing, const Tensor& left, const Tensor& right) {
+  return outgoing ? at::bmm(left, right.transpose(1, 2)) : at::bmm(left.transpose(1, 2), right);
+}
+
+enum { kLeftGate, kLeftValue, kRightGate, kRightValue, kOutputGate, kOutput, kProjections };
+
+struct UpdateFunction : Function<UpdateFunction> {
+  // `parameters`: the input and output norms' weight and bias, the six projection weights, then the biases that exist;
+  // `bias_of` says which projection each of those belongs to.
+  static Tensor forward(AutogradContext* ctx, const Tensor& pair, const MaybeTensor& mask, bool outgoing, double in_eps, double out_eps,
+                        at::TensorList parameters, const std::vector<int64_t>& bias_of) {
+    const auto type = pair.scalar_type();
+    const int64_t channels = pair.size(-1), tokens = pair.size(-2);
+    const Tensor* weights = &parameters[4];
+    const int64_t hidden = weights[0].size(0);
+    const UpdateShape s{dtype_code(type), int32_t(pair.numel() / (tokens * tokens * channels)), int32_t(tokens),
+                        int32_t((tokens + 7) / 8 * 8), int32_t(hidden)};
+    const c10::cuda::CUDAGuard guard(pair.device());
+    void* stream = current_stream(pair);
+    Tensor biases[kProjections];
+    bool stacked_has_bias = false;
+    for (size_t i = 0; i < bias_of.size(); ++i) {
+      biases[bias_of[i]] = parameters[10 + i];
+      stacked_has_bias = stacked_has_bias || bias_of[i] != kOutput;
+    }
+    // rows of the projections: left gate | left value | right gate | right value | output gate
+    const Tensor stacked = at::cat({weights[0], weights[1], weights[2], weights[3], weights[4]}).to(type);
+    Tensor stacked_bias;
+    if (stacked_has_bias) {
+      std::vector<Tensor> pieces;
+      for (int i = 0; i < kOutput; ++i) pieces.push_back(biases[i].defined() ? biases[i].to(type) : at::zeros({weights[i].size(0)}, pair.options()));
+      stacked_bias = at::cat(pieces);
+    }
+    const Tensor out_matrix = weights[kOutput].to(type);
+    const Tensor rows = rows_of(pair, channels), in_w = parameters[0].contiguous(), out_w = parameters[2].contiguous();
+    Normed x = norm_forward(rows, in_w, parameters[1].contiguous(), in_eps, true);
+    const Tensor proj = stacked_has_bias ? at::linear(x.y, stacked, stacked_bias) : at::linear(x.y, stacked);
+    const int64_t ld = proj.size(1);
+    const Tensor weight = mask.has_value() ? mask->to(type).expand(pair.sizes().slice(0, pair.dim() - 1)).contiguous() : Tensor();
+    const Tensor planes = at::empty({2, s.prefix * hidden, s.padded, s.padded}, pair.options());
+    const Tensor left = planes.select(0, 0), right = planes.select(0, 1);
+    check_status(oops_ta_pair_gate_forward(s.code, s.prefix, s.tokens, s.padded, s.hidden, proj.data_ptr(), ld, data_of(weight), left.data_ptr(),
+                                           right.data_ptr(), stream),
+                 "triangle_multiplication pair gate");
+    const Tensor update = contract(outgoing, left, right);
+    const Tensor normed = at::empty({s.cells(), hidden}, pair.options()), stats = floats_like(pair, {2, s.cells()});
+    check_status(oops_ta_channel_norm_forward(s.code, dtype_code(out_w.scalar_type()), s.prefix, s.tokens, s.padded, s.hidden, update.data_ptr(),
+                                              out_w.data_ptr(), parameters[3].contiguous().data_ptr(), float(out_eps), normed.data_ptr(),
+                                              stats.data_ptr<float>(), stats.data_ptr<float>() + s.cells(), stream),
+                 "triangle_multiplication output norm");
+    const Tensor values = biases[kOutput].defined() ? at::linear(normed, out_matrix, biases[kOutput].to(type)) : at::linear(normed, out_matrix);
+    const Tensor out = at::empty(pair.sizes(), pair.options());
+    const char* gate = static_cast<const char*>(proj.data_ptr()) + 4 * hidden * proj.element_size();
+    check_status(oops_ta_output_gate_forward(s.code, s.cells(), int32_t(channels), values.data_ptr(), gate, ld, out.data_ptr(), stream),
+                 "triangle_multiplication output gate");
+    if (ctx) {
+      ctx->set_materialize_grads(false);
+      ctx->save_for_backward({rows, in_w, x.stats, x.y, stacked, proj, weight, left, right, update, out_w, stats, normed, out_matrix, values});
+      ctx->saved_data["outgoing"] = outgoing;
+      ctx->saved_data["shape"] = pair.sizes().vec();
+      ctx->saved_data["dims"] = std::vector<int64_t>{s.prefix, s.tokens, s.padded, s.hidden, mask.has_value()};
+      ctx->saved_data["bias_of"] = bias_of;
+      std::vector<int64_t> types;
+      for (const Tensor& p : parameters) types.push_back(int64_t(p.scalar_type()));
+      ctx->saved_data["types"] = types;
+    }
+    return out;
+  }
+
+  static variable_list backward(AutogradContext* ctx, const variable_list& grad_outputs) {
+    const std::vector<int64_t> dims = ctx->saved_data["dims"].toIntVector(), bias_of = ctx->saved_data["bias_of"].toIntVector(),
+                               types = ctx->saved_data["types"].toIntVector();
+    // inputs: pair, mask, outgoing, in_eps, out_eps, parameters..., bias_of
+    constexpr size_t kFirst = 5;
+    variable_list result(kFirst + types.size() + 1);
+    if (!grad_outputs[0].defined()) return result;
+    variable_list saved = ctx->get_saved_variables();
+    for (Tensor& t : saved)
+      if (t.defined()) t = t.contiguous();
+    const Tensor &rows = saved[0], &in_w = saved[1], &stats1 = saved[2], &x = saved[3], &stacked = saved[4], &proj = saved[5], &weight = saved[6],
+                 &left = saved[7], &right = saved[8], &update = saved[9], &out_w = saved[10], &stats2 = saved[11], &normed = saved[12],
+                 &out_matrix = saved[13], &values = saved[14];
+    const UpdateShape s{dtype_code(proj.scalar_type()), int32_t(dims[0]), int32_t(dims[1]), int32_t(dims[2]), int32_t(dims[3])};
+    const size_t edge = dims[4] ? 2 : 1;  // first parameter's edge: behind the pair and, when it was given, the mask
+    auto need = [&](size_t parameter) { return ctx->needs_input_grad(edge + parameter); };
+    auto give = [&](size_t parameter, const Tensor& grad) { result[kFirst + parameter] = grad.to(at::ScalarType(types[parameter])); };
+    const int64_t hidden = s.hidden, cells = proj.size(0), ld = proj.size(1), channels = x.size(1);
+    const c10::cuda::CUDAGuard guard(proj.device());
+    void* stream = current_stream(proj);
+    const Tensor dout = rows_of(grad_outputs[0].resolve_neg().to(proj.scalar_type()), channels).contiguous();
+
+    const Tensor dvalues = at::empty_like(values), dproj = at::empty_like(proj);
+    const int64_t gate_at = 4 * hidden * proj.element_size();
+    check_status(oops_ta_output_gate_backward(s.code, cells, int32_t(channels), dout.data_ptr(), values.data_ptr(),
+                                              static_cast<const char*>(proj.data_ptr()) + gate_at, ld, dvalues.data_ptr(),
+                                              static_cast<char*>(dproj.data_ptr()) + gate_at, ld, stream),
+                 "triangle_multiplication output gate");
+    size_t output_bias = 0;
+    bool other_bias = false;
+    for (size_t i = 0; i < bias_of.size(); ++i) {
+      if (bias_of[i] == kOutput) output_bias = 10 + i;
+      else other_bias = other_bias || need(10 + i);
+    }
+    if (need(4 + kOutput)) give(4 + kOutput, at::mm(dvalues.t(), normed));
+    if (output_bias && need(output_bias)) give(output_bias, dvalues.sum(0));
+    const Tensor dnormed = at::mm(dvalues, out_matrix), dupdate = at::empty_like(update);
+    const Tensor dw2 = need(2) ? at::empty_like(out_w) : Tensor(), db2 = need(3) ? at::empty_like(out_w) : Tensor();
+    const uint64_t bytes = oops_ta_channel_norm_backward_workspace_bytes(s.code, s.prefix, s.tokens, s.padded, s.hidden);
+    const Tensor scratch = bytes_like(proj, bytes);
+    check_status(oops_ta_channel_norm_backward(s.code, dtype_code(out_w.scalar_type()), s.prefix, s.tokens, s.padded, s.hidden,
+                                               dnormed.data_ptr(), update.data_ptr(), out_w.data_ptr(), stats2.data_ptr<float>(),
+                                               stats2.data_ptr<float>() + cells, dupdate.data_ptr(), data_of(dw2), data_of(db2),
+                                               scratch.data_ptr(), bytes, stream),
+                 "triangle_multiplication output norm");
+    result[kFirst + 2] = dw2;
+    result[kFirst + 3] = db2;
+    bool weights_wanted = false;
+    for (size_t i = 0; i < size_t(kOutput); ++i) weights_wanted = weights_wanted || need(4 + i);
+    const bool pair_wanted = ctx->needs_input_grad(0), norm_wanted = pair_wanted || need(0) || need(1);
+    if (!weights_wanted && !other_bias && !norm_wanted) return result;
+
+    const bool outgoing = ctx->saved_data["outgoing"].toBool();
+    const Tensor dleft = outgoing ? at::bmm(dupdate, right) : at::bmm(right, dupdate.transpose(1, 2));
+    const Tensor dright = outgoing ? at::bmm(dupdate.transpose(1, 2), left) : at::bmm(left, dupdate);
+    check_status(oops_ta_pair_gate_backward(s.code, s.prefix, s.tokens, s.padded, s.hidden, proj.data_ptr(), ld, data_of(weight),
+                                            dleft.data_ptr(), dright.data_ptr(), dproj.data_ptr(), ld, stream),
+                 "triangle_multiplication pair gate");
+    auto piece = [&](const Tensor& t, int64_t which) { return t.narrow(0, which * hidden, which == kOutputGate ? channels : hidden); };
+    if (weights_wanted) {
+      const Tensor stacked_grad = at::mm(dproj.t(), x);
+      for (int64_t i = 0; i < kOutput; ++i)
+        if (need(4 + i)) give(4 + i, piece(stacked_grad, i));
+    }
+    if (other_bias) {
+      const Tensor sums = dproj.sum(0);
+      for (size_t i = 0; i < bias_of.size(); ++i)
+        if (bias_of[i] != kOutput && need(10 + i)) give(10 + i, piece(sums, bias_of[i]));
+    }
+    if (norm_wanted) {
+      NormGradients grads = norm_backward(at::mm(dproj, stacked), rows_of(rows, channels), in_w, stats1, in_w.scalar_type(), pair_wanted,
+                                          need(0), need(1));
+      if (pair_wanted) result[0] = grads.dx.view(ctx->saved_data["shape"].toIntVector());
+      result[kFirst] = grads.dweight;
+      result[kFirst + 1] = grads.dbias;
+    }
+    return result;
+  }
+};
+
+// ---------------------------------------------------------------------------------------------
+// Python boundary
+// ---------------------------------------------------------------------------------------------
+
+MaybeTensor maybe_tensor(PyObject* o) { return o == Py_None ? MaybeTensor() : MaybeTensor(THPVariable_Unpack(o)); }
+bool tensor_or_none(PyObject* o) { return o == Py_None || THPVariable_Check(o); }
+std::optional<double> maybe_double(PyObject* o) {
+  if (o == Py_None) return std::nullopt;
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) throw python_error();
+  return v;
+}
+
+PyObject* wrap(std::optional<Tensor>&& t) {
+  if (!t.has_value()) Py_RETURN_NONE;
+  return THPVariable_Wrap(std::move(*t));
+}
+
+// triangle_attention(query, key, value, mask, bias, scale, flags) -> Tensor or None
+PyObject* py_triangle_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 7, "triangle_attention takes 7 arguments");
+  if (!THPVariable_Check(a[0]) || !THPVariable_Check(a[1]) || !THPVariable_Check(a[2]) || !tensor_or_none(a[3]) || !tensor_or_none(a[4]))
+    Py_RETURN_NONE;
+  const Tensor &q = THPVariable_Unpack(a[0]), &k = THPVariable_Unpack(a[1]), &v = THPVariable_Unpack(a[2]);
+  const MaybeTensor mask = maybe_tensor(a[3]), bias = maybe_tensor(a[4]);
+  const std::optional<double> scale = maybe_double(a[5]);
+  const int64_t flags = PyLong_AsLongLong(a[6]);
+  std::optional<Tensor> out;
+  {
+    py::gil_scoped_release no_gil;
+    out = dense_attention(q, k, v, mask, bias, scale, flags);
+  }
+  return wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// triangle_attention_gated(query, key, value, gate, mask, bias, scale, flags) -> Tensor or None
+PyObject* py_gated_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 8, "triangle_attention_gated takes 8 arguments");
+  for (int i = 0; i < 4; ++i)
+    if (!THPVariable_Check(a[i])) Py_RETURN_NONE;
+  if (!tensor_or_none(a[4]) || !tensor_or_none(a[5])) Py_RETURN_NONE;
+  const Tensor &q = THPVariable_Unpack(a[0]), &k = THPVariable_Unpack(a[1]), &v = THPVariable_Unpack(a[2]), &g = THPVariable_Unpack(a[3]);
+  const MaybeTensor mask = maybe_tensor(a[4]), bias = maybe_tensor(a[5]);
+  const std::optional<double> scale = maybe_double(a[6]);
+  const int64_t flags = PyLong_AsLongLong(a[7]);
+  std::optional<Tensor> out;
+  {
+    py::gil_scoped_release no_gil;
+    out = dense_gated_attention(q, k, v, g, mask, bias, scale, flags);
+  }
+  return wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// layer_norm(x, width, weight, bias, eps) -> Tensor or None
+PyObject* py_layer_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 5, "layer_norm takes 5 arguments");
+  if (!THPVariable_Check(a[0]) || !PyLong_Check(a[1]) || !tensor_or_none(a[2]) || !tensor_or_none(a[3])) Py_RETURN_NONE;
+  const Tensor& x = THPVariable_Unpack(a[0]);
+  const int64_t width = PyLong_AsLongLong(a[1]);
+  const MaybeTensor weight = maybe_tensor(a[2]), bias = maybe_tensor(a[3]);
+  const double eps = *maybe_double(a[4]);
+  std::optional<Tensor> out;
+  {
+    py::gil_scoped_release no_gil;
+    out = layer_norm(x, width, weight, bias, eps);
+  }
+  return wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef g_fast_methods[] = {
+    {"triangle_attention", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_triangle_attention)), METH_FASTCALL, nullptr},
+    {"triangle_attention_gated", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_gated_attention)), METH_FASTCALL, nullptr},
+    {"layer_norm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_layer_norm)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+}  // namespace
+
+PYBIND11_MODULE(_native, m) {
+  PyModule_AddFunctions(m.ptr(), g_fast_methods);
+  using NoGil = py::call_guard<py::gil_scoped_release>;
+  auto or_empty = [](const MaybeTensor& t) { return t.value_or(Tensor()); };
+  m.def("set_unsupported_error", [](py::object type) { g_unsupported_error = type.release().ptr(); });
+  m.def("check_device_status", [](bool enabled) { return g_check_status.exchange(enabled); });
+  m.def("attend", [](const Tensor& q, const Tensor& k, const Tensor& v, const MaybeTensor& mask, const MaybeTensor& bias, double scale,
+                     const std::vector<int64_t>& geometry, int64_t flags) {
+    return attend(q, k, v, mask, bias, scale, Geometry::decode(geometry), flags);
+  }, NoGil());
+  m.def("gated_attend", &gated_attend, NoGil());
+  m.def("run_forward", [or_empty](const std::vector<int64_t>& geometry, const Tensor& q, const Tensor& k, const Tensor& v,
+                                  const MaybeTensor& mask, const MaybeTensor& bias, double scale, int64_t flags, bool want_lse) {
+    auto [out, lse] = run_forward(Geometry::decode(geometry), q, k, v, or_empty(mask), or_empty(bias), scale, flags, want_lse);
+    return std::make_tuple(out, lse.defined() ? MaybeTensor(lse) : MaybeTensor());
+  }, NoGil());
+  m.def("run_backward", [or_empty](const std::vector<int64_t>& geometry, const Tensor& grad_out, const Tensor& q, const Tensor& k,
+                                   const Tensor& v, const MaybeTensor& mask, const MaybeTensor& bias, const Tensor& out, const Tensor& lse,
+                                   double scale, int64_t flags, const std::vector<bool>& need, const MaybeTensor& scratch,
+                                   bool dbias_f32) {
+    Gradients g = run_backward(Geometry::decode(geometry), grad_out, q, k, v, or_empty(mask), or_empty(bias), out, lse, scale, flags, need[0],
+                               need[1], need[2], need[3], or_empty(scratch),
+                               dbias_f32 ? std::optional<at::ScalarType>(at::kFloat) : std::nullopt);
+    auto maybe = [](const Tensor& t) { return t.defined() ? MaybeTensor(t) : MaybeTensor(); };
+    return std::make_tuple(maybe(g.dq), maybe(g.dk), maybe(g.dv), maybe(g.dbias));
+  }, NoGil());
+  m.def("sigmoid_gate", [](const Tensor& attention, const Tensor& gate) { return Tensor(GateFunction::apply(attention, gate)); }, NoGil());
+  m.def("run_gate", &run_gate, NoGil());
+  m.def("pair_update", [](const Tensor& pair, const MaybeTensor& mask, bool outgoing, double in_eps, double out_eps,
+                          const std::vector<Tensor>& parameters, const std::vector<int64_t>& bias_of) {
+    bool wanted = pair.requires_grad();
+    for (const Tensor& p : parameters) wanted = wanted || p.requires_grad();
+    if (at::GradMode::is_enabled() && wanted)
+      return Tensor(UpdateFunction::apply(pair, mask, outgoing, in_eps, out_eps, at::TensorList(parameters), bias_of));
+    return UpdateFunction::forward(nullptr, pair, mask, outgoing, in_eps, out_eps, parameters, bias_of);
+  }, NoGil());
+}

@@ -16,8 +16,10 @@ from typing import Iterable, Optional
 
 import torch
 from torch import Tensor
+from torch.autograd import forward_ad
 
-from ..runtime import cabi, require_no_forward_mode, require_same_device, unsupported
+from ..runtime import require_no_forward_mode, require_same_device, unsupported
+from ..runtime.native import native
 from ..runtime.nested_tensor import is_nested
 
 _NAME = "layer_norm"
@@ -26,87 +28,23 @@ _DTYPE_CODES = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
 _HALF = (torch.float16, torch.bfloat16)
 
 
-def _rows_of(t: Tensor, width: int) -> Tensor:
-    """`t` as (rows, width) with contiguous rows; a view when the layout allows it."""
-    flat = t.reshape(-1, width)
-    if (width > 1 and flat.stride(1) != 1) or (flat.shape[0] > 1 and flat.stride(0) < width):
-        flat = flat.contiguous()
-    return flat
-
-
-def _check_status(status: int) -> None:
-    if status:
-        raise unsupported(_NAME, cabi.status_message(status))
-
-
-def forward_rows(rows_in: Tensor, weight: Optional[Tensor], bias: Optional[Tensor], eps: float):
-    """`(y, mean, rstd)` of (rows, width) activations; contiguous parameters of one dtype."""
-    rows, width = rows_in.shape
-    out = torch.empty((rows, width), dtype=rows_in.dtype, device=rows_in.device)
-    stats = torch.empty((2, rows), dtype=torch.float32, device=rows_in.device)
-    affine = weight if weight is not None else bias
-    lib = cabi.library()
-    with torch.cuda.device(rows_in.device):
-        _check_status(lib.oops_ta_layer_norm_forward(
-            _DTYPE_CODES[rows_in.dtype], _DTYPE_CODES[affine.dtype if affine is not None else rows_in.dtype], rows, width,
-            rows_in.data_ptr(), rows_in.stride(0) if rows > 1 else width, weight.data_ptr() if weight is not None else None,
-            bias.data_ptr() if bias is not None else None, float(eps), out.data_ptr(), width, stats.data_ptr(),
-            stats.data_ptr() + 4 * rows, torch.cuda.current_stream(rows_in.device).cuda_stream))
-    return out, stats[0], stats[1]
-
-
-def backward_rows(dy: Tensor, rows_in: Tensor, weight: Optional[Tensor], mean: Tensor, rstd: Tensor, affine_dtype: torch.dtype,
-                  need_x: bool, need_w: bool, need_b: bool):
-    """`(dx, dweight, dbias)` (None where not wanted) of at least one row."""
-    rows, width = rows_in.shape
-    device = rows_in.device
-    dx = torch.empty((rows, width), dtype=rows_in.dtype, device=device) if need_x else None
-    dw = torch.empty(width, dtype=affine_dtype, device=device) if need_w else None
-    db = torch.empty(width, dtype=affine_dtype, device=device) if need_b else None
-    lib = cabi.library()
-    need = lib.oops_ta_layer_norm_backward_workspace_bytes(rows, width) if (need_w or need_b) else 0
-    scratch = torch.empty(max(int(need), 1), dtype=torch.uint8, device=device)
-    with torch.cuda.device(device):
-        _check_status(lib.oops_ta_layer_norm_backward(
-            _DTYPE_CODES[rows_in.dtype], _DTYPE_CODES[affine_dtype], rows, width, dy.data_ptr(), dy.stride(0) if rows > 1 else width,
-            rows_in.data_ptr(), rows_in.stride(0) if rows > 1 else width, weight.data_ptr() if weight is not None else None,
-            mean.data_ptr(), rstd.data_ptr(), dx.data_ptr() if need_x else None, width,
-            dw.data_ptr() if need_w else None, db.data_ptr() if need_b else None, scratch.data_ptr(), int(need),
-            torch.cuda.current_stream(device).cuda_stream))
-    return dx, dw, db
-
-
-class _LayerNorm(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x: Tensor, weight: Optional[Tensor], bias: Optional[Tensor], eps: float):
-        rows_in = _rows_of(x.detach(), x.shape[-1])
-        affine = next((p for p in (weight, bias) if p is not None), None)
-        w = weight.detach().contiguous() if weight is not None else None
-        b = bias.detach().contiguous() if bias is not None else None
-        out, mean, rstd = forward_rows(rows_in, w, b, eps)
-        ctx.save_for_backward(rows_in, w, mean, rstd)
-        ctx.has_weight, ctx.has_bias = weight is not None, bias is not None
-        ctx.affine_dtype = affine.dtype if affine is not None else x.dtype
-        ctx.shape = x.shape
-        return out.view(x.shape)
-
-    @staticmethod
-    def backward(ctx, grad_out: Tensor):
-        rows_in, w, mean, rstd = ctx.saved_tensors
-        dy = _rows_of(grad_out, rows_in.shape[1])
-        need_x, need_w, need_b = ctx.needs_input_grad[0], ctx.has_weight and ctx.needs_input_grad[1], ctx.has_bias and ctx.needs_input_grad[2]
-        dx, dw, db = backward_rows(dy, rows_in, w, mean, rstd, ctx.affine_dtype, need_x, need_w, need_b)
-        return (dx.view(ctx.shape) if need_x else None), dw, db, None
-
-
 def layer_norm(input, normalized_shape, weight: Optional[Tensor] = None, bias: Optional[Tensor] = None, eps: float = 1e-5):
     """Normalize the final feature dimension of CUDA activations; see the module docstring."""
+    width = normalized_shape if isinstance(normalized_shape, int) else None
+    if width is not None and forward_ad._current_level < 0:
+        out = native().layer_norm(input, width, weight, bias, eps)
+        if out is not None:
+            return out
     if is_nested(input):
         return _layer_norm_nested(input, normalized_shape, weight, bias, eps)
     require_no_forward_mode(_NAME, input, weight, bias)
     require_same_device(_NAME, input, weight, bias)
     check_admission(input, normalized_shape, weight, bias)
-    return _LayerNorm.apply(input, weight, bias, eps)
+    input, weight, bias = (t if t is None else t.resolve_neg() for t in (input, weight, bias))
+    out = native().layer_norm(input, input.shape[-1], weight, bias, eps)
+    if out is None:  # served layouts behind a transform or a tensor subclass
+        raise unsupported(_NAME, "does not support torch.func transforms or dispatching tensor subclasses")
+    return out
 
 
 def check_admission(input, normalized_shape, weight: Optional[Tensor], bias: Optional[Tensor]) -> None:

@@ -24,8 +24,9 @@ import torch
 from torch import Tensor
 from torch.nn import functional as F
 
-from ..normalization.layer_norm import _rows_of, backward_rows, check_admission, forward_rows, layer_norm
-from ..runtime import cabi, require_no_forward_mode, require_same_device, unsupported
+from ..normalization.layer_norm import check_admission, layer_norm
+from ..runtime import require_no_forward_mode, require_same_device, unsupported
+from ..runtime.native import native
 from ..runtime.nested_tensor import is_nested
 
 _NAME = "triangle_multiplication"
@@ -68,10 +69,13 @@ def triangle_multiplication(pair, pair_mask: Optional[Tensor] = None, *, directi
     projections = (left_gate_weight, left_value_weight, right_gate_weight, right_value_weight, output_gate_weight, output_weight)
     biases = (left_gate_bias, left_value_bias, right_gate_bias, right_value_bias, output_gate_bias, output_bias)
     if _fused_serves(pair, pair_mask, hidden, (*projections, *biases)):
-        check_admission(pair, channels, input_norm_weight, input_norm_bias)
-        check_admission(pair.new_empty(1, dtype=pair.dtype).expand(hidden), hidden, output_norm_weight, output_norm_bias)
-        return _FusedUpdate.apply(pair, pair_mask, direction == "outgoing", input_norm_weight, input_norm_bias, input_norm_eps,
-                                  output_norm_weight, output_norm_bias, output_norm_eps, *projections, *biases)
+        for width, weight, bias in ((channels, input_norm_weight, input_norm_bias), (hidden, output_norm_weight, output_norm_bias)):
+            if weight.dtype is not bias.dtype or weight.dtype not in (pair.dtype, torch.float32):
+                check_admission(pair.new_empty(width), width, weight, bias)  # raises
+        norms = [input_norm_weight, input_norm_bias, output_norm_weight, output_norm_bias]
+        given = [i for i, bias in enumerate(biases) if bias is not None]
+        return native().pair_update(pair, pair_mask, direction == "outgoing", float(input_norm_eps), float(output_norm_eps),
+                                    [*norms, *projections, *(biases[i] for i in given)], given)
 
     x = layer_norm(pair, channels, input_norm_weight, input_norm_bias, input_norm_eps)
     weight = 1.0 if pair_mask is None else pair_mask.to(x.dtype).unsqueeze(-1)
@@ -113,115 +117,3 @@ def _fused_serves(pair: Tensor, mask: Optional[Tensor], hidden: int, parameters)
         and (mask is None or (not mask.requires_grad and not mask.is_complex() and mask.dim() < pair.dim()
                               and all(own in (1, want) for own, want in zip(reversed(mask.shape), reversed(pair.shape[:-1])))))
     )
-
-
-def _run(name: str, device: torch.device, *arguments) -> None:
-    with torch.cuda.device(device):
-        status = getattr(cabi.library(), name)(*arguments, torch.cuda.current_stream(device).cuda_stream)
-    if status:
-        raise RuntimeError(f"{_NAME} {name} failed: {cabi.status_message(status)}")
-
-
-def _address(tensor: Optional[Tensor]) -> Optional[int]:
-    return None if tensor is None else tensor.data_ptr()
-
-
-def _contract(outgoing: bool, left: Tensor, right: Tensor) -> Tensor:
-    """update[i, j] = sum_k left[i, k] right[j, k] (outgoing) or sum_k left[k, i] right[k, j], plane by plane."""
-    return torch.bmm(left, right.transpose(1, 2)) if outgoing else torch.bmm(left.transpose(1, 2), right)
-
-
-class _FusedUpdate(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, pair, mask, outgoing, in_weight, in_bias, in_eps, out_weight, out_bias, out_eps, *parameters):
-        weights, biases = parameters[:6], parameters[6:]
-        dtype, device, channels = pair.dtype, pair.device, pair.shape[-1]
-        hidden, tokens = weights[0].shape[0], pair.shape[-2]
-        prefix = pair.numel() // (tokens * tokens * channels)
-        padded = -(-tokens // 8) * 8
-        cells, code = prefix * tokens * tokens, cabi.DTYPE_CODE[dtype]
-        dims = (prefix, tokens, padded, hidden)
-        # rows of the projections: left gate | left value | right gate | right value | output gate
-        stacked = torch.cat([w.detach() for w in weights[:5]]).to(dtype)
-        stacked_bias = None
-        if any(b is not None for b in biases[:5]):
-            stacked_bias = torch.cat([w.new_zeros(w.shape[0]) if b is None else b.detach().to(w.dtype)
-                                      for w, b in zip(weights[:5], biases[:5])]).to(dtype)
-        out_matrix = weights[5].detach().to(dtype)
-        rows_in = _rows_of(pair.detach(), channels)
-        x, mean1, rstd1 = forward_rows(rows_in, in_weight.detach().contiguous(), in_bias.detach().contiguous(), in_eps)
-        proj = F.linear(x, stacked, stacked_bias)
-        ld = proj.shape[1]
-        weight = None if mask is None else mask.detach().to(dtype).expand(pair.shape[:-1]).contiguous()
-        planes = torch.empty((2, prefix * hidden, padded, padded), dtype=dtype, device=device)
-        left, right = planes[0], planes[1]
-        _run("oops_ta_pair_gate_forward", device, code, *dims, proj.data_ptr(), ld, _address(weight), left.data_ptr(), right.data_ptr())
-        update = _contract(outgoing, left, right)
-        normed = torch.empty((cells, hidden), dtype=dtype, device=device)
-        stats2 = torch.empty((2, cells), dtype=torch.float32, device=device)
-        out_w = out_weight.detach().contiguous()
-        _run("oops_ta_channel_norm_forward", device, code, cabi.DTYPE_CODE[out_w.dtype], *dims, update.data_ptr(), out_w.data_ptr(),
-             out_bias.detach().contiguous().data_ptr(), float(out_eps), normed.data_ptr(), stats2.data_ptr(), stats2[1].data_ptr())
-        values = F.linear(normed, out_matrix, None if biases[5] is None else biases[5].detach().to(dtype))
-        out = torch.empty(pair.shape, dtype=dtype, device=device)
-        gate_at = proj.data_ptr() + 4 * hidden * proj.element_size()
-        _run("oops_ta_output_gate_forward", device, code, cells, channels, values.data_ptr(), gate_at, ld, out.data_ptr())
-        ctx.set_materialize_grads(False)
-        ctx.save_for_backward(rows_in, in_weight.detach().contiguous(), mean1, rstd1, x, stacked, proj, weight, left, right, update, out_w,
-                              stats2, normed, out_matrix, values)
-        ctx.outgoing, ctx.dims, ctx.shape = outgoing, dims, pair.shape
-        ctx.like = [None if p is None else p.dtype for p in parameters]
-        return out
-
-    @staticmethod
-    def backward(ctx, grad_out):
-        if grad_out is None:
-            return (None,) * 21
-        (rows_in, in_w, mean1, rstd1, x, stacked, proj, weight, left, right, update, out_w, stats2, normed, out_matrix,
-         values) = (t if t is None else t.contiguous() for t in ctx.saved_tensors)
-        need = ctx.needs_input_grad
-        dims, device, code = ctx.dims, proj.device, cabi.DTYPE_CODE[proj.dtype]
-        hidden, (cells, ld), channels = dims[3], proj.shape, x.shape[1]
-        grads: list = [None] * 21
-        dout = _rows_of(grad_out.resolve_neg().to(proj.dtype), channels).contiguous()
-
-        dvalues, dproj = torch.empty_like(values), torch.empty_like(proj)
-        gate_offset = 4 * hidden * proj.element_size()
-        _run("oops_ta_output_gate_backward", device, code, cells, channels, dout.data_ptr(), values.data_ptr(),
-             proj.data_ptr() + gate_offset, ld, dvalues.data_ptr(), dproj.data_ptr() + gate_offset, ld)
-        if need[14]:
-            grads[14] = (dvalues.t() @ normed).to(ctx.like[5])
-        if need[20]:
-            grads[20] = dvalues.sum(0).to(ctx.like[11])
-        dnormed = dvalues @ out_matrix
-        dupdate = torch.empty_like(update)
-        dw2 = torch.empty_like(out_w) if need[6] else None
-        db2 = torch.empty_like(out_w) if need[7] else None
-        nbytes = cabi.library().oops_ta_channel_norm_backward_workspace_bytes(code, *dims)
-        scratch = torch.empty(int(nbytes), dtype=torch.uint8, device=device)
-        _run("oops_ta_channel_norm_backward", device, code, cabi.DTYPE_CODE[out_w.dtype], *dims, dnormed.data_ptr(), update.data_ptr(),
-             out_w.data_ptr(), stats2.data_ptr(), stats2[1].data_ptr(), dupdate.data_ptr(), _address(dw2), _address(db2),
-             scratch.data_ptr(), int(nbytes))
-        grads[6], grads[7] = dw2, db2
-        if not any(need[i] for i in (0, 3, 4, *range(9, 14), *range(15, 20))):
-            return tuple(grads)
-        if ctx.outgoing:
-            dleft, dright = torch.bmm(dupdate, right), torch.bmm(dupdate.transpose(1, 2), left)
-        else:
-            dleft, dright = torch.bmm(right, dupdate.transpose(1, 2)), torch.bmm(left, dupdate)
-        _run("oops_ta_pair_gate_backward", device, code, *dims, proj.data_ptr(), ld, _address(weight), dleft.data_ptr(),
-             dright.data_ptr(), dproj.data_ptr(), ld)
-        extents = [hidden] * 4 + [channels]
-        if any(need[9:14]):
-            stacked_grad = dproj.t() @ x
-            for i, piece in enumerate(stacked_grad.split(extents)):
-                if need[9 + i]:
-                    grads[9 + i] = piece.to(ctx.like[i])
-        if any(need[15:20]):
-            for i, piece in enumerate(dproj.sum(0).split(extents)):
-                if need[15 + i]:
-                    grads[15 + i] = piece.to(ctx.like[6 + i])
-        if need[0] or need[3] or need[4]:
-            dx, grads[3], grads[4] = backward_rows(dproj @ stacked, rows_in, in_w, mean1, rstd1, in_w.dtype, need[0], need[3], need[4])
-            grads[0] = None if dx is None else dx.view(ctx.shape)
-        return tuple(grads)
