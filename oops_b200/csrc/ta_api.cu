@@ -63,6 +63,12 @@ int validate(const oops_ta_problem* p, bool need_pointers) {
 
 bool force_generic(const oops_ta_problem* p) { return (p->flags & OOPS_TA_FLAG_FORCE_GENERIC) != 0; }
 
+// The forward pass of a problem the tcgen05 kernels do not take.
+int untiled_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, cudaStream_t stream) {
+  if (!force_generic(&p) && f32_forward_applies(p)) return f32_forward(p, out, lse, stream);
+  return generic_forward(p, out, lse, stream);
+}
+
 int check_device() {
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess) return fail(OOPS_TA_CUDA_ERROR, "cudaGetDevice failed");
@@ -119,6 +125,7 @@ int oops_ta_uses_tensor_path(const oops_ta_problem* problem, int backward) {
 uint64_t oops_ta_forward_workspace_bytes(const oops_ta_problem* problem) {
   if (validate(problem, false)) return 0;
   if (!force_generic(problem) && tensor_forward_applies(*problem)) return tensor_forward_workspace(*problem);
+  if (!force_generic(problem) && f32_forward_applies(*problem)) return 0;
   return generic_forward_workspace(*problem);
 }
 
@@ -126,6 +133,7 @@ uint64_t oops_ta_backward_workspace_bytes(const oops_ta_problem* problem, const 
   if (validate(problem, false) || !grads) return 0;
   if (!force_generic(problem) && tensor_backward_applies(*problem, grads))
     return tensor_backward_workspace(*problem, *grads);
+  if (!force_generic(problem) && f32_backward_applies(*problem)) return f32_backward_workspace(*problem, *grads);
   return generic_backward_workspace(*problem, *grads);
 }
 
@@ -138,7 +146,7 @@ int oops_ta_forward(const oops_ta_problem* problem, const oops_ta_pair* out, flo
   g_error[0] = 0;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (!force_generic(problem) && tensor_forward_applies(*problem)) return tensor_forward(*problem, *out, lse, s);
-  return generic_forward(*problem, *out, lse, s);
+  return untiled_forward(*problem, *out, lse, s);
 }
 
 int oops_ta_forward_gated(const oops_ta_problem* problem, const oops_ta_pair* gate, const oops_ta_pair* gated,
@@ -157,7 +165,7 @@ int oops_ta_forward_gated(const oops_ta_problem* problem, const oops_ta_pair* ga
   // layout-agnostic kernels: the attention values first (into `plain`, or into `gated` itself when the caller
   // keeps no ungated copy), then the element-wise gate
   const oops_ta_pair& values = kept.ptr ? kept : *gated;
-  status = generic_forward(*problem, values, lse, s);
+  status = untiled_forward(*problem, values, lse, s);
   if (status) return status;
   return gate_forward(problem->dtype, problem->batch, problem->rows, problem->cols, problem->heads, problem->head_dim, values,
                       *gate, *gated, s);
@@ -337,6 +345,7 @@ int oops_ta_backward(const oops_ta_problem* problem, const oops_ta_pair* out, co
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (!force_generic(problem) && tensor_backward_applies(*problem, grads))
     return tensor_backward(*problem, *out, *dout, lse, *grads, s);
+  if (!force_generic(problem) && f32_backward_applies(*problem)) return f32_backward(*problem, *out, *dout, lse, *grads, s);
   return generic_backward(*problem, *out, *dout, lse, *grads, s);
 }
 

@@ -28,6 +28,14 @@ int generic_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* ls
 int generic_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_ta_pair& dout, const float* lse,
                      const oops_ta_grads& g, cudaStream_t stream);
 
+// FFMA kernels that keep the scores on chip (f32, head_dim <= 64, any strides).
+bool f32_forward_applies(const oops_ta_problem& p);
+bool f32_backward_applies(const oops_ta_problem& p);
+uint64_t f32_backward_workspace(const oops_ta_problem& p, const oops_ta_grads& g);
+int f32_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, cudaStream_t stream);
+int f32_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_ta_pair& dout, const float* lse,
+                 const oops_ta_grads& g, cudaStream_t stream);
+
 // The layout-agnostic forward pass on the library's built-in scratch array (no caller workspace).
 uint64_t static_forward_capacity();
 int static_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, cudaStream_t stream);
