@@ -66,6 +66,7 @@ bool force_generic(const oops_ta_problem* p) { return (p->flags & OOPS_TA_FLAG_F
 // The forward pass of a problem the tcgen05 kernels do not take.
 int untiled_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, cudaStream_t stream) {
   if (!force_generic(&p) && f32_forward_applies(p)) return f32_forward(p, out, lse, stream);
+  if (!force_generic(&p) && mma_applies(p)) return mma_forward(p, out, lse, stream);
   return generic_forward(p, out, lse, stream);
 }
 
@@ -125,7 +126,7 @@ int oops_ta_uses_tensor_path(const oops_ta_problem* problem, int backward) {
 uint64_t oops_ta_forward_workspace_bytes(const oops_ta_problem* problem) {
   if (validate(problem, false)) return 0;
   if (!force_generic(problem) && tensor_forward_applies(*problem)) return tensor_forward_workspace(*problem);
-  if (!force_generic(problem) && f32_forward_applies(*problem)) return 0;
+  if (!force_generic(problem) && (f32_forward_applies(*problem) || mma_applies(*problem))) return 0;
   return generic_forward_workspace(*problem);
 }
 
@@ -134,6 +135,7 @@ uint64_t oops_ta_backward_workspace_bytes(const oops_ta_problem* problem, const 
   if (!force_generic(problem) && tensor_backward_applies(*problem, grads))
     return tensor_backward_workspace(*problem, *grads);
   if (!force_generic(problem) && f32_backward_applies(*problem)) return f32_backward_workspace(*problem, *grads);
+  if (!force_generic(problem) && mma_applies(*problem)) return mma_backward_workspace(*problem, *grads);
   return generic_backward_workspace(*problem, *grads);
 }
 
@@ -346,6 +348,7 @@ int oops_ta_backward(const oops_ta_problem* problem, const oops_ta_pair* out, co
   if (!force_generic(problem) && tensor_backward_applies(*problem, grads))
     return tensor_backward(*problem, *out, *dout, lse, *grads, s);
   if (!force_generic(problem) && f32_backward_applies(*problem)) return f32_backward(*problem, *out, *dout, lse, *grads, s);
+  if (!force_generic(problem) && mma_applies(*problem)) return mma_backward(*problem, *out, *dout, lse, *grads, s);
   return generic_backward(*problem, *out, *dout, lse, *grads, s);
 }
 

@@ -36,6 +36,13 @@ int f32_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, c
 int f32_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_ta_pair& dout, const float* lse,
                  const oops_ta_grads& g, cudaStream_t stream);
 
+// Register-level matrix-product kernels (f16/bf16, head_dim <= 64, any strides and bias type).
+bool mma_applies(const oops_ta_problem& p);
+uint64_t mma_backward_workspace(const oops_ta_problem& p, const oops_ta_grads& g);
+int mma_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, cudaStream_t stream);
+int mma_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_ta_pair& dout, const float* lse,
+                 const oops_ta_grads& g, cudaStream_t stream);
+
 // The layout-agnostic forward pass on the library's built-in scratch array (no caller workspace).
 uint64_t static_forward_capacity();
 int static_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, cudaStream_t stream);

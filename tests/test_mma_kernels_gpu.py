@@ -1,0 +1,70 @@
+"""The 16-bit kernels for head sizes and layouts the tcgen05 kernels do not take, at the sizes where their 64 x 64 tiles and
+16-channel groups end: head sizes that are no multiple of 8, unaligned rows, f32 biases, masks that drop tiles and rows,
+several parts of the bias gradient; against the oracle in f64.  Products are exact or carry 16 mantissa bits, so the forward
+result is off by its own rounding (half a unit: 2^-9 bf16, 2^-12 f16, of the largest value; twice that is allowed); the
+gradients see the rounded output through delta = sum(out * dout), whose error is that rounding times |dout| summed over the
+head (sqrt(64) at most): eight times the forward bound."""
+
+import pytest
+import torch
+
+from oracle import triangle_oracle as oracle
+from oops_b200 import triangle_attention
+from oops_b200.runtime import cabi
+
+pytestmark = pytest.mark.gpu
+ROUNDING = {torch.bfloat16: 2.0**-8, torch.float16: 2.0**-11}
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,cols,heads,dim,bias_kind,mask_kind,layout",
+                         [(3, 1, 2, 8, "none", "none", "plain"), (5, 63, 3, 1, "shared", "random", "plain"),
+                          (40, 64, 2, 64, "shared", "ones", "plain"), (9, 65, 2, 40, "full", "tokens", "plain"),
+                          (70, 130, 2, 24, "shared32", "tokens", "swapped"), (6, 200, 2, 48, "shared", "random", "head"),
+                          (4, 97, 2, 33, "full32", "random", "swapped"), (8, 72, 2, 32, "shared", "random", "odd"),
+                          (5, 136, 2, 32, "shared32", "none", "plain")])
+def test_tile_edges(cuda, dtype, rows, cols, heads, dim, bias_kind, mask_kind, layout):
+    gen = torch.Generator().manual_seed(cols)
+    shape = (1, rows, cols, heads, dim)
+    q, k, v = ((0.5 * torch.randn(shape, generator=gen)).to(dtype) for _ in range(3))
+    up = torch.randn(shape, generator=gen).to(dtype)
+    bias = None
+    if bias_kind != "none":
+        groups = 1 if bias_kind.startswith("shared") else rows
+        bias = torch.randn(1, groups, heads, cols, cols, generator=gen).to(torch.float32 if bias_kind.endswith("32") else dtype)
+    mask = {"none": None, "ones": torch.ones(1, rows, cols, dtype=torch.bool),
+            "random": torch.rand(1, rows, cols, generator=gen) > 0.3,
+            "tokens": ((torch.arange(cols) < max(1, cols // 2 - 3)) & (torch.arange(rows)[:, None] > 1))[None]}[mask_kind]
+    if mask is not None:  # dropped keys may hold anything
+        k, v = k.masked_fill(~mask[..., None, None], float("inf")), v.masked_fill(~mask[..., None, None], float("nan"))
+
+    def laid_out(t):
+        t = t.to(cuda)
+        if layout == "swapped":
+            t = t.transpose(1, 2).contiguous().transpose(1, 2)
+        elif layout == "head":
+            t = t.transpose(2, 3).contiguous().transpose(2, 3)
+        elif layout == "odd":  # rows that start 2 bytes behind a 16-byte boundary
+            t = torch.nn.functional.pad(t, (1, 0))[..., 1:]
+        return t.detach().requires_grad_(True)
+
+    leaves = [laid_out(t) for t in (q, k, v)] + ([] if bias is None else [bias.to(cuda).requires_grad_(True)])
+    problem = cabi.make_problem(leaves[0].detach(), leaves[1].detach(), leaves[2].detach(), None,
+                                None if bias is None else leaves[3].detach(), dim**-0.5)
+    assert cabi.library().oops_ta_uses_tensor_path(cabi.byref(problem), 1) == 0
+    out = triangle_attention(*leaves[:3], None if mask is None else mask.to(cuda), None if bias is None else leaves[3])
+    grads = torch.autograd.grad(out, leaves, up.to(cuda))
+
+    finite = [torch.nan_to_num(t.double(), nan=0.0, posinf=0.0) for t in (q, k, v)]
+    ref = [t.requires_grad_(True) for t in finite] + ([] if bias is None else [bias.double().requires_grad_(True)])
+    want = oracle.reference_dense(ref[0], ref[1], ref[2], mask, None if bias is None else ref[3], compute_dtype=torch.float64)
+    want_grads = torch.autograd.grad(want, ref, up.double())
+    for name, got, exact in zip(("out", "dq", "dk", "dv", "dbias"), (out, *grads), (want, *want_grads)):
+        got, exact = got.detach().double().cpu(), exact.detach()
+        bound = ROUNDING[dtype] * (1 if name == "out" else 8) * max(1.0, float(exact.abs().max()))
+        error = float((got - exact).abs().max())
+        assert error <= bound, (name, error, bound)
+    if mask is not None:
+        assert torch.count_nonzero(out.detach().cpu()[~mask.any(-1)]) == 0
+        for grad in grads[1:3]:
+            assert torch.count_nonzero(grad.cpu()[~mask]) == 0
