@@ -78,6 +78,10 @@ def gate_attention_output(attention, single, gate_weight: Tensor, output_weight:
         ValueError: ranks, shapes, devices or dense/ragged representations disagree.
         OOpsUnsupportedError: ragged operands, non-CUDA tensors, unsupported dtypes.
     """
+    if not torch.compiler.is_compiling() and forward_ad._current_level < 0:
+        out = native().gate_attention_output(attention, single, gate_weight, output_weight)
+        if out is not None:
+            return out
     if is_nested(attention) or is_nested(single):
         if is_nested(attention) != is_nested(single):
             raise ValueError(

@@ -21,10 +21,12 @@ from typing import Optional
 
 import torch
 from torch import Tensor
+from torch.autograd import forward_ad
 
 from ...runtime import require_no_forward_mode, require_same_device, unsupported
+from ...runtime.native import native
 from ...runtime.nested_tensor import is_nested
-from ..triangle.triangle_attention import triangle_attention
+from ..triangle.triangle_attention import _flags, triangle_attention
 
 _NAME = "pair_bias_attention"
 
@@ -32,6 +34,10 @@ _NAME = "pair_bias_attention"
 def pair_bias_attention(query, key, value, mask: Optional[Tensor] = None, pair_bias: Optional[Tensor] = None, *,
                         scale: Optional[float] = None):
     """Scaled dot-product attention with an optional additive pair bias; see the module docstring."""
+    if not torch.compiler.is_compiling() and forward_ad._current_level < 0:
+        out = native().pair_bias_attention(query, key, value, mask, pair_bias, scale, _flags())
+        if out is not None:
+            return out
     if any(is_nested(t) for t in (query, key, value, mask, pair_bias)):
         raise unsupported(_NAME, "serves dense operands only (NestedTensor variants are not built)")
     require_no_forward_mode(_NAME, query, key, value, pair_bias)

@@ -6,6 +6,7 @@
 // What it saves is host time: a Python autograd function with its ctypes structures cost 75 us per forward call and
 // 250 us per forward + reverse call, more than the kernels of calls below about 300 x 300 tokens take.
 // The kernels are reached through the C ABI only (include/oops_ta.h); PyTorch provides memory, streams and autograd.
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -218,12 +219,12 @@ Tensor result_like(const Tensor& t) {
   return out;
 }
 
-// `gate` and `plain` are undefined except for the gated form, whose result is the gated tensor.
+// `gate` and `plain` are undefined except for the gated form, whose result is the gated tensor; `into` lends the result's memory.
 std::tuple<Tensor, Tensor> run_forward(const Geometry& g, const Tensor& query, const Tensor& key, const Tensor& value,
                                        const Tensor& mask, const Tensor& bias, double scale, int64_t flags, bool want_lse,
-                                       const Tensor& gate = {}, const Tensor& plain = {}) {
+                                       const Tensor& gate = {}, const Tensor& plain = {}, const Tensor& into = {}) {
   const c10::cuda::CUDAGuard guard(query.device());
-  Tensor out = gate.defined() ? at::empty(query.sizes(), query.options()) : result_like(query);
+  Tensor out = into.defined() ? into : gate.defined() ? at::empty(query.sizes(), query.options()) : result_like(query);
   Tensor lse = want_lse ? floats_like(query, {g.lse_size(query)}) : Tensor();
   void* stream = current_stream(query);
   for_each_sample(g, query, [&](const Sample& s, size_t i) {
@@ -532,6 +533,154 @@ std::optional<Tensor> dense_gated_attention(const Tensor& query, const Tensor& k
                       scale.has_value() ? *scale : 1.0 / std::sqrt(double(query.size(-1))), flags);
 }
 
+// linear(sigmoid(linear(single, gate_weight)) * attention_flat, output_weight) as one node.
+struct GateOutputFunction : Function<GateOutputFunction> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& attention, const Tensor& single, const Tensor& gate_weight,
+                        const Tensor& output_weight) {
+    const auto type = attention.scalar_type();
+    const int64_t heads = attention.size(-3), tokens = attention.size(-2), dim = attention.size(-1);
+    const Tensor values = unit_inner(attention.reshape({-1, heads, tokens, dim}));
+    const Tensor rows = single.reshape({-1, single.size(-1)}), wg = gate_weight.to(type), wo = output_weight.to(type);
+    const Tensor gate = at::linear(rows, wg), gated = at::empty_like(gate);
+    auto as_pairs = [&](const Tensor& t) { return t.view({values.size(0), 1, tokens, heads, dim}); };
+    run_gate(head_major(values), as_pairs(gate), as_pairs(gated));
+    std::vector<int64_t> shape = single.sizes().vec();
+    shape.back() = wo.size(0);
+    if (ctx) {
+      ctx->save_for_backward({values, rows, wg, wo, gate, gated});
+      ctx->saved_data["attention"] = attention.sizes().vec();
+      ctx->saved_data["single"] = single.sizes().vec();
+      ctx->saved_data["types"] = std::vector<int64_t>{int64_t(gate_weight.scalar_type()), int64_t(output_weight.scalar_type())};
+    }
+    return at::_unsafe_view(at::linear(gated, wo), shape);
+  }
+  static variable_list backward(AutogradContext* ctx, const variable_list& grad_outputs) {
+    variable_list saved = ctx->get_saved_variables();
+    const Tensor values = unit_inner(saved[0]), rows = saved[1], wg = saved[2], wo = saved[3], gate = saved[4].contiguous(), gated = saved[5];
+    const std::vector<int64_t> types = ctx->saved_data["types"].toIntVector();
+    const int64_t heads = values.size(1), tokens = values.size(2), dim = values.size(3);
+    const Tensor dout = grad_outputs[0].resolve_neg().to(gate.scalar_type()).reshape({-1, wo.size(0)});
+    variable_list result(4);
+    if (ctx->needs_input_grad(3)) result[3] = at::mm(dout.t(), gated).to(at::ScalarType(types[1]));
+    const bool need_attention = ctx->needs_input_grad(0), need_gate = ctx->needs_input_grad(1) || ctx->needs_input_grad(2);
+    if (!need_attention && !need_gate) return result;
+    const Tensor dgated = at::mm(dout, wo), dgate = need_gate ? at::empty_like(gate) : Tensor();
+    const Tensor dvalues = need_attention ? at::empty(values.sizes(), values.options()) : Tensor();
+    auto as_pairs = [&](const Tensor& t) { return t.defined() ? t.view({values.size(0), 1, tokens, heads, dim}) : t; };
+    run_gate_backward(head_major(values), as_pairs(gate), as_pairs(dgated), head_major(dvalues), as_pairs(dgate));
+    if (need_attention) result[0] = dvalues.view(ctx->saved_data["attention"].toIntVector());
+    if (ctx->needs_input_grad(1)) result[1] = at::mm(dgate, wg).view(ctx->saved_data["single"].toIntVector());
+    if (ctx->needs_input_grad(2)) result[2] = at::mm(dgate.t(), rows).to(at::ScalarType(types[0]));
+    return result;
+  }
+};
+
+std::optional<Tensor> gate_output(const Tensor& attention, const Tensor& single, const Tensor& gate_weight, const Tensor& output_weight) {
+  if (!plain_context() || at::autocast::is_autocast_enabled(at::kCUDA)) return std::nullopt;
+  for (const Tensor* t : {&attention, &single, &gate_weight, &output_weight})
+    if (!plain_tensor(*t) || t->device() != attention.device() || !t->is_floating_point()) return std::nullopt;
+  const int64_t rank = attention.dim();
+  if (rank < 3 || rank > 5 || single.dim() + 1 != rank || gate_weight.dim() != 2 || output_weight.dim() != 2) return std::nullopt;
+  if (dtype_code(attention.scalar_type()) < 0 || single.scalar_type() != attention.scalar_type() || attention.numel() == 0) return std::nullopt;
+  const int64_t channels = attention.size(-3) * attention.size(-1);
+  if (single.sizes().slice(0, rank - 3) != attention.sizes().slice(0, rank - 3) || single.size(-2) != attention.size(-2)) return std::nullopt;
+  if (gate_weight.size(0) != channels || gate_weight.size(1) != single.size(-1) || output_weight.size(1) != channels) return std::nullopt;
+  if (at::GradMode::is_enabled() &&
+      (attention.requires_grad() || single.requires_grad() || gate_weight.requires_grad() || output_weight.requires_grad()))
+    return GateOutputFunction::apply(attention, single, gate_weight, output_weight);
+  return GateOutputFunction::forward(nullptr, attention, single, gate_weight, output_weight);
+}
+
+// ---------------------------------------------------------------------------------------------
+// token attention with a pair bias
+// ---------------------------------------------------------------------------------------------
+
+// (*prefix, S, H, N, D) operands as (B, S, N, H, D) views of the pair kernels, and results back; ranks 3 and 4 omit leading axes.
+Tensor tokens_as_pairs(const Tensor& t) {
+  const int64_t rank = t.dim();
+  return t.reshape({-1, rank > 3 ? t.size(-4) : 1, t.size(-3), t.size(-2), t.size(-1)}).permute({0, 1, 3, 2, 4});
+}
+Tensor pairs_as_tokens(const Tensor& pairs, at::IntArrayRef shape) {
+  return pairs.defined() ? pairs.permute({0, 1, 3, 2, 4}).reshape(shape) : pairs;
+}
+Tensor token_bias(const Tensor& bias) {
+  const int64_t rank = bias.dim();
+  return aligned_bias(bias.reshape({-1, rank > 3 ? bias.size(-4) : 1, bias.size(-3), bias.size(-2), bias.size(-1)}), bias.size(-1));
+}
+Tensor token_mask(const Tensor& mask, const Tensor& query) {
+  if (!mask.defined()) return mask;
+  const int64_t groups = query.dim() > 3 ? query.size(-4) : 1, tokens = query.size(-2);
+  const Tensor rows = mask.reshape({-1, mask.dim() > 1 ? mask.size(-2) : 1, tokens});
+  return rows.expand({rows.size(0), groups, tokens});
+}
+
+struct TokenFunction : Function<TokenFunction> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& query, const Tensor& key, const Tensor& value, const MaybeTensor& mask,
+                        const MaybeTensor& bias, double scale, int64_t flags) {
+    const Tensor laid_bias = bias.has_value() ? token_bias(*bias) : Tensor();
+    const Tensor laid_mask = token_mask(mask.value_or(Tensor()), query);
+    const Tensor q = unit_inner(tokens_as_pairs(query)), k = key.is_same(query) ? q : unit_inner(tokens_as_pairs(key)),
+                 v = value.is_same(query) ? q : value.is_same(key) ? k : unit_inner(tokens_as_pairs(value));
+    const Tensor result = at::empty(query.sizes(), query.options());
+    auto [out, lse] = run_forward(Geometry(), q, k, v, laid_mask, laid_bias, scale, flags, ctx != nullptr, {}, {}, tokens_as_pairs(result));
+    if (ctx) {
+      ctx->set_materialize_grads(false);
+      ctx->save_for_backward({q, k, v, laid_mask, laid_bias, result, lse});
+      ctx->saved_data["shape"] = query.sizes().vec();
+      ctx->saved_data["bias_shape"] = bias.has_value() ? bias->sizes().vec() : std::vector<int64_t>();
+      ctx->saved_data["scale"] = scale;
+      ctx->saved_data["flags"] = flags;
+    }
+    return result;
+  }
+  static variable_list backward(AutogradContext* ctx, const variable_list& grad_outputs) {
+    variable_list result(7);
+    if (!grad_outputs[0].defined()) return result;
+    const variable_list saved = ctx->get_saved_variables();
+    const Geometry g;
+    const Tensor q = canonical_pair(g, saved[0]), k = canonical_pair(g, saved[1]), v = canonical_pair(g, saved[2]), mask = saved[3],
+                 bias = saved[4], out = canonical_pair(g, tokens_as_pairs(saved[5]));
+    const Tensor grad_out = canonical_pair(g, tokens_as_pairs(grad_outputs[0].resolve_neg().to(q.scalar_type())));
+    Gradients grads = run_backward(g, grad_out, q, k, v, mask, bias, out, saved[6].contiguous(), ctx->saved_data["scale"].toDouble(),
+                                   ctx->saved_data["flags"].toInt(), ctx->needs_input_grad(0), ctx->needs_input_grad(1),
+                                   ctx->needs_input_grad(2), bias.defined() && ctx->needs_input_grad(mask.defined() ? 4 : 3));
+    const std::vector<int64_t> shape = ctx->saved_data["shape"].toIntVector();
+    result[0] = pairs_as_tokens(grads.dq, shape);
+    result[1] = pairs_as_tokens(grads.dk, shape);
+    result[2] = pairs_as_tokens(grads.dv, shape);
+    if (grads.dbias.defined()) result[4] = grads.dbias.reshape(ctx->saved_data["bias_shape"].toIntVector());
+    return result;
+  }
+};
+
+std::optional<Tensor> token_attention(const Tensor& query, const Tensor& key, const Tensor& value, const MaybeTensor& mask,
+                                      const MaybeTensor& bias, std::optional<double> scale, int64_t flags) {
+  if (!plain_context()) return std::nullopt;
+  for (const Tensor* t : {&query, &key, &value})
+    if (!plain_tensor(*t) || t->device() != query.device() || t->scalar_type() != query.scalar_type() || t->sizes() != query.sizes())
+      return std::nullopt;
+  const int64_t rank = query.dim();
+  if (rank < 3 || dtype_code(query.scalar_type()) < 0 || query.numel() == 0 || query.size(-1) > 256) return std::nullopt;
+  const int64_t groups = rank > 3 ? query.size(-4) : 1, heads = query.size(-3), tokens = query.size(-2), prefix = std::max<int64_t>(rank - 4, 0);
+  if (mask.has_value()) {  // (*prefix, S|1, K)
+    if (!plain_tensor(*mask) || mask->device() != query.device() || mask->scalar_type() != at::kBool || mask->dim() != rank - 2 ||
+        mask->size(-1) != tokens || mask->sizes().slice(0, prefix) != query.sizes().slice(0, prefix))
+      return std::nullopt;
+    if (mask->dim() > 1 && mask->size(-2) != 1 && mask->size(-2) != groups) return std::nullopt;
+  }
+  if (bias.has_value()) {  // (*prefix, S|1, H, Q, K)
+    if (!plain_tensor(*bias) || bias->device() != query.device() || bias->scalar_type() != query.scalar_type() || bias->dim() != rank ||
+        bias->sizes().slice(0, prefix) != query.sizes().slice(0, prefix) || bias->size(-3) != heads || bias->size(-2) != tokens ||
+        bias->size(-1) != tokens)
+      return std::nullopt;
+    if (rank > 3 && bias->size(-4) != 1 && bias->size(-4) != groups) return std::nullopt;
+  }
+  const double factor = scale.has_value() ? *scale : 1.0 / std::sqrt(double(query.size(-1)));
+  if (at::GradMode::is_enabled() && (query.requires_grad() || key.requires_grad() || value.requires_grad() || requires_grad(bias)))
+    return TokenFunction::apply(query, key, value, mask, bias, factor, flags);
+  return TokenFunction::forward(nullptr, query, key, value, mask, bias, factor, flags);
+}
+
 // ---------------------------------------------------------------------------------------------
 // layer norm
 // ---------------------------------------------------------------------------------------------
@@ -547,10 +696,11 @@ struct Normed {
   Tensor y, stats;  // stats: (2, rows) f32, mean and reciprocal standard deviation
 };
 
-Normed norm_forward(const Tensor& rows_in, const Tensor& weight, const Tensor& bias, double eps, bool keep_stats) {
+// The result has `shape` (that of the rows, or of the tensor they are a view of).
+Normed norm_forward(const Tensor& rows_in, const Tensor& weight, const Tensor& bias, double eps, bool keep_stats, at::IntArrayRef shape) {
   const c10::cuda::CUDAGuard guard(rows_in.device());
   const int64_t rows = rows_in.size(0), width = rows_in.size(1);
-  Normed n{at::empty({rows, width}, rows_in.options()), keep_stats ? floats_like(rows_in, {2, rows}) : Tensor()};
+  Normed n{at::empty(shape, rows_in.options()), keep_stats ? floats_like(rows_in, {2, rows}) : Tensor()};
   const auto affine = weight.defined() ? weight.scalar_type() : bias.defined() ? bias.scalar_type() : rows_in.scalar_type();
   float* stats = keep_stats ? n.stats.data_ptr<float>() : nullptr;
   const int status = oops_ta_layer_norm_forward(
@@ -587,12 +737,12 @@ struct LayerNormFunction : Function<LayerNormFunction> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const MaybeTensor& weight, const MaybeTensor& bias, double eps) {
     const Tensor rows = rows_of(x, x.size(-1));
     const Tensor w = weight.has_value() ? weight->contiguous() : Tensor(), b = bias.has_value() ? bias->contiguous() : Tensor();
-    Normed n = norm_forward(rows, w, b, eps, true);
+    Normed n = norm_forward(rows, w, b, eps, true, x.sizes());
     ctx->save_for_backward({rows, w, n.stats});
     ctx->saved_data["shape"] = x.sizes().vec();
     ctx->saved_data["affine"] = int64_t(w.defined() ? w.scalar_type() : b.defined() ? b.scalar_type() : x.scalar_type());
     ctx->saved_data["has_bias"] = b.defined();
-    return n.y.view(x.sizes());
+    return n.y;
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grad_outputs) {
     const variable_list saved = ctx->get_saved_variables();
@@ -628,7 +778,7 @@ std::optional<Tensor> layer_norm(const Tensor& x, int64_t width, const MaybeTens
   if (at::GradMode::is_enabled() && (x.requires_grad() || requires_grad(weight) || requires_grad(bias)))
     return LayerNormFunction::apply(x, weight, bias, eps);
   const Tensor w = weight.has_value() ? weight->contiguous() : Tensor(), b = bias.has_value() ? bias->contiguous() : Tensor();
-  return norm_forward(rows_of(x, width), w, b, eps, false).y.view(x.sizes());
+  return norm_forward(rows_of(x, width), w, b, eps, false, x.sizes()).y;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -677,7 +827,7 @@ struct UpdateFunction : Function<UpdateFunction> {
     }
     const Tensor out_matrix = weights[kOutput].to(type);
     const Tensor rows = rows_of(pair, channels), in_w = parameters[0].contiguous(), out_w = parameters[2].contiguous();
-    Normed x = norm_forward(rows, in_w, parameters[1].contiguous(), in_eps, true);
+    Normed x = norm_forward(rows, in_w, parameters[1].contiguous(), in_eps, true, rows.sizes());
     const Tensor proj = stacked_has_bias ? at::linear(x.y, stacked, stacked_bias) : at::linear(x.y, stacked);
     const int64_t ld = proj.size(1);
     const Tensor weight = mask.has_value() ? mask->to(type).expand(pair.sizes().slice(0, pair.dim() - 1)).contiguous() : Tensor();
@@ -809,10 +959,11 @@ PyObject* wrap(std::optional<Tensor>&& t) {
   return THPVariable_Wrap(std::move(*t));
 }
 
-// triangle_attention(query, key, value, mask, bias, scale, flags) -> Tensor or None
-PyObject* py_triangle_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
+// triangle_attention / pair_bias_attention(query, key, value, mask, bias, scale, flags) -> Tensor or None
+template <auto Attention>
+PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  TORCH_CHECK(n == 7, "triangle_attention takes 7 arguments");
+  TORCH_CHECK(n == 7, "attention takes 7 arguments");
   if (!THPVariable_Check(a[0]) || !THPVariable_Check(a[1]) || !THPVariable_Check(a[2]) || !tensor_or_none(a[3]) || !tensor_or_none(a[4]))
     Py_RETURN_NONE;
   const Tensor &q = THPVariable_Unpack(a[0]), &k = THPVariable_Unpack(a[1]), &v = THPVariable_Unpack(a[2]);
@@ -822,7 +973,7 @@ PyObject* py_triangle_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   std::optional<Tensor> out;
   {
     py::gil_scoped_release no_gil;
-    out = dense_attention(q, k, v, mask, bias, scale, flags);
+    out = Attention(q, k, v, mask, bias, scale, flags);
   }
   return wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -848,6 +999,23 @@ PyObject* py_gated_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// gate_attention_output(attention, single, gate_weight, output_weight) -> Tensor or None
+PyObject* py_gate_output(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 4, "gate_attention_output takes 4 arguments");
+  for (int i = 0; i < 4; ++i)
+    if (!THPVariable_Check(a[i])) Py_RETURN_NONE;
+  std::optional<Tensor> out;
+  {
+    const Tensor &attention = THPVariable_Unpack(a[0]), &single = THPVariable_Unpack(a[1]), &wg = THPVariable_Unpack(a[2]),
+                 &wo = THPVariable_Unpack(a[3]);
+    py::gil_scoped_release no_gil;
+    out = gate_output(attention, single, wg, wo);
+  }
+  return wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
 // layer_norm(x, width, weight, bias, eps) -> Tensor or None
 PyObject* py_layer_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -867,7 +1035,9 @@ PyObject* py_layer_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 PyMethodDef g_fast_methods[] = {
-    {"triangle_attention", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_triangle_attention)), METH_FASTCALL, nullptr},
+    {"triangle_attention", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_attention<dense_attention>)), METH_FASTCALL, nullptr},
+    {"pair_bias_attention", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_attention<token_attention>)), METH_FASTCALL, nullptr},
+    {"gate_attention_output", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_gate_output)), METH_FASTCALL, nullptr},
     {"triangle_attention_gated", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_gated_attention)), METH_FASTCALL, nullptr},
     {"layer_norm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_layer_norm)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};

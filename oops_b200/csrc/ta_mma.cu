@@ -270,12 +270,14 @@ __device__ __forceinline__ const BiasType<T, B32>* bias_plane(const MmaProblem& 
 template <bool B32>
 constexpr int bias_bytes() { return kT * bias_pitch<B32>() * (B32 ? 4 : 2); }
 
+// Q passes through the second stage's memory into registers: four CTAs then fit an SM, 592 at once, where three left the
+// 512 CTAs of a 4-sample, 16-head, 512-token call a second wave of 68.
 template <typename T, int DP, bool B32>
-__global__ void __launch_bounds__(kThreads) mma_forward_kernel(const MmaProblem p) {
+__global__ void __launch_bounds__(kThreads, 4) mma_forward_kernel(const MmaProblem p) {
   extern __shared__ __align__(16) uint8_t mma_smem[];
   constexpr int kStage = 2 * tile_elems<DP>() * 2 + bias_bytes<B32>();  // K | V | bias
-  T* Q = reinterpret_cast<T*>(mma_smem);
-  uint8_t* stages = mma_smem + tile_elems<DP>() * 2;
+  uint8_t* stages = mma_smem;
+  T* Q = reinterpret_cast<T*>(stages + kStage);
   int idx = blockIdx.x;
   const int tiles = (p.cols + kT - 1) / kT, qt = idx % tiles;
   idx /= tiles;
@@ -294,6 +296,7 @@ __global__ void __launch_bounds__(kThreads) mma_forward_kernel(const MmaProblem 
       load_bias<BiasType<T, B32>, bias_pitch<B32>()>(reinterpret_cast<BiasType<T, B32>*>(at + 2 * tile_elems<DP>() * 2), plane, p, qt * kT, kt * kT);
   };
   load_tile<T, DP>(Q, p.q, p, b, r, h, qt * kT, nullptr);
+  copies_commit();
   request(0);
   copies_commit();
   uint32_t q[DP / 16][4];
@@ -301,13 +304,16 @@ __global__ void __launch_bounds__(kThreads) mma_forward_kernel(const MmaProblem 
 #pragma unroll
   for (int i = 0; i < DP / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
   const float c = p.scale * kLog2e;
+  copies_wait<1>();
+  __syncthreads();
+  load_rows<T, DP>(q, Q, warp * 16);
+  __syncthreads();
 
   for (int kt = 0; kt < tiles; ++kt) {
     if (kt + 1 < tiles) request(kt + 1);
     copies_commit();
     copies_wait<1>();
     __syncthreads();
-    if (kt == 0) load_rows<T, DP>(q, Q, warp * 16);
     const uint64_t bits = keep_bits(p, keep, kt * kT);
     const uint8_t* at = stages + (kt & 1) * kStage;
     if (bits) {  // the same for every warp
@@ -816,7 +822,7 @@ int mma_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, c
     using T = decltype(type);
     constexpr int DP = decltype(width)::value;
     constexpr bool B32 = decltype(b32)::value;
-    return launch(mma_forward_kernel<T, DP, B32>, m, row_tiles(p), 5 * tile_elems<DP>() * 2 + 2 * bias_bytes<B32>(), stream, "mma forward");
+    return launch(mma_forward_kernel<T, DP, B32>, m, row_tiles(p), 4 * tile_elems<DP>() * 2 + 2 * bias_bytes<B32>(), stream, "mma forward");
   });
 }
 
