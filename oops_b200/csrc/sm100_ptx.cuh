@@ -39,19 +39,18 @@ __device__ __forceinline__ void mbar_arrive_warp(uint32_t bar) {
   __syncwarp();
   if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
 }
-constexpr uint32_t kSuspendHintNs = 20000;  // 20 us per probe; the bounded wait below re-probes until its own limit
+// The hardware parks the warp until the phase completes or a limit of its own runs out.  With a suspend-time hint (20 us)
+// the warp was woken by every barrier event of the CTA instead, some 18 times per step of the forward kernel: 2 % slower.
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t done;
-  // The suspend-time hint lets the hardware park the warp until the phase completes (or the hint expires)
-  // instead of returning at once, so a waiting warp does not burn issue slots of the warps that compute.
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t"
       "}\n"
       : "=r"(done)
-      : "r"(bar), "r"(parity), "r"(kSuspendHintNs)
+      : "r"(bar), "r"(parity)
       : "memory");
   return done != 0;
 }
@@ -140,6 +139,12 @@ __device__ __forceinline__ float4 ldcg_f4(const float4* p) {
 __device__ __forceinline__ uint4 lds_v4_here(const void* p) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(smem_u32(p)));
+  return v;
+}
+
+__device__ __forceinline__ uint4 lds_v4_at(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
   return v;
 }
 

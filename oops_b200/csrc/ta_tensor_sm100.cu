@@ -1,12 +1,21 @@
 // tcgen05 / TMEM / TMA triangle-attention kernels for sm_100a (f16 and bf16, head_dim 32).
 //
 // Forward (replaces the reference's Triton `_attend`, oops/attention/triangle/triton/kernel.py:150-262):
-// one CTA owns one (batch, row, head) and a pair of 128-query tiles.  A producer warp streams
-// 128-key K/V tiles and 128x128 bias tiles into shared memory with TMA; one thread issues
-// tcgen05.mma for S = Q K^T (accumulator in tensor memory) and O += P V (P read back from tensor
-// memory, V from shared memory); two softmax warpgroups, one per query tile, read S from tensor
-// memory, add the bias, apply the key mask, run the online softmax in base 2 and write P (packed
-// 16-bit) over S.  While one warpgroup is in its softmax the tensor core works on the other tile.
+// a CTA works on two 128-query tiles.  With a row-shared bias (or none) the tiles are the same queries of two neighbouring
+// pair rows, which read one bias tile; with a per-row bias they are neighbouring query tiles of one row, which read one
+// K/V stream.  A producer warp streams 64-key K/V tiles and 128 x 64 bias tiles into shared memory with TMA; one thread
+// issues tcgen05.mma for S = Q K^T (accumulator in tensor memory) and O += P V (P read back from tensor memory,
+// V from shared memory); one softmax warpgroup per tile (a thread owns a query) turns S into P.
+//
+// The softmax has no row maximum in its steady state.  The maximum of a row's first step (with a kept key) is its
+// reference; later steps take 2^(x - reference) as they come, 16 columns at a time, and look at the step's sum only: a
+// sum of 2^10 or more (or a NaN) sends the warp back over the step, which still stands in tensor memory, to raise the
+// reference and rescale the accumulators.  Probabilities therefore stay below 2^10, inside the f32, bf16 and f16 ranges.
+// Against a maximum per step this saves the comparisons, and above all the wait: no exponential depended on the last
+// score of a step any more, scores need not be held in registers, and an exponential costs 5 instead of 9.5 issue slots.
+// What bounds it: the special-function unit, one ex2 per score at 16 per clock and SM.
+#include <type_traits>
+
 #include "ta_tensor_common.cuh"
 
 namespace oops_ta {
@@ -20,43 +29,44 @@ constexpr int kKeys = 64;                        // keys per step
 constexpr int kQBytes = kTile * kHeadDim * 2;    // 8 KiB: one 128-query Q tile
 constexpr int kKvBytes = kKeys * kHeadDim * 2;   // 4 KiB: one K or V step
 constexpr int kBiasBytes = kTile * kKeys * 2;    // 16 KiB: one 128 x 64 bias tile (one swizzle-128 box)
-constexpr int kFwdThreads = 320;                 // 2 softmax warpgroups + producer warp + MMA warp
+constexpr int kFwdThreads = 352;                 // 2 softmax warpgroups + producer warp + 2 MMA warps
 constexpr int kFwdTmemCols = 256;                // S 2x64 | P 2x32 | O 2x32; two CTAs share an SM
 constexpr int kMaxKeepWords = 512;               // keep-bit table: one bit per key column, cols <= 16384
-#ifndef TA_FWD_POLY_EVERY
-#define TA_FWD_POLY_EVERY 0
-#endif
-constexpr int kFwdPolyEvery = TA_FWD_POLY_EVERY;  // every n-th pair of a thread's logits takes the polynomial exp2 (0: none)
 
+// ROWS: the two tiles belong to two pair rows (own K/V rings, one bias ring); otherwise to one row (one K/V ring, own
+// bias rings).
+template <bool ROWS>
 struct FwdSmem {
-  static constexpr int q = 0;                          // [2]
-  static constexpr int k = q + 2 * kQBytes;            // [kStages]
-  static constexpr int v = k + kStages * kKvBytes;     // [kStages]
-  static constexpr int bias = v + kStages * kKvBytes;  // [2 tiles][2 buffers]
-  static constexpr int bars = bias + 4 * kBiasBytes;
+  static constexpr int kv_rings = ROWS ? 2 : 1, bias_rings = ROWS ? 1 : 2;
+  static constexpr int q = 0;                                     // [2]
+  static constexpr int k = q + 2 * kQBytes;                       // [kv_rings][kStages]
+  static constexpr int v = k + kv_rings * kStages * kKvBytes;     // [kv_rings][kStages]
+  static constexpr int bias = v + kv_rings * kStages * kKvBytes;  // [bias_rings][2 buffers]
+  static constexpr int bars = bias + bias_rings * 2 * kBiasBytes;
   // barrier indices (8 bytes each)
-  static constexpr int q_full = 0;                     // [2]
-  static constexpr int k_full = q_full + 2;            // [kStages]
-  static constexpr int k_empty = k_full + kStages;     // [kStages]
-  static constexpr int v_full = k_empty + kStages;     // [kStages]
-  static constexpr int v_empty = v_full + kStages;     // [kStages]
-  static constexpr int v_ready = v_empty + kStages;    // [kStages]
-  static constexpr int bias_full = v_ready + kStages;  // [2 tiles][2 buffers]
-  static constexpr int bias_empty = bias_full + 4;     // [2][2]
-  static constexpr int s_full = bias_empty + 4;        // [2]
-  static constexpr int p_full = s_full + 2;            // [2]
-  static constexpr int o_final = p_full + 2;           // [2]
-  static constexpr int s_free = o_final + 2;           // [2] S has been read into registers
-  static constexpr int pv_done = s_free + 2;           // [2] the latest P V product has completed
+  static constexpr int q_full = 0;                                // [2]
+  static constexpr int k_full = q_full + 2;                       // [kv_rings][kStages]
+  static constexpr int k_empty = k_full + kv_rings * kStages;
+  static constexpr int v_full = k_empty + kv_rings * kStages;
+  static constexpr int v_empty = v_full + kv_rings * kStages;
+  static constexpr int v_ready = v_empty + kv_rings * kStages;    // rows of dropped keys have been cleared
+  static constexpr int bias_full = v_ready + kv_rings * kStages;  // [bias_rings][2 buffers]
+  static constexpr int bias_empty = bias_full + bias_rings * 2;
+  static constexpr int s_full = bias_empty + bias_rings * 2;      // [2] S of a step is in tensor memory
+  static constexpr int p_full = s_full + 2;                       // [2] P is there, and S may be overwritten
+  static constexpr int pv_done = p_full + 2;                      // [2] the latest P V product has completed
   static constexpr int num_bars = pv_done + 2;
   static constexpr int tmem_slot = bars + num_bars * 8;
   static constexpr int abort_flag = tmem_slot + 4;
-  static constexpr int drop_flags = abort_flag + 4;    // [8] per-warp: the mask drops a key of this row
-  static constexpr int keep = drop_flags + 32;         // [kMaxKeepWords] u32
-  static constexpr int total = keep + kMaxKeepWords * 4;
+  static constexpr int drop_flags = abort_flag + 4;               // [8] per-warp: the mask drops a key of this row
+  static constexpr int step_count = drop_flags + 32;
+  static constexpr int steps = step_count + 4;                    // [256] u16: steps with a kept key (with a mask)
+  static constexpr int keep = (steps + 512 + 15) / 16 * 16;       // [kv_rings][kMaxKeepWords] u32
+  static constexpr int total = keep + kv_rings * kMaxKeepWords * 4;
+  static constexpr int bytes = total + 1024;                      // slack to align the base to 1 KiB
 };
-constexpr int kFwdSmemBytes = FwdSmem::total + 1024;  // slack to align the base to 1 KiB
-static_assert(kFwdSmemBytes <= 113 * 1024, "two forward CTAs must fit in one SM's shared memory");
+static_assert(FwdSmem<true>::bytes <= 113 * 1024 && FwdSmem<false>::bytes <= 113 * 1024,
+              "two forward CTAs must fit in one SM's shared memory");
 
 struct FwdParams {
   CUtensorMap map_q, map_k, map_v, map_bias;
@@ -66,7 +76,7 @@ struct FwdParams {
   const uint8_t* mask;
   int64_t m_sb, m_sr, m_sc;
   int batch, rows, cols, heads, bias_groups;
-  int q_pairs, k_steps;
+  int q_items, k_steps;  // query tiles (ROWS) or pairs of query tiles of a row; key steps
   int out_vec16;
   float scale;
   // gated epilogue (GATED instantiations): gated = sigmoid(gate) * out goes to `out`, the ungated values to `plain`
@@ -77,362 +87,391 @@ struct FwdParams {
   int gate_vec16, plain_vec16;
 };
 
-// The running maximum is only raised when a step exceeds it by more than this (natural-log units):
-// probabilities then stay below e^kRescaleSlack, far inside the f32 / 16-bit ranges, and the
-// accumulator rescale (a tensor-memory round trip) is skipped for almost every step.
-constexpr float kRescaleSlack = 5.545177444f;  // 8 * ln 2
+constexpr float kStepSumLimit = 1024.f;  // a step's sum of probabilities that sends its warp back for a new reference
 
-template <typename T, bool HAS_BIAS, bool GATED>
+template <typename T, bool HAS_BIAS, bool GATED, bool ROWS>
 __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_constant__ FwdParams P) {
+  using Smem = FwdSmem<ROWS>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + FwdSmem::abort_flag);
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + FwdSmem::tmem_slot);
-  uint32_t* keep_words = reinterpret_cast<uint32_t*>(smem_gen + FwdSmem::keep);
-  auto bar = [&](int index) -> uint32_t { return smem_base + FwdSmem::bars + index * 8; };
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + Smem::abort_flag);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + Smem::tmem_slot);
+  uint32_t* keep_words = reinterpret_cast<uint32_t*>(smem_gen + Smem::keep);
+  volatile int* step_count = reinterpret_cast<volatile int*>(smem_gen + Smem::step_count);
+  uint16_t* step_list = reinterpret_cast<uint16_t*>(smem_gen + Smem::steps);
+  auto bar = [&](int index) -> uint32_t { return smem_base + Smem::bars + index * 8; };
 
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
   if (device_failed()) return;
 
-  // work decomposition: query pair fastest, then head, row, batch
+  // work decomposition: query item fastest, then head, row (or pair of rows), batch
   int idx = blockIdx.x;
-  const int qp = idx % P.q_pairs;
-  idx /= P.q_pairs;
+  const int qi = idx % P.q_items;
+  idx /= P.q_items;
   const int h = idx % P.heads;
   idx /= P.heads;
-  const int r = idx % P.rows;
-  const int b = idx / P.rows;
-  const int q0 = qp * 2 * kTile;
-  const int n_tiles = (q0 + kTile < P.cols) ? 2 : 1;
-  const int KS = P.k_steps;
-  const int g = P.bias_groups == 1 ? 0 : r;
+  const int row_items = ROWS ? (P.rows + 1) / 2 : P.rows;
+  const int r0 = (idx % row_items) * (ROWS ? 2 : 1);
+  const int b = idx / row_items;
+  const int q0 = qi * (ROWS ? kTile : 2 * kTile);
+  const int n_tiles = (ROWS ? r0 + 1 < P.rows : q0 + kTile < P.cols) ? 2 : 1;
+  const int n_rings = ROWS ? n_tiles : 1;
+  const int g = P.bias_groups == 1 ? 0 : r0;
   const bool has_mask = P.mask != nullptr;
   // Steps need keep-bits when there is a mask or when the last key step is ragged.
   const bool has_bits = has_mask || (P.cols % kKeys) != 0;
+  auto row_of = [&](int w) { return ROWS ? r0 + w : r0; };
+  auto first_query = [&](int w) { return ROWS ? q0 : q0 + w * kTile; };
 
   if (tid == 0) {
     *abort_flag = 0;
-    for (int i = 0; i < 2; ++i) mbar_init(bar(FwdSmem::q_full + i), 1);
-    for (int i = 0; i < kStages; ++i) {
-      mbar_init(bar(FwdSmem::k_full + i), 1);
-      mbar_init(bar(FwdSmem::k_empty + i), 1);
-      mbar_init(bar(FwdSmem::v_full + i), 1);
-      mbar_init(bar(FwdSmem::v_empty + i), 1);
-      mbar_init(bar(FwdSmem::v_ready + i), kTile / 32);
+    for (int i = 0; i < 2; ++i) mbar_init(bar(Smem::q_full + i), 1);
+    for (int i = 0; i < Smem::kv_rings * kStages; ++i) {
+      mbar_init(bar(Smem::k_full + i), 1);
+      mbar_init(bar(Smem::k_empty + i), ROWS ? 1 : n_tiles);
+      mbar_init(bar(Smem::v_full + i), 1);
+      mbar_init(bar(Smem::v_empty + i), ROWS ? 1 : n_tiles);
+      mbar_init(bar(Smem::v_ready + i), kTile / 32);
     }
-    for (int i = 0; i < 4; ++i) {
-      mbar_init(bar(FwdSmem::bias_full + i), 1);
-      mbar_init(bar(FwdSmem::bias_empty + i), kTile / 32);
+    for (int i = 0; i < Smem::bias_rings * 2; ++i) {
+      mbar_init(bar(Smem::bias_full + i), 1);
+      mbar_init(bar(Smem::bias_empty + i), ROWS ? n_tiles * (kTile / 32) : kTile / 32);
     }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(FwdSmem::s_full + i), 1);
-      mbar_init(bar(FwdSmem::p_full + i), kTile / 32);
-      mbar_init(bar(FwdSmem::o_final + i), 1);
-      mbar_init(bar(FwdSmem::s_free + i), kTile / 32);
-      mbar_init(bar(FwdSmem::pv_done + i), 1);
+      mbar_init(bar(Smem::s_full + i), 1);
+      mbar_init(bar(Smem::p_full + i), kTile / 32);
+      mbar_init(bar(Smem::pv_done + i), 1);
     }
     fence_barrier_init();
   }
   if (warp == 9) {
-    tmem_alloc(smem_base + FwdSmem::tmem_slot, kFwdTmemCols);
+    tmem_alloc(smem_base + Smem::tmem_slot, kFwdTmemCols);
     tmem_relinquish();
     tc_fence_before_sync();
   }
-  uint32_t* drop_flags = reinterpret_cast<uint32_t*>(smem_gen + FwdSmem::drop_flags);
+  uint32_t* drop_flags = reinterpret_cast<uint32_t*>(smem_gen + Smem::drop_flags);
   if (has_bits && warp < 8) {
-    // one bit per key of this pair row: kept by the mask and inside the row
-    const uint8_t* mask_row = has_mask ? P.mask + b * P.m_sb + int64_t(r) * P.m_sr : nullptr;
+    // one bit per key of the pair row: kept by the mask and inside the row (warps 0-3: first row, 4-7: second row; one
+    // row: all warps)
+    const int ring = ROWS ? warp >> 2 : 0;
     bool dropped_any = false;
-    for (int word = warp; word < KS * 2; word += 8) {
-      const int key = word * 32 + lane;
-      bool keep = key < P.cols;
-      if (keep && has_mask) {
-        keep = mask_row[int64_t(key) * P.m_sc] != 0;
-        dropped_any |= !keep;
+    if (ring < n_rings) {
+      const uint8_t* mask_row = has_mask ? P.mask + b * P.m_sb + int64_t(row_of(ring)) * P.m_sr : nullptr;
+      for (int word = ROWS ? warp & 3 : warp; word < P.k_steps * 2; word += ROWS ? 4 : 8) {
+        const int key = word * 32 + lane;
+        bool keep = key < P.cols;
+        if (keep && has_mask) {
+          keep = mask_row[int64_t(key) * P.m_sc] != 0;
+          dropped_any |= !keep;
+        }
+        const uint32_t bits = __ballot_sync(0xffffffffu, keep);
+        if (lane == 0) keep_words[ring * kMaxKeepWords + word] = bits;
       }
-      const uint32_t bits = __ballot_sync(0xffffffffu, keep);
-      if (lane == 0) keep_words[word] = bits;
     }
     dropped_any = __any_sync(0xffffffffu, dropped_any);
     if (lane == 0) drop_flags[warp] = dropped_any ? 1u : 0u;
   }
   __syncthreads();
+  if (has_mask) {
+    // The steps in which some row of the CTA keeps a key, in order: padding is neither loaded nor computed.
+    if (warp == 0) {
+      int count = 0;
+      for (int first = 0; first < P.k_steps; first += 32) {
+        const int j = first + lane;
+        uint32_t any = 0;
+        if (j < P.k_steps)
+          for (int ring = 0; ring < n_rings; ++ring)
+            any |= keep_words[ring * kMaxKeepWords + 2 * j] | keep_words[ring * kMaxKeepWords + 2 * j + 1];
+        const uint32_t live = __ballot_sync(0xffffffffu, any != 0);
+        if (any != 0) step_list[count + __popc(live & ((1u << lane) - 1))] = uint16_t(j);
+        count += __popc(live);
+      }
+      if (lane == 0) *step_count = count;
+    }
+    __syncthreads();
+  }
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  // Value rows only need the sign-off handshake when the mask really drops a key of this row.
-  bool signoff = false;
-  if (has_mask) {
+  const int KS = has_mask ? *step_count : P.k_steps;
+  auto step_at = [&](int i) { return has_mask ? int(step_list[i]) : i; };
+  // Value rows only need the sign-off handshake when the mask really drops a key of the row.
+  auto needs_signoff = [&](int w) {
+    bool drops = false;
+    if (has_mask) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) signoff |= drop_flags[i] != 0;
-  }
+      for (int i = 0; i < 8; ++i) drops |= (!ROWS || (i >> 2) == w) && drop_flags[i] != 0;
+    }
+    return drops;
+  };
   // tensor-memory columns
   constexpr int kSCol = 0, kPCol = 2 * kKeys, kOCol = 2 * kKeys + 2 * (kKeys / 2);
 
   if (warp == 8) {
     // ------------------------------------------------------------------ producer (one thread)
-    if (lane == 0) {
+    if (lane == 0 && KS > 0) {
       bool ok = true;
       for (int w = 0; w < n_tiles; ++w) {
-        mbar_expect_tx(bar(FwdSmem::q_full + w), kQBytes);
-        tma_load_5d(smem_base + FwdSmem::q + w * kQBytes, &P.map_q, bar(FwdSmem::q_full + w), 0, h, q0 + w * kTile, r, b);
+        mbar_expect_tx(bar(Smem::q_full + w), kQBytes);
+        tma_load_5d(smem_base + Smem::q + w * kQBytes, &P.map_q, bar(Smem::q_full + w), 0, h, first_query(w), row_of(w), b);
       }
-      for (int j = 0; j < KS && ok; ++j) {
-        const int st = j % kStages, round = j / kStages;
-        if (j >= kStages) ok = mbar_wait(bar(FwdSmem::k_empty + st), (round - 1) & 1, abort_flag);
-        if (!ok) break;
-        mbar_expect_tx(bar(FwdSmem::k_full + st), kKvBytes);
-        tma_load_5d(smem_base + FwdSmem::k + st * kKvBytes, &P.map_k, bar(FwdSmem::k_full + st), 0, h, j * kKeys, r, b);
+      for (int i = 0; i < KS && ok; ++i) {
+        const int st = i % kStages, round = i / kStages, key = step_at(i) * kKeys;
+        for (int ring = 0; ring < n_rings && ok; ++ring) {
+          const int slot = ring * kStages + st;
+          if (i >= kStages) ok = mbar_wait(bar(Smem::k_empty + slot), (round - 1) & 1, abort_flag);
+          if (!ok) break;
+          mbar_expect_tx(bar(Smem::k_full + slot), kKvBytes);
+          tma_load_5d(smem_base + Smem::k + slot * kKvBytes, &P.map_k, bar(Smem::k_full + slot), 0, h, key, row_of(ring), b);
+        }
         if (HAS_BIAS) {
-          const int buf = j & 1;
-          for (int w = 0; w < n_tiles && ok; ++w) {
-            const int slot = w * 2 + buf;
-            if (j >= 2) ok = mbar_wait(bar(FwdSmem::bias_empty + slot), ((j >> 1) - 1) & 1, abort_flag);
+          for (int ring = 0; ring < (ROWS ? 1 : n_tiles) && ok; ++ring) {
+            const int slot = ring * 2 + (i & 1);
+            if (i >= 2) ok = mbar_wait(bar(Smem::bias_empty + slot), ((i >> 1) - 1) & 1, abort_flag);
             if (!ok) break;
-            mbar_expect_tx(bar(FwdSmem::bias_full + slot), kBiasBytes);
-            tma_load_5d(smem_base + FwdSmem::bias + slot * kBiasBytes, &P.map_bias, bar(FwdSmem::bias_full + slot),
-                        j * kKeys, q0 + w * kTile, h, g, b);
+            mbar_expect_tx(bar(Smem::bias_full + slot), kBiasBytes);
+            tma_load_5d(smem_base + Smem::bias + slot * kBiasBytes, &P.map_bias, bar(Smem::bias_full + slot), key, first_query(ring),
+                        h, g, b);
           }
         }
-        if (j >= kStages) ok = mbar_wait(bar(FwdSmem::v_empty + st), (round - 1) & 1, abort_flag);
-        if (!ok) break;
-        mbar_expect_tx(bar(FwdSmem::v_full + st), kKvBytes);
-        tma_load_5d(smem_base + FwdSmem::v + st * kKvBytes, &P.map_v, bar(FwdSmem::v_full + st), 0, h, j * kKeys, r, b);
+        for (int ring = 0; ring < n_rings && ok; ++ring) {
+          const int slot = ring * kStages + st;
+          if (i >= kStages) ok = mbar_wait(bar(Smem::v_empty + slot), (round - 1) & 1, abort_flag);
+          if (!ok) break;
+          mbar_expect_tx(bar(Smem::v_full + slot), kKvBytes);
+          tma_load_5d(smem_base + Smem::v + slot * kKvBytes, &P.map_v, bar(Smem::v_full + slot), 0, h, key, row_of(ring), b);
+        }
       }
     }
-  } else if (warp == 9) {
-    // ------------------------------------------------------------------ MMA issuer (one thread)
-    if (lane == 0) {
+  } else if (warp >= 9 && warp - 9 < n_tiles) {
+    // ------------------------------------------------------------------ MMA issuers (one thread per tile)
+    const int w = warp - 9, ring = (ROWS ? w : 0) * kStages;
+    if (lane == 0 && KS > 0) {
       constexpr uint32_t fmt = Half2<T>::kFormat;
       constexpr uint32_t idesc_qk = instr_desc(fmt, 0, 0, kTile, kKeys);
       constexpr uint32_t idesc_pv = instr_desc(fmt, 0, 1, kTile, kHeadDim);
-      bool ok = true;
-      for (int w = 0; w < n_tiles && ok; ++w) ok = mbar_wait(bar(FwdSmem::q_full + w), 0, abort_flag);
+      const bool signoff = needs_signoff(w);
+      const uint32_t s_t = tmem_base + kSCol + w * kKeys, p_t = tmem_base + kPCol + w * (kKeys / 2), o_t = tmem_base + kOCol + w * kHeadDim;
+      const uint64_t qdesc = smem_desc(smem_base + Smem::q + w * kQBytes, 16, 512, kSwizzle64B);
+      const uint64_t kdesc0 = smem_desc(smem_base + Smem::k + ring * kKvBytes, 16, 512, kSwizzle64B);
+      const uint64_t vdesc0 = smem_desc(smem_base + Smem::v + ring * kKvBytes, 16, 512, kSwizzle64B);
       // S[128 x 64] = Q[128 x 32] K[64 x 32]^T; both K-major, 64-byte swizzle: 8-row groups 512 bytes apart,
       // each 16-channel step advances 32 bytes inside the swizzle span.
-      auto issue_qk = [&](int j, int w) {
-        const int st = j % kStages;
-        const uint64_t qdesc = smem_desc(smem_base + FwdSmem::q + w * kQBytes, 16, 512, kSwizzle64B);
-        const uint64_t kdesc = smem_desc(smem_base + FwdSmem::k + st * kKvBytes, 16, 512, kSwizzle64B);
+      auto issue_qk = [&](int st) {
+        const uint64_t kdesc = kdesc0 + uint64_t((st * kKvBytes) >> 4);
 #pragma unroll
         for (int kk = 0; kk < kHeadDim / 16; ++kk)
-          mma_ss(tmem_base + kSCol + w * kKeys, qdesc + uint64_t(kk * 2), kdesc + uint64_t(kk * 2), idesc_qk, kk > 0 ? 1u : 0u);
-        mma_commit(bar(FwdSmem::s_full + w));
-        if (w == n_tiles - 1) mma_commit(bar(FwdSmem::k_empty + st));
+          mma_ss(s_t, qdesc + uint64_t(kk * 2), kdesc + uint64_t(kk * 2), idesc_qk, kk > 0 ? 1u : 0u);
+        mma_commit(bar(Smem::s_full + w));
+        mma_commit(bar(Smem::k_empty + ring + st));
       };
-      if (ok) ok = mbar_wait(bar(FwdSmem::k_full), 0, abort_flag);
+      bool ok = mbar_wait(bar(Smem::q_full + w), 0, abort_flag);
+      if (ok) ok = mbar_wait(bar(Smem::k_full + ring), 0, abort_flag);
       if (ok) {
         tc_fence_after_sync();
-        for (int w = 0; w < n_tiles; ++w) issue_qk(0, w);
+        issue_qk(0);
       }
-      for (int j = 0; j < KS && ok; ++j) {
-        if (j + 1 < KS) {
-          // next score tiles: issued as soon as a warpgroup has pulled S(j) into registers, so that S(j+1) is
-          // ready when its softmax of step j ends (P has its own tensor-memory columns)
-          ok = mbar_wait(bar(FwdSmem::k_full + (j + 1) % kStages), ((j + 1) / kStages) & 1, abort_flag);
-          for (int w = 0; w < n_tiles && ok; ++w) {
-            ok = mbar_wait(bar(FwdSmem::s_free + w), j & 1, abort_flag);
-            if (!ok) break;
-            tc_fence_after_sync();
-            issue_qk(j + 1, w);
-          }
-        }
-        const int st = j % kStages;
-        for (int w = 0; w < n_tiles && ok; ++w) {
-          ok = mbar_wait(bar(FwdSmem::p_full + w), j & 1, abort_flag);
-          if (ok && w == 0) {
-            ok = mbar_wait(bar(FwdSmem::v_full + st), (j / kStages) & 1, abort_flag);
-            // with a mask, warpgroup 0 signs off every value step after clearing the rows of dropped keys
-            if (ok && signoff) ok = mbar_wait(bar(FwdSmem::v_ready + st), (j / kStages) & 1, abort_flag);
-          }
-          if (!ok) break;
-          tc_fence_after_sync();
-          // O[128 x 32] += P[128 x 64] V[64 x 32]; V is MN-major (channel contiguous), 64-byte swizzle:
-          // 8-key groups are 512 bytes apart, each 16-key step advances 1024 bytes.
-          const uint32_t p_tmem = tmem_base + kPCol + w * (kKeys / 2);
-          const uint32_t o_tmem = tmem_base + kOCol + w * kHeadDim;
-          const uint64_t vdesc = smem_desc(smem_base + FwdSmem::v + st * kKvBytes, 16, 512, kSwizzle64B);
+      int st = 0, round = 0;
+      for (int i = 0; i < KS && ok; ++i) {
+        const int next = st + 1 == kStages ? 0 : st + 1, next_round = next == 0 ? round + 1 : round;
+        // the operands of the next score product and of this value product arrive ahead of the probabilities
+        if (i + 1 < KS) ok = mbar_wait(bar(Smem::k_full + ring + next), next_round & 1, abort_flag);
+        if (ok) ok = mbar_wait(bar(Smem::v_full + ring + st), round & 1, abort_flag);
+        // with a mask, a warpgroup signs off every value step after clearing the rows of dropped keys
+        if (ok && signoff) ok = mbar_wait(bar(Smem::v_ready + ring + st), round & 1, abort_flag);
+        if (ok) ok = mbar_wait(bar(Smem::p_full + w), i & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after_sync();
+        if (i + 1 < KS) issue_qk(next);  // the softmax waits for this one
+        // O[128 x 32] += P[128 x 64] V[64 x 32]; V is MN-major (channel contiguous), 64-byte swizzle:
+        // 8-key groups are 512 bytes apart, each 16-key step advances 1024 bytes.
+        const uint64_t vdesc = vdesc0 + uint64_t((st * kKvBytes) >> 4);
 #pragma unroll
-          for (int kk = 0; kk < kKeys / 16; ++kk)
-            mma_ts(o_tmem, p_tmem + kk * 8, vdesc + uint64_t(kk * (1024 >> 4)), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
-          mma_commit(bar(FwdSmem::pv_done + w));
-          if (j == KS - 1) mma_commit(bar(FwdSmem::o_final + w));
-          if (w == n_tiles - 1) mma_commit(bar(FwdSmem::v_empty + st));
-        }
+        for (int kk = 0; kk < kKeys / 16; ++kk)
+          mma_ts(o_t, p_t + kk * 8, vdesc + uint64_t(kk * (1024 >> 4)), idesc_pv, (i > 0 || kk > 0) ? 1u : 0u);
+        mma_commit(bar(Smem::pv_done + w));
+        mma_commit(bar(Smem::v_empty + ring + st));
+        st = next;
+        round = next_round;
       }
     }
   } else if ((warp >> 2) < n_tiles) {
     // ------------------------------------------------------------------ softmax warpgroups
-    const int w = warp >> 2;
+    const int w = warp >> 2, ring = ROWS ? w : 0, r = row_of(w);
     const int t = tid & (kTile - 1);
     const uint32_t lane_field = uint32_t((warp & 3) * 32) << 16;
     const uint32_t s_tmem = tmem_base + lane_field + kSCol + w * kKeys;
     const uint32_t p_tmem = tmem_base + lane_field + kPCol + w * (kKeys / 2);
     const uint32_t o_tmem = tmem_base + lane_field + kOCol + w * kHeadDim;
-    const int q_index = q0 + w * kTile + t;
-    const f32x2 scale2 = pack2(P.scale, P.scale);
-    const f32x2 log2e2 = pack2(kLog2e, kLog2e);
-    float m_run = -INFINITY, l_run = 0.f;
+    const int q_index = first_query(w) + t;
+    const float c = P.scale * kLog2e;
+    const f32x2 c2 = pack2(c, c), log2e2 = pack2(kLog2e, kLog2e);
+    const bool signs_off = needs_signoff(w) && (ROWS || w == 0);
+    float ref = -INFINITY, l_run = 0.f;  // reference (base-2 logit) and sum of the row
     bool ok = true;
 
-    for (int j = 0; j < KS && ok; ++j) {
-      uint32_t bits[2] = {0xffffffffu, 0xffffffffu};
-      bool all_kept = true;
-      if (has_bits) {
-        const uint2 wds = *reinterpret_cast<const uint2*>(keep_words + j * 2);
-        bits[0] = wds.x; bits[1] = wds.y;
-        all_kept = (wds.x & wds.y) == 0xffffffffu;
-      }
-      if (signoff && w == 0) {
+    for (int i = 0; i < KS && ok; ++i) {
+      uint2 bits = make_uint2(0xffffffffu, 0xffffffffu);  // keys 0-31 and 32-63 of the step
+      if (has_bits) bits = *reinterpret_cast<const uint2*>(keep_words + ring * kMaxKeepWords + step_at(i) * 2);
+      const bool all_kept = (bits.x & bits.y) == 0xffffffffu;
+      if (signs_off) {
         // Values of dropped keys must not reach the tensor core (0 * inf): clear their rows in shared memory.
         // Every step is signed off (one barrier phase per step); only steps with dropped keys are touched.
-        const int st = j % kStages;
+        const int slot = ring * kStages + i % kStages;
         if (!all_kept) {
-          ok = mbar_wait(bar(FwdSmem::v_full + st), (j / kStages) & 1, abort_flag);
+          ok = mbar_wait(bar(Smem::v_full + slot), (i / kStages) & 1, abort_flag);
           if (!ok) break;
-          if (t < kKeys && ((bits[t >> 5] >> (t & 31)) & 1u) == 0) {
-            uint4* row = reinterpret_cast<uint4*>(smem_gen + FwdSmem::v + st * kKvBytes + t * 64);
+          if (t < kKeys && (((t < 32 ? bits.x : bits.y) >> (t & 31)) & 1u) == 0) {
+            uint4* row = reinterpret_cast<uint4*>(smem_gen + Smem::v + slot * kKvBytes + t * 64);
             row[0] = row[1] = row[2] = row[3] = make_uint4(0, 0, 0, 0);
           }
           fence_proxy_async_smem();
         }
-        mbar_arrive_warp(bar(FwdSmem::v_ready + st));
+        mbar_arrive_warp(bar(Smem::v_ready + slot));
       }
 
-      // the two phases the step needs are probed together: one round trip to the barrier words when both are complete
-      const bool s_there = mbar_test(bar(FwdSmem::s_full + w), j & 1);
-      const bool bias_there = HAS_BIAS && mbar_test(bar(FwdSmem::bias_full + w * 2 + (j & 1)), (j >> 1) & 1);
-      ok = mbar_wait_probed(s_there, bar(FwdSmem::s_full + w), j & 1, abort_flag);
+      const int bias_slot = (ROWS ? 0 : w * 2) + (i & 1);
+      // the phases the step needs are probed together: one round trip to the barrier words when all are complete
+      const bool s_there = mbar_test(bar(Smem::s_full + w), i & 1);
+      const bool bias_there = HAS_BIAS && mbar_test(bar(Smem::bias_full + bias_slot), (i >> 1) & 1);
+      ok = mbar_wait_probed(s_there, bar(Smem::s_full + w), i & 1, abort_flag);
+      if (ok && HAS_BIAS) ok = mbar_wait_probed(bias_there, bar(Smem::bias_full + bias_slot), (i >> 1) & 1, abort_flag);
       if (!ok) break;
       tc_fence_after_sync();
-      f32x2 x[kKeys / 2];
-      static_assert(kKeys == 64, "two 32-column loads per step");
-      {
-        // nothing stands between the loads and their wait, and the registers are read only after it
-        uint32_t raw0[32], raw1[32];
-        tmem_ld32(s_tmem, raw0);
-        tmem_ld32(s_tmem + 32, raw1);
-        tmem_wait_ld();
-        tmem_loaded(raw0);
-        tmem_loaded(raw1);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          x[i] = pack2(__uint_as_float(raw0[2 * i]), __uint_as_float(raw0[2 * i + 1]));
-          x[16 + i] = pack2(__uint_as_float(raw1[2 * i]), __uint_as_float(raw1[2 * i + 1]));
-        }
-      }
-      tc_fence_before_sync();
-      mbar_arrive_warp(bar(FwdSmem::s_free + w));
+      // swizzled row of the bias tile: 16-byte chunk n holds keys 8 n .. 8 n + 7
+      const uint32_t bias_row = smem_base + Smem::bias + bias_slot * kBiasBytes + t * 128 + ((t & 7) << 4);
 
-      if (HAS_BIAS) {
-        const int slot = w * 2 + (j & 1);
-        ok = mbar_wait_probed(bias_there, bar(FwdSmem::bias_full + slot), (j >> 1) & 1, abort_flag);
-        if (!ok) break;
-        const uint8_t* row = smem_gen + FwdSmem::bias + slot * kBiasBytes + t * 128;
-        uint4 bv[8];
+      // Base-2 logits x + shift of 16 columns, as eight pairs; dropped keys become -inf.
+      auto logits16 = [&](int chunk, const uint32_t (&s)[16], const uint4 (&bw)[2], f32x2 shift2, bool drops, f32x2 (&x)[8]) {
+        const uint32_t words[8] = {bw[0].x, bw[0].y, bw[0].z, bw[0].w, bw[1].x, bw[1].y, bw[1].z, bw[1].w};
 #pragma unroll
-        for (int c = 0; c < 8; ++c) bv[c] = *reinterpret_cast<const uint4*>(row + ((c ^ (t & 7)) << 4));
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          x[c * 4 + 0] = fma2(x[c * 4 + 0], scale2, Half2<T>::widen(bv[c].x));
-          x[c * 4 + 1] = fma2(x[c * 4 + 1], scale2, Half2<T>::widen(bv[c].y));
-          x[c * 4 + 2] = fma2(x[c * 4 + 2], scale2, Half2<T>::widen(bv[c].z));
-          x[c * 4 + 3] = fma2(x[c * 4 + 3], scale2, Half2<T>::widen(bv[c].w));
-        }
-        mbar_arrive_warp(bar(FwdSmem::bias_empty + slot));
-      } else {
-#pragma unroll
-        for (int i = 0; i < kKeys / 2; ++i) x[i] = mul2(x[i], scale2);
-      }
-      if (!all_kept) {
-#pragma unroll
-        for (int i = 0; i < kKeys / 2; ++i) {
-          float lo, hi;
-          unpack2(x[i], lo, hi);
-          if (((bits[(2 * i) >> 5] >> ((2 * i) & 31)) & 1u) == 0) lo = -INFINITY;
-          if (((bits[(2 * i + 1) >> 5] >> ((2 * i + 1) & 31)) & 1u) == 0) hi = -INFINITY;
-          x[i] = pack2(lo, hi);
-        }
-      }
-      float peaks[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        float lo, hi;
-        unpack2(x[i], lo, hi);
-        peaks[i] = fmaxf(lo, hi);
-      }
-#pragma unroll
-      for (int i = 8; i < kKeys / 2; ++i) {
-        float lo, hi;
-        unpack2(x[i], lo, hi);
-        peaks[i & 7] = max3(peaks[i & 7], lo, hi);
-      }
-      const float peak = fmaxf(max3(peaks[0], peaks[1], peaks[2]), max3(max3(peaks[3], peaks[4], peaks[5]), peaks[6], peaks[7]));
-      // raise the running maximum only when it is exceeded by more than the slack (always on the first finite step)
-      const bool raise = peak > m_run + kRescaleSlack || (m_run == -INFINITY && peak > -INFINITY);
-      const float m_old = m_run;
-      if (raise) m_run = peak;
-      const float m_use = (m_run == -INFINITY) ? 0.f : m_run;
-      const float alpha = raise ? ex2((m_old - m_use) * kLog2e) : 1.f;
-      const float shift = -m_use * kLog2e;
-      const f32x2 shift2 = pack2(shift, shift);
-      f32x2 totals[4] = {pack2(0.f, 0.f), pack2(0.f, 0.f), pack2(0.f, 0.f), pack2(0.f, 0.f)};
-      uint32_t packed[kKeys / 2];
-      if (kFwdPolyEvery > 0 && all_kept) {
-        // every kFwdPolyEvery-th pair takes its 2^x from the FMA pipe; steps with dropped keys (-inf logits, whose
-        // probability must be exactly zero) keep the special-function unit for every element
-        const float shift_unit = fmaf(shift, 1.f / 128.f, float(-kExp2PolyLow) / 128.f);
-#pragma unroll
-        for (int i = 0; i < kKeys / 2; ++i) {
-          f32x2 p;
-          if ((i % (kFwdPolyEvery > 0 ? kFwdPolyEvery : 1)) == kFwdPolyEvery - 1) {
-            float x_lo, x_hi;
-            unpack2(x[i], x_lo, x_hi);
-            p = ex2_poly_unit(pack2(fma_sat(x_lo, kLog2e / 128.f, shift_unit), fma_sat(x_hi, kLog2e / 128.f, shift_unit)));
-          } else {
+        for (int n = 0; n < 8; ++n) {
+          const f32x2 s2 = pack2(__uint_as_float(s[2 * n]), __uint_as_float(s[2 * n + 1]));
+          x[n] = fma2(s2, c2, HAS_BIAS ? fma2(Half2<T>::widen(words[n]), log2e2, shift2) : shift2);
+          if (drops) {
+            const uint32_t kept = (chunk < 2 ? bits.x : bits.y) >> ((chunk & 1) * 16 + 2 * n);
             float lo, hi;
-            unpack2(fma2(x[i], log2e2, shift2), lo, hi);
-            p = pack2(ex2(lo), ex2(hi));
+            unpack2(x[n], lo, hi);
+            if ((kept & 1u) == 0) lo = -INFINITY;
+            if ((kept & 2u) == 0) hi = -INFINITY;
+            x[n] = pack2(lo, hi);
           }
-          totals[i & 3] = add2(totals[i & 3], p);
-          float p0, p1;
-          unpack2(p, p0, p1);
-          packed[i] = Half2<T>::pack(p0, p1);
         }
-      } else {
+      };
+      // The largest base-2 logit of the step.
+      auto step_peak = [&]() -> float {
+        float peak = -INFINITY;
+#pragma unroll 1
+        for (int chunk = 0; chunk < 4; ++chunk) {
+          uint32_t s[16];
+          uint4 bw[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+          if (HAS_BIAS) {
+            bw[0] = lds_v4_at(bias_row ^ uint32_t((chunk * 2) << 4));
+            bw[1] = lds_v4_at(bias_row ^ uint32_t((chunk * 2 + 1) << 4));
+          }
+          tmem_ld16(s_tmem + chunk * 16, s);
+          tmem_wait_ld();
+          tmem_loaded(s);
+          f32x2 x[8];
+          logits16(chunk, s, bw, pack2(0.f, 0.f), true, x);
 #pragma unroll
-        for (int i = 0; i < kKeys / 2; ++i) {
-          float lo, hi;
-          unpack2(fma2(x[i], log2e2, shift2), lo, hi);
-          const float p0 = ex2(lo), p1 = ex2(hi);
-          totals[i & 3] = add2(totals[i & 3], pack2(p0, p1));
-          packed[i] = Half2<T>::pack(p0, p1);
+          for (int n = 0; n < 8; ++n) {
+            float lo, hi;
+            unpack2(x[n], lo, hi);
+            peak = max3(peak, lo, hi);
+          }
         }
-      }
-      float t_lo, t_hi;
-      unpack2(add2(add2(totals[0], totals[1]), add2(totals[2], totals[3])), t_lo, t_hi);
-      l_run = l_run * alpha + (t_lo + t_hi);
-      if (j > 0) {
-        // the previous P V product must have finished with O and with the P columns before either is touched
-        ok = mbar_wait(bar(FwdSmem::pv_done + w), (j - 1) & 1, abort_flag);
+        return peak;
+      };
+      // Raises the reference of the rows whose step needs it, and rescales what they have summed so far.
+      auto raise = [&](bool wanted) -> bool {
+        tmem_wait_st();  // probabilities of a pass that is about to be repeated
+        const float peak = step_peak();
+        const bool raised = wanted && peak > ref;
+        const float alpha = raised ? ex2(ref - peak) : 1.f;  // 0 for a row without a reference so far
+        if (raised) {
+          ref = peak;
+          l_run *= alpha;
+        }
+        if (i > 0 && __any_sync(0xffffffffu, raised)) {
+          if (!mbar_wait(bar(Smem::pv_done + w), (i - 1) & 1, abort_flag)) return false;
+          tc_fence_after_sync();
+          uint32_t acc[32];
+          tmem_ld32(o_tmem, acc);
+          tmem_wait_ld();
+          tmem_loaded(acc);
+#pragma unroll
+          for (int n = 0; n < 32; ++n) acc[n] = __float_as_uint(__uint_as_float(acc[n]) * alpha);
+          tmem_st32(o_tmem, acc);
+          tmem_wait_st();
+        }
+        return true;
+      };
+      // Probabilities of the step into tensor memory; returns their sum.
+      bool p_free = i == 0;
+      auto step_pass = [&](auto drops) -> float {
+        const float shift = ref == -INFINITY ? 0.f : -ref;
+        const f32x2 shift2 = pack2(shift, shift);
+        f32x2 totals[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
+        uint32_t s[2][16], packed[16];
+        uint4 bw[2][2] = {{make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)}, {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)}};
+        tmem_ld16(s_tmem, s[0]);
+        if (HAS_BIAS) {
+          bw[0][0] = lds_v4_at(bias_row ^ uint32_t((0) << 4));
+          bw[0][1] = lds_v4_at(bias_row ^ uint32_t((1) << 4));
+        }
+#pragma unroll
+        for (int chunk = 0; chunk < 4; ++chunk) {
+          tmem_wait_ld();
+          tmem_loaded(s[chunk & 1]);
+          if (chunk < 3) {  // the next 16 columns travel under the arithmetic of these
+            tmem_ld16(s_tmem + (chunk + 1) * 16, s[(chunk + 1) & 1]);
+            if (HAS_BIAS) {
+              bw[(chunk + 1) & 1][0] = lds_v4_at(bias_row ^ uint32_t((chunk * 2 + 2) << 4));
+              bw[(chunk + 1) & 1][1] = lds_v4_at(bias_row ^ uint32_t((chunk * 2 + 3) << 4));
+            }
+          }
+          f32x2 x[8];
+          logits16(chunk, s[chunk & 1], bw[chunk & 1], shift2, decltype(drops)::value, x);
+#pragma unroll
+          for (int n = 0; n < 8; ++n) {
+            float lo, hi;
+            unpack2(x[n], lo, hi);
+            const float p0 = ex2(lo), p1 = ex2(hi);
+            totals[n & 1] = add2(totals[n & 1], pack2(p0, p1));
+            packed[(chunk & 1) * 8 + n] = Half2<T>::pack(p0, p1);
+          }
+          if (chunk & 1) {
+            if (!p_free) {  // the previous P V product must have finished with the P columns
+              ok = mbar_wait(bar(Smem::pv_done + w), (i - 1) & 1, abort_flag);
+              tc_fence_after_sync();
+              p_free = true;
+            }
+            tmem_st16(p_tmem + (chunk >> 1) * 16, packed);
+          }
+        }
+        float lo, hi;
+        unpack2(add2(totals[0], totals[1]), lo, hi);
+        return lo + hi;
+      };
+      float sum = 0.f;
+      bool wanted = ref == -INFINITY;
+#pragma unroll 1
+      for (int attempt = 0; attempt < 2 && ok; ++attempt) {
+        if (__any_sync(0xffffffffu, wanted)) ok = raise(wanted);
+        else if (attempt > 0) break;
         if (!ok) break;
-        tc_fence_after_sync();
+        sum = all_kept ? step_pass(std::false_type{}) : step_pass(std::true_type{});
+        wanted = !(sum < kStepSumLimit);
       }
-      if (j > 0 && __any_sync(0xffffffffu, raise)) {
-        uint32_t acc[32];
-        tmem_ld32(o_tmem, acc);
-        tmem_wait_ld();
-        tmem_loaded(acc);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) * alpha);
-        tmem_st32(o_tmem, acc);
-      }
-      tmem_st32(p_tmem, packed);
+      if (!ok) break;
+      l_run += sum;
       tmem_wait_st();
       tc_fence_before_sync();
-      mbar_arrive_warp(bar(FwdSmem::p_full + w));
+      mbar_arrive_warp(bar(Smem::p_full + w));
+      if (HAS_BIAS) mbar_arrive_warp(bar(Smem::bias_empty + bias_slot));
     }
 
     // Gated epilogue: the thread's 32 gate logits are requested before the wait for the last product, so that their
@@ -443,13 +482,17 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
 #pragma unroll
       for (int i = 0; i < 4; ++i) gate_words[i] = ldg_v4_here_if(reinterpret_cast<const uint4*>(g) + i, true);
     }
-    if (ok) ok = mbar_wait(bar(FwdSmem::o_final + w), 0, abort_flag);
+    if (ok && KS > 0) ok = mbar_wait(bar(Smem::pv_done + w), (KS - 1) & 1, abort_flag);
     if (ok) {
       tc_fence_after_sync();
       uint32_t acc[32];
-      tmem_ld32(o_tmem, acc);
-      tmem_wait_ld();
-      tmem_loaded(acc);
+#pragma unroll
+      for (int n = 0; n < 32; ++n) acc[n] = 0u;
+      if (KS > 0) {  // otherwise no product has written the accumulator
+        tmem_ld32(o_tmem, acc);
+        tmem_wait_ld();
+        tmem_loaded(acc);
+      }
       if (q_index < P.cols) {
         const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
         uint32_t o2[16];
@@ -499,9 +542,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
         }
         store_row(P.out, P.o_sb, P.o_sr, P.o_sc, P.o_sh, P.out_vec16, o2);
         if (P.lse) {
-          const float m_use = (m_run == -INFINITY) ? 0.f : m_run;
-          P.lse[((int64_t(b) * P.rows + r) * P.heads + h) * P.cols + q_index] =
-              l_run > 0.f ? (m_use + lg2(l_run) * kLn2) : 0.f;
+          P.lse[((int64_t(b) * P.rows + r) * P.heads + h) * P.cols + q_index] = l_run > 0.f ? (ref + lg2(l_run)) * kLn2 : 0.f;
         }
       }
     }
@@ -557,7 +598,7 @@ bool tensor_forward_applies(const oops_ta_problem& p) {
     if (p.cols == 1) return false;
   }
   if (p.cols > kMaxKeepWords * 32) return false;
-  const int64_t ctas = int64_t(p.batch) * p.rows * p.heads * ceil_div(p.cols, 2 * kTile);
+  const int64_t ctas = int64_t(p.batch) * p.rows * p.heads * ceil_div(p.cols, kTile);
   return ctas <= 0x7fffffffll;
 }
 
@@ -613,24 +654,32 @@ int launch_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse
   P.cols = p.cols;
   P.heads = p.heads;
   P.bias_groups = p.bias_groups;
-  P.q_pairs = (int)ceil_div(p.cols, 2 * kTile);
+  // A row-shared bias (or none) pairs rows: one bias tile serves two, and no CTA is half empty at an odd number of
+  // query tiles.  A per-row bias has nothing to share between rows; a single row has no partner.
+  const bool pair_rows = p.bias_groups <= 1 && p.rows > 1;
+  P.q_items = (int)ceil_div(p.cols, pair_rows ? kTile : 2 * kTile);
   P.k_steps = (int)ceil_div(p.cols, kKeys);
   P.scale = p.scale;
-  const unsigned grid = (unsigned)(int64_t(p.batch) * p.rows * p.heads * P.q_pairs);
+  const unsigned grid = (unsigned)(int64_t(p.batch) * (pair_rows ? ceil_div(p.rows, 2) : p.rows) * p.heads * P.q_items);
 
-  auto launch = [&](auto kernel) -> int {
+  auto launch = [&](auto kernel, int smem) -> int {
     // the attribute belongs to the (kernel, device) pair: it is set on every launch so that a host thread that
     // moves between devices never launches without it (the call costs well under a microsecond)
-    const int rc = reserve_smem(kernel, kFwdSmemBytes);
+    const int rc = reserve_smem(kernel, smem);
     if (rc) return rc;
-    kernel<<<grid, kFwdThreads, kFwdSmemBytes, stream>>>(P);
+    kernel<<<grid, kFwdThreads, smem, stream>>>(P);
     count_launch();
     return check_launch("tcgen05 forward");
   };
   auto pick = [&](auto type_tag) -> int {
     using T = decltype(type_tag);
-    if (gate) return has_bias ? launch(ta_fwd_kernel<T, true, true>) : launch(ta_fwd_kernel<T, false, true>);
-    return has_bias ? launch(ta_fwd_kernel<T, true, false>) : launch(ta_fwd_kernel<T, false, false>);
+    auto paired = [&](auto rows) -> int {
+      constexpr bool ROWS = decltype(rows)::value;
+      constexpr int smem = FwdSmem<ROWS>::bytes;
+      if (gate) return has_bias ? launch(ta_fwd_kernel<T, true, true, ROWS>, smem) : launch(ta_fwd_kernel<T, false, true, ROWS>, smem);
+      return has_bias ? launch(ta_fwd_kernel<T, true, false, ROWS>, smem) : launch(ta_fwd_kernel<T, false, false, ROWS>, smem);
+    };
+    return pair_rows ? paired(std::true_type{}) : paired(std::false_type{});
   };
   return p.dtype == OOPS_TA_BF16 ? pick(__nv_bfloat16{}) : pick(__half{});
 }
