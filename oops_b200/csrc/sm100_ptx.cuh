@@ -148,6 +148,10 @@ __device__ __forceinline__ uint4 lds_v4_at(uint32_t addr) {
   return v;
 }
 
+__device__ __forceinline__ void sts_v4_at(uint32_t addr, uint4 v) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
 // Four words from global memory when `take` is set, zeros otherwise; like the loads above it keeps its place and its
 // result is not touched before the caller uses it.
 __device__ __forceinline__ uint4 ldg_v4_here_if(const void* p, bool take) {

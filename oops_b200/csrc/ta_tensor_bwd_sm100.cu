@@ -45,32 +45,74 @@ constexpr int kRing = 4;                                // ring depth of the str
 // small helper kernels
 // ---------------------------------------------------------------------------------------------
 
+// delta[b][r][h][q] = sum_d O * dO.  Four lanes share a (cell, head): a warp reads 512 contiguous bytes of each tensor when
+// heads and cells are contiguous (one lane per (cell, head) read 64 bytes at 64-byte strides).  `row_inner`: cells of
+// neighbouring rows, not columns, are neighbours in memory (the ending-node form).  The blocks behind those of delta look at
+// the mask: live[b][r] has bit k set when some key of columns 128 k .. 128 k + 127 of the row is kept, and behind the rows'
+// words one word per eight rows tells whether they drop any key.
 template <typename T>
-__global__ void delta_kernel(oops_ta_pair out, oops_ta_pair dout, float* delta, int64_t total, int cols, int heads,
-                             int rows, int vec_ok) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const int q = i % cols;
-  const int h = (i / cols) % heads;
-  const int r = (i / (int64_t(cols) * heads)) % rows;
-  const int64_t b = i / (int64_t(cols) * heads * rows);
-  const T* o = reinterpret_cast<const T*>(out.ptr) + b * out.sb + int64_t(r) * out.sr + int64_t(q) * out.sc + h * out.sh;
-  const T* d = reinterpret_cast<const T*>(dout.ptr) + b * dout.sb + int64_t(r) * dout.sr + int64_t(q) * dout.sc + h * dout.sh;
-  float total_dot = 0.f;
-  if (vec_ok) {
+__global__ void __launch_bounds__(256, 8) prepare_kernel(oops_ta_pair out, oops_ta_pair dout, float* delta, uint32_t total, int cols,
+                                                      int heads, int rows, int vec_ok, int row_inner, uint32_t delta_blocks,
+                                                      const uint8_t* mask, int64_t m_sb, int64_t m_sr, int64_t m_sc,
+                                                      uint32_t* live, int num_rows) {
+  if (blockIdx.x >= delta_blocks) {
+    const int block = int(blockIdx.x - delta_blocks), row = block * 8 + int(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    bool dropped = false;
+    if (row < num_rows) {
+      const uint8_t* bytes = mask + (row / rows) * m_sb + int64_t(row % rows) * m_sr;
+      uint32_t bits = 0;
+      for (int first = 0; first < cols; first += 128) {
+        bool any = false;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const uint4 a = reinterpret_cast<const uint4*>(o)[c];
-      const uint4 g = reinterpret_cast<const uint4*>(d)[c];
+        for (int i = 0; i < 4; ++i) {
+          const int key = first + i * 32 + lane;
+          if (key < cols) {
+            const bool keep = bytes[int64_t(key) * m_sc] != 0;
+            any |= keep;
+            dropped |= !keep;
+          }
+        }
+        if (__any_sync(0xffffffffu, any)) bits |= 1u << (first / 128);
+      }
+      if (lane == 0) live[row] = bits;
+    }
+    const int drops = __syncthreads_or(dropped);
+    if (threadIdx.x == 0) live[num_rows + block] = uint32_t(drops != 0);
+    return;
+  }
+  const uint32_t item = blockIdx.x * 64u + (threadIdx.x >> 2);
+  const int part = threadIdx.x & 3;
+  float dot = 0.f;
+  int64_t at = 0;
+  if (item < total) {
+    const uint32_t h = item % uint32_t(heads), cell = item / uint32_t(heads);
+    const uint32_t inner = row_inner ? uint32_t(rows) : uint32_t(cols), outer = row_inner ? uint32_t(cols) : uint32_t(rows);
+    const uint32_t i = cell % inner, rest = cell / inner, o = rest % outer, b = rest / outer;
+    const uint32_t r = row_inner ? i : o, q = row_inner ? o : i;
+    const T* po = reinterpret_cast<const T*>(out.ptr) + b * out.sb + int64_t(r) * out.sr + int64_t(q) * out.sc + h * out.sh + part * 8;
+    const T* pd = reinterpret_cast<const T*>(dout.ptr) + b * dout.sb + int64_t(r) * dout.sr + int64_t(q) * dout.sc + h * dout.sh + part * 8;
+    at = ((int64_t(b) * rows + r) * heads + h) * cols + q;
+    if (vec_ok) {
+      const uint4 a = *reinterpret_cast<const uint4*>(po), g = *reinterpret_cast<const uint4*>(pd);
       const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        total_dot += Half2<T>::lo(aw[e]) * Half2<T>::lo(gw[e]) + Half2<T>::hi(aw[e]) * Half2<T>::hi(gw[e]);
+      for (int e = 0; e < 4; ++e) dot += Half2<T>::lo(aw[e]) * Half2<T>::lo(gw[e]) + Half2<T>::hi(aw[e]) * Half2<T>::hi(gw[e]);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 8; ++c) dot += float(po[c]) * float(pd[c]);
     }
-  } else {
-    for (int c = 0; c < kHeadDim; ++c) total_dot += float(o[c]) * float(d[c]);
   }
-  delta[i] = total_dot;
+  dot += __shfl_xor_sync(0xffffffffu, dot, 1);
+  dot += __shfl_xor_sync(0xffffffffu, dot, 2);
+  if (item < total && part == 0) delta[at] = dot;
+}
+
+// Whether the mask that prepare_kernel has looked at keeps every key (one warp's answer).
+__device__ __forceinline__ bool keeps_all(const uint32_t* live, int num_rows, int lane) {
+  const int words = (num_rows + 7) / 8;
+  bool drops = false;
+  for (int i = lane; i < words; i += 32) drops |= __ldg(live + num_rows + i) != 0;
+  return !__any_sync(0xffffffffu, drops);
 }
 
 // dst[z][k][q] = src[z][q][k] for 16-bit elements; dst rows are `dst_stride` elements apart.
@@ -882,27 +924,36 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) ta_bwd_dkv_kernel(const 
 // ---------------------------------------------------------------------------------------------
 // fused dQ / dK / dV kernel: one pass over the score tiles of a pair row
 // ---------------------------------------------------------------------------------------------
-// CTA = (batch, row, head).  The row's query tiles are taken in groups of up to 6; for every group, every key tile and
-// every query tile of the group: S = Q K^T and dP = dO V^T (128 x 128, tensor memory) -> the four warpgroups (a thread
+// An item of the walk is a (batch, row, head).  Its query tiles are taken in groups of up to 6; for every group, every key
+// tile and every query tile of the group: S = Q K^T and dP = dO V^T (128 x 128, tensor memory) -> the four warpgroups (a thread
 // owns a query, a warpgroup 32 of the 128 keys) compute P and dS once and write them, 16-bit, into two shared-memory
 // images whose rows are queries and whose 128-byte-swizzled columns are keys.  The tensor core reads those images three
 // ways: dV += P^T dO and dK += dS^T Q take them as MN-major A operands (M = keys), dQ += dS K as a K-major A operand
 // (M = queries).  dQ of the group's query tiles, dK and dV of the current key tile stay in tensor memory:
 // S 128 | dP 128 | dK 32 | dV 32 | dQ 6 x 32 = 512 columns.  One `ex2` per logit and five products, where the
-// separate dQ and dK/dV kernels spend two and seven.  The images cost shared-memory bandwidth (64 KB written and
-// 96 KB read per 128 x 128 step), which is what bounds this kernel.
+// separate dQ and dK/dV kernels spend two and seven.
+// What bounds it: a step of some 2600 clocks spends 1100 in its arithmetic, where the exponentials (1024 clocks of the
+// special-function units) and the issue slots are both full, and the rest in moving images, bias and scores (some 2000 clocks
+// of the shared-memory port are busy) between barriers that all sixteen warps pass together.  Hence no branch, fence or
+// generic-address store in a step's body, and the writers of the images do not fence: they release a barrier, and the
+// issuer that acquires it fences once for all of them before its products read (N = 768: 1190 -> 1120 us with both).
+// Halving the step between two sets of warps that run half a step apart was tried: the single P image couples them, 3 to 10 %
+// slower.
 // Rows of more than 768 columns have several groups.  The CTA walks them in order and carries the f32 sums of dK and
 // dV of every key tile from group to group in a scratch slot that belongs to its SM (one CTA is resident per SM, so
 // the slot is private while the CTA runs, and at 128 bytes per key and tensor it stays in L2): the thread that owns a
 // key adds what the slot holds, and stores 16-bit dK/dV after the last group.  The order of the sums is fixed, so the
 // gradients are bitwise reproducible, and no partial planes or reduction kernels exist.
+// Where a row is one group, the CTA goes through several items without a stop: the copies and score products of the next one
+// run under the last steps and the read-out of this one.  (A CTA per item spent half of its time on set-up and read-out at
+// 256 columns: 4 steps in 26000 clocks.  N = 256: 86 -> 58 us, N = 768: 1190 -> 1032 us with what is named above.)
 
+constexpr int kFMaxCols = 4096;          // longest row taken: 32 key tiles
 constexpr int kFMaxQTiles = 6;
 constexpr int kFThreads = 608;  // 16 element-wise warps, TMA producer, score issuer, accumulation issuer
 constexpr int kFProducerWarp = 16, kFScoreWarp = 17, kFAccWarp = 18;
 constexpr int kFImage = 2 * 16384;       // P or dS of a step: two 64-key halves of 128 rows x 128 bytes
 constexpr int kFBias = 2 * kBiasStep;    // 128 x 128 bias tile as two 64-key boxes (staging: copied to registers at once)
-constexpr int kFKeepWords = 128;         // keep-bit table of a row
 constexpr int kFSlots = 256;             // scratch slots of the group-to-group sums: one per SM id
 
 struct FSmem {
@@ -918,8 +969,7 @@ struct FSmem {
   static constexpr int qd_empty = qd_full + 3;         // [3]
   static constexpr int kv_full = qd_empty + 3;         // [2]
   static constexpr int kv_empty = kv_full + 2;         // [2]
-  static constexpr int k_ready = kv_empty + 2;         // [2] dropped keys' rows cleared (only with a dropping mask)
-  static constexpr int bias_full = k_ready + 2;
+  static constexpr int bias_full = kv_empty + 2;
   static constexpr int bias_empty = bias_full + 1;     // every warp has copied its words of the tile to registers
   static constexpr int sd_full = bias_empty + 1;       // S and dP of a step are in tensor memory
   static constexpr int sd_free = sd_full + 1;          // all warps have read them
@@ -931,9 +981,7 @@ struct FSmem {
   static constexpr int num_bars = dq_free + 1;
   static constexpr int tmem_slot = bars + num_bars * 8;
   static constexpr int abort_flag = tmem_slot + 4;
-  static constexpr int drop_flags = abort_flag + 4;    // [16]
-  static constexpr int keep = drop_flags + 64;
-  static constexpr int total = keep + kFKeepWords * 4;
+  static constexpr int total = abort_flag + 4;
 };
 constexpr int kFSmemBytes = FSmem::total + 1024;
 static_assert(kFSmemBytes <= 232448, "fused reverse kernel: shared memory over the per-CTA limit");
@@ -946,124 +994,68 @@ struct FParams {
   const float* lse;
   const float* delta;
   const uint8_t* mask;
+  const uint32_t* live;  // what prepare_kernel has found out about the mask
   int64_t m_sb, m_sr, m_sc;
-  int batch, rows, cols, heads, bias_groups;
+  int batch, rows, cols, heads, bias_groups, items;
   int q_tiles, k_tiles, groups, tiles_per_group;
   int write_dq, write_dk, write_dv;
   float scale;
 };
 
-// The walk over a pair row's steps, identical in every role of the kernel: groups of query tiles outermost, then key
-// tiles, then the query tiles of the group.  Ring slots and barrier phases count steps and key tiles across groups.
+// The walk over a CTA's steps, identical in every role of the kernel: parts outermost, then key tiles, then query tiles.
+// A part is a group of query tiles of the CTA's one item, or, where a row is a single group, a whole item of the several
+// that the CTA works through.  Ring slots and barrier phases count steps, key tiles and parts.  (Trip counts come from the
+// launch parameters alone: with counts read from memory the compiler takes the loops for divergent and guards every
+// branch in them, which cost the kernel 8 %.)
+template <bool GROUPS>
 struct FWalk {
-  int tiles_per_group, q_tiles, k_tiles, groups;
-  int g, kt, qi, nq;  // group, key tile, query tile within the group, query tiles of the group
-  int s, ktc;         // steps and key tiles walked so far
+  int tiles_per_group, q_tiles, k_tiles, parts, item_step;
+  int part, item, first;  // part, its item, its first query tile
+  int kt, qi, nq;         // key tile, query tile within the part, query tiles of the part
+  int s, ktc;             // steps and key tiles walked so far
   __device__ FWalk(const FParams& P)
-      : tiles_per_group(P.tiles_per_group), q_tiles(P.q_tiles), k_tiles(P.k_tiles), groups(P.groups), g(0), kt(0), qi(0),
-        nq(min(P.tiles_per_group, P.q_tiles)), s(0), ktc(0) {}
-  __device__ bool done() const { return g >= groups; }
-  __device__ int qt() const { return g * tiles_per_group + qi; }
+      : tiles_per_group(P.tiles_per_group), q_tiles(P.q_tiles), k_tiles(P.k_tiles), parts(GROUPS ? P.groups : P.items),
+        item_step(int(gridDim.x)), part(0), item(int(blockIdx.x)), first(0), kt(0), qi(0), nq(min(P.tiles_per_group, P.q_tiles)),
+        s(0), ktc(0) {}
+  __device__ bool done() const { return GROUPS ? part >= parts : item >= parts; }
+  __device__ int qt() const { return GROUPS ? first + qi : qi; }
+  __device__ void next_tile() {
+    ++ktc;
+    if (++kt < k_tiles) return;
+    kt = 0;
+    ++part;
+    if (GROUPS) {
+      first += tiles_per_group;
+      nq = min(tiles_per_group, q_tiles - first);
+    } else {
+      item += item_step;
+    }
+  }
   __device__ void next() {
     ++s;
     if (++qi < nq) return;
     qi = 0;
-    ++ktc;
-    if (++kt < k_tiles) return;
-    kt = 0;
-    ++g;
-    nq = min(tiles_per_group, q_tiles - g * tiles_per_group);
+    next_tile();
   }
 };
 
-template <typename T, bool HAS_BIAS>
-__global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid_constant__ FParams P) {
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + FSmem::abort_flag);
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + FSmem::tmem_slot);
-  uint32_t* keep_words = reinterpret_cast<uint32_t*>(smem_gen + FSmem::keep);
+// GROUPS: rows of several groups of query tiles.  BITS: some key may be dropped, by the mask or because the last key tile
+// is ragged.
+template <typename T, bool HAS_BIAS, bool GROUPS, bool BITS>
+__device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base, uint8_t* smem_gen, volatile int* abort_flag,
+                                           uint32_t tmem_base, int tid, int warp, int lane) {
   auto bar = [&](int index) -> uint32_t { return smem_base + FSmem::bars + index * 8; };
-
-  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-  if (device_failed()) return;
-  int idx = blockIdx.x;
-  const int h = idx % P.heads;
-  idx /= P.heads;
-  const int r = idx % P.rows;
-  const int b = idx / P.rows;
-  const int KT = P.k_tiles;
-  const int bias_group = P.bias_groups == 1 ? 0 : r;
-  const bool has_mask = P.mask != nullptr;
-  const bool has_bits = has_mask || (P.cols % kTile) != 0;
+  const bool has_mask = BITS && P.mask != nullptr;
+  constexpr bool has_bits = BITS;
   // tensor-memory columns
   constexpr int kSCol = 0, kDpCol = 128, kDkCol = 256, kDvCol = 288, kDqCol = 320;
-
-  if (tid == 0) {
-    *abort_flag = 0;
-    for (int i = 0; i < 3; ++i) {
-      mbar_init(bar(FSmem::qd_full + i), 1);
-      mbar_init(bar(FSmem::qd_empty + i), 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(FSmem::pds_full + i), 16);
-      mbar_init(bar(FSmem::pds_done + i), 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(FSmem::kv_full + i), 1);
-      mbar_init(bar(FSmem::kv_empty + i), 1);
-      mbar_init(bar(FSmem::k_ready + i), 4);
-    }
-    mbar_init(bar(FSmem::p_done), 1);
-    mbar_init(bar(FSmem::bias_full), 1);
-    mbar_init(bar(FSmem::bias_empty), 16);
-    mbar_init(bar(FSmem::sd_full), 1);
-    mbar_init(bar(FSmem::sd_free), 16);
-    mbar_init(bar(FSmem::dkv_free), 8);
-    mbar_init(bar(FSmem::dq_free), 16);
-    fence_barrier_init();
-  }
-  if (warp == kFScoreWarp) {
-    tmem_alloc(smem_base + FSmem::tmem_slot, 512);
-    tmem_relinquish();
-    tc_fence_before_sync();
-  }
-  __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
-  // keep-bit table (one bit per key of this pair row), built by the element-wise warps while the first copies fly
-  uint32_t* drop_flags = reinterpret_cast<uint32_t*>(smem_gen + FSmem::drop_flags);
-  bool signoff = false;
-  if (has_bits && warp != kFProducerWarp) {
-    if (warp < 16) {
-      const uint8_t* mask_row = has_mask ? P.mask + b * P.m_sb + int64_t(r) * P.m_sr : nullptr;
-      bool dropped_any = false;
-      for (int word = warp; word < KT * 4; word += 16) {
-        const int key = word * 32 + lane;
-        bool keep = key < P.cols;
-        if (keep && has_mask) {
-          keep = mask_row[int64_t(key) * P.m_sc] != 0;
-          dropped_any |= !keep;
-        }
-        const uint32_t bits = __ballot_sync(0xffffffffu, keep);
-        if (lane == 0) keep_words[word] = bits;
-      }
-      dropped_any = __any_sync(0xffffffffu, dropped_any);
-      if (lane == 0) drop_flags[warp] = dropped_any ? 1u : 0u;
-    }
-    named_barrier_sync(1, kFThreads - 32);
-    if (has_mask) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) signoff |= drop_flags[i] != 0;
-    }
-  }
 
   if (warp == kFProducerWarp) {
     if (lane == 0) {
       bool ok = true;
-      for (FWalk w(P); !w.done() && ok; w.next()) {
+      for (FWalk<GROUPS> w(P); !w.done() && ok; w.next()) {
         const int s = w.s, kt = w.kt, qt = w.qt(), qs = s % 3;
+        const int row = w.item / P.heads, h = w.item - row * P.heads, b = row / P.rows, r = row - b * P.rows;
         if (w.qi == 0) {
           const int ks = w.ktc & 1;
           if (w.ktc >= 2) ok = mbar_wait(bar(FSmem::kv_empty + ks), ((w.ktc >> 1) - 1) & 1, abort_flag);
@@ -1083,7 +1075,7 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
           mbar_expect_tx(bar(FSmem::bias_full), kFBias);
           for (int box = 0; box < 2; ++box)
             tma_load_5d(smem_base + FSmem::bias + box * kBiasStep, &P.map_bias, bar(FSmem::bias_full), kt * kTile + box * 64,
-                        qt * kTile, h, bias_group, b);
+                        qt * kTile, h, P.bias_groups == 1 ? 0 : r, b);
         }
       }
     }
@@ -1091,13 +1083,10 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
     {
       constexpr uint32_t idesc = instr_desc(Half2<T>::kFormat, 0, 0, kTile, kTile);
       bool ok = true;
-      for (FWalk w(P); !w.done() && ok; w.next()) {
+      for (FWalk<GROUPS> w(P); !w.done() && ok; w.next()) {
         const int s = w.s, qs = s % 3, ks = w.ktc & 1;
         ok = mbar_wait_warp(bar(FSmem::qd_full + qs), (s / 3) & 1, abort_flag);
-        if (ok && w.qi == 0) {
-          ok = mbar_wait_warp(bar(FSmem::kv_full + ks), (w.ktc >> 1) & 1, abort_flag);
-          if (ok && signoff) ok = mbar_wait_warp(bar(FSmem::k_ready + ks), (w.ktc >> 1) & 1, abort_flag);
-        }
+        if (ok && w.qi == 0) ok = mbar_wait_warp(bar(FSmem::kv_full + ks), (w.ktc >> 1) & 1, abort_flag);
         if (ok && s > 0) ok = mbar_wait_warp(bar(FSmem::sd_free), (s - 1) & 1, abort_flag);
         if (!ok) break;
         tc_fence_after_sync();
@@ -1120,16 +1109,17 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
       constexpr uint32_t idesc_t = instr_desc(fmt, 1, 1, kTile, kHeadDim);  // A = image^T (M = keys), B MN-major
       constexpr uint32_t idesc_q = instr_desc(fmt, 0, 1, kTile, kHeadDim);  // A = image (M = queries), B MN-major
       bool ok = true;
-      for (FWalk w(P); !w.done() && ok; w.next()) {
+      for (FWalk<GROUPS> w(P); !w.done() && ok; w.next()) {
         const int s = w.s, kt = w.kt, qi = w.qi, qs = s % 3, ks = w.ktc & 1;
         ok = mbar_wait_warp(bar(FSmem::qd_full + qs), (s / 3) & 1, abort_flag);
         if (ok) ok = mbar_wait_warp(bar(FSmem::kv_full + ks), (w.ktc >> 1) & 1, abort_flag);
         if (ok) ok = mbar_wait_warp(bar(FSmem::pds_full + (s & 1)), (s >> 1) & 1, abort_flag);
         // dK and dV of the previous key tile must have been read out before they are overwritten,
-        // and so must dQ of the previous group of query tiles
+        // and so must dQ of the previous part
         if (ok && qi == 0 && w.ktc > 0) ok = mbar_wait_warp(bar(FSmem::dkv_free), (w.ktc - 1) & 1, abort_flag);
-        if (ok && qi == 0 && kt == 0 && w.g > 0) ok = mbar_wait_warp(bar(FSmem::dq_free), (w.g - 1) & 1, abort_flag);
+        if (ok && qi == 0 && kt == 0 && w.part > 0) ok = mbar_wait_warp(bar(FSmem::dq_free), (w.part - 1) & 1, abort_flag);
         if (!ok) break;
+        fence_proxy_async_smem();  // the images (and cleared key rows) were written through the generic proxy
         tc_fence_after_sync();
         const uint32_t ps = smem_base + FSmem::ps, dss = smem_base + FSmem::dss + (s & 1) * kFImage;
         const uint64_t qdesc = smem_desc(smem_base + FSmem::q + qs * kBigTile, 16, 512, kSwizzle64B);     // MN-major B
@@ -1160,23 +1150,41 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
     const uint32_t lanes_t = tmem_base + lane_field;
     const float scale = P.scale;
     const f32x2 c2 = pack2(scale * kLog2e, scale * kLog2e), log2e2 = pack2(kLog2e, kLog2e);
-    const int64_t stat_base = ((int64_t(b) * P.rows + r) * P.heads + h) * P.cols;
-    // statistics of this thread's query in a step's query tile, fetched one step ahead and left untouched till then
-    auto fetch_stats = [&](const FWalk& at, float& lse_raw, float& delta_raw) {
+    // Statistics of this thread's query in a step's query tile (items count (batch, row, head) as the statistics do), fetched
+    // one step ahead and left untouched till then.
+    const int64_t stat0 = int64_t(blockIdx.x) * P.cols;
+    auto fetch_stats = [&](const FWalk<GROUPS>& at, float& lse_raw, float& delta_raw) {
       lse_raw = INFINITY;
       delta_raw = 0.f;
       const int q = at.qt() * kTile + t;
       if (!at.done() && q < P.cols) {
-        lse_raw = ldg_f32_here(P.lse + stat_base + q);
-        delta_raw = ldg_f32_here(P.delta + stat_base + q);
+        const int64_t stat = GROUPS ? stat0 + q : int64_t(uint32_t(at.item) * uint32_t(P.cols) + uint32_t(q));
+        lse_raw = ldg_f32_here(P.lse + stat);
+        delta_raw = ldg_f32_here(P.delta + stat);
       }
+    };
+    // The kept bit of this lane's key of a key tile (32 keys of this warpgroup), fetched a key tile ahead.
+    auto mask_row_of = [&](int item) -> const uint8_t* {
+      const int row = item / P.heads, b = row / P.rows;
+      return P.mask + b * P.m_sb + int64_t(row - b * P.rows) * P.m_sr;
+    };
+    auto fetch_keep = [&](const uint8_t* row, const FWalk<GROUPS>& at) -> uint32_t {
+      const int key = at.kt * kTile + wg * 32 + lane;
+      if (at.done() || key >= P.cols) return 0;
+      return has_mask ? ldg_u8_here(row + int64_t(key) * P.m_sc) : 1u;
+    };
+    const int row0 = int(blockIdx.x) / P.heads, h0 = int(blockIdx.x) - row0 * P.heads, b0 = row0 / P.rows, r0 = row0 - b0 * P.rows;
+    auto item_row = [&](const oops_ta_pair& t, int item) -> T* {
+      if (GROUPS) return reinterpret_cast<T*>(t.ptr) + b0 * t.sb + int64_t(r0) * t.sr + h0 * t.sh;
+      const int row = item / P.heads, b = row / P.rows;
+      return reinterpret_cast<T*>(t.ptr) + b * t.sb + int64_t(row - b * P.rows) * t.sr + int64_t(item - row * P.heads) * t.sh;
     };
     uint32_t sm_id;
     asm volatile("mov.u32 %0, %%smid;" : "=r"(sm_id));
     // dK (warpgroup 0) and dV (warpgroup 1) of key tile kt, complete for the query tiles of group g: lanes are keys.
     // With several groups the f32 sums travel from group to group through this SM's scratch slot (the same thread
     // owns a key in every group), and the last group stores the 16-bit result.
-    auto store_key_tile = [&](int g, int kt) {
+    auto store_key_tile = [&](int item, int g, int kt) {
       if (wg > 1) return;
       uint32_t acc[32];
       tmem_ld32(lanes_t + (wg == 0 ? kDkCol : kDvCol), acc);
@@ -1188,7 +1196,7 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
       if (key >= P.cols) return;
       const bool wanted = wg == 0 ? P.write_dk != 0 : P.write_dv != 0;
       if (!wanted) return;
-      if (P.groups > 1) {
+      if (GROUPS) {
         // plane i of the slot holds channels 4i .. 4i+3 of every key, so that a warp's 32 keys are 512 contiguous bytes
         float4* slot = reinterpret_cast<float4*>(P.slots) + (int64_t(sm_id) * 2 + wg) * 8 * P.slot_keys + key;
         if (g == 0) {
@@ -1205,32 +1213,31 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
         return;
       }
       const oops_ta_pair& o = wg == 0 ? P.dk : P.dv;
-      T* dst = reinterpret_cast<T*>(o.ptr) + b * o.sb + int64_t(r) * o.sr + int64_t(key) * o.sc + h * o.sh;
-      store_row32<T>(dst, acc, wg == 0 ? scale : 1.f, pair_vec_ok(o));
+      store_row32<T>(item_row(o, item) + int64_t(key) * o.sc, acc, wg == 0 ? scale : 1.f, pair_vec_ok(o));
     };
-    // dQ of the query tiles of group g (tile qi is read out by warpgroup qi % 4; lanes are queries); every warp then
-    // reports that the accumulators may be overwritten by the next group
-    auto store_query_tiles = [&](int g) {
-      const int tiles = min(P.tiles_per_group, P.q_tiles - g * P.tiles_per_group);
+    // dQ of a part, whose query tiles start with `first` (tile qi is read out by warpgroup qi % 4; lanes are queries); every
+    // warp then reports that the accumulators may be overwritten by the next part
+    auto store_query_tiles = [&](int item, int first) {
+      const int tiles = min(P.tiles_per_group, P.q_tiles - first);
       for (int qi = wg; qi < tiles; qi += 4) {
         uint32_t acc[32];
         tmem_ld32(lanes_t + kDqCol + qi * kHeadDim, acc);
         tmem_wait_ld();
         tmem_loaded(acc);
-        const int q_index = (g * P.tiles_per_group + qi) * kTile + t;
-        if (q_index < P.cols && P.write_dq) {
-          T* dst = reinterpret_cast<T*>(P.dq.ptr) + b * P.dq.sb + int64_t(r) * P.dq.sr + int64_t(q_index) * P.dq.sc + h * P.dq.sh;
-          store_row32<T>(dst, acc, scale, pair_vec_ok(P.dq));
-        }
+        const int q_index = (first + qi) * kTile + t;
+        if (q_index < P.cols && P.write_dq)
+          store_row32<T>(item_row(P.dq, item) + int64_t(q_index) * P.dq.sc, acc, scale, pair_vec_ok(P.dq));
       }
       tc_fence_before_sync();
       mbar_arrive_warp(bar(FSmem::dq_free));
     };
-    FWalk w(P);
+    FWalk<GROUPS> w(P);
     float lse_next, delta_next;
     fetch_stats(w, lse_next, delta_next);
+    const uint8_t* mask_row = has_mask ? mask_row_of(w.item) : nullptr;  // of the key tile to come
+    uint32_t keep_raw = has_bits ? fetch_keep(mask_row, w) : 0u, bits = 0xffffffffu;
     bool ok = true;
-    if (P.groups > 1 && sm_id >= uint32_t(kFSlots)) {  // no scratch slot for this SM id: give up like a wait that ran out
+    if (GROUPS && sm_id >= uint32_t(kFSlots)) {  // no scratch slot for this SM id: give up like a wait that ran out
       *abort_flag = 1;
       ok = false;
     }
@@ -1238,16 +1245,26 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
     // bias row of this thread's query in the staging tile: box (wg >> 1), 16-byte chunks (wg & 1) * 4 .. + 3
     const uint8_t* bias_row = smem_gen + FSmem::bias + (wg >> 1) * kBiasStep + t * 128 + (((t & 7) ^ ((wg & 1) * 4)) << 4);
 
-    int last_g = 0, last_kt = 0;  // group and key tile of the previous step
-    for (; !w.done() && ok; last_g = w.g, last_kt = w.kt, w.next()) {
+    int last_item = 0, last_part = 0, last_first = 0, last_kt = 0;  // of the previous step
+    for (; !w.done() && ok; last_item = w.item, last_part = w.part, last_first = w.first, last_kt = w.kt, w.next()) {
       const int s = w.s, kt = w.kt, qi = w.qi, buf = s & 1;
-      if (s > 0) {
-        // The images of step s - 1 are handed to the products only now: their stores have drained under the read-out
-        // and the loop's turn-around, and the fence stands before anything this step requests, so it does not wait;
-        // the accumulating issuer has slack to spare.
-        fence_proxy_async_smem();
-        mbar_arrive_warp(bar(FSmem::pds_full + (buf ^ 1)));
+      if (has_bits && qi == 0) {
+        bits = __ballot_sync(0xffffffffu, keep_raw != 0);
+        FWalk<GROUPS> ahead = w;
+        ahead.next_tile();
+        if (!GROUPS && has_mask && ahead.kt == 0 && !ahead.done()) mask_row = mask_row_of(ahead.item);
+        keep_raw = fetch_keep(mask_row, ahead);
+        if (has_mask && bits != 0xffffffffu) {
+          // Key rows of dropped keys must not reach the dQ product (0 * inf): they are cleared in shared memory, eight of
+          // this warpgroup's 32 by each warp.  The scores of these keys are dropped whatever they are.
+          ok = mbar_wait(bar(FSmem::kv_full + (w.ktc & 1)), (w.ktc >> 1) & 1, abort_flag);
+          if (!ok) break;
+          const int key = (warp & 3) * 8 + (lane >> 2);
+          if (((bits >> key) & 1u) == 0)
+            sts_v4_at(smem_base + FSmem::k + (w.ktc & 1) * kBigTile + (wg * 32 + key) * 64 + (lane & 3) * 16, make_uint4(0, 0, 0, 0));
+        }
       }
+      if (s > 0) mbar_arrive_warp(bar(FSmem::pds_full + (buf ^ 1)));  // the images of step s - 1, their stores drained by now
       // The three phases the step needs first are probed together (one round trip to the barrier words); in the steady
       // state, where these warps are the slow side of the pipeline, all three are complete.
       const bool bias_there = HAS_BIAS && mbar_test(bar(FSmem::bias_full), s & 1);
@@ -1255,12 +1272,11 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
       const bool scores_there = mbar_test(bar(FSmem::sd_full), s & 1);
       const float neg_lse2 = -lse_next * kLog2e, neg_delta = -delta_next;
       {
-        FWalk ahead = w;
+        FWalk<GROUPS> ahead = w;
         ahead.next();
         fetch_stats(ahead, lse_next, delta_next);
       }
       const f32x2 nl1 = pack2(neg_lse2, neg_lse2), nd1 = pack2(neg_delta, neg_delta);
-      const uint32_t bits = has_bits ? keep_words[kt * 4 + wg] : 0xffffffffu;
       // The step's bias words are requested at once; the staging tile is handed back as soon as they have arrived
       // (below, after the first scores have been fetched), so that the next tile's copy runs under this step's arithmetic.
       uint4 bias_words[4] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
@@ -1270,18 +1286,6 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
 #pragma unroll
         for (int c = 0; c < 4; ++c) bias_words[c] = lds_v4_here(swizzled_chunk(bias_row, c));
       }
-      if (signoff && qi == 0 && warp < 4) {
-        // key rows of dropped keys must not reach the dQ product (0 * inf): clear them in shared memory
-        const int ks = w.ktc & 1;
-        ok = mbar_wait(bar(FSmem::kv_full + ks), (w.ktc >> 1) & 1, abort_flag);
-        if (!ok) break;
-        if (((keep_words[kt * 4 + (t >> 5)] >> (t & 31)) & 1u) == 0) {
-          uint4* row = reinterpret_cast<uint4*>(smem_gen + FSmem::k + ks * kBigTile + t * 64);
-          row[0] = row[1] = row[2] = row[3] = make_uint4(0, 0, 0, 0);
-        }
-        fence_proxy_async_smem();
-        mbar_arrive_warp(bar(FSmem::k_ready + ks));
-      }
       // this step's dS image was last read by the products of step s - 2, the P image by the dV products of s - 1
       ok = mbar_wait_probed(image_free, bar(FSmem::pds_done + buf), ((s >> 1) - 1) & 1, abort_flag);
       if (ok) ok = mbar_wait_probed(scores_there, bar(FSmem::sd_full), s & 1, abort_flag);
@@ -1289,57 +1293,64 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
       tc_fence_after_sync();
       // image rows are queries; this warpgroup's 32 keys are chunks (wg & 1) * 4 .. + 3 of half (wg >> 1)
       const int row_at = (wg >> 1) * 16384 + t * 128 + (((t & 7) ^ ((wg & 1) * 4)) << 4);
-      uint8_t* p_row = smem_gen + FSmem::ps + row_at;
-      uint8_t* ds_row = smem_gen + FSmem::dss + buf * kFImage + row_at;
+      const uint32_t p_row = smem_base + FSmem::ps + row_at;
+      const uint32_t ds_row = smem_base + FSmem::dss + buf * kFImage + row_at;
       uint32_t p_packed[16];
-      // Eight columns of S and dP at a time; the next eight are requested as soon as the current ones have arrived
-      // and travel under the current eight's arithmetic.
-      uint32_t sraw[2][8], draw[2][8];
       bool p_free = s < 1;
-      tmem_ld8(lanes_t + kSCol + wg * 32, sraw[0]);
-      tmem_ld8(lanes_t + kDpCol + wg * 32, draw[0]);
+      // (Two copies of the body: a test per eight columns splits the step into blocks that the compiler cannot interleave.)
+      auto step_body = [&](auto drops_keys) {
+        // Eight columns of S and dP at a time; the next eight are requested as soon as the current ones have arrived
+        // and travel under the current eight's arithmetic.
+        uint32_t sraw[2][8], draw[2][8];
+        tmem_ld8(lanes_t + kSCol + wg * 32, sraw[0]);
+        tmem_ld8(lanes_t + kDpCol + wg * 32, draw[0]);
 #pragma unroll
-      for (int c8 = 0; c8 < 4; ++c8) {
-        tmem_wait_ld();
-        tmem_loaded(sraw[c8 & 1]);
-        tmem_loaded(draw[c8 & 1]);
-        if (c8 == 0 && HAS_BIAS) {
-          // the bias words must have returned before the tile is handed back (the copy of the next tile may land at once)
+        for (int c8 = 0; c8 < 4; ++c8) {
+          tmem_wait_ld();
+          tmem_loaded(sraw[c8 & 1]);
+          tmem_loaded(draw[c8 & 1]);
+          if (c8 == 0 && HAS_BIAS) {
+            // the bias words must have returned before the tile is handed back (the copy of the next tile may land at once)
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
-            asm volatile("" ::"r"(bias_words[c].x), "r"(bias_words[c].y), "r"(bias_words[c].z), "r"(bias_words[c].w) : "memory");
-          mbar_arrive_warp(bar(FSmem::bias_empty));
-        }
-        if (c8 < 3) {
-          tmem_ld8(lanes_t + kSCol + wg * 32 + (c8 + 1) * 8, sraw[(c8 + 1) & 1]);
-          tmem_ld8(lanes_t + kDpCol + wg * 32 + (c8 + 1) * 8, draw[(c8 + 1) & 1]);
-        } else {
-          tc_fence_before_sync();
-          mbar_arrive_warp(bar(FSmem::sd_free));
-          // the P image's phase is probed here; the answer travels under the last eight columns' arithmetic
-          if (s >= 1) p_free = mbar_test(bar(FSmem::p_done), (s - 1) & 1);
-        }
-        f32x2 p2[4], ds2[4];
-        score_grad8_words<T, HAS_BIAS>(sraw[c8 & 1], draw[c8 & 1], bias_words[c8], c2, log2e2, nl1, nd1, p2, ds2);
-        if (bits != 0xffffffffu) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            p2[i] = select2(p2[i], bits, c8 * 8 + 2 * i);
-            ds2[i] = select2(ds2[i], bits, c8 * 8 + 2 * i);
+            for (int c = 0; c < 4; ++c)
+              asm volatile("" ::"r"(bias_words[c].x), "r"(bias_words[c].y), "r"(bias_words[c].z), "r"(bias_words[c].w) : "memory");
+            mbar_arrive_warp(bar(FSmem::bias_empty));
           }
-        }
+          if (c8 < 3) {
+            tmem_ld8(lanes_t + kSCol + wg * 32 + (c8 + 1) * 8, sraw[(c8 + 1) & 1]);
+            tmem_ld8(lanes_t + kDpCol + wg * 32 + (c8 + 1) * 8, draw[(c8 + 1) & 1]);
+          } else {
+            tc_fence_before_sync();
+            mbar_arrive_warp(bar(FSmem::sd_free));
+            // the P image's phase is probed here; the answer travels under the last eight columns' arithmetic
+            if (s >= 1) p_free = mbar_test(bar(FSmem::p_done), (s - 1) & 1);
+          }
+          f32x2 p2[4], ds2[4];
+          score_grad8_words<T, HAS_BIAS>(sraw[c8 & 1], draw[c8 & 1], bias_words[c8], c2, log2e2, nl1, nd1, p2, ds2);
+          if (decltype(drops_keys)::value) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) p_packed[c8 * 4 + i] = pack16<T>(p2[i]);
-        *reinterpret_cast<uint4*>(const_cast<uint8_t*>(swizzled_chunk(ds_row, c8))) =
-            make_uint4(pack16<T>(ds2[0]), pack16<T>(ds2[1]), pack16<T>(ds2[2]), pack16<T>(ds2[3]));
-      }
+            for (int i = 0; i < 4; ++i) {
+              p2[i] = select2(p2[i], bits, c8 * 8 + 2 * i);
+              ds2[i] = select2(ds2[i], bits, c8 * 8 + 2 * i);
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) p_packed[c8 * 4 + i] = pack16<T>(p2[i]);
+          sts_v4_at(ds_row ^ uint32_t(c8 << 4),
+                    make_uint4(pack16<T>(ds2[0]), pack16<T>(ds2[1]), pack16<T>(ds2[2]), pack16<T>(ds2[3])));
+        }
+      };
+      if (bits == 0xffffffffu)
+        step_body(std::false_type{});
+      else
+        step_body(std::true_type{});
       // the single P image is free once the dV products of the previous step have read it; by now they have
       ok = mbar_wait_probed(p_free, bar(FSmem::p_done), (s - 1) & 1, abort_flag);
       if (!ok) break;
 #pragma unroll
       for (int c = 0; c < 4; ++c)
-        *reinterpret_cast<uint4*>(const_cast<uint8_t*>(swizzled_chunk(p_row, c))) =
-            make_uint4(p_packed[4 * c], p_packed[4 * c + 1], p_packed[4 * c + 2], p_packed[4 * c + 3]);
+        sts_v4_at(p_row ^ uint32_t(c << 4),
+                  make_uint4(p_packed[4 * c], p_packed[4 * c + 1], p_packed[4 * c + 2], p_packed[4 * c + 3]));
       if (qi == 0 && s > 0) {
         // A new key tile: dK and dV of the previous one are complete once the products of step s - 1 are (a commit
         // covers every product issued before it); a new group also finds its predecessor's dQ complete.  The products
@@ -1348,13 +1359,12 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
         ok = mbar_wait(bar(FSmem::pds_done + ((s - 1) & 1)), ((s - 1) >> 1) & 1, abort_flag);
         if (!ok) break;
         tc_fence_after_sync();
-        store_key_tile(last_g, last_kt);
-        if (kt == 0) store_query_tiles(last_g);
+        store_key_tile(last_item, last_part, last_kt);
+        if (kt == 0) store_query_tiles(last_item, last_first);
       }
     }
     const int steps = w.s;
     if (ok && steps > 0) {  // the images of the last step
-      fence_proxy_async_smem();
       mbar_arrive_warp(bar(FSmem::pds_full + ((steps - 1) & 1)));
     }
 
@@ -1362,26 +1372,26 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
     if (ok && steps > 0) ok = mbar_wait(bar(FSmem::pds_done + ((steps - 1) & 1)), ((steps - 1) >> 1) & 1, abort_flag);
     if (ok && steps > 0) {
       tc_fence_after_sync();
-      store_key_tile(P.groups - 1, KT - 1);
-      store_query_tiles(P.groups - 1);
+      store_key_tile(last_item, last_part, last_kt);
+      store_query_tiles(last_item, last_first);
     }
-    if (P.groups > 1) {
+    if (GROUPS) {
       // The row's dK and dV now stand complete in this SM's slot (f32, summed group by group in a fixed order by the
       // thread that owns the key).  Every warp passes the barrier, whatever became of its waits; the 16-bit rows are
       // then written by all of them: four lanes share a key, so a warp stores eight 64-byte rows per instruction.
       __threadfence();
       named_barrier_sync(2, 16 * 32);
       if (*abort_flag == 0) {
-        const int items = 2 * P.cols * 4;  // (tensor, key, eight channels)
-        for (int item = tid; item < items; item += 16 * 32) {
-          const int j = item & 3, key = (item >> 2) % P.cols, which = (item >> 2) / P.cols;
+        const int words = 2 * P.cols * 4;  // (tensor, key, eight channels)
+        for (int at = tid; at < words; at += 16 * 32) {
+          const int j = at & 3, key = (at >> 2) % P.cols, which = (at >> 2) / P.cols;
           const bool wanted = which == 0 ? P.write_dk != 0 : P.write_dv != 0;
           if (!wanted) continue;
           const float4* slot = reinterpret_cast<const float4*>(P.slots) + (int64_t(sm_id) * 2 + which) * 8 * P.slot_keys + key;
           const float4 lo = ldcg_f4(slot + (2 * j) * P.slot_keys), hi = ldcg_f4(slot + (2 * j + 1) * P.slot_keys);
           const float f = which == 0 ? scale : 1.f;
           const oops_ta_pair& o = which == 0 ? P.dk : P.dv;
-          T* dst = reinterpret_cast<T*>(o.ptr) + b * o.sb + int64_t(r) * o.sr + int64_t(key) * o.sc + h * o.sh + j * 8;
+          T* dst = item_row(o, int(blockIdx.x)) + int64_t(key) * o.sc + j * 8;
           const uint32_t w0 = Half2<T>::pack(lo.x * f, lo.y * f), w1 = Half2<T>::pack(lo.z * f, lo.w * f);
           const uint32_t w2 = Half2<T>::pack(hi.x * f, hi.y * f), w3 = Half2<T>::pack(hi.z * f, hi.w * f);
           if (pair_vec_ok(o)) {
@@ -1399,6 +1409,58 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
       }
     }
   }
+}
+
+// MASKED: there is a mask or a ragged last key tile.  A mask that keeps everything takes the walk without tests (the
+// tests, and above all what they do to the compiler's schedule, cost 8 %).
+template <typename T, bool HAS_BIAS, bool GROUPS, bool MASKED>
+__global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid_constant__ FParams P) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + FSmem::abort_flag);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + FSmem::tmem_slot);
+  auto bar = [&](int index) -> uint32_t { return smem_base + FSmem::bars + index * 8; };
+
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  if (device_failed()) return;
+  if (tid == 0) {
+    *abort_flag = 0;
+    for (int i = 0; i < 3; ++i) {
+      mbar_init(bar(FSmem::qd_full + i), 1);
+      mbar_init(bar(FSmem::qd_empty + i), 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar(FSmem::pds_full + i), 16);
+      mbar_init(bar(FSmem::pds_done + i), 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar(FSmem::kv_full + i), 1);
+      mbar_init(bar(FSmem::kv_empty + i), 1);
+    }
+    mbar_init(bar(FSmem::p_done), 1);
+    mbar_init(bar(FSmem::bias_full), 1);
+    mbar_init(bar(FSmem::bias_empty), 16);
+    mbar_init(bar(FSmem::sd_full), 1);
+    mbar_init(bar(FSmem::sd_free), 16);
+    mbar_init(bar(FSmem::dkv_free), 8);
+    mbar_init(bar(FSmem::dq_free), 16);
+    fence_barrier_init();
+  }
+  if (warp == kFScoreWarp) {
+    tmem_alloc(smem_base + FSmem::tmem_slot, 512);
+    tmem_relinquish();
+    tc_fence_before_sync();
+  }
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  bool plain = !MASKED;
+  if (MASKED && P.mask && P.cols % kTile == 0) plain = keeps_all(P.live, P.batch * P.rows, lane);
+  if (plain)
+    fused_walk<T, HAS_BIAS, GROUPS, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane);
+  else if (MASKED)
+    fused_walk<T, HAS_BIAS, GROUPS, true>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane);
   teardown(abort_flag, tmem_base, kFScoreWarp);
 }
 
@@ -1418,6 +1480,7 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
 // fixed order (no atomics, bitwise reproducible either way).
 
 constexpr int kDbRing = 4;
+constexpr int kDbListRows = 8192;       // longest part whose rows without a kept key are passed over
 constexpr int kDbStage = 4 * kBigTile;  // Q | dO | K | V of one row: 128 x 32 each
 #ifndef TA_DB_POLY_EVERY
 #define TA_DB_POLY_EVERY 0
@@ -1435,7 +1498,9 @@ struct DbSmem {
   static constexpr int num_bars = sd_free + 2;
   static constexpr int tmem_slot = bars + num_bars * 8;
   static constexpr int abort_flag = tmem_slot + 4;
-  static constexpr int total = abort_flag + 4;
+  static constexpr int row_count = abort_flag + 4;
+  static constexpr int row_list = (row_count + 4 + 15) / 16 * 16;  // [kDbListRows] u16: rows of the part with a kept key in the tile
+  static constexpr int total = row_list + kDbListRows * 2;
 };
 constexpr int kDbSmemBytes = DbSmem::total + 1024;
 static_assert(kDbSmemBytes <= 232448, "shared-bias kernel: shared memory over the per-CTA limit");
@@ -1449,58 +1514,24 @@ struct DbParams {
   const float* lse;
   const float* delta;
   const uint8_t* mask;
+  const uint32_t* live;  // [batch][rows] key tiles with a kept key (with a mask and at most 32 key tiles)
   int64_t m_sb, m_sr, m_sc;
   int batch, rows, cols, heads;
   int tiles, num_parts, rows_per_part;
   float scale;
 };
 
-template <typename T>
-__global__ void __launch_bounds__(kDbThreads, 1) ta_bwd_dbias_kernel(const __grid_constant__ DbParams P) {
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + DbSmem::abort_flag);
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + DbSmem::tmem_slot);
+// BITS: some key may be dropped.  LISTED: the rows that keep no key of the tile add nothing, and every role walks the others
+// through a list.
+template <typename T, bool BITS, bool LISTED>
+__device__ __forceinline__ void dbias_walk(const DbParams& P, uint32_t smem_base, uint8_t* smem_gen, volatile int* abort_flag,
+                                           uint32_t tmem_base, int tid, int warp, int lane, int b, int h, int qt, int kt, int part,
+                                           int row_lo, int part_rows) {
   auto bar = [&](int index) -> uint32_t { return smem_base + DbSmem::bars + index * 8; };
-
-  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-  if (device_failed()) return;
-  int idx = blockIdx.x;
-  const int kt = idx % P.tiles;
-  idx /= P.tiles;
-  const int qt = idx % P.tiles;
-  idx /= P.tiles;
-  const int h = idx % P.heads;
-  idx /= P.heads;
-  const int b = idx % P.batch;
-  const int part = idx / P.batch;
-  const int row_lo = part * P.rows_per_part;
-  const int row_hi = min(P.rows, row_lo + P.rows_per_part);
-  const int n_rows = max(0, row_hi - row_lo);
-  const bool has_mask = P.mask != nullptr;
-
-  if (tid == 0) {
-    *abort_flag = 0;
-    mbar_init(bar(DbSmem::bias_full), 1);
-    for (int i = 0; i < kDbRing; ++i) {
-      mbar_init(bar(DbSmem::row_full + i), 1);
-      mbar_init(bar(DbSmem::row_empty + i), 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(DbSmem::sd_full + i), 1);
-      mbar_init(bar(DbSmem::sd_free + i), kDbElemWarps);
-    }
-    fence_barrier_init();
-  }
-  if (warp == kDbMmaWarp) {
-    tmem_alloc(smem_base + DbSmem::tmem_slot, 512);
-    tmem_relinquish();
-    tc_fence_before_sync();
-  }
-  __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const bool has_mask = BITS && P.mask != nullptr;
+  const uint16_t* row_list = reinterpret_cast<const uint16_t*>(smem_gen + DbSmem::row_list);
+  const int n_rows = LISTED ? *reinterpret_cast<volatile int*>(smem_gen + DbSmem::row_count) : part_rows;
+  auto part_row = [&](int i) -> int { return LISTED ? int(row_list[i]) : i; };  // i-th row walked, counted within the part
 
   if (warp == kDbProducerWarp) {
     if (lane == 0) {
@@ -1510,7 +1541,7 @@ __global__ void __launch_bounds__(kDbThreads, 1) ta_bwd_dbias_kernel(const __gri
         tma_load_5d(smem_base + DbSmem::bias + box * kBiasStep, &P.map_bias, bar(DbSmem::bias_full), kt * kTile + box * 64,
                     qt * kTile, h, 0, b);
       for (int i = 0; i < n_rows && ok; ++i) {
-        const int st = i % kDbRing, round = i / kDbRing, r = row_lo + i;
+        const int st = i % kDbRing, round = i / kDbRing, r = row_lo + part_row(i);
         if (i >= kDbRing) ok = mbar_wait(bar(DbSmem::row_empty + st), (round - 1) & 1, abort_flag);
         if (!ok) break;
         mbar_expect_tx(bar(DbSmem::row_full + st), kDbStage);
@@ -1579,20 +1610,20 @@ __global__ void __launch_bounds__(kDbThreads, 1) ta_bwd_dbias_kernel(const __gri
 #pragma unroll
     for (int i = 0; i < 16; ++i) acc2[i] = pack2(0.f, 0.f);
 
-    const bool need_bits = has_mask || key_base + 32 > P.cols;
+    const bool need_bits = BITS && (has_mask || key_base + 32 > P.cols);
     const int64_t stat_stride = int64_t(P.heads) * P.cols;
     const int64_t stat_first = ((int64_t(b) * P.rows + row_lo) * P.heads + h) * P.cols + q_index;
     // Prefetch of the next row's statistics and mask byte: the loaded words stay untouched until that row's turn
     // (any arithmetic on them here would wait for the load).
     auto load_stats = [&](int i, float& lse_raw, float& delta_raw, uint32_t& keep_raw) {
-      const int r = row_lo + i;
       lse_raw = INFINITY;
       delta_raw = 0.f;
       keep_raw = 0;
       if (i < n_rows) {
+        const int at = part_row(i), r = row_lo + at;
         if (q_valid) {
-          lse_raw = ldg_f32_here(P.lse + stat_first + int64_t(i) * stat_stride);
-          delta_raw = ldg_f32_here(P.delta + stat_first + int64_t(i) * stat_stride);
+          lse_raw = ldg_f32_here(P.lse + stat_first + int64_t(at) * stat_stride);
+          delta_raw = ldg_f32_here(P.delta + stat_first + int64_t(at) * stat_stride);
         }
         const int key = key_base + lane;
         if (key < P.cols) {
@@ -1679,7 +1710,7 @@ __global__ void __launch_bounds__(kDbThreads, 1) ta_bwd_dbias_kernel(const __gri
           work4(quad + 1, s_b, d_b);
         }
       };
-      if (bits == 0xffffffffu)
+      if (!BITS || bits == 0xffffffffu)
         row_body(std::false_type{});
       else
         row_body(std::true_type{});
@@ -1743,6 +1774,77 @@ __global__ void __launch_bounds__(kDbThreads, 1) ta_bwd_dbias_kernel(const __gri
       }
     }
   }
+}
+
+enum DbRows { kDbAllKept, kDbTested, kDbMasked };  // no dropped key; keys tested, no list; mask with a list
+
+// A mask that keeps everything takes the walk without tests and without a list (looking at them costs 5 to 8 %).
+template <typename T, int ROWS>
+__global__ void __launch_bounds__(kDbThreads, 1) ta_bwd_dbias_kernel(const __grid_constant__ DbParams P) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + DbSmem::abort_flag);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + DbSmem::tmem_slot);
+  auto bar = [&](int index) -> uint32_t { return smem_base + DbSmem::bars + index * 8; };
+
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  if (device_failed()) return;
+  int idx = blockIdx.x;
+  const int kt = idx % P.tiles;
+  idx /= P.tiles;
+  const int qt = idx % P.tiles;
+  idx /= P.tiles;
+  const int h = idx % P.heads;
+  idx /= P.heads;
+  const int b = idx % P.batch;
+  const int part = idx / P.batch;
+  const int row_lo = part * P.rows_per_part;
+  const int row_hi = min(P.rows, row_lo + P.rows_per_part);
+  const int part_rows = max(0, row_hi - row_lo);
+  uint16_t* row_list = reinterpret_cast<uint16_t*>(smem_gen + DbSmem::row_list);
+  volatile int* row_count = reinterpret_cast<volatile int*>(smem_gen + DbSmem::row_count);
+  bool plain = ROWS == kDbAllKept;
+  if (ROWS == kDbMasked && P.cols % kTile == 0) plain = keeps_all(P.live, P.batch * P.rows, lane);
+  if (ROWS == kDbMasked && !plain && warp == 0) {
+    int count = 0;
+#pragma unroll 4
+    for (int first = 0; first < part_rows; first += 32) {
+      const int i = first + lane;
+      const bool is_live = i < part_rows && ((__ldg(P.live + int64_t(b) * P.rows + row_lo + i) >> kt) & 1u) != 0;
+      const uint32_t bits = __ballot_sync(0xffffffffu, is_live);
+      if (is_live) row_list[count + __popc(bits & ((1u << lane) - 1))] = uint16_t(i);
+      count += __popc(bits);
+    }
+    if (lane == 0) *row_count = count;
+  }
+
+  if (tid == 0) {
+    *abort_flag = 0;
+    mbar_init(bar(DbSmem::bias_full), 1);
+    for (int i = 0; i < kDbRing; ++i) {
+      mbar_init(bar(DbSmem::row_full + i), 1);
+      mbar_init(bar(DbSmem::row_empty + i), 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar(DbSmem::sd_full + i), 1);
+      mbar_init(bar(DbSmem::sd_free + i), kDbElemWarps);
+    }
+    fence_barrier_init();
+  }
+  if (warp == kDbMmaWarp) {
+    tmem_alloc(smem_base + DbSmem::tmem_slot, 512);
+    tmem_relinquish();
+    tc_fence_before_sync();
+  }
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  if (ROWS != kDbTested && plain)
+    dbias_walk<T, false, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, b, h, qt, kt, part, row_lo, part_rows);
+  else if (ROWS != kDbAllKept)
+    dbias_walk<T, true, ROWS == kDbMasked>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, b, h, qt, kt, part, row_lo,
+                                           part_rows);
   teardown(abort_flag, tmem_base, kDbMmaWarp, 512);
 }
 
@@ -1785,16 +1887,16 @@ uint64_t fused_slot_bytes(const oops_ta_problem& p) {
 }
 
 // The single-pass kernel serves calls that want dQ together with dK or dV and no per-row bias gradient, on rows
-// whose keep-bit table fits its shared memory (4096 columns).
+// of up to 4096 columns (32 key tiles, one bit each in the words that describe a row's mask).
 bool fused_applies(const oops_ta_problem& p, const oops_ta_grads& g) {
   if ((p.flags & OOPS_TA_FLAG_SPLIT_REVERSE) != 0) return false;
   if (g.dbias && p.bias_groups > 1) return false;
-  if (ceil_div(p.cols, 32) > kFKeepWords) return false;
+  if (p.cols > kFMaxCols) return false;
   return g.dq.ptr != nullptr && (g.dk.ptr != nullptr || g.dv.ptr != nullptr);
 }
 
 struct Layout {
-  uint64_t delta, bias_t, pair_parts, parts, total;
+  uint64_t delta, live, bias_t, pair_parts, parts, total;
 };
 
 Layout workspace_layout(const oops_ta_problem& p, const oops_ta_grads& g) {
@@ -1802,6 +1904,8 @@ Layout workspace_layout(const oops_ta_problem& p, const oops_ta_grads& g) {
   uint64_t at = 0;
   l.delta = at;
   at += align256(uint64_t(p.batch) * p.rows * p.heads * p.cols * sizeof(float));
+  l.live = at;
+  if (p.mask) at += align256(uint64_t(p.batch) * p.rows * sizeof(uint32_t) * 2);
   l.bias_t = at;
   const bool fused = fused_applies(p, g);
   if (p.bias_groups != 0 && (g.dk.ptr || g.dv.ptr) && !fused)
@@ -1842,12 +1946,20 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
   const bool shared_bias_grad = g.dbias && p.bias_groups == 1;
   int status;
 
+  // Key tiles with a kept key, one bit each: rows of more than 32 tiles (which the single-pass kernel does not take) go
+  // without, as do calls without a mask.
+  uint32_t* live = p.mask && ceil_div(p.cols, kTile) <= 32 ? reinterpret_cast<uint32_t*>(base + layout.live) : nullptr;
+
   if ((p.flags & OOPS_TA_FLAG_REUSE_DELTA) == 0) {  // delta = rowsum(O * dO)
     const int64_t total = int64_t(p.batch) * p.rows * p.heads * p.cols;
     const int vec_ok = (reinterpret_cast<uintptr_t>(out.ptr) & 15) == 0 && (reinterpret_cast<uintptr_t>(dout.ptr) & 15) == 0 &&
                        out.sb % 8 == 0 && out.sr % 8 == 0 && out.sc % 8 == 0 && out.sh % 8 == 0 && dout.sb % 8 == 0 &&
                        dout.sr % 8 == 0 && dout.sc % 8 == 0 && dout.sh % 8 == 0;
-    delta_kernel<T><<<(unsigned)ceil_div(total, 256), 256, 0, stream>>>(out, dout, delta, total, p.cols, p.heads, p.rows, vec_ok);
+    const unsigned delta_blocks = (unsigned)ceil_div(total, 64);
+    const unsigned mask_blocks = live ? (unsigned)ceil_div(int64_t(p.batch) * p.rows, 8) : 0u;
+    prepare_kernel<T><<<delta_blocks + mask_blocks, 256, 0, stream>>>(out, dout, delta, (uint32_t)total, p.cols, p.heads, p.rows, vec_ok,
+                                                                      dout.sr < dout.sc, delta_blocks, p.mask, p.mask_sb, p.mask_sr,
+                                                                      p.mask_sc, live, p.batch * p.rows);
     count_launch();
     status = check_launch("tcgen05 delta");
     if (status) return status;
@@ -1880,6 +1992,8 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
     P.cols = p.cols;
     P.heads = p.heads;
     P.bias_groups = p.bias_groups;
+    P.live = live;
+    P.items = p.batch * p.rows * p.heads;
     P.q_tiles = (int)ceil_div(p.cols, kTile);
     P.k_tiles = P.q_tiles;
     P.groups = fused_groups(p);
@@ -1889,7 +2003,10 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
       P.slots = reinterpret_cast<float*>(base + layout.pair_parts);
       P.slot_keys = fused_slot_keys(p);
     }
-    const unsigned grid = (unsigned)(int64_t(p.batch) * p.rows * p.heads);
+    // A CTA works through several items where a row is one group of query tiles: the copies and score products of the next
+    // item run under the last steps and the read-out of this one (N = 256: 84 -> 68 us).  Rows of several groups keep a CTA
+    // to themselves, which sums their dK and dV in its SM's slot.
+    const unsigned grid = (unsigned)(P.groups > 1 ? P.items : std::min(P.items, sm_count()));
     auto go = [&](auto kernel) -> int {
       const int rc = reserve_smem(kernel, kFSmemBytes);
       if (rc) return rc;
@@ -1897,7 +2014,14 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
       count_launch();
       return check_launch("tcgen05 dQ/dK/dV");
     };
-    status = has_bias ? go(ta_bwd_fused_kernel<T, true>) : go(ta_bwd_fused_kernel<T, false>);
+    const bool has_bits = p.mask || p.cols % kTile != 0;
+    auto pick = [&](auto bias, auto groups) {
+      return has_bits ? go(ta_bwd_fused_kernel<T, decltype(bias)::value, decltype(groups)::value, true>)
+                      : go(ta_bwd_fused_kernel<T, decltype(bias)::value, decltype(groups)::value, false>);
+    };
+    using Yes = std::true_type;
+    using No = std::false_type;
+    status = P.groups > 1 ? (has_bias ? pick(Yes{}, Yes{}) : pick(No{}, Yes{})) : (has_bias ? pick(Yes{}, No{}) : pick(No{}, No{}));
     if (status) return status;
   }
 
@@ -2014,9 +2138,12 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
     P.heads = p.heads;
     P.tiles = (int)ceil_div(p.cols, kTile);
     P.rows_per_part = (int)ceil_div(p.rows, P.num_parts);
+    P.live = live;
     P.scale = p.scale;
     const unsigned grid = (unsigned)(int64_t(P.num_parts) * p.batch * p.heads * P.tiles * P.tiles);
-    auto kernel = ta_bwd_dbias_kernel<T>;
+    auto kernel = !p.mask && p.cols % kTile == 0                ? ta_bwd_dbias_kernel<T, kDbAllKept>
+                  : live && P.rows_per_part <= kDbListRows ? ta_bwd_dbias_kernel<T, kDbMasked>
+                                                           : ta_bwd_dbias_kernel<T, kDbTested>;
     status = reserve_smem(kernel, kDbSmemBytes);
     if (status) return status;
     kernel<<<grid, kDbThreads, kDbSmemBytes, stream>>>(P);
@@ -2044,7 +2171,7 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
 bool tensor_backward_applies(const oops_ta_problem& p, const oops_ta_grads* g) {
   if (!tensor_forward_applies(p)) return false;
   const int64_t rows = int64_t(p.batch) * p.rows * p.heads * p.cols;
-  if (rows > 0x7fffffffll * 64) return false;
+  if (rows > 0x7fffffffll) return false;  // (cell, head) pairs are counted in 32 bits
   (void)g;
   return true;
 }

@@ -4,6 +4,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "sm100_ptx.cuh"
@@ -117,6 +118,19 @@ int encode_bias(CUtensorMap* map, const oops_ta_problem& p, const void* ptr, int
   const int64_t strides[4] = {s_outer, sh, sg, sb};
   const uint32_t box[5] = {64, box_outer, 1, 1, 1};
   return encode_map(map, p.dtype, ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, what);
+}
+
+int sm_count() {
+  constexpr int kMaxDevices = 64;
+  static std::atomic<int> counts[kMaxDevices];
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices) return 148;
+  int count = counts[device].load(std::memory_order_relaxed);
+  if (count == 0) {
+    if (cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || count <= 0) count = 148;
+    counts[device].store(count, std::memory_order_relaxed);
+  }
+  return count;
 }
 
 template <typename Kernel>
