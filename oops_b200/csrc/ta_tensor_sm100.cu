@@ -7,13 +7,15 @@
 // issues tcgen05.mma for S = Q K^T (accumulator in tensor memory) and O += P V (P read back from tensor memory,
 // V from shared memory); one softmax warpgroup per tile (a thread owns a query) turns S into P.
 //
-// The softmax has no row maximum in its steady state.  The maximum of a row's first step (with a kept key) is its
-// reference; later steps take 2^(x - reference) as they come, 16 columns at a time, and look at the step's sum only: a
+// The softmax has no row maximum in its steady state.  The maximum of the first 16 columns (that keep a key) of a
+// row's first step is its reference; later steps take 2^(x - reference) as they come, 16 columns at a time, and look at the step's sum only: a
 // sum of 2^10 or more (or a NaN) sends the warp back over the step, which still stands in tensor memory, to raise the
 // reference and rescale the accumulators.  Probabilities therefore stay below 2^10, inside the f32, bf16 and f16 ranges.
 // Against a maximum per step this saves the comparisons, and above all the wait: no exponential depended on the last
 // score of a step any more, scores need not be held in registers, and an exponential costs 5 instead of 9.5 issue slots.
-// What bounds it: the special-function unit, one ex2 per score at 16 per clock and SM.
+// What bounds it: issue slots and, close behind, the special-function unit, one ex2 per score at 16 per clock and SM (0.40 of
+// the 0.70 ms at N = 768).  Hence two copies of the roles: a CTA whose rows keep every key walks without tests on kept bits
+// (N = 768: 757 -> 703 us, N = 2048: 12.4 -> 11.7 ms).
 #include <type_traits>
 
 #include "ta_tensor_common.cuh"
@@ -22,7 +24,6 @@ namespace oops_ta {
 namespace {
 
 using namespace ptx;
-
 
 constexpr int kStages = 3;                       // K/V ring depth
 constexpr int kKeys = 64;                        // keys per step
@@ -89,113 +90,22 @@ struct FwdParams {
 
 constexpr float kStepSumLimit = 1024.f;  // a step's sum of probabilities that sends its warp back for a new reference
 
-template <typename T, bool HAS_BIAS, bool GATED, bool ROWS>
-__global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_constant__ FwdParams P) {
+// What the CTA's roles do once its set-up stands.  BITS: some key may be dropped, by the mask or because the last key step is
+// ragged.
+template <typename T, bool HAS_BIAS, bool GATED, bool ROWS, bool BITS>
+__device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base, uint8_t* smem_gen, volatile int* abort_flag,
+                                         uint32_t tmem_base, int tid, int warp, int lane, int h, int r0, int b, int q0, int n_tiles) {
   using Smem = FwdSmem<ROWS>;
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + Smem::abort_flag);
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + Smem::tmem_slot);
-  uint32_t* keep_words = reinterpret_cast<uint32_t*>(smem_gen + Smem::keep);
-  volatile int* step_count = reinterpret_cast<volatile int*>(smem_gen + Smem::step_count);
-  uint16_t* step_list = reinterpret_cast<uint16_t*>(smem_gen + Smem::steps);
+  const uint32_t* keep_words = reinterpret_cast<const uint32_t*>(smem_gen + Smem::keep);
+  const uint16_t* step_list = reinterpret_cast<const uint16_t*>(smem_gen + Smem::steps);
+  const uint32_t* drop_flags = reinterpret_cast<const uint32_t*>(smem_gen + Smem::drop_flags);
   auto bar = [&](int index) -> uint32_t { return smem_base + Smem::bars + index * 8; };
-
-  const int tid = threadIdx.x;
-  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-  const int lane = tid & 31;
-  if (device_failed()) return;
-
-  // work decomposition: query item fastest, then head, row (or pair of rows), batch
-  int idx = blockIdx.x;
-  const int qi = idx % P.q_items;
-  idx /= P.q_items;
-  const int h = idx % P.heads;
-  idx /= P.heads;
-  const int row_items = ROWS ? (P.rows + 1) / 2 : P.rows;
-  const int r0 = (idx % row_items) * (ROWS ? 2 : 1);
-  const int b = idx / row_items;
-  const int q0 = qi * (ROWS ? kTile : 2 * kTile);
-  const int n_tiles = (ROWS ? r0 + 1 < P.rows : q0 + kTile < P.cols) ? 2 : 1;
   const int n_rings = ROWS ? n_tiles : 1;
   const int g = P.bias_groups == 1 ? 0 : r0;
-  const bool has_mask = P.mask != nullptr;
-  // Steps need keep-bits when there is a mask or when the last key step is ragged.
-  const bool has_bits = has_mask || (P.cols % kKeys) != 0;
+  const bool has_mask = BITS && P.mask != nullptr;
   auto row_of = [&](int w) { return ROWS ? r0 + w : r0; };
   auto first_query = [&](int w) { return ROWS ? q0 : q0 + w * kTile; };
-
-  if (tid == 0) {
-    *abort_flag = 0;
-    for (int i = 0; i < 2; ++i) mbar_init(bar(Smem::q_full + i), 1);
-    for (int i = 0; i < Smem::kv_rings * kStages; ++i) {
-      mbar_init(bar(Smem::k_full + i), 1);
-      mbar_init(bar(Smem::k_empty + i), ROWS ? 1 : n_tiles);
-      mbar_init(bar(Smem::v_full + i), 1);
-      mbar_init(bar(Smem::v_empty + i), ROWS ? 1 : n_tiles);
-      mbar_init(bar(Smem::v_ready + i), kTile / 32);
-    }
-    for (int i = 0; i < Smem::bias_rings * 2; ++i) {
-      mbar_init(bar(Smem::bias_full + i), 1);
-      mbar_init(bar(Smem::bias_empty + i), ROWS ? n_tiles * (kTile / 32) : kTile / 32);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(Smem::s_full + i), 1);
-      mbar_init(bar(Smem::p_full + i), kTile / 32);
-      mbar_init(bar(Smem::pv_done + i), 1);
-    }
-    fence_barrier_init();
-  }
-  if (warp == 9) {
-    tmem_alloc(smem_base + Smem::tmem_slot, kFwdTmemCols);
-    tmem_relinquish();
-    tc_fence_before_sync();
-  }
-  uint32_t* drop_flags = reinterpret_cast<uint32_t*>(smem_gen + Smem::drop_flags);
-  if (has_bits && warp < 8) {
-    // one bit per key of the pair row: kept by the mask and inside the row (warps 0-3: first row, 4-7: second row; one
-    // row: all warps)
-    const int ring = ROWS ? warp >> 2 : 0;
-    bool dropped_any = false;
-    if (ring < n_rings) {
-      const uint8_t* mask_row = has_mask ? P.mask + b * P.m_sb + int64_t(row_of(ring)) * P.m_sr : nullptr;
-      for (int word = ROWS ? warp & 3 : warp; word < P.k_steps * 2; word += ROWS ? 4 : 8) {
-        const int key = word * 32 + lane;
-        bool keep = key < P.cols;
-        if (keep && has_mask) {
-          keep = mask_row[int64_t(key) * P.m_sc] != 0;
-          dropped_any |= !keep;
-        }
-        const uint32_t bits = __ballot_sync(0xffffffffu, keep);
-        if (lane == 0) keep_words[ring * kMaxKeepWords + word] = bits;
-      }
-    }
-    dropped_any = __any_sync(0xffffffffu, dropped_any);
-    if (lane == 0) drop_flags[warp] = dropped_any ? 1u : 0u;
-  }
-  __syncthreads();
-  if (has_mask) {
-    // The steps in which some row of the CTA keeps a key, in order: padding is neither loaded nor computed.
-    if (warp == 0) {
-      int count = 0;
-      for (int first = 0; first < P.k_steps; first += 32) {
-        const int j = first + lane;
-        uint32_t any = 0;
-        if (j < P.k_steps)
-          for (int ring = 0; ring < n_rings; ++ring)
-            any |= keep_words[ring * kMaxKeepWords + 2 * j] | keep_words[ring * kMaxKeepWords + 2 * j + 1];
-        const uint32_t live = __ballot_sync(0xffffffffu, any != 0);
-        if (any != 0) step_list[count + __popc(live & ((1u << lane) - 1))] = uint16_t(j);
-        count += __popc(live);
-      }
-      if (lane == 0) *step_count = count;
-    }
-    __syncthreads();
-  }
-  tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
-  const int KS = has_mask ? *step_count : P.k_steps;
+  const int KS = has_mask ? *reinterpret_cast<volatile int*>(smem_gen + Smem::step_count) : P.k_steps;
   auto step_at = [&](int i) { return has_mask ? int(step_list[i]) : i; };
   // Value rows only need the sign-off handshake when the mask really drops a key of the row.
   auto needs_signoff = [&](int w) {
@@ -314,7 +224,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
 
     for (int i = 0; i < KS && ok; ++i) {
       uint2 bits = make_uint2(0xffffffffu, 0xffffffffu);  // keys 0-31 and 32-63 of the step
-      if (has_bits) bits = *reinterpret_cast<const uint2*>(keep_words + ring * kMaxKeepWords + step_at(i) * 2);
+      if (BITS) bits = *reinterpret_cast<const uint2*>(keep_words + ring * kMaxKeepWords + step_at(i) * 2);
       const bool all_kept = (bits.x & bits.y) == 0xffffffffu;
       if (signs_off) {
         // Values of dropped keys must not reach the tensor core (0 * inf): clear their rows in shared memory.
@@ -360,8 +270,8 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
           }
         }
       };
-      // The largest base-2 logit of the step.
-      auto step_peak = [&]() -> float {
+      // The largest base-2 logit of the step; for a first reference, of as many of its columns as give every row one.
+      auto step_peak = [&](bool first) -> float {
         float peak = -INFINITY;
 #pragma unroll 1
         for (int chunk = 0; chunk < 4; ++chunk) {
@@ -382,13 +292,14 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
             unpack2(x[n], lo, hi);
             peak = max3(peak, lo, hi);
           }
+          if (first && !__any_sync(0xffffffffu, peak == -INFINITY)) break;
         }
         return peak;
       };
       // Raises the reference of the rows whose step needs it, and rescales what they have summed so far.
-      auto raise = [&](bool wanted) -> bool {
+      auto raise = [&](bool wanted, int attempt) -> bool {
         tmem_wait_st();  // probabilities of a pass that is about to be repeated
-        const float peak = step_peak();
+        const float peak = step_peak(attempt == 0);
         const bool raised = wanted && peak > ref;
         const float alpha = raised ? ex2(ref - peak) : 1.f;  // 0 for a row without a reference so far
         if (raised) {
@@ -460,10 +371,10 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
       bool wanted = ref == -INFINITY;
 #pragma unroll 1
       for (int attempt = 0; attempt < 2 && ok; ++attempt) {
-        if (__any_sync(0xffffffffu, wanted)) ok = raise(wanted);
+        if (__any_sync(0xffffffffu, wanted)) ok = raise(wanted, attempt);
         else if (attempt > 0) break;
         if (!ok) break;
-        sum = all_kept ? step_pass(std::false_type{}) : step_pass(std::true_type{});
+        sum = !BITS || all_kept ? step_pass(std::false_type{}) : step_pass(std::true_type{});
         wanted = !(sum < kStepSumLimit);
       }
       if (!ok) break;
@@ -547,6 +458,122 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
       }
     }
   }
+}
+
+template <typename T, bool HAS_BIAS, bool GATED, bool ROWS>
+__global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_constant__ FwdParams P) {
+  using Smem = FwdSmem<ROWS>;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + Smem::abort_flag);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + Smem::tmem_slot);
+  uint32_t* keep_words = reinterpret_cast<uint32_t*>(smem_gen + Smem::keep);
+  volatile int* step_count = reinterpret_cast<volatile int*>(smem_gen + Smem::step_count);
+  uint16_t* step_list = reinterpret_cast<uint16_t*>(smem_gen + Smem::steps);
+  auto bar = [&](int index) -> uint32_t { return smem_base + Smem::bars + index * 8; };
+
+  const int tid = threadIdx.x;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int lane = tid & 31;
+  if (device_failed()) return;
+
+  // work decomposition: query item fastest, then head, row (or pair of rows), batch
+  int idx = blockIdx.x;
+  const int qi = idx % P.q_items;
+  idx /= P.q_items;
+  const int h = idx % P.heads;
+  idx /= P.heads;
+  const int row_items = ROWS ? (P.rows + 1) / 2 : P.rows;
+  const int r0 = (idx % row_items) * (ROWS ? 2 : 1);
+  const int b = idx / row_items;
+  const int q0 = qi * (ROWS ? kTile : 2 * kTile);
+  const int n_tiles = (ROWS ? r0 + 1 < P.rows : q0 + kTile < P.cols) ? 2 : 1;
+  const int n_rings = ROWS ? n_tiles : 1;
+  const bool has_mask = P.mask != nullptr;
+  // Steps need keep-bits when there is a mask or when the last key step is ragged.
+  const bool has_bits = has_mask || (P.cols % kKeys) != 0;
+  auto row_of = [&](int w) { return ROWS ? r0 + w : r0; };
+
+  if (tid == 0) {
+    *abort_flag = 0;
+    for (int i = 0; i < 2; ++i) mbar_init(bar(Smem::q_full + i), 1);
+    for (int i = 0; i < Smem::kv_rings * kStages; ++i) {
+      mbar_init(bar(Smem::k_full + i), 1);
+      mbar_init(bar(Smem::k_empty + i), ROWS ? 1 : n_tiles);
+      mbar_init(bar(Smem::v_full + i), 1);
+      mbar_init(bar(Smem::v_empty + i), ROWS ? 1 : n_tiles);
+      mbar_init(bar(Smem::v_ready + i), kTile / 32);
+    }
+    for (int i = 0; i < Smem::bias_rings * 2; ++i) {
+      mbar_init(bar(Smem::bias_full + i), 1);
+      mbar_init(bar(Smem::bias_empty + i), ROWS ? n_tiles * (kTile / 32) : kTile / 32);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar(Smem::s_full + i), 1);
+      mbar_init(bar(Smem::p_full + i), kTile / 32);
+      mbar_init(bar(Smem::pv_done + i), 1);
+    }
+    fence_barrier_init();
+  }
+  if (warp == 9) {
+    tmem_alloc(smem_base + Smem::tmem_slot, kFwdTmemCols);
+    tmem_relinquish();
+    tc_fence_before_sync();
+  }
+  uint32_t* drop_flags = reinterpret_cast<uint32_t*>(smem_gen + Smem::drop_flags);
+  if (has_bits && warp < 8) {
+    // one bit per key of the pair row: kept by the mask and inside the row (warps 0-3: first row, 4-7: second row; one
+    // row: all warps)
+    const int ring = ROWS ? warp >> 2 : 0;
+    bool dropped_any = false;
+    if (ring < n_rings) {
+      const uint8_t* mask_row = has_mask ? P.mask + b * P.m_sb + int64_t(row_of(ring)) * P.m_sr : nullptr;
+      for (int word = ROWS ? warp & 3 : warp; word < P.k_steps * 2; word += ROWS ? 4 : 8) {
+        const int key = word * 32 + lane;
+        bool keep = key < P.cols;
+        if (keep && has_mask) {
+          keep = mask_row[int64_t(key) * P.m_sc] != 0;
+          dropped_any |= !keep;
+        }
+        const uint32_t bits = __ballot_sync(0xffffffffu, keep);
+        if (lane == 0) keep_words[ring * kMaxKeepWords + word] = bits;
+      }
+    }
+    dropped_any = __any_sync(0xffffffffu, dropped_any);
+    if (lane == 0) drop_flags[warp] = dropped_any ? 1u : 0u;
+  }
+  __syncthreads();
+  // Rows of which every key is kept take the walk without tests.
+  bool plain = P.cols % kKeys == 0;
+  if (has_mask) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) plain &= drop_flags[i] == 0;
+  }
+  if (has_mask && !plain) {
+    // The steps in which some row of the CTA keeps a key, in order: padding is neither loaded nor computed.
+    if (warp == 0) {
+      int count = 0;
+      for (int first = 0; first < P.k_steps; first += 32) {
+        const int j = first + lane;
+        uint32_t any = 0;
+        if (j < P.k_steps)
+          for (int ring = 0; ring < n_rings; ++ring)
+            any |= keep_words[ring * kMaxKeepWords + 2 * j] | keep_words[ring * kMaxKeepWords + 2 * j + 1];
+        const uint32_t live = __ballot_sync(0xffffffffu, any != 0);
+        if (any != 0) step_list[count + __popc(live & ((1u << lane) - 1))] = uint16_t(j);
+        count += __popc(live);
+      }
+      if (lane == 0) *step_count = count;
+    }
+    __syncthreads();
+  }
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  if (plain)
+    fwd_walk<T, HAS_BIAS, GATED, ROWS, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, h, r0, b, q0, n_tiles);
+  else
+    fwd_walk<T, HAS_BIAS, GATED, ROWS, true>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, h, r0, b, q0, n_tiles);
   teardown(abort_flag, tmem_base, 9, kFwdTmemCols);
 }
 
