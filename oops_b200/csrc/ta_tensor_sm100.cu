@@ -14,8 +14,9 @@
 // Against a maximum per step this saves the comparisons, and above all the wait: no exponential depended on the last
 // score of a step any more, scores need not be held in registers, and an exponential costs 5 instead of 9.5 issue slots.
 // What bounds it: issue slots and, close behind, the special-function unit, one ex2 per score at 16 per clock and SM (0.40 of
-// the 0.70 ms at N = 768).  Hence two copies of the roles: a CTA whose rows keep every key walks without tests on kept bits
-// (N = 768: 757 -> 703 us, N = 2048: 12.4 -> 11.7 ms).
+// the 0.70 ms at N = 768).  Hence no tests on kept bits where nothing is dropped: a CTA whose rows keep every key walks a copy
+// of the roles without them (N = 768: 757 -> 703 us), and otherwise the steps that every row keeps whole come first, in a
+// loop of their own (the order of the keys is free; N = 1024, 1000 kept: 1659 -> 1618 us).
 #include <type_traits>
 
 #include "ta_tensor_common.cuh"
@@ -61,8 +62,9 @@ struct FwdSmem {
   static constexpr int abort_flag = tmem_slot + 4;
   static constexpr int drop_flags = abort_flag + 4;               // [8] per-warp: the mask drops a key of this row
   static constexpr int step_count = drop_flags + 32;
-  static constexpr int steps = step_count + 4;                    // [256] u16: steps with a kept key (with a mask)
-  static constexpr int keep = (steps + 512 + 15) / 16 * 16;       // [kv_rings][kMaxKeepWords] u32
+  static constexpr int full_count = step_count + 4;
+  static constexpr int steps = full_count + 4;                    // [2][256] u16: full steps, other steps with a kept key
+  static constexpr int keep = (steps + 1024 + 15) / 16 * 16;       // [kv_rings][kMaxKeepWords] u32
   static constexpr int total = keep + kv_rings * kMaxKeepWords * 4;
   static constexpr int bytes = total + 1024;                      // slack to align the base to 1 KiB
 };
@@ -90,11 +92,12 @@ struct FwdParams {
 
 constexpr float kStepSumLimit = 1024.f;  // a step's sum of probabilities that sends its warp back for a new reference
 
-// What the CTA's roles do once its set-up stands.  BITS: some key may be dropped, by the mask or because the last key step is
-// ragged.
-template <typename T, bool HAS_BIAS, bool GATED, bool ROWS, bool BITS>
+// What the CTA's roles do once its set-up stands.  PLAIN: every key of every row is kept.  `masked`: otherwise the mask drops
+// some, and the step list stands.
+template <typename T, bool HAS_BIAS, bool GATED, bool ROWS, bool PLAIN>
 __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base, uint8_t* smem_gen, volatile int* abort_flag,
-                                         uint32_t tmem_base, int tid, int warp, int lane, int h, int r0, int b, int q0, int n_tiles) {
+                                         uint32_t tmem_base, int tid, int warp, int lane, int h, int r0, int b, int q0, int n_tiles,
+                                         bool masked) {
   using Smem = FwdSmem<ROWS>;
   const uint32_t* keep_words = reinterpret_cast<const uint32_t*>(smem_gen + Smem::keep);
   const uint16_t* step_list = reinterpret_cast<const uint16_t*>(smem_gen + Smem::steps);
@@ -102,15 +105,16 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
   auto bar = [&](int index) -> uint32_t { return smem_base + Smem::bars + index * 8; };
   const int n_rings = ROWS ? n_tiles : 1;
   const int g = P.bias_groups == 1 ? 0 : r0;
-  const bool has_mask = BITS && P.mask != nullptr;
+  const bool listed = !PLAIN && masked;
   auto row_of = [&](int w) { return ROWS ? r0 + w : r0; };
   auto first_query = [&](int w) { return ROWS ? q0 : q0 + w * kTile; };
-  const int KS = has_mask ? *reinterpret_cast<volatile int*>(smem_gen + Smem::step_count) : P.k_steps;
-  auto step_at = [&](int i) { return has_mask ? int(step_list[i]) : i; };
+  const int KS = listed ? *reinterpret_cast<volatile int*>(smem_gen + Smem::step_count) : P.k_steps;
+  const int full_steps = PLAIN ? KS : listed ? *reinterpret_cast<volatile int*>(smem_gen + Smem::full_count) : P.cols / kKeys;  // come first; the others test their kept bits
+  auto step_at = [&](int i) { return listed ? int(step_list[i < full_steps ? i : 256 + i - full_steps]) : i; };
   // Value rows only need the sign-off handshake when the mask really drops a key of the row.
   auto needs_signoff = [&](int w) {
     bool drops = false;
-    if (has_mask) {
+    if (listed) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) drops |= (!ROWS || (i >> 2) == w) && drop_flags[i] != 0;
     }
@@ -189,8 +193,11 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
         // the operands of the next score product and of this value product arrive ahead of the probabilities
         if (i + 1 < KS) ok = mbar_wait(bar(Smem::k_full + ring + next), next_round & 1, abort_flag);
         if (ok) ok = mbar_wait(bar(Smem::v_full + ring + st), round & 1, abort_flag);
-        // with a mask, a warpgroup signs off every value step after clearing the rows of dropped keys
-        if (ok && signoff) ok = mbar_wait(bar(Smem::v_ready + ring + st), round & 1, abort_flag);
+        // a warpgroup signs off the value steps with dropped keys after clearing their rows
+        if (ok && signoff && i >= full_steps) {
+          const int j = i - full_steps;
+          ok = mbar_wait(bar(Smem::v_ready + ring + j % kStages), (j / kStages) & 1, abort_flag);
+        }
         if (ok) ok = mbar_wait(bar(Smem::p_full + w), i & 1, abort_flag);
         if (!ok) break;
         tc_fence_after_sync();
@@ -222,24 +229,22 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
     float ref = -INFINITY, l_run = 0.f;  // reference (base-2 logit) and sum of the row
     bool ok = true;
 
-    for (int i = 0; i < KS && ok; ++i) {
+    // One step; `drops`: some of its keys are dropped.
+    auto step = [&](int i, auto drops) {
+      constexpr bool kDrops = decltype(drops)::value;
       uint2 bits = make_uint2(0xffffffffu, 0xffffffffu);  // keys 0-31 and 32-63 of the step
-      if (BITS) bits = *reinterpret_cast<const uint2*>(keep_words + ring * kMaxKeepWords + step_at(i) * 2);
-      const bool all_kept = (bits.x & bits.y) == 0xffffffffu;
-      if (signs_off) {
+      if (kDrops) bits = *reinterpret_cast<const uint2*>(keep_words + ring * kMaxKeepWords + step_at(i) * 2);
+      if (kDrops && signs_off) {
         // Values of dropped keys must not reach the tensor core (0 * inf): clear their rows in shared memory.
-        // Every step is signed off (one barrier phase per step); only steps with dropped keys are touched.
         const int slot = ring * kStages + i % kStages;
-        if (!all_kept) {
-          ok = mbar_wait(bar(Smem::v_full + slot), (i / kStages) & 1, abort_flag);
-          if (!ok) break;
-          if (t < kKeys && (((t < 32 ? bits.x : bits.y) >> (t & 31)) & 1u) == 0) {
-            uint4* row = reinterpret_cast<uint4*>(smem_gen + Smem::v + slot * kKvBytes + t * 64);
-            row[0] = row[1] = row[2] = row[3] = make_uint4(0, 0, 0, 0);
-          }
-          fence_proxy_async_smem();
+        ok = mbar_wait(bar(Smem::v_full + slot), (i / kStages) & 1, abort_flag);
+        if (!ok) return;
+        if (t < kKeys && (((t < 32 ? bits.x : bits.y) >> (t & 31)) & 1u) == 0) {
+          uint4* row = reinterpret_cast<uint4*>(smem_gen + Smem::v + slot * kKvBytes + t * 64);
+          row[0] = row[1] = row[2] = row[3] = make_uint4(0, 0, 0, 0);
         }
-        mbar_arrive_warp(bar(Smem::v_ready + slot));
+        fence_proxy_async_smem();
+        mbar_arrive_warp(bar(Smem::v_ready + ring * kStages + (i - full_steps) % kStages));
       }
 
       const int bias_slot = (ROWS ? 0 : w * 2) + (i & 1);
@@ -248,19 +253,19 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
       const bool bias_there = HAS_BIAS && mbar_test(bar(Smem::bias_full + bias_slot), (i >> 1) & 1);
       ok = mbar_wait_probed(s_there, bar(Smem::s_full + w), i & 1, abort_flag);
       if (ok && HAS_BIAS) ok = mbar_wait_probed(bias_there, bar(Smem::bias_full + bias_slot), (i >> 1) & 1, abort_flag);
-      if (!ok) break;
+      if (!ok) return;
       tc_fence_after_sync();
       // swizzled row of the bias tile: 16-byte chunk n holds keys 8 n .. 8 n + 7
       const uint32_t bias_row = smem_base + Smem::bias + bias_slot * kBiasBytes + t * 128 + ((t & 7) << 4);
 
       // Base-2 logits x + shift of 16 columns, as eight pairs; dropped keys become -inf.
-      auto logits16 = [&](int chunk, const uint32_t (&s)[16], const uint4 (&bw)[2], f32x2 shift2, bool drops, f32x2 (&x)[8]) {
+      auto logits16 = [&](int chunk, const uint32_t (&s)[16], const uint4 (&bw)[2], f32x2 shift2, f32x2 (&x)[8]) {
         const uint32_t words[8] = {bw[0].x, bw[0].y, bw[0].z, bw[0].w, bw[1].x, bw[1].y, bw[1].z, bw[1].w};
 #pragma unroll
         for (int n = 0; n < 8; ++n) {
           const f32x2 s2 = pack2(__uint_as_float(s[2 * n]), __uint_as_float(s[2 * n + 1]));
           x[n] = fma2(s2, c2, HAS_BIAS ? fma2(Half2<T>::widen(words[n]), log2e2, shift2) : shift2);
-          if (drops) {
+          if (kDrops) {
             const uint32_t kept = (chunk < 2 ? bits.x : bits.y) >> ((chunk & 1) * 16 + 2 * n);
             float lo, hi;
             unpack2(x[n], lo, hi);
@@ -285,7 +290,7 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
           tmem_wait_ld();
           tmem_loaded(s);
           f32x2 x[8];
-          logits16(chunk, s, bw, pack2(0.f, 0.f), true, x);
+          logits16(chunk, s, bw, pack2(0.f, 0.f), x);
 #pragma unroll
           for (int n = 0; n < 8; ++n) {
             float lo, hi;
@@ -297,9 +302,9 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
         return peak;
       };
       // Raises the reference of the rows whose step needs it, and rescales what they have summed so far.
-      auto raise = [&](bool wanted, int attempt) -> bool {
+      auto raise = [&](bool wanted, bool first) -> bool {
         tmem_wait_st();  // probabilities of a pass that is about to be repeated
-        const float peak = step_peak(attempt == 0);
+        const float peak = step_peak(first);
         const bool raised = wanted && peak > ref;
         const float alpha = raised ? ex2(ref - peak) : 1.f;  // 0 for a row without a reference so far
         if (raised) {
@@ -322,7 +327,7 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
       };
       // Probabilities of the step into tensor memory; returns their sum.
       bool p_free = i == 0;
-      auto step_pass = [&](auto drops) -> float {
+      auto step_pass = [&]() -> float {
         const float shift = ref == -INFINITY ? 0.f : -ref;
         const f32x2 shift2 = pack2(shift, shift);
         f32x2 totals[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
@@ -345,7 +350,7 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
             }
           }
           f32x2 x[8];
-          logits16(chunk, s[chunk & 1], bw[chunk & 1], shift2, decltype(drops)::value, x);
+          logits16(chunk, s[chunk & 1], bw[chunk & 1], shift2, x);
 #pragma unroll
           for (int n = 0; n < 8; ++n) {
             float lo, hi;
@@ -371,19 +376,23 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
       bool wanted = ref == -INFINITY;
 #pragma unroll 1
       for (int attempt = 0; attempt < 2 && ok; ++attempt) {
-        if (__any_sync(0xffffffffu, wanted)) ok = raise(wanted, attempt);
+        if (__any_sync(0xffffffffu, wanted)) ok = raise(wanted, attempt == 0);
         else if (attempt > 0) break;
-        if (!ok) break;
-        sum = !BITS || all_kept ? step_pass(std::false_type{}) : step_pass(std::true_type{});
+        if (!ok) return;
+        sum = step_pass();
         wanted = !(sum < kStepSumLimit);
       }
-      if (!ok) break;
+      if (!ok) return;
       l_run += sum;
       tmem_wait_st();
       tc_fence_before_sync();
       mbar_arrive_warp(bar(Smem::p_full + w));
       if (HAS_BIAS) mbar_arrive_warp(bar(Smem::bias_empty + bias_slot));
-    }
+    };
+    int i = 0;
+    for (; i < full_steps && ok; ++i) step(i, std::false_type{});
+    if (!PLAIN)
+      for (; i < KS && ok; ++i) step(i, std::true_type{});
 
     // Gated epilogue: the thread's 32 gate logits are requested before the wait for the last product, so that their
     // trip from global memory runs under it (the words are not touched until the output row is ready).
@@ -470,6 +479,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + Smem::tmem_slot);
   uint32_t* keep_words = reinterpret_cast<uint32_t*>(smem_gen + Smem::keep);
   volatile int* step_count = reinterpret_cast<volatile int*>(smem_gen + Smem::step_count);
+  volatile int* full_count = reinterpret_cast<volatile int*>(smem_gen + Smem::full_count);
   uint16_t* step_list = reinterpret_cast<uint16_t*>(smem_gen + Smem::steps);
   auto bar = [&](int index) -> uint32_t { return smem_base + Smem::bars + index * 8; };
 
@@ -544,36 +554,50 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
     if (lane == 0) drop_flags[warp] = dropped_any ? 1u : 0u;
   }
   __syncthreads();
-  // Rows of which every key is kept take the walk without tests.
-  bool plain = P.cols % kKeys == 0;
+  bool listed = false;  // the mask drops a key of some row of the CTA
   if (has_mask) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) plain &= drop_flags[i] == 0;
+    for (int i = 0; i < 8; ++i) listed |= drop_flags[i] != 0;
   }
-  if (has_mask && !plain) {
-    // The steps in which some row of the CTA keeps a key, in order: padding is neither loaded nor computed.
+  if (listed) {
+    // The steps in which every row of the CTA keeps every key, then those in which some row keeps some: padding is neither
+    // loaded nor computed.
     if (warp == 0) {
-      int count = 0;
+      int full = 0, partial = 0;
       for (int first = 0; first < P.k_steps; first += 32) {
         const int j = first + lane;
-        uint32_t any = 0;
-        if (j < P.k_steps)
-          for (int ring = 0; ring < n_rings; ++ring)
-            any |= keep_words[ring * kMaxKeepWords + 2 * j] | keep_words[ring * kMaxKeepWords + 2 * j + 1];
-        const uint32_t live = __ballot_sync(0xffffffffu, any != 0);
-        if (any != 0) step_list[count + __popc(live & ((1u << lane) - 1))] = uint16_t(j);
-        count += __popc(live);
+        uint32_t any = 0, all = 0xffffffffu;
+        if (j < P.k_steps) {
+#pragma unroll
+          for (int ring = 0; ring < Smem::kv_rings; ++ring) {
+            if (ring >= n_rings) break;
+            const uint2 words = *reinterpret_cast<const uint2*>(keep_words + ring * kMaxKeepWords + 2 * j);
+            any |= words.x | words.y;
+            all &= words.x & words.y;
+          }
+        }
+        const bool is_full = any != 0 && all == 0xffffffffu, is_partial = any != 0 && all != 0xffffffffu;
+        const uint32_t fulls = __ballot_sync(0xffffffffu, is_full), partials = __ballot_sync(0xffffffffu, is_partial);
+        const uint32_t below = (1u << lane) - 1;
+        if (is_full) step_list[full + __popc(fulls & below)] = uint16_t(j);
+        if (is_partial) step_list[256 + partial + __popc(partials & below)] = uint16_t(j);
+        full += __popc(fulls);
+        partial += __popc(partials);
       }
-      if (lane == 0) *step_count = count;
+      if (lane == 0) {
+        *full_count = full;
+        *step_count = full + partial;
+      }
     }
     __syncthreads();
   }
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  if (plain)
-    fwd_walk<T, HAS_BIAS, GATED, ROWS, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, h, r0, b, q0, n_tiles);
+  if (!listed && P.cols % kKeys == 0)
+    fwd_walk<T, HAS_BIAS, GATED, ROWS, true>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, h, r0, b, q0, n_tiles, false);
   else
-    fwd_walk<T, HAS_BIAS, GATED, ROWS, true>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, h, r0, b, q0, n_tiles);
+    fwd_walk<T, HAS_BIAS, GATED, ROWS, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, h, r0, b, q0, n_tiles,
+                                              listed);
   teardown(abort_flag, tmem_base, 9, kFwdTmemCols);
 }
 
