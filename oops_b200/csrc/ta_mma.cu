@@ -14,7 +14,11 @@
 //             keys); a 64 x 64 tile of the row-shared bias gradient, rows innermost, summed in registers.  Each makes the
 //             scores it needs again (9 products instead of 5): token attention has too few rows and heads to give a
 //             CTA a whole row, and nothing has to be added across CTAs, so results are reproducible.
-// 4 samples, 16 heads of 64 channels, 512 tokens, forward + reverse: 1178 us in 9 launches on the earlier path.
+// 4 samples, 16 heads of 64 channels, 512 tokens: 35 us forward and 136 us reverse, against 1178 us in 9 launches with scores
+// in memory.  Bound by issue slots (two thirds of them element-wise work on the scores) at twelve warps per SM: packed f32
+// arithmetic, no tests on kept keys where a tile keeps all, first products without a zeroed accumulator, and, in the
+// reverse, row operands read again from shared memory instead of held in 64 registers (238 -> 168 registers, two -> three
+// CTAs per SM) took 45 and 171 us to these figures.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -83,6 +87,10 @@ struct Pair16<__nv_bfloat16> {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
   }
+  static __device__ __forceinline__ void mma_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {  // c = a b
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+  }
 };
 template <>
 struct Pair16<__half> {
@@ -94,6 +102,10 @@ struct Pair16<__half> {
   static __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+  }
+  static __device__ __forceinline__ void mma_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {  // c = a b
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
   }
 };
 
@@ -176,21 +188,43 @@ __device__ __forceinline__ void load_rows(uint32_t (&a)[DP / 16][4], const T* ti
   for (int kc = 0; kc < DP / 16; ++kc) ldmatrix4(a[kc], tile + (row0 + (lane & 15)) * pitch<DP>() + kc * 16 + (lane >> 4) * 8);
 }
 
+template <typename T, int NT>
+__device__ __forceinline__ void score_step(float (&s)[NT][4], const uint32_t (&a)[4], const T* columns, int pitch, bool first) {
+#pragma unroll
+  for (int np = 0; np < NT / 2; ++np) {
+    uint32_t b[4];
+    ldmatrix4(b, columns + np * 16 * pitch);
+    if (first) {
+      Pair16<T>::mma_first(s[2 * np], a, b[0], b[1]);
+      Pair16<T>::mma_first(s[2 * np + 1], a, b[2], b[3]);
+    } else {
+      Pair16<T>::mma(s[2 * np], a, b[0], b[1]);
+      Pair16<T>::mma(s[2 * np + 1], a, b[2], b[3]);
+    }
+  }
+}
+
 // s[nt] = rows x (columns col0 + 8 nt ...)^T over the channels: NT tiles of 8 columns.
 template <typename T, int DP, int NT>
 __device__ __forceinline__ void scores(float (&s)[NT][4], const uint32_t (&a)[DP / 16][4], const T* tile, int col0) {
   const int lane = threadIdx.x & 31;
+  const T* columns = tile + (col0 + (lane & 7) + (lane >> 4) * 8) * pitch<DP>() + ((lane >> 3) & 1) * 8;
 #pragma unroll
-  for (int nt = 0; nt < NT; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+  for (int kc = 0; kc < DP / 16; ++kc) score_step<T, NT>(s, a[kc], columns + kc * 16, pitch<DP>(), kc == 0);
+}
+
+// The same with the rows fetched from their tile (row0 ...) as they are needed: registers for shared-memory reads.
+template <typename T, int DP, int NT>
+__device__ __forceinline__ void scores(float (&s)[NT][4], const T* rows, int row0, const T* tile, int col0) {
+  const int lane = threadIdx.x & 31;
+  const T* columns = tile + (col0 + (lane & 7) + (lane >> 4) * 8) * pitch<DP>() + ((lane >> 3) & 1) * 8;
+  const T* row = rows + (row0 + (lane & 15)) * pitch<DP>() + (lane >> 4) * 8;
 #pragma unroll
-  for (int kc = 0; kc < DP / 16; ++kc)
-#pragma unroll
-    for (int np = 0; np < NT / 2; ++np) {
-      uint32_t b[4];
-      ldmatrix4(b, tile + (col0 + np * 16 + (lane & 7) + (lane >> 4) * 8) * pitch<DP>() + kc * 16 + ((lane >> 3) & 1) * 8);
-      Pair16<T>::mma(s[2 * np], a[kc], b[0], b[1]);
-      Pair16<T>::mma(s[2 * np + 1], a[kc], b[2], b[3]);
-    }
+  for (int kc = 0; kc < DP / 16; ++kc) {
+    uint32_t a[4];
+    ldmatrix4(a, row + kc * 16);
+    score_step<T, NT>(s, a, columns + kc * 16, pitch<DP>(), kc == 0);
+  }
 }
 
 // acc += w (16 rows x 8 NT columns, f32, as a 16-bit value and its remainder) x tile rows col0 ... (channels as columns)
@@ -204,8 +238,8 @@ __device__ __forceinline__ void accumulate(float (&acc)[DP / 8][4], const float 
     for (int i = 0; i < 4; ++i) {
       const float x = w[2 * kc + (i >> 1)][(i & 1) * 2], y = w[2 * kc + (i >> 1)][(i & 1) * 2 + 1];
       hi[i] = Pair16<T>::pack(x, y);
-      const float2 near = Pair16<T>::widen(hi[i]);
-      lo[i] = Pair16<T>::pack(x - near.x, y - near.y);
+      const float2 rest = __ffma2_rn(Pair16<T>::widen(hi[i]), make_float2(-1.f, -1.f), make_float2(x, y));
+      lo[i] = Pair16<T>::pack(rest.x, rest.y);
     }
 #pragma unroll
     for (int np = 0; np < DP / 16; ++np) {
@@ -216,6 +250,24 @@ __device__ __forceinline__ void accumulate(float (&acc)[DP / 8][4], const float 
       Pair16<T>::mma(acc[2 * np + 1], hi, b[2], b[3]);
       Pair16<T>::mma(acc[2 * np + 1], lo, b[2], b[3]);
     }
+  }
+}
+
+__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 pair_of(const float (&s)[4], int half) { return make_float2(s[2 * half], s[2 * half + 1]); }
+__device__ __forceinline__ void set_pair(float (&s)[4], int half, float2 v) {
+  s[2 * half] = v.x;
+  s[2 * half + 1] = v.y;
+}
+// Columns 8 nt + 2 t, + 1 of an accumulator become `value` where their bit is not set.
+template <int NT>
+__device__ __forceinline__ void drop_columns(float (&s)[NT][4], uint64_t bits, int t, float value) {
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) {
+    const uint32_t kept = uint32_t(bits >> (nt * 8 + 2 * t));
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (((kept >> (i & 1)) & 1) == 0) s[nt][i] = value;
   }
 }
 
@@ -322,21 +374,20 @@ __global__ void __launch_bounds__(kThreads, 4) mma_forward_kernel(const MmaProbl
       float s[8][4];
       scores<T, DP, 8>(s, q, K, 0);
       // base-2 logits, then the online softmax of rows g and g + 8 (a quad of lanes holds a row)
-      float peak[2] = {-INFINITY, -INFINITY};
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-          const int col = nt * 8 + 2 * t;
-          float2 add = make_float2(0.f, 0.f);
-          if (plane) add = bias_pair<T, B32>(bias, warp * 16 + g + 8 * half, col);
-          float &x = s[nt][2 * half], &y = s[nt][2 * half + 1];
-          x = fmaf(x, c, add.x * kLog2e);
-          y = fmaf(y, c, add.y * kLog2e);
-          if (((bits >> col) & 1) == 0) x = -INFINITY;
-          if (((bits >> col) & 2) == 0) y = -INFINITY;
-          peak[half] = fmaxf(peak[half], fmaxf(x, y));
+          float2 add = both(0.f);
+          if (plane) add = __fmul2_rn(bias_pair<T, B32>(bias, warp * 16 + g + 8 * half, nt * 8 + 2 * t), both(kLog2e));
+          set_pair(s[nt], half, __ffma2_rn(pair_of(s[nt], half), both(c), add));
         }
+      if (bits != ~0ull) drop_columns(s, bits, t, -INFINITY);
+      float peak[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) peak[i >> 1] = fmaxf(peak[i >> 1], s[nt][i]);
       float shrink[2];
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
@@ -349,13 +400,18 @@ __global__ void __launch_bounds__(kThreads, 4) mma_forward_kernel(const MmaProbl
         peak[half] = base;
         l[half] *= shrink[half];
       }
+      float2 sum[2] = {both(0.f), both(0.f)};
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          s[nt][i] = ex2(s[nt][i] - peak[i >> 1]);
-          l[i >> 1] += s[nt][i];
+        for (int half = 0; half < 2; ++half) {
+          const float2 x = __fadd2_rn(pair_of(s[nt], half), both(-peak[half]));
+          const float2 e = make_float2(ex2(x.x), ex2(x.y));
+          set_pair(s[nt], half, e);
+          sum[half] = __fadd2_rn(sum[half], e);
         }
+#pragma unroll
+      for (int half = 0; half < 2; ++half) l[half] += sum[half].x + sum[half].y;
 #pragma unroll
       for (int i = 0; i < DP / 8; ++i) {
         o[i][0] *= shrink[0];
@@ -445,7 +501,6 @@ __device__ __forceinline__ void query_gradient(const MmaProblem& p, uint8_t* sme
     norm[half] = at < p.cols ? -p.lse[stat] * kLog2e : -INFINITY;
     delta[half] = at < p.cols ? p.delta[stat] : 0.f;
   }
-  uint32_t q[DP / 16][4], dout[DP / 16][4];
   float dq[DP / 8][4];
 #pragma unroll
   for (int i = 0; i < DP / 8; ++i) dq[i][0] = dq[i][1] = dq[i][2] = dq[i][3] = 0.f;
@@ -455,10 +510,6 @@ __device__ __forceinline__ void query_gradient(const MmaProblem& p, uint8_t* sme
     copies_commit();
     copies_wait<1>();
     __syncthreads();
-    if (kt == 0) {
-      load_rows<T, DP>(q, Q, warp * 16);
-      load_rows<T, DP>(dout, Q + tile_elems<DP>(), warp * 16);
-    }
     const uint64_t all = keep_bits(p, keep, kt * kT);
     const uint8_t* at = stages + (kt & 1) * kStage;
     const T* K = reinterpret_cast<const T*>(at);
@@ -467,20 +518,18 @@ __device__ __forceinline__ void query_gradient(const MmaProblem& p, uint8_t* sme
     for (int col0 = 0; col0 < kT; col0 += 32) {  // 32 keys at a time keep the registers of three CTAs per SM
       const uint32_t bits = uint32_t(all >> col0);
       float s[4][4], dp[4][4];
-      scores<T, DP, 4>(s, q, K, col0);
-      scores<T, DP, 4>(dp, dout, K + tile_elems<DP>(), col0);
+      scores<T, DP, 4>(s, Q, warp * 16, K, col0);
+      scores<T, DP, 4>(dp, Q + tile_elems<DP>(), warp * 16, K + tile_elems<DP>(), col0);
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-          const int col = nt * 8 + 2 * t;
-          float2 add = make_float2(0.f, 0.f);
-          if (plane) add = bias_pair<T, B32>(bias, warp * 16 + g + 8 * half, col0 + col);
-          const float x = ex2(fmaf(s[nt][2 * half], c, fmaf(add.x, kLog2e, norm[half])));
-          const float y = ex2(fmaf(s[nt][2 * half + 1], c, fmaf(add.y, kLog2e, norm[half])));
-          s[nt][2 * half] = (bits >> col) & 1 ? x * (dp[nt][2 * half] - delta[half]) : 0.f;
-          s[nt][2 * half + 1] = (bits >> col) & 2 ? y * (dp[nt][2 * half + 1] - delta[half]) : 0.f;
+          float2 shift = both(norm[half]);
+          if (plane) shift = __ffma2_rn(bias_pair<T, B32>(bias, warp * 16 + g + 8 * half, col0 + nt * 8 + 2 * t), both(kLog2e), shift);
+          const float2 x = __ffma2_rn(pair_of(s[nt], half), both(c), shift);
+          set_pair(s[nt], half, __fmul2_rn(make_float2(ex2(x.x), ex2(x.y)), __fadd2_rn(pair_of(dp[nt], half), both(-delta[half]))));
         }
+      if (bits != 0xffffffffu) drop_columns(s, bits, t, 0.f);
       if (p.dbias && p.bias_groups > 1) {
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
@@ -530,9 +579,9 @@ __device__ __forceinline__ void key_gradient(const MmaProblem& p, uint8_t* smem,
   load_tile<T, DP>(K + tile_elems<DP>(), p.v, p, b, r, h, kt * kT, keep);
   request(0);
   copies_commit();
-  const uint64_t bits = keep_bits(p, keep, kt * kT) >> (warp * 16 + g);
+  const uint64_t all = keep_bits(p, keep, kt * kT), bits = all >> (warp * 16 + g);
+  const bool all_kept = all == ~0ull;
   const bool kept[2] = {(bits & 1) != 0, ((bits >> 8) & 1) != 0};
-  uint32_t k[DP / 16][4], v[DP / 16][4];
   float dk[DP / 8][4], dv[DP / 8][4];
 #pragma unroll
   for (int i = 0; i < DP / 8; ++i)
@@ -544,10 +593,6 @@ __device__ __forceinline__ void key_gradient(const MmaProblem& p, uint8_t* smem,
     copies_commit();
     copies_wait<1>();
     __syncthreads();
-    if (qt == 0) {
-      load_rows<T, DP>(k, K, warp * 16);
-      load_rows<T, DP>(v, K + tile_elems<DP>(), warp * 16);
-    }
     const uint8_t* at = stages + (qt & 1) * kStage;
     const T* Q = reinterpret_cast<const T*>(at);
     const uint8_t* bias = at + 2 * tile_elems<DP>() * 2;
@@ -555,8 +600,8 @@ __device__ __forceinline__ void key_gradient(const MmaProblem& p, uint8_t* smem,
 #pragma unroll 1
     for (int col0 = 0; col0 < kT; col0 += 32) {
       float s[4][4], dp[4][4];
-      scores<T, DP, 4>(s, k, Q, col0);
-      scores<T, DP, 4>(dp, v, Q + tile_elems<DP>(), col0);
+      scores<T, DP, 4>(s, K, warp * 16, Q, col0);
+      scores<T, DP, 4>(dp, K + tile_elems<DP>(), warp * 16, Q + tile_elems<DP>(), col0);
       // the bias tile has queries as rows: its 8 x 8 blocks are read transposed
       float2 add[4][2];
 #pragma unroll
@@ -590,13 +635,18 @@ __device__ __forceinline__ void key_gradient(const MmaProblem& p, uint8_t* smem,
         const float2 delta = *reinterpret_cast<const float2*>(stats + kT + col0 + nt * 8 + 2 * t);
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-          const float x = ex2(fmaf(s[nt][2 * half], c, fmaf(add[nt][half].x, kLog2e, norm.x)));
-          const float y = ex2(fmaf(s[nt][2 * half + 1], c, fmaf(add[nt][half].y, kLog2e, norm.y)));
-          s[nt][2 * half] = kept[half] ? x : 0.f;
-          s[nt][2 * half + 1] = kept[half] ? y : 0.f;
-          dp[nt][2 * half] = kept[half] ? x * (dp[nt][2 * half] - delta.x) : 0.f;
-          dp[nt][2 * half + 1] = kept[half] ? y * (dp[nt][2 * half + 1] - delta.y) : 0.f;
+          const float2 x = __ffma2_rn(pair_of(s[nt], half), both(c), __ffma2_rn(add[nt][half], both(kLog2e), norm));
+          const float2 e = make_float2(ex2(x.x), ex2(x.y));
+          set_pair(s[nt], half, e);
+          set_pair(dp[nt], half, __fmul2_rn(e, __fadd2_rn(pair_of(dp[nt], half), make_float2(-delta.x, -delta.y))));
         }
+      }
+      if (!all_kept) {
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (!kept[i >> 1]) s[nt][i] = dp[nt][i] = 0.f;
       }
       if (p.dv.ptr) accumulate<T, DP, 4>(dv, s, Q + tile_elems<DP>(), col0);
       if (p.dk.ptr) accumulate<T, DP, 4>(dk, dp, Q, col0);
@@ -626,9 +676,19 @@ __device__ __forceinline__ void bias_gradient(const MmaProblem& p, uint8_t* smem
   const int b = idx % p.batch, part = idx / p.batch;
   const int first = part * p.rows_per_part, last = min(p.rows, first + p.rows_per_part);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const uint8_t* bias = smem + 2 * kStage;
-  load_bias<BiasType<T, B32>, bias_pitch<B32>()>(reinterpret_cast<BiasType<T, B32>*>(smem + 2 * kStage), bias_plane<T, B32>(p, b, 0, h), p,
-                                                 qt * kT, kt * kT);
+  // the thread's bias values stay in registers: [8 columns][row g, row g + 8][two neighbours]
+  using Bias = BiasType<T, B32>;
+  const Bias* plane = bias_plane<T, B32>(p, b, 0, h);
+  Bias add[8][2][2];
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int query = qt * kT + warp * 16 + g + 8 * half, key = kt * kT + nt * 8 + 2 * t;
+      const Bias* from = plane + int64_t(query) * p.b_sq + int64_t(key) * p.b_sk;
+      add[nt][half][0] = query < p.cols && key < p.cols ? from[0] : Bias(0.f);
+      add[nt][half][1] = query < p.cols && key + 1 < p.cols ? from[p.b_sk] : Bias(0.f);
+    }
   auto request = [&](int r) {
     T* at = reinterpret_cast<T*>(smem + ((r - first) & 1) * kStage);
     const uint8_t* keep = p.mask ? p.mask + b * p.m_sb + int64_t(r) * p.m_sr : nullptr;
@@ -660,26 +720,32 @@ __device__ __forceinline__ void bias_gradient(const MmaProblem& p, uint8_t* smem
     __syncthreads();
     const T* Q = reinterpret_cast<const T*>(smem + ((r - first) & 1) * kStage);
     if (all) {
-      uint32_t q[DP / 16][4], dout[DP / 16][4];
-      load_rows<T, DP>(q, Q, warp * 16);
-      load_rows<T, DP>(dout, Q + tile_elems<DP>(), warp * 16);
 #pragma unroll
       for (int col0 = 0; col0 < kT; col0 += 32) {
         const uint32_t bits = uint32_t(all >> col0);
         float s[4][4], dp[4][4];
-        scores<T, DP, 4>(s, q, Q + 2 * tile_elems<DP>(), col0);
-        scores<T, DP, 4>(dp, dout, Q + 3 * tile_elems<DP>(), col0);
+        scores<T, DP, 4>(s, Q, warp * 16, Q + 2 * tile_elems<DP>(), col0);
+        scores<T, DP, 4>(dp, Q + tile_elems<DP>(), warp * 16, Q + 3 * tile_elems<DP>(), col0);
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
-            const int col = nt * 8 + 2 * t;
-            const float2 add = bias_pair<T, B32>(bias, warp * 16 + g + 8 * half, col0 + col);
-            const float x = ex2(fmaf(s[nt][2 * half], c, fmaf(add.x, kLog2e, norm[half])));
-            const float y = ex2(fmaf(s[nt][2 * half + 1], c, fmaf(add.y, kLog2e, norm[half])));
-            float* to = acc[col0 / 8 + nt] + 2 * half;
-            if ((bits >> col) & 1) to[0] = fmaf(x, dp[nt][2 * half] - delta[half], to[0]);
-            if ((bits >> col) & 2) to[1] = fmaf(y, dp[nt][2 * half + 1] - delta[half], to[1]);
+            const Bias* two = add[col0 / 8 + nt][half];
+            const float2 x = __ffma2_rn(pair_of(s[nt], half), both(c),
+                                        __ffma2_rn(make_float2(float(two[0]), float(two[1])), both(kLog2e), both(norm[half])));
+            set_pair(s[nt], half, make_float2(ex2(x.x), ex2(x.y)));
+            set_pair(dp[nt], half, __fadd2_rn(pair_of(dp[nt], half), both(-delta[half])));
+          }
+        if (bits != 0xffffffffu) {
+          drop_columns(s, bits, t, 0.f);
+          drop_columns(dp, bits, t, 0.f);
+        }
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            float (&to)[4] = acc[col0 / 8 + nt];
+            set_pair(to, half, __ffma2_rn(pair_of(s[nt], half), pair_of(dp[nt], half), pair_of(to, half)));
           }
       }
     }
@@ -702,7 +768,7 @@ __device__ __forceinline__ void bias_gradient(const MmaProblem& p, uint8_t* smem
 }
 
 template <typename T, int DP, bool B32>
-__global__ void __launch_bounds__(kThreads) mma_backward_kernel(const MmaProblem p) {
+__global__ void __launch_bounds__(kThreads, DP <= 32 ? 4 : 3) mma_backward_kernel(const MmaProblem p) {
   extern __shared__ __align__(16) uint8_t mma_smem[];
   const int idx = blockIdx.x;
   if (idx < p.dkv_ctas) key_gradient<T, DP, B32>(p, mma_smem, idx);
@@ -877,7 +943,7 @@ int mma_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
     constexpr int DP = decltype(width)::value;
     constexpr bool B32 = decltype(b32)::value;
     constexpr int rows_smem = 6 * tile_elems<DP>() * 2 + 2 * (bias_bytes<B32>() + 2 * kT * 4);
-    constexpr int bias_smem = 8 * tile_elems<DP>() * 2 + bias_bytes<B32>();
+    constexpr int bias_smem = 8 * tile_elems<DP>() * 2;
     return launch(mma_backward_kernel<T, DP, B32>, m, grid, shared_gradient(p, g) ? std::max(rows_smem, bias_smem) : rows_smem, stream,
                   "mma backward");
   });
