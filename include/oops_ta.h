@@ -265,6 +265,14 @@ int oops_ta_pair_mask_packed(const uint8_t* token_values, const int64_t* token_o
                              uint8_t* out, void* stream);
 
 /*
+ * A 16-bit bias (batch, groups, heads, cols, cols) of any element strides (`strides`: batch, group, head, query, key), copied
+ * to contiguous rows of ceil(cols / 8) * 8 elements whose padding is zero: the layout that the tcgen05 kernels read a bias
+ * in when cols is no multiple of 8 or the bias is a permuted view.  `dst` is 16-byte aligned.
+ */
+int oops_ta_bias_rows(int32_t batch, int32_t groups, int32_t heads, int32_t cols, const void* src, const int64_t* strides,
+                      void* dst, void* stream);
+
+/*
  * Forward pass that needs no workspace from the caller and allocates nothing.
  *
  * It has no counterpart in the reference.  It is for hosts that cannot hand over scratch memory when

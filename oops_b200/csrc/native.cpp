@@ -393,11 +393,32 @@ bool dense_operands_fit(const Tensor& query, const Tensor& key, const Tensor& va
   return true;
 }
 
-// Contiguous bias; 16-bit biases get 16-byte aligned rows (the TMA kernels need them): the key axis is padded.
+// The values of a 16-bit (B, G, H, N, N) bias in contiguous rows of whole 16-byte words, seen as (B, G, H, N, N).
+Tensor padded_bias(const Tensor& bias) {
+  const c10::cuda::CUDAGuard guard(bias.device());
+  const int64_t cols = bias.size(4), row = (cols + 7) / 8 * 8;
+  const Tensor rows = at::empty({bias.size(0), bias.size(1), bias.size(2), cols, row}, bias.options());
+  check_status(oops_ta_bias_rows(int32_t(bias.size(0)), int32_t(bias.size(1)), int32_t(bias.size(2)), int32_t(cols), bias.data_ptr(),
+                                 bias.strides().data(), rows.data_ptr(), current_stream(bias)),
+               "triangle_attention bias rows");
+  return row == cols ? rows : rows.narrow(-1, 0, cols);
+}
+
+struct PaddedBiasFunction : Function<PaddedBiasFunction> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& bias) {
+    ctx->set_materialize_grads(false);
+    return padded_bias(bias);
+  }
+  static variable_list backward(AutogradContext*, const variable_list& grad_outputs) { return {grad_outputs[0]}; }
+};
+
+// 16-byte aligned bias rows, which the TMA kernels need (16-bit biases: the key axis is padded); otherwise contiguous.
 Tensor aligned_bias(const Tensor& bias, int64_t cols) {
-  Tensor b = as_batch(bias, 4).contiguous();
-  if (b.element_size() == 2 && cols % 8 != 0) b = at::constant_pad_nd(b, {0, 8 - cols % 8}).narrow(-1, 0, cols);
-  return b;
+  const Tensor b = as_batch(bias, 4);
+  if (b.element_size() != 2) return b.contiguous();
+  if (b.is_contiguous() && cols % 8 == 0) return b;
+  const Tensor values = b.resolve_neg().resolve_conj();
+  return at::GradMode::is_enabled() && values.requires_grad() ? PaddedBiasFunction::apply(values) : padded_bias(values);
 }
 
 std::optional<Tensor> dense_attention(const Tensor& query, const Tensor& key, const Tensor& value, const MaybeTensor& mask,

@@ -333,6 +333,18 @@ int oops_ta_pair_mask_packed(const uint8_t* token_values, const int64_t* token_o
   return packed_pair_mask(token_values, token_offsets, samples, chunks, out, reinterpret_cast<cudaStream_t>(stream));
 }
 
+int oops_ta_bias_rows(int32_t batch, int32_t groups, int32_t heads, int32_t cols, const void* src, const int64_t* strides,
+                      void* dst, void* stream) {
+  if (batch < 0 || groups < 0 || heads < 0 || cols < 0) return fail(OOPS_TA_INVALID_ARGUMENT, "negative extent");
+  if (int64_t(batch) * groups * heads * cols > 0 && (!src || !strides || !dst))
+    return fail(OOPS_TA_INVALID_ARGUMENT, "src, strides or dst is NULL");
+  if ((reinterpret_cast<uintptr_t>(dst) & 15) != 0) return fail(OOPS_TA_UNSUPPORTED_LAYOUT, "dst is not 16-byte aligned");
+  const int status = check_device();
+  if (status) return status;
+  g_error[0] = 0;
+  return bias_rows(batch, groups, heads, cols, src, strides, dst, reinterpret_cast<cudaStream_t>(stream));
+}
+
 int oops_ta_backward(const oops_ta_problem* problem, const oops_ta_pair* out, const oops_ta_pair* dout,
                      const float* lse, const oops_ta_grads* grads, void* stream) {
   int status = validate(problem, true);

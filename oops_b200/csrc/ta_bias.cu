@@ -1,0 +1,74 @@
+// Bias rows for the TMA kernels: a 16-bit bias (batch, group, head, query, key) of any strides copied to contiguous rows of
+// whole 16-byte words, zeros behind the last key.  One launch for what took a permuting copy, a fill and a padding copy.
+//
+// Bound by latency and, for a bias as a linear map over the pair leaves it (heads innermost), by strided reads.  A thread
+// writes one word of eight keys.  Neighbouring threads then take the heads of the same cells where the heads are the
+// neighbours in memory, so that a warp's reads share their sectors, and the next words of the row otherwise.
+// N = 100, 4 heads: 3.9 -> 2.1 us and one launch less; attention of N = 499 with a projected bias: 260 -> 244 us.
+#include "ta_internal.h"
+
+namespace oops_ta {
+namespace {
+
+struct BiasRows {
+  const uint16_t* src;
+  uint16_t* dst;
+  int64_t s_b, s_g, s_h, s_q, s_k;
+  uint32_t words, heads, cols, groups, total;  // words of a row
+  int heads_inner;
+};
+
+__global__ void __launch_bounds__(256) bias_rows_kernel(const BiasRows p) {
+  uint32_t i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= p.total) return;
+  uint32_t h = 0, word;
+  if (p.heads_inner) {
+    h = i % p.heads;
+    i /= p.heads;
+  }
+  word = i % p.words;
+  i /= p.words;
+  const uint32_t q = i % p.cols;
+  i /= p.cols;
+  if (!p.heads_inner) {
+    h = i % p.heads;
+    i /= p.heads;
+  }
+  const uint32_t g = i % p.groups, b = i / p.groups;
+  const uint16_t* src = p.src + b * p.s_b + g * p.s_g + h * p.s_h + q * p.s_q;
+  uint32_t packed[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (uint32_t e = 0; e < 8; ++e) {
+    const uint32_t key = word * 8 + e;
+    if (key < p.cols) packed[e / 2] |= uint32_t(src[int64_t(key) * p.s_k]) << (e % 2 * 16);
+  }
+  const int64_t row = ((int64_t(b) * p.groups + g) * p.heads + h) * p.cols + q;
+  reinterpret_cast<uint4*>(p.dst)[row * p.words + word] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+}
+
+}  // namespace
+
+int bias_rows(int batch, int groups, int heads, int cols, const void* src, const int64_t strides[5], void* dst, cudaStream_t stream) {
+  BiasRows p{};
+  p.src = reinterpret_cast<const uint16_t*>(src);
+  p.dst = reinterpret_cast<uint16_t*>(dst);
+  p.s_b = strides[0];
+  p.s_g = strides[1];
+  p.s_h = strides[2];
+  p.s_q = strides[3];
+  p.s_k = strides[4];
+  p.words = uint32_t(ceil_div(cols, 8));
+  p.heads = uint32_t(heads);
+  p.cols = uint32_t(cols);
+  p.groups = uint32_t(groups);
+  p.heads_inner = heads > 1 && p.s_h < p.s_k;
+  const int64_t total = int64_t(batch) * groups * heads * cols * p.words;
+  if (total == 0) return OOPS_TA_OK;
+  if (total > 0xffffff00ll) return fail(OOPS_TA_LIMIT_EXCEEDED, "bias of %lld words", (long long)total);
+  p.total = uint32_t(total);
+  bias_rows_kernel<<<(unsigned)ceil_div(total, 256), 256, 0, stream>>>(p);
+  count_launch();
+  return check_launch("bias rows");
+}
+
+}  // namespace oops_ta

@@ -67,6 +67,8 @@ int gate_backward(int dtype, int batch, int rows, int cols, int heads, int head_
 int packed_pair_mask(const uint8_t* tokens, const int64_t* token_offsets, int samples, int64_t chunks, uint8_t* out,
                      cudaStream_t stream);
 int packed_pair_mask_max_samples();
+// 16-bit bias of any strides (batch, group, head, query, key) to contiguous rows of ceil(cols / 8) 16-byte words.
+int bias_rows(int batch, int groups, int heads, int cols, const void* src, const int64_t strides[5], void* dst, cudaStream_t stream);
 // Layer normalisation over the last axis of (rows, width) activations (row strides in elements, contiguous rows);
 // weight / bias / gradients of them may be NULL; affine_dtype is the activation dtype or f32.
 uint64_t layer_norm_backward_workspace_bytes(int64_t rows, int width);
