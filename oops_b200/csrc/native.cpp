@@ -942,7 +942,11 @@ struct UpdateFunction : Function<UpdateFunction> {
                  "triangle_multiplication pair gate");
     auto piece = [&](const Tensor& t, int64_t which) { return t.narrow(0, which * hidden, which == kOutputGate ? channels : hidden); };
     if (weights_wanted) {
-      const Tensor stacked_grad = at::mm(dproj.t(), x);
+      Tensor stacked_grad = at::mm(dproj.t(), x);
+      // weights of one type share a conversion, of which each gets its rows
+      bool same_type = true;
+      for (size_t i = 5; i < 4 + size_t(kOutput); ++i) same_type = same_type && types[i] == types[4];
+      if (same_type) stacked_grad = stacked_grad.to(at::ScalarType(types[4]));
       for (int64_t i = 0; i < kOutput; ++i)
         if (need(4 + i)) give(4 + i, piece(stacked_grad, i));
     }

@@ -5,6 +5,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 #include "ta_internal.h"
 
@@ -70,6 +71,16 @@ int untiled_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* ls
   return generic_forward(p, out, lse, stream);
 }
 
+// Bytes that kernels have been allowed, by (kernel, device).  Entries are only added, and an allowance only grows, under the
+// lock; readers need none.
+struct Allowance {
+  std::atomic<uint64_t> key;
+  std::atomic<int> bytes;
+};
+constexpr uint32_t kAllowances = 1024;
+Allowance g_allowances[kAllowances];
+std::mutex g_allowance_lock;
+
 int check_device() {
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess) return fail(OOPS_TA_CUDA_ERROR, "cudaGetDevice failed");
@@ -88,6 +99,35 @@ int check_device() {
 }
 
 }  // namespace
+
+int reserve_dynamic_smem(const void* kernel, int bytes) {
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return fail(OOPS_TA_CUDA_ERROR, "cudaGetDevice failed");
+  const uint64_t key = uint64_t(reinterpret_cast<uintptr_t>(kernel)) ^ (uint64_t(device + 1) << 56);
+  const uint32_t start = uint32_t((key * 0x9e3779b97f4a7c15ull) >> 54);  // ten bits
+  auto find = [&]() -> Allowance* {  // the key's entry, or the empty one it would take
+    for (uint32_t i = 0; i < kAllowances; ++i) {
+      Allowance& a = g_allowances[(start + i) % kAllowances];
+      const uint64_t there = a.key.load(std::memory_order_acquire);
+      if (there == key || there == 0) return &a;
+    }
+    return nullptr;
+  };
+  Allowance* own = find();
+  if (own && own->key.load(std::memory_order_acquire) == key && own->bytes.load(std::memory_order_acquire) >= bytes) return OOPS_TA_OK;
+  const std::lock_guard<std::mutex> guard(g_allowance_lock);
+  own = find();
+  const bool known = own && own->key.load(std::memory_order_relaxed) == key;
+  if (known && own->bytes.load(std::memory_order_relaxed) >= bytes) return OOPS_TA_OK;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+    return fail(OOPS_TA_CUDA_ERROR, "cannot reserve %d bytes of shared memory", bytes);
+  if (own) {
+    own->bytes.store(bytes, std::memory_order_release);
+    own->key.store(key, std::memory_order_release);
+  }
+  return OOPS_TA_OK;
+}
+
 }  // namespace oops_ta
 
 using namespace oops_ta;

@@ -588,8 +588,8 @@ F32Problem describe(const oops_ta_problem& p) {
 template <typename Kernel>
 int launch(Kernel kernel, const F32Problem& f, int64_t grid, int floats, cudaStream_t stream, const char* what) {
   const int smem = floats * int(sizeof(float));
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-    return fail(OOPS_TA_CUDA_ERROR, "cannot reserve %d bytes of shared memory", smem);
+  const int status = reserve_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+  if (status) return status;
   kernel<<<(unsigned)grid, kThreads, smem, stream>>>(f);
   count_launch();
   return check_launch(what);

@@ -17,6 +17,10 @@ void count_launch(int n = 1);
 // Checks the last launch and converts a CUDA error into a status.
 int check_launch(const char* what);
 
+// Allows the kernel `bytes` of dynamic shared memory on the current device; remembered, so that only a kernel's first launch
+// on a device asks the driver (1 us a call).
+int reserve_dynamic_smem(const void* kernel, int bytes);
+
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 size_t dtype_size(int dtype);

@@ -840,8 +840,8 @@ MmaProblem describe(const oops_ta_problem& p) {
 
 template <typename Kernel>
 int launch(Kernel kernel, const MmaProblem& m, int64_t grid, int smem, cudaStream_t stream, const char* what) {
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-    return fail(OOPS_TA_CUDA_ERROR, "cannot reserve %d bytes of shared memory", smem);
+  const int status = reserve_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+  if (status) return status;
   kernel<<<(unsigned)grid, kThreads, smem, stream>>>(m);
   count_launch();
   return check_launch(what);

@@ -111,28 +111,48 @@ __device__ __forceinline__ int64_t token_at(const PairShape& s, int b, int64_t p
 // gated projections
 // ---------------------------------------------------------------------------------------------
 // Row m of `proj` holds [left gate | left value | right gate | right value | ...], `hidden` channels each.
-// CTA = (32 words of tokens, 32 channels, prefix element): half of the threads make `left`, half `right`.  The channel
-// chunk is the fastest index: a token's 64-byte pieces are touched by neighbouring CTAs while their lines are in L2.
+// The channels of `left` and `right`, each rounded up to eight, form one axis.  CTA = (32 words of tokens, 64 of that axis,
+// prefix element): a token's piece of a projection is then 128 contiguous bytes of a 16-bit type (64-byte pieces: 55 and
+// 90 us forward and reverse at N = 384, 128 channels).  The channel chunk is the fastest index: neighbouring CTAs touch a
+// token's other pieces while their pages are open.
+
+struct GateTile {  // rows = channels; rows 32 .. 63 stand four words on, so that a warp's eight channel groups miss each other's banks
+  uint32_t words[64 * kPitch + 4];
+  __device__ __forceinline__ uint32_t& at(int row, int word) { return words[row * kPitch + (row >> 5) * 4 + word]; }
+};
+
+// Where channel group `o` (the first of eight) of the common axis lies: its side, channel within the side, and how many of
+// the eight exist.
+struct GateGroup {
+  int side, channel, n;
+  __device__ GateGroup(const PairShape& s, int o) {
+    const int rounded = (s.hidden + 7) / 8 * 8;
+    side = o >= rounded;
+    channel = o - side * rounded;
+    n = o < 2 * rounded ? s.hidden - channel : 0;
+  }
+};
+__host__ __device__ inline int gate_chunks(int hidden) { return (2 * ((hidden + 7) / 8 * 8) + 63) / 64; }
 
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) pair_gate_forward_kernel(PairShape s, const T* __restrict__ proj, int64_t ld,
                                                                 const T* __restrict__ mask, uint32_t* __restrict__ left,
                                                                 uint32_t* __restrict__ right) {
   constexpr int W = tokens_per_word<T>();
-  __shared__ uint32_t tile[2][32][kPitch];
-  const int chunks = (s.hidden + 31) / 32, chunk = blockIdx.x % chunks, b = blockIdx.y;
+  __shared__ GateTile tile;
+  const int chunks = gate_chunks(s.hidden), chunk = blockIdx.x % chunks, b = blockIdx.y;
   const int64_t first = int64_t(blockIdx.x / chunks) * 32;  // first word of the tile in a plane
-  const int side = threadIdx.x >> 7, cg = threadIdx.x & 3, word = (threadIdx.x >> 2) & 31;
-  const int c = chunk * 32 + cg * 8, n = s.hidden - c;
+  const int cg = threadIdx.x & 7, word = threadIdx.x >> 3;
+  const GateGroup own(s, chunk * 64 + cg * 8);
   float out[W][8];
 #pragma unroll
   for (int e = 0; e < W; ++e) {
     const int64_t m = token_at(s, b, (first + word) * W + e);
     float gate[8], value[8];
-    if (m >= 0 && n > 0) {
-      const T* row = proj + m * ld + side * 2 * s.hidden + c;
-      load8<T, VEC>(row, n, gate);
-      load8<T, VEC>(row + s.hidden, n, value);
+    if (m >= 0 && own.n > 0) {
+      const T* row = proj + m * ld + own.side * 2 * s.hidden + own.channel;
+      load8<T, VEC>(row, own.n, gate);
+      load8<T, VEC>(row + s.hidden, own.n, value);
       const float weight = mask ? float(mask[m]) : 1.f;
 #pragma unroll
       for (int i = 0; i < 8; ++i) out[e][i] = weight * sigmoid_of<T>(gate[i]) * value[i];
@@ -144,15 +164,17 @@ __global__ void __launch_bounds__(256) pair_gate_forward_kernel(PairShape s, con
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     float both[2] = {out[0][i], out[W - 1][i]};
-    tile[side][cg * 8 + i][word] = to_word<T>(both);
+    tile.at(cg * 8 + i, word) = to_word<T>(both);
   }
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int64_t words = s.plane() / W;
-  for (int row = threadIdx.x >> 5; row < 64; row += 8) {
-    const int ch = chunk * 32 + (row & 31);
-    if (ch < s.hidden)
-      (row < 32 ? left : right)[(int64_t(b) * s.hidden + ch) * words + first + lane] = tile[row >> 5][row & 31][lane];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {  // a warp's eight rows are one channel group
+    const GateGroup group(s, chunk * 64 + (threadIdx.x >> 5) * 8);
+    if (i < group.n)
+      (group.side ? right : left)[(int64_t(b) * s.hidden + group.channel + i) * words + first + lane] =
+          tile.at((threadIdx.x >> 5) * 8 + i, lane);
   }
 }
 
@@ -162,38 +184,37 @@ __global__ void __launch_bounds__(256) pair_gate_backward_kernel(PairShape s, co
                                                                  const uint32_t* __restrict__ dright, T* __restrict__ dproj,
                                                                  int64_t ld_d) {
   constexpr int W = tokens_per_word<T>();
-  __shared__ uint32_t tile[2][32][kPitch];
-  const int chunks = (s.hidden + 31) / 32, chunk = blockIdx.x % chunks, b = blockIdx.y;
+  __shared__ GateTile tile;
+  const int chunks = gate_chunks(s.hidden), chunk = blockIdx.x % chunks, b = blockIdx.y;
   const int64_t first = int64_t(blockIdx.x / chunks) * 32;
   {
     const int lane = threadIdx.x & 31;
     const int64_t words = s.plane() / W;
+    const GateGroup group(s, chunk * 64 + (threadIdx.x >> 5) * 8);
 #pragma unroll
-    for (int row = threadIdx.x >> 5; row < 64; row += 8) {
-      const int ch = chunk * 32 + (row & 31);
-      tile[row >> 5][row & 31][lane] =
-          ch < s.hidden ? (row < 32 ? dleft : dright)[(int64_t(b) * s.hidden + ch) * words + first + lane] : 0u;
-    }
+    for (int i = 0; i < 8; ++i)
+      tile.at((threadIdx.x >> 5) * 8 + i, lane) =
+          i < group.n ? (group.side ? dright : dleft)[(int64_t(b) * s.hidden + group.channel + i) * words + first + lane] : 0u;
   }
-  const int side = threadIdx.x >> 7, cg = threadIdx.x & 3, word = (threadIdx.x >> 2) & 31;
-  const int c = chunk * 32 + cg * 8, n = s.hidden - c;
+  const int cg = threadIdx.x & 7, word = threadIdx.x >> 3;
+  const GateGroup own(s, chunk * 64 + cg * 8);
   float gate[W][8], value[W][8], weight[W];
   int64_t at[W];
 #pragma unroll
   for (int e = 0; e < W; ++e) {
-    const int64_t m = n > 0 ? token_at(s, b, (first + word) * W + e) : -1;
+    const int64_t m = own.n > 0 ? token_at(s, b, (first + word) * W + e) : -1;
     at[e] = m;
     if (m >= 0) {
-      const T* row = proj + m * ld + side * 2 * s.hidden + c;
-      load8<T, VEC>(row, n, gate[e]);
-      load8<T, VEC>(row + s.hidden, n, value[e]);
+      const T* row = proj + m * ld + own.side * 2 * s.hidden + own.channel;
+      load8<T, VEC>(row, own.n, gate[e]);
+      load8<T, VEC>(row + s.hidden, own.n, value[e]);
       weight[e] = mask ? float(mask[m]) : 1.f;
     }
   }
   __syncthreads();
   float grad[8][2];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) from_word<T>(tile[side][cg * 8 + i][word], grad[i]);
+  for (int i = 0; i < 8; ++i) from_word<T>(tile.at(cg * 8 + i, word), grad[i]);
 #pragma unroll
   for (int e = 0; e < W; ++e) {
     if (at[e] < 0) continue;
@@ -204,9 +225,9 @@ __global__ void __launch_bounds__(256) pair_gate_backward_kernel(PairShape s, co
       dvalue[i] = up * sg;
       dgate[i] = up * value[e][i] * sg * (1.f - sg);
     }
-    T* row = dproj + at[e] * ld_d + side * 2 * s.hidden + c;
-    store8<T, VEC>(row, n, dgate);
-    store8<T, VEC>(row + s.hidden, n, dvalue);
+    T* row = dproj + at[e] * ld_d + own.side * 2 * s.hidden + own.channel;
+    store8<T, VEC>(row, own.n, dgate);
+    store8<T, VEC>(row + s.hidden, own.n, dvalue);
   }
 }
 
@@ -557,7 +578,7 @@ int pair_gate_forward(int dtype, int prefix, int tokens, int padded, int hidden,
     using T = decltype(t);
     constexpr int kVec = 16 / int(sizeof(T));
     const bool vec = hidden % 8 == 0 && ld % kVec == 0 && aligned16(proj);
-    const dim3 grid((unsigned)(s.plane() / (32 * tokens_per_word<T>()) * ceil_div(hidden, 32)), (unsigned)prefix);
+    const dim3 grid((unsigned)(s.plane() / (32 * tokens_per_word<T>()) * gate_chunks(hidden)), (unsigned)prefix);
     auto kernel = vec ? pair_gate_forward_kernel<T, true> : pair_gate_forward_kernel<T, false>;
     kernel<<<grid, 256, 0, stream>>>(s, reinterpret_cast<const T*>(proj), ld, reinterpret_cast<const T*>(mask),
                                      reinterpret_cast<uint32_t*>(left), reinterpret_cast<uint32_t*>(right));
@@ -575,7 +596,7 @@ int pair_gate_backward(int dtype, int prefix, int tokens, int padded, int hidden
     using T = decltype(t);
     constexpr int kVec = 16 / int(sizeof(T));
     const bool vec = hidden % 8 == 0 && ld % kVec == 0 && ld_d % kVec == 0 && aligned16(proj) && aligned16(dproj);
-    const dim3 grid((unsigned)(s.plane() / (32 * tokens_per_word<T>()) * ceil_div(hidden, 32)), (unsigned)prefix);
+    const dim3 grid((unsigned)(s.plane() / (32 * tokens_per_word<T>()) * gate_chunks(hidden)), (unsigned)prefix);
     auto kernel = vec ? pair_gate_backward_kernel<T, true> : pair_gate_backward_kernel<T, false>;
     kernel<<<grid, 256, 0, stream>>>(s, reinterpret_cast<const T*>(proj), ld, reinterpret_cast<const T*>(mask),
                                      reinterpret_cast<const uint32_t*>(dleft), reinterpret_cast<const uint32_t*>(dright),
@@ -596,8 +617,10 @@ int channel_norm_forward(int dtype, int affine_dtype, int prefix, int tokens, in
     const bool vec = hidden % 8 == 0 && aligned16(y);
     const size_t smem = norm_smem_bytes<T>(s, 1, false);
     auto kernel = vec ? channel_norm_forward_kernel<T, A, true> : channel_norm_forward_kernel<T, A, false>;
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-      return fail(OOPS_TA_CUDA_ERROR, "cannot reserve %d bytes of shared memory", int(smem));
+    if (smem > 48 * 1024) {
+      const int rc = reserve_dynamic_smem(reinterpret_cast<const void*>(kernel), int(smem));
+      if (rc) return rc;
+    }
     const dim3 grid((unsigned)(s.plane() / (32 * tokens_per_word<T>())), (unsigned)prefix);
     kernel<<<grid, kNormThreads, smem, stream>>>(s, reinterpret_cast<const uint32_t*>(update), weight, bias, eps,
                                                  reinterpret_cast<T*>(y), mean, rstd);
@@ -627,8 +650,10 @@ int channel_norm_backward(int dtype, int affine_dtype, int prefix, int tokens, i
     const bool vec = hidden % 8 == 0 && aligned16(dy);
     const size_t smem = norm_smem_bytes<T>(s, 2, true);
     auto kernel = vec ? channel_norm_backward_kernel<T, A, true> : channel_norm_backward_kernel<T, A, false>;
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-      return fail(OOPS_TA_CUDA_ERROR, "cannot reserve %d bytes of shared memory", int(smem));
+    if (smem > 48 * 1024) {
+      const int rc = reserve_dynamic_smem(reinterpret_cast<const void*>(kernel), int(smem));
+      if (rc) return rc;
+    }
     kernel<<<(unsigned)grid, kNormThreads, smem, stream>>>(s, s.plane() / (32 * tokens_per_word<T>()),
                                                            reinterpret_cast<const T*>(dy), reinterpret_cast<const uint32_t*>(update),
                                                            weight, mean, rstd, reinterpret_cast<uint32_t*>(dupdate), dw_parts,

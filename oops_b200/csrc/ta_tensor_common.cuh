@@ -135,9 +135,7 @@ int sm_count() {
 
 template <typename Kernel>
 int reserve_smem(Kernel kernel, int bytes) {
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
-    return fail(OOPS_TA_CUDA_ERROR, "cannot reserve %d bytes of shared memory", bytes);
-  return OOPS_TA_OK;
+  return reserve_dynamic_smem(reinterpret_cast<const void*>(kernel), bytes);
 }
 
 }  // namespace
