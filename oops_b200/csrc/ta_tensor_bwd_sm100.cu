@@ -48,8 +48,9 @@ constexpr int kRing = 4;                                // ring depth of the str
 // delta[b][r][h][q] = sum_d O * dO.  Four lanes share a (cell, head): a warp reads 512 contiguous bytes of each tensor when
 // heads and cells are contiguous (one lane per (cell, head) read 64 bytes at 64-byte strides).  `row_inner`: cells of
 // neighbouring rows, not columns, are neighbours in memory (the ending-node form).  The blocks behind those of delta look at
-// the mask: live[b][r] has bit k set when some key of columns 128 k .. 128 k + 127 of the row is kept, and behind the rows'
-// words one word per eight rows tells whether they drop any key.
+// the mask: live[b][r] has bit k set when some key of columns 128 k .. 128 k + 127 of the row is kept, the
+// second word of a row whether all of them are, the third how many keys a row keeps if these are its first ones (else ~0), and
+// behind the rows' words one word per eight rows tells whether they drop any key.
 template <typename T>
 __global__ void __launch_bounds__(256, 8) prepare_kernel(oops_ta_pair out, oops_ta_pair dout, float* delta, uint32_t total, int cols,
                                                       int heads, int rows, int vec_ok, int row_inner, uint32_t delta_blocks,
@@ -60,24 +61,32 @@ __global__ void __launch_bounds__(256, 8) prepare_kernel(oops_ta_pair out, oops_
     bool dropped = false;
     if (row < num_rows) {
       const uint8_t* bytes = mask + (row / rows) * m_sb + int64_t(row % rows) * m_sr;
-      uint32_t bits = 0;
+      uint32_t bits = 0, full = 0;
+      int count = 0, end = 0;  // kept keys, and one behind the last of them
       for (int first = 0; first < cols; first += 128) {
-        bool any = false;
+        bool any = false, all = true;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int key = first + i * 32 + lane;
-          if (key < cols) {
-            const bool keep = bytes[int64_t(key) * m_sc] != 0;
-            any |= keep;
-            dropped |= !keep;
-          }
+          const bool keep = key < cols && bytes[int64_t(key) * m_sc] != 0;
+          any |= keep;
+          all &= keep || key >= cols;
+          const uint32_t kept = __ballot_sync(0xffffffffu, keep);
+          count += __popc(kept);
+          if (kept != 0) end = first + i * 32 + 32 - __clz(int(kept));
         }
         if (__any_sync(0xffffffffu, any)) bits |= 1u << (first / 128);
+        if (__all_sync(0xffffffffu, all)) full |= 1u << (first / 128);
+        else dropped = true;
       }
-      if (lane == 0) live[row] = bits;
+      if (lane == 0) {
+        live[row] = bits;
+        live[num_rows + row] = full;
+        live[2 * num_rows + row] = count == end ? uint32_t(count) : ~0u;
+      }
     }
     const int drops = __syncthreads_or(dropped);
-    if (threadIdx.x == 0) live[num_rows + block] = uint32_t(drops != 0);
+    if (threadIdx.x == 0) live[3 * num_rows + block] = uint32_t(drops != 0);
     return;
   }
   const uint32_t item = blockIdx.x * 64u + (threadIdx.x >> 2);
@@ -111,7 +120,8 @@ __global__ void __launch_bounds__(256, 8) prepare_kernel(oops_ta_pair out, oops_
 __device__ __forceinline__ bool keeps_all(const uint32_t* live, int num_rows, int lane) {
   const int words = (num_rows + 7) / 8;
   bool drops = false;
-  for (int i = lane; i < words; i += 32) drops |= __ldg(live + num_rows + i) != 0;
+#pragma unroll 4
+  for (int i = lane; i < words; i += 32) drops |= __ldg(live + 3 * num_rows + i) != 0;
   return !__any_sync(0xffffffffu, drops);
 }
 
@@ -1499,7 +1509,8 @@ struct DbSmem {
   static constexpr int tmem_slot = bars + num_bars * 8;
   static constexpr int abort_flag = tmem_slot + 4;
   static constexpr int row_count = abort_flag + 4;
-  static constexpr int row_list = (row_count + 4 + 15) / 16 * 16;  // [kDbListRows] u16: rows of the part with a kept key in the tile
+  static constexpr int keys_end = row_count + 4;
+  static constexpr int row_list = (keys_end + 4 + 15) / 16 * 16;  // [kDbListRows] u16: rows of the part with a kept key in the tile
   static constexpr int total = row_list + kDbListRows * 2;
 };
 constexpr int kDbSmemBytes = DbSmem::total + 1024;
@@ -1521,12 +1532,12 @@ struct DbParams {
   float scale;
 };
 
-// BITS: some key may be dropped.  LISTED: the rows that keep no key of the tile add nothing, and every role walks the others
-// through a list.
+// BITS: rows may drop keys of the tile, each its own; otherwise they keep the same ones, those before `end`.  LISTED: the rows
+// that keep no key of the tile add nothing, and every role walks the others through a list.
 template <typename T, bool BITS, bool LISTED>
 __device__ __forceinline__ void dbias_walk(const DbParams& P, uint32_t smem_base, uint8_t* smem_gen, volatile int* abort_flag,
                                            uint32_t tmem_base, int tid, int warp, int lane, int b, int h, int qt, int kt, int part,
-                                           int row_lo, int part_rows) {
+                                           int row_lo, int part_rows, int end) {
   auto bar = [&](int index) -> uint32_t { return smem_base + DbSmem::bars + index * 8; };
   const bool has_mask = BITS && P.mask != nullptr;
   const uint16_t* row_list = reinterpret_cast<const uint16_t*>(smem_gen + DbSmem::row_list);
@@ -1615,12 +1626,13 @@ __device__ __forceinline__ void dbias_walk(const DbParams& P, uint32_t smem_base
     const int64_t stat_first = ((int64_t(b) * P.rows + row_lo) * P.heads + h) * P.cols + q_index;
     // Prefetch of the next row's statistics and mask byte: the loaded words stay untouched until that row's turn
     // (any arithmetic on them here would wait for the load).
+    int ahead = n_rows > 0 ? part_row(0) : 0;  // the row whose words are fetched next: list entries are read a row earlier still
     auto load_stats = [&](int i, float& lse_raw, float& delta_raw, uint32_t& keep_raw) {
       lse_raw = INFINITY;
       delta_raw = 0.f;
       keep_raw = 0;
       if (i < n_rows) {
-        const int at = part_row(i), r = row_lo + at;
+        const int at = LISTED ? ahead : i, r = row_lo + at;
         if (q_valid) {
           lse_raw = ldg_f32_here(P.lse + stat_first + int64_t(at) * stat_stride);
           delta_raw = ldg_f32_here(P.delta + stat_first + int64_t(at) * stat_stride);
@@ -1635,6 +1647,7 @@ __device__ __forceinline__ void dbias_walk(const DbParams& P, uint32_t smem_base
     float next_lse, next_dl;
     uint32_t next_keep;
     load_stats(0, next_lse, next_dl, next_keep);
+    if (LISTED) ahead = row_list[1];
 
     bool scores_there = false;  // answer of the probe the previous row sent for this row's scores
     for (int i = 0; i < n_rows && ok; ++i) {
@@ -1642,6 +1655,7 @@ __device__ __forceinline__ void dbias_walk(const DbParams& P, uint32_t smem_base
       const float neg_lse2 = -next_lse * kLog2e, neg_delta = -next_dl;
       const bool keep_lane = next_keep != 0;
       load_stats(i + 1, next_lse, next_dl, next_keep);
+      if (LISTED) ahead = row_list[min(i + 2, kDbListRows - 1)];
       const uint32_t bits = need_bits ? __ballot_sync(0xffffffffu, keep_lane) : 0xffffffffu;
       const f32x2 nl1 = pack2(neg_lse2, neg_lse2), nd1 = pack2(neg_delta, neg_delta);
       const float nl_unit = fmaf(neg_lse2, kUnit, kUnitShift);
@@ -1715,6 +1729,14 @@ __device__ __forceinline__ void dbias_walk(const DbParams& P, uint32_t smem_base
       else
         row_body(std::true_type{});
     }
+    if (!BITS && key_base + 32 > end) {  // keys that no row keeps
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        float lo, hi;
+        unpack2(acc2[i], lo, hi);
+        acc2[i] = pack2(key_base + 2 * i < end ? lo : 0.f, key_base + 2 * i + 1 < end ? hi : 0.f);
+      }
+    }
     if (ok && q_valid) {
       if (P.num_parts == 1 && P.dbias_f32) {
         float* dst = reinterpret_cast<float*>(P.dbias) + b * P.db_sb + h * P.db_sh + int64_t(q_index) * P.db_sq +
@@ -1776,9 +1798,11 @@ __device__ __forceinline__ void dbias_walk(const DbParams& P, uint32_t smem_base
   }
 }
 
-enum DbRows { kDbAllKept, kDbTested, kDbMasked };  // no dropped key; keys tested, no list; mask with a list
+// No dropped key; keys tested, no list; mask with a list.  Keys behind a ragged end need no test: their sums are not stored.
+enum DbRows { kDbAllKept, kDbTested, kDbMasked };
 
-// A mask that keeps everything takes the walk without tests and without a list (looking at them costs 5 to 8 %).
+// Rows that keep the same keys of the tile, up to some end, are walked without tests, and without the list where that is all
+// rows (tests and list cost 5 to 8 % even where nothing is dropped, tests 20 % and more where they take effect).
 template <typename T, int ROWS>
 __global__ void __launch_bounds__(kDbThreads, 1) ta_bwd_dbias_kernel(const __grid_constant__ DbParams P) {
   extern __shared__ uint8_t smem_raw[];
@@ -1804,19 +1828,37 @@ __global__ void __launch_bounds__(kDbThreads, 1) ta_bwd_dbias_kernel(const __gri
   const int part_rows = max(0, row_hi - row_lo);
   uint16_t* row_list = reinterpret_cast<uint16_t*>(smem_gen + DbSmem::row_list);
   volatile int* row_count = reinterpret_cast<volatile int*>(smem_gen + DbSmem::row_count);
-  bool plain = ROWS == kDbAllKept;
-  if (ROWS == kDbMasked && P.cols % kTile == 0) plain = keeps_all(P.live, P.batch * P.rows, lane);
-  if (ROWS == kDbMasked && !plain && warp == 0) {
+  // Where the listed rows keep the same keys of the tile, all up to a common end (a mask of real tokens), they are walked
+  // without tests and what stands behind the end is not stored; -1 otherwise.
+  volatile int* keys_end = reinterpret_cast<volatile int*>(smem_gen + DbSmem::keys_end);
+  if (ROWS == kDbMasked && warp == 0) {
+    const uint32_t* live = P.live + int64_t(b) * P.rows + row_lo;
+    const int64_t all_rows = int64_t(P.batch) * P.rows;
+    const uint32_t *full = live + all_rows, *length = live + 2 * all_rows;
     int count = 0;
-#pragma unroll 4
+    bool kept = true;
+    uint32_t shortest = ~0u, longest = 0;
+#pragma unroll 8
     for (int first = 0; first < part_rows; first += 32) {
-      const int i = first + lane;
-      const bool is_live = i < part_rows && ((__ldg(P.live + int64_t(b) * P.rows + row_lo + i) >> kt) & 1u) != 0;
+      const int i = min(first + lane, part_rows - 1);  // loads without conditions: many in flight
+      const uint32_t tiles = __ldg(live + i), whole = __ldg(full + i), keys = __ldg(length + i);
+      const bool is_live = first + lane < part_rows && ((tiles >> kt) & 1u) != 0;
       const uint32_t bits = __ballot_sync(0xffffffffu, is_live);
-      if (is_live) row_list[count + __popc(bits & ((1u << lane) - 1))] = uint16_t(i);
+      if (is_live) {
+        kept &= ((whole >> kt) & 1u) != 0;
+        shortest = min(shortest, keys);
+        longest = max(longest, keys);
+        row_list[count + __popc(bits & ((1u << lane) - 1))] = uint16_t(i);
+      }
       count += __popc(bits);
     }
-    if (lane == 0) *row_count = count;
+    kept = __all_sync(0xffffffffu, kept);
+    shortest = __reduce_min_sync(0xffffffffu, shortest);
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if (lane == 0) {
+      *row_count = count;
+      *keys_end = kept ? P.cols : shortest == longest && int(longest) >= 0 ? int(longest) : -1;
+    }
   }
 
   if (tid == 0) {
@@ -1840,11 +1882,20 @@ __global__ void __launch_bounds__(kDbThreads, 1) ta_bwd_dbias_kernel(const __gri
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  if (ROWS != kDbTested && plain)
-    dbias_walk<T, false, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, b, h, qt, kt, part, row_lo, part_rows);
-  else if (ROWS != kDbAllKept)
-    dbias_walk<T, true, ROWS == kDbMasked>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, b, h, qt, kt, part, row_lo,
-                                           part_rows);
+  const int end = ROWS == kDbMasked ? *keys_end : P.cols;
+  const bool kept = end >= 0, whole = kept && (ROWS != kDbMasked || *row_count == part_rows);
+  auto walk = [&](auto tests, auto listed) {
+    dbias_walk<T, decltype(tests)::value, decltype(listed)::value>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, b, h, qt,
+                                                                   kt, part, row_lo, part_rows, kept ? end : P.cols);
+  };
+  if (ROWS != kDbTested && whole)
+    walk(std::false_type{}, std::false_type{});
+  else if (ROWS == kDbMasked && kept)
+    walk(std::false_type{}, std::true_type{});
+  else if (ROWS == kDbMasked)
+    walk(std::true_type{}, std::true_type{});
+  else if (ROWS == kDbTested)
+    walk(std::true_type{}, std::false_type{});
   teardown(abort_flag, tmem_base, kDbMmaWarp, 512);
 }
 
@@ -1905,7 +1956,7 @@ Layout workspace_layout(const oops_ta_problem& p, const oops_ta_grads& g) {
   l.delta = at;
   at += align256(uint64_t(p.batch) * p.rows * p.heads * p.cols * sizeof(float));
   l.live = at;
-  if (p.mask) at += align256(uint64_t(p.batch) * p.rows * sizeof(uint32_t) * 2);
+  if (p.mask) at += align256(uint64_t(p.batch) * p.rows * sizeof(uint32_t) * 4);
   l.bias_t = at;
   const bool fused = fused_applies(p, g);
   if (p.bias_groups != 0 && (g.dk.ptr || g.dv.ptr) && !fused)
@@ -2141,7 +2192,7 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
     P.live = live;
     P.scale = p.scale;
     const unsigned grid = (unsigned)(int64_t(P.num_parts) * p.batch * p.heads * P.tiles * P.tiles);
-    auto kernel = !p.mask && p.cols % kTile == 0                ? ta_bwd_dbias_kernel<T, kDbAllKept>
+    auto kernel = !p.mask                                   ? ta_bwd_dbias_kernel<T, kDbAllKept>
                   : live && P.rows_per_part <= kDbListRows ? ta_bwd_dbias_kernel<T, kDbMasked>
                                                            : ta_bwd_dbias_kernel<T, kDbTested>;
     status = reserve_smem(kernel, kDbSmemBytes);
