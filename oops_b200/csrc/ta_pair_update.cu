@@ -113,8 +113,8 @@ __device__ __forceinline__ int64_t token_at(const PairShape& s, int b, int64_t p
 // Row m of `proj` holds [left gate | left value | right gate | right value | ...], `hidden` channels each.
 // The channels of `left` and `right`, each rounded up to eight, form one axis.  CTA = (32 words of tokens, 64 of that axis,
 // prefix element): a token's piece of a projection is then 128 contiguous bytes of a 16-bit type (64-byte pieces: 55 and
-// 90 us forward and reverse at N = 384, 128 channels).  The channel chunk is the fastest index: neighbouring CTAs touch a
-// token's other pieces while their pages are open.
+// 90 us forward and reverse at N = 384, 128 channels; now 52 and 78, the reverse with five CTAs per SM instead of
+// four).  The channel chunk is the fastest index: neighbouring CTAs touch a token's other pieces while their pages are open.
 
 struct GateTile {  // rows = channels; rows 32 .. 63 stand four words on, so that a warp's eight channel groups miss each other's banks
   uint32_t words[64 * kPitch + 4];
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(256) pair_gate_forward_kernel(PairShape s, con
 }
 
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(256) pair_gate_backward_kernel(PairShape s, const T* __restrict__ proj, int64_t ld,
+__global__ void __launch_bounds__(256, VEC ? 5 : 4) pair_gate_backward_kernel(PairShape s, const T* __restrict__ proj, int64_t ld,
                                                                  const T* __restrict__ mask, const uint32_t* __restrict__ dleft,
                                                                  const uint32_t* __restrict__ dright, T* __restrict__ dproj,
                                                                  int64_t ld_d) {

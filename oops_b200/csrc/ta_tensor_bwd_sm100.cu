@@ -1484,18 +1484,13 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
 // one query and 32 of the tile's keys) add dS into f32 registers.  Everything that does not depend on the row stays
 // in registers for the whole kernel: the thread's 32 bias values, already multiplied by log2(e), and the running
 // sums.  Per logit the loop then costs one packed add (bias - lse), one packed multiply-add (exponent), `ex2`, one
-// packed add (dP - delta) and one packed multiply-add (sum += P (dP - delta)).  A compile-time share of the `ex2`
-// runs as a polynomial on the FMA pipe.  With enough tiles to fill the SMs there is a single part and the CTA stores
+// packed add (dP - delta) and one packed multiply-add (sum += P (dP - delta)).  With enough tiles to fill the SMs there is a single part and the CTA stores
 // the final 16-bit gradient itself; small problems split the rows into parts whose f32 planes a last kernel adds in a
 // fixed order (no atomics, bitwise reproducible either way).
 
 constexpr int kDbRing = 4;
 constexpr int kDbListRows = 8192;       // longest part whose rows without a kept key are passed over
 constexpr int kDbStage = 4 * kBigTile;  // Q | dO | K | V of one row: 128 x 32 each
-#ifndef TA_DB_POLY_EVERY
-#define TA_DB_POLY_EVERY 0
-#endif
-constexpr int kDbPolyEvery = TA_DB_POLY_EVERY;  // every n-th pair of a thread's logits takes the polynomial exp2 (0: none)
 struct DbSmem {
   static constexpr int bias = 0;                         // 128 queries x 128 keys as two 64-key boxes (prologue only)
   static constexpr int ring = bias + 2 * kBiasStep;      // [kDbRing] stages
@@ -1597,9 +1592,7 @@ __device__ __forceinline__ void dbias_walk(const DbParams& P, uint32_t smem_base
     const bool q_valid = q_index < P.cols;
     const int key_base = kt * kTile + wg * 32;
     const float scale = P.scale;
-    constexpr float kUnit = 1.f / 128.f, kUnitShift = float(-kExp2PolyLow) / 128.f;
     const f32x2 c2 = pack2(scale * kLog2e, scale * kLog2e);
-    const float c_unit = scale * kLog2e * kUnit;
 
     // The thread's bias values, times log2(e), for the whole kernel.
     bool ok = mbar_wait(bar(DbSmem::bias_full), 0, abort_flag);
@@ -1658,7 +1651,6 @@ __device__ __forceinline__ void dbias_walk(const DbParams& P, uint32_t smem_base
       if (LISTED) ahead = row_list[min(i + 2, kDbListRows - 1)];
       const uint32_t bits = need_bits ? __ballot_sync(0xffffffffu, keep_lane) : 0xffffffffu;
       const f32x2 nl1 = pack2(neg_lse2, neg_lse2), nd1 = pack2(neg_delta, neg_delta);
-      const float nl_unit = fmaf(neg_lse2, kUnit, kUnitShift);
       ok = mbar_wait_probed(scores_there, bar(DbSmem::sd_full + buf), (i >> 1) & 1, abort_flag);
       if (!ok) break;
       tc_fence_after_sync();
@@ -1676,20 +1668,9 @@ __device__ __forceinline__ void dbias_walk(const DbParams& P, uint32_t smem_base
             const int pair = quad * 2 + j;
             const f32x2 s2 = pack2(__uint_as_float(sraw[2 * j]), __uint_as_float(sraw[2 * j + 1]));
             const f32x2 d2 = pack2(__uint_as_float(draw[2 * j]), __uint_as_float(draw[2 * j + 1]));
-            f32x2 p;
-            if (kDbPolyEvery > 0 && (pair % (kDbPolyEvery > 0 ? kDbPolyEvery : 1)) == kDbPolyEvery - 1) {
-              // exponent x = s c + bias log2e - lse log2e, as u = sat((x - low) / 128)
-              float b_lo, b_hi, s_lo, s_hi;
-              unpack2(bias2[pair], b_lo, b_hi);
-              unpack2(s2, s_lo, s_hi);
-              const float u_lo = fma_sat(s_lo, c_unit, fmaf(b_lo, kUnit, nl_unit));
-              const float u_hi = fma_sat(s_hi, c_unit, fmaf(b_hi, kUnit, nl_unit));
-              p = ex2_poly_unit(pack2(u_lo, u_hi));
-            } else {
-              float lo, hi;
-              unpack2(fma2(s2, c2, add2(bias2[pair], nl1)), lo, hi);
-              p = pack2(ex2(lo), ex2(hi));
-            }
+            float lo, hi;
+            unpack2(fma2(s2, c2, add2(bias2[pair], nl1)), lo, hi);
+            f32x2 p = pack2(ex2(lo), ex2(hi));
             f32x2 dd = add2(d2, nd1);
             if (decltype(drops_keys)::value) {
               p = select2(p, bits, 2 * pair);
