@@ -125,12 +125,10 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
 
   if (warp == 8) {
     // ------------------------------------------------------------------ producer (one thread)
-    if (lane == 0 && KS > 0) {
+    if (lane == 0) {
       bool ok = true;
-      for (int w = 0; w < n_tiles; ++w) {
-        mbar_expect_tx(bar(Smem::q_full + w), kQBytes);
-        tma_load_5d(smem_base + Smem::q + w * kQBytes, &P.map_q, bar(Smem::q_full + w), 0, h, first_query(w), row_of(w), b);
-      }
+      if (KS == 0)  // nobody else waits for the queries: the CTA must not leave before they have landed
+        for (int w = 0; w < n_tiles && ok; ++w) ok = mbar_wait(bar(Smem::q_full + w), 0, abort_flag);
       for (int i = 0; i < KS && ok; ++i) {
         const int st = i % kStages, round = i / kStages, key = step_at(i) * kKeys;
         for (int ring = 0; ring < n_rings && ok; ++ring) {
@@ -505,26 +503,30 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
   const bool has_bits = has_mask || (P.cols % kKeys) != 0;
   auto row_of = [&](int w) { return ROWS ? r0 + w : r0; };
 
-  if (tid == 0) {
-    *abort_flag = 0;
-    for (int i = 0; i < 2; ++i) mbar_init(bar(Smem::q_full + i), 1);
-    for (int i = 0; i < Smem::kv_rings * kStages; ++i) {
-      mbar_init(bar(Smem::k_full + i), 1);
-      mbar_init(bar(Smem::k_empty + i), ROWS ? 1 : n_tiles);
-      mbar_init(bar(Smem::v_full + i), 1);
-      mbar_init(bar(Smem::v_empty + i), ROWS ? 1 : n_tiles);
-      mbar_init(bar(Smem::v_ready + i), kTile / 32);
+  if (warp == 8) {
+    // The producer warp sets the barriers up, a lane each, and requests the queries: both run beside the look at the mask.
+    for (int i = lane; i < Smem::num_bars; i += 32) {
+      int arrivals = 1;
+      if ((i >= Smem::k_empty && i < Smem::v_full) || (i >= Smem::v_empty && i < Smem::v_ready)) arrivals = ROWS ? 1 : n_tiles;
+      if (i >= Smem::v_ready && i < Smem::bias_full) arrivals = kTile / 32;
+      if (i >= Smem::bias_empty && i < Smem::s_full) arrivals = ROWS ? n_tiles * (kTile / 32) : kTile / 32;
+      if (i >= Smem::p_full && i < Smem::pv_done) arrivals = kTile / 32;
+      mbar_init(bar(i), arrivals);
     }
-    for (int i = 0; i < Smem::bias_rings * 2; ++i) {
-      mbar_init(bar(Smem::bias_full + i), 1);
-      mbar_init(bar(Smem::bias_empty + i), ROWS ? n_tiles * (kTile / 32) : kTile / 32);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(Smem::s_full + i), 1);
-      mbar_init(bar(Smem::p_full + i), kTile / 32);
-      mbar_init(bar(Smem::pv_done + i), 1);
-    }
+    if (lane == 0) *abort_flag = 0;
     fence_barrier_init();
+    __syncwarp();
+    if (lane == 0) {
+      for (int w = 0; w < n_tiles; ++w) {
+        mbar_expect_tx(bar(Smem::q_full + w), kQBytes);
+        tma_load_5d(smem_base + Smem::q + w * kQBytes, &P.map_q, bar(Smem::q_full + w), 0, h, ROWS ? q0 : q0 + w * kTile, row_of(w), b);
+      }
+    }
+  }
+  if (warp == 10 && lane == 0) {
+    prefetch_tensormap(&P.map_k);
+    prefetch_tensormap(&P.map_v);
+    if (HAS_BIAS) prefetch_tensormap(&P.map_bias);
   }
   if (warp == 9) {
     tmem_alloc(smem_base + Smem::tmem_slot, kFwdTmemCols);
