@@ -57,7 +57,8 @@ struct FwdSmem {
   static constexpr int s_full = bias_empty + bias_rings * 2;      // [2] S of a step is in tensor memory
   static constexpr int p_full = s_full + 2;                       // [2] P is there, and S may be overwritten
   static constexpr int pv_done = p_full + 2;                      // [2] the latest P V product has completed
-  static constexpr int num_bars = pv_done + 2;
+  static constexpr int q_empty = pv_done + 2;                     // [2] every score product of an item has completed (PERSIST)
+  static constexpr int num_bars = q_empty + 2;
   static constexpr int tmem_slot = bars + num_bars * 8;
   static constexpr int abort_flag = tmem_slot + 4;
   static constexpr int drop_flags = abort_flag + 4;               // [8] per-warp: the mask drops a key of this row
@@ -79,6 +80,7 @@ struct FwdParams {
   const uint8_t* mask;
   int64_t m_sb, m_sr, m_sc;
   int batch, rows, cols, heads, bias_groups;
+  int items;             // query items x heads x rows (or pairs of rows) x batch
   int q_items, k_steps;  // query tiles (ROWS) or pairs of query tiles of a row; key steps
   int out_vec16;
   float scale;
@@ -92,22 +94,37 @@ struct FwdParams {
 
 constexpr float kStepSumLimit = 1024.f;  // a step's sum of probabilities that sends its warp back for a new reference
 
+// Where item `idx` lies: query item fastest, then head, row (or pair of rows), batch.
+struct FwdItem {
+  int h, r0, b, q0;
+};
+template <bool ROWS>
+__device__ __forceinline__ FwdItem fwd_item(const FwdParams& P, int idx) {
+  const int qi = idx % P.q_items;
+  idx /= P.q_items;
+  const int h = idx % P.heads;
+  idx /= P.heads;
+  const int row_items = ROWS ? (P.rows + 1) / 2 : P.rows;
+  return {h, (idx % row_items) * (ROWS ? 2 : 1), idx / row_items, qi * (ROWS ? kTile : 2 * kTile)};
+}
+
 // What the CTA's roles do once its set-up stands.  PLAIN: every key of every row is kept.  `masked`: otherwise the mask drops
-// some, and the step list stands.
-template <typename T, bool HAS_BIAS, bool GATED, bool ROWS, bool PLAIN>
+// some, and the step list stands.  PERSIST: the CTA goes on to further items, the first step's copies and score products of
+// the next one under the last steps and the output of this one; barrier phases count steps across items.
+template <typename T, bool HAS_BIAS, bool GATED, bool ROWS, bool PERSIST, bool PLAIN>
 __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base, uint8_t* smem_gen, volatile int* abort_flag,
-                                         uint32_t tmem_base, int tid, int warp, int lane, int h, int r0, int b, int q0, int n_tiles,
-                                         bool masked) {
+                                         uint32_t tmem_base, int tid, int warp, int lane, FwdItem at, int n_tiles, bool masked) {
   using Smem = FwdSmem<ROWS>;
   const uint32_t* keep_words = reinterpret_cast<const uint32_t*>(smem_gen + Smem::keep);
   const uint16_t* step_list = reinterpret_cast<const uint16_t*>(smem_gen + Smem::steps);
   const uint32_t* drop_flags = reinterpret_cast<const uint32_t*>(smem_gen + Smem::drop_flags);
   auto bar = [&](int index) -> uint32_t { return smem_base + Smem::bars + index * 8; };
   const int n_rings = ROWS ? n_tiles : 1;
-  const int g = P.bias_groups == 1 ? 0 : r0;
   const bool listed = !PLAIN && masked;
-  auto row_of = [&](int w) { return ROWS ? r0 + w : r0; };
-  auto first_query = [&](int w) { return ROWS ? q0 : q0 + w * kTile; };
+  // (a last row without a partner is its own partner in a persistent walk, whose barriers count two tiles)
+  auto row_of = [&](int w) { return ROWS ? (PERSIST ? min(at.r0 + w, P.rows - 1) : at.r0 + w) : at.r0; };
+  auto first_query = [&](int w) { return ROWS ? at.q0 : at.q0 + w * kTile; };
+  auto item_there = [&](int item, int turn) { return PERSIST ? item < P.items : turn == 0; };
   const int KS = listed ? *reinterpret_cast<volatile int*>(smem_gen + Smem::step_count) : P.k_steps;
   const int full_steps = PLAIN ? KS : listed ? *reinterpret_cast<volatile int*>(smem_gen + Smem::full_count) : P.cols / kKeys;  // come first; the others test their kept bits
   auto step_at = [&](int i) { return listed ? int(step_list[i < full_steps ? i : 256 + i - full_steps]) : i; };
@@ -129,31 +146,43 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
       bool ok = true;
       if (KS == 0)  // nobody else waits for the queries: the CTA must not leave before they have landed
         for (int w = 0; w < n_tiles && ok; ++w) ok = mbar_wait(bar(Smem::q_full + w), 0, abort_flag);
-      for (int i = 0; i < KS && ok; ++i) {
-        const int st = i % kStages, round = i / kStages, key = step_at(i) * kKeys;
-        for (int ring = 0; ring < n_rings && ok; ++ring) {
-          const int slot = ring * kStages + st;
-          if (i >= kStages) ok = mbar_wait(bar(Smem::k_empty + slot), (round - 1) & 1, abort_flag);
-          if (!ok) break;
-          mbar_expect_tx(bar(Smem::k_full + slot), kKvBytes);
-          tma_load_5d(smem_base + Smem::k + slot * kKvBytes, &P.map_k, bar(Smem::k_full + slot), 0, h, key, row_of(ring), b);
-        }
-        if (HAS_BIAS) {
-          for (int ring = 0; ring < (ROWS ? 1 : n_tiles) && ok; ++ring) {
-            const int slot = ring * 2 + (i & 1);
-            if (i >= 2) ok = mbar_wait(bar(Smem::bias_empty + slot), ((i >> 1) - 1) & 1, abort_flag);
+      int n = 0;  // steps so far
+      for (int item = int(blockIdx.x), turn = 0; ok && item_there(item, turn); item += int(gridDim.x), ++turn) {
+        if (PERSIST && turn > 0) {
+          at = fwd_item<ROWS>(P, item);
+          for (int w = 0; w < n_tiles && ok; ++w) {
+            ok = mbar_wait(bar(Smem::q_empty + w), (turn - 1) & 1, abort_flag);
             if (!ok) break;
-            mbar_expect_tx(bar(Smem::bias_full + slot), kBiasBytes);
-            tma_load_5d(smem_base + Smem::bias + slot * kBiasBytes, &P.map_bias, bar(Smem::bias_full + slot), key, first_query(ring),
-                        h, g, b);
+            mbar_expect_tx(bar(Smem::q_full + w), kQBytes);
+            tma_load_5d(smem_base + Smem::q + w * kQBytes, &P.map_q, bar(Smem::q_full + w), 0, at.h, first_query(w), row_of(w), at.b);
           }
         }
-        for (int ring = 0; ring < n_rings && ok; ++ring) {
-          const int slot = ring * kStages + st;
-          if (i >= kStages) ok = mbar_wait(bar(Smem::v_empty + slot), (round - 1) & 1, abort_flag);
-          if (!ok) break;
-          mbar_expect_tx(bar(Smem::v_full + slot), kKvBytes);
-          tma_load_5d(smem_base + Smem::v + slot * kKvBytes, &P.map_v, bar(Smem::v_full + slot), 0, h, key, row_of(ring), b);
+        for (int i = 0; i < KS && ok; ++i, ++n) {
+          const int st = n % kStages, round = n / kStages, key = step_at(i) * kKeys;
+          for (int ring = 0; ring < n_rings && ok; ++ring) {
+            const int slot = ring * kStages + st;
+            if (n >= kStages) ok = mbar_wait(bar(Smem::k_empty + slot), (round - 1) & 1, abort_flag);
+            if (!ok) break;
+            mbar_expect_tx(bar(Smem::k_full + slot), kKvBytes);
+            tma_load_5d(smem_base + Smem::k + slot * kKvBytes, &P.map_k, bar(Smem::k_full + slot), 0, at.h, key, row_of(ring), at.b);
+          }
+          if (HAS_BIAS) {
+            for (int ring = 0; ring < (ROWS ? 1 : n_tiles) && ok; ++ring) {
+              const int slot = ring * 2 + (n & 1);
+              if (n >= 2) ok = mbar_wait(bar(Smem::bias_empty + slot), ((n >> 1) - 1) & 1, abort_flag);
+              if (!ok) break;
+              mbar_expect_tx(bar(Smem::bias_full + slot), kBiasBytes);
+              tma_load_5d(smem_base + Smem::bias + slot * kBiasBytes, &P.map_bias, bar(Smem::bias_full + slot), key, first_query(ring),
+                          at.h, P.bias_groups == 1 ? 0 : at.r0, at.b);
+            }
+          }
+          for (int ring = 0; ring < n_rings && ok; ++ring) {
+            const int slot = ring * kStages + st;
+            if (n >= kStages) ok = mbar_wait(bar(Smem::v_empty + slot), (round - 1) & 1, abort_flag);
+            if (!ok) break;
+            mbar_expect_tx(bar(Smem::v_full + slot), kKvBytes);
+            tma_load_5d(smem_base + Smem::v + slot * kKvBytes, &P.map_v, bar(Smem::v_full + slot), 0, at.h, key, row_of(ring), at.b);
+          }
         }
       }
     }
@@ -184,48 +213,62 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
       if (ok) {
         tc_fence_after_sync();
         issue_qk(0);
+        if (PERSIST && KS == 1) mma_commit(bar(Smem::q_empty + w));
       }
-      int st = 0, round = 0;
-      for (int i = 0; i < KS && ok; ++i) {
-        const int next = st + 1 == kStages ? 0 : st + 1, next_round = next == 0 ? round + 1 : round;
-        // the operands of the next score product and of this value product arrive ahead of the probabilities
-        if (i + 1 < KS) ok = mbar_wait(bar(Smem::k_full + ring + next), next_round & 1, abort_flag);
-        if (ok) ok = mbar_wait(bar(Smem::v_full + ring + st), round & 1, abort_flag);
-        // a warpgroup signs off the value steps with dropped keys after clearing their rows
-        if (ok && signoff && i >= full_steps) {
-          const int j = i - full_steps;
-          ok = mbar_wait(bar(Smem::v_ready + ring + j % kStages), (j / kStages) & 1, abort_flag);
-        }
-        if (ok) ok = mbar_wait(bar(Smem::p_full + w), i & 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after_sync();
-        if (i + 1 < KS) issue_qk(next);  // the softmax waits for this one
-        // O[128 x 32] += P[128 x 64] V[64 x 32]; V is MN-major (channel contiguous), 64-byte swizzle:
-        // 8-key groups are 512 bytes apart, each 16-key step advances 1024 bytes.
-        const uint64_t vdesc = vdesc0 + uint64_t((st * kKvBytes) >> 4);
+      int st = 0, round = 0, n = 0;
+      for (int item = int(blockIdx.x), turn = 0; ok && item_there(item, turn); item += int(gridDim.x), ++turn) {
+        for (int i = 0; i < KS && ok; ++i, ++n) {
+          const int next = st + 1 == kStages ? 0 : st + 1, next_round = next == 0 ? round + 1 : round;
+          // the operands of the next score product and of this value product arrive ahead of the probabilities
+          if (i + 1 < KS) ok = mbar_wait(bar(Smem::k_full + ring + next), next_round & 1, abort_flag);
+          if (ok) ok = mbar_wait(bar(Smem::v_full + ring + st), round & 1, abort_flag);
+          // a warpgroup signs off the value steps with dropped keys after clearing their rows
+          if (ok && signoff && i >= full_steps) {
+            const int j = i - full_steps;
+            ok = mbar_wait(bar(Smem::v_ready + ring + j % kStages), (j / kStages) & 1, abort_flag);
+          }
+          if (ok) ok = mbar_wait(bar(Smem::p_full + w), n & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after_sync();
+          if (i + 1 < KS) {
+            issue_qk(next);  // the softmax waits for this one
+            if (PERSIST && i + 2 == KS) mma_commit(bar(Smem::q_empty + w));
+          }
+          // O[128 x 32] += P[128 x 64] V[64 x 32]; V is MN-major (channel contiguous), 64-byte swizzle:
+          // 8-key groups are 512 bytes apart, each 16-key step advances 1024 bytes.
+          const uint64_t vdesc = vdesc0 + uint64_t((st * kKvBytes) >> 4);
 #pragma unroll
-        for (int kk = 0; kk < kKeys / 16; ++kk)
-          mma_ts(o_t, p_t + kk * 8, vdesc + uint64_t(kk * (1024 >> 4)), idesc_pv, (i > 0 || kk > 0) ? 1u : 0u);
-        mma_commit(bar(Smem::pv_done + w));
-        mma_commit(bar(Smem::v_empty + ring + st));
-        st = next;
-        round = next_round;
+          for (int kk = 0; kk < kKeys / 16; ++kk)
+            mma_ts(o_t, p_t + kk * 8, vdesc + uint64_t(kk * (1024 >> 4)), idesc_pv, (i > 0 || kk > 0) ? 1u : 0u);
+          mma_commit(bar(Smem::pv_done + w));
+          mma_commit(bar(Smem::v_empty + ring + st));
+          if (PERSIST && i + 1 == KS && item + int(gridDim.x) < P.items) {  // the first scores of the next item
+            ok = mbar_wait(bar(Smem::q_full + w), (turn + 1) & 1, abort_flag);
+            if (ok) ok = mbar_wait(bar(Smem::k_full + ring + next), next_round & 1, abort_flag);
+            if (!ok) break;
+            tc_fence_after_sync();
+            issue_qk(next);
+            if (KS == 1) mma_commit(bar(Smem::q_empty + w));
+          }
+          st = next;
+          round = next_round;
+        }
       }
     }
   } else if ((warp >> 2) < n_tiles) {
     // ------------------------------------------------------------------ softmax warpgroups
-    const int w = warp >> 2, ring = ROWS ? w : 0, r = row_of(w);
+    const int w = warp >> 2, ring = ROWS ? w : 0;
     const int t = tid & (kTile - 1);
     const uint32_t lane_field = uint32_t((warp & 3) * 32) << 16;
     const uint32_t s_tmem = tmem_base + lane_field + kSCol + w * kKeys;
     const uint32_t p_tmem = tmem_base + lane_field + kPCol + w * (kKeys / 2);
     const uint32_t o_tmem = tmem_base + lane_field + kOCol + w * kHeadDim;
-    const int q_index = first_query(w) + t;
     const float c = P.scale * kLog2e;
     const f32x2 c2 = pack2(c, c), log2e2 = pack2(kLog2e, kLog2e);
     const bool signs_off = needs_signoff(w) && (ROWS || w == 0);
     float ref = -INFINITY, l_run = 0.f;  // reference (base-2 logit) and sum of the row
     bool ok = true;
+    int base = 0;  // steps of the items before
 
     // One step; `drops`: some of its keys are dropped.
     auto step = [&](int i, auto drops) {
@@ -245,12 +288,13 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
         mbar_arrive_warp(bar(Smem::v_ready + ring * kStages + (i - full_steps) % kStages));
       }
 
-      const int bias_slot = (ROWS ? 0 : w * 2) + (i & 1);
+      const int n = base + i;
+      const int bias_slot = (ROWS ? 0 : w * 2) + (n & 1);
       // the phases the step needs are probed together: one round trip to the barrier words when all are complete
-      const bool s_there = mbar_test(bar(Smem::s_full + w), i & 1);
-      const bool bias_there = HAS_BIAS && mbar_test(bar(Smem::bias_full + bias_slot), (i >> 1) & 1);
-      ok = mbar_wait_probed(s_there, bar(Smem::s_full + w), i & 1, abort_flag);
-      if (ok && HAS_BIAS) ok = mbar_wait_probed(bias_there, bar(Smem::bias_full + bias_slot), (i >> 1) & 1, abort_flag);
+      const bool s_there = mbar_test(bar(Smem::s_full + w), n & 1);
+      const bool bias_there = HAS_BIAS && mbar_test(bar(Smem::bias_full + bias_slot), (n >> 1) & 1);
+      ok = mbar_wait_probed(s_there, bar(Smem::s_full + w), n & 1, abort_flag);
+      if (ok && HAS_BIAS) ok = mbar_wait_probed(bias_there, bar(Smem::bias_full + bias_slot), (n >> 1) & 1, abort_flag);
       if (!ok) return;
       tc_fence_after_sync();
       // swizzled row of the bias tile: 16-byte chunk n holds keys 8 n .. 8 n + 7
@@ -310,7 +354,7 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
           l_run *= alpha;
         }
         if (i > 0 && __any_sync(0xffffffffu, raised)) {
-          if (!mbar_wait(bar(Smem::pv_done + w), (i - 1) & 1, abort_flag)) return false;
+          if (!mbar_wait(bar(Smem::pv_done + w), (n - 1) & 1, abort_flag)) return false;
           tc_fence_after_sync();
           uint32_t acc[32];
           tmem_ld32(o_tmem, acc);
@@ -359,7 +403,7 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
           }
           if (chunk & 1) {
             if (!p_free) {  // the previous P V product must have finished with the P columns
-              ok = mbar_wait(bar(Smem::pv_done + w), (i - 1) & 1, abort_flag);
+              ok = mbar_wait(bar(Smem::pv_done + w), (n - 1) & 1, abort_flag);
               tc_fence_after_sync();
               p_free = true;
             }
@@ -387,20 +431,28 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
       mbar_arrive_warp(bar(Smem::p_full + w));
       if (HAS_BIAS) mbar_arrive_warp(bar(Smem::bias_empty + bias_slot));
     };
+    for (int item = int(blockIdx.x), turn = 0; ok && item_there(item, turn); item += int(gridDim.x), ++turn, base += KS) {
+    if (PERSIST) {
+      ref = -INFINITY;
+      l_run = 0.f;
+    }
     int i = 0;
     for (; i < full_steps && ok; ++i) step(i, std::false_type{});
     if (!PLAIN)
       for (; i < KS && ok; ++i) step(i, std::true_type{});
 
+    if (PERSIST) at = fwd_item<ROWS>(P, item);  // (not held through the steps)
+    const int r = row_of(w), h = at.h, b = at.b, q_index = first_query(w) + t;
+    const bool stored = q_index < P.cols && (!PERSIST || !ROWS || at.r0 + w < P.rows);
     // Gated epilogue: the thread's 32 gate logits are requested before the wait for the last product, so that their
     // trip from global memory runs under it (the words are not touched until the output row is ready).
     uint4 gate_words[4] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
-    if (GATED && P.gate_vec16 && ok && q_index < P.cols) {
+    if (GATED && P.gate_vec16 && ok && stored) {
       const T* g = reinterpret_cast<const T*>(P.gate) + b * P.g_sb + int64_t(r) * P.g_sr + int64_t(q_index) * P.g_sc + h * P.g_sh;
 #pragma unroll
       for (int i = 0; i < 4; ++i) gate_words[i] = ldg_v4_here_if(reinterpret_cast<const uint4*>(g) + i, true);
     }
-    if (ok && KS > 0) ok = mbar_wait(bar(Smem::pv_done + w), (KS - 1) & 1, abort_flag);
+    if (ok && KS > 0) ok = mbar_wait(bar(Smem::pv_done + w), (base + KS - 1) & 1, abort_flag);
     if (ok) {
       tc_fence_after_sync();
       uint32_t acc[32];
@@ -411,7 +463,7 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
         tmem_wait_ld();
         tmem_loaded(acc);
       }
-      if (q_index < P.cols) {
+      if (stored) {
         const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
         uint32_t o2[16];
 #pragma unroll
@@ -464,10 +516,11 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
         }
       }
     }
+    }
   }
 }
 
-template <typename T, bool HAS_BIAS, bool GATED, bool ROWS>
+template <typename T, bool HAS_BIAS, bool GATED, bool ROWS, bool PERSIST>
 __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_constant__ FwdParams P) {
   using Smem = FwdSmem<ROWS>;
   extern __shared__ uint8_t smem_raw[];
@@ -486,22 +539,14 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
   const int lane = tid & 31;
   if (device_failed()) return;
 
-  // work decomposition: query item fastest, then head, row (or pair of rows), batch
-  int idx = blockIdx.x;
-  const int qi = idx % P.q_items;
-  idx /= P.q_items;
-  const int h = idx % P.heads;
-  idx /= P.heads;
-  const int row_items = ROWS ? (P.rows + 1) / 2 : P.rows;
-  const int r0 = (idx % row_items) * (ROWS ? 2 : 1);
-  const int b = idx / row_items;
-  const int q0 = qi * (ROWS ? kTile : 2 * kTile);
-  const int n_tiles = (ROWS ? r0 + 1 < P.rows : q0 + kTile < P.cols) ? 2 : 1;
+  const FwdItem at = fwd_item<ROWS>(P, int(blockIdx.x));
+  const int h = at.h, r0 = at.r0, b = at.b, q0 = at.q0;
+  const int n_tiles = PERSIST || (ROWS ? r0 + 1 < P.rows : q0 + kTile < P.cols) ? 2 : 1;
   const int n_rings = ROWS ? n_tiles : 1;
-  const bool has_mask = P.mask != nullptr;
+  const bool has_mask = !PERSIST && P.mask != nullptr;
   // Steps need keep-bits when there is a mask or when the last key step is ragged.
   const bool has_bits = has_mask || (P.cols % kKeys) != 0;
-  auto row_of = [&](int w) { return ROWS ? r0 + w : r0; };
+  auto row_of = [&](int w) { return ROWS ? (PERSIST ? min(r0 + w, P.rows - 1) : r0 + w) : r0; };
 
   if (warp == 8) {
     // The producer warp sets the barriers up, a lane each, and requests the queries: both run beside the look at the mask.
@@ -596,10 +641,9 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   if (!listed && P.cols % kKeys == 0)
-    fwd_walk<T, HAS_BIAS, GATED, ROWS, true>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, h, r0, b, q0, n_tiles, false);
+    fwd_walk<T, HAS_BIAS, GATED, ROWS, PERSIST, true>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, at, n_tiles, false);
   else
-    fwd_walk<T, HAS_BIAS, GATED, ROWS, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, h, r0, b, q0, n_tiles,
-                                              listed);
+    fwd_walk<T, HAS_BIAS, GATED, ROWS, PERSIST, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, at, n_tiles, listed);
   teardown(abort_flag, tmem_base, 9, kFwdTmemCols);
 }
 
@@ -713,11 +757,16 @@ int launch_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse
   P.q_items = (int)ceil_div(p.cols, pair_rows ? kTile : 2 * kTile);
   P.k_steps = (int)ceil_div(p.cols, kKeys);
   P.scale = p.scale;
-  const unsigned grid = (unsigned)(int64_t(p.batch) * (pair_rows ? ceil_div(p.rows, 2) : p.rows) * p.heads * P.q_items);
+  P.items = (int)(int64_t(p.batch) * (pair_rows ? ceil_div(p.rows, 2) : p.rows) * p.heads * P.q_items);
+  // Without a mask, a CTA that has a place on an SM goes on to further items as soon as there are more items than places.  It
+  // pays where items are short: set-up, first copies and output cost as much as three steps (4 steps, N = 256 and two samples:
+  // 76 -> 70 us, 6: 111 -> 107, 8: 240 -> 236 at N = 499; 12: 697 -> 707, the counters of the longer walk cost more).  With a
+  // mask every item has a step list of its own, and its CTA to itself.
+  const int places = 2 * sm_count();
+  const bool persistent = pair_rows && !p.mask && P.k_steps <= 8 && P.items > places;
+  const unsigned grid = (unsigned)(persistent ? places : P.items);
 
   auto launch = [&](auto kernel, int smem) -> int {
-    // the attribute belongs to the (kernel, device) pair: it is set on every launch so that a host thread that
-    // moves between devices never launches without it (the call costs well under a microsecond)
     const int rc = reserve_smem(kernel, smem);
     if (rc) return rc;
     kernel<<<grid, kFwdThreads, smem, stream>>>(P);
@@ -726,13 +775,15 @@ int launch_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse
   };
   auto pick = [&](auto type_tag) -> int {
     using T = decltype(type_tag);
-    auto paired = [&](auto rows) -> int {
-      constexpr bool ROWS = decltype(rows)::value;
+    auto paired = [&](auto rows, auto persist) -> int {
+      constexpr bool ROWS = decltype(rows)::value, PERSIST = decltype(persist)::value;
       constexpr int smem = FwdSmem<ROWS>::bytes;
-      if (gate) return has_bias ? launch(ta_fwd_kernel<T, true, true, ROWS>, smem) : launch(ta_fwd_kernel<T, false, true, ROWS>, smem);
-      return has_bias ? launch(ta_fwd_kernel<T, true, false, ROWS>, smem) : launch(ta_fwd_kernel<T, false, false, ROWS>, smem);
+      if (gate)
+        return has_bias ? launch(ta_fwd_kernel<T, true, true, ROWS, PERSIST>, smem) : launch(ta_fwd_kernel<T, false, true, ROWS, PERSIST>, smem);
+      return has_bias ? launch(ta_fwd_kernel<T, true, false, ROWS, PERSIST>, smem) : launch(ta_fwd_kernel<T, false, false, ROWS, PERSIST>, smem);
     };
-    return pair_rows ? paired(std::true_type{}) : paired(std::false_type{});
+    if (persistent) return paired(std::true_type{}, std::true_type{});
+    return pair_rows ? paired(std::true_type{}, std::false_type{}) : paired(std::false_type{}, std::false_type{});
   };
   return p.dtype == OOPS_TA_BF16 ? pick(__nv_bfloat16{}) : pick(__half{});
 }
