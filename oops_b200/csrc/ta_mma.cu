@@ -259,6 +259,13 @@ __device__ __forceinline__ void set_pair(float (&s)[4], int half, float2 v) {
   s[2 * half] = v.x;
   s[2 * half + 1] = v.y;
 }
+// exp(score * scale + bias - lse), `norm` = -lse.  The logit is made as the forward pass makes it and the norm comes off before
+// the change of base: with log2(e) multiplied into either of them, a row whose logits are all far from zero (a bias of -1e9,
+// or the lowest value of the type) would see the two round apart, or overflow, instead of cancelling.
+__device__ __forceinline__ float2 probability(float2 score, float scale, float2 bias, float2 norm) {
+  const float2 x = __fmul2_rn(__fadd2_rn(__ffma2_rn(score, both(scale), bias), norm), both(kLog2e));
+  return make_float2(ex2(x.x), ex2(x.y));
+}
 // Columns 8 nt + 2 t, + 1 of an accumulator become `value` where their bit is not set.
 template <int NT>
 __device__ __forceinline__ void drop_columns(float (&s)[NT][4], uint64_t bits, int t, float value) {
@@ -355,7 +362,6 @@ __global__ void __launch_bounds__(kThreads, 4) mma_forward_kernel(const MmaProbl
   float o[DP / 8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 #pragma unroll
   for (int i = 0; i < DP / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-  const float c = p.scale * kLog2e;
   copies_wait<1>();
   __syncthreads();
   load_rows<T, DP>(q, Q, warp * 16);
@@ -373,14 +379,14 @@ __global__ void __launch_bounds__(kThreads, 4) mma_forward_kernel(const MmaProbl
       const void* bias = at + 2 * tile_elems<DP>() * 2;
       float s[8][4];
       scores<T, DP, 8>(s, q, K, 0);
-      // base-2 logits, then the online softmax of rows g and g + 8 (a quad of lanes holds a row)
+      // logits, then the online softmax of rows g and g + 8 (a quad of lanes holds a row)
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           float2 add = both(0.f);
-          if (plane) add = __fmul2_rn(bias_pair<T, B32>(bias, warp * 16 + g + 8 * half, nt * 8 + 2 * t), both(kLog2e));
-          set_pair(s[nt], half, __ffma2_rn(pair_of(s[nt], half), both(c), add));
+          if (plane) add = bias_pair<T, B32>(bias, warp * 16 + g + 8 * half, nt * 8 + 2 * t);
+          set_pair(s[nt], half, __ffma2_rn(pair_of(s[nt], half), both(p.scale), add));
         }
       if (bits != ~0ull) drop_columns(s, bits, t, -INFINITY);
       float peak[2] = {-INFINITY, -INFINITY};
@@ -396,7 +402,7 @@ __global__ void __launch_bounds__(kThreads, 4) mma_forward_kernel(const MmaProbl
         const float before = m[half];
         m[half] = fmaxf(before, peak[half]);
         const float base = m[half] == -INFINITY ? 0.f : m[half];
-        shrink[half] = ex2(before - base);
+        shrink[half] = ex2((before - base) * kLog2e);
         peak[half] = base;
         l[half] *= shrink[half];
       }
@@ -405,7 +411,7 @@ __global__ void __launch_bounds__(kThreads, 4) mma_forward_kernel(const MmaProbl
       for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-          const float2 x = __fadd2_rn(pair_of(s[nt], half), both(-peak[half]));
+          const float2 x = __fmul2_rn(__fadd2_rn(pair_of(s[nt], half), both(-peak[half])), both(kLog2e));
           const float2 e = make_float2(ex2(x.x), ex2(x.y));
           set_pair(s[nt], half, e);
           sum[half] = __fadd2_rn(sum[half], e);
@@ -430,7 +436,7 @@ __global__ void __launch_bounds__(kThreads, 4) mma_forward_kernel(const MmaProbl
     const int at = qt * kT + warp * 16 + g + 8 * half;
     const bool some = l[half] > 0.f || l[half] != l[half];
     if (p.lse && t == 0 && at < p.cols)
-      p.lse[((int64_t(b) * p.rows + r) * p.heads + h) * p.cols + at] = some ? (m[half] + __log2f(l[half])) * 0.6931471805599453f : 0.f;
+      p.lse[((int64_t(b) * p.rows + r) * p.heads + h) * p.cols + at] = some ? m[half] + __log2f(l[half]) * 0.6931471805599453f : 0.f;
     l[half] = some ? 1.f / l[half] : 0.f;
   }
   store_rows<T, DP>(p.out, p, b, r, h, qt * kT + warp * 16, o, l[0], l[1]);
@@ -498,13 +504,12 @@ __device__ __forceinline__ void query_gradient(const MmaProblem& p, uint8_t* sme
   for (int half = 0; half < 2; ++half) {
     const int at = row0 + 8 * half;
     const int64_t stat = ((int64_t(b) * p.rows + r) * p.heads + h) * p.cols + at;
-    norm[half] = at < p.cols ? -p.lse[stat] * kLog2e : -INFINITY;
+    norm[half] = at < p.cols ? -p.lse[stat] : -INFINITY;
     delta[half] = at < p.cols ? p.delta[stat] : 0.f;
   }
   float dq[DP / 8][4];
 #pragma unroll
   for (int i = 0; i < DP / 8; ++i) dq[i][0] = dq[i][1] = dq[i][2] = dq[i][3] = 0.f;
-  const float c = p.scale * kLog2e;
   for (int kt = 0; kt < tiles; ++kt) {
     if (kt + 1 < tiles) request(kt + 1);
     copies_commit();
@@ -524,10 +529,10 @@ __device__ __forceinline__ void query_gradient(const MmaProblem& p, uint8_t* sme
       for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-          float2 shift = both(norm[half]);
-          if (plane) shift = __ffma2_rn(bias_pair<T, B32>(bias, warp * 16 + g + 8 * half, col0 + nt * 8 + 2 * t), both(kLog2e), shift);
-          const float2 x = __ffma2_rn(pair_of(s[nt], half), both(c), shift);
-          set_pair(s[nt], half, __fmul2_rn(make_float2(ex2(x.x), ex2(x.y)), __fadd2_rn(pair_of(dp[nt], half), both(-delta[half]))));
+          float2 add = both(0.f);
+          if (plane) add = bias_pair<T, B32>(bias, warp * 16 + g + 8 * half, col0 + nt * 8 + 2 * t);
+          const float2 e = probability(pair_of(s[nt], half), p.scale, add, both(norm[half]));
+          set_pair(s[nt], half, __fmul2_rn(e, __fadd2_rn(pair_of(dp[nt], half), both(-delta[half]))));
         }
       if (bits != 0xffffffffu) drop_columns(s, bits, t, 0.f);
       if (p.dbias && p.bias_groups > 1) {
@@ -551,7 +556,7 @@ __device__ __forceinline__ void query_gradient(const MmaProblem& p, uint8_t* sme
 // dK and dV of 64 keys: S^T = K Q^T, dP^T = V dO^T, dV += P^T dO, dK += dS^T Q.
 template <typename T, int DP, bool B32>
 __device__ __forceinline__ void key_gradient(const MmaProblem& p, uint8_t* smem, int idx) {
-  constexpr int kStage = 2 * tile_elems<DP>() * 2 + bias_bytes<B32>() + 2 * kT * 4;  // Q | dO | bias | -lse*log2e | delta
+  constexpr int kStage = 2 * tile_elems<DP>() * 2 + bias_bytes<B32>() + 2 * kT * 4;  // Q | dO | bias | -lse | delta
   T* K = reinterpret_cast<T*>(smem);
   uint8_t* stages = smem + 2 * tile_elems<DP>() * 2;
   const int tiles = (p.cols + kT - 1) / kT, kt = idx % tiles;
@@ -572,7 +577,7 @@ __device__ __forceinline__ void key_gradient(const MmaProblem& p, uint8_t* smem,
       load_bias<BiasType<T, B32>, bias_pitch<B32>()>(reinterpret_cast<BiasType<T, B32>*>(at), plane, p, qt * kT, kt * kT);
     float* stats = reinterpret_cast<float*>(at + bias_bytes<B32>());
     const int q = qt * kT + (threadIdx.x & 63);
-    if (threadIdx.x < kT) stats[threadIdx.x] = q < p.cols ? -p.lse[stat0 + q] * kLog2e : -INFINITY;
+    if (threadIdx.x < kT) stats[threadIdx.x] = q < p.cols ? -p.lse[stat0 + q] : -INFINITY;
     else stats[threadIdx.x] = q < p.cols ? p.delta[stat0 + q] : 0.f;
   };
   load_tile<T, DP>(K, p.k, p, b, r, h, kt * kT, keep);
@@ -587,7 +592,6 @@ __device__ __forceinline__ void key_gradient(const MmaProblem& p, uint8_t* smem,
   for (int i = 0; i < DP / 8; ++i)
 #pragma unroll
     for (int e = 0; e < 4; ++e) dk[i][e] = dv[i][e] = 0.f;
-  const float c = p.scale * kLog2e;
   for (int qt = 0; qt < tiles; ++qt) {
     if (qt + 1 < tiles) request(qt + 1);
     copies_commit();
@@ -635,8 +639,7 @@ __device__ __forceinline__ void key_gradient(const MmaProblem& p, uint8_t* smem,
         const float2 delta = *reinterpret_cast<const float2*>(stats + kT + col0 + nt * 8 + 2 * t);
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-          const float2 x = __ffma2_rn(pair_of(s[nt], half), both(c), __ffma2_rn(add[nt][half], both(kLog2e), norm));
-          const float2 e = make_float2(ex2(x.x), ex2(x.y));
+          const float2 e = probability(pair_of(s[nt], half), p.scale, add[nt][half], norm);
           set_pair(s[nt], half, e);
           set_pair(dp[nt], half, __fmul2_rn(e, __fadd2_rn(pair_of(dp[nt], half), make_float2(-delta.x, -delta.y))));
         }
@@ -700,7 +703,6 @@ __device__ __forceinline__ void bias_gradient(const MmaProblem& p, uint8_t* smem
   float acc[8][4];
 #pragma unroll
   for (int nt = 0; nt < 8; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-  const float c = p.scale * kLog2e;
   const int row0 = qt * kT + warp * 16 + g;
   if (first < last) request(first);
   copies_commit();
@@ -712,7 +714,7 @@ __device__ __forceinline__ void bias_gradient(const MmaProblem& p, uint8_t* smem
     for (int half = 0; half < 2; ++half) {
       const int at = row0 + 8 * half;
       const int64_t stat = ((int64_t(b) * p.rows + r) * p.heads + h) * p.cols + at;
-      norm[half] = at < p.cols ? -p.lse[stat] * kLog2e : -INFINITY;
+      norm[half] = at < p.cols ? -p.lse[stat] : -INFINITY;
       delta[half] = at < p.cols ? p.delta[stat] : 0.f;
     }
     const uint64_t all = keep_bits(p, p.mask ? p.mask + b * p.m_sb + int64_t(r) * p.m_sr : nullptr, kt * kT);
@@ -731,9 +733,7 @@ __device__ __forceinline__ void bias_gradient(const MmaProblem& p, uint8_t* smem
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
             const Bias* two = add[col0 / 8 + nt][half];
-            const float2 x = __ffma2_rn(pair_of(s[nt], half), both(c),
-                                        __ffma2_rn(make_float2(float(two[0]), float(two[1])), both(kLog2e), both(norm[half])));
-            set_pair(s[nt], half, make_float2(ex2(x.x), ex2(x.y)));
+            set_pair(s[nt], half, probability(pair_of(s[nt], half), p.scale, make_float2(float(two[0]), float(two[1])), both(norm[half])));
             set_pair(dp[nt], half, __fadd2_rn(pair_of(dp[nt], half), both(-delta[half])));
           }
         if (bits != 0xffffffffu) {

@@ -10,6 +10,7 @@ import torch
 
 from oracle import triangle_oracle as oracle
 from oops_b200 import triangle_attention
+from oops_b200.attention.triangle.triangle_attention import layout_agnostic_kernels
 from oops_b200.runtime import cabi
 
 pytestmark = pytest.mark.gpu
@@ -68,3 +69,35 @@ def test_tile_edges(cuda, dtype, rows, cols, heads, dim, bias_kind, mask_kind, l
         assert torch.count_nonzero(out.detach().cpu()[~mask.any(-1)]) == 0
         for grad in grads[1:3]:
             assert torch.count_nonzero(grad.cpu()[~mask]) == 0
+
+
+@pytest.mark.parametrize("dtype,bias_dtype,low", [(torch.bfloat16, torch.bfloat16, -1e9), (torch.bfloat16, torch.bfloat16, None),
+                                                  (torch.bfloat16, torch.float32, -1e9), (torch.float16, torch.float32, None),
+                                                  (torch.float16, torch.float16, None)])
+@pytest.mark.parametrize("dim", [24, 64])
+def test_rows_under_a_low_bias(cuda, dtype, bias_dtype, low, dim):
+    """Half of the queries have every key under a large negative bias (None: the lowest value of its type).  Their logits lose
+    digits in f32 (all of them at -1e9, where the softmax is uniform); results and gradients are those that the
+    layout-agnostic kernels take from the same f32 logits and lse.  Both paths round the result once; the gradients see it
+    through delta (see the top of the file)."""
+    gen = torch.Generator().manual_seed(dim)
+    rows, cols, heads = 5, 70, 2
+    q, k, v, up = (torch.randn(1, rows, cols, heads, dim, generator=gen).to(dtype).to(cuda) for _ in range(4))
+    bias = torch.randn(1, 1, heads, cols, cols, generator=gen).to(bias_dtype)
+    low = torch.finfo(bias_dtype).min if low is None else low
+    bias[..., cols // 2:, :] = low
+
+    def call():
+        leaves = [t.detach().requires_grad_(True) for t in (q, k, v, bias.to(cuda))]
+        out = triangle_attention(*leaves[:3], None, leaves[3])
+        return [out.detach(), *torch.autograd.grad(out, leaves, up)]
+
+    got = call()
+    with layout_agnostic_kernels():
+        want = call()
+    for name, a, b in zip(("out", "dq", "dk", "dv", "dbias"), got, want):
+        bound = 2 * ROUNDING[dtype] * (1 if name == "out" else 8) * max(1.0, float(b.double().abs().max()))
+        assert float((a.double() - b.double()).abs().max()) <= bound, name
+    if low < -2.0**29:
+        uniform = v.double().mean(2, keepdim=True).expand(-1, -1, cols - cols // 2, -1, -1)
+        assert float((got[0][:, :, cols // 2:].double() - uniform).abs().max()) <= ROUNDING[dtype] * float(v.double().abs().max())
