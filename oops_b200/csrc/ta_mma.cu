@@ -6,8 +6,9 @@
 // Calls of this kind are small -- token attention, odd head sizes -- and bound by latency and by the element-wise work
 // on the scores, not by the tensor pipe; fragments go from product to softmax to product in registers, which needs no
 // tensor-memory round trips, no 16-byte rules and no padding of the head size beyond 16.
-// The path it takes over kept probabilities in f32; so does this one to well below the rounding of its results:
-// probabilities and dS enter their products as a pair of 16-bit numbers (value and remainder, 16 mantissa bits for bf16).
+// The path it takes over kept probabilities and dS in f32; here they enter their products as a pair of 16-bit numbers (value
+// and remainder: 16 digits in bf16, 22 in f16), well below the rounding of the results.  f16 lacks the exponents of f32:
+// its probabilities are raised by 2^14 and its rows of dS scaled by a running power of two (RowScale).
 //
 //   forward   CTA = (batch, row, head, 64 queries), four warps of 16 queries, 64-key steps, online softmax.
 //   reverse   one launch, three kinds of CTA: dQ of 64 queries; dK and dV of 64 keys (scores transposed, a warp owns 16
@@ -74,10 +75,14 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+// kWide: the type has the exponents of f32.  kUp: exponent that probabilities are raised by before they are split (f16 ends at
+// 2^-24, which would cut those below 2^-10 of the largest short of 16 digits; 2^14 leaves room below 65504 for rounding).
 template <typename T>
 struct Pair16;
 template <>
 struct Pair16<__nv_bfloat16> {
+  static constexpr bool kWide = true;
+  static constexpr float kUp = 0.f;
   static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&v);
@@ -94,6 +99,8 @@ struct Pair16<__nv_bfloat16> {
 };
 template <>
 struct Pair16<__half> {
+  static constexpr bool kWide = false;
+  static constexpr float kUp = 14.f;
   static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
     const __half2 v = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&v);
@@ -259,13 +266,62 @@ __device__ __forceinline__ void set_pair(float (&s)[4], int half, float2 v) {
   s[2 * half] = v.x;
   s[2 * half + 1] = v.y;
 }
-// exp(score * scale + bias - lse), `norm` = -lse.  The logit is made as the forward pass makes it and the norm comes off before
-// the change of base: with log2(e) multiplied into either of them, a row whose logits are all far from zero (a bias of -1e9,
-// or the lowest value of the type) would see the two round apart, or overflow, instead of cancelling.
-__device__ __forceinline__ float2 probability(float2 score, float scale, float2 bias, float2 norm) {
-  const float2 x = __fmul2_rn(__fadd2_rn(__ffma2_rn(score, both(scale), bias), norm), both(kLog2e));
+// exp(x) 2^kUp
+template <typename T>
+__device__ __forceinline__ float2 ex2_above(float2 x) {
+  x = Pair16<T>::kWide ? __fmul2_rn(x, both(kLog2e)) : __ffma2_rn(x, both(kLog2e), both(Pair16<T>::kUp));
   return make_float2(ex2(x.x), ex2(x.y));
 }
+// exp(score * scale + bias - lse) 2^kUp, `norm` = -lse.  The logit is made as the forward pass makes it and the norm comes off before
+// the change of base: with log2(e) multiplied into either of them, a row whose logits are all far from zero (a bias of -1e9,
+// or the lowest value of the type) would see the two round apart, or overflow, instead of cancelling.
+template <typename T>
+__device__ __forceinline__ float2 probability(float2 score, float scale, float2 bias, float2 norm) {
+  return ex2_above<T>(__fadd2_rn(__ffma2_rn(score, both(scale), bias), norm));
+}
+
+// Power of two that a row of dS is multiplied by before its split into 16-bit numbers, and its accumulator with it.  f16 has
+// neither the exponents that dS reaches under a scaled loss (infinite above 65504) nor those of small gradients (nothing
+// below 2^-25), both of which K or Q can bring back into its range.  The scale starts high and only falls: a step whose largest
+// value would pass 2^15 brings that value to 2^14, and the accumulator along.  What is small against an earlier step loses no
+// more than an f32 sum would: its digits end 2^-38 below that step's largest value.  (bf16 needs none of this.)
+template <typename T>
+struct RowScale {
+  int up[2] = {110, 110};  // exponents, of rows g and g + 8
+
+  template <int DP, int NT>
+  __device__ __forceinline__ void apply(float (&w)[NT][4], float (&acc)[DP / 8][4]) {
+    if constexpr (!Pair16<T>::kWide) {
+      float peak[2] = {0.f, 0.f};
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) peak[i >> 1] = fmaxf(peak[i >> 1], fabsf(w[nt][i]));
+      float factor[2] = {power(up[0]), power(up[1])};
+      if (__any_sync(0xffffffffu, fmaxf(peak[0] * factor[0], peak[1] * factor[1]) > 32768.f)) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          peak[half] = fmaxf(peak[half], __shfl_xor_sync(0xffffffffu, peak[half], 1));
+          peak[half] = fmaxf(peak[half], __shfl_xor_sync(0xffffffffu, peak[half], 2));
+          // exponent of the largest value to 14
+          const int wanted = min(up[half], 14 - (int(__float_as_uint(peak[half]) >> 23) - 127));
+          const float shrink = ex2(float(wanted - up[half]));
+          up[half] = wanted;
+          factor[half] = power(wanted);
+#pragma unroll
+          for (int i = 0; i < DP / 8; ++i) set_pair(acc[i], half, __fmul2_rn(pair_of(acc[i], half), both(shrink)));
+        }
+      }
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) set_pair(w[nt], half, __fmul2_rn(pair_of(w[nt], half), both(factor[half])));
+    }
+  }
+  // What the accumulator's rows are to be multiplied by.
+  __device__ __forceinline__ float undo(int half) const { return Pair16<T>::kWide ? 1.f : power(-up[half]); }
+  static __device__ __forceinline__ float power(int exponent) { return __uint_as_float(uint32_t(exponent + 127) << 23); }
+};
 // Columns 8 nt + 2 t, + 1 of an accumulator become `value` where their bit is not set.
 template <int NT>
 __device__ __forceinline__ void drop_columns(float (&s)[NT][4], uint64_t bits, int t, float value) {
@@ -411,8 +467,7 @@ __global__ void __launch_bounds__(kThreads, 4) mma_forward_kernel(const MmaProbl
       for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-          const float2 x = __fmul2_rn(__fadd2_rn(pair_of(s[nt], half), both(-peak[half])), both(kLog2e));
-          const float2 e = make_float2(ex2(x.x), ex2(x.y));
+          const float2 e = ex2_above<T>(__fadd2_rn(pair_of(s[nt], half), both(-peak[half])));
           set_pair(s[nt], half, e);
           sum[half] = __fadd2_rn(sum[half], e);
         }
@@ -436,7 +491,7 @@ __global__ void __launch_bounds__(kThreads, 4) mma_forward_kernel(const MmaProbl
     const int at = qt * kT + warp * 16 + g + 8 * half;
     const bool some = l[half] > 0.f || l[half] != l[half];
     if (p.lse && t == 0 && at < p.cols)
-      p.lse[((int64_t(b) * p.rows + r) * p.heads + h) * p.cols + at] = some ? m[half] + __log2f(l[half]) * 0.6931471805599453f : 0.f;
+      p.lse[((int64_t(b) * p.rows + r) * p.heads + h) * p.cols + at] = some ? m[half] + (__log2f(l[half]) - Pair16<T>::kUp) * 0.6931471805599453f : 0.f;
     l[half] = some ? 1.f / l[half] : 0.f;
   }
   store_rows<T, DP>(p.out, p, b, r, h, qt * kT + warp * 16, o, l[0], l[1]);
@@ -476,6 +531,7 @@ __global__ void __launch_bounds__(256) mma_delta_kernel(const MmaProblem p, int6
 // dQ of 64 queries: S = Q K^T, dP = dO V^T, dQ += dS K; the per-row bias gradient is dS itself.
 template <typename T, int DP, bool B32>
 __device__ __forceinline__ void query_gradient(const MmaProblem& p, uint8_t* smem, int idx) {
+  constexpr float kDown = Pair16<T>::kWide ? 1.f : 1.f / 16384.f;  // takes 2^kUp back
   constexpr int kStage = 2 * tile_elems<DP>() * 2 + bias_bytes<B32>();
   T* Q = reinterpret_cast<T*>(smem);
   uint8_t* stages = smem + 2 * tile_elems<DP>() * 2;
@@ -510,6 +566,7 @@ __device__ __forceinline__ void query_gradient(const MmaProblem& p, uint8_t* sme
   float dq[DP / 8][4];
 #pragma unroll
   for (int i = 0; i < DP / 8; ++i) dq[i][0] = dq[i][1] = dq[i][2] = dq[i][3] = 0.f;
+  RowScale<T> rows;
   for (int kt = 0; kt < tiles; ++kt) {
     if (kt + 1 < tiles) request(kt + 1);
     copies_commit();
@@ -531,7 +588,7 @@ __device__ __forceinline__ void query_gradient(const MmaProblem& p, uint8_t* sme
         for (int half = 0; half < 2; ++half) {
           float2 add = both(0.f);
           if (plane) add = bias_pair<T, B32>(bias, warp * 16 + g + 8 * half, col0 + nt * 8 + 2 * t);
-          const float2 e = probability(pair_of(s[nt], half), p.scale, add, both(norm[half]));
+          const float2 e = probability<T>(pair_of(s[nt], half), p.scale, add, both(norm[half]));
           set_pair(s[nt], half, __fmul2_rn(e, __fadd2_rn(pair_of(dp[nt], half), both(-delta[half]))));
         }
       if (bits != 0xffffffffu) drop_columns(s, bits, t, 0.f);
@@ -543,19 +600,24 @@ __device__ __forceinline__ void query_gradient(const MmaProblem& p, uint8_t* sme
             const int query = row0 + 8 * (i >> 1), key = kt * kT + col0 + nt * 8 + 2 * t + (i & 1);
             if (query < p.cols && key < p.cols)
               reinterpret_cast<BiasType<T, B32>*>(p.dbias)[b * p.db_sb + int64_t(r) * p.db_sg + h * p.db_sh + int64_t(query) * p.db_sq +
-                                                          int64_t(key) * p.db_sk] = BiasType<T, B32>(s[nt][i]);
+                                                          int64_t(key) * p.db_sk] = BiasType<T, B32>(s[nt][i] * kDown);
           }
       }
-      if (p.dq.ptr) accumulate<T, DP, 4>(dq, s, K, col0);
+      if (p.dq.ptr) {
+        rows.template apply<DP, 4>(s, dq);
+        accumulate<T, DP, 4>(dq, s, K, col0);
+      }
     }
     __syncthreads();
   }
-  if (p.dq.ptr) store_rows<T, DP>(p.dq, p, b, r, h, qt * kT + warp * 16, dq, p.scale, p.scale);
+  if (p.dq.ptr)
+    store_rows<T, DP>(p.dq, p, b, r, h, qt * kT + warp * 16, dq, rows.undo(0) * (p.scale * kDown), rows.undo(1) * (p.scale * kDown));
 }
 
 // dK and dV of 64 keys: S^T = K Q^T, dP^T = V dO^T, dV += P^T dO, dK += dS^T Q.
 template <typename T, int DP, bool B32>
 __device__ __forceinline__ void key_gradient(const MmaProblem& p, uint8_t* smem, int idx) {
+  constexpr float kDown = Pair16<T>::kWide ? 1.f : 1.f / 16384.f;  // takes 2^kUp back
   constexpr int kStage = 2 * tile_elems<DP>() * 2 + bias_bytes<B32>() + 2 * kT * 4;  // Q | dO | bias | -lse | delta
   T* K = reinterpret_cast<T*>(smem);
   uint8_t* stages = smem + 2 * tile_elems<DP>() * 2;
@@ -592,6 +654,7 @@ __device__ __forceinline__ void key_gradient(const MmaProblem& p, uint8_t* smem,
   for (int i = 0; i < DP / 8; ++i)
 #pragma unroll
     for (int e = 0; e < 4; ++e) dk[i][e] = dv[i][e] = 0.f;
+  RowScale<T> rows;
   for (int qt = 0; qt < tiles; ++qt) {
     if (qt + 1 < tiles) request(qt + 1);
     copies_commit();
@@ -639,7 +702,7 @@ __device__ __forceinline__ void key_gradient(const MmaProblem& p, uint8_t* smem,
         const float2 delta = *reinterpret_cast<const float2*>(stats + kT + col0 + nt * 8 + 2 * t);
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-          const float2 e = probability(pair_of(s[nt], half), p.scale, add[nt][half], norm);
+          const float2 e = probability<T>(pair_of(s[nt], half), p.scale, add[nt][half], norm);
           set_pair(s[nt], half, e);
           set_pair(dp[nt], half, __fmul2_rn(e, __fadd2_rn(pair_of(dp[nt], half), make_float2(-delta.x, -delta.y))));
         }
@@ -652,7 +715,10 @@ __device__ __forceinline__ void key_gradient(const MmaProblem& p, uint8_t* smem,
             if (!kept[i >> 1]) s[nt][i] = dp[nt][i] = 0.f;
       }
       if (p.dv.ptr) accumulate<T, DP, 4>(dv, s, Q + tile_elems<DP>(), col0);
-      if (p.dk.ptr) accumulate<T, DP, 4>(dk, dp, Q, col0);
+      if (p.dk.ptr) {
+        rows.template apply<DP, 4>(dp, dk);
+        accumulate<T, DP, 4>(dk, dp, Q, col0);
+      }
     }
     __syncthreads();
   }
@@ -662,13 +728,15 @@ __device__ __forceinline__ void key_gradient(const MmaProblem& p, uint8_t* smem,
 #pragma unroll
     for (int e = 0; e < 4; ++e)
       if (!kept[e >> 1]) dk[i][e] = dv[i][e] = 0.f;
-  if (p.dk.ptr) store_rows<T, DP>(p.dk, p, b, r, h, kt * kT + warp * 16, dk, p.scale, p.scale);
-  if (p.dv.ptr) store_rows<T, DP>(p.dv, p, b, r, h, kt * kT + warp * 16, dv, 1.f, 1.f);
+  if (p.dk.ptr)
+    store_rows<T, DP>(p.dk, p, b, r, h, kt * kT + warp * 16, dk, rows.undo(0) * (p.scale * kDown), rows.undo(1) * (p.scale * kDown));
+  if (p.dv.ptr) store_rows<T, DP>(p.dv, p, b, r, h, kt * kT + warp * 16, dv, kDown, kDown);
 }
 
 // A 64 x 64 tile of the row-shared bias gradient: the sum of dS over the part's rows.
 template <typename T, int DP, bool B32>
 __device__ __forceinline__ void bias_gradient(const MmaProblem& p, uint8_t* smem, int idx) {
+  constexpr float kDown = Pair16<T>::kWide ? 1.f : 1.f / 16384.f;
   constexpr int kStage = 4 * tile_elems<DP>() * 2;  // Q | dO | K | V of a row
   const int tiles = (p.cols + kT - 1) / kT, kt = idx % tiles;
   idx /= tiles;
@@ -733,7 +801,7 @@ __device__ __forceinline__ void bias_gradient(const MmaProblem& p, uint8_t* smem
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
             const Bias* two = add[col0 / 8 + nt][half];
-            set_pair(s[nt], half, probability(pair_of(s[nt], half), p.scale, make_float2(float(two[0]), float(two[1])), both(norm[half])));
+            set_pair(s[nt], half, probability<T>(pair_of(s[nt], half), p.scale, make_float2(float(two[0]), float(two[1])), both(norm[half])));
             set_pair(dp[nt], half, __fadd2_rn(pair_of(dp[nt], half), both(-delta[half])));
           }
         if (bits != 0xffffffffu) {
@@ -758,11 +826,11 @@ __device__ __forceinline__ void bias_gradient(const MmaProblem& p, uint8_t* smem
       const int query = row0 + 8 * (i >> 1), key = kt * kT + nt * 8 + 2 * t + (i & 1);
       if (query >= p.cols || key >= p.cols) continue;
       if (p.num_parts > 1) {
-        p.parts[(((int64_t(part) * p.batch + b) * p.heads + h) * p.cols + query) * p.cols + key] = acc[nt][i];
+        p.parts[(((int64_t(part) * p.batch + b) * p.heads + h) * p.cols + query) * p.cols + key] = acc[nt][i] * kDown;
       } else {
         const int64_t at = b * p.db_sb + h * p.db_sh + int64_t(query) * p.db_sq + int64_t(key) * p.db_sk;
-        if (p.dbias_f32) reinterpret_cast<float*>(p.dbias)[at] = acc[nt][i];
-        else reinterpret_cast<T*>(p.dbias)[at] = T(acc[nt][i]);
+        if (p.dbias_f32) reinterpret_cast<float*>(p.dbias)[at] = acc[nt][i] * kDown;
+        else reinterpret_cast<T*>(p.dbias)[at] = T(acc[nt][i] * kDown);
       }
     }
 }

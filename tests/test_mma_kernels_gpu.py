@@ -101,3 +101,49 @@ def test_rows_under_a_low_bias(cuda, dtype, bias_dtype, low, dim):
     if low < -2.0**29:
         uniform = v.double().mean(2, keepdim=True).expand(-1, -1, cols - cols // 2, -1, -1)
         assert float((got[0][:, :, cols // 2:].double() - uniform).abs().max()) <= ROUNDING[dtype] * float(v.double().abs().max())
+
+
+@pytest.mark.parametrize("dim,cols", [(24, 70), (64, 64), (16, 130)])
+@pytest.mark.parametrize("kind", ["scaled loss", "small gradients", "rising", "light keys"])
+def test_f16_gradients_outside_the_range_of_f16(cuda, kind, dim, cols):
+    """dS above 65504, dS below 2^-25, steps whose dS grows by 2^22 and more from one key or query tile to the next, and
+    probabilities below 2^-25, each with results that f16 holds.  Bounds as at the top of the file, relative to the largest
+    value of the result, and half a unit of the smallest f16 numbers (2^-25) on top."""
+    gen = torch.Generator().manual_seed(dim)
+    rows, heads = 2, 2
+    shape = (1, rows, cols, heads, dim)
+    q, k, v, up = (torch.randn(shape, generator=gen) for _ in range(4))
+    bias = torch.randn(1, 1, heads, cols, cols, generator=gen)
+    checked = (0, 1, 2, 3, 4)
+    if kind == "scaled loss":  # dP = sum_d dO V is some 2^18 (its 2^-3 share still passes 65504), dQ and dK some 2^-8 of it
+        up = 2.0**14 * (1 + 0.1 * up)
+        v = torch.where(torch.rand(1, rows, cols, heads, 1, generator=gen) < 0.5, -1.0, 1.0) * (2 + 0.1 * v)
+        q, k, bias = 2.0**-9 * q, 2.0**-9 * k, bias.clone()
+        bias[..., :2] += 6  # two keys carry most of the weight
+        checked = (1, 2)  # dV passes 65504 where it sums that upstream over all queries
+    elif kind == "small gradients":
+        up, k, q = 2.0**-16 * up, 512 * k, q / 512
+    elif kind == "rising":
+        behind = torch.arange(cols) // 64  # the first tile of keys weighs 2^-29, its queries get an upstream of 2^-14
+        bias[..., behind == 0] -= 20.0 * int(behind.max())
+        up = up * (2.0**-14 * 2.0 ** (22.0 * behind.clamp(max=1)))[:, None, None]
+    else:
+        bias[..., cols // 2:] -= 14
+        up = 1000 * up
+        checked = (3,)
+    q, k, v, up, bias = (t.to(torch.float16) for t in (q, k, v, up, bias))
+    leaves = [t.to(cuda).requires_grad_(True) for t in (q, k, v, bias)]
+    out = triangle_attention(*leaves[:3], None, leaves[3])
+    results = [out.detach(), *torch.autograd.grad(out, leaves, up.to(cuda))]
+    ref = [t.double().requires_grad_(True) for t in (q, k, v, bias)]
+    want = oracle.reference_dense(ref[0], ref[1], ref[2], None, ref[3], compute_dtype=torch.float64)
+    wants = [want.detach(), *torch.autograd.grad(want, ref, up.double())]
+    for i in checked:
+        got, exact = results[i].double().cpu(), wants[i]
+        if kind == "light keys":  # the gradient of the values behind the bias step, on its own scale
+            got, exact = got[:, :, cols // 2:], exact[:, :, cols // 2:]
+        largest = float(exact.abs().max())
+        assert largest < 65504, (i, largest)
+        bound = ROUNDING[torch.float16] * (1 if i == 0 else 8) * largest + 2.0**-25
+        error = float((got - exact).abs().max())
+        assert error <= bound, (("out", "dq", "dk", "dv", "dbias")[i], error, bound, largest)
