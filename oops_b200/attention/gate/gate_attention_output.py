@@ -23,7 +23,7 @@ from torch import Tensor
 from torch.autograd import forward_ad
 from torch.nn import functional as F
 
-from ...runtime import cabi, require_no_forward_mode, require_same_device, unsupported
+from ...runtime import cabi, require_no_forward_mode, require_no_proxy_tracing, require_same_device, tracing, unsupported
 from ...runtime.native import native
 from ...runtime.nested_tensor import is_nested
 from ..triangle import function as _function
@@ -58,6 +58,34 @@ def _check_gate_output(attention: Tensor, single: Tensor, gate_weight: Tensor, o
 def _run_gate(attention5: Tensor, gate5: Tensor, out5: Tensor) -> None:
     """``out5 = sigmoid(gate5) * attention5`` on ``(B, R, C, H, D)`` views."""
     native().run_gate(attention5, gate5, out5)
+
+
+class _TracedGate(torch.autograd.Function):
+    """``sigmoid(gate5) * attention5`` on ``(B, R, C, H, D)`` values, as ``torch.jit.trace`` can record it."""
+
+    @staticmethod
+    def forward(ctx, attention5, gate5):
+        attention5, gate5 = _unit_inner(attention5), _unit_inner(gate5)
+        out5 = torch.empty(gate5.shape, dtype=gate5.dtype, device=gate5.device)
+        _run_gate(attention5, gate5, out5)
+        ctx.save_for_backward(attention5, gate5)
+        return out5
+
+    @staticmethod
+    def backward(ctx, grad5):
+        attention5, gate5 = (_unit_inner(t) for t in ctx.saved_tensors)
+        d_attention, d_gate = (torch.empty(t.shape, dtype=t.dtype, device=t.device) for t in (attention5, gate5))
+        native().run_gate_backward(attention5, gate5, _unit_inner(grad5.resolve_neg().to(gate5.dtype)), d_attention, d_gate)
+        return d_attention, d_gate
+
+
+def _sigmoid_gate(attention4: Tensor, gate: Tensor) -> Tensor:
+    """``sigmoid(gate) * attention`` for ``(B, H, Q, D)`` attention and ``(B, Q, H * D)`` gate."""
+    if not tracing():
+        return native().sigmoid_gate(attention4, gate)
+    heads, head_size = int(attention4.shape[1]), int(attention4.shape[3])
+    gated5 = _TracedGate.apply(attention4.permute(0, 2, 1, 3).unsqueeze(1), gate.unflatten(-1, (heads, head_size)).unsqueeze(1))
+    return gated5.squeeze(1).flatten(-2)
 
 
 def gate_attention_output(attention, single, gate_weight: Tensor, output_weight: Tensor):
@@ -97,11 +125,12 @@ def gate_attention_output(attention, single, gate_weight: Tensor, output_weight:
             _OPERATOR, "requires CUDA float16/bfloat16/float32 attention and single of one dtype",
             attention=f"{tuple(attention.shape)} {attention.dtype} {attention.device}", single_dtype=single.dtype,
         )
+    require_no_proxy_tracing(_OPERATOR)
     lead = tuple(attention.shape[:-3])
     attention4 = attention.reshape(-1, *attention.shape[-3:]) if len(lead) != 1 else attention
     single3 = single.reshape(-1, *single.shape[-2:]) if len(lead) != 1 else single
     gate = F.linear(single3, gate_weight.to(single3.dtype))
-    gated = native().sigmoid_gate(attention4, gate)
+    gated = _sigmoid_gate(attention4, gate)
     result = F.linear(gated, output_weight.to(gated.dtype))
     return result.reshape(*lead, *result.shape[-2:]) if len(lead) != 1 else result
 
@@ -150,7 +179,11 @@ def triangle_attention_gated(query: Tensor, key: Tensor, value: Tensor, gate: Te
         bias5 = triangle_bias.resolve_neg().resolve_conj().contiguous()
         if bias5.element_size() == 2 and cols % 8 != 0:
             bias5 = torch.nn.functional.pad(bias5, (0, -cols % 8))[..., :cols]
-    scale = head_size**-0.5 if scale is None else float(scale)
+    scale = float(head_size**-0.5 if scale is None else scale)
+    require_no_proxy_tracing(operator)
+    if tracing():
+        plain = _function.TracedAttention.apply(q5, k5, v5, mask3, bias5, scale, _function.DenseGeometry(), _flags())
+        return _TracedGate.apply(plain, g5)
     return native().gated_attend(q5, k5, v5, g5, mask3, bias5, scale, _flags())
 
 

@@ -26,7 +26,7 @@ from typing import List, Optional, Sequence, Tuple
 import torch
 from torch import Tensor
 
-from ...runtime import cabi, unsupported
+from ...runtime import cabi, proxy_tracing, tracing, unsupported
 from ...runtime.native import native
 
 
@@ -151,7 +151,7 @@ def run_backward(
 # FakeTensorMode, where tensors carry no data pointers.  Takes the place of the reference's
 # `ooperators::_triangle_attention_forward/_backward` ops and their `register_fake` shape functions
 # (oops/attention/triangle/triton/ops.py:156-366).  Eager calls keep the compiled
-# autograd node (native.cpp).
+# autograd node (native.cpp), and torch.jit.trace gets a Python one.
 # ----------------------------------------------------------------------------------------------
 
 
@@ -177,6 +177,40 @@ def decode_geometry(code: Sequence[int]):
                           bias_row_strides=rows)
 
 
+def _reverse_of_saved(geometry, grad_out, query, key, value, mask, bias, out, lse, scale, flags, need):
+    """``run_backward`` on what was saved for it, whose strides hooks or a recorded graph may have changed."""
+    query, key, value, out = (geometry.canonical_pair(t) for t in (query, key, value, out))
+    grad_out = geometry.canonical_pair(grad_out.resolve_neg().to(query.dtype))
+    if bias is not None:
+        bias = geometry.canonical_bias(bias)
+    if mask is not None and not isinstance(geometry, DenseGeometry):
+        mask = mask.contiguous()
+    return run_backward(geometry, grad_out, query, key, value, mask, bias, out, lse.contiguous(), scale, flags, need)
+
+
+class TracedAttention(torch.autograd.Function):
+    """The node as ``torch.jit.trace`` can record it."""
+
+    @staticmethod
+    def forward(ctx, query, key, value, mask, bias, scale, geometry, flags):
+        ctx.set_materialize_grads(False)
+        wanted = any(ctx.needs_input_grad[i] for i in (0, 1, 2, 4))
+        out, lse = run_forward(geometry, query, key, value, mask, bias, scale, flags, want_lse=wanted)
+        if wanted:
+            ctx.save_for_backward(query, key, value, mask, bias, out, lse)
+            ctx.scale, ctx.geometry, ctx.flags = scale, geometry, flags
+        return out
+
+    @staticmethod
+    def backward(ctx, grad_out):
+        if grad_out is None:
+            return (None,) * 8
+        query, key, value, mask, bias, out, lse = ctx.saved_tensors
+        need = tuple(ctx.needs_input_grad[i] for i in (0, 1, 2, 4))
+        dq, dk, dv, dbias = _reverse_of_saved(ctx.geometry, grad_out, query, key, value, mask, bias, out, lse, ctx.scale, ctx.flags, need)
+        return dq, dk, dv, None, dbias, None, None, None
+
+
 @torch.library.custom_op("oops_b200::triangle_attention_forward", mutates_args=())
 def _forward_op(
     query: Tensor, key: Tensor, value: Tensor, mask: Optional[Tensor], bias: Optional[Tensor], scale: float,
@@ -200,16 +234,8 @@ def _backward_op(
     grad_out: Tensor, query: Tensor, key: Tensor, value: Tensor, mask: Optional[Tensor], bias: Optional[Tensor],
     out: Tensor, lse: Tensor, scale: float, geometry: List[int], flags: int, need: List[bool],
 ) -> Tuple[Tensor, Tensor, Tensor, Tensor]:
-    geom = decode_geometry(geometry)
-    query_given, key_given, value_given, bias_given = query, key, value, bias
-    query, key, value, out = (geom.canonical_pair(t) for t in (query, key, value, out))
-    grad_out = geom.canonical_pair(grad_out.resolve_neg().to(query.dtype))
-    if bias is not None:
-        bias = geom.canonical_bias(bias)
-    if mask is not None and not isinstance(geom, DenseGeometry):
-        mask = mask.contiguous()
-    given = (query_given, key_given, value_given, bias_given)
-    grads = run_backward(geom, grad_out, query, key, value, mask, bias, out, lse.contiguous(), scale, flags, need)
+    given = (query, key, value, bias)
+    grads = _reverse_of_saved(decode_geometry(geometry), grad_out, query, key, value, mask, bias, out, lse, scale, flags, need)
     empty = torch.empty(0, dtype=query.dtype, device=query.device)
 
     def laid_out_like(grad, operand):
@@ -255,7 +281,7 @@ _forward_op.register_autograd(_dispatch_backward, setup_context=_dispatch_setup)
 
 
 def _needs_dispatcher(*tensors: Optional[Tensor]) -> bool:
-    if torch.compiler.is_compiling():
+    if torch.compiler.is_compiling() or proxy_tracing():
         return True
     from torch._subclasses.fake_tensor import is_fake
 
@@ -269,4 +295,6 @@ def apply(query, key, value, mask, bias, scale, geometry, flags=0) -> Tensor:
         return out
     if torch._C._functorch.peek_interpreter_stack() is not None:
         raise unsupported("triangle_attention", "does not support torch.func transforms")
+    if tracing():
+        return TracedAttention.apply(query, key, value, mask, bias, float(scale), geometry, flags)
     return native().attend(query, key, value, mask, bias, scale, encode_geometry(geometry), flags)

@@ -12,6 +12,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include <atomic>
@@ -77,9 +78,9 @@ bool requires_grad(const MaybeTensor& t) { return t.has_value() && t->defined() 
 void* data_of(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 void* data_of(const MaybeTensor& t) { return t.has_value() ? data_of(*t) : nullptr; }
 
-// No dispatch mode or transform is active that would have to see the operations of a call.
+// No dispatch mode, transform or tracer is active that would have to see the operations of a call.
 bool plain_context() {
-  return !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
+  return !c10::impl::TorchDispatchModeTLS::any_modes_set() && !torch::jit::tracer::isTracing() &&
          !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
 }
 
@@ -1097,6 +1098,22 @@ PYBIND11_MODULE(_native, m) {
   }, NoGil());
   m.def("sigmoid_gate", [](const Tensor& attention, const Tensor& gate) { return Tensor(GateFunction::apply(attention, gate)); }, NoGil());
   m.def("run_gate", &run_gate, NoGil());
+  m.def("run_gate_backward", &run_gate_backward, NoGil());
+  m.def("layer_norm_forward", [or_empty](const Tensor& x, const MaybeTensor& weight, const MaybeTensor& bias, double eps) {
+    TORCH_CHECK(norm_operands_fit(x, weight, bias, x.dim() ? x.size(-1) : 0), "layer_norm operands do not fit");
+    const Tensor w = or_empty(weight), b = or_empty(bias);
+    Normed n = norm_forward(rows_of(x, x.size(-1)), w.defined() ? w.contiguous() : w, b.defined() ? b.contiguous() : b, eps, true, x.sizes());
+    return std::make_tuple(n.y, n.stats);
+  }, NoGil());
+  m.def("layer_norm_backward", [or_empty](const Tensor& dy, const Tensor& x, const MaybeTensor& weight, const MaybeTensor& bias,
+                                          const Tensor& stats, const std::vector<bool>& need) {
+    const Tensor w = or_empty(weight), rows = rows_of(x, x.size(-1));
+    const auto affine = w.defined() ? w.scalar_type() : bias.has_value() ? bias->scalar_type() : x.scalar_type();
+    NormGradients g = norm_backward(rows_of(dy.resolve_neg(), x.size(-1)), rows, w.defined() ? w.contiguous() : w, stats.contiguous(), affine,
+                                    need[0], need[1], need[2]);
+    auto maybe = [](const Tensor& t) { return t.defined() ? MaybeTensor(t) : MaybeTensor(); };
+    return std::make_tuple(g.dx.defined() ? MaybeTensor(g.dx.view(x.sizes())) : MaybeTensor(), maybe(g.dweight), maybe(g.dbias));
+  }, NoGil());
   m.def("pair_update", [](const Tensor& pair, const MaybeTensor& mask, bool outgoing, double in_eps, double out_eps,
                           const std::vector<Tensor>& parameters, const std::vector<int64_t>& bias_of) {
     bool wanted = pair.requires_grad();

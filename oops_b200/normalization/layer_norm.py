@@ -18,7 +18,7 @@ import torch
 from torch import Tensor
 from torch.autograd import forward_ad
 
-from ..runtime import require_no_forward_mode, require_same_device, unsupported
+from ..runtime import require_no_forward_mode, require_no_proxy_tracing, require_same_device, tracing, unsupported
 from ..runtime.native import native
 from ..runtime.nested_tensor import is_nested
 
@@ -41,10 +41,29 @@ def layer_norm(input, normalized_shape, weight: Optional[Tensor] = None, bias: O
     require_same_device(_NAME, input, weight, bias)
     check_admission(input, normalized_shape, weight, bias)
     input, weight, bias = (t if t is None else t.resolve_neg() for t in (input, weight, bias))
+    require_no_proxy_tracing(_NAME)
+    if tracing():
+        return _TracedLayerNorm.apply(input, weight, bias, float(eps))
     out = native().layer_norm(input, input.shape[-1], weight, bias, eps)
     if out is None:  # served layouts behind a transform or a tensor subclass
         raise unsupported(_NAME, "does not support torch.func transforms or dispatching tensor subclasses")
     return out
+
+
+class _TracedLayerNorm(torch.autograd.Function):
+    """The node as ``torch.jit.trace`` can record it."""
+
+    @staticmethod
+    def forward(ctx, x, weight, bias, eps):
+        out, stats = native().layer_norm_forward(x, weight, bias, eps)
+        ctx.save_for_backward(x, weight, bias, stats)
+        return out
+
+    @staticmethod
+    def backward(ctx, grad_out):
+        x, weight, bias, stats = ctx.saved_tensors
+        need = [ctx.needs_input_grad[0], weight is not None and ctx.needs_input_grad[1], bias is not None and ctx.needs_input_grad[2]]
+        return (*native().layer_norm_backward(grad_out, x, weight, bias, stats, need), None)
 
 
 def check_admission(input, normalized_shape, weight: Optional[Tensor], bias: Optional[Tensor]) -> None:

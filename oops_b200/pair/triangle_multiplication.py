@@ -25,7 +25,7 @@ from torch import Tensor
 from torch.nn import functional as F
 
 from ..normalization.layer_norm import check_admission, layer_norm
-from ..runtime import require_no_forward_mode, require_same_device, unsupported
+from ..runtime import proxy_tracing, require_no_forward_mode, require_same_device, tracing, unsupported
 from ..runtime.native import native
 from ..runtime.nested_tensor import is_nested
 
@@ -112,7 +112,7 @@ def _fused_serves(pair: Tensor, mask: Optional[Tensor], hidden: int, parameters)
         pair.dtype in _DTYPES and pair.numel() > 0 and 0 < hidden <= _MAX_HIDDEN
         and type(pair) in (Tensor, torch.nn.Parameter)
         and not torch.compiler.is_compiling() and not torch.is_autocast_enabled("cuda")
-        and torch._C._functorch.peek_interpreter_stack() is None
+        and torch._C._functorch.peek_interpreter_stack() is None and not tracing() and not proxy_tracing()
         and all(p is None or (p.is_floating_point() and p.dim() in (1, 2)) for p in parameters)
         and (mask is None or (not mask.requires_grad and not mask.is_complex() and mask.dim() < pair.dim()
                               and all(own in (1, want) for own, want in zip(reversed(mask.shape), reversed(pair.shape[:-1])))))

@@ -76,7 +76,22 @@ def require_no_forward_mode(operator: str, *tensors: Tensor | None) -> None:
         )
 
 
+def tracing() -> bool:
+    """True under ``torch.jit.trace``, which records Python autograd functions but not the compiled nodes."""
+    return torch._C._get_tracing_state() is not None
+
+
+def proxy_tracing() -> bool:
+    """True under ``make_fx``, which records dispatcher operators only: what a kernel launch writes would be lost."""
+    return torch._C._get_dispatch_mode(torch._C._TorchDispatchModeKey.PROXY) is not None
+
+
+def require_no_proxy_tracing(operator: str) -> None:
+    if proxy_tracing():
+        raise unsupported(operator, "cannot be recorded by make_fx")
+
+
 __all__ = [
-    "unsupported", "is_compiling", "require_same_device", "require_shape", "forward_mode_active",
+    "unsupported", "tracing", "proxy_tracing", "require_no_proxy_tracing", "is_compiling", "require_same_device", "require_shape", "forward_mode_active",
     "require_no_forward_mode",
 ]
