@@ -795,12 +795,17 @@ bool norm_operands_fit(const Tensor& x, const MaybeTensor& weight, const MaybeTe
   return true;
 }
 
-std::optional<Tensor> layer_norm(const Tensor& x, int64_t width, const MaybeTensor& weight, const MaybeTensor& bias, double eps) {
-  if (!plain_context() || !norm_operands_fit(x, weight, bias, width)) return std::nullopt;
+// Without a look at the context: under a dispatch mode the allocations go through it, the launches do not.
+std::optional<Tensor> layer_norm_node(const Tensor& x, int64_t width, const MaybeTensor& weight, const MaybeTensor& bias, double eps) {
+  if (!norm_operands_fit(x, weight, bias, width)) return std::nullopt;
   if (at::GradMode::is_enabled() && (x.requires_grad() || requires_grad(weight) || requires_grad(bias)))
     return LayerNormFunction::apply(x, weight, bias, eps);
   const Tensor w = weight.has_value() ? weight->contiguous() : Tensor(), b = bias.has_value() ? bias->contiguous() : Tensor();
   return norm_forward(rows_of(x, width), w, b, eps, false, x.sizes()).y;
+}
+
+std::optional<Tensor> layer_norm(const Tensor& x, int64_t width, const MaybeTensor& weight, const MaybeTensor& bias, double eps) {
+  return plain_context() ? layer_norm_node(x, width, weight, bias, eps) : std::nullopt;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1099,6 +1104,7 @@ PYBIND11_MODULE(_native, m) {
   m.def("sigmoid_gate", [](const Tensor& attention, const Tensor& gate) { return Tensor(GateFunction::apply(attention, gate)); }, NoGil());
   m.def("run_gate", &run_gate, NoGil());
   m.def("run_gate_backward", &run_gate_backward, NoGil());
+  m.def("layer_norm_node", &layer_norm_node, NoGil());
   m.def("layer_norm_forward", [or_empty](const Tensor& x, const MaybeTensor& weight, const MaybeTensor& bias, double eps) {
     TORCH_CHECK(norm_operands_fit(x, weight, bias, x.dim() ? x.size(-1) : 0), "layer_norm operands do not fit");
     const Tensor w = or_empty(weight), b = or_empty(bias);

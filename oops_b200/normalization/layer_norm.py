@@ -44,7 +44,9 @@ def layer_norm(input, normalized_shape, weight: Optional[Tensor] = None, bias: O
     require_no_proxy_tracing(_NAME)
     if tracing():
         return _TracedLayerNorm.apply(input, weight, bias, float(eps))
-    out = native().layer_norm(input, input.shape[-1], weight, bias, eps)
+    out = None
+    if torch._C._functorch.peek_interpreter_stack() is None:
+        out = native().layer_norm_node(input, input.shape[-1], weight, bias, eps)
     if out is None:  # served layouts behind a transform or a tensor subclass
         raise unsupported(_NAME, "does not support torch.func transforms or dispatching tensor subclasses")
     return out

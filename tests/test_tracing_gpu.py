@@ -1,9 +1,10 @@
 """Calls that something records: ``torch.jit.trace`` and ``make_fx`` must take the operator itself into their graph, not the
-memory that its launch filled while they looked on, or refuse."""
+memory that its launch filled while they looked on, or refuse; a dispatch mode that only looks on changes nothing."""
 
 import pytest
 import torch
 from torch.fx.experimental.proxy_tensor import make_fx
+from torch.utils._python_dispatch import TorchDispatchMode
 
 import oops_b200 as oops
 
@@ -62,3 +63,17 @@ def test_make_fx_records_the_operator_or_refuses(cuda, name):
     else:
         with pytest.raises(oops.OOpsUnsupportedError):
             make_fx(f)(*first)
+
+
+@pytest.mark.parametrize("name", OPERATORS)
+def test_a_dispatch_mode_may_look_on(cuda, name):
+    class Looker(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    values, f = operands(name, cuda, 1.0)
+    want = with_grads(f, values)
+    with Looker():
+        got = with_grads(f, values)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
