@@ -129,7 +129,7 @@ def gate_attention_output(attention, single, gate_weight: Tensor, output_weight:
     lead = tuple(attention.shape[:-3])
     attention4 = attention.reshape(-1, *attention.shape[-3:]) if len(lead) != 1 else attention
     single3 = single.reshape(-1, *single.shape[-2:]) if len(lead) != 1 else single
-    gate = F.linear(single3, gate_weight.to(single3.dtype))
+    gate = F.linear(single3, gate_weight.to(single3.dtype)).to(attention.dtype)  # (autocast has a type of its own)
     gated = _sigmoid_gate(attention4, gate)
     result = F.linear(gated, output_weight.to(gated.dtype))
     return result.reshape(*lead, *result.shape[-2:]) if len(lead) != 1 else result

@@ -445,7 +445,21 @@ std::optional<Tensor> dense_attention(const Tensor& query, const Tensor& key, co
 
 oops_ta_pair dense_pair(const Tensor& t) { return pair_of(Geometry(), Sample(), t); }
 
+// The kernels read every operand of a gate as the attention's type and shape.
+void check_gate_operands(const Tensor& attention, std::initializer_list<const Tensor*> others) {
+  for (const Tensor* t : others)
+    TORCH_CHECK(!t->defined() || (t->scalar_type() == attention.scalar_type() && t->sizes() == attention.sizes()),
+                "gate_attention_output gate kernel: operands of ", attention.scalar_type(), " ", attention.sizes(), " and ",
+                t->scalar_type(), " ", t->sizes());
+}
+
+// Library products inside a node keep their operands' type, whatever region the reverse pass is called from.
+struct NoAutocast {
+  c10::impl::ExcludeDispatchKeyGuard guard{c10::DispatchKeySet(c10::DispatchKey::AutocastCUDA)};
+};
+
 void run_gate(const Tensor& attention, const Tensor& gate, const Tensor& out) {
+  check_gate_operands(attention, {&gate, &out});
   const c10::cuda::CUDAGuard guard(attention.device());
   const oops_ta_pair a = dense_pair(attention), g = dense_pair(gate), o = dense_pair(out);
   check_status(oops_ta_gate_forward(dtype_code(attention.scalar_type()), attention.size(0), attention.size(1), attention.size(2),
@@ -454,6 +468,7 @@ void run_gate(const Tensor& attention, const Tensor& gate, const Tensor& out) {
 }
 
 void run_gate_backward(const Tensor& attention, const Tensor& gate, const Tensor& dout, const Tensor& dattention, const Tensor& dgate) {
+  check_gate_operands(attention, {&gate, &dout, &dattention, &dgate});
   const c10::cuda::CUDAGuard guard(attention.device());
   const oops_ta_pair a = dense_pair(attention), g = dense_pair(gate), u = dense_pair(dout), da = dense_pair(dattention),
                      dg = dense_pair(dgate);
@@ -577,6 +592,7 @@ struct GateOutputFunction : Function<GateOutputFunction> {
     return at::_unsafe_view(at::linear(gated, wo), shape);
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grad_outputs) {
+    const NoAutocast no_autocast;
     variable_list saved = ctx->get_saved_variables();
     const Tensor values = unit_inner(saved[0]), rows = saved[1], wg = saved[2], wo = saved[3], gate = saved[4].contiguous(), gated = saved[5];
     const std::vector<int64_t> types = ctx->saved_data["types"].toIntVector();
@@ -889,6 +905,7 @@ struct UpdateFunction : Function<UpdateFunction> {
   }
 
   static variable_list backward(AutogradContext* ctx, const variable_list& grad_outputs) {
+    const NoAutocast no_autocast;
     const std::vector<int64_t> dims = ctx->saved_data["dims"].toIntVector(), bias_of = ctx->saved_data["bias_of"].toIntVector(),
                                types = ctx->saved_data["types"].toIntVector();
     // inputs: pair, mask, outgoing, in_eps, out_eps, parameters..., bias_of
