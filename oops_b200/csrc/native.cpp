@@ -995,12 +995,14 @@ struct UpdateFunction : Function<UpdateFunction> {
 
 MaybeTensor maybe_tensor(PyObject* o) { return o == Py_None ? MaybeTensor() : MaybeTensor(THPVariable_Unpack(o)); }
 bool tensor_or_none(PyObject* o) { return o == Py_None || THPVariable_Check(o); }
-std::optional<double> maybe_double(PyObject* o) {
-  if (o == Py_None) return std::nullopt;
+bool is_number(PyObject* o) { return PyFloat_Check(o) || PyLong_Check(o); }  // anything else is converted, or refused, in Python
+double number(PyObject* o) {
   const double v = PyFloat_AsDouble(o);
   if (v == -1.0 && PyErr_Occurred()) throw python_error();
   return v;
 }
+std::optional<double> maybe_number(PyObject* o) { return o == Py_None ? std::nullopt : std::optional<double>(number(o)); }
+bool number_or_none(PyObject* o) { return o == Py_None || is_number(o); }
 
 PyObject* wrap(std::optional<Tensor>&& t) {
   if (!t.has_value()) Py_RETURN_NONE;
@@ -1012,11 +1014,12 @@ template <auto Attention>
 PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 7, "attention takes 7 arguments");
-  if (!THPVariable_Check(a[0]) || !THPVariable_Check(a[1]) || !THPVariable_Check(a[2]) || !tensor_or_none(a[3]) || !tensor_or_none(a[4]))
+  if (!THPVariable_Check(a[0]) || !THPVariable_Check(a[1]) || !THPVariable_Check(a[2]) || !tensor_or_none(a[3]) || !tensor_or_none(a[4]) ||
+      !number_or_none(a[5]))
     Py_RETURN_NONE;
   const Tensor &q = THPVariable_Unpack(a[0]), &k = THPVariable_Unpack(a[1]), &v = THPVariable_Unpack(a[2]);
   const MaybeTensor mask = maybe_tensor(a[3]), bias = maybe_tensor(a[4]);
-  const std::optional<double> scale = maybe_double(a[5]);
+  const std::optional<double> scale = maybe_number(a[5]);
   const int64_t flags = PyLong_AsLongLong(a[6]);
   std::optional<Tensor> out;
   {
@@ -1033,10 +1036,10 @@ PyObject* py_gated_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   TORCH_CHECK(n == 8, "triangle_attention_gated takes 8 arguments");
   for (int i = 0; i < 4; ++i)
     if (!THPVariable_Check(a[i])) Py_RETURN_NONE;
-  if (!tensor_or_none(a[4]) || !tensor_or_none(a[5])) Py_RETURN_NONE;
+  if (!tensor_or_none(a[4]) || !tensor_or_none(a[5]) || !number_or_none(a[6])) Py_RETURN_NONE;
   const Tensor &q = THPVariable_Unpack(a[0]), &k = THPVariable_Unpack(a[1]), &v = THPVariable_Unpack(a[2]), &g = THPVariable_Unpack(a[3]);
   const MaybeTensor mask = maybe_tensor(a[4]), bias = maybe_tensor(a[5]);
-  const std::optional<double> scale = maybe_double(a[6]);
+  const std::optional<double> scale = maybe_number(a[6]);
   const int64_t flags = PyLong_AsLongLong(a[7]);
   std::optional<Tensor> out;
   {
@@ -1068,11 +1071,13 @@ PyObject* py_gate_output(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_layer_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 5, "layer_norm takes 5 arguments");
-  if (!THPVariable_Check(a[0]) || !PyLong_Check(a[1]) || !tensor_or_none(a[2]) || !tensor_or_none(a[3])) Py_RETURN_NONE;
+  if (!THPVariable_Check(a[0]) || !PyLong_Check(a[1]) || !tensor_or_none(a[2]) || !tensor_or_none(a[3]) || !is_number(a[4])) Py_RETURN_NONE;
   const Tensor& x = THPVariable_Unpack(a[0]);
-  const int64_t width = PyLong_AsLongLong(a[1]);
+  int overflow = 0;
+  const int64_t width = PyLong_AsLongLongAndOverflow(a[1], &overflow);
+  if (overflow) Py_RETURN_NONE;
   const MaybeTensor weight = maybe_tensor(a[2]), bias = maybe_tensor(a[3]);
-  const double eps = *maybe_double(a[4]);
+  const double eps = number(a[4]);
   std::optional<Tensor> out;
   {
     py::gil_scoped_release no_gil;

@@ -42,8 +42,9 @@ def layer_norm(input, normalized_shape, weight: Optional[Tensor] = None, bias: O
     check_admission(input, normalized_shape, weight, bias)
     input, weight, bias = (t if t is None else t.resolve_neg() for t in (input, weight, bias))
     require_no_proxy_tracing(_NAME)
+    eps = float(eps)
     if tracing():
-        return _TracedLayerNorm.apply(input, weight, bias, float(eps))
+        return _TracedLayerNorm.apply(input, weight, bias, eps)
     out = None
     if torch._C._functorch.peek_interpreter_stack() is None:
         out = native().layer_norm_node(input, input.shape[-1], weight, bias, eps)
