@@ -458,13 +458,16 @@ struct NoAutocast {
   c10::impl::ExcludeDispatchKeyGuard guard{c10::DispatchKeySet(c10::DispatchKey::AutocastCUDA)};
 };
 
+void check_gate_status(int status) {
+  TORCH_CHECK(status == OOPS_TA_OK, "gate_attention_output gate kernel failed: ", oops_ta_status_string(status), ": ", oops_ta_last_error());
+}
+
 void run_gate(const Tensor& attention, const Tensor& gate, const Tensor& out) {
   check_gate_operands(attention, {&gate, &out});
   const c10::cuda::CUDAGuard guard(attention.device());
   const oops_ta_pair a = dense_pair(attention), g = dense_pair(gate), o = dense_pair(out);
-  check_status(oops_ta_gate_forward(dtype_code(attention.scalar_type()), attention.size(0), attention.size(1), attention.size(2),
-                                    attention.size(3), attention.size(4), &a, &g, &o, current_stream(attention)),
-               "gate_attention_output gate kernel");
+  check_gate_status(oops_ta_gate_forward(dtype_code(attention.scalar_type()), attention.size(0), attention.size(1), attention.size(2),
+                                    attention.size(3), attention.size(4), &a, &g, &o, current_stream(attention)));
 }
 
 void run_gate_backward(const Tensor& attention, const Tensor& gate, const Tensor& dout, const Tensor& dattention, const Tensor& dgate) {
@@ -472,9 +475,8 @@ void run_gate_backward(const Tensor& attention, const Tensor& gate, const Tensor
   const c10::cuda::CUDAGuard guard(attention.device());
   const oops_ta_pair a = dense_pair(attention), g = dense_pair(gate), u = dense_pair(dout), da = dense_pair(dattention),
                      dg = dense_pair(dgate);
-  check_status(oops_ta_gate_backward(dtype_code(attention.scalar_type()), attention.size(0), attention.size(1), attention.size(2),
-                                     attention.size(3), attention.size(4), &a, &g, &u, &da, &dg, current_stream(attention)),
-               "gate_attention_output gate kernel");
+  check_gate_status(oops_ta_gate_backward(dtype_code(attention.scalar_type()), attention.size(0), attention.size(1), attention.size(2),
+                                     attention.size(3), attention.size(4), &a, &g, &u, &da, &dg, current_stream(attention)));
 }
 
 // (B, H, Q, D) values as the C ABI's (B, 1, Q, H, D), and (B, Q, H * D) rows as the same.

@@ -103,3 +103,10 @@ def test_gated_triangle_attention_against_the_oracles(cuda, dtype, n, dim, bias_
     assert torch.equal(fused, got.detach())
     composed = (torch.sigmoid(leaves[3].detach().float()) * plain.float()).to(dtype)
     parity.check(f"{tag} fused vs composed", fused, composed.double(), 2.0 ** -7 * max(1.0, float(composed.abs().max())) if dtype is not torch.float32 else 1e-5)
+
+
+def test_an_empty_call_is_a_runtime_error(cuda):
+    attention, single = torch.zeros(0, 2, 8, 16, device=cuda), torch.zeros(0, 8, 24, device=cuda)
+    with pytest.raises(RuntimeError, match="gate kernel failed") as raised:
+        gate_attention_output(attention, single, torch.zeros(32, 24, device=cuda), torch.zeros(24, 32, device=cuda))
+    assert not isinstance(raised.value, ValueError)
