@@ -109,7 +109,7 @@ _MAX_HIDDEN = 512  # a tile of the channel-norm kernel holds all channels of its
 def _fused_serves(pair: Tensor, mask: Optional[Tensor], hidden: int, parameters) -> bool:
     """Plain eager calls with floating-point parameters; a mask that takes no gradient and expands to the pair's cells."""
     return (
-        pair.dtype in _DTYPES and pair.numel() > 0 and 0 < hidden <= _MAX_HIDDEN
+        pair.dtype in _DTYPES and pair.numel() > 0 and 0 < hidden <= _MAX_HIDDEN and _fits_a_launch(pair)
         and type(pair) in (Tensor, torch.nn.Parameter)
         and not torch.compiler.is_compiling() and not torch.is_autocast_enabled("cuda")
         and torch._C._functorch.peek_interpreter_stack() is None and not tracing() and not proxy_tracing()
@@ -117,3 +117,9 @@ def _fused_serves(pair: Tensor, mask: Optional[Tensor], hidden: int, parameters)
         and (mask is None or (not mask.requires_grad and not mask.is_complex() and mask.dim() < pair.dim()
                               and all(own in (1, want) for own, want in zip(reversed(mask.shape), reversed(pair.shape[:-1])))))
     )
+
+
+def _fits_a_launch(pair: Tensor) -> bool:
+    """Prefix elements are the second grid axis of the passes; cells of a padded plane are counted in 32 bits."""
+    tokens, channels = pair.shape[-2:]
+    return pair.numel() // (tokens * tokens * channels) <= 65535 and (-(-tokens // 8) * 8) ** 2 < 2**31

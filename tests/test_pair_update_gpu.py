@@ -39,3 +39,17 @@ def test_tile_edges(dtype, prefix, tokens, channels, hidden, direction, masked):
         # one token normalises a rank-one update: its gradients are differences of equal terms, judged absolutely
         bound = TOL[dtype] * max(1.0, float(ref.detach().abs().max()))
         assert float((got.detach().double().cpu() - ref.detach()).abs().max()) <= bound, name
+
+
+def test_more_prefix_elements_than_a_grid_axis_holds(cuda):
+    gen = torch.Generator().manual_seed(7)
+    weights = {k: w.to(cuda) for k, w in _weights(gen, 8, 8, True).items()}
+    pair = torch.randn(65537, 9, 9, 8, generator=gen).to(cuda).requires_grad_(True)
+    out = oops.triangle_multiplication(pair, **weights)
+    (grad,) = torch.autograd.grad(out.sum(), pair)
+    for part in (slice(0, 3), slice(65530, 65537)):
+        piece = pair.detach()[part].requires_grad_(True)
+        want = oops.triangle_multiplication(piece, **weights)
+        (want_grad,) = torch.autograd.grad(want.sum(), piece)
+        for got, exact in ((out[part], want), (grad[part], want_grad)):
+            assert float((got - exact).abs().max()) <= TOL[torch.float32] * max(1.0, float(exact.abs().max()))

@@ -1,0 +1,13 @@
+"""Which calls of the triangle multiplicative update take the fused passes and which are composed from single operations."""
+
+import pytest
+import torch
+
+from oops_b200.pair.triangle_multiplication import _fused_serves
+
+
+@pytest.mark.parametrize("shape,hidden,serves", [((65535, 16, 16, 8), 8, True), ((65536, 16, 16, 8), 8, False), ((256, 256, 16, 16, 8), 8, False),
+                                                 ((46336, 46336, 1), 1, True), ((46344, 46344, 1), 1, False), ((46344, 46344, 1), 512, False),
+                                                 ((16, 16, 8), 512, True), ((16, 16, 8), 513, False)])
+def test_launch_limits(shape, hidden, serves):
+    assert _fused_serves(torch.empty(shape, device="meta"), None, hidden, ()) is serves
