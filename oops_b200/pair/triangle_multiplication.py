@@ -68,7 +68,7 @@ def triangle_multiplication(pair, pair_mask: Optional[Tensor] = None, *, directi
 
     projections = (left_gate_weight, left_value_weight, right_gate_weight, right_value_weight, output_gate_weight, output_weight)
     biases = (left_gate_bias, left_value_bias, right_gate_bias, right_value_bias, output_gate_bias, output_bias)
-    if _fused_serves(pair, pair_mask, hidden, (*projections, *biases)):
+    if _fused_serves(pair, pair_mask, hidden, projections, biases):
         for width, weight, bias in ((channels, input_norm_weight, input_norm_bias), (hidden, output_norm_weight, output_norm_bias)):
             if weight.dtype is not bias.dtype or weight.dtype not in (pair.dtype, torch.float32):
                 check_admission(pair.new_empty(width), width, weight, bias)  # raises
@@ -106,14 +106,16 @@ _DTYPES = (torch.float32, torch.float16, torch.bfloat16)
 _MAX_HIDDEN = 512  # a tile of the channel-norm kernel holds all channels of its tokens in shared memory
 
 
-def _fused_serves(pair: Tensor, mask: Optional[Tensor], hidden: int, parameters) -> bool:
-    """Plain eager calls with floating-point parameters; a mask that takes no gradient and expands to the pair's cells."""
+def _fused_serves(pair: Tensor, mask: Optional[Tensor], hidden: int, projections, biases) -> bool:
+    """Plain eager calls with floating-point parameters, one bias value per projection row (what broadcasts otherwise is
+    composed); a mask that takes no gradient and expands to the pair's cells."""
     return (
         pair.dtype in _DTYPES and pair.numel() > 0 and 0 < hidden <= _MAX_HIDDEN and _fits_a_launch(pair)
         and type(pair) in (Tensor, torch.nn.Parameter)
         and not torch.compiler.is_compiling() and not torch.is_autocast_enabled("cuda")
         and torch._C._functorch.peek_interpreter_stack() is None and not tracing() and not proxy_tracing()
-        and all(p is None or (p.is_floating_point() and p.dim() in (1, 2)) for p in parameters)
+        and all(p.is_floating_point() for p in projections)
+        and all(b is None or (b.is_floating_point() and b.shape == p.shape[:1]) for p, b in zip(projections, biases))
         and (mask is None or (not mask.requires_grad and not mask.is_complex() and mask.dim() < pair.dim()
                               and all(own in (1, want) for own, want in zip(reversed(mask.shape), reversed(pair.shape[:-1])))))
     )

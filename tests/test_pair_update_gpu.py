@@ -53,3 +53,16 @@ def test_more_prefix_elements_than_a_grid_axis_holds(cuda):
         (want_grad,) = torch.autograd.grad(want.sum(), piece)
         for got, exact in ((out[part], want), (grad[part], want_grad)):
             assert float((got - exact).abs().max()) <= TOL[torch.float32] * max(1.0, float(exact.abs().max()))
+
+
+@pytest.mark.parametrize("name,rows", [("left_gate_bias", 24), ("output_bias", 16), ("output_gate_bias", 16)])
+def test_projection_biases_that_broadcast(cuda, name, rows):
+    gen = torch.Generator().manual_seed(8)
+    weights = {k: w.to(cuda) for k, w in _weights(gen, 16, 24, False).items()}
+    pair, value = torch.randn(1, 12, 12, 16, generator=gen).to(cuda), torch.randn(1, generator=gen).to(cuda)
+    want = oops.triangle_multiplication(pair, **weights, **{name: value.expand(rows).contiguous()})
+    for bias in (value, value.expand(1, rows)):
+        got = oops.triangle_multiplication(pair, **weights, **{name: bias})
+        assert float((got - want).abs().max()) <= TOL[torch.float32] * max(1.0, float(want.abs().max()))
+    with pytest.raises(RuntimeError):
+        oops.triangle_multiplication(pair, **weights, **{name: value.expand(rows + 1)})

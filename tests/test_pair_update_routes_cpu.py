@@ -10,4 +10,11 @@ from oops_b200.pair.triangle_multiplication import _fused_serves
                                                  ((46336, 46336, 1), 1, True), ((46344, 46344, 1), 1, False), ((46344, 46344, 1), 512, False),
                                                  ((16, 16, 8), 512, True), ((16, 16, 8), 513, False)])
 def test_launch_limits(shape, hidden, serves):
-    assert _fused_serves(torch.empty(shape, device="meta"), None, hidden, ()) is serves
+    assert _fused_serves(torch.empty(shape, device="meta"), None, hidden, (), ()) is serves
+
+
+@pytest.mark.parametrize("shape,serves", [((8,), True), ((1,), False), ((1, 8), False), ((7,), False), ((16, 8), False)])
+def test_bias_shapes(shape, serves):
+    projections = [torch.empty(8, 4) for _ in range(6)]
+    biases = [None] * 5 + [torch.empty(shape)]
+    assert _fused_serves(torch.empty(1, 16, 16, 4), None, 8, projections, biases) is serves
