@@ -174,7 +174,7 @@ uint64_t oops_ta_backward_workspace_bytes(const oops_ta_problem* problem, const 
   if (validate(problem, false) || !grads) return 0;
   if (!force_generic(problem) && tensor_backward_applies(*problem, grads))
     return tensor_backward_workspace(*problem, *grads);
-  if (!force_generic(problem) && f32_backward_applies(*problem)) return f32_backward_workspace(*problem, *grads);
+  if (!force_generic(problem) && f32_backward_applies(*problem, *grads)) return f32_backward_workspace(*problem, *grads);
   if (!force_generic(problem) && mma_applies(*problem)) return mma_backward_workspace(*problem, *grads);
   return generic_backward_workspace(*problem, *grads);
 }
@@ -399,7 +399,7 @@ int oops_ta_backward(const oops_ta_problem* problem, const oops_ta_pair* out, co
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (!force_generic(problem) && tensor_backward_applies(*problem, grads))
     return tensor_backward(*problem, *out, *dout, lse, *grads, s);
-  if (!force_generic(problem) && f32_backward_applies(*problem)) return f32_backward(*problem, *out, *dout, lse, *grads, s);
+  if (!force_generic(problem) && f32_backward_applies(*problem, *grads)) return f32_backward(*problem, *out, *dout, lse, *grads, s);
   if (!force_generic(problem) && mma_applies(*problem)) return mma_backward(*problem, *out, *dout, lse, *grads, s);
   return generic_backward(*problem, *out, *dout, lse, *grads, s);
 }

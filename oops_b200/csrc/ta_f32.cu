@@ -613,15 +613,21 @@ bool wants_ds(const oops_ta_problem& p, const oops_ta_grads& g) { return g.dbias
 
 }  // namespace
 
-// Head sizes above 64 would not leave room for two CTAs per SM: they stay with the kernels that keep logits in memory, as
-// does the reverse pass of fewer rows and heads than half the SMs (its CTA owns a whole row).
+// Head sizes above 64 would not leave room for two CTAs per SM: they stay with the kernels that keep logits in memory.
 bool f32_forward_applies(const oops_ta_problem& p) {
   return p.dtype == OOPS_TA_F32 && p.head_dim <= 64 &&
          int64_t(p.batch) * p.rows * p.heads * ceil_div(p.cols, kT) <= 0x7fffffffll;
 }
 
-bool f32_backward_applies(const oops_ta_problem& p) {
-  return f32_forward_applies(p) && int64_t(p.batch) * p.rows * p.heads >= 74;
+// A CTA of the reverse pass owns a whole row of a head, so a launch must have enough of those; rows that the dS budget splits
+// over launches count by the launch, and pay for every launch's tail.  Against the kernels that split every row into tiles,
+// reverse call with 4 heads and a shared-bias gradient (16 / 32 / 64 channels): 112 CTAs a launch (768 columns) take 0.65 /
+// 0.78 / 0.89 of their time, 80 (896) 0.85 / 1.03 / 1.18, 48 (1152) 1.36 / 1.66 / 1.91, 16 (2048) 2.6 / 3.2 / 3.9.  In one launch
+// 76 take 0.78 (512 columns), 74 0.75 (1024 columns, no bias gradient).
+bool f32_backward_applies(const oops_ta_problem& p, const oops_ta_grads& g) {
+  if (!f32_forward_applies(p)) return false;
+  const int rows = wants_ds(p, g) ? ds_block_rows(p) : p.rows;
+  return int64_t(p.batch) * rows * p.heads >= (rows < p.rows ? 96 : 74);
 }
 
 uint64_t f32_backward_workspace(const oops_ta_problem& p, const oops_ta_grads& g) {

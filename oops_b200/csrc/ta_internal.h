@@ -34,7 +34,7 @@ int generic_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oo
 
 // FFMA kernels that keep the scores on chip (f32, head_dim <= 64, any strides).
 bool f32_forward_applies(const oops_ta_problem& p);
-bool f32_backward_applies(const oops_ta_problem& p);
+bool f32_backward_applies(const oops_ta_problem& p, const oops_ta_grads& g);
 uint64_t f32_backward_workspace(const oops_ta_problem& p, const oops_ta_grads& g);
 int f32_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, cudaStream_t stream);
 int f32_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_ta_pair& dout, const float* lse,

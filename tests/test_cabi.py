@@ -97,3 +97,23 @@ def test_kernel_selection_is_host_only():
     forced = _tensor_problem()
     forced.flags = cabi.FLAG_FORCE_GENERIC
     assert lib.oops_ta_uses_tensor_path(ctypes.byref(forced), 0) == 0
+
+
+def test_f32_reverse_pass_counts_the_rows_of_a_launch():
+    """The one-pass f32 kernel gives a CTA a whole row and head, and a launch as many rows as its scratch holds: with too
+    few of them, whatever the whole call has, the kernels that split rows into tiles take the call (told by their scratch)."""
+    lib = cabi.library()
+
+    def one_pass(rows, cols, heads, bias_gradient, batch=1):
+        g = cabi.Grads()
+        g.dq.ptr = g.dk.ptr = g.dv.ptr = 0x10000
+        g.dbias = 0x20000 if bias_gradient else None
+        sizes = []
+        for flags in (0, cabi.FLAG_FORCE_GENERIC):
+            p = _problem(dtype=cabi.F32, bias_dtype=cabi.F32, batch=batch, rows=rows, cols=cols, heads=heads, bias_groups=1, flags=flags)
+            sizes.append(lib.oops_ta_backward_workspace_bytes(ctypes.byref(p), ctypes.byref(g)))
+        return sizes[0] != sizes[1]
+
+    assert one_pass(64, 64, 4, True) and one_pass(768, 768, 4, True) and one_pass(2048, 2048, 4, False)
+    assert not one_pass(18, 512, 4, True) and one_pass(19, 512, 4, True)
+    assert not one_pass(1024, 1024, 4, True) and not one_pass(2048, 2048, 4, True) and not one_pass(2048, 2048, 16, True, batch=2)

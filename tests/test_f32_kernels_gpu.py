@@ -8,6 +8,7 @@ import torch
 
 from oracle import triangle_oracle as oracle
 from oops_b200 import triangle_attention
+from oops_b200.runtime import cabi
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +40,21 @@ def test_tile_edges(cuda, cols, dim, bias_kind, mask_kind, swapped):
     if mask is not None:
         empty = ~mask.any(-1)
         assert torch.count_nonzero(out.detach().cpu()[empty]) == 0
+
+
+def test_bias_gradient_over_several_launches(cuda):
+    """832 columns of 4 heads: 24 rows of dS fit the scratch of a launch, so 30 rows take two, and the second adds."""
+    gen = torch.Generator().manual_seed(1)
+    rows, cols, heads, dim = 30, 832, 4, 8
+    q, k, v, up = (torch.randn(1, rows, cols, heads, dim, generator=gen) for _ in range(4))
+    bias = torch.randn(1, 1, heads, cols, cols, generator=gen)
+    leaves = [t.to(cuda).requires_grad_(True) for t in (q, k, v, bias)]
+    out = triangle_attention(*leaves[:3], None, leaves[3])
+    before = cabi.launch_count()
+    grads = torch.autograd.grad(out, leaves, up.to(cuda))
+    assert cabi.launch_count() - before == 4  # a reverse pass and a sum per launch
+    ref = [t.to(cuda, torch.float64).requires_grad_(True) for t in (q, k, v, bias)]
+    want = oracle.reference_dense(*ref[:3], None, ref[3], compute_dtype=torch.float64)
+    for name, got, exact in zip(("dq", "dk", "dv", "dbias"), grads, torch.autograd.grad(want, ref, up.to(cuda, torch.float64))):
+        bound = (cols + dim + rows) * 2.0**-22 * max(1.0, float(exact.abs().max()))
+        assert float((got.double() - exact).abs().max()) <= bound, name
