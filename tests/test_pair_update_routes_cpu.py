@@ -18,3 +18,10 @@ def test_bias_shapes(shape, serves):
     projections = [torch.empty(8, 4) for _ in range(6)]
     biases = [None] * 5 + [torch.empty(shape)]
     assert _fused_serves(torch.empty(1, 16, 16, 4), None, 8, projections, biases) is serves
+
+
+@pytest.mark.parametrize("dtype,prefix,tokens,serves", [(torch.bfloat16, 4096, 2, False), (torch.bfloat16, 4096, 6, False), (torch.bfloat16, 4096, 3, True),
+                                                        (torch.bfloat16, 4096, 1, False), (torch.bfloat16, 4096, 8, True), (torch.bfloat16, 1024, 2, True),
+                                                        (torch.float32, 4096, 4, False), (torch.float32, 4096, 5, True), (torch.float32, 16, 1, True)])
+def test_many_grids_that_are_mostly_padding(dtype, prefix, tokens, serves):
+    assert _fused_serves(torch.empty(prefix, tokens, tokens, 64, dtype=dtype, device="meta"), None, 64, (), ()) is serves
