@@ -1144,8 +1144,12 @@ PYBIND11_MODULE(_native, m) {
     auto maybe = [](const Tensor& t) { return t.defined() ? MaybeTensor(t) : MaybeTensor(); };
     return std::make_tuple(g.dx.defined() ? MaybeTensor(g.dx.view(x.sizes())) : MaybeTensor(), maybe(g.dweight), maybe(g.dbias));
   }, NoGil());
-  m.def("pair_update", [](const Tensor& pair, const MaybeTensor& mask, bool outgoing, double in_eps, double out_eps,
-                          const std::vector<Tensor>& parameters, const std::vector<int64_t>& bias_of) {
+  m.def("pair_update", [](const Tensor& pair_in, const MaybeTensor& mask_in, bool outgoing, double in_eps, double out_eps,
+                          std::vector<Tensor> parameters, const std::vector<int64_t>& bias_of) {
+    // the passes read memory, which a lazily negated view does not describe
+    const Tensor pair = pair_in.resolve_neg();
+    const MaybeTensor mask = mask_in.has_value() ? MaybeTensor(mask_in->resolve_neg()) : mask_in;
+    for (Tensor& p : parameters) p = p.resolve_neg();
     bool wanted = pair.requires_grad();
     for (const Tensor& p : parameters) wanted = wanted || p.requires_grad();
     if (at::GradMode::is_enabled() && wanted)

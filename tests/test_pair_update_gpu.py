@@ -66,3 +66,12 @@ def test_projection_biases_that_broadcast(cuda, name, rows):
         assert float((got - want).abs().max()) <= TOL[torch.float32] * max(1.0, float(want.abs().max()))
     with pytest.raises(RuntimeError):
         oops.triangle_multiplication(pair, **weights, **{name: value.expand(rows + 1)})
+
+
+def test_lazily_negated_operands(cuda):
+    gen = torch.Generator().manual_seed(9)
+    pair, mask = torch.randn(1, 12, 12, 16, generator=gen).to(cuda), torch.rand(1, 12, 12, generator=gen).to(cuda)
+    weights = {k: w.to(cuda) for k, w in _weights(gen, 16, 24, True).items()}
+    want = oops.triangle_multiplication(-pair, -mask, **{k: -w for k, w in weights.items()})
+    got = oops.triangle_multiplication(torch._neg_view(pair), torch._neg_view(mask), **{k: torch._neg_view(w) for k, w in weights.items()})
+    assert torch.equal(got, want)
