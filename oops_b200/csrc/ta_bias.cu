@@ -14,27 +14,30 @@ struct BiasRows {
   const uint16_t* src;
   uint16_t* dst;
   int64_t s_b, s_g, s_h, s_q, s_k;
-  uint32_t words, heads, cols, groups, total;  // words of a row
+  uint32_t words, heads, cols, groups;  // words of a row
+  uint64_t total;
   int heads_inner;
 };
 
+// I counts words: 32 bits up to 64 GB of them.
+template <typename I>
 __global__ void __launch_bounds__(256) bias_rows_kernel(const BiasRows p) {
-  uint32_t i = blockIdx.x * 256u + threadIdx.x;
-  if (i >= p.total) return;
+  I i = I(blockIdx.x) * 256u + threadIdx.x;
+  if (i >= I(p.total)) return;
   uint32_t h = 0, word;
   if (p.heads_inner) {
-    h = i % p.heads;
+    h = uint32_t(i % p.heads);
     i /= p.heads;
   }
-  word = i % p.words;
+  word = uint32_t(i % p.words);
   i /= p.words;
-  const uint32_t q = i % p.cols;
+  const uint32_t q = uint32_t(i % p.cols);
   i /= p.cols;
   if (!p.heads_inner) {
-    h = i % p.heads;
+    h = uint32_t(i % p.heads);
     i /= p.heads;
   }
-  const uint32_t g = i % p.groups, b = i / p.groups;
+  const uint32_t g = uint32_t(i % p.groups), b = uint32_t(i / p.groups);
   const uint16_t* src = p.src + b * p.s_b + g * p.s_g + h * p.s_h + q * p.s_q;
   uint32_t packed[4] = {0, 0, 0, 0};
 #pragma unroll
@@ -64,9 +67,10 @@ int bias_rows(int batch, int groups, int heads, int cols, const void* src, const
   p.heads_inner = heads > 1 && p.s_h < p.s_k;
   const int64_t total = int64_t(batch) * groups * heads * cols * p.words;
   if (total == 0) return OOPS_TA_OK;
-  if (total > 0xffffff00ll) return fail(OOPS_TA_LIMIT_EXCEEDED, "bias of %lld words", (long long)total);
-  p.total = uint32_t(total);
-  bias_rows_kernel<<<(unsigned)ceil_div(total, 256), 256, 0, stream>>>(p);
+  if (ceil_div(total, 256) > 0x7fffffffll) return fail(OOPS_TA_LIMIT_EXCEEDED, "bias of %lld words", (long long)total);
+  p.total = uint64_t(total);
+  const auto kernel = total > 0xffffff00ll ? bias_rows_kernel<uint64_t> : bias_rows_kernel<uint32_t>;
+  kernel<<<(unsigned)ceil_div(total, 256), 256, 0, stream>>>(p);
   count_launch();
   return check_launch("bias rows");
 }

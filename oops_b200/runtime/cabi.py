@@ -39,7 +39,7 @@ EXPORTS = (
     "oops_ta_forward_gated", "oops_ta_gate_forward", "oops_ta_gate_backward", "oops_ta_pair_mask_packed", "oops_ta_layer_norm_backward_workspace_bytes", "oops_ta_layer_norm_forward",
     "oops_ta_layer_norm_backward", "oops_ta_pair_gate_forward", "oops_ta_pair_gate_backward",
     "oops_ta_channel_norm_forward", "oops_ta_channel_norm_backward_workspace_bytes", "oops_ta_channel_norm_backward",
-    "oops_ta_output_gate_forward", "oops_ta_output_gate_backward",
+    "oops_ta_output_gate_forward", "oops_ta_output_gate_backward", "oops_ta_bias_rows",
 )
 
 
@@ -137,6 +137,8 @@ def library() -> ctypes.CDLL:
     lib.oops_ta_output_gate_backward.restype = c_int
     lib.oops_ta_output_gate_backward.argtypes = ([c_int, c_int64, c_int32] + [c_void_p] * 3 + [c_int64] + [c_void_p] * 2
                                                  + [c_int64, c_void_p])
+    lib.oops_ta_bias_rows.restype = c_int
+    lib.oops_ta_bias_rows.argtypes = [c_int32] * 4 + [c_void_p, POINTER(c_int64), c_void_p, c_void_p]
     lib.oops_ta_selftest_wait_limit.restype = c_int
     lib.oops_ta_selftest_wait_limit.argtypes = [c_void_p]
     lib.oops_ta_device_status.restype = c_int

@@ -43,3 +43,21 @@ def test_gradient_keeps_its_place(cuda, n, layout):
     up = torch.randn(q.shape, generator=gen).to(cuda, torch.bfloat16)
     results = [torch.autograd.grad(triangle_attention(q, k, v, None, b), b, up)[0] for b in (bias, padded)]
     assert results[0].shape == bias.shape and torch.equal(*results)
+
+
+def test_more_words_than_32_bits_count(cuda):
+    """2^32 words: one plane of 16384 x 16384 values seen by 128 heads."""
+    torch.cuda.empty_cache()
+    heads, n = 128, 16384
+    if torch.cuda.mem_get_info(cuda)[0] < heads * n * n * 2 + (8 << 30):
+        pytest.skip("needs 72 GB of device memory")
+    plane = torch.randint(-(2**15), 2**15, (n, n), dtype=torch.int16, device=cuda)
+    rows = torch.empty(heads, n, n, dtype=torch.int16, device=cuda)
+    rows[-1, -1].fill_(-1)
+    stream = torch.cuda.current_stream(cuda).cuda_stream
+    assert cabi.library().oops_ta_bias_rows(1, 1, heads, n, ctypes.c_void_p(plane.data_ptr()), (ctypes.c_int64 * 5)(0, 0, 0, n, 1),
+                                            ctypes.c_void_p(rows.data_ptr()), ctypes.c_void_p(stream)) == 0
+    for head in (0, 63, 127):
+        assert torch.equal(rows[head], plane)
+    del rows
+    torch.cuda.empty_cache()
