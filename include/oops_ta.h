@@ -73,12 +73,13 @@ typedef enum oops_ta_status {
                                          gradients of several calls -- the row shards of one problem on several
                                          GPUs -- and round once.  No counterpart in the reference, which has no
                                          multi-GPU path.                                                         */
-#define OOPS_TA_FLAG_REUSE_DELTA 16u  /* reverse pass: the workspace already holds delta = rowsum(O * dO) from an
-                                         earlier oops_ta_backward call on the same problem, output, upstream
-                                         gradient and workspace; it is not recomputed.  Lets a caller split one
-                                         reverse pass into two calls (bias gradient first, so that its exchange
-                                         overlaps the other gradients) without paying for delta twice.  Honoured by
-                                         the tcgen05 kernels; the layout-agnostic kernels recompute.            */
+#define OOPS_TA_FLAG_REUSE_DELTA 16u  /* reverse pass: the workspace already starts with delta = rowsum(O * dO) (f32, [batch][rows]
+                                         [heads][cols]) from an earlier oops_ta_backward call on the same problem,
+                                         output, upstream gradient and workspace; it is not recomputed.  Lets a caller
+                                         split one reverse pass into two calls (bias gradient first, so that its exchange
+                                         overlaps the other gradients) without paying for delta twice.  Honoured by the
+                                         tcgen05 kernels and the register-level 16-bit kernels; the f32 and the
+                                         layout-agnostic kernels recompute.                                          */
 
 typedef struct oops_ta_pair {
   void* ptr;

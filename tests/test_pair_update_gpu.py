@@ -51,7 +51,7 @@ def test_more_prefix_elements_than_a_grid_axis_holds(cuda):
         piece = pair.detach()[part].requires_grad_(True)
         want = oops.triangle_multiplication(piece, **weights)
         (want_grad,) = torch.autograd.grad(want.sum(), piece)
-        for got, exact in ((out[part], want), (grad[part], want_grad)):
+        for got, exact in ((out.detach()[part], want.detach()), (grad[part], want_grad)):
             assert float((got - exact).abs().max()) <= TOL[torch.float32] * max(1.0, float(exact.abs().max()))
 
 
