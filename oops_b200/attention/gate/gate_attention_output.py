@@ -23,7 +23,7 @@ from torch import Tensor
 from torch.autograd import forward_ad
 from torch.nn import functional as F
 
-from ...runtime import cabi, require_no_forward_mode, require_no_proxy_tracing, require_same_device, tracing, unsupported
+from ...runtime import cabi, require_no_forward_mode, require_no_proxy_tracing, require_same_device, result_like, tracing, unsupported
 from ...runtime.native import native
 from ...runtime.nested_tensor import is_nested
 from ..triangle import function as _function
@@ -82,7 +82,7 @@ class _TracedGate(torch.autograd.Function):
 def _sigmoid_gate(attention4: Tensor, gate: Tensor) -> Tensor:
     """``sigmoid(gate) * attention`` for ``(B, H, Q, D)`` attention and ``(B, Q, H * D)`` gate."""
     if not tracing():
-        return native().sigmoid_gate(attention4, gate)
+        return result_like(native().sigmoid_gate(attention4, gate), gate)
     heads, head_size = int(attention4.shape[1]), int(attention4.shape[3])
     gated5 = _TracedGate.apply(attention4.permute(0, 2, 1, 3).unsqueeze(1), gate.unflatten(-1, (heads, head_size)).unsqueeze(1))
     return gated5.squeeze(1).flatten(-2)

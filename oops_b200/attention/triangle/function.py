@@ -26,7 +26,7 @@ from typing import List, Optional, Sequence, Tuple
 import torch
 from torch import Tensor
 
-from ...runtime import cabi, proxy_tracing, tracing, unsupported
+from ...runtime import cabi, proxy_tracing, result_like, tracing, unsupported
 from ...runtime.native import native
 
 
@@ -297,4 +297,4 @@ def apply(query, key, value, mask, bias, scale, geometry, flags=0) -> Tensor:
         raise unsupported("triangle_attention", "does not support torch.func transforms")
     if tracing():
         return TracedAttention.apply(query, key, value, mask, bias, float(scale), geometry, flags)
-    return native().attend(query, key, value, mask, bias, scale, encode_geometry(geometry), flags)
+    return result_like(native().attend(query, key, value, mask, bias, scale, encode_geometry(geometry), flags), query)

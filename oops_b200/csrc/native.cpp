@@ -996,7 +996,9 @@ struct UpdateFunction : Function<UpdateFunction> {
 // ---------------------------------------------------------------------------------------------
 
 MaybeTensor maybe_tensor(PyObject* o) { return o == Py_None ? MaybeTensor() : MaybeTensor(THPVariable_Unpack(o)); }
-bool tensor_or_none(PyObject* o) { return o == Py_None || THPVariable_Check(o); }
+// The entries take tensors and parameters; a subclass, whose results are of its own kind, goes through the Python path.
+bool is_tensor(PyObject* o) { return THPVariable_CheckExact(o); }
+bool tensor_or_none(PyObject* o) { return o == Py_None || is_tensor(o); }
 bool is_number(PyObject* o) { return PyFloat_Check(o) || PyLong_Check(o); }  // anything else is converted, or refused, in Python
 double number(PyObject* o) {
   const double v = PyFloat_AsDouble(o);
@@ -1016,7 +1018,7 @@ template <auto Attention>
 PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 7, "attention takes 7 arguments");
-  if (!THPVariable_Check(a[0]) || !THPVariable_Check(a[1]) || !THPVariable_Check(a[2]) || !tensor_or_none(a[3]) || !tensor_or_none(a[4]) ||
+  if (!is_tensor(a[0]) || !is_tensor(a[1]) || !is_tensor(a[2]) || !tensor_or_none(a[3]) || !tensor_or_none(a[4]) ||
       !number_or_none(a[5]))
     Py_RETURN_NONE;
   const Tensor &q = THPVariable_Unpack(a[0]), &k = THPVariable_Unpack(a[1]), &v = THPVariable_Unpack(a[2]);
@@ -1037,7 +1039,7 @@ PyObject* py_gated_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 8, "triangle_attention_gated takes 8 arguments");
   for (int i = 0; i < 4; ++i)
-    if (!THPVariable_Check(a[i])) Py_RETURN_NONE;
+    if (!is_tensor(a[i])) Py_RETURN_NONE;
   if (!tensor_or_none(a[4]) || !tensor_or_none(a[5]) || !number_or_none(a[6])) Py_RETURN_NONE;
   const Tensor &q = THPVariable_Unpack(a[0]), &k = THPVariable_Unpack(a[1]), &v = THPVariable_Unpack(a[2]), &g = THPVariable_Unpack(a[3]);
   const MaybeTensor mask = maybe_tensor(a[4]), bias = maybe_tensor(a[5]);
@@ -1057,7 +1059,7 @@ PyObject* py_gate_output(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 4, "gate_attention_output takes 4 arguments");
   for (int i = 0; i < 4; ++i)
-    if (!THPVariable_Check(a[i])) Py_RETURN_NONE;
+    if (!is_tensor(a[i])) Py_RETURN_NONE;
   std::optional<Tensor> out;
   {
     const Tensor &attention = THPVariable_Unpack(a[0]), &single = THPVariable_Unpack(a[1]), &wg = THPVariable_Unpack(a[2]),
@@ -1073,7 +1075,7 @@ PyObject* py_gate_output(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_layer_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 5, "layer_norm takes 5 arguments");
-  if (!THPVariable_Check(a[0]) || !PyLong_Check(a[1]) || !tensor_or_none(a[2]) || !tensor_or_none(a[3]) || !is_number(a[4])) Py_RETURN_NONE;
+  if (!is_tensor(a[0]) || !PyLong_Check(a[1]) || !tensor_or_none(a[2]) || !tensor_or_none(a[3]) || !is_number(a[4])) Py_RETURN_NONE;
   const Tensor& x = THPVariable_Unpack(a[0]);
   int overflow = 0;
   const int64_t width = PyLong_AsLongLongAndOverflow(a[1], &overflow);

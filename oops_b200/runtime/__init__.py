@@ -76,6 +76,14 @@ def require_no_forward_mode(operator: str, *tensors: Tensor | None) -> None:
         )
 
 
+def result_like(result: Tensor, operand: Tensor) -> Tensor:
+    """``result`` as the kind of tensor that ``operand`` allocates (a subclass keeps its type through an operator)."""
+    if type(operand) in (Tensor, torch.nn.Parameter):
+        return result
+    kind = type(operand.new_empty(0))
+    return result if kind is type(result) else result.as_subclass(kind)
+
+
 def tracing() -> bool:
     """True under ``torch.jit.trace``, which records Python autograd functions but not the compiled nodes."""
     return torch._C._get_tracing_state() is not None
@@ -92,6 +100,6 @@ def require_no_proxy_tracing(operator: str) -> None:
 
 
 __all__ = [
-    "unsupported", "tracing", "proxy_tracing", "require_no_proxy_tracing", "is_compiling", "require_same_device", "require_shape", "forward_mode_active",
+    "unsupported", "result_like", "tracing", "proxy_tracing", "require_no_proxy_tracing", "is_compiling", "require_same_device", "require_shape", "forward_mode_active",
     "require_no_forward_mode",
 ]
