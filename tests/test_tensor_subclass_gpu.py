@@ -27,7 +27,8 @@ def test_results_keep_the_type(cuda, dtype):
         want = call(leaf)
         got = call(label(leaf))
         assert type(got) is Labelled and torch.equal(got.as_subclass(torch.Tensor), want)
-        grads = [torch.autograd.grad(out.as_subclass(torch.Tensor).sum(), leaf)[0] for out in (got, want)]
-        assert torch.equal(grads[0].as_subclass(torch.Tensor), grads[1])
+        first, second = (torch.autograd.grad(out.as_subclass(torch.Tensor).sum(), leaf)[0].as_subclass(torch.Tensor) for out in (got, want))
+        # (the gradients of a tensor that is query, key and value at once are added in the order the engine meets them)
+        assert float((first - second).norm()) <= 4 * torch.finfo(dtype).eps * float(second.norm())
     parameter = torch.nn.Parameter(q.detach())
     assert type(oops.triangle_attention(parameter, parameter, parameter)) is torch.Tensor
