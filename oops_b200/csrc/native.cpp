@@ -585,32 +585,34 @@ struct GateOutputFunction : Function<GateOutputFunction> {
     run_gate(head_major(values), as_pairs(gate), as_pairs(gated));
     std::vector<int64_t> shape = single.sizes().vec();
     shape.back() = wo.size(0);
-    if (ctx) {
-      ctx->save_for_backward({values, rows, wg, wo, gate, gated});
-      ctx->saved_data["attention"] = attention.sizes().vec();
-      ctx->saved_data["single"] = single.sizes().vec();
-      ctx->saved_data["types"] = std::vector<int64_t>{int64_t(gate_weight.scalar_type()), int64_t(output_weight.scalar_type())};
-    }
+    if (ctx) ctx->save_for_backward({attention, single, gate_weight, output_weight, gate, gated});
     return at::_unsafe_view(at::linear(gated, wo), shape);
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grad_outputs) {
     const NoAutocast no_autocast;
-    variable_list saved = ctx->get_saved_variables();
-    const Tensor values = unit_inner(saved[0]), rows = saved[1], wg = saved[2], wo = saved[3], gate = saved[4].contiguous(), gated = saved[5];
-    const std::vector<int64_t> types = ctx->saved_data["types"].toIntVector();
-    const int64_t heads = values.size(1), tokens = values.size(2), dim = values.size(3);
-    const Tensor dout = grad_outputs[0].resolve_neg().to(gate.scalar_type()).reshape({-1, wo.size(0)});
+    const variable_list saved = ctx->get_saved_variables();
+    const Tensor &attention = saved[0], &single = saved[1];
+    const auto type = attention.scalar_type(), gate_type = saved[2].scalar_type(), output_type = saved[3].scalar_type();
+    const int64_t heads = attention.size(-3), tokens = attention.size(-2), dim = attention.size(-1);
+    const Tensor values = unit_inner(attention.reshape({-1, heads, tokens, dim})), rows = single.reshape({-1, single.size(-1)}),
+                 wg = saved[2].to(type), wo = saved[3].to(type);
+    Tensor gate = saved[4].contiguous(), gated = saved[5];
+    if (at::GradMode::is_enabled()) {  // a graph of the gradients is wanted: they are products of these, which are made to have one
+      gate = at::linear(rows, wg);
+      gated = GateFunction::apply(values, gate.view({values.size(0), tokens, heads * dim})).view(gate.sizes());
+    }
+    const Tensor dout = grad_outputs[0].resolve_neg().to(type).reshape({-1, wo.size(0)});
     variable_list result(4);
-    if (ctx->needs_input_grad(3)) result[3] = at::mm(dout.t(), gated).to(at::ScalarType(types[1]));
+    if (ctx->needs_input_grad(3)) result[3] = at::mm(dout.t(), gated).to(output_type);
     const bool need_attention = ctx->needs_input_grad(0), need_gate = ctx->needs_input_grad(1) || ctx->needs_input_grad(2);
     if (!need_attention && !need_gate) return result;
     const Tensor dgated = at::mm(dout, wo), dgate = need_gate ? at::empty_like(gate) : Tensor();
     const Tensor dvalues = need_attention ? at::empty(values.sizes(), values.options()) : Tensor();
     auto as_pairs = [&](const Tensor& t) { return t.defined() ? t.view({values.size(0), 1, tokens, heads, dim}) : t; };
     run_gate_backward(head_major(values), as_pairs(gate), as_pairs(dgated), head_major(dvalues), as_pairs(dgate));
-    if (need_attention) result[0] = dvalues.view(ctx->saved_data["attention"].toIntVector());
-    if (ctx->needs_input_grad(1)) result[1] = at::mm(dgate, wg).view(ctx->saved_data["single"].toIntVector());
-    if (ctx->needs_input_grad(2)) result[2] = at::mm(dgate.t(), rows).to(at::ScalarType(types[0]));
+    if (need_attention) result[0] = dvalues.view(attention.sizes());
+    if (ctx->needs_input_grad(1)) result[1] = at::mm(dgate, wg).view(single.sizes());
+    if (ctx->needs_input_grad(2)) result[2] = at::mm(dgate.t(), rows).to(gate_type);
     return result;
   }
 };
@@ -843,7 +845,27 @@ Tensor contract(bool outgoing, const Tensor& left, const Tensor& right) {
 
 enum { kLeftGate, kLeftValue, kRightGate, kRightValue, kOutputGate, kOutput, kProjections };
 
+// The update from single operations, with the graph that a second differentiation needs (operands as UpdateFunction has them).
+Tensor composed_update(const Tensor& pair, const Tensor& mask, bool outgoing, double in_eps, double out_eps, at::TensorList parameters,
+                       const std::vector<int64_t>& bias_of) {
+  const auto type = pair.scalar_type();
+  MaybeTensor biases[kProjections];
+  for (size_t i = 0; i < bias_of.size(); ++i) biases[bias_of[i]] = parameters[10 + i].to(type);
+  auto project = [&](const Tensor& x, int which) { return at::linear(x, parameters[4 + which].to(type), biases[which]); };
+  const Tensor x = LayerNormFunction::apply(pair, MaybeTensor(parameters[0]), MaybeTensor(parameters[1]), in_eps);
+  const Tensor weight = mask.defined() ? mask.to(type).unsqueeze(-1) : Tensor();
+  auto side = [&](int gate) {  // channel-major
+    const Tensor open = at::sigmoid(project(x, gate));
+    return ((weight.defined() ? weight * open : open) * project(x, gate + 1)).movedim(-1, -3);
+  };
+  const Tensor left = side(kLeftGate), right = side(kRightGate);
+  const Tensor update = at::matmul(outgoing ? left : left.transpose(-1, -2), outgoing ? right.transpose(-1, -2) : right).movedim(-3, -1);
+  const Tensor normed = LayerNormFunction::apply(update.contiguous(), MaybeTensor(parameters[2]), MaybeTensor(parameters[3]), out_eps);
+  return project(normed, kOutput) * at::sigmoid(project(x, kOutputGate));
+}
+
 struct UpdateFunction : Function<UpdateFunction> {
+  static constexpr size_t kFirst = 5;  // inputs: pair, mask, outgoing, in_eps, out_eps, parameters..., bias_of
   // `parameters`: the input and output norms' weight and bias, the six projection weights, then the biases that exist;
   // `bias_of` says which projection each of those belongs to.
   static Tensor forward(AutogradContext* ctx, const Tensor& pair, const MaybeTensor& mask, bool outgoing, double in_eps, double out_eps,
@@ -894,9 +916,11 @@ struct UpdateFunction : Function<UpdateFunction> {
                  "triangle_multiplication output gate");
     if (ctx) {
       ctx->set_materialize_grads(false);
-      ctx->save_for_backward({rows, in_w, x.stats, x.y, stacked, proj, weight, left, right, update, out_w, stats, normed, out_matrix, values});
+      variable_list kept{pair, x.stats, x.y, stacked, proj, weight, left, right, update, stats, normed, out_matrix, values, mask.value_or(Tensor())};
+      kept.insert(kept.end(), parameters.begin(), parameters.end());
+      ctx->save_for_backward(kept);
       ctx->saved_data["outgoing"] = outgoing;
-      ctx->saved_data["shape"] = pair.sizes().vec();
+      ctx->saved_data["eps"] = std::vector<double>{in_eps, out_eps};
       ctx->saved_data["dims"] = std::vector<int64_t>{s.prefix, s.tokens, s.padded, s.hidden, mask.has_value()};
       ctx->saved_data["bias_of"] = bias_of;
       std::vector<int64_t> types;
@@ -906,20 +930,38 @@ struct UpdateFunction : Function<UpdateFunction> {
     return out;
   }
 
+  // With a graph of the gradients wanted, they come from the composed form (as far as its nodes have one themselves).
+  static variable_list differentiable_backward(AutogradContext* ctx, const Tensor& dout, const variable_list& saved, size_t first,
+                                               const std::vector<int64_t>& bias_of, size_t edge, variable_list result) {
+    const std::vector<double> eps = ctx->saved_data["eps"].toDoubleVector();
+    const variable_list parameters(saved.begin() + first, saved.end());
+    const Tensor out = composed_update(saved[0], saved[first - 1], ctx->saved_data["outgoing"].toBool(), eps[0], eps[1], parameters, bias_of);
+    variable_list inputs;
+    std::vector<size_t> places;
+    for (size_t i = 0; i <= parameters.size(); ++i) {
+      if (!ctx->needs_input_grad(i == 0 ? 0 : edge + i - 1)) continue;
+      inputs.push_back(i == 0 ? saved[0] : parameters[i - 1]);
+      places.push_back(i == 0 ? 0 : kFirst + i - 1);
+    }
+    const variable_list grads = torch::autograd::grad({out}, inputs, {dout.to(out.scalar_type())}, std::nullopt, true, true);
+    for (size_t i = 0; i < places.size(); ++i) result[places[i]] = grads[i];
+    return result;
+  }
+
   static variable_list backward(AutogradContext* ctx, const variable_list& grad_outputs) {
     const NoAutocast no_autocast;
     const std::vector<int64_t> dims = ctx->saved_data["dims"].toIntVector(), bias_of = ctx->saved_data["bias_of"].toIntVector(),
                                types = ctx->saved_data["types"].toIntVector();
-    // inputs: pair, mask, outgoing, in_eps, out_eps, parameters..., bias_of
-    constexpr size_t kFirst = 5;
     variable_list result(kFirst + types.size() + 1);
     if (!grad_outputs[0].defined()) return result;
     variable_list saved = ctx->get_saved_variables();
-    for (Tensor& t : saved)
-      if (t.defined()) t = t.contiguous();
-    const Tensor &rows = saved[0], &in_w = saved[1], &stats1 = saved[2], &x = saved[3], &stacked = saved[4], &proj = saved[5], &weight = saved[6],
-                 &left = saved[7], &right = saved[8], &update = saved[9], &out_w = saved[10], &stats2 = saved[11], &normed = saved[12],
-                 &out_matrix = saved[13], &values = saved[14];
+    constexpr size_t kKept = 14;  // then the parameters
+    if (at::GradMode::is_enabled()) return differentiable_backward(ctx, grad_outputs[0], saved, kKept, bias_of, dims[4] ? 2 : 1, std::move(result));
+    for (size_t i = 1; i < saved.size(); ++i)
+      if (saved[i].defined()) saved[i] = saved[i].contiguous();
+    const Tensor &pair = saved[0], &stats1 = saved[1], &x = saved[2], &stacked = saved[3], &proj = saved[4], &weight = saved[5],
+                 &left = saved[6], &right = saved[7], &update = saved[8], &stats2 = saved[9], &normed = saved[10], &out_matrix = saved[11],
+                 &values = saved[12], &in_w = saved[kKept], &out_w = saved[kKept + 2];
     const UpdateShape s{dtype_code(proj.scalar_type()), int32_t(dims[0]), int32_t(dims[1]), int32_t(dims[2]), int32_t(dims[3])};
     const size_t edge = dims[4] ? 2 : 1;  // first parameter's edge: behind the pair and, when it was given, the mask
     auto need = [&](size_t parameter) { return ctx->needs_input_grad(edge + parameter); };
@@ -981,9 +1023,9 @@ struct UpdateFunction : Function<UpdateFunction> {
         if (bias_of[i] != kOutput && need(10 + i)) give(10 + i, piece(sums, bias_of[i]));
     }
     if (norm_wanted) {
-      NormGradients grads = norm_backward(at::mm(dproj, stacked), rows_of(rows, channels), in_w, stats1, in_w.scalar_type(), pair_wanted,
+      NormGradients grads = norm_backward(at::mm(dproj, stacked), rows_of(pair, channels), in_w, stats1, in_w.scalar_type(), pair_wanted,
                                           need(0), need(1));
-      if (pair_wanted) result[0] = grads.dx.view(ctx->saved_data["shape"].toIntVector());
+      if (pair_wanted) result[0] = grads.dx.view(pair.sizes());
       result[kFirst] = grads.dweight;
       result[kFirst + 1] = grads.dbias;
     }
