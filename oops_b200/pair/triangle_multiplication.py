@@ -103,6 +103,7 @@ def _cast(bias: Optional[Tensor], like: Tensor) -> Optional[Tensor]:
 # ----------------------------------------------------------------------------------------------
 
 _DTYPES = (torch.float32, torch.float16, torch.bfloat16)
+_PLAIN = (Tensor, torch.nn.Parameter)
 _MAX_HIDDEN = 512  # a tile of the channel-norm kernel holds all channels of its tokens in shared memory
 
 
@@ -111,7 +112,7 @@ def _fused_serves(pair: Tensor, mask: Optional[Tensor], hidden: int, projections
     composed); a mask that takes no gradient and expands to the pair's cells."""
     return (
         pair.dtype in _DTYPES and pair.numel() > 0 and 0 < hidden <= _MAX_HIDDEN and _fits_a_launch(pair) and not _mostly_padding(pair, hidden)
-        and type(pair) in (Tensor, torch.nn.Parameter)
+        and type(pair) in _PLAIN and all(type(p) in _PLAIN for p in (*projections, *biases) if p is not None)
         and not torch.compiler.is_compiling() and not torch.is_autocast_enabled("cuda")
         and torch._C._functorch.peek_interpreter_stack() is None and not tracing() and not proxy_tracing()
         and all(p.is_floating_point() for p in projections)

@@ -25,3 +25,14 @@ def test_bias_shapes(shape, serves):
                                                         (torch.float32, 4096, 4, False), (torch.float32, 4096, 5, True), (torch.float32, 16, 1, True)])
 def test_many_grids_that_are_mostly_padding(dtype, prefix, tokens, serves):
     assert _fused_serves(torch.empty(prefix, tokens, tokens, 64, dtype=dtype, device="meta"), None, 64, (), ()) is serves
+
+
+def test_subclasses_are_composed():
+    class Labelled(torch.Tensor):
+        pass
+
+    plain = [torch.empty(8, 4) for _ in range(6)]
+    pair = torch.empty(1, 16, 16, 4)
+    assert _fused_serves(pair, None, 8, [torch.nn.Parameter(p) for p in plain], [None] * 6)
+    assert not _fused_serves(pair.as_subclass(Labelled), None, 8, plain, [None] * 6)
+    assert not _fused_serves(pair, None, 8, [*plain[:5], plain[5].as_subclass(Labelled)], [None] * 6)
