@@ -37,8 +37,7 @@ def _nvcc() -> str:
 # Kernels that keep tensor-memory loads in flight under arithmetic: a load writes its destination registers when the
 # data arrives, so a spill (or copy) of such a register between issue and wait would save stale data.  ptxas must
 # report no spill stores for them; the build fails otherwise.
-# (The forward kernels go by their translation unit, ta_tensor_sm100.cu, whose name is part of their mangled names.)
-NO_SPILL_KERNELS = ("ta_tensor_sm100_cu", "ta_bwd_fused_kernel", "ta_bwd_dbias_kernel")
+NO_SPILL_KERNELS = ("ta_fwd_kernel", "ta_bwd_fused_kernel", "ta_bwd_dbias_kernel")
 
 
 def _spilling_entries(ptxas_log: str, kernels) -> list:
