@@ -3,8 +3,8 @@
 // Forward (replaces the reference's Triton `_attend`, oops/attention/triangle/triton/kernel.py:150-262):
 // a CTA works on two 128-query tiles.  With a row-shared bias (or none) the tiles are the same queries of two neighbouring
 // pair rows, which read one bias tile; with a per-row bias they are neighbouring query tiles of one row, which read one
-// K/V stream.  A producer warp streams 64-key K/V tiles and 128 x 64 bias tiles into shared memory with TMA; one thread
-// issues tcgen05.mma for S = Q K^T (accumulator in tensor memory) and O += P V (P read back from tensor memory,
+// K/V stream.  A producer warp streams 64-key K/V tiles and 128 x 64 bias tiles into shared memory with TMA; a thread per
+// tile issues tcgen05.mma for S = Q K^T (accumulator in tensor memory) and O += P V (P read back from tensor memory,
 // V from shared memory); one softmax warpgroup per tile (a thread owns a query) turns S into P.
 //
 // The softmax has no row maximum in its steady state.  The maximum of the first 16 columns (that keep a key) of a
@@ -288,13 +288,13 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
         mbar_arrive_warp(bar(Smem::v_ready + ring * kStages + (i - full_steps) % kStages));
       }
 
-      const int n = base + i;
-      const int bias_slot = (ROWS ? 0 : w * 2) + (n & 1);
+      const int at_step = base + i;  // over all items: what barrier phases count
+      const int bias_slot = (ROWS ? 0 : w * 2) + (at_step & 1);
       // the phases the step needs are probed together: one round trip to the barrier words when all are complete
-      const bool s_there = mbar_test(bar(Smem::s_full + w), n & 1);
-      const bool bias_there = HAS_BIAS && mbar_test(bar(Smem::bias_full + bias_slot), (n >> 1) & 1);
-      ok = mbar_wait_probed(s_there, bar(Smem::s_full + w), n & 1, abort_flag);
-      if (ok && HAS_BIAS) ok = mbar_wait_probed(bias_there, bar(Smem::bias_full + bias_slot), (n >> 1) & 1, abort_flag);
+      const bool s_there = mbar_test(bar(Smem::s_full + w), at_step & 1);
+      const bool bias_there = HAS_BIAS && mbar_test(bar(Smem::bias_full + bias_slot), (at_step >> 1) & 1);
+      ok = mbar_wait_probed(s_there, bar(Smem::s_full + w), at_step & 1, abort_flag);
+      if (ok && HAS_BIAS) ok = mbar_wait_probed(bias_there, bar(Smem::bias_full + bias_slot), (at_step >> 1) & 1, abort_flag);
       if (!ok) return;
       tc_fence_after_sync();
       // swizzled row of the bias tile: 16-byte chunk n holds keys 8 n .. 8 n + 7
@@ -354,7 +354,7 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
           l_run *= alpha;
         }
         if (i > 0 && __any_sync(0xffffffffu, raised)) {
-          if (!mbar_wait(bar(Smem::pv_done + w), (n - 1) & 1, abort_flag)) return false;
+          if (!mbar_wait(bar(Smem::pv_done + w), (at_step - 1) & 1, abort_flag)) return false;
           tc_fence_after_sync();
           uint32_t acc[32];
           tmem_ld32(o_tmem, acc);
@@ -403,7 +403,7 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
           }
           if (chunk & 1) {
             if (!p_free) {  // the previous P V product must have finished with the P columns
-              ok = mbar_wait(bar(Smem::pv_done + w), (n - 1) & 1, abort_flag);
+              ok = mbar_wait(bar(Smem::pv_done + w), (at_step - 1) & 1, abort_flag);
               tc_fence_after_sync();
               p_free = true;
             }
