@@ -105,38 +105,8 @@ def library() -> ctypes.CDLL:
     lib.oops_ta_forward_static.argtypes = [POINTER(Problem), POINTER(Pair), c_void_p, c_void_p]
     lib.oops_ta_forward_static_capacity.restype = c_uint64
     lib.oops_ta_launch_count.restype = c_uint64
-    lib.oops_ta_forward_gated.restype = c_int
-    lib.oops_ta_forward_gated.argtypes = [POINTER(Problem), POINTER(Pair), POINTER(Pair), POINTER(Pair), c_void_p, c_void_p]
-    lib.oops_ta_gate_forward.restype = c_int
-    lib.oops_ta_gate_forward.argtypes = [c_int] * 6 + [POINTER(Pair)] * 3 + [c_void_p]
-    lib.oops_ta_gate_backward.restype = c_int
-    lib.oops_ta_gate_backward.argtypes = [c_int] * 6 + [POINTER(Pair)] * 5 + [c_void_p]
     lib.oops_ta_pair_mask_packed.restype = c_int
     lib.oops_ta_pair_mask_packed.argtypes = [c_void_p, c_void_p, c_int32, c_int64, c_void_p, c_void_p]
-    lib.oops_ta_layer_norm_backward_workspace_bytes.restype = c_uint64
-    lib.oops_ta_layer_norm_backward_workspace_bytes.argtypes = [c_int64, c_int32]
-    lib.oops_ta_layer_norm_forward.restype = c_int
-    lib.oops_ta_layer_norm_forward.argtypes = [c_int, c_int, c_int64, c_int32, c_void_p, c_int64, c_void_p, c_void_p, c_float,
-                                               c_void_p, c_int64, c_void_p, c_void_p, c_void_p]
-    lib.oops_ta_layer_norm_backward.restype = c_int
-    lib.oops_ta_layer_norm_backward.argtypes = [c_int, c_int, c_int64, c_int32, c_void_p, c_int64, c_void_p, c_int64, c_void_p,
-                                                c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_uint64,
-                                                c_void_p]
-    lib.oops_ta_pair_gate_forward.restype = c_int
-    lib.oops_ta_pair_gate_forward.argtypes = [c_int] + [c_int32] * 4 + [c_void_p, c_int64] + [c_void_p] * 4
-    lib.oops_ta_pair_gate_backward.restype = c_int
-    lib.oops_ta_pair_gate_backward.argtypes = [c_int] + [c_int32] * 4 + [c_void_p, c_int64] + [c_void_p] * 4 + [c_int64, c_void_p]
-    lib.oops_ta_channel_norm_forward.restype = c_int
-    lib.oops_ta_channel_norm_forward.argtypes = [c_int, c_int] + [c_int32] * 4 + [c_void_p] * 3 + [c_float] + [c_void_p] * 4
-    lib.oops_ta_channel_norm_backward_workspace_bytes.restype = c_uint64
-    lib.oops_ta_channel_norm_backward_workspace_bytes.argtypes = [c_int] + [c_int32] * 4
-    lib.oops_ta_channel_norm_backward.restype = c_int
-    lib.oops_ta_channel_norm_backward.argtypes = [c_int, c_int] + [c_int32] * 4 + [c_void_p] * 9 + [c_uint64, c_void_p]
-    lib.oops_ta_output_gate_forward.restype = c_int
-    lib.oops_ta_output_gate_forward.argtypes = [c_int, c_int64, c_int32, c_void_p, c_void_p, c_int64, c_void_p, c_void_p]
-    lib.oops_ta_output_gate_backward.restype = c_int
-    lib.oops_ta_output_gate_backward.argtypes = ([c_int, c_int64, c_int32] + [c_void_p] * 3 + [c_int64] + [c_void_p] * 2
-                                                 + [c_int64, c_void_p])
     lib.oops_ta_bias_rows.restype = c_int
     lib.oops_ta_bias_rows.argtypes = [c_int32] * 4 + [c_void_p, POINTER(c_int64), c_void_p, c_void_p]
     lib.oops_ta_selftest_wait_limit.restype = c_int
