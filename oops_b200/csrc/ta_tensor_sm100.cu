@@ -7,8 +7,9 @@
 // tile issues tcgen05.mma for S = Q K^T (accumulator in tensor memory) and O += P V (P read back from tensor memory,
 // V from shared memory); one softmax warpgroup per tile (a thread owns a query) turns S into P.
 //
-// The softmax has no row maximum in its steady state.  The maximum of the first 16 columns (that keep a key) of a
-// row's first step is its reference; later steps take 2^(x - reference) as they come, 16 columns at a time, and look at the step's sum only: a
+// The softmax has no row maximum in its steady state.  The maximum of a row's first step is its reference (that probability
+// is then 1, which 16 bits hold exactly; a reference from fewer columns left every large one rounded, and short rows 2 to 5 %
+// further from the exact result); later steps take 2^(x - reference) as they come, 16 columns at a time, and look at the step's sum only: a
 // sum of 2^10 or more (or a NaN) sends the warp back over the step, which still stands in tensor memory, to raise the
 // reference and rescale the accumulators.  Probabilities therefore stay below 2^10, inside the f32, bf16 and f16 ranges.
 // Against a maximum per step this saves the comparisons, and above all the wait: no exponential depended on the last
@@ -317,8 +318,8 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
           }
         }
       };
-      // The largest base-2 logit of the step; for a first reference, of as many of its columns as give every row one.
-      auto step_peak = [&](bool first) -> float {
+      // The largest base-2 logit of the step.
+      auto step_peak = [&]() -> float {
         float peak = -INFINITY;
 #pragma unroll 1
         for (int chunk = 0; chunk < 4; ++chunk) {
@@ -339,14 +340,13 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
             unpack2(x[n], lo, hi);
             peak = max3(peak, lo, hi);
           }
-          if (first && !__any_sync(0xffffffffu, peak == -INFINITY)) break;
         }
         return peak;
       };
       // Raises the reference of the rows whose step needs it, and rescales what they have summed so far.
-      auto raise = [&](bool wanted, bool first) -> bool {
+      auto raise = [&](bool wanted) -> bool {
         tmem_wait_st();  // probabilities of a pass that is about to be repeated
-        const float peak = step_peak(first);
+        const float peak = step_peak();
         const bool raised = wanted && peak > ref;
         const float alpha = raised ? ex2(ref - peak) : 1.f;  // 0 for a row without a reference so far
         if (raised) {
@@ -418,7 +418,7 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
       bool wanted = ref == -INFINITY;
 #pragma unroll 1
       for (int attempt = 0; attempt < 2 && ok; ++attempt) {
-        if (__any_sync(0xffffffffu, wanted)) ok = raise(wanted, attempt == 0);
+        if (__any_sync(0xffffffffu, wanted)) ok = raise(wanted);
         else if (attempt > 0) break;
         if (!ok) return;
         sum = step_pass();

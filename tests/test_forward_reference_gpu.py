@@ -51,3 +51,22 @@ def test_references(cuda, dtype, kind, rows, n, mask_kind, full):
     assert error <= 2 * ROUNDING[dtype] * float(torch.nan_to_num(v.double(), nan=0.0).abs().max()), error
     if mask is not None:
         assert torch.count_nonzero(out.cpu()[~mask.any(-1)]) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,n,column", [(60, 64, 40), (60, 136, 63), (1, 512, 17), (40, 100, 30)])
+def test_the_largest_probability_of_the_first_step_is_exact(cuda, dtype, rows, n, column):
+    """One key of the first step carries 0.6 to 0.95 of every row.  Its probability is the reference, 1 before the division by
+    the sum, so the result is off by its own rounding and the rounding of the light keys: less than 1.15 of the result's
+    rounding in the 2-norm, where a rounded largest probability makes it 1.4."""
+    gen = torch.Generator().manual_seed(n)
+    heads = 2
+    q, k, v = ((0.5 * torch.randn(1, rows, n, heads, 32, generator=gen)).to(dtype) for _ in range(3))
+    bias = torch.randn(1, 1, heads, n, n, generator=gen)
+    bias[..., column] += 2.0 + torch.log(torch.tensor(float(n)))
+    bias = bias.to(dtype)
+    with torch.no_grad():
+        out = triangle_attention(q.to(cuda), k.to(cuda), v.to(cuda), None, bias.to(cuda)).double().cpu()
+    want = oracle.reference_dense(q.double(), k.double(), v.double(), None, bias.double(), compute_dtype=torch.float64)
+    rounding = float((want.to(dtype).double() - want).norm())
+    assert float((out - want).norm()) <= 1.15 * rounding
