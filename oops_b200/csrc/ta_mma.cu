@@ -16,7 +16,8 @@
 //             scores it needs again (9 products instead of 5): token attention has too few rows and heads to give a
 //             CTA a whole row, and nothing has to be added across CTAs, so results are reproducible.
 // 4 samples, 16 heads of 64 channels, 512 tokens: 35 us forward and 136 us reverse, against 1178 us in 9 launches with scores
-// in memory.  Bound by issue slots (two thirds of them element-wise work on the scores) at twelve warps per SM: packed f32
+// in memory.  Bound by latency at twelve to sixteen warps per SM, element-wise work and products in turn (counters of that call:
+// issue slots 50 % and the tensor pipe 38 % busy forward, 36 and 33 % in the reverse, HBM idle): packed f32
 // arithmetic, no tests on kept keys where a tile keeps all, first products without a zeroed accumulator, and, in the
 // reverse, row operands read again from shared memory instead of held in 64 registers (238 -> 168 registers, two -> three
 // CTAs per SM) took 45 and 171 us to these figures.
@@ -932,7 +933,8 @@ int by_kind(const oops_ta_problem& p, F&& run) {
 
 }  // namespace
 
-// Head sizes above 64 would spill the accumulators of the dK/dV part; they stay with the kernels that keep logits in memory.
+// Head sizes above 64 would need more accumulators in the dK/dV part than there are registers (up to 64 every instance of the
+// reverse spills 8 to 24 bytes already); they stay with the kernels that keep logits in memory.
 bool mma_applies(const oops_ta_problem& p) {
   if (p.dtype != OOPS_TA_F16 && p.dtype != OOPS_TA_BF16) return false;
   if (p.head_dim > 64) return false;

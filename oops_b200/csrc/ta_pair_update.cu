@@ -114,7 +114,7 @@ __device__ __forceinline__ int64_t token_at(const PairShape& s, int b, int64_t p
 // The channels of `left` and `right`, each rounded up to eight, form one axis.  CTA = (32 words of tokens, 64 of that axis,
 // prefix element): a token's piece of a projection is then 128 contiguous bytes of a 16-bit type (64-byte pieces: 55 and
 // 90 us forward and reverse at N = 384, 128 channels; now 52 and 78, the reverse with five CTAs per SM instead of
-// four).  The channel chunk is the fastest index: neighbouring CTAs touch a token's other pieces while their pages are open.
+// four, which pays although the 16-bit instances then spill 60 bytes a thread).  The channel chunk is the fastest index: neighbouring CTAs touch a token's other pieces while their pages are open.
 
 struct GateTile {  // rows = channels; rows 32 .. 63 stand four words on, so that a warp's eight channel groups miss each other's banks
   uint32_t words[64 * kPitch + 4];

@@ -14,8 +14,8 @@
 // reference and rescale the accumulators.  Probabilities therefore stay below 2^10, inside the f32, bf16 and f16 ranges.
 // Against a maximum per step this saves the comparisons, and above all the wait: no exponential depended on the last
 // score of a step any more, scores need not be held in registers, and an exponential costs 5 instead of 9.5 issue slots.
-// What bounds it: issue slots and, close behind, the special-function unit, one ex2 per score at 16 per clock and SM (0.40 of
-// the 0.70 ms at N = 768).  Hence no tests on kept bits where nothing is dropped: a CTA whose rows keep every key walks a copy
+// What bounds it: the element-wise warps' streams, with issue slots (57 %) and the special-function unit (59 %; one ex2 per
+// score at 16 per clock and SM, 0.40 of the 0.73 ms at N = 768) the busiest units.  Hence no tests on kept bits where nothing is dropped: a CTA whose rows keep every key walks a copy
 // of the roles without them (N = 768: 757 -> 703 us), and otherwise the steps that every row keeps whole come first, in a
 // loop of their own (the order of the keys is free; N = 1024, 1000 kept: 1659 -> 1618 us).
 #include <type_traits>
