@@ -415,7 +415,8 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
         return lo + hi;
       };
       float sum = 0.f;
-      bool wanted = ref == -INFINITY;
+      // (a row that keeps no key of the step looks for no reference in it: its partner's steps are walked beside dead rows too)
+      bool wanted = ref == -INFINITY && (!kDrops || (bits.x | bits.y) != 0u);
 #pragma unroll 1
       for (int attempt = 0; attempt < 2 && ok; ++attempt) {
         if (__any_sync(0xffffffffu, wanted)) ok = raise(wanted);
