@@ -17,7 +17,8 @@
 // What bounds it: the element-wise warps' streams, with issue slots (57 %) and the special-function unit (59 %; one ex2 per
 // score at 16 per clock and SM, 0.40 of the 0.73 ms at N = 768) the busiest units.  Hence no tests on kept bits where nothing is dropped: a CTA whose rows keep every key walks a copy
 // of the roles without them (N = 768: 757 -> 703 us), and otherwise the steps that every row keeps whole come first, in a
-// loop of their own (the order of the keys is free; N = 1024, 1000 kept: 1659 -> 1618 us).
+// loop of their own (the order of the keys is free; N = 1024, 1000 kept: 1659 -> 1618 us), and a step that one of two rows
+// keeps costs the other a row of zeros (N = 1000, rows that keep alternate blocks of 64 keys: 1966 -> 1466 us).
 #include <type_traits>
 
 #include "ta_tensor_common.cuh"
@@ -415,15 +416,28 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
         return lo + hi;
       };
       float sum = 0.f;
-      // (a row that keeps no key of the step looks for no reference in it: its partner's steps are walked beside dead rows too)
-      bool wanted = ref == -INFINITY && (!kDrops || (bits.x | bits.y) != 0u);
+      if (kDrops && !PERSIST && (bits.x | bits.y) == 0u) {
+        // The row keeps no key of the step, which is walked for its partner: no look for a reference, no exponentials.  (Without a
+        // mask there is no such step.)
+        if (!p_free) {
+          ok = mbar_wait(bar(Smem::pv_done + w), (at_step - 1) & 1, abort_flag);
+          tc_fence_after_sync();
+        }
+        uint32_t zeros[16];
+#pragma unroll
+        for (int n = 0; n < 16; ++n) zeros[n] = 0u;
+        tmem_st16(p_tmem, zeros);
+        tmem_st16(p_tmem + 16, zeros);
+      } else {
+        bool wanted = ref == -INFINITY;
 #pragma unroll 1
-      for (int attempt = 0; attempt < 2 && ok; ++attempt) {
-        if (__any_sync(0xffffffffu, wanted)) ok = raise(wanted);
-        else if (attempt > 0) break;
-        if (!ok) return;
-        sum = step_pass();
-        wanted = !(sum < kStepSumLimit);
+        for (int attempt = 0; attempt < 2 && ok; ++attempt) {
+          if (__any_sync(0xffffffffu, wanted)) ok = raise(wanted);
+          else if (attempt > 0) break;
+          if (!ok) return;
+          sum = step_pass();
+          wanted = !(sum < kStepSumLimit);
+        }
       }
       if (!ok) return;
       l_run += sum;

@@ -45,3 +45,26 @@ def test_gradients(cuda, dtype, rows, n, heads, mask_kind, bias_kind):
         assert torch.count_nonzero(got.cpu()[empty]) == 0
     for got in grads[1:3]:
         assert torch.count_nonzero(got.cpu()[~mask]) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,n,full", [(6, 256, False), (5, 328, False), (4, 200, True), (1, 392, False)])
+def test_steps_that_only_one_row_of_a_pair_keeps(cuda, dtype, rows, n, full):
+    """Neighbouring rows keep alternate blocks of 64 keys, and one row keeps none at all: each walks steps that only its
+    partner keeps.  Bound: probabilities and result rounded to 16 bits, of values that reach max|v|, twice."""
+    from oracle import triangle_oracle as oracle
+
+    gen = torch.Generator().manual_seed(n)
+    heads = 2
+    q, k, v = ((0.5 * torch.randn(1, rows, n, heads, 32, generator=gen)).to(dtype) for _ in range(3))
+    bias = torch.randn(1, rows if full else 1, heads, n, n, generator=gen).to(dtype)
+    mask = ((torch.arange(n) // 64 + torch.arange(rows)[:, None]) % 2 == 0)[None].clone()
+    mask[:, 3:4] = False
+    k, v = k.masked_fill(~mask[..., None, None], float("inf")), v.masked_fill(~mask[..., None, None], float("nan"))
+    with torch.no_grad():
+        out = triangle_attention(q.to(cuda), k.to(cuda), v.to(cuda), mask.to(cuda), bias.to(cuda)).double().cpu()
+    finite = torch.nan_to_num(v.double(), nan=0.0)
+    want = oracle.reference_dense(q.double(), torch.nan_to_num(k.double(), posinf=0.0), finite, mask, bias.double(), compute_dtype=torch.float64)
+    bound = 2 * (2.0**-8 if dtype is torch.bfloat16 else 2.0**-11) * float(finite.abs().max())
+    assert float((out - want).abs().max()) <= bound
+    assert torch.count_nonzero(out[~mask.any(-1)]) == 0
