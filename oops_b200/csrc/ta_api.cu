@@ -418,8 +418,8 @@ uint64_t oops_ta_forward_static_capacity(void) { return static_forward_capacity(
 
 int oops_ta_device_status(int reset) {
   const int forward = forward_device_status(reset);
-  const int backward = backward_device_status(reset);
-  return forward ? forward : backward;
+  const int backward = backward_device_status(reset), wide = wide_device_status(reset);
+  return forward ? forward : backward ? backward : wide;
 }
 
 int oops_ta_selftest_wait_limit(void* stream) {

@@ -47,6 +47,15 @@ int mma_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, c
 int mma_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_ta_pair& dout, const float* lse,
                  const oops_ta_grads& g, cudaStream_t stream);
 
+// tcgen05 kernels of the same calls for bf16 operands without a mask whose rows are 16-byte words.  The reverse is a part of
+// mma_backward: row dots, scratch and the sum of the bias gradient's parts are the same.
+bool wide_forward_applies(const oops_ta_problem& p, const oops_ta_pair& out);
+int wide_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, cudaStream_t stream);
+bool wide_backward_applies(const oops_ta_problem& p, const oops_ta_pair& dout, const oops_ta_grads& g);
+int wide_backward(const oops_ta_problem& p, const oops_ta_pair& dout, const float* lse, const float* delta, const oops_ta_grads& g,
+                  int num_parts, float* parts, cudaStream_t stream);
+int wide_device_status(int reset);
+
 // The layout-agnostic forward pass on the library's built-in scratch array (no caller workspace).
 uint64_t static_forward_capacity();
 int static_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, cudaStream_t stream);
@@ -106,7 +115,7 @@ int output_gate_backward(int dtype, int64_t rows, int channels, const void* dout
 int tensor_forward_gated(const oops_ta_problem& p, const oops_ta_pair& gate, const oops_ta_pair& gated,
                          const oops_ta_pair& plain, float* lse, cudaStream_t stream);
 
-// Read (and optionally clear) the device-side status words of the two tcgen05 translation units;
+// Read (and optionally clear) the device-side status words of the tcgen05 translation units;
 // both synchronise with the device.
 int forward_device_status(int reset);
 // Launches the bounded-wait self-test kernel of the forward translation unit (its wait runs out after 1 ms).

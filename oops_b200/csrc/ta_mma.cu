@@ -1,6 +1,6 @@
 // Triangle attention of 16-bit operands at head sizes and layouts the tcgen05 kernels do not take (head size up to 64
-// other than 32, strides or addresses that are no multiples of 16 bytes, an f32 bias): register-level matrix products
-// (mma.sync m16n8k16, f32 accumulation), operands staged by cp.async.  Definition as in the reference's kernels
+// other than 32 in f16, under a mask or in calls of few columns, strides or addresses that are no multiples of 16 bytes, an f32
+// bias): register-level matrix products (mma.sync m16n8k16, f32 accumulation), operands staged by cp.async.  Definition as in the reference's kernels
 // (oops/attention/triangle/triton/kernel.py:128-147, :250-261, :499-564, :682-714, :856).
 //
 // Calls of this kind are small -- token attention, odd head sizes -- and bound by latency and by the element-wise work
@@ -950,6 +950,7 @@ uint64_t mma_backward_workspace(const oops_ta_problem& p, const oops_ta_grads& g
 }
 
 int mma_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, cudaStream_t stream) {
+  if (wide_forward_applies(p, out)) return wide_forward(p, out, lse, stream);
   MmaProblem m = describe(p);
   m.out = out;
   m.lse = lse;
@@ -1008,7 +1009,8 @@ int mma_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
   const int64_t grid = int64_t(m.dkv_ctas) + m.dq_ctas +
                        (shared_gradient(p, g) ? int64_t(m.num_parts) * p.batch * p.heads * tiles * tiles : 0);
   if (grid == 0) return OOPS_TA_OK;
-  int status = by_kind(p, [&](auto type, auto width, auto b32) -> int {
+  const bool wide = wide_backward_applies(p, dout, g);
+  int status = wide ? wide_backward(p, dout, lse, m.delta, g, m.num_parts, m.parts, stream) : by_kind(p, [&](auto type, auto width, auto b32) -> int {
     using T = decltype(type);
     constexpr int DP = decltype(width)::value;
     constexpr bool B32 = decltype(b32)::value;
