@@ -126,8 +126,10 @@ struct WideFwdSmem {
   static constexpr int v_full = 7, v_empty = 9;   // [2] with the bias tile of the step
   static constexpr int s_full = 11;               // [2] scores are in tensor memory
   static constexpr int p_full = 13;               // [2] probabilities have taken their place
-  static constexpr int pv_done = 15;              // the latest value product has completed
-  static constexpr int num_bars = 16;
+  // [2] the value product of the step has completed (a barrier per buffer: waiters may be two steps behind the last product, and a
+  // parity tells a phase from its neighbours only)
+  static constexpr int pv_done = 15;
+  static constexpr int num_bars = 17;
   static constexpr int tmem_slot = bars + num_bars * 8;
   static constexpr int abort_flag = tmem_slot + 4;
   static constexpr int failed = abort_flag + 4;   // a kernel before this one has given up a wait
@@ -218,10 +220,10 @@ __global__ void __launch_bounds__(kWideFwdThreads, 2) ta_wide_fwd_kernel(const _
         if (!ok) break;
         tc_fence_after_sync();
         sum_product(tmem_base + kOCol, tmem_base + (i & 1) * kStep, k_major(smem_base + Smem::v + (i & 1) * kColTile), i == 0);
-        mma_commit(bar(Smem::pv_done));
+        mma_commit(bar(Smem::pv_done + (i & 1)));
         mma_commit(bar(Smem::v_empty + (i & 1)));
         if (i + 2 < steps) {  // their columns hold the probabilities that this product reads
-          ok = mbar_wait(bar(Smem::pv_done), i & 1, abort_flag);
+          ok = mbar_wait(bar(Smem::pv_done + (i & 1)), (i >> 1) & 1, abort_flag);
           if (ok) issue_scores(i + 2);
         }
       }
@@ -282,7 +284,7 @@ __global__ void __launch_bounds__(kWideFwdThreads, 2) ta_wide_fwd_kernel(const _
       if (i > 0 && __any_sync(0xffffffffu, raised)) {
         const float shrink = raised ? ex2((ref - peak) * kLog2e) : 1.f;  // 0 for a row without a reference so far
         l_run *= shrink;
-        ok = mbar_wait(bar(Smem::pv_done), (i - 1) & 1, abort_flag);
+        ok = mbar_wait(bar(Smem::pv_done + ((i - 1) & 1)), ((i - 1) >> 1) & 1, abort_flag);
         if (!ok) break;
         tc_fence_after_sync();
 #pragma unroll 1
@@ -319,7 +321,7 @@ __global__ void __launch_bounds__(kWideFwdThreads, 2) ta_wide_fwd_kernel(const _
       tc_fence_before_sync();
       mbar_arrive_warp(bar(Smem::p_full + (i & 1)));
     }
-    if (ok) ok = mbar_wait(bar(Smem::pv_done), (steps - 1) & 1, abort_flag);
+    if (ok) ok = mbar_wait(bar(Smem::pv_done + ((steps - 1) & 1)), ((steps - 1) >> 1) & 1, abort_flag);
     if (ok) {
       tc_fence_after_sync();
       const int query = q0 + t;
@@ -356,8 +358,8 @@ struct WideBwdSmem {
   static constexpr int rows_full = 0;
   static constexpr int stage_full = 1, stage_empty = 3;  // [2]
   static constexpr int scores_full = 5, scores_taken = 7;  // [2]
-  static constexpr int sums_done = 9;
-  static constexpr int num_bars = 10;
+  static constexpr int sums_done = 9;  // [2] by step, for the same reason as the forward kernel's pv_done
+  static constexpr int num_bars = 11;
   static constexpr int tmem_slot = bars + num_bars * 8;
   static constexpr int abort_flag = tmem_slot + 4;
   static constexpr int failed = abort_flag + 4;   // a kernel before this one has given up a wait
@@ -414,7 +416,7 @@ __device__ __forceinline__ void wide_rows(const WideParams& P, uint32_t smem_bas
         ok = mbar_wait(bar(Smem::stage_full + (i & 1)), (i >> 1) & 1, abort_flag);
         // the columns hold what the sums of an earlier step read
         const int before = KIND == kKeys ? i - 1 : i - 2;
-        if (ok && before >= 0) ok = mbar_wait(bar(Smem::sums_done), before & 1, abort_flag);
+        if (ok && before >= 0) ok = mbar_wait(bar(Smem::sums_done + (before & 1)), (before >> 1) & 1, abort_flag);
         if (!ok) return;
         tc_fence_after_sync();
         score_product(tmem_base + kSCol, a0, k_major(column_tile(i, 0)), channel_steps);
@@ -431,7 +433,7 @@ __device__ __forceinline__ void wide_rows(const WideParams& P, uint32_t smem_bas
         const uint64_t b0 = k_major(column_tile(i, 0)), b1 = k_major(column_tile(i, 1));
         if (KIND == kKeys) sum_product(tmem_base + kAcc1, tmem_base + kSCol, b1, i == 0);  // dV += P^T dO
         sum_product(tmem_base + kAcc0, tmem_base + d_col(i), b0, i == 0);                  // dK += dS^T Q, dQ += dS K
-        mma_commit(bar(Smem::sums_done));
+        mma_commit(bar(Smem::sums_done + (i & 1)));
         mma_commit(bar(Smem::stage_empty + (i & 1)));
         if (KIND == kKeys && i + 1 < steps) issue_scores(i + 1);
       }
@@ -523,7 +525,7 @@ __device__ __forceinline__ void wide_rows(const WideParams& P, uint32_t smem_bas
         for (int rest = i + 1; rest < steps; ++rest) named_barrier_sync(1, kWideElemWarps * 32);
       }
     }
-    if (ok) ok = mbar_wait(bar(Smem::sums_done), (steps - 1) & 1, abort_flag);
+    if (ok) ok = mbar_wait(bar(Smem::sums_done + ((steps - 1) & 1)), ((steps - 1) >> 1) & 1, abort_flag);
     if (ok) {
       tc_fence_after_sync();
       if (KIND == kKeys) {  // a warpgroup per gradient
