@@ -274,6 +274,38 @@ int oops_ta_bias_rows(int32_t batch, int32_t groups, int32_t heads, int32_t cols
                       void* dst, void* stream);
 
 /*
+ * Up to OOPS_TA_MAX_PRODUCTS independent products C = A B^T of 16-bit operands in one launch: A is (m, k), B is (n, k), C is (m, n); a
+ * transposed operand is given as the (k, m) or (k, n) matrix that it is the transpose of, with rows `ld` elements apart.
+ * What happens to a tile of C:
+ *   PLAIN         it is rounded to the type and stored.
+ *   GATE          that, and gated = sigmoid(C) * values: row i of C belongs to column i % tokens of batch i / tokens of `values`, its
+ *                 channel j to channel j % dim of head j / dim (a pair tensor whose row axis is not used).
+ *   GATE_REVERSE  C is not stored: with C the gradient of `gated`, dvalues = C * sigmoid(gate) (skipped where its ptr is NULL) and
+ *                 the gradient of the gate, C * values * s * (1 - s), goes to `gated` (skipped where NULL).
+ * These are the products around the gate in the reference's gate_attention_output (oops/attention/gate/composed.py:47-53).
+ * n and dim are multiples of 8, all rows start on 16-byte boundaries; oops_ta_products_supported says whether a list is served.
+ */
+#define OOPS_TA_MAX_PRODUCTS 2
+enum oops_ta_product_epilogue { OOPS_TA_PRODUCT_PLAIN = 0, OOPS_TA_PRODUCT_GATE = 1, OOPS_TA_PRODUCT_GATE_REVERSE = 2 };
+typedef struct oops_ta_product {
+  const void* a;
+  int64_t a_ld;
+  const void* b;
+  int64_t b_ld;
+  void* c;
+  int64_t c_ld;
+  int32_t m, n, k, a_transposed, b_transposed, epilogue;
+  oops_ta_pair values, dvalues;
+  const void* gate;
+  int64_t gate_ld;
+  void* gated;
+  int64_t gated_ld;
+  int32_t tokens, dim;
+} oops_ta_product;
+int oops_ta_products_supported(int dtype, const oops_ta_product* list, int32_t count);
+int oops_ta_products(int dtype, const oops_ta_product* list, int32_t count, void* stream);
+
+/*
  * Forward pass that needs no workspace from the caller and allocates nothing.
  *
  * It has no counterpart in the reference.  It is for hosts that cannot hand over scratch memory when

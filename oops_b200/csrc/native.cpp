@@ -485,6 +485,9 @@ Tensor token_major(const Tensor& t, int64_t heads, int64_t dim) {
   return t.defined() ? t.view({t.size(0), 1, t.size(1), heads, dim}) : t;
 }
 
+// The same without a tensor for it.
+oops_ta_pair head_pair(const Tensor& t) { return {t.data_ptr(), t.stride(0), 0, t.stride(2), t.stride(1)}; }
+
 // gated[b, q, h * D + d] = sigmoid(gate[b, q, h * D + d]) * attention[b, h, q, d]
 struct GateFunction : Function<GateFunction> {
   static Tensor forward(AutogradContext* ctx, const Tensor& attention_in, const Tensor& gate_in) {
@@ -572,6 +575,45 @@ std::optional<Tensor> dense_gated_attention(const Tensor& query, const Tensor& k
                       scale.has_value() ? *scale : 1.0 / std::sqrt(double(query.size(-1))), flags);
 }
 
+// C = A B^T as the C ABI describes it; operands are contiguous matrices, or `.t()` of one, of more than one column.
+oops_ta_product product(const Tensor& a, const Tensor& b, const Tensor& c, int64_t m, int64_t n, int64_t k) {
+  oops_ta_product p{};
+  auto operand = [](const Tensor& t, const void*& ptr, int64_t& ld, int32_t& transposed) {
+    transposed = t.stride(0) == 1 && t.size(0) > 1;
+    ptr = t.data_ptr();
+    ld = transposed ? t.size(0) : t.size(1);
+  };
+  operand(a, p.a, p.a_ld, p.a_transposed);
+  operand(b, p.b, p.b_ld, p.b_transposed);
+  p.c = data_of(c);
+  p.c_ld = n;
+  p.m = int32_t(m);
+  p.n = int32_t(n);
+  p.k = int32_t(k);
+  return p;
+}
+
+// Whether the output step's products run on this library's kernels: `rows` of `in` channels, `inner` channels between the two products,
+// `out` channels behind.  What they save is launches (2048 rows, 384 / 1024 / 384 channels, forward and reverse: 172 us of host work a call
+// with the library's products and the gate between them, 92 with these; on the device alone 39 and 45 us, 64 rows 19.3 and 18.9).  From
+// some thousand rows on the device takes longer than the host, and the library's larger tiles are the better ones (3072 rows
+// 47 and 58 us, 12288 rows 131 and 194).
+constexpr int64_t kOwnProductValues = 2048 * 1024;
+bool own_products(at::ScalarType type, int64_t rows, int64_t in, int64_t inner, int64_t out, int64_t dim) {
+  return (type == at::kBFloat16 || type == at::kHalf) && rows > 0 && in > 0 && out > 0 && in % 8 == 0 && inner % 8 == 0 && out % 8 == 0 &&
+         dim % 8 == 0 && rows <= kOwnProductValues && in <= kOwnProductValues && inner <= kOwnProductValues && out <= kOwnProductValues &&
+         rows * std::max(std::max(in, inner), out) <= kOwnProductValues && inner * std::max(in, out) <= kOwnProductValues;
+}
+bool whole_words(const Tensor& t) {  // a matrix, or pairs, whose every eighth element starts a 16-byte word
+  if ((reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) != 0) return false;
+  for (int64_t i = 0; i < t.dim(); ++i)
+    if (t.stride(i) != 1 && t.stride(i) % 8 != 0) return false;
+  return true;
+}
+void run_products(const Tensor& like, const oops_ta_product* list, int count) {
+  check_gate_status(oops_ta_products(dtype_code(like.scalar_type()), list, count, current_stream(like)));
+}
+
 // linear(sigmoid(linear(single, gate_weight)) * attention_flat, output_weight) as one node.
 struct GateOutputFunction : Function<GateOutputFunction> {
   static Tensor forward(AutogradContext* ctx, const Tensor& attention, const Tensor& single, const Tensor& gate_weight,
@@ -580,11 +622,30 @@ struct GateOutputFunction : Function<GateOutputFunction> {
     const int64_t heads = attention.size(-3), tokens = attention.size(-2), dim = attention.size(-1);
     const Tensor values = unit_inner(attention.reshape({-1, heads, tokens, dim}));
     const Tensor rows = single.reshape({-1, single.size(-1)}), wg = gate_weight.to(type), wo = output_weight.to(type);
+    std::vector<int64_t> shape = single.sizes().vec();
+    shape.back() = wo.size(0);
+    const int64_t count = rows.size(0), in = rows.size(1), inner = heads * dim, out_channels = wo.size(0);
+    if (own_products(type, count, in, inner, out_channels, dim) && rows.is_contiguous() && wg.is_contiguous() && wo.is_contiguous() &&
+        whole_words(rows) && whole_words(wg) && whole_words(wo) && whole_words(values)) {
+      const c10::cuda::CUDAGuard guard(attention.device());
+      const Tensor gate = at::empty({count, inner}, rows.options()), gated = at::empty({count, inner}, rows.options()),
+                   out = at::empty(shape, rows.options());
+      oops_ta_product open = product(rows, wg, gate, count, inner, in);
+      open.epilogue = OOPS_TA_PRODUCT_GATE;
+      open.values = head_pair(values);
+      open.gated = gated.data_ptr();
+      open.gated_ld = inner;
+      open.tokens = int32_t(tokens);
+      open.dim = int32_t(dim);
+      run_products(rows, &open, 1);
+      const oops_ta_product project = product(gated, wo, out, count, out_channels, inner);
+      run_products(rows, &project, 1);
+      if (ctx) ctx->save_for_backward({attention, single, gate_weight, output_weight, gate, gated});
+      return out;
+    }
     const Tensor gate = at::linear(rows, wg), gated = at::empty_like(gate);
     auto as_pairs = [&](const Tensor& t) { return t.view({values.size(0), 1, tokens, heads, dim}); };
     run_gate(head_major(values), as_pairs(gate), as_pairs(gated));
-    std::vector<int64_t> shape = single.sizes().vec();
-    shape.back() = wo.size(0);
     if (ctx) ctx->save_for_backward({attention, single, gate_weight, output_weight, gate, gated});
     return at::_unsafe_view(at::linear(gated, wo), shape);
   }
@@ -603,8 +664,52 @@ struct GateOutputFunction : Function<GateOutputFunction> {
     }
     const Tensor dout = grad_outputs[0].resolve_neg().to(type).reshape({-1, wo.size(0)});
     variable_list result(4);
-    if (ctx->needs_input_grad(3)) result[3] = at::mm(dout.t(), gated).to(output_type);
     const bool need_attention = ctx->needs_input_grad(0), need_gate = ctx->needs_input_grad(1) || ctx->needs_input_grad(2);
+    const int64_t count = rows.size(0), in = rows.size(1), inner = heads * dim, out_channels = wo.size(0);
+    if (!at::GradMode::is_enabled() && own_products(type, count, in, inner, out_channels, dim) && rows.is_contiguous() && wg.is_contiguous() &&
+        wo.is_contiguous() && dout.is_contiguous() && gated.is_contiguous() && whole_words(rows) && whole_words(wg) && whole_words(wo) &&
+        whole_words(values) && whole_words(dout) && whole_words(gate) && whole_words(gated)) {
+      // Two launches: the gradient of what lies behind the gate and what follows from it, then the gate's own product.
+      const c10::cuda::CUDAGuard guard(attention.device());
+      oops_ta_product list[2];
+      int products = 0;
+      Tensor dvalues, dgate, dsingle, dwg, dwo;
+      if (ctx->needs_input_grad(3)) {
+        dwo = at::empty({out_channels, inner}, rows.options());
+        list[products++] = product(dout.t(), gated.t(), dwo, out_channels, inner, count);
+      }
+      if (need_attention || need_gate) {
+        if (need_attention) dvalues = at::empty(values.sizes(), values.options());
+        if (need_gate) dgate = at::empty({count, inner}, rows.options());
+        oops_ta_product& p = list[products++] = product(dout, wo.t(), Tensor(), count, inner, out_channels);
+        p.epilogue = OOPS_TA_PRODUCT_GATE_REVERSE;
+        p.values = head_pair(values);
+        if (need_attention) p.dvalues = head_pair(dvalues);
+        p.gate = gate.data_ptr();
+        p.gate_ld = inner;
+        p.gated = data_of(dgate);
+        p.gated_ld = inner;
+        p.tokens = int32_t(tokens);
+        p.dim = int32_t(dim);
+      }
+      if (products) run_products(rows, list, products);
+      products = 0;
+      if (ctx->needs_input_grad(2)) {
+        dwg = at::empty({inner, in}, rows.options());
+        list[products++] = product(dgate.t(), rows.t(), dwg, inner, in, count);
+      }
+      if (ctx->needs_input_grad(1)) {
+        dsingle = at::empty(single.sizes(), rows.options());
+        list[products++] = product(dgate, wg.t(), dsingle, count, in, inner);
+      }
+      if (products) run_products(rows, list, products);
+      if (need_attention) result[0] = dvalues.view(attention.sizes());
+      result[1] = dsingle;
+      if (dwg.defined()) result[2] = dwg.to(gate_type);
+      if (dwo.defined()) result[3] = dwo.to(output_type);
+      return result;
+    }
+    if (ctx->needs_input_grad(3)) result[3] = at::mm(dout.t(), gated).to(output_type);
     if (!need_attention && !need_gate) return result;
     const Tensor dgated = at::mm(dout, wo), dgate = need_gate ? at::empty_like(gate) : Tensor();
     const Tensor dvalues = need_attention ? at::empty(values.sizes(), values.options()) : Tensor();

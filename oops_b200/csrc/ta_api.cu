@@ -385,6 +385,18 @@ int oops_ta_bias_rows(int32_t batch, int32_t groups, int32_t heads, int32_t cols
   return bias_rows(batch, groups, heads, cols, src, strides, dst, reinterpret_cast<cudaStream_t>(stream));
 }
 
+int oops_ta_products_supported(int dtype, const oops_ta_product* list, int32_t count) {
+  return list && products_supported(dtype, list, count) ? 1 : 0;
+}
+
+int oops_ta_products(int dtype, const oops_ta_product* list, int32_t count, void* stream) {
+  if (!list) return fail(OOPS_TA_INVALID_ARGUMENT, "list is NULL");
+  const int status = check_device();
+  if (status) return status;
+  g_error[0] = 0;
+  return products(dtype, list, count, reinterpret_cast<cudaStream_t>(stream));
+}
+
 int oops_ta_backward(const oops_ta_problem* problem, const oops_ta_pair* out, const oops_ta_pair* dout,
                      const float* lse, const oops_ta_grads* grads, void* stream) {
   int status = validate(problem, true);
@@ -418,8 +430,8 @@ uint64_t oops_ta_forward_static_capacity(void) { return static_forward_capacity(
 
 int oops_ta_device_status(int reset) {
   const int forward = forward_device_status(reset);
-  const int backward = backward_device_status(reset), wide = wide_device_status(reset);
-  return forward ? forward : backward ? backward : wide;
+  const int backward = backward_device_status(reset), wide = wide_device_status(reset), product = products_device_status(reset);
+  return forward ? forward : backward ? backward : wide ? wide : product;
 }
 
 int oops_ta_selftest_wait_limit(void* stream) {

@@ -56,6 +56,11 @@ int wide_backward(const oops_ta_problem& p, const oops_ta_pair& dout, const floa
                   int num_parts, float* parts, cudaStream_t stream);
 int wide_device_status(int reset);
 
+// Products of 16-bit operands with the gate of an output projection in their epilogues (include/oops_ta.h).
+bool products_supported(int dtype, const oops_ta_product* list, int count);
+int products(int dtype, const oops_ta_product* list, int count, cudaStream_t stream);
+int products_device_status(int reset);
+
 // The layout-agnostic forward pass on the library's built-in scratch array (no caller workspace).
 uint64_t static_forward_capacity();
 int static_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, cudaStream_t stream);

@@ -40,6 +40,7 @@ EXPORTS = (
     "oops_ta_layer_norm_backward", "oops_ta_pair_gate_forward", "oops_ta_pair_gate_backward",
     "oops_ta_channel_norm_forward", "oops_ta_channel_norm_backward_workspace_bytes", "oops_ta_channel_norm_backward",
     "oops_ta_output_gate_forward", "oops_ta_output_gate_backward", "oops_ta_bias_rows",
+    "oops_ta_products_supported", "oops_ta_products",
 )
 
 
