@@ -45,39 +45,54 @@ constexpr int kRing = 4;                                // ring depth of the str
 // small helper kernels
 // ---------------------------------------------------------------------------------------------
 
-// delta[b][r][h][q] = sum_d O * dO.  Four lanes share a (cell, head): a warp reads 512 contiguous bytes of each tensor when
-// heads and cells are contiguous (one lane per (cell, head) read 64 bytes at 64-byte strides).  `row_inner`: cells of
-// neighbouring rows, not columns, are neighbours in memory (the ending-node form).  The blocks behind those of delta look at
+// delta[b][r][h][q] = sum_d O * dO.  Four lanes share a cell and take its heads four at a time: a warp's loads cover eight cells, 64 bytes of
+// a head each, and the lanes end with a head's sum each.  `row_inner`: cells of
+// neighbouring rows, not columns, are neighbours in memory (the ending-node form).  The first blocks look at
 // the mask: live[b][r] has bit k set when some key of columns 128 k .. 128 k + 127 of the row is kept, the
 // second word of a row whether all of them are, the third how many keys a row keeps if these are its first ones (else ~0), and
 // behind the rows' words one word per eight rows tells whether they drop any key.
+// Bound by HBM.  With a (cell, head) per four lanes the divisions that place it were as many instructions as HBM had time for, and the
+// mask's blocks, last in the grid and a load at a time, ran on alone.  N = 256, two samples: 18.4 -> 11.7 us; N = 768: 71.8 -> 50.3 us
+// (302 MB of tensors and 9 of sums: 6.2 TB/s of the copy's 6.56).
 template <typename T>
-__global__ void __launch_bounds__(256, 8) prepare_kernel(oops_ta_pair out, oops_ta_pair dout, float* delta, uint32_t total, int cols,
-                                                      int heads, int rows, int vec_ok, int row_inner, uint32_t delta_blocks,
+__global__ void __launch_bounds__(256, 4) prepare_kernel(oops_ta_pair out, oops_ta_pair dout, float* delta, uint32_t cells, int cols,
+                                                      int heads, int rows, int vec_ok, int row_inner, uint32_t mask_blocks,
                                                       const uint8_t* mask, int64_t m_sb, int64_t m_sr, int64_t m_sc,
                                                       uint32_t* live, int num_rows) {
-  if (blockIdx.x >= delta_blocks) {
-    const int block = int(blockIdx.x - delta_blocks), row = block * 8 + int(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (blockIdx.x < mask_blocks) {
+    const int block = int(blockIdx.x), row = block * 8 + int(threadIdx.x >> 5), lane = threadIdx.x & 31;
     bool dropped = false;
     if (row < num_rows) {
       const uint8_t* bytes = mask + (row / rows) * m_sb + int64_t(row % rows) * m_sr;
       uint32_t bits = 0, full = 0;
       int count = 0, end = 0;  // kept keys, and one behind the last of them
-      for (int first = 0; first < cols; first += 128) {
-        bool any = false, all = true;
+      constexpr int kBatch = 16;  // words of 32 keys whose bytes travel together
+      for (int first = 0; first < cols; first += kBatch * 32) {
+        uint32_t kept[kBatch];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < kBatch; ++i) {
           const int key = first + i * 32 + lane;
-          const bool keep = key < cols && bytes[int64_t(key) * m_sc] != 0;
-          any |= keep;
-          all &= keep || key >= cols;
-          const uint32_t kept = __ballot_sync(0xffffffffu, keep);
-          count += __popc(kept);
-          if (kept != 0) end = first + i * 32 + 32 - __clz(int(kept));
+          kept[i] = key < cols ? ldg_u8_here(bytes + int64_t(key) * m_sc) : 0u;
         }
-        if (__any_sync(0xffffffffu, any)) bits |= 1u << (first / 128);
-        if (__all_sync(0xffffffffu, all)) full |= 1u << (first / 128);
-        else dropped = true;
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) kept[i] = __ballot_sync(0xffffffffu, kept[i] != 0);
+#pragma unroll
+        for (int tile = 0; tile < kBatch / 4; ++tile) {
+          uint32_t any = 0;
+          int wanted = 0, found = 0;
+#pragma unroll
+          for (int i = 4 * tile; i < 4 * tile + 4; ++i) {
+            any |= kept[i];
+            found += __popc(kept[i]);
+            wanted += min(32, max(0, cols - (first + i * 32)));
+            if (kept[i] != 0) end = first + i * 32 + 32 - __clz(int(kept[i]));
+          }
+          count += found;
+          if (wanted == 0) break;
+          if (any != 0) bits |= 1u << (first / 128 + tile);
+          if (found == wanted) full |= 1u << (first / 128 + tile);
+          else dropped = true;
+        }
       }
       if (lane == 0) {
         live[row] = bits;
@@ -89,31 +104,48 @@ __global__ void __launch_bounds__(256, 8) prepare_kernel(oops_ta_pair out, oops_
     if (threadIdx.x == 0) live[3 * num_rows + block] = uint32_t(drops != 0);
     return;
   }
-  const uint32_t item = blockIdx.x * 64u + (threadIdx.x >> 2);
+  const uint32_t cell = (blockIdx.x - mask_blocks) * 64u + (threadIdx.x >> 2);
   const int part = threadIdx.x & 3;
-  float dot = 0.f;
-  int64_t at = 0;
-  if (item < total) {
-    const uint32_t h = item % uint32_t(heads), cell = item / uint32_t(heads);
-    const uint32_t inner = row_inner ? uint32_t(rows) : uint32_t(cols), outer = row_inner ? uint32_t(cols) : uint32_t(rows);
-    const uint32_t i = cell % inner, rest = cell / inner, o = rest % outer, b = rest / outer;
-    const uint32_t r = row_inner ? i : o, q = row_inner ? o : i;
-    const T* po = reinterpret_cast<const T*>(out.ptr) + b * out.sb + int64_t(r) * out.sr + int64_t(q) * out.sc + h * out.sh + part * 8;
-    const T* pd = reinterpret_cast<const T*>(dout.ptr) + b * dout.sb + int64_t(r) * dout.sr + int64_t(q) * dout.sc + h * dout.sh + part * 8;
-    at = ((int64_t(b) * rows + r) * heads + h) * cols + q;
+  const bool there = cell < cells;  // (a warp's lanes stay together for the exchange)
+  const uint32_t inner = row_inner ? uint32_t(rows) : uint32_t(cols), outer = row_inner ? uint32_t(cols) : uint32_t(rows);
+  const uint32_t i = cell % inner, rest = cell / inner, o = rest % outer, b = rest / outer;
+  const uint32_t r = row_inner ? i : o, q = row_inner ? o : i;
+  const T* po = reinterpret_cast<const T*>(out.ptr) + b * out.sb + int64_t(r) * out.sr + int64_t(q) * out.sc + part * 8;
+  const T* pd = reinterpret_cast<const T*>(dout.ptr) + b * dout.sb + int64_t(r) * dout.sr + int64_t(q) * dout.sc + part * 8;
+  float* to = delta + (int64_t(b) * rows + r) * heads * cols + q;
+  for (int h0 = 0; h0 < heads; h0 += 4) {
+    float dot[4] = {0.f, 0.f, 0.f, 0.f};
     if (vec_ok) {
-      const uint4 a = *reinterpret_cast<const uint4*>(po), g = *reinterpret_cast<const uint4*>(pd);
-      const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
+      uint4 a[4], g[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) dot += Half2<T>::lo(aw[e]) * Half2<T>::lo(gw[e]) + Half2<T>::hi(aw[e]) * Half2<T>::hi(gw[e]);
-    } else {
+      for (int n = 0; n < 4; ++n) {
+        const bool take = there && h0 + n < heads;
+        a[n] = ldg_v4_here_if(po + int64_t(h0 + n) * out.sh, take);
+        g[n] = ldg_v4_here_if(pd + int64_t(h0 + n) * dout.sh, take);
+      }
 #pragma unroll
-      for (int c = 0; c < 8; ++c) dot += float(po[c]) * float(pd[c]);
+      for (int n = 0; n < 4; ++n) {
+        const uint32_t aw[4] = {a[n].x, a[n].y, a[n].z, a[n].w}, gw[4] = {g[n].x, g[n].y, g[n].z, g[n].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) dot[n] += Half2<T>::lo(aw[e]) * Half2<T>::lo(gw[e]) + Half2<T>::hi(aw[e]) * Half2<T>::hi(gw[e]);
+      }
+    } else if (there) {
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        if (h0 + n >= heads) break;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) dot[n] += float(po[int64_t(h0 + n) * out.sh + c]) * float(pd[int64_t(h0 + n) * dout.sh + c]);
+      }
     }
+    float own = 0.f;
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      dot[n] += __shfl_xor_sync(0xffffffffu, dot[n], 1);
+      dot[n] += __shfl_xor_sync(0xffffffffu, dot[n], 2);
+      if (n == part) own = dot[n];
+    }
+    if (there && h0 + part < heads) to[int64_t(h0 + part) * cols] = own;
   }
-  dot += __shfl_xor_sync(0xffffffffu, dot, 1);
-  dot += __shfl_xor_sync(0xffffffffu, dot, 2);
-  if (item < total && part == 0) delta[at] = dot;
 }
 
 // Whether the mask that prepare_kernel has looked at keeps every key (one warp's answer).
@@ -147,19 +179,31 @@ __global__ void transpose_bias_kernel(const uint16_t* src, uint16_t* dst, int co
   }
 }
 
+// dbias = the sum of its parts in their order.  `quads`: a thread takes four keys, whose rows are whole 16-byte words (N = 256, two
+// samples: 9.2 -> 5.0 us; the ragged sample of 700 tokens: 45.8 -> 11.9).
 template <typename T>
-__global__ void reduce_parts_kernel(const float* parts, int num_parts, void* dbias, int64_t sb, int64_t sh, int64_t sq,
-                                    int64_t sk, int batch, int heads, int cols) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t plane = int64_t(batch) * heads * cols * cols;
+__global__ void __launch_bounds__(256) reduce_parts_kernel(const float* parts, int num_parts, void* dbias, int64_t sb, int64_t sh, int64_t sq,
+                                                           int64_t sk, int heads, int cols, int64_t plane, int quads) {
+  const int64_t at = int64_t(blockIdx.x) * 256 + threadIdx.x, i = quads ? at * 4 : at;
   if (i >= plane) return;
-  float total = 0.f;
-  for (int p = 0; p < num_parts; ++p) total += parts[int64_t(p) * plane + i];
-  const int k = i % cols;
-  const int q = (i / cols) % cols;
-  const int h = (i / (int64_t(cols) * cols)) % heads;
-  const int64_t b = i / (int64_t(cols) * cols * heads);
-  reinterpret_cast<T*>(dbias)[b * sb + h * sh + int64_t(q) * sq + int64_t(k) * sk] = T(total);
+  const int64_t row = i / cols;  // (batch, head, query)
+  const int k = int(i - row * cols), q = int(row % cols), h = int(row / cols % heads);
+  T* to = reinterpret_cast<T*>(dbias) + row / cols / heads * sb + h * sh + int64_t(q) * sq + int64_t(k) * sk;
+  if (quads) {
+    float4 total = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int p = 0; p < num_parts; ++p) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(parts + int64_t(p) * plane + i));
+      total = make_float4(total.x + v.x, total.y + v.y, total.z + v.z, total.w + v.w);
+    }
+    if constexpr (sizeof(T) == 4) *reinterpret_cast<float4*>(to) = total;
+    else *reinterpret_cast<uint2*>(to) = make_uint2(Half2<T>::pack(total.x, total.y), Half2<T>::pack(total.z, total.w));
+  } else {
+    float total = 0.f;
+#pragma unroll 4
+    for (int p = 0; p < num_parts; ++p) total += __ldg(parts + int64_t(p) * plane + i);
+    *to = T(total);
+  }
 }
 
 // 16-bit row store of 32 channels from f32 accumulator words, scaled.
@@ -1985,14 +2029,15 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
   // delta = rowsum(O * dO), unless an earlier call has left it, and what the kernels ask about the mask, which they must find
   // whatever the workspace holds (a second call with a mask: 159 -> 169 us at 96 rows of 768 columns, 1165 -> 1168 at 768).
   const int64_t total = (p.flags & OOPS_TA_FLAG_REUSE_DELTA) != 0 ? 0 : int64_t(p.batch) * p.rows * p.heads * p.cols;
-  const unsigned delta_blocks = (unsigned)ceil_div(total, 64);
+  const int64_t cells = p.heads > 0 ? total / p.heads : 0;
+  const unsigned delta_blocks = (unsigned)ceil_div(cells, 64);
   const unsigned mask_blocks = live ? (unsigned)ceil_div(int64_t(p.batch) * p.rows, 8) : 0u;
   if (delta_blocks + mask_blocks > 0) {
     const int vec_ok = (reinterpret_cast<uintptr_t>(out.ptr) & 15) == 0 && (reinterpret_cast<uintptr_t>(dout.ptr) & 15) == 0 &&
                        out.sb % 8 == 0 && out.sr % 8 == 0 && out.sc % 8 == 0 && out.sh % 8 == 0 && dout.sb % 8 == 0 &&
                        dout.sr % 8 == 0 && dout.sc % 8 == 0 && dout.sh % 8 == 0;
-    prepare_kernel<T><<<delta_blocks + mask_blocks, 256, 0, stream>>>(out, dout, delta, (uint32_t)total, p.cols, p.heads, p.rows, vec_ok,
-                                                                      dout.sr < dout.sc, delta_blocks, p.mask, p.mask_sb, p.mask_sr,
+    prepare_kernel<T><<<delta_blocks + mask_blocks, 256, 0, stream>>>(out, dout, delta, (uint32_t)cells, p.cols, p.heads, p.rows, vec_ok,
+                                                                      dout.sr < dout.sc, mask_blocks, p.mask, p.mask_sb, p.mask_sr,
                                                                       p.mask_sc, live, p.batch * p.rows);
     count_launch();
     status = check_launch("tcgen05 delta");
@@ -2186,12 +2231,15 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
     if (status) return status;
     if (P.num_parts > 1) {
       const int64_t plane = int64_t(p.batch) * p.heads * p.cols * p.cols;
+      const int quads = p.cols % 4 == 0 && g.dbias_sk == 1 && (reinterpret_cast<uintptr_t>(g.dbias) & 15) == 0 && g.dbias_sb % 4 == 0 &&
+                        g.dbias_sh % 4 == 0 && g.dbias_sq % 4 == 0;
+      const unsigned blocks = (unsigned)ceil_div(quads ? plane / 4 : plane, 256);
       if (P.dbias_f32)
-        reduce_parts_kernel<float><<<(unsigned)ceil_div(plane, 256), 256, 0, stream>>>(
-            P.parts, P.num_parts, g.dbias, g.dbias_sb, g.dbias_sh, g.dbias_sq, g.dbias_sk, p.batch, p.heads, p.cols);
+        reduce_parts_kernel<float><<<blocks, 256, 0, stream>>>(P.parts, P.num_parts, g.dbias, g.dbias_sb, g.dbias_sh, g.dbias_sq, g.dbias_sk,
+                                                               p.heads, p.cols, plane, quads);
       else
-        reduce_parts_kernel<T><<<(unsigned)ceil_div(plane, 256), 256, 0, stream>>>(
-            P.parts, P.num_parts, g.dbias, g.dbias_sb, g.dbias_sh, g.dbias_sq, g.dbias_sk, p.batch, p.heads, p.cols);
+        reduce_parts_kernel<T><<<blocks, 256, 0, stream>>>(P.parts, P.num_parts, g.dbias, g.dbias_sb, g.dbias_sh, g.dbias_sq, g.dbias_sk,
+                                                           p.heads, p.cols, plane, quads);
       count_launch();
       status = check_launch("tcgen05 shared-bias reduce");
       if (status) return status;
