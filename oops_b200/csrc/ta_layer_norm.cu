@@ -11,6 +11,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <initializer_list>
 #include <type_traits>
 
@@ -22,13 +23,7 @@ namespace {
 constexpr int kLnWarps = 8;             // warps (= rows in flight) per CTA
 constexpr int kLnCached = 1024;         // widest row kept in registers
 constexpr int kLnPerLane = kLnCached / 32;
-#ifndef TA_LN_CTAS
-#define TA_LN_CTAS 4
-#endif
-#ifndef TA_LN_UNROLL
-#define TA_LN_UNROLL 4
-#endif
-constexpr int kLnCtasPerSm = TA_LN_CTAS;        // resident CTAs the row-sharing kernels are compiled for (register cap 64)
+constexpr int kLnCtasPerSm = 4;         // most CTAs that a launch has per SM
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -261,7 +256,7 @@ __global__ void __launch_bounds__(kLnWarps * 32) layer_norm_backward_kernel(LnSh
 // ---- rows of up to 1024 elements with 16-byte accesses: LPR lanes share a row, each holding GROUPS groups of V
 // elements; a warp works on 32 / LPR rows at once and on kLnUnroll such row blocks per loop turn, so that enough
 // loads are in flight to cover the memory latency (a 128-channel bf16 row is only 256 bytes).
-constexpr int kLnUnroll = TA_LN_UNROLL;
+constexpr int kLnUnroll = 4;
 
 template <int LPR>
 __device__ __forceinline__ float row_sum(float v) {
@@ -317,8 +312,30 @@ __device__ __forceinline__ uint4 ln_pack2(const ln2 (&in)[V / 2]) {
   }
 }
 
-template <typename T, typename A, int V, int GROUPS, int LPR>
-__global__ void __launch_bounds__(kLnWarps * 32, GROUPS == 1 ? kLnCtasPerSm : 1) layer_norm_forward_rows_kernel(LnShape s, const T* __restrict__ x,
+// Row blocks that a lane has asked for stand in shared memory, 16 bytes of its own each, which no other lane touches: the blocks of the
+// next turn travel under the arithmetic of this one, and cost no registers (held in registers they spill).  A warp's blocks of a turn
+// are neighbours, 2 KB in a row.  768 x 768 rows of 128 channels, bf16: forward 64.9 -> 50.8 us (5.9 TB/s; the copy reaches 6.56),
+// reverse 86.9 -> 75.0 (6.0 TB/s); 200000 rows of 256: 39.6 -> 30.5 and 68.1 -> 53.9; f32 rows of 512 bytes that fill the L2 several times over
+// were at 6.2 TB/s and stay there.
+constexpr int ln_turn(int groups, int tensors, bool staged) { return staged ? kLnUnroll / (groups * tensors) : kLnUnroll / tensors; }  // row blocks
+// Resident CTAs per SM: with a turn ahead, two keep HBM busy and have the registers for four blocks' arithmetic side by side; f32 forward
+// rows need fewer registers (700000 x 128: 120 us with two, 116 with three, 131 with four).
+constexpr int ln_ctas(int tensors, int size, bool staged) { return !staged ? kLnCtasPerSm : size == 4 && tensors == 1 ? 3 : 2; }
+constexpr int kLnStage = kLnUnroll * kLnWarps * 32 * 16;  // bytes of a turn of a CTA, whatever the groups and tensors
+__device__ __forceinline__ void ln_copy16(uint32_t to, const void* from, bool take) {  // zeros where it is not taken
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from), "r"(take ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void ln_copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void ln_copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ uint4 ln_take16(uint32_t at) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
+  return v;
+}
+
+template <typename T, typename A, int V, int GROUPS, int LPR, bool STAGED>
+__global__ void __launch_bounds__(kLnWarps * 32, STAGED || GROUPS == 1 ? ln_ctas(1, sizeof(T), STAGED) : 1) layer_norm_forward_rows_kernel(LnShape s, const T* __restrict__ x,
                                                                                 const void* __restrict__ weight,
                                                                                 const void* __restrict__ bias, float eps,
                                                                                 T* __restrict__ y, float* __restrict__ mean_out,
@@ -339,23 +356,59 @@ __global__ void __launch_bounds__(kLnWarps * 32, GROUPS == 1 ? kLnCtasPerSm : 1)
     }
   const int64_t blocks = (s.rows + kRowsPerWarp - 1) / kRowsPerWarp;  // row blocks of one warp
   const int64_t stride = int64_t(gridDim.x) * kLnWarps;
-  for (int64_t blk0 = int64_t(blockIdx.x) * kLnWarps + warp; blk0 < blocks; blk0 += stride * kLnUnroll) {
-    uint4 raw[kLnUnroll][GROUPS];
+  constexpr int kTurn = ln_turn(GROUPS, 1, STAGED);
+  extern __shared__ __align__(16) float ln_smem[];
+  const uint32_t mine = (uint32_t)__cvta_generic_to_shared(ln_smem) + threadIdx.x * 16;
+  constexpr uint32_t kPiece = kLnWarps * 32 * 16;  // 16 bytes of every lane
+  // A warp's blocks of a turn are neighbours.  `left` rows are there from the turn's first one on; a turn later they are `ahead` fewer.
+  constexpr int64_t apart = kRowsPerWarp;
+  const int64_t ahead = stride * kTurn * kRowsPerWarp, x_apart = apart * s.x_stride, y_apart = apart * s.y_stride;
+  const int64_t first = (int64_t(blockIdx.x) * kLnWarps + warp) * kTurn;
+  int64_t row = first * kRowsPerWarp + sub, left = s.rows - row;
+  const T* from = x + row * s.x_stride + l * V;
+  T* to = y + row * s.y_stride + l * V;
+  auto request = [&](int64_t left, uint32_t at) {  // `from` is the turn's first row
 #pragma unroll
-    for (int u = 0; u < kLnUnroll; ++u) {
-      const int64_t row = (blk0 + u * stride) * kRowsPerWarp + sub;
+    for (int u = 0; u < kTurn; ++u) {
 #pragma unroll
       for (int g = 0; g < GROUPS; ++g) {
-        const int i = (g * LPR + l) * V;
-        raw[u][g] = make_uint4(0, 0, 0, 0);  // zero bits are 0.0 in every served type
-        if (blk0 + u * stride < blocks && row < s.rows && i < s.width)
-          raw[u][g] = *reinterpret_cast<const uint4*>(x + row * s.x_stride + i);
+        const bool take = u * apart < left && (g * LPR + l) * V < s.width;
+        ln_copy16(at + (u * GROUPS + g) * kPiece, take ? from + u * x_apart + g * LPR * V : x, take);
       }
     }
+    from += ahead * s.x_stride;
+  };
+  if constexpr (STAGED) {
+    request(left, mine);
+    ln_copies_commit();
+  }
+  uint32_t stage = 0;
+  for (int64_t blk0 = first; blk0 < blocks; blk0 += stride * kTurn, row += ahead, left -= ahead, to += ahead * s.y_stride) {
+    uint4 raw[kTurn][GROUPS];
+    if constexpr (STAGED) {
+      request(left - ahead, mine + (stage ^ kLnStage));
+      ln_copies_commit();
+      ln_copies_wait<1>();
 #pragma unroll
-    for (int u = 0; u < kLnUnroll; ++u) {
-      const int64_t row = (blk0 + u * stride) * kRowsPerWarp + sub;
-      const bool live = blk0 + u * stride < blocks && row < s.rows;
+      for (int u = 0; u < kTurn; ++u)
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) raw[u][g] = ln_take16(mine + stage + (u * GROUPS + g) * kPiece);
+      stage ^= kLnStage;
+    } else {
+#pragma unroll
+      for (int u = 0; u < kTurn; ++u) {
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) {
+          raw[u][g] = make_uint4(0, 0, 0, 0);  // zero bits are 0.0 in every served type
+          if (u * apart < left && (g * LPR + l) * V < s.width)
+            raw[u][g] = *reinterpret_cast<const uint4*>(from + u * x_apart + g * LPR * V);
+        }
+      }
+      from += ahead * s.x_stride;
+    }
+#pragma unroll
+    for (int u = 0; u < kTurn; ++u) {
+      const bool live = u * apart < left;
       ln2 v[GROUPS][P];
       ln2 sum2 = ln_both(0.f);
 #pragma unroll
@@ -379,8 +432,8 @@ __global__ void __launch_bounds__(kLnWarps * 32, GROUPS == 1 ? kLnCtasPerSm : 1)
       const float rstd = rsqrtf(row_sum<LPR>(sq2.x + sq2.y) * inv_width + eps);
       if (!live) continue;
       if (l == 0) {
-        if (mean_out) mean_out[row] = mean;
-        if (rstd_out) rstd_out[row] = rstd;
+        if (mean_out) mean_out[row + u * apart] = mean;
+        if (rstd_out) rstd_out[row + u * apart] = rstd;
       }
       const ln2 rstd2 = ln_both(rstd);
 #pragma unroll
@@ -390,15 +443,15 @@ __global__ void __launch_bounds__(kLnWarps * 32, GROUPS == 1 ? kLnCtasPerSm : 1)
           ln2 out[P];
 #pragma unroll
           for (int e = 0; e < P; ++e) out[e] = ln_fma2(ln_mul2(v[g][e], rstd2), w[g][e], b[g][e]);
-          *reinterpret_cast<uint4*>(y + row * s.y_stride + i) = ln_pack2<T, V>(out);
+          *reinterpret_cast<uint4*>(to + u * y_apart + g * LPR * V) = ln_pack2<T, V>(out);
         }
       }
     }
   }
 }
 
-template <typename T, typename A, int V, int GROUPS, int LPR>
-__global__ void __launch_bounds__(kLnWarps * 32, GROUPS == 1 ? kLnCtasPerSm : 1) layer_norm_backward_rows_kernel(LnShape s, const T* __restrict__ dy,
+template <typename T, typename A, int V, int GROUPS, int LPR, bool STAGED>
+__global__ void __launch_bounds__(kLnWarps * 32, STAGED || GROUPS == 1 ? ln_ctas(2, sizeof(T), STAGED) : 1) layer_norm_backward_rows_kernel(LnShape s, const T* __restrict__ dy,
                                                                                  const T* __restrict__ x,
                                                                                  const void* __restrict__ weight,
                                                                                  const float* __restrict__ mean_in,
@@ -406,8 +459,8 @@ __global__ void __launch_bounds__(kLnWarps * 32, GROUPS == 1 ? kLnCtasPerSm : 1)
                                                                                  T* __restrict__ dx, float* __restrict__ dw_parts,
                                                                                  float* __restrict__ db_parts) {
   constexpr int kRowsPerWarp = 32 / LPR, P = V / 2;
-  constexpr int kU = kLnUnroll / 2;  // two tensors are read per row
-  extern __shared__ float ln_smem[];  // [kLnWarps * kRowsPerWarp][width] when partials are wanted
+  constexpr int kU = ln_turn(GROUPS, 2, STAGED);  // two tensors are read per row
+  extern __shared__ __align__(16) float ln_smem[];  // two turns' row blocks; then [kLnWarps * kRowsPerWarp][width] when partials are wanted
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / LPR, l = lane % LPR;
   const float inv_width = 1.f / float(s.width);
   ln2 w[GROUPS][P], dw[GROUPS][P], db[GROUPS][P];
@@ -422,29 +475,81 @@ __global__ void __launch_bounds__(kLnWarps * 32, GROUPS == 1 ? kLnCtasPerSm : 1)
     }
   const int64_t blocks = (s.rows + kRowsPerWarp - 1) / kRowsPerWarp;
   const int64_t stride = int64_t(gridDim.x) * kLnWarps;
-  for (int64_t blk0 = int64_t(blockIdx.x) * kLnWarps + warp; blk0 < blocks; blk0 += stride * kU) {
+  const uint32_t mine = (uint32_t)__cvta_generic_to_shared(ln_smem) + threadIdx.x * 16;
+  constexpr uint32_t kPiece = kLnWarps * 32 * 16;  // 16 bytes of every lane
+  // A warp's blocks of a turn are neighbours.  `left` rows are there from the turn's first one on; a turn later they are `ahead` fewer.
+  constexpr int64_t apart = kRowsPerWarp;
+  const int64_t ahead = stride * kU * kRowsPerWarp, x_apart = apart * s.x_stride, g_apart = apart * s.dy_stride, d_apart = apart * s.dx_stride;
+  const int64_t first = (int64_t(blockIdx.x) * kLnWarps + warp) * kU, row0 = first * kRowsPerWarp + sub;
+  int64_t left = s.rows - row0;
+  const T* from_x = x + row0 * s.x_stride + l * V;
+  const T* from_g = dy + row0 * s.dy_stride + l * V;
+  T* to = dx + row0 * s.dx_stride + l * V;
+  const float* mean_at = mean_in + row0;
+  const float* rstd_at = rstd_in + row0;
+  float mean_next[kU], rstd_next[kU];
+  auto request = [&](int64_t left, uint32_t at) {  // the pointers are at the turn's first row
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const bool there = u * apart < left;
+      mean_next[u] = there ? mean_at[u * apart] : 0.f;
+      rstd_next[u] = there ? rstd_at[u * apart] : 0.f;
+      if constexpr (STAGED) {
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) {
+          const bool take = there && (g * LPR + l) * V < s.width;
+          ln_copy16(at + (2 * (u * GROUPS + g)) * kPiece, take ? from_x + u * x_apart + g * LPR * V : x, take);
+          ln_copy16(at + (2 * (u * GROUPS + g) + 1) * kPiece, take ? from_g + u * g_apart + g * LPR * V : dy, take);
+        }
+      }
+    }
+    mean_at += ahead;
+    rstd_at += ahead;
+    if constexpr (STAGED) {
+      from_x += ahead * s.x_stride;
+      from_g += ahead * s.dy_stride;
+      ln_copies_commit();
+    }
+  };
+  request(left, mine);
+  uint32_t stage = 0;
+  for (int64_t blk0 = first; blk0 < blocks; blk0 += stride * kU, left -= ahead, to += ahead * s.dx_stride) {
     uint4 xraw[kU][GROUPS], graw[kU][GROUPS];
     float mean[kU], rstd[kU];
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
-      const int64_t row = (blk0 + u * stride) * kRowsPerWarp + sub;
-      const bool live = blk0 + u * stride < blocks && row < s.rows;
-      mean[u] = live ? mean_in[row] : 0.f;
-      rstd[u] = live ? rstd_in[row] : 0.f;
+      mean[u] = mean_next[u];
+      rstd[u] = rstd_next[u];
+    }
+    request(left - ahead, mine + (stage ^ kLnStage));
+    if constexpr (STAGED) {
+      ln_copies_wait<1>();
 #pragma unroll
-      for (int g = 0; g < GROUPS; ++g) {
-        const int i = (g * LPR + l) * V;
-        xraw[u][g] = graw[u][g] = make_uint4(0, 0, 0, 0);
-        if (live && i < s.width) {
-          xraw[u][g] = *reinterpret_cast<const uint4*>(x + row * s.x_stride + i);
-          graw[u][g] = *reinterpret_cast<const uint4*>(dy + row * s.dy_stride + i);
+      for (int u = 0; u < kU; ++u)
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) {
+          xraw[u][g] = ln_take16(mine + stage + (2 * (u * GROUPS + g)) * kPiece);
+          graw[u][g] = ln_take16(mine + stage + (2 * (u * GROUPS + g) + 1) * kPiece);
+        }
+      stage ^= kLnStage;
+    } else {
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) {
+          xraw[u][g] = graw[u][g] = make_uint4(0, 0, 0, 0);
+          if (u * apart < left && (g * LPR + l) * V < s.width) {
+            xraw[u][g] = *reinterpret_cast<const uint4*>(from_x + u * x_apart + g * LPR * V);
+            graw[u][g] = *reinterpret_cast<const uint4*>(from_g + u * g_apart + g * LPR * V);
+          }
         }
       }
+      from_x += ahead * s.x_stride;
+      from_g += ahead * s.dy_stride;
     }
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
-      const int64_t row = (blk0 + u * stride) * kRowsPerWarp + sub;
-      const bool live = blk0 + u * stride < blocks && row < s.rows;
+      const bool live = u * apart < left;
       const ln2 rstd2 = ln_both(rstd[u]), neg_mean2 = ln_both(-mean[u]);
       ln2 xh[GROUPS][P], gw[GROUPS][P];
       ln2 c1 = ln_both(0.f), c2 = ln_both(0.f);
@@ -474,7 +579,7 @@ __global__ void __launch_bounds__(kLnWarps * 32, GROUPS == 1 ? kLnCtasPerSm : 1)
           ln2 out[P];
 #pragma unroll
           for (int e = 0; e < P; ++e) out[e] = ln_mul2(ln_fma2(xh[g][e], neg_m1, ln_add2(gw[g][e], neg_m2)), rstd2);
-          *reinterpret_cast<uint4*>(dx + row * s.dx_stride + i) = ln_pack2<T, V>(out);
+          *reinterpret_cast<uint4*>(to + u * d_apart + g * LPR * V) = ln_pack2<T, V>(out);
         }
       }
     }
@@ -552,11 +657,11 @@ __global__ void __launch_bounds__(256) layer_norm_reduce_parts_kernel(const floa
 constexpr int kLnMaxWidth = 8192;
 constexpr int kLnWideParts = 64;
 
-int ln_grid(int64_t rows) {
+int ln_grid(int64_t rows, int ctas = kLnCtasPerSm) {
   int device = 0, sms = 148;
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   const int64_t wanted = (rows + kLnWarps - 1) / kLnWarps;
-  return int(wanted < int64_t(sms) * kLnCtasPerSm ? wanted : int64_t(sms) * kLnCtasPerSm);
+  return int(wanted < int64_t(sms) * ctas ? wanted : int64_t(sms) * ctas);
 }
 
 bool ln_vector_ok(int vec, int width, std::initializer_list<const void*> pointers, std::initializer_list<int64_t> strides) {
@@ -579,15 +684,19 @@ int forward_typed(const LnShape& s, const void* x, const void* weight, const voi
   T* yp = reinterpret_cast<T*>(y);
   const int units = (s.width + kVec - 1) / kVec;  // 16-byte groups of a row
   if (vec && units <= 128) {
-#define OOPS_LN_FWD(GROUPS, LPR)                                                                                         \
-  layer_norm_forward_rows_kernel<T, A, kVec, GROUPS, LPR>                                                                \
-      <<<ln_grid((s.rows + 32 / LPR - 1) / (32 / LPR)), threads, 0, stream>>>(s, xp, weight, bias, eps, yp, mean, rstd)
-    if (units <= 8) OOPS_LN_FWD(1, 8);
-    else if (units <= 16) OOPS_LN_FWD(1, 16);
-    else if (units <= 32) OOPS_LN_FWD(1, 32);
-    else if (units <= 64) OOPS_LN_FWD(2, 32);
-    else OOPS_LN_FWD(4, 32);
-#undef OOPS_LN_FWD
+    auto rows = [&](auto groups, auto lanes, auto staged) {
+      constexpr int GROUPS = decltype(groups)::value, LPR = decltype(lanes)::value;
+      constexpr bool STAGED = decltype(staged)::value;
+      layer_norm_forward_rows_kernel<T, A, kVec, GROUPS, LPR, STAGED>
+          <<<ln_grid((s.rows + 32 / LPR - 1) / (32 / LPR), ln_ctas(1, sizeof(T), STAGED)), threads, STAGED ? 2 * kLnStage : 0, stream>>>(
+              s, xp, weight, bias, eps, yp, mean, rstd);
+    };
+    using std::integral_constant;
+    if (units <= 8) rows(integral_constant<int, 1>{}, integral_constant<int, 8>{}, std::true_type{});
+    else if (units <= 16) rows(integral_constant<int, 1>{}, integral_constant<int, 16>{}, std::true_type{});
+    else if (units <= 32) rows(integral_constant<int, 2>{}, integral_constant<int, 16>{}, std::true_type{});
+    else if (units <= 64) rows(integral_constant<int, 2>{}, integral_constant<int, 32>{}, std::true_type{});
+    else rows(integral_constant<int, 4>{}, integral_constant<int, 32>{}, std::false_type{});
   } else if (cached && vec)
     layer_norm_forward_kernel<T, A, kVec, true><<<grid, threads, 0, stream>>>(s, xp, weight, bias, eps, yp, mean, rstd);
   else if (cached)
@@ -610,7 +719,8 @@ int backward_typed(const LnShape& s, const void* dy, const void* x, const void* 
   const int units = (s.width + kVec - 1) / kVec;
   const bool shared_rows = vec && units <= 128;  // several lanes (not always a whole warp) share a row
   const int lpr = units <= 8 ? 8 : units <= 16 ? 16 : 32;
-  if (shared_rows) grid = ln_grid((s.rows + 32 / lpr - 1) / (32 / lpr));
+  const bool staged = units <= 64;
+  if (shared_rows) grid = ln_grid((s.rows + 32 / lpr - 1) / (32 / lpr), ln_ctas(2, sizeof(T), staged));
   const int num_parts = cached ? grid : int(s.rows < kLnWideParts ? s.rows : kLnWideParts);
   float* dw_parts = dweight ? workspace : nullptr;
   float* db_parts = dbias ? workspace + int64_t(num_parts) * s.width : nullptr;
@@ -619,16 +729,18 @@ int backward_typed(const LnShape& s, const void* dy, const void* x, const void* 
   T* dp = reinterpret_cast<T*>(dx);
   const size_t smem = cached && parts_wanted ? size_t(kLnWarps) * s.width * sizeof(float) : 0;
   if (shared_rows) {
-    const size_t rows_smem = parts_wanted ? size_t(kLnWarps) * (32 / lpr) * s.width * sizeof(float) : 0;
-#define OOPS_LN_BWD(GROUPS, LPR)                                                                                         \
-  layer_norm_backward_rows_kernel<T, A, kVec, GROUPS, LPR>                                                               \
-      <<<grid, threads, rows_smem, stream>>>(s, gp, xp, weight, mean, rstd, dp, dw_parts, db_parts)
-    if (units <= 8) OOPS_LN_BWD(1, 8);
-    else if (units <= 16) OOPS_LN_BWD(1, 16);
-    else if (units <= 32) OOPS_LN_BWD(1, 32);
-    else if (units <= 64) OOPS_LN_BWD(2, 32);
-    else OOPS_LN_BWD(4, 32);
-#undef OOPS_LN_BWD
+    const size_t parts_smem = parts_wanted ? size_t(kLnWarps) * (32 / lpr) * s.width * sizeof(float) : 0;
+    auto rows = [&](auto groups_of, auto lanes, auto staged) {
+      constexpr bool STAGED = decltype(staged)::value;
+      layer_norm_backward_rows_kernel<T, A, kVec, decltype(groups_of)::value, decltype(lanes)::value, STAGED>
+          <<<grid, threads, std::max(parts_smem, size_t(STAGED ? 2 * kLnStage : 0)), stream>>>(s, gp, xp, weight, mean, rstd, dp, dw_parts, db_parts);
+    };
+    using std::integral_constant;
+    if (units <= 8) rows(integral_constant<int, 1>{}, integral_constant<int, 8>{}, std::true_type{});
+    else if (units <= 16) rows(integral_constant<int, 1>{}, integral_constant<int, 16>{}, std::true_type{});
+    else if (units <= 32) rows(integral_constant<int, 1>{}, integral_constant<int, 32>{}, std::true_type{});
+    else if (units <= 64) rows(integral_constant<int, 2>{}, integral_constant<int, 32>{}, std::true_type{});
+    else rows(integral_constant<int, 4>{}, integral_constant<int, 32>{}, std::false_type{});
   } else if (cached && vec)
     layer_norm_backward_kernel<T, A, kVec, true><<<grid, threads, smem, stream>>>(s, gp, xp, weight, mean, rstd, dp, dw_parts, db_parts);
   else if (cached)

@@ -1,0 +1,33 @@
+"""Layer norm on rows that travel through shared memory a turn ahead: row counts on either side of a turn of a warp and of all of them, widths on
+either side of the lane groups that share a row, strided rows, gradients wanted in part; against f64.  The norm of a 16-bit result's error
+is that of its rounding (half a unit at most: 2^-9 bf16, 2^-12 f16 of the values); f32 sums of up to 512 terms are off by some
+units of 2^-24 (the parameters' gradients by those of a sum over the rows)."""
+
+import pytest
+import torch
+
+import oops_b200 as oops
+
+pytestmark = pytest.mark.gpu
+ROUNDING = {torch.bfloat16: 2.0**-8, torch.float16: 2.0**-11, torch.float32: 1e-6}
+
+
+@pytest.mark.parametrize("dtype,rows,width,stride", [(torch.bfloat16, 1, 128, 0), (torch.float16, 9, 8, 0), (torch.bfloat16, 4737, 72, 0),
+                                                     (torch.bfloat16, 19000, 128, 136), (torch.float16, 4735, 200, 0),
+                                                     (torch.bfloat16, 2371, 264, 520), (torch.float32, 33, 4, 0), (torch.float32, 9473, 68, 0),
+                                                     (torch.float32, 7105, 128, 132), (torch.float32, 2369, 256, 0)])
+def test_edges(cuda, dtype, rows, width, stride):
+    gen = torch.Generator(device=cuda).manual_seed(rows)
+    storage = torch.randn(rows, stride or width, device=cuda, generator=gen).to(dtype)
+    x = storage[:, :width].detach().requires_grad_(True)
+    w, b = (torch.randn(width, device=cuda, generator=gen).requires_grad_(True) for _ in range(2))
+    up = torch.randn(rows, width, device=cuda, generator=gen).to(dtype)
+    y = oops.layer_norm(x, width, w, b)
+    grads = torch.autograd.grad(y, (x, w, b), up, retain_graph=True)
+    exact = [t.detach().double().requires_grad_(True) for t in (x, w, b)]
+    want = torch.nn.functional.layer_norm(exact[0], (width,), exact[1], exact[2])
+    for name, got, ref in zip(("y", "dx", "dw", "db"), (y, *grads), (want, *torch.autograd.grad(want, exact, up.double()))):
+        bound = ROUNDING[dtype if name in ("y", "dx") else torch.float32]
+        assert float((got.detach().double() - ref).norm()) <= bound * max(float(ref.norm()), 1e-3), name
+    dw, = torch.autograd.grad(y, (w,), up)
+    assert torch.equal(dw, grads[1])
