@@ -62,6 +62,26 @@ __device__ __forceinline__ void load8(const T* p, int n, float (&out)[8]) {
   }
 }
 
+// The same as they were loaded, so that several can be under way without eight registers each.
+template <typename T, bool VEC>
+struct Raw8 {
+  uint4 words[sizeof(T) / 2];
+  __device__ __forceinline__ void load(const T* p, int n, bool take) {
+#pragma unroll
+    for (int i = 0; i < int(sizeof(T) / 2); ++i) words[i] = make_uint4(0, 0, 0, 0);
+    if (!take) return;
+    if constexpr (VEC) {
+#pragma unroll
+      for (int i = 0; i < int(sizeof(T) / 2); ++i) words[i] = reinterpret_cast<const uint4*>(p)[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i < n) reinterpret_cast<T*>(words)[i] = p[i];
+    }
+  }
+  __device__ __forceinline__ float operator[](int i) const { return float(reinterpret_cast<const T*>(words)[i]); }
+};
+
 template <typename T, bool VEC>
 __device__ __forceinline__ void store8(T* p, int n, const float (&in)[8]) {
   if constexpr (VEC && sizeof(T) == 2) {
@@ -113,8 +133,10 @@ __device__ __forceinline__ int64_t token_at(const PairShape& s, int b, int64_t p
 // Row m of `proj` holds [left gate | left value | right gate | right value | ...], `hidden` channels each.
 // The channels of `left` and `right`, each rounded up to eight, form one axis.  CTA = (32 words of tokens, 64 of that axis,
 // prefix element): a token's piece of a projection is then 128 contiguous bytes of a 16-bit type (64-byte pieces: 55 and
-// 90 us forward and reverse at N = 384, 128 channels; now 52 and 78, the reverse with five CTAs per SM instead of
-// four, which pays although the 16-bit instances then spill 60 bytes a thread).  The channel chunk is the fastest index: neighbouring CTAs touch a token's other pieces while their pages are open.
+// 90 us forward and reverse at N = 384, 128 channels).  Pieces are kept as they were loaded until the arithmetic needs them: converted at
+// once, a token's loads waited for those of the token before, and the reverse spilled 60 bytes a thread at five CTAs per SM (51.4 and 78.2 us;
+// now 48.3 with eight CTAs and 62.2 with six, of 34.5 and 57.6 at the copy's rate).  The channel chunk is the
+// fastest index: neighbouring CTAs touch a token's other pieces while their pages are open.
 
 struct GateTile {  // rows = channels; rows 32 .. 63 stand four words on, so that a warp's eight channel groups miss each other's banks
   uint32_t words[64 * kPitch + 4];
@@ -135,7 +157,7 @@ struct GateGroup {
 __host__ __device__ inline int gate_chunks(int hidden) { return (2 * ((hidden + 7) / 8 * 8) + 63) / 64; }
 
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(256) pair_gate_forward_kernel(PairShape s, const T* __restrict__ proj, int64_t ld,
+__global__ void __launch_bounds__(256, 8) pair_gate_forward_kernel(PairShape s, const T* __restrict__ proj, int64_t ld,
                                                                 const T* __restrict__ mask, uint32_t* __restrict__ left,
                                                                 uint32_t* __restrict__ right) {
   constexpr int W = tokens_per_word<T>();
@@ -144,26 +166,22 @@ __global__ void __launch_bounds__(256) pair_gate_forward_kernel(PairShape s, con
   const int64_t first = int64_t(blockIdx.x / chunks) * 32;  // first word of the tile in a plane
   const int cg = threadIdx.x & 7, word = threadIdx.x >> 3;
   const GateGroup own(s, chunk * 64 + cg * 8);
-  float out[W][8];
+  Raw8<T, VEC> gate[W], value[W];
+  float weight[W];
 #pragma unroll
   for (int e = 0; e < W; ++e) {
     const int64_t m = token_at(s, b, (first + word) * W + e);
-    float gate[8], value[8];
-    if (m >= 0 && own.n > 0) {
-      const T* row = proj + m * ld + own.side * 2 * s.hidden + own.channel;
-      load8<T, VEC>(row, own.n, gate);
-      load8<T, VEC>(row + s.hidden, own.n, value);
-      const float weight = mask ? float(mask[m]) : 1.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) out[e][i] = weight * sigmoid_of<T>(gate[i]) * value[i];
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) out[e][i] = 0.f;
-    }
+    const bool there = m >= 0 && own.n > 0;
+    const T* row = proj + m * ld + own.side * 2 * s.hidden + own.channel;
+    gate[e].load(row, own.n, there);
+    value[e].load(row + s.hidden, own.n, there);
+    weight[e] = !there ? 0.f : mask ? float(mask[m]) : 1.f;
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    float both[2] = {out[0][i], out[W - 1][i]};
+    float both[2];
+#pragma unroll
+    for (int e = 0; e < W; ++e) both[e] = weight[e] * sigmoid_of<T>(gate[e][i]) * value[e][i];
     tile.at(cg * 8 + i, word) = to_word<T>(both);
   }
   __syncthreads();
@@ -179,7 +197,7 @@ __global__ void __launch_bounds__(256) pair_gate_forward_kernel(PairShape s, con
 }
 
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(256, VEC ? 5 : 4) pair_gate_backward_kernel(PairShape s, const T* __restrict__ proj, int64_t ld,
+__global__ void __launch_bounds__(256, VEC ? 6 : 4) pair_gate_backward_kernel(PairShape s, const T* __restrict__ proj, int64_t ld,
                                                                  const T* __restrict__ mask, const uint32_t* __restrict__ dleft,
                                                                  const uint32_t* __restrict__ dright, T* __restrict__ dproj,
                                                                  int64_t ld_d) {
@@ -198,30 +216,31 @@ __global__ void __launch_bounds__(256, VEC ? 5 : 4) pair_gate_backward_kernel(Pa
   }
   const int cg = threadIdx.x & 7, word = threadIdx.x >> 3;
   const GateGroup own(s, chunk * 64 + cg * 8);
-  float gate[W][8], value[W][8], weight[W];
+  Raw8<T, VEC> gate[W], value[W];
+  float weight[W];
   int64_t at[W];
 #pragma unroll
   for (int e = 0; e < W; ++e) {
     const int64_t m = own.n > 0 ? token_at(s, b, (first + word) * W + e) : -1;
     at[e] = m;
-    if (m >= 0) {
-      const T* row = proj + m * ld + own.side * 2 * s.hidden + own.channel;
-      load8<T, VEC>(row, own.n, gate[e]);
-      load8<T, VEC>(row + s.hidden, own.n, value[e]);
-      weight[e] = mask ? float(mask[m]) : 1.f;
-    }
+    const T* row = proj + m * ld + own.side * 2 * s.hidden + own.channel;
+    gate[e].load(row, own.n, m >= 0);
+    value[e].load(row + s.hidden, own.n, m >= 0);
+    weight[e] = m < 0 ? 0.f : mask ? float(mask[m]) : 1.f;
   }
   __syncthreads();
-  float grad[8][2];
+  uint32_t grad[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) from_word<T>(tile.at(cg * 8 + i, word), grad[i]);
+  for (int i = 0; i < 8; ++i) grad[i] = tile.at(cg * 8 + i, word);
 #pragma unroll
   for (int e = 0; e < W; ++e) {
     if (at[e] < 0) continue;
     float dgate[8], dvalue[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float sg = sigmoid_of<T>(gate[e][i]), up = grad[i][e] * weight[e];
+      float both[2];
+      from_word<T>(grad[i], both);
+      const float sg = sigmoid_of<T>(gate[e][i]), up = both[e] * weight[e];
       dvalue[i] = up * sg;
       dgate[i] = up * value[e][i] * sg * (1.f - sg);
     }
