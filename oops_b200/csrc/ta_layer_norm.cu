@@ -448,6 +448,7 @@ __global__ void __launch_bounds__(kLnWarps * 32, STAGED || GROUPS == 1 ? ln_ctas
       }
     }
   }
+  if constexpr (STAGED) ln_copies_wait<0>();  // (the request for a turn that does not come)
 }
 
 template <typename T, typename A, int V, int GROUPS, int LPR, bool STAGED>
@@ -584,6 +585,8 @@ __global__ void __launch_bounds__(kLnWarps * 32, STAGED || GROUPS == 1 ? ln_ctas
       }
     }
   }
+  // The request for a turn that does not come is still under way, as zeros; the sums below take the memory that it writes.
+  if constexpr (STAGED) ln_copies_wait<0>();
   if (dw_parts != nullptr || db_parts != nullptr) {
     constexpr int kSubs = kLnWarps * kRowsPerWarp;
     for (int pass = 0; pass < 2; ++pass) {

@@ -31,3 +31,24 @@ def test_edges(cuda, dtype, rows, width, stride):
         assert float((got.detach().double() - ref).norm()) <= bound * max(float(ref.norm()), 1e-3), name
     dw, = torch.autograd.grad(y, (w,), up)
     assert torch.equal(dw, grads[1])
+
+
+@pytest.mark.parametrize("width,turns,short", [(128, 1, 0), (128, 2, 0), (128, 2, 3), (64, 2, 0), (256, 2, 1), (512, 2, 0), (128, 3, 0), (128, 1, 9000)])
+def test_parameter_gradients_after_the_last_request(cuda, width, turns, short):
+    """The sums of the parameters' gradients take the shared memory that the request for a turn behind the last one writes zeros to: row counts
+    of an even and an odd number of turns, and warps that have none.  The sums have an order, so that all repetitions agree."""
+    sms = torch.cuda.get_device_properties(cuda).multi_processor_count
+    lanes = 8 if width <= 64 else 16 if width <= 128 else 32
+    rows = sms * 2 * 8 * (4 // (2 * max(1, width // 256))) * (32 // lanes) * turns - short  # CTAs, warps, row blocks of a turn, rows of a block
+    gen = torch.Generator(device=cuda).manual_seed(width + turns)
+    x = torch.randn(rows, width, device=cuda, generator=gen).bfloat16()
+    up = torch.randn(rows, width, device=cuda, generator=gen).bfloat16()
+    w, b = (torch.randn(width, device=cuda, generator=gen).requires_grad_(True) for _ in range(2))
+    y = oops.layer_norm(x, width, w, b)
+    first = torch.autograd.grad(y, (w, b), up, retain_graph=True)
+    for _ in range(50):
+        assert all(torch.equal(p, q) for p, q in zip(torch.autograd.grad(y, (w, b), up, retain_graph=True), first))
+    exact = [t.detach().double().requires_grad_(True) for t in (x, w, b)]
+    want = torch.autograd.grad(torch.nn.functional.layer_norm(exact[0], (width,), exact[1], exact[2]), exact[1:], up.double())
+    for got, ref in zip(first, want):
+        assert float((got.double() - ref).norm()) <= ROUNDING[torch.float32] * float(ref.norm())
