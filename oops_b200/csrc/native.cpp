@@ -445,12 +445,12 @@ std::optional<Tensor> dense_attention(const Tensor& query, const Tensor& key, co
 
 oops_ta_pair dense_pair(const Tensor& t) { return pair_of(Geometry(), Sample(), t); }
 
-// The kernels read every operand of a gate as the attention's type and shape.
+// The kernels read every operand of a gate as the attention's type and shape, on its device.
 void check_gate_operands(const Tensor& attention, std::initializer_list<const Tensor*> others) {
   for (const Tensor* t : others)
-    TORCH_CHECK(!t->defined() || (t->scalar_type() == attention.scalar_type() && t->sizes() == attention.sizes()),
-                "gate_attention_output gate kernel: operands of ", attention.scalar_type(), " ", attention.sizes(), " and ",
-                t->scalar_type(), " ", t->sizes());
+    TORCH_CHECK(!t->defined() || (t->scalar_type() == attention.scalar_type() && t->sizes() == attention.sizes() && t->device() == attention.device()),
+                "gate_attention_output gate kernel: operands of ", attention.scalar_type(), " ", attention.sizes(), " on ", attention.device(),
+                " and ", t->scalar_type(), " ", t->sizes(), " on ", t->device());
 }
 
 // Library products inside a node keep their operands' type, whatever region the reverse pass is called from.
@@ -610,6 +610,12 @@ bool whole_words(const Tensor& t) {  // a matrix, or pairs, whose every eighth e
     if (t.stride(i) != 1 && t.stride(i) % 8 != 0) return false;
   return true;
 }
+// What a product takes as a raw address: a whole matrix of this type and size.  Saved tensors come back through hooks, as whatever these
+// return; what does not fit takes the library's products, which check their operands.
+bool product_matrix(const Tensor& t, const Tensor& like, int64_t rows, int64_t cols) {
+  return plain_tensor(t) && t.scalar_type() == like.scalar_type() && t.device() == like.device() && t.dim() == 2 && t.size(0) == rows &&
+         t.size(1) == cols && t.is_contiguous() && whole_words(t);
+}
 void run_products(const Tensor& like, const oops_ta_product* list, int count) {
   check_gate_status(oops_ta_products(dtype_code(like.scalar_type()), list, count, current_stream(like)));
 }
@@ -625,8 +631,8 @@ struct GateOutputFunction : Function<GateOutputFunction> {
     std::vector<int64_t> shape = single.sizes().vec();
     shape.back() = wo.size(0);
     const int64_t count = rows.size(0), in = rows.size(1), inner = heads * dim, out_channels = wo.size(0);
-    if (own_products(type, count, in, inner, out_channels, dim) && rows.is_contiguous() && wg.is_contiguous() && wo.is_contiguous() &&
-        whole_words(rows) && whole_words(wg) && whole_words(wo) && whole_words(values)) {
+    if (own_products(type, count, in, inner, out_channels, dim) && product_matrix(rows, attention, count, in) &&
+        product_matrix(wg, attention, inner, in) && product_matrix(wo, attention, out_channels, inner) && whole_words(values)) {
       const c10::cuda::CUDAGuard guard(attention.device());
       const Tensor gate = at::empty({count, inner}, rows.options()), gated = at::empty({count, inner}, rows.options()),
                    out = at::empty(shape, rows.options());
@@ -666,9 +672,11 @@ struct GateOutputFunction : Function<GateOutputFunction> {
     variable_list result(4);
     const bool need_attention = ctx->needs_input_grad(0), need_gate = ctx->needs_input_grad(1) || ctx->needs_input_grad(2);
     const int64_t count = rows.size(0), in = rows.size(1), inner = heads * dim, out_channels = wo.size(0);
-    if (!at::GradMode::is_enabled() && own_products(type, count, in, inner, out_channels, dim) && rows.is_contiguous() && wg.is_contiguous() &&
-        wo.is_contiguous() && dout.is_contiguous() && gated.is_contiguous() && whole_words(rows) && whole_words(wg) && whole_words(wo) &&
-        whole_words(values) && whole_words(dout) && whole_words(gate) && whole_words(gated)) {
+    if (!at::GradMode::is_enabled() && own_products(type, count, in, inner, out_channels, dim) && plain_tensor(values) &&
+        whole_words(values) && count == values.size(0) * tokens && product_matrix(rows, attention, count, in) &&
+        product_matrix(wg, attention, inner, in) && product_matrix(wo, attention, out_channels, inner) &&
+        product_matrix(dout, attention, count, out_channels) && product_matrix(gate, attention, count, inner) &&
+        product_matrix(gated, attention, count, inner)) {
       // Two launches: the gradient of what lies behind the gate and what follows from it, then the gate's own product.
       const c10::cuda::CUDAGuard guard(attention.device());
       oops_ta_product list[2];
