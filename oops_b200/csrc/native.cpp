@@ -85,7 +85,7 @@ bool plain_context() {
 }
 
 bool plain_tensor(const Tensor& t) {
-  static const c10::DispatchKeySet special({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched,
+  static const c10::DispatchKeySet special({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::Batched,
                                             c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Functionalize,
                                             c10::DispatchKey::ZeroTensor, c10::DispatchKey::Negative,
                                             c10::DispatchKey::Conjugate});
@@ -611,7 +611,7 @@ bool whole_words(const Tensor& t) {  // a matrix, or pairs, whose every eighth e
   return true;
 }
 // What a product takes as a raw address: a whole matrix of this type and size.  Saved tensors come back through hooks, as whatever these
-// return; what does not fit takes the library's products, which check their operands.
+// return, and a gradient may be a batched one; what does not fit takes the library's products, which check their operands.
 bool product_matrix(const Tensor& t, const Tensor& like, int64_t rows, int64_t cols) {
   return plain_tensor(t) && t.scalar_type() == like.scalar_type() && t.device() == like.device() && t.dim() == 2 && t.size(0) == rows &&
          t.size(1) == cols && t.is_contiguous() && whole_words(t);
@@ -672,7 +672,7 @@ struct GateOutputFunction : Function<GateOutputFunction> {
     variable_list result(4);
     const bool need_attention = ctx->needs_input_grad(0), need_gate = ctx->needs_input_grad(1) || ctx->needs_input_grad(2);
     const int64_t count = rows.size(0), in = rows.size(1), inner = heads * dim, out_channels = wo.size(0);
-    if (!at::GradMode::is_enabled() && own_products(type, count, in, inner, out_channels, dim) && plain_tensor(values) &&
+    if (!at::GradMode::is_enabled() && plain_context() && own_products(type, count, in, inner, out_channels, dim) && plain_tensor(values) &&
         whole_words(values) && count == values.size(0) * tokens && product_matrix(rows, attention, count, in) &&
         product_matrix(wg, attention, inner, in) && product_matrix(wo, attention, out_channels, inner) &&
         product_matrix(dout, attention, count, out_channels) && product_matrix(gate, attention, count, inner) &&

@@ -1,8 +1,10 @@
 """Saved tensors of the output step that come back through hooks as something else: another type, size or device raises (a value of theirs
-is never read as if it fitted), another layout of the same values gives the same gradients."""
+is never read as if it fitted), another layout of the same values gives the same gradients; batched gradients and dispatch modes
+reach the library's products."""
 
 import pytest
 import torch
+from torch.utils._python_dispatch import TorchDispatchMode
 
 from oops_b200 import gate_attention_output
 
@@ -51,3 +53,28 @@ def test_other_layouts_of_the_same_values(cuda, which):
     for change in (strided, off_a_word):
         for got, ref in zip(with_hook(leaves, upstream, which, change), want):  # (sums in another order)
             assert float((got.double() - ref.double()).norm()) <= 2.0**-7 * float(ref.double().norm())
+
+
+def test_batched_gradients(cuda):
+    """The gradient of the weight behind the gate is a plain product, which takes a batch of upstream gradients."""
+    leaves, upstream = leaves_and_upstream(cuda)
+    batch = torch.stack([upstream, -2 * upstream])
+    got, = torch.autograd.grad(gate_attention_output(*leaves), [leaves[3]], batch, is_grads_batched=True)
+    for one, up in zip(got, batch):
+        want, = torch.autograd.grad(gate_attention_output(*leaves), [leaves[3]], up)
+        assert float((one.double() - want.double()).norm()) <= 2.0**-7 * float(want.double().norm())
+
+
+def test_a_dispatch_mode_sees_the_products_of_the_reverse(cuda):
+    leaves, upstream = leaves_and_upstream(cuda)
+    seen = []
+
+    class Recorder(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(func)
+            return func(*args, **(kwargs or {}))
+
+    out = gate_attention_output(*leaves)
+    with Recorder():
+        torch.autograd.grad(out, leaves, upstream)
+    assert torch.ops.aten.mm.default in seen
