@@ -283,7 +283,8 @@ int oops_ta_bias_rows(int32_t batch, int32_t groups, int32_t heads, int32_t cols
  *   GATE_REVERSE  C is not stored: with C the gradient of `gated`, dvalues = C * sigmoid(gate) (skipped where its ptr is NULL) and
  *                 the gradient of the gate, C * values * s * (1 - s), goes to `gated` (skipped where NULL).
  * These are the products around the gate in the reference's gate_attention_output (oops/attention/gate/composed.py:47-53).
- * n and dim are multiples of 8, all rows start on 16-byte boundaries; oops_ta_products_supported says whether a list is served.
+ * n and dim are multiples of 8, all rows start on 16-byte boundaries and are no nearer than they are long; oops_ta_products_supported
+ * says whether a list is served, and what it does not serve is refused without a launch.
  */
 #define OOPS_TA_MAX_PRODUCTS 2
 enum oops_ta_product_epilogue { OOPS_TA_PRODUCT_PLAIN = 0, OOPS_TA_PRODUCT_GATE = 1, OOPS_TA_PRODUCT_GATE_REVERSE = 2 };

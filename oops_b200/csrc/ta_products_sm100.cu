@@ -223,19 +223,24 @@ __global__ void __launch_bounds__(kProductThreads, 2) ta_products_kernel(const _
   teardown(abort_flag, tmem_base, kIssuer, kProductTmemCols);
 }
 
-bool words(const void* p, int64_t ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 8 == 0 && ld < int64_t(1) << 39; }
+// A matrix of `cols` columns whose rows start on 16-byte words; strides of a tensor map are below 2^40 bytes.
+bool words(const void* p, int64_t ld, int64_t cols) {
+  return p && (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 8 == 0 && ld >= cols && ld < int64_t(1) << 39;
+}
 bool pair_words(const oops_ta_pair& t) {
-  return (reinterpret_cast<uintptr_t>(t.ptr) & 15) == 0 && t.sb % 8 == 0 && t.sc % 8 == 0 && t.sh % 8 == 0;
+  return t.ptr && (reinterpret_cast<uintptr_t>(t.ptr) & 15) == 0 && t.sb % 8 == 0 && t.sc % 8 == 0 && t.sh % 8 == 0;
 }
 
 bool product_ok(const oops_ta_product& p) {
-  if (p.m <= 0 || p.n <= 0 || p.k <= 0 || p.n % 8 != 0) return false;
-  if (p.a_ld < (p.a_transposed ? p.m : p.k) || p.b_ld < (p.b_transposed ? p.n : p.k)) return false;
-  if (!words(p.a, p.a_ld) || !words(p.b, p.b_ld)) return false;
-  if (p.epilogue != OOPS_TA_PRODUCT_GATE_REVERSE && !words(p.c, p.c_ld)) return false;
+  if (p.m <= 0 || p.n <= 0 || p.k <= 0 || p.n % 8 != 0 || p.m > 0x7fffffff - kBm || p.n > 0x7fffffff - kBn || p.k > 0x7fffffff - kBk) return false;
+  if (!words(p.a, p.a_ld, p.a_transposed ? p.m : p.k) || !words(p.b, p.b_ld, p.b_transposed ? p.n : p.k)) return false;
+  const bool reverse = p.epilogue == OOPS_TA_PRODUCT_GATE_REVERSE;
+  if (!reverse && !words(p.c, p.c_ld, p.n)) return false;
   if (p.epilogue == OOPS_TA_PRODUCT_PLAIN) return true;
-  if (p.tokens <= 0 || p.dim <= 0 || p.dim % 8 != 0 || !pair_words(p.values) || !words(p.gated, p.gated_ld)) return false;
-  return p.epilogue == OOPS_TA_PRODUCT_GATE || (words(p.gate, p.gate_ld) && (!p.dvalues.ptr || pair_words(p.dvalues)));
+  if (p.epilogue != OOPS_TA_PRODUCT_GATE && !reverse) return false;
+  if (p.tokens <= 0 || p.dim <= 0 || p.dim % 8 != 0 || !pair_words(p.values)) return false;
+  if ((p.gated || !reverse) && !words(p.gated, p.gated_ld, p.n)) return false;
+  return !reverse || (words(p.gate, p.gate_ld, p.n) && (!p.dvalues.ptr || pair_words(p.dvalues)));
 }
 
 int encode_operand(CUtensorMap* map, int dtype, const void* ptr, int64_t ld, int rows, int k, bool transposed, uint32_t box_rows, const char* what) {
@@ -250,13 +255,13 @@ int64_t tiles_of(const oops_ta_product& p) { return ceil_div(p.m, kBm) * ceil_di
 }  // namespace
 
 bool products_supported(int dtype, const oops_ta_product* list, int count) {
-  if (dtype != OOPS_TA_BF16 && dtype != OOPS_TA_F16) return false;
+  if ((dtype != OOPS_TA_BF16 && dtype != OOPS_TA_F16) || count < 1 || count > OOPS_TA_MAX_PRODUCTS) return false;
   int64_t tiles = 0;
   for (int i = 0; i < count; ++i) {
     if (!product_ok(list[i])) return false;
     tiles += tiles_of(list[i]);
   }
-  return count >= 1 && count <= OOPS_TA_MAX_PRODUCTS && tiles <= 0x7fffffffll;
+  return tiles <= 0x7fffffffll;
 }
 
 int products(int dtype, const oops_ta_product* list, int count, cudaStream_t stream) {
