@@ -70,6 +70,7 @@ struct LnShape {
   int64_t rows;
   int width;
   int64_t x_stride, y_stride, dy_stride, dx_stride;  // row strides in elements
+  int share = 0;  // row blocks of a warp where a turn of every warp is more than there are (the kernels that share rows)
 };
 
 // affine parameters may be of the activation type or f32 ("master" parameters of 16-bit activations)
@@ -363,8 +364,9 @@ __global__ void __launch_bounds__(kLnWarps * 32, STAGED || GROUPS == 1 ? ln_ctas
   // A warp's blocks of a turn are neighbours.  `left` rows are there from the turn's first one on; a turn later they are `ahead` fewer.
   constexpr int64_t apart = kRowsPerWarp;
   const int64_t ahead = stride * kTurn * kRowsPerWarp, x_apart = apart * s.x_stride, y_apart = apart * s.y_stride;
-  const int64_t first = (int64_t(blockIdx.x) * kLnWarps + warp) * kTurn;
+  const int64_t first = (int64_t(blockIdx.x) * kLnWarps + warp) * s.share;
   int64_t row = first * kRowsPerWarp + sub, left = s.rows - row;
+  if (s.share < kTurn) left = min(left, s.share * apart);
   const T* from = x + row * s.x_stride + l * V;
   T* to = y + row * s.y_stride + l * V;
   auto request = [&](int64_t left, uint32_t at) {  // `from` is the turn's first row
@@ -386,7 +388,7 @@ __global__ void __launch_bounds__(kLnWarps * 32, STAGED || GROUPS == 1 ? ln_ctas
   for (int64_t blk0 = first; blk0 < blocks; blk0 += stride * kTurn, row += ahead, left -= ahead, to += ahead * s.y_stride) {
     uint4 raw[kTurn][GROUPS];
     if constexpr (STAGED) {
-      request(left - ahead, mine + (stage ^ kLnStage));
+      if (blk0 + stride * kTurn < blocks) request(left - ahead, mine + (stage ^ kLnStage));
       ln_copies_commit();
       ln_copies_wait<1>();
 #pragma unroll
@@ -481,8 +483,9 @@ __global__ void __launch_bounds__(kLnWarps * 32, STAGED || GROUPS == 1 ? ln_ctas
   // A warp's blocks of a turn are neighbours.  `left` rows are there from the turn's first one on; a turn later they are `ahead` fewer.
   constexpr int64_t apart = kRowsPerWarp;
   const int64_t ahead = stride * kU * kRowsPerWarp, x_apart = apart * s.x_stride, g_apart = apart * s.dy_stride, d_apart = apart * s.dx_stride;
-  const int64_t first = (int64_t(blockIdx.x) * kLnWarps + warp) * kU, row0 = first * kRowsPerWarp + sub;
+  const int64_t first = (int64_t(blockIdx.x) * kLnWarps + warp) * s.share, row0 = first * kRowsPerWarp + sub;
   int64_t left = s.rows - row0;
+  if (s.share < kU) left = min(left, s.share * apart);
   const T* from_x = x + row0 * s.x_stride + l * V;
   const T* from_g = dy + row0 * s.dy_stride + l * V;
   T* to = dx + row0 * s.dx_stride + l * V;
@@ -660,12 +663,25 @@ __global__ void __launch_bounds__(256) layer_norm_reduce_parts_kernel(const floa
 constexpr int kLnMaxWidth = 8192;
 constexpr int kLnWideParts = 64;
 
-int ln_grid(int64_t rows, int ctas = kLnCtasPerSm) {
+int sm_total() {
   int device = 0, sms = 148;
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  const int64_t wanted = (rows + kLnWarps - 1) / kLnWarps;
-  return int(wanted < int64_t(sms) * ctas ? wanted : int64_t(sms) * ctas);
+  return sms;
 }
+
+// The launch of a kernel that shares rows: `share` row blocks of a warp in a turn, and as many CTAs as then have rows.  A turn is all of its
+// blocks except where they would leave SMs without any: a warp works through its blocks in turn (64 f32 rows of 384: 3.6 us with four a
+// warp, 3.1 with one), but more warps than one CTA per SM has gain nothing (4096 of them: 5.7 us with four, 9.5 with one).
+struct LnLaunch {
+  int grid, share;
+};
+LnLaunch ln_launch(int64_t rows, int lanes, int turn, int ctas_per_sm) {
+  const int64_t blocks = (rows + 32 / lanes - 1) / (32 / lanes), warps = int64_t(sm_total()) * kLnWarps;
+  const int64_t share = std::min<int64_t>(turn, (blocks + warps - 1) / warps);
+  return {int(std::min<int64_t>(int64_t(sm_total()) * ctas_per_sm, (blocks + share * kLnWarps - 1) / (share * kLnWarps))), int(share)};
+}
+
+int ln_grid(int64_t rows) { return int(std::min<int64_t>((rows + kLnWarps - 1) / kLnWarps, int64_t(sm_total()) * kLnCtasPerSm)); }
 
 bool ln_vector_ok(int vec, int width, std::initializer_list<const void*> pointers, std::initializer_list<int64_t> strides) {
   if (width % vec) return false;
@@ -690,9 +706,11 @@ int forward_typed(const LnShape& s, const void* x, const void* weight, const voi
     auto rows = [&](auto groups, auto lanes, auto staged) {
       constexpr int GROUPS = decltype(groups)::value, LPR = decltype(lanes)::value;
       constexpr bool STAGED = decltype(staged)::value;
+      const LnLaunch launch = ln_launch(s.rows, LPR, ln_turn(GROUPS, 1, STAGED), ln_ctas(1, sizeof(T), STAGED));
+      LnShape shared = s;
+      shared.share = launch.share;
       layer_norm_forward_rows_kernel<T, A, kVec, GROUPS, LPR, STAGED>
-          <<<ln_grid((s.rows + 32 / LPR - 1) / (32 / LPR), ln_ctas(1, sizeof(T), STAGED)), threads, STAGED ? 2 * kLnStage : 0, stream>>>(
-              s, xp, weight, bias, eps, yp, mean, rstd);
+          <<<launch.grid, threads, STAGED ? 2 * kLnStage : 0, stream>>>(shared, xp, weight, bias, eps, yp, mean, rstd);
     };
     using std::integral_constant;
     if (units <= 8) rows(integral_constant<int, 1>{}, integral_constant<int, 8>{}, std::true_type{});
@@ -723,7 +741,8 @@ int backward_typed(const LnShape& s, const void* dy, const void* x, const void* 
   const bool shared_rows = vec && units <= 128;  // several lanes (not always a whole warp) share a row
   const int lpr = units <= 8 ? 8 : units <= 16 ? 16 : 32;
   const bool staged = units <= 64;
-  if (shared_rows) grid = ln_grid((s.rows + 32 / lpr - 1) / (32 / lpr), ln_ctas(2, sizeof(T), staged));
+  const LnLaunch launch = ln_launch(s.rows, lpr, ln_turn(units <= 32 ? 1 : units <= 64 ? 2 : 4, 2, staged), ln_ctas(2, sizeof(T), staged));
+  if (shared_rows) grid = launch.grid;
   const int num_parts = cached ? grid : int(s.rows < kLnWideParts ? s.rows : kLnWideParts);
   float* dw_parts = dweight ? workspace : nullptr;
   float* db_parts = dbias ? workspace + int64_t(num_parts) * s.width : nullptr;
@@ -734,9 +753,13 @@ int backward_typed(const LnShape& s, const void* dy, const void* x, const void* 
   if (shared_rows) {
     const size_t parts_smem = parts_wanted ? size_t(kLnWarps) * (32 / lpr) * s.width * sizeof(float) : 0;
     auto rows = [&](auto groups_of, auto lanes, auto staged) {
+      constexpr int GROUPS = decltype(groups_of)::value, LPR = decltype(lanes)::value;
       constexpr bool STAGED = decltype(staged)::value;
-      layer_norm_backward_rows_kernel<T, A, kVec, decltype(groups_of)::value, decltype(lanes)::value, STAGED>
-          <<<grid, threads, std::max(parts_smem, size_t(STAGED ? 2 * kLnStage : 0)), stream>>>(s, gp, xp, weight, mean, rstd, dp, dw_parts, db_parts);
+      LnShape shared = s;
+      shared.share = launch.share;
+      layer_norm_backward_rows_kernel<T, A, kVec, GROUPS, LPR, STAGED>
+          <<<grid, threads, std::max(parts_smem, size_t(STAGED ? 2 * kLnStage : 0)), stream>>>(shared, gp, xp, weight, mean, rstd, dp, dw_parts,
+                                                                                              db_parts);
     };
     using std::integral_constant;
     if (units <= 8) rows(integral_constant<int, 1>{}, integral_constant<int, 8>{}, std::true_type{});

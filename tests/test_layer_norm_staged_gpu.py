@@ -52,3 +52,21 @@ def test_parameter_gradients_after_the_last_request(cuda, width, turns, short):
     want = torch.autograd.grad(torch.nn.functional.layer_norm(exact[0], (width,), exact[1], exact[2]), exact[1:], up.double())
     for got, ref in zip(first, want):
         assert float((got.double() - ref).norm()) <= ROUNDING[torch.float32] * float(ref.norm())
+
+
+@pytest.mark.parametrize("dtype,width", [(torch.bfloat16, 128), (torch.float16, 384), (torch.float32, 384), (torch.float32, 64)])
+@pytest.mark.parametrize("share,off", [(1, 0), (1, 1), (2, 0), (2, 1), (3, 1), (4, -1)])
+def test_shares_of_a_turn(cuda, dtype, width, share, off):
+    """Fewer row blocks than a turn of one CTA per SM: row counts on either side of one, two, three and four blocks a warp."""
+    sms = torch.cuda.get_device_properties(cuda).multi_processor_count
+    units = width * dtype.itemsize // 16
+    rows = sms * 8 * share * (4 if units <= 8 else 2 if units <= 16 else 1) + off
+    gen = torch.Generator(device=cuda).manual_seed(rows)
+    x, up = (torch.randn(rows, width, device=cuda, generator=gen).to(dtype) for _ in range(2))
+    leaves = [x.requires_grad_(True)] + [torch.randn(width, device=cuda, generator=gen).requires_grad_(True) for _ in range(2)]
+    y = oops.layer_norm(leaves[0], width, leaves[1], leaves[2])
+    exact = [t.detach().double().requires_grad_(True) for t in leaves]
+    want = torch.nn.functional.layer_norm(exact[0], (width,), exact[1], exact[2])
+    for name, got, ref in zip(("y", "dx", "dw", "db"), (y, *torch.autograd.grad(y, leaves, up)), (want, *torch.autograd.grad(want, exact, up.double()))):
+        bound = ROUNDING[dtype if name in ("y", "dx") else torch.float32]
+        assert float((got.detach().double() - ref).norm()) <= bound * float(ref.norm()), name
