@@ -146,6 +146,11 @@ int oops_ta_supported(const oops_ta_problem* problem);
    pass is asked about. */
 int oops_ta_uses_tensor_path(const oops_ta_problem* problem, int backward);
 
+/* 1 if a problem of another head size takes the tcgen05 kernels that serve those (bf16, no mask, up to 64 channels), 0 if not,
+   negative status on error: a forward pass into `result` where `grads` is NULL, else the reverse pass of the upstream gradient
+   `result`.  Host only; pointers are not dereferenced. */
+int oops_ta_uses_wide_path(const oops_ta_problem* problem, const oops_ta_pair* result, const oops_ta_grads* grads);
+
 /* Scratch bytes oops_ta_forward needs for this problem (may be 0). */
 uint64_t oops_ta_forward_workspace_bytes(const oops_ta_problem* problem);
 

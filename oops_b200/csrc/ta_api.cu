@@ -163,6 +163,15 @@ int oops_ta_uses_tensor_path(const oops_ta_problem* problem, int backward) {
   return backward ? (tensor_backward_applies(*problem, nullptr) ? 1 : 0) : (tensor_forward_applies(*problem) ? 1 : 0);
 }
 
+int oops_ta_uses_wide_path(const oops_ta_problem* problem, const oops_ta_pair* result, const oops_ta_grads* grads) {
+  const int status = validate(problem, false);
+  if (status) return -status;
+  if (!result) return -fail(OOPS_TA_INVALID_ARGUMENT, "result is NULL");
+  const bool others = force_generic(problem) || (grads ? tensor_backward_applies(*problem, grads) : tensor_forward_applies(*problem));
+  if (others || !mma_applies(*problem)) return 0;
+  return (grads ? wide_backward_applies(*problem, *result, *grads) : wide_forward_applies(*problem, *result)) ? 1 : 0;
+}
+
 uint64_t oops_ta_forward_workspace_bytes(const oops_ta_problem* problem) {
   if (validate(problem, false)) return 0;
   if (!force_generic(problem) && tensor_forward_applies(*problem)) return tensor_forward_workspace(*problem);

@@ -794,11 +794,15 @@ bool served(const oops_ta_problem& p) {
 
 }  // namespace
 
+static int padded_dim(const oops_ta_problem& p) { return (int)ceil_div(p.head_dim, 16) * 16; }
+
 // A call of few columns and channels ends before the barriers, tensor memory and copies of these kernels are set up: 64 problems of 64
 // columns and 16 channels take 3.3 us at register level and 4.3 here, 128 columns and 24 channels 5.1 and 5.5; with 48
-// channels it is 6.6 and 5.8, and 8 problems of 128 columns and 64 channels take 7.0 and 5.3.
+// channels it is 6.6 and 5.8, and 8 problems of 128 columns and 64 channels take 7.0 and 5.3.  Up to 16 channels on half of the SMs it
+// is longer columns that pay (8 problems of 300 columns: 7.9 and 8.2, of 384: 9.1 and 8.7; 384 problems of 300: 39 and 34).
 bool wide_forward_applies(const oops_ta_problem& p, const oops_ta_pair& out) {
-  return int64_t(p.cols) * (ceil_div(p.head_dim, 16) * 16) > 4096 && served(p) && stored_whole(out);
+  const int channels = padded_dim(p), least = channels == 16 && row_ctas(p) <= 74 ? 383 * 16 : 4096;
+  return int64_t(p.cols) * channels > least && served(p) && stored_whole(out);
 }
 
 int wide_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, cudaStream_t stream) {
@@ -815,11 +819,34 @@ int wide_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse, 
                        : launch(ta_wide_fwd_kernel<false>, P, row_ctas(p), kWideFwdThreads, WideFwdSmem::bytes, stream, "wide forward");
 }
 
-// All sizes: with every gradient wanted, 64 problems of 64 columns and 16 channels take 11.3 us (12.3 at register level), 8
-// problems of 64 columns and 64 channels 8.0 (14.8).
+// Which of the two reverse kernels is the faster one, from 8 to 768 columns in 1, some and many problems (a row and head each), times of the
+// register-level kernels first.  Tiles of 128 rows against 64: up to 64 columns half of a tile is empty, from 129 to 192 a quarter, which
+// costs more than the tensor pipe saves where there are few channels; and a CTA takes longer to set up than a small call does to end.
+//   bias gradient alone     here: 13 / 7 us (8 problems of 64 columns and 64 channels) to 583 / 137 (384 of 768); never slower.
+//   up to 64 columns        without a bias gradient here only where 48 or more channels fit one wave (148 problems of 64 columns and 64 channels:
+//                           11.5 / 9.6; 4096: 155 / 168, with 16 channels 81 / 134); with one here from 24 channels on (4096 problems: 220 / 209; 16
+//                           channels 173 / 188, 8 problems of them 9.1 / 7.4).
+//   more, 16 channels       129 to 192 columns at register level (1024 problems of 160: 108 / 122 us), but for many problems of more than 8 channels with a
+//                           bias gradient (162 / 154; 8 channels 161 / 167; 48 problems of 16 19 / 21); else by problems and columns (8 problems of 256:
+//                           11.8 / 12.7, with the bias gradient 12.2 / 12.7, of 384 18.1 / 17.1; 28 of 300, queries alone: 11.6 / 12.3; 1024 of 256: 177 / 154
+//                           and 265 / 206).
+//   more, 32 channels       on a quarter of the SMs without a bias gradient at register level below 256 columns (8 of 192: 11.3 / 12.0).
+//   more, 48 channels       here (8 problems of 65 columns: 10.9 / 10.1; 1024 of 256: 331 / 193).
+static bool wide_backward_pays(const oops_ta_problem& p, const oops_ta_grads& g) {
+  const bool keys = g.dk.ptr || g.dv.ptr, queries = g.dq.ptr != nullptr;
+  if (!keys && !queries) return true;
+  const int channels = padded_dim(p);
+  const int64_t problems = row_ctas(p), ctas = problems * (int(keys) + int(queries));
+  if (p.cols <= 64) return g.dbias ? channels >= 32 || problems <= 16 : channels >= 48 && ctas <= 296;
+  if (channels >= 48) return true;
+  if (channels == 32) return g.dbias || ctas > 37 || p.cols >= 256;
+  if (p.cols > kTile && p.cols <= 192) return g.dbias && p.head_dim > 8 && problems > 296;
+  return g.dbias ? problems > 32 || p.cols >= 384 : problems > (keys && queries ? 37 : 148) || p.cols >= 1024;
+}
+
 bool wide_backward_applies(const oops_ta_problem& p, const oops_ta_pair& dout, const oops_ta_grads& g) {
   if (p.bias_groups > 1 && g.dbias) return false;
-  if (!served(p) || !pair_ok(dout, p) || !mappable(dout)) return false;
+  if (!wide_backward_pays(p, g) || !served(p) || !pair_ok(dout, p) || !mappable(dout)) return false;
   for (const oops_ta_pair* t : {&g.dq, &g.dk, &g.dv})
     if (t->ptr && !stored_whole(*t)) return false;
   const int64_t tiles = int64_t(p.batch) * p.heads * ceil_div(p.cols, kTile) * ceil_div(p.cols, kStep);

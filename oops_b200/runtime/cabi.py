@@ -40,7 +40,7 @@ EXPORTS = (
     "oops_ta_layer_norm_backward", "oops_ta_pair_gate_forward", "oops_ta_pair_gate_backward",
     "oops_ta_channel_norm_forward", "oops_ta_channel_norm_backward_workspace_bytes", "oops_ta_channel_norm_backward",
     "oops_ta_output_gate_forward", "oops_ta_output_gate_backward", "oops_ta_bias_rows",
-    "oops_ta_products_supported", "oops_ta_products",
+    "oops_ta_products_supported", "oops_ta_products", "oops_ta_uses_wide_path",
 )
 
 
@@ -94,6 +94,8 @@ def library() -> ctypes.CDLL:
     lib.oops_ta_supported.argtypes = [POINTER(Problem)]
     lib.oops_ta_uses_tensor_path.restype = c_int
     lib.oops_ta_uses_tensor_path.argtypes = [POINTER(Problem), c_int]
+    lib.oops_ta_uses_wide_path.restype = c_int
+    lib.oops_ta_uses_wide_path.argtypes = [POINTER(Problem), POINTER(Pair), POINTER(Grads)]
     lib.oops_ta_forward_workspace_bytes.restype = c_uint64
     lib.oops_ta_forward_workspace_bytes.argtypes = [POINTER(Problem)]
     lib.oops_ta_backward_workspace_bytes.restype = c_uint64
