@@ -594,15 +594,28 @@ oops_ta_product product(const Tensor& a, const Tensor& b, const Tensor& c, int64
 }
 
 // Whether the output step's products run on this library's kernels: `rows` of `in` channels, `inner` channels between the two products,
-// `out` channels behind.  What they save is launches (2048 rows, 384 / 1024 / 384 channels, forward and reverse: 172 us of host work a call
-// with the library's products and the gate between them, 92 with these; on the device alone 39 and 45 us, 64 rows 19.3 and 18.9).  From
-// some thousand rows on the device takes longer than the host, and the library's larger tiles are the better ones (3072 rows
-// 47 and 58 us, 12288 rows 131 and 194).
-constexpr int64_t kOwnProductValues = 2048 * 1024;
+// `out` channels behind.  What they save is launches: 31 us of host work a call in the forward pass with the library's products and
+// the gate between them, 14 to 17 with these; 155 with the reverse, 91.  On the device alone, in us (library / these):
+//   rows x heads x channels, in = out   forward        with the reverse
+//   64 x 16 x 64, 384                   9.0 / 9.7      21.0 / 19.5
+//   512 x 16 x 64, 384                  9.9 / 10.8     26.9 / 24.5
+//   1024 x 16 x 64, 384                 11.0 / 11.9    31.0 / 29.9
+//   1536 x 16 x 64, 384                 12.3 / 14.9    34.7 / 34.4
+//   2048 x 16 x 64, 384                 13.7 / 16.2    38.9 / 43.2
+//   2304 x 16 x 64, 384                 13.9 / 16.1    41.0 / 44.7
+//   2560 x 16 x 64, 384                 14.8 / 20.3    42.5 / 50.9
+//   8192 x 8 x 32, 384                  13.8 / 17.2    53.1 / 46.9
+//   16384 x 8 x 16, 128                 11.9 / 11.5    52.5 / 40.8
+//   32768 x 16 x 24, 128                36.2 / 51.4    111.9 / 133.6
+//   65536 x 8 x 16, 128                 28.9 / 39.9    103.3 / 131.7
+//   256 x 32 x 64, 768                  10.8 / 13.6    30.7 / 36.3
+// They take a call while what they may cost a device that never waits for the host (a tenth with the reverse) is small beside what they
+// save one that does; beyond, the library's larger tiles are the better ones.
+constexpr int64_t kOwnProductWork = int64_t(7) << 28, kOwnProductWeights = 5 << 18, kOwnProductRows = 1 << 15;
 bool own_products(at::ScalarType type, int64_t rows, int64_t in, int64_t inner, int64_t out, int64_t dim) {
   return (type == at::kBFloat16 || type == at::kHalf) && rows > 0 && in > 0 && out > 0 && in % 8 == 0 && inner % 8 == 0 && out % 8 == 0 &&
-         dim % 8 == 0 && rows <= kOwnProductValues && in <= kOwnProductValues && inner <= kOwnProductValues && out <= kOwnProductValues &&
-         rows * std::max(std::max(in, inner), out) <= kOwnProductValues && inner * std::max(in, out) <= kOwnProductValues;
+         dim % 8 == 0 && rows <= kOwnProductRows && in <= kOwnProductWeights && inner <= kOwnProductWeights && out <= kOwnProductWeights &&
+         inner * std::max(in, out) <= kOwnProductWeights && rows * (in + out) <= kOwnProductWork / inner;
 }
 bool whole_words(const Tensor& t) {  // a matrix, or pairs, whose every eighth element starts a 16-byte word
   if ((reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) != 0) return false;
@@ -634,8 +647,7 @@ struct GateOutputFunction : Function<GateOutputFunction> {
     if (own_products(type, count, in, inner, out_channels, dim) && product_matrix(rows, attention, count, in) &&
         product_matrix(wg, attention, inner, in) && product_matrix(wo, attention, out_channels, inner) && whole_words(values)) {
       const c10::cuda::CUDAGuard guard(attention.device());
-      const Tensor gate = at::empty({count, inner}, rows.options()), gated = at::empty({count, inner}, rows.options()),
-                   out = at::empty(shape, rows.options());
+      const Tensor gate = at::empty({count, inner}, rows.options()), gated = at::empty({count, inner}, rows.options());
       oops_ta_product open = product(rows, wg, gate, count, inner, in);
       open.epilogue = OOPS_TA_PRODUCT_GATE;
       open.values = head_pair(values);
@@ -644,9 +656,10 @@ struct GateOutputFunction : Function<GateOutputFunction> {
       open.tokens = int32_t(tokens);
       open.dim = int32_t(dim);
       run_products(rows, &open, 1);
+      if (ctx) ctx->save_for_backward({attention, single, gate_weight, output_weight, gate, gated});
+      const Tensor out = at::empty(shape, rows.options());
       const oops_ta_product project = product(gated, wo, out, count, out_channels, inner);
       run_products(rows, &project, 1);
-      if (ctx) ctx->save_for_backward({attention, single, gate_weight, output_weight, gate, gated});
       return out;
     }
     const Tensor gate = at::linear(rows, wg), gated = at::empty_like(gate);
