@@ -15,12 +15,12 @@
 //             keys); a 64 x 64 tile of the row-shared bias gradient, rows innermost, summed in registers.  Each makes the
 //             scores it needs again (9 products instead of 5): token attention has too few rows and heads to give a
 //             CTA a whole row, and nothing has to be added across CTAs, so results are reproducible.
-// 4 samples, 16 heads of 64 channels, 512 tokens: 35 us forward and 136 us reverse, against 1178 us in 9 launches with scores
-// in memory.  Bound by latency at twelve to sixteen warps per SM, element-wise work and products in turn (counters of that call:
-// issue slots 50 % and the tensor pipe 38 % busy forward, 36 and 33 % in the reverse, HBM idle): packed f32
-// arithmetic, no tests on kept keys where a tile keeps all, first products without a zeroed accumulator, and, in the
-// reverse, row operands read again from shared memory instead of held in 64 registers (238 -> 168 registers, two -> three
-// CTAs per SM) took 45 and 171 us to these figures.
+// 4 samples, 16 heads of 64 channels, 512 tokens, f16: 35 us forward and 144 us reverse (bf16 with a mask 37 and 143; without one it goes to the
+// tcgen05 kernels), against 1178 us in 9 launches with scores in memory.  Bound by latency at twelve to sixteen warps per SM, element-wise work and
+// products in turn (counters of the bf16 call while it came here: issue slots 50 % and the tensor pipe 38 % busy forward, 36 and 33 %
+// in the reverse, HBM idle): packed f32 arithmetic, no tests on kept keys where a tile keeps all, first products without a zeroed accumulator,
+// and, in the reverse, row operands read again from shared memory instead of held in 64 registers (238 -> 168 registers, two -> three
+// CTAs per SM) took 45 and 171 us to 35 and 136 in bf16.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 

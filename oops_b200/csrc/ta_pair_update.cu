@@ -135,7 +135,7 @@ __device__ __forceinline__ int64_t token_at(const PairShape& s, int b, int64_t p
 // prefix element): a token's piece of a projection is then 128 contiguous bytes of a 16-bit type (64-byte pieces: 55 and
 // 90 us forward and reverse at N = 384, 128 channels).  Pieces are kept as they were loaded until the arithmetic needs them: converted at
 // once, a token's loads waited for those of the token before, and the reverse spilled 60 bytes a thread at five CTAs per SM (51.4 and 78.2 us;
-// now 48.3 with eight CTAs and 62.2 with six, of 34.5 and 57.6 at the copy's rate).  The channel chunk is the
+// now 48.3 with eight CTAs and 62.2 with six, where a 16-bit thread spills 4, of 34.5 and 57.6 at the copy's rate).  The channel chunk is the
 // fastest index: neighbouring CTAs touch a token's other pieces while their pages are open.
 
 struct GateTile {  // rows = channels; rows 32 .. 63 stand four words on, so that a warp's eight channel groups miss each other's banks

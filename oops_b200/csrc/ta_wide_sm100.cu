@@ -15,10 +15,11 @@
 //             summed in registers.  Each makes the scores it needs again, as token attention has too few rows and heads to
 //             give a CTA a whole row; nothing is added across CTAs, so results are reproducible.
 // What bounds them is the chain of a step (scores, element-wise work, sums, and the trips between them), which the second CTA of an
-// SM runs under; the special-function units need 3 us of a forward pass of 4 samples, 16 heads of 64 channels and 512 tokens, the
-// tensor pipe 17 of its reverse.  That call took 35 us forward and 136 reverse at register level, and takes 14 and 56 here, with the
-// same errors against f64 (1.66e-3 of every result's norm, its rounding).  With queries as rows the next scores are issued ahead
-// of the sums (dP has a second buffer there): 24 -> 22 us for dQ alone.
+// SM runs under; no unit is full (counters of 4 samples, 16 heads of 64 channels and 512 tokens: tensor pipe 15 % busy forward and 20 % in the
+// reverse, issue slots 28 and 35 %, special-function units 21 and 22 %).  That call took 35 us forward and 136 reverse at register
+// level, and takes 14 and 57 here, with the same errors against f64 (1.66e-3 of every result's norm, its rounding).  With queries as rows the next
+// scores are issued ahead of the sums (dP has a second buffer there): 24 -> 22 us for dQ alone.  Masks are not served: a step has no place yet for the
+// test of a mask tile.
 #include <algorithm>
 #include <type_traits>
 
