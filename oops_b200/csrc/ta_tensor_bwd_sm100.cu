@@ -54,8 +54,9 @@ constexpr int kRing = 4;                                // ring depth of the str
 // Bound by HBM.  With a (cell, head) per four lanes the divisions that place it were as many instructions as HBM had time for, and the
 // mask's blocks, last in the grid and a load at a time, ran on alone.  N = 256, two samples: 18.4 -> 11.7 us; N = 768: 71.8 -> 50.3 us
 // (302 MB of tensors and 9 of sums: 6.2 TB/s of the copy's 6.56).
-template <typename T>
-__global__ void __launch_bounds__(256, 4) prepare_kernel(oops_ta_pair out, oops_ta_pair dout, float* delta, uint32_t cells, int cols,
+// HEADS == 1: one head, whose group would be three idle loads and whose registers would halve the CTAs of an SM (N = 256: 3.8 us, as a group 5.3).
+template <typename T, int HEADS>
+__global__ void __launch_bounds__(256, HEADS == 1 ? 6 : 4) prepare_kernel(oops_ta_pair out, oops_ta_pair dout, float* delta, uint32_t cells, int cols,
                                                       int heads, int rows, int vec_ok, int row_inner, uint32_t mask_blocks,
                                                       const uint8_t* mask, int64_t m_sb, int64_t m_sr, int64_t m_sc,
                                                       uint32_t* live, int num_rows) {
@@ -113,25 +114,25 @@ __global__ void __launch_bounds__(256, 4) prepare_kernel(oops_ta_pair out, oops_
   const T* po = reinterpret_cast<const T*>(out.ptr) + b * out.sb + int64_t(r) * out.sr + int64_t(q) * out.sc + part * 8;
   const T* pd = reinterpret_cast<const T*>(dout.ptr) + b * dout.sb + int64_t(r) * dout.sr + int64_t(q) * dout.sc + part * 8;
   float* to = delta + (int64_t(b) * rows + r) * heads * cols + q;
-  for (int h0 = 0; h0 < heads; h0 += 4) {
-    float dot[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int h0 = 0; h0 < heads; h0 += HEADS) {
+    float dot[HEADS] = {};
     if (vec_ok) {
-      uint4 a[4], g[4];
+      uint4 a[HEADS], g[HEADS];
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
+      for (int n = 0; n < HEADS; ++n) {
         const bool take = there && h0 + n < heads;
         a[n] = ldg_v4_here_if(po + int64_t(h0 + n) * out.sh, take);
         g[n] = ldg_v4_here_if(pd + int64_t(h0 + n) * dout.sh, take);
       }
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
+      for (int n = 0; n < HEADS; ++n) {
         const uint32_t aw[4] = {a[n].x, a[n].y, a[n].z, a[n].w}, gw[4] = {g[n].x, g[n].y, g[n].z, g[n].w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) dot[n] += Half2<T>::lo(aw[e]) * Half2<T>::lo(gw[e]) + Half2<T>::hi(aw[e]) * Half2<T>::hi(gw[e]);
       }
     } else if (there) {
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
+      for (int n = 0; n < HEADS; ++n) {
         if (h0 + n >= heads) break;
 #pragma unroll
         for (int c = 0; c < 8; ++c) dot[n] += float(po[int64_t(h0 + n) * out.sh + c]) * float(pd[int64_t(h0 + n) * dout.sh + c]);
@@ -139,12 +140,12 @@ __global__ void __launch_bounds__(256, 4) prepare_kernel(oops_ta_pair out, oops_
     }
     float own = 0.f;
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
+    for (int n = 0; n < HEADS; ++n) {
       dot[n] += __shfl_xor_sync(0xffffffffu, dot[n], 1);
       dot[n] += __shfl_xor_sync(0xffffffffu, dot[n], 2);
       if (n == part) own = dot[n];
     }
-    if (there && h0 + part < heads) to[int64_t(h0 + part) * cols] = own;
+    if (there && part < HEADS && h0 + part < heads) to[int64_t(h0 + part) * cols] = own;
   }
 }
 
@@ -2036,9 +2037,10 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
     const int vec_ok = (reinterpret_cast<uintptr_t>(out.ptr) & 15) == 0 && (reinterpret_cast<uintptr_t>(dout.ptr) & 15) == 0 &&
                        out.sb % 8 == 0 && out.sr % 8 == 0 && out.sc % 8 == 0 && out.sh % 8 == 0 && dout.sb % 8 == 0 &&
                        dout.sr % 8 == 0 && dout.sc % 8 == 0 && dout.sh % 8 == 0;
-    prepare_kernel<T><<<delta_blocks + mask_blocks, 256, 0, stream>>>(out, dout, delta, (uint32_t)cells, p.cols, p.heads, p.rows, vec_ok,
-                                                                      dout.sr < dout.sc, mask_blocks, p.mask, p.mask_sb, p.mask_sr,
-                                                                      p.mask_sc, live, p.batch * p.rows);
+    auto kernel = p.heads == 1 ? prepare_kernel<T, 1> : prepare_kernel<T, 4>;
+    kernel<<<delta_blocks + mask_blocks, 256, 0, stream>>>(out, dout, delta, (uint32_t)cells, p.cols, p.heads, p.rows, vec_ok,
+                                                           dout.sr < dout.sc, mask_blocks, p.mask, p.mask_sb, p.mask_sr, p.mask_sc, live,
+                                                           p.batch * p.rows);
     count_launch();
     status = check_launch("tcgen05 delta");
     if (status) return status;

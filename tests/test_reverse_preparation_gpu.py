@@ -33,3 +33,11 @@ def test_gradients(cuda, dtype, rows, cols, heads, kept, swapped):
     for name, got, ref in zip(("out", "dq", "dk", "dv", "dbias"), (out, *grads), want):
         error = float((got.detach().float().cpu() - ref).abs().max())
         assert error <= 2e-2 * max(1.0, float(ref.abs().max())), (name, error)
+
+
+@pytest.mark.parametrize("dtype,rows,cols,heads,kept,swapped", [(torch.bfloat16, 40, 130, 1, 129, False), (torch.float16, 10, 520, 1, None, True),
+                                                                (torch.bfloat16, 20, 268, 1, None, False), (torch.float16, 20, 284, 1, 280, False),
+                                                                (torch.bfloat16, 12, 196, 2, None, False)])
+def test_one_head(cuda, dtype, rows, cols, heads, kept, swapped):
+    """One head, whose dots have an instance of their own; bias gradients on either side of where their parts are added four keys a thread."""
+    test_gradients(cuda, dtype, rows, cols, heads, kept, swapped)
