@@ -62,24 +62,28 @@ __device__ __forceinline__ void load8(const T* p, int n, float (&out)[8]) {
   }
 }
 
-// The same as they were loaded, so that several can be under way without eight registers each.
+// The same as they were loaded, so that several can be under way without eight registers each (VEC; element by element, packing waits for each).
 template <typename T, bool VEC>
 struct Raw8 {
   uint4 words[sizeof(T) / 2];
   __device__ __forceinline__ void load(const T* p, int n, bool take) {
 #pragma unroll
-    for (int i = 0; i < int(sizeof(T) / 2); ++i) words[i] = make_uint4(0, 0, 0, 0);
-    if (!take) return;
-    if constexpr (VEC) {
-#pragma unroll
-      for (int i = 0; i < int(sizeof(T) / 2); ++i) words[i] = reinterpret_cast<const uint4*>(p)[i];
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (i < n) reinterpret_cast<T*>(words)[i] = p[i];
-    }
+    for (int i = 0; i < int(sizeof(T) / 2); ++i) words[i] = take ? reinterpret_cast<const uint4*>(p)[i] : make_uint4(0, 0, 0, 0);
   }
   __device__ __forceinline__ float operator[](int i) const { return float(reinterpret_cast<const T*>(words)[i]); }
+};
+template <typename T>
+struct Raw8<T, false> {
+  float values[8];
+  __device__ __forceinline__ void load(const T* p, int n, bool take) {
+    if (take) {
+      load8<T, false>(p, n, values);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) values[i] = 0.f;
+    }
+  }
+  __device__ __forceinline__ float operator[](int i) const { return values[i]; }
 };
 
 template <typename T, bool VEC>
@@ -157,7 +161,7 @@ struct GateGroup {
 __host__ __device__ inline int gate_chunks(int hidden) { return (2 * ((hidden + 7) / 8 * 8) + 63) / 64; }
 
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(256, 8) pair_gate_forward_kernel(PairShape s, const T* __restrict__ proj, int64_t ld,
+__global__ void __launch_bounds__(256, VEC ? 8 : 1) pair_gate_forward_kernel(PairShape s, const T* __restrict__ proj, int64_t ld,
                                                                 const T* __restrict__ mask, uint32_t* __restrict__ left,
                                                                 uint32_t* __restrict__ right) {
   constexpr int W = tokens_per_word<T>();
@@ -166,23 +170,48 @@ __global__ void __launch_bounds__(256, 8) pair_gate_forward_kernel(PairShape s, 
   const int64_t first = int64_t(blockIdx.x / chunks) * 32;  // first word of the tile in a plane
   const int cg = threadIdx.x & 7, word = threadIdx.x >> 3;
   const GateGroup own(s, chunk * 64 + cg * 8);
-  Raw8<T, VEC> gate[W], value[W];
-  float weight[W];
+  if constexpr (VEC) {
+    Raw8<T, VEC> gate[W], value[W];
+    float weight[W];
 #pragma unroll
-  for (int e = 0; e < W; ++e) {
-    const int64_t m = token_at(s, b, (first + word) * W + e);
-    const bool there = m >= 0 && own.n > 0;
-    const T* row = proj + m * ld + own.side * 2 * s.hidden + own.channel;
-    gate[e].load(row, own.n, there);
-    value[e].load(row + s.hidden, own.n, there);
-    weight[e] = !there ? 0.f : mask ? float(mask[m]) : 1.f;
-  }
+    for (int e = 0; e < W; ++e) {
+      const int64_t m = token_at(s, b, (first + word) * W + e);
+      const bool there = m >= 0 && own.n > 0;
+      const T* row = proj + m * ld + own.side * 2 * s.hidden + own.channel;
+      gate[e].load(row, own.n, there);
+      value[e].load(row + s.hidden, own.n, there);
+      weight[e] = !there ? 0.f : mask ? float(mask[m]) : 1.f;
+    }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float both[2];
+    for (int i = 0; i < 8; ++i) {
+      float both[2];
 #pragma unroll
-    for (int e = 0; e < W; ++e) both[e] = weight[e] * sigmoid_of<T>(gate[e][i]) * value[e][i];
-    tile.at(cg * 8 + i, word) = to_word<T>(both);
+      for (int e = 0; e < W; ++e) both[e] = weight[e] * sigmoid_of<T>(gate[e][i]) * value[e][i];
+      tile.at(cg * 8 + i, word) = to_word<T>(both);
+    }
+  } else {
+    float out[W][8];
+#pragma unroll
+    for (int e = 0; e < W; ++e) {
+      const int64_t m = token_at(s, b, (first + word) * W + e);
+      float gate[8], value[8];
+      if (m >= 0 && own.n > 0) {
+        const T* row = proj + m * ld + own.side * 2 * s.hidden + own.channel;
+        load8<T, false>(row, own.n, gate);
+        load8<T, false>(row + s.hidden, own.n, value);
+        const float weight = mask ? float(mask[m]) : 1.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) out[e][i] = weight * sigmoid_of<T>(gate[i]) * value[i];
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) out[e][i] = 0.f;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float both[2] = {out[0][i], out[W - 1][i]};
+      tile.at(cg * 8 + i, word) = to_word<T>(both);
+    }
   }
   __syncthreads();
   const int lane = threadIdx.x & 31;
@@ -216,6 +245,7 @@ __global__ void __launch_bounds__(256, VEC ? 6 : 4) pair_gate_backward_kernel(Pa
   }
   const int cg = threadIdx.x & 7, word = threadIdx.x >> 3;
   const GateGroup own(s, chunk * 64 + cg * 8);
+  constexpr bool kWords = VEC || W == 1;
   Raw8<T, VEC> gate[W], value[W];
   float weight[W];
   int64_t at[W];
@@ -224,14 +254,23 @@ __global__ void __launch_bounds__(256, VEC ? 6 : 4) pair_gate_backward_kernel(Pa
     const int64_t m = own.n > 0 ? token_at(s, b, (first + word) * W + e) : -1;
     at[e] = m;
     const T* row = proj + m * ld + own.side * 2 * s.hidden + own.channel;
-    gate[e].load(row, own.n, m >= 0);
-    value[e].load(row + s.hidden, own.n, m >= 0);
-    weight[e] = m < 0 ? 0.f : mask ? float(mask[m]) : 1.f;
+    if (kWords) {
+      gate[e].load(row, own.n, m >= 0);
+      value[e].load(row + s.hidden, own.n, m >= 0);
+      weight[e] = m < 0 ? 0.f : mask ? float(mask[m]) : 1.f;
+    } else if (m >= 0) {  // element by element one branch for all of a token's loads, which would otherwise be converted before the next ones
+      gate[e].load(row, own.n, true);
+      value[e].load(row + s.hidden, own.n, true);
+      weight[e] = mask ? float(mask[m]) : 1.f;
+    }
   }
   __syncthreads();
-  uint32_t grad[8];
+  float grad[8][2];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) grad[i] = tile.at(cg * 8 + i, word);
+  for (int i = 0; i < 8; ++i) {
+    if constexpr (kWords) grad[i][0] = __uint_as_float(tile.at(cg * 8 + i, word));  // (a word, split where it is needed)
+    else from_word<T>(tile.at(cg * 8 + i, word), grad[i]);
+  }
 #pragma unroll
   for (int e = 0; e < W; ++e) {
     if (at[e] < 0) continue;
@@ -239,7 +278,8 @@ __global__ void __launch_bounds__(256, VEC ? 6 : 4) pair_gate_backward_kernel(Pa
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       float both[2];
-      from_word<T>(grad[i], both);
+      if constexpr (kWords) from_word<T>(__float_as_uint(grad[i][0]), both);
+      else both[e] = grad[i][e];
       const float sg = sigmoid_of<T>(gate[e][i]), up = both[e] * weight[e];
       dvalue[i] = up * sg;
       dgate[i] = up * value[e][i] * sg * (1.f - sg);
@@ -261,15 +301,15 @@ __device__ __forceinline__ float affine_of(const void* p, int i, float missing) 
   return p ? float(reinterpret_cast<const A*>(p)[i]) : missing;
 }
 
-// Parameters c .. c + 7, `n` of which exist.
+// Parameters c .. c + 7 (c is a multiple of eight).
 template <typename A>
-__device__ __forceinline__ void affine8(const void* p, int c, int n, float missing, float (&out)[8]) {
+__device__ __forceinline__ void affine8(const void* p, int c, float missing, float (&out)[8]) {
   const A* from = reinterpret_cast<const A*>(p) + c;
-  if (p && n >= 8 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {  // (c is a multiple of eight)
+  if (p && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
     load8<A, true>(from, 8, out);
   } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) out[i] = p && i < n ? float(from[i]) : missing;
+    for (int i = 0; i < 8; ++i) out[i] = p ? float(from[i]) : missing;
   }
 }
 
@@ -352,8 +392,10 @@ __global__ void __launch_bounds__(kNormThreads) channel_norm_forward_kernel(Pair
   for (int e = 0; e < W; ++e) at[e] = token_at(s, b, (int64_t(blockIdx.x) * 32 + word) * W + e);
   for (int c = (threadIdx.x >> 7) * 32 + cg * 8; c < s.hidden; c += 64) {
     float v[8][2], w[8], offset[8];  // parameters once for all of the word's tokens (fetched one by one for each: 23.5 us at N = 384, now 21.8)
-    affine8<A>(weight, c, s.hidden - c, 1.f, w);
-    affine8<A>(bias, c, s.hidden - c, 0.f, offset);
+    if constexpr (VEC) {
+      affine8<A>(weight, c, 1.f, w);
+      affine8<A>(bias, c, 0.f, offset);
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i)
       if (VEC || c + i < s.hidden) from_word<T>(tile[(c + i) * kPitch + word], v[i]);
@@ -365,7 +407,8 @@ __global__ void __launch_bounds__(kNormThreads) channel_norm_forward_kernel(Pair
 #pragma unroll
       for (int i = 0; i < 8; ++i)
         out[i] = VEC || c + i < s.hidden
-                     ? (v[i][e] - mean) * rstd * w[i] + offset[i] : 0.f;
+                     ? (v[i][e] - mean) * rstd * (VEC ? w[i] : affine_of<A>(weight, c + i, 1.f)) + (VEC ? offset[i] : affine_of<A>(bias, c + i, 0.f))
+                     : 0.f;
       store8<T, VEC>(y + at[e] * s.hidden + c, s.hidden - c, out);
     }
   }
