@@ -139,7 +139,7 @@ __device__ __forceinline__ int64_t token_at(const PairShape& s, int b, int64_t p
 // prefix element): a token's piece of a projection is then 128 contiguous bytes of a 16-bit type (64-byte pieces: 55 and
 // 90 us forward and reverse at N = 384, 128 channels).  Pieces are kept as they were loaded until the arithmetic needs them: converted at
 // once, a token's loads waited for those of the token before, and the reverse spilled 60 bytes a thread at five CTAs per SM (51.4 and 78.2 us;
-// now 48.3 with eight CTAs and 62.2 with six, where a 16-bit thread spills 4, of 34.5 and 57.6 at the copy's rate).  The channel chunk is the
+// now 48.3 with eight CTAs and 62.2 with six, where a 16-bit thread spills 4, of 34.5 and 57.6 at the copy's rate); an f32 word is one token, whose forward pass gains nothing by it: N = 384, 64 channels, 42.9 us and 44.3).  The channel chunk is the
 // fastest index: neighbouring CTAs touch a token's other pieces while their pages are open.
 
 struct GateTile {  // rows = channels; rows 32 .. 63 stand four words on, so that a warp's eight channel groups miss each other's banks
@@ -161,7 +161,7 @@ struct GateGroup {
 __host__ __device__ inline int gate_chunks(int hidden) { return (2 * ((hidden + 7) / 8 * 8) + 63) / 64; }
 
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(256, VEC ? 8 : 1) pair_gate_forward_kernel(PairShape s, const T* __restrict__ proj, int64_t ld,
+__global__ void __launch_bounds__(256, 8) pair_gate_forward_kernel(PairShape s, const T* __restrict__ proj, int64_t ld,
                                                                 const T* __restrict__ mask, uint32_t* __restrict__ left,
                                                                 uint32_t* __restrict__ right) {
   constexpr int W = tokens_per_word<T>();
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(256, VEC ? 8 : 1) pair_gate_forward_kernel(Pai
   const int64_t first = int64_t(blockIdx.x / chunks) * 32;  // first word of the tile in a plane
   const int cg = threadIdx.x & 7, word = threadIdx.x >> 3;
   const GateGroup own(s, chunk * 64 + cg * 8);
-  if constexpr (VEC) {
+  if constexpr (VEC && W == 2) {
     Raw8<T, VEC> gate[W], value[W];
     float weight[W];
 #pragma unroll
@@ -197,8 +197,8 @@ __global__ void __launch_bounds__(256, VEC ? 8 : 1) pair_gate_forward_kernel(Pai
       float gate[8], value[8];
       if (m >= 0 && own.n > 0) {
         const T* row = proj + m * ld + own.side * 2 * s.hidden + own.channel;
-        load8<T, false>(row, own.n, gate);
-        load8<T, false>(row + s.hidden, own.n, value);
+        load8<T, VEC>(row, own.n, gate);
+        load8<T, VEC>(row + s.hidden, own.n, value);
         const float weight = mask ? float(mask[m]) : 1.f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) out[e][i] = weight * sigmoid_of<T>(gate[i]) * value[i];
