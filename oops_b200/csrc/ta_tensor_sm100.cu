@@ -57,8 +57,9 @@ struct FwdSmem {
   static constexpr int bias_full = v_ready + kv_rings * kStages;  // [bias_rings][2 buffers]
   static constexpr int bias_empty = bias_full + bias_rings * 2;
   static constexpr int s_full = bias_empty + bias_rings * 2;      // [2] S of a step is in tensor memory
-  static constexpr int p_full = s_full + 2;                       // [2] P is there, and S may be overwritten
-  static constexpr int pv_done = p_full + 2;                      // [2] the latest P V product has completed
+  static constexpr int p_full = s_full + 2;                       // [2] P is in tensor memory
+  static constexpr int s_free = p_full + 2;                       // [2] the scores of a step are in registers
+  static constexpr int pv_done = s_free + 2;                      // [2] the latest P V product has completed
   static constexpr int q_empty = pv_done + 2;                     // [2] every score product of an item has completed (PERSIST)
   static constexpr int num_bars = q_empty + 2;
   static constexpr int tmem_slot = bars + num_bars * 8;
@@ -94,7 +95,8 @@ struct FwdParams {
   int gate_vec16, plain_vec16;
 };
 
-constexpr float kStepSumLimit = 1024.f;  // a step's sum of probabilities that sends its warp back for a new reference
+// What sends a step's warp back for a new reference: the sum of the probabilities of the first 48 columns, or a base-2 logit of the last 16.
+constexpr float kStepSumLimit = 1024.f, kLastColumnsLimit = 6.f;
 
 // Where item `idx` lies: query item fastest, then head, row (or pair of rows), batch.
 struct FwdItem {
@@ -221,8 +223,17 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
       for (int item = int(blockIdx.x), turn = 0; ok && item_there(item, turn); item += int(gridDim.x), ++turn) {
         for (int i = 0; i < KS && ok; ++i, ++n) {
           const int next = st + 1 == kStages ? 0 : st + 1, next_round = next == 0 ? round + 1 : round;
-          // the operands of the next score product and of this value product arrive ahead of the probabilities
-          if (i + 1 < KS) ok = mbar_wait(bar(Smem::k_full + ring + next), next_round & 1, abort_flag);
+          // The next scores (of this item or the next one) overwrite these as soon as the last columns are in registers.
+          const bool more = i + 1 < KS, turns = PERSIST && !more && item + int(gridDim.x) < P.items;
+          if (turns) ok = mbar_wait(bar(Smem::q_full + w), (turn + 1) & 1, abort_flag);
+          if (ok && (more || turns)) {
+            ok = mbar_wait(bar(Smem::k_full + ring + next), next_round & 1, abort_flag);
+            if (ok) ok = mbar_wait(bar(Smem::s_free + w), n & 1, abort_flag);
+            if (!ok) break;
+            tc_fence_after_sync();
+            issue_qk(next);
+            if (PERSIST && (more ? i + 2 == KS : KS == 1)) mma_commit(bar(Smem::q_empty + w));
+          }
           if (ok) ok = mbar_wait(bar(Smem::v_full + ring + st), round & 1, abort_flag);
           // a warpgroup signs off the value steps with dropped keys after clearing their rows
           if (ok && signoff && i >= full_steps) {
@@ -232,10 +243,6 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
           if (ok) ok = mbar_wait(bar(Smem::p_full + w), n & 1, abort_flag);
           if (!ok) break;
           tc_fence_after_sync();
-          if (i + 1 < KS) {
-            issue_qk(next);  // the softmax waits for this one
-            if (PERSIST && i + 2 == KS) mma_commit(bar(Smem::q_empty + w));
-          }
           // O[128 x 32] += P[128 x 64] V[64 x 32]; V is MN-major (channel contiguous), 64-byte swizzle:
           // 8-key groups are 512 bytes apart, each 16-key step advances 1024 bytes.
           const uint64_t vdesc = vdesc0 + uint64_t((st * kKvBytes) >> 4);
@@ -244,14 +251,6 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
             mma_ts(o_t, p_t + kk * 8, vdesc + uint64_t(kk * (1024 >> 4)), idesc_pv, (i > 0 || kk > 0) ? 1u : 0u);
           mma_commit(bar(Smem::pv_done + w));
           mma_commit(bar(Smem::v_empty + ring + st));
-          if (PERSIST && i + 1 == KS && item + int(gridDim.x) < P.items) {  // the first scores of the next item
-            ok = mbar_wait(bar(Smem::q_full + w), (turn + 1) & 1, abort_flag);
-            if (ok) ok = mbar_wait(bar(Smem::k_full + ring + next), next_round & 1, abort_flag);
-            if (!ok) break;
-            tc_fence_after_sync();
-            issue_qk(next);
-            if (KS == 1) mma_commit(bar(Smem::q_empty + w));
-          }
           st = next;
           round = next_round;
         }
@@ -368,9 +367,10 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
         }
         return true;
       };
-      // Probabilities of the step into tensor memory; returns their sum.
+      // Probabilities of the step into tensor memory; returns their sum.  Before the exponentials of the last columns the
+      // scores are given back for the next product, unless the step has to be repeated (`wanted`, only asked where `may_repeat`).
       bool p_free = i == 0;
-      auto step_pass = [&]() -> float {
+      auto step_pass = [&](bool may_repeat, bool& wanted) -> float {
         const float shift = ref == -INFINITY ? 0.f : -ref;
         const f32x2 shift2 = pack2(shift, shift);
         f32x2 totals[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
@@ -394,6 +394,21 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
           }
           f32x2 x[8];
           logits16(chunk, s[chunk & 1], bw[chunk & 1], shift2, x);
+          if (chunk == 3) {
+            float lo, hi, peak = -INFINITY;
+            unpack2(add2(totals[0], totals[1]), lo, hi);
+            const float before = lo + hi;
+#pragma unroll
+            for (int n = 0; n < 8; ++n) {
+              unpack2(x[n], lo, hi);
+              peak = max3(peak, lo, hi);
+            }
+            wanted = may_repeat && !(before < kStepSumLimit && peak < kLastColumnsLimit);
+            if (__any_sync(0xffffffffu, wanted)) return 0.f;
+            tc_fence_before_sync();
+            mbar_arrive_warp(bar(Smem::s_free + w));
+            if (HAS_BIAS) mbar_arrive_warp(bar(Smem::bias_empty + bias_slot));
+          }
 #pragma unroll
           for (int n = 0; n < 8; ++n) {
             float lo, hi;
@@ -423,6 +438,8 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
           ok = mbar_wait(bar(Smem::pv_done + w), (at_step - 1) & 1, abort_flag);
           tc_fence_after_sync();
         }
+        mbar_arrive_warp(bar(Smem::s_free + w));
+        if (HAS_BIAS) mbar_arrive_warp(bar(Smem::bias_empty + bias_slot));
         uint32_t zeros[16];
 #pragma unroll
         for (int n = 0; n < 16; ++n) zeros[n] = 0u;
@@ -435,8 +452,7 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
           if (__any_sync(0xffffffffu, wanted)) ok = raise(wanted);
           else if (attempt > 0) break;
           if (!ok) return;
-          sum = step_pass();
-          wanted = !(sum < kStepSumLimit);
+          sum = step_pass(attempt == 0, wanted);
         }
       }
       if (!ok) return;
@@ -444,7 +460,6 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
       tmem_wait_st();
       tc_fence_before_sync();
       mbar_arrive_warp(bar(Smem::p_full + w));
-      if (HAS_BIAS) mbar_arrive_warp(bar(Smem::bias_empty + bias_slot));
     };
     for (int item = int(blockIdx.x), turn = 0; ok && item_there(item, turn); item += int(gridDim.x), ++turn, base += KS) {
     if (PERSIST) {
@@ -570,7 +585,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
       if ((i >= Smem::k_empty && i < Smem::v_full) || (i >= Smem::v_empty && i < Smem::v_ready)) arrivals = ROWS ? 1 : n_tiles;
       if (i >= Smem::v_ready && i < Smem::bias_full) arrivals = kTile / 32;
       if (i >= Smem::bias_empty && i < Smem::s_full) arrivals = ROWS ? n_tiles * (kTile / 32) : kTile / 32;
-      if (i >= Smem::p_full && i < Smem::pv_done) arrivals = kTile / 32;
+      if (i >= Smem::p_full && i < Smem::pv_done) arrivals = kTile / 32;  // (s_free among them)
       mbar_init(bar(i), arrivals);
     }
     if (lane == 0) *abort_flag = 0;
