@@ -152,6 +152,18 @@ __device__ __forceinline__ void sts_v4_at(uint32_t addr, uint4 v) {
   asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
+__device__ __forceinline__ uint32_t lds_u32_at(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ void lds_f2_at(uint32_t addr, float& a, float& b) {
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(addr));
+}
+__device__ __forceinline__ void sts_f2_at(uint32_t addr, float a, float b) {
+  asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(a), "f"(b) : "memory");
+}
+
 // Four words from global memory when `take` is set, zeros otherwise; like the loads above it keeps its place and its
 // result is not touched before the caller uses it.
 __device__ __forceinline__ uint4 ldg_v4_here_if(const void* p, bool take) {

@@ -235,9 +235,9 @@ __device__ __forceinline__ bool pair_vec_ok(const oops_ta_pair& t) {
 // ---------------------------------------------------------------------------------------------
 // shared pieces of the three tensor kernels
 // ---------------------------------------------------------------------------------------------
-// 608 threads: warps 0-15 are four warpgroups of 128 threads that do the element-wise work, warp 16 is
+// The single-pass kernel has 640 threads: warps 0-15 are four warpgroups of 128 threads that do the element-wise work, warp 16 is
 // the TMA producer, warp 17 issues the score products (S, dP) and owns the tensor-memory allocation, warp 18
-// issues the accumulating products (dQ, or dK and dV); the shared-bias kernel leaves warp 18 idle.  Two issuing
+// issues the accumulating products (dQ, or dK and dV), warp 19 prepares statistics and masked tiles; the shared-bias kernel has neither.  Two issuing
 // threads keep the tensor core fed: neither kind of product waits behind the other's barrier.  The element-wise
 // work of the reverse pass has no reduction along a score row, so the 64 columns of a step are split
 // between two warpgroups that address the same tensor-memory lanes (warp % 4 selects the lanes).
@@ -992,6 +992,12 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) ta_bwd_dkv_kernel(const 
 // of the shared-memory port are busy) between barriers that all sixteen warps pass together.  Hence no branch, fence or
 // generic-address store in a step's body, and the writers of the images do not fence: they release a barrier, and the
 // issuer that acquires it fences once for all of them before its products read (N = 768: 1190 -> 1120 us with both).
+// A statistics warp of its own puts -log2(e) lse and -delta of a part's queries into a table, a tile at a time and a part ahead, where every
+// thread used to fetch both for every step (N = 768: 1036 -> 1004 us, 1024: 2934 -> 2842, 2048: 22.7 -> 22.0 ms), and makes the row dots where
+// that is hidden (kOwnDeltaCols).  With a mask it also clears the rows of dropped keys and values in shared memory before any
+// product may read them; the element-wise warps give dropped keys a bias of minus infinity (their words are in registers) instead of
+// testing every probability in a second copy of the step's body (N = 384, 360 kept: 187 -> 179 us; 512: 378 -> 357), and the read-out
+// of a key tile stores zeros for them.
 // Halving the step between two sets of warps that run half a step apart was tried: the single P image couples them, 3 to 10 %
 // slower.
 // Rows of more than 768 columns have several groups.  The CTA walks them in order and carries the f32 sums of dK and
@@ -1005,8 +1011,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) ta_bwd_dkv_kernel(const 
 
 constexpr int kFMaxCols = 4096;          // longest row taken: 32 key tiles
 constexpr int kFMaxQTiles = 6;
-constexpr int kFThreads = 608;  // 16 element-wise warps, TMA producer, score issuer, accumulation issuer
-constexpr int kFProducerWarp = 16, kFScoreWarp = 17, kFAccWarp = 18;
+constexpr int kFThreads = 640;  // 16 element-wise warps, TMA producer, score issuer, accumulation issuer, statistics
+constexpr int kFProducerWarp = 16, kFScoreWarp = 17, kFAccWarp = 18, kFStatWarp = 19;
 constexpr int kFImage = 2 * 16384;       // P or dS of a step: two 64-key halves of 128 rows x 128 bytes
 constexpr int kFBias = 2 * kBiasStep;    // 128 x 128 bias tile as two 64-key boxes (staging: copied to registers at once)
 constexpr int kFSlots = 256;             // scratch slots of the group-to-group sums: one per SM id
@@ -1019,7 +1025,9 @@ struct FSmem {
   static constexpr int ps = v + 2 * kBigTile;          // P image (read by the dV products only, freed early)
   static constexpr int dss = ps + kFImage;             // [2] dS image
   static constexpr int bias = dss + 2 * kFImage;       // one staging tile
-  static constexpr int bars = bias + kFBias;
+  static constexpr int stats = bias + kFBias;          // [2][6][128] of two f32: statistics of a part's queries
+  static constexpr int kept = stats + 2 * kFMaxQTiles * kTile * 8;  // [4][4] u32: kept keys of a key tile
+  static constexpr int bars = kept + 64;
   static constexpr int qd_full = 0;                    // [3]
   static constexpr int qd_empty = qd_full + 3;         // [3]
   static constexpr int kv_full = qd_empty + 3;         // [2]
@@ -1033,7 +1041,10 @@ struct FSmem {
   static constexpr int p_done = pds_done + 2;          // the dV products have consumed the P image
   static constexpr int dkv_free = p_done + 1;          // dK and dV of a finished key tile have been read out
   static constexpr int dq_free = dkv_free + 1;         // dQ of a finished group of query tiles has been read out
-  static constexpr int num_bars = dq_free + 1;
+  static constexpr int stat_full = dq_free + 1;        // [2][6] the statistics of a query tile stand
+  static constexpr int stat_free = stat_full + 2 * kFMaxQTiles;  // [2] every warp is done with those of a part
+  static constexpr int kv_ready = stat_free + 2;       // [2] dropped keys have been cleared, and `kept` stands (masks)
+  static constexpr int num_bars = kv_ready + 2;
   static constexpr int tmem_slot = bars + num_bars * 8;
   static constexpr int abort_flag = tmem_slot + 4;
   static constexpr int total = abort_flag + 4;
@@ -1047,7 +1058,9 @@ struct FParams {
   float* slots;     // [kFSlots][2][8][slot_keys][4] f32: sums of dK and dV carried from group to group (groups > 1)
   int64_t slot_keys;
   const float* lse;
-  const float* delta;
+  float* delta;     // read, or written from `out` and `dout` where own_delta is set
+  oops_ta_pair out, dout;
+  int own_delta;
   const uint8_t* mask;
   const uint32_t* live;  // what prepare_kernel has found out about the mask
   int64_t m_sb, m_sr, m_sc;
@@ -1141,7 +1154,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       for (FWalk<GROUPS> w(P); !w.done() && ok; w.next()) {
         const int s = w.s, qs = s % 3, ks = w.ktc & 1;
         ok = mbar_wait_warp(bar(FSmem::qd_full + qs), (s / 3) & 1, abort_flag);
-        if (ok && w.qi == 0) ok = mbar_wait_warp(bar(FSmem::kv_full + ks), (w.ktc >> 1) & 1, abort_flag);
+        if (ok && w.qi == 0) ok = mbar_wait_warp(bar((has_mask ? FSmem::kv_ready : FSmem::kv_full) + ks), (w.ktc >> 1) & 1, abort_flag);
         if (ok && s > 0) ok = mbar_wait_warp(bar(FSmem::sd_free), (s - 1) & 1, abort_flag);
         if (!ok) break;
         tc_fence_after_sync();
@@ -1198,6 +1211,112 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
         if (qi == w.nq - 1) mma_commit_warp(bar(FSmem::kv_empty + ks));
       }
     }
+  } else if (warp == kFStatWarp) {
+    // Statistics of a part's queries, a tile at a time and a part ahead: -log2(e) lse, and -delta, which is rowsum(O * dO) where the
+    // caller has not left it.  Four lanes share a query, eight channels each.
+    bool ok = true;
+    auto tile_stats = [&](int part, int item, int first, int qi) {
+      const int buffer = part & 1, row = item / P.heads, h = item - row * P.heads, b = row / P.rows, r = row - b * P.rows;
+      const int64_t stat = int64_t(item) * P.cols;
+      const uint32_t table = smem_base + FSmem::stats + (buffer * kFMaxQTiles + qi) * (kTile * 8);
+      const int q0 = (first + qi) * kTile;
+      if (!P.own_delta) {
+        float lse[4], delta[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int q = q0 + j * 32 + lane;
+          lse[j] = q < P.cols ? ldg_f32_here(P.lse + stat + q) : INFINITY;
+          delta[j] = q < P.cols ? ldg_f32_here(P.delta + stat + q) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sts_f2_at(table + (j * 32 + lane) * 8, -lse[j] * kLog2e, -delta[j]);
+      } else {
+        const T* po = reinterpret_cast<const T*>(P.out.ptr) + b * P.out.sb + int64_t(r) * P.out.sr + h * P.out.sh + (lane & 3) * 8;
+        const T* pd = reinterpret_cast<const T*>(P.dout.ptr) + b * P.dout.sb + int64_t(r) * P.dout.sr + h * P.dout.sh + (lane & 3) * 8;
+#pragma unroll 1
+        for (int j = 0; j < kTile; j += 32) {
+          const int q = q0 + j + lane;
+          const float lse = q < P.cols ? ldg_f32_here(P.lse + stat + q) : INFINITY;
+          uint4 o[4], g[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int at = q0 + j + i * 8 + (lane >> 2);
+            o[i] = ldg_v4_here_if(po + int64_t(at) * P.out.sc, at < P.cols);
+            g[i] = ldg_v4_here_if(pd + int64_t(at) * P.dout.sc, at < P.cols);
+          }
+          float own = 0.f;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t ow[4] = {o[i].x, o[i].y, o[i].z, o[i].w}, gw[4] = {g[i].x, g[i].y, g[i].z, g[i].w};
+            float dot = 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) dot += Half2<T>::lo(ow[e]) * Half2<T>::lo(gw[e]) + Half2<T>::hi(ow[e]) * Half2<T>::hi(gw[e]);
+            dot += __shfl_xor_sync(0xffffffffu, dot, 1);
+            dot += __shfl_xor_sync(0xffffffffu, dot, 2);
+            const float mine = __shfl_sync(0xffffffffu, dot, (lane & 7) * 4);  // query i * 8 + lane % 8
+            if ((lane >> 3) == i) own = mine;
+          }
+          if (q < P.cols) P.delta[stat + q] = own;
+          sts_f2_at(table + (j + lane) * 8, -lse * kLog2e, -own);
+        }
+      }
+      mbar_arrive_warp(bar(FSmem::stat_full + buffer * kFMaxQTiles + qi));
+    };
+    FWalk<GROUPS> w(P);
+    uint32_t bytes[4] = {0, 0, 0, 0};  // of the mask, for the key tile to come
+    auto fetch_mask = [&](const FWalk<GROUPS>& at) {
+      if (!has_mask || at.done()) return;
+      const int row = at.item / P.heads, b = row / P.rows;
+      const uint8_t* mask_row = P.mask + b * P.m_sb + int64_t(row - b * P.rows) * P.m_sr;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int key = at.kt * kTile + i * 32 + lane;
+        bytes[i] = key < P.cols ? ldg_u8_here(mask_row + int64_t(key) * P.m_sc) : 0u;
+      }
+    };
+    fetch_mask(w);
+    for (; !w.done() && ok; w.next_tile()) {
+      const int kt = w.kt;
+      if (has_mask) {
+        const int slot = w.ktc & 1;
+        uint32_t kept[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) kept[i] = __ballot_sync(0xffffffffu, bytes[i] != 0);
+        FWalk<GROUPS> next = w;
+        next.next_tile();
+        fetch_mask(next);
+        ok = mbar_wait_warp(bar(FSmem::kv_full + slot), (w.ktc >> 1) & 1, abort_flag);
+        if (!ok) break;
+        if (lane == 0) sts_v4_at(smem_base + FSmem::kept + (w.ktc & 3) * 16, make_uint4(kept[0], kept[1], kept[2], kept[3]));
+        if ((kept[0] & kept[1] & kept[2] & kept[3]) != 0xffffffffu) {
+          // Dropped keys and values must not reach a product (0 * inf): their rows are cleared.
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (((kept[i] >> lane) & 1u) != 0) continue;
+            const uint32_t at = slot * kBigTile + (i * 32 + lane) * 64;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              sts_v4_at(smem_base + FSmem::k + at + c * 16, make_uint4(0, 0, 0, 0));
+              sts_v4_at(smem_base + FSmem::v + at + c * 16, make_uint4(0, 0, 0, 0));
+            }
+          }
+          fence_proxy_async_smem();
+        }
+        mbar_arrive_warp(bar(FSmem::kv_ready + slot));
+      }
+      // The tiles of the first part, then a tile of the next part for every key tile of this one.
+      FWalk<GROUPS> ahead = w;
+      ahead.kt = P.k_tiles - 1;
+      ahead.next_tile();
+      const bool there = !ahead.done() && kt < ahead.nq;
+      if (there && kt == 0 && ahead.part >= 2) ok = mbar_wait_warp(bar(FSmem::stat_free + (ahead.part & 1)), ((ahead.part >> 1) - 1) & 1, abort_flag);
+      if (!ok) break;
+#pragma unroll 1
+      for (int n = w.ktc == 0 ? -w.nq : 0; n < (there ? 1 : 0); ++n) {
+        const bool own = n < 0;
+        tile_stats(own ? 0 : ahead.part, own ? w.item : ahead.item, own ? w.first : ahead.first, own ? w.nq + n : kt);
+      }
+    }
   } else if (warp < 16) {
     const int wg = warp >> 2;  // 32 of the step's 128 keys
     const int t = tid & (kTile - 1);
@@ -1205,29 +1324,6 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     const uint32_t lanes_t = tmem_base + lane_field;
     const float scale = P.scale;
     const f32x2 c2 = pack2(scale * kLog2e, scale * kLog2e), log2e2 = pack2(kLog2e, kLog2e);
-    // Statistics of this thread's query in a step's query tile (items count (batch, row, head) as the statistics do), fetched
-    // one step ahead and left untouched till then.
-    const int64_t stat0 = int64_t(blockIdx.x) * P.cols;
-    auto fetch_stats = [&](const FWalk<GROUPS>& at, float& lse_raw, float& delta_raw) {
-      lse_raw = INFINITY;
-      delta_raw = 0.f;
-      const int q = at.qt() * kTile + t;
-      if (!at.done() && q < P.cols) {
-        const int64_t stat = GROUPS ? stat0 + q : int64_t(uint32_t(at.item) * uint32_t(P.cols) + uint32_t(q));
-        lse_raw = ldg_f32_here(P.lse + stat);
-        delta_raw = ldg_f32_here(P.delta + stat);
-      }
-    };
-    // The kept bit of this lane's key of a key tile (32 keys of this warpgroup), fetched a key tile ahead.
-    auto mask_row_of = [&](int item) -> const uint8_t* {
-      const int row = item / P.heads, b = row / P.rows;
-      return P.mask + b * P.m_sb + int64_t(row - b * P.rows) * P.m_sr;
-    };
-    auto fetch_keep = [&](const uint8_t* row, const FWalk<GROUPS>& at) -> uint32_t {
-      const int key = at.kt * kTile + wg * 32 + lane;
-      if (at.done() || key >= P.cols) return 0;
-      return has_mask ? ldg_u8_here(row + int64_t(key) * P.m_sc) : 1u;
-    };
     const int row0 = int(blockIdx.x) / P.heads, h0 = int(blockIdx.x) - row0 * P.heads, b0 = row0 / P.rows, r0 = row0 - b0 * P.rows;
     auto item_row = [&](const oops_ta_pair& t, int item) -> T* {
       if (GROUPS) return reinterpret_cast<T*>(t.ptr) + b0 * t.sb + int64_t(r0) * t.sr + h0 * t.sh;
@@ -1239,7 +1335,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     // dK (warpgroup 0) and dV (warpgroup 1) of key tile kt, complete for the query tiles of group g: lanes are keys.
     // With several groups the f32 sums travel from group to group through this SM's scratch slot (the same thread
     // owns a key in every group), and the last group stores the 16-bit result.
-    auto store_key_tile = [&](int item, int g, int kt) {
+    auto store_key_tile = [&](int item, int g, int kt, int tile) {  // `tile` counts key tiles
       if (wg > 1) return;
       uint32_t acc[32];
       tmem_ld32(lanes_t + (wg == 0 ? kDkCol : kDvCol), acc);
@@ -1251,6 +1347,10 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       if (key >= P.cols) return;
       const bool wanted = wg == 0 ? P.write_dk != 0 : P.write_dv != 0;
       if (!wanted) return;
+      if (has_mask && ((lds_u32_at(smem_base + FSmem::kept + (tile & 3) * 16 + (t >> 5) * 4) >> lane) & 1u) == 0) {
+#pragma unroll
+        for (int n = 0; n < 32; ++n) acc[n] = 0u;  // a dropped key, whatever the queries and the upstream gradient hold
+      }
       if (GROUPS) {
         // plane i of the slot holds channels 4i .. 4i+3 of every key, so that a warp's 32 keys are 512 contiguous bytes
         float4* slot = reinterpret_cast<float4*>(P.slots) + (int64_t(sm_id) * 2 + wg) * 8 * P.slot_keys + key;
@@ -1287,10 +1387,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       mbar_arrive_warp(bar(FSmem::dq_free));
     };
     FWalk<GROUPS> w(P);
-    float lse_next, delta_next;
-    fetch_stats(w, lse_next, delta_next);
-    const uint8_t* mask_row = has_mask ? mask_row_of(w.item) : nullptr;  // of the key tile to come
-    uint32_t keep_raw = has_bits ? fetch_keep(mask_row, w) : 0u, bits = 0xffffffffu;
+    uint32_t bits = 0xffffffffu;  // kept keys among this warpgroup's 32
     bool ok = true;
     if (GROUPS && sm_id >= uint32_t(kFSlots)) {  // no scratch slot for this SM id: give up like a wait that ran out
       *abort_flag = 1;
@@ -1300,37 +1397,26 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     // bias row of this thread's query in the staging tile: box (wg >> 1), 16-byte chunks (wg & 1) * 4 .. + 3
     const uint8_t* bias_row = smem_gen + FSmem::bias + (wg >> 1) * kBiasStep + t * 128 + (((t & 7) ^ ((wg & 1) * 4)) << 4);
 
-    int last_item = 0, last_part = 0, last_first = 0, last_kt = 0;  // of the previous step
-    for (; !w.done() && ok; last_item = w.item, last_part = w.part, last_first = w.first, last_kt = w.kt, w.next()) {
-      const int s = w.s, kt = w.kt, qi = w.qi, buf = s & 1;
-      if (has_bits && qi == 0) {
-        bits = __ballot_sync(0xffffffffu, keep_raw != 0);
-        FWalk<GROUPS> ahead = w;
-        ahead.next_tile();
-        if (!GROUPS && has_mask && ahead.kt == 0 && !ahead.done()) mask_row = mask_row_of(ahead.item);
-        keep_raw = fetch_keep(mask_row, ahead);
-        if (has_mask && bits != 0xffffffffu) {
-          // Key rows of dropped keys must not reach the dQ product (0 * inf): they are cleared in shared memory, eight of
-          // this warpgroup's 32 by each warp.  The scores of these keys are dropped whatever they are.
-          ok = mbar_wait(bar(FSmem::kv_full + (w.ktc & 1)), (w.ktc >> 1) & 1, abort_flag);
-          if (!ok) break;
-          const int key = (warp & 3) * 8 + (lane >> 2);
-          if (((bits >> key) & 1u) == 0)
-            sts_v4_at(smem_base + FSmem::k + (w.ktc & 1) * kBigTile + (wg * 32 + key) * 64 + (lane & 3) * 16, make_uint4(0, 0, 0, 0));
-        }
-      }
+    int last_item = 0, last_part = 0, last_first = 0, last_kt = 0, last_tile = 0;  // of the previous step
+    for (; !w.done() && ok; last_item = w.item, last_part = w.part, last_first = w.first, last_kt = w.kt, last_tile = w.ktc, w.next()) {
+      const int s = w.s, kt = w.kt, qi = w.qi, buf = s & 1, table = (w.part & 1) * kFMaxQTiles + qi;
       if (s > 0) mbar_arrive_warp(bar(FSmem::pds_full + (buf ^ 1)));  // the images of step s - 1, their stores drained by now
       // The three phases the step needs first are probed together (one round trip to the barrier words); in the steady
       // state, where these warps are the slow side of the pipeline, all three are complete.
       const bool bias_there = HAS_BIAS && mbar_test(bar(FSmem::bias_full), s & 1);
       const bool image_free = s < 2 || mbar_test(bar(FSmem::pds_done + buf), ((s >> 1) - 1) & 1);
       const bool scores_there = mbar_test(bar(FSmem::sd_full), s & 1);
-      const float neg_lse2 = -lse_next * kLog2e, neg_delta = -delta_next;
-      {
-        FWalk<GROUPS> ahead = w;
-        ahead.next();
-        fetch_stats(ahead, lse_next, delta_next);
+      const bool stats_there = kt > 0 || mbar_test(bar(FSmem::stat_full + table), (w.part >> 1) & 1);
+      if (has_mask && qi == 0) {
+        const bool kept_there = mbar_test(bar(FSmem::kv_ready + (w.ktc & 1)), (w.ktc >> 1) & 1);
+        ok = mbar_wait_probed(kept_there, bar(FSmem::kv_ready + (w.ktc & 1)), (w.ktc >> 1) & 1, abort_flag);
+        if (!ok) break;
+        bits = lds_u32_at(smem_base + FSmem::kept + (w.ktc & 3) * 16 + wg * 4);
       }
+      ok = mbar_wait_probed(stats_there, bar(FSmem::stat_full + table), (w.part >> 1) & 1, abort_flag);
+      if (!ok) break;
+      float neg_lse2, neg_delta;
+      lds_f2_at(smem_base + FSmem::stats + (table * kTile + t) * 8, neg_lse2, neg_delta);
       const f32x2 nl1 = pack2(neg_lse2, neg_lse2), nd1 = pack2(neg_delta, neg_delta);
       // The step's bias words are requested at once; the staging tile is handed back as soon as they have arrived
       // (below, after the first scores have been fetched), so that the next tile's copy runs under this step's arithmetic.
@@ -1346,6 +1432,30 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       if (ok) ok = mbar_wait_probed(scores_there, bar(FSmem::sd_full), s & 1, abort_flag);
       if (!ok) break;
       tc_fence_after_sync();
+      if (has_bits && qi == 0) {
+        if (!has_mask) {
+          const int there = P.cols - kt * kTile - wg * 32;
+          bits = there >= 32 ? 0xffffffffu : there <= 0 ? 0u : (1u << there) - 1;
+        }
+        bits = __shfl_sync(0xffffffffu, bits, 0);
+      }
+      // Keys behind the row's end have zeros for operands and bias: what comes out for them is 2^nl and 2^nl nd, which nobody stores
+      // and which meet zeros in dQ, unless they leave the range of 16 bits.
+      if (HAS_BIAS && has_bits && bits != 0xffffffffu && (has_mask || __any_sync(0xffffffffu, !(neg_lse2 < 10.f && fabsf(neg_delta) < 32.f)))) {
+        // Dropped keys get a bias of minus infinity: no test in the body below.
+        constexpr uint32_t kNone = Half2<T>::kFormat == 1 ? 0xff80u : 0xfc00u;
+        auto drop = [&](uint32_t& word, int key) {
+          if (((bits >> key) & 1u) == 0) word = (word & 0xffff0000u) | kNone;
+          if (((bits >> (key + 1)) & 1u) == 0) word = (word & 0xffffu) | (kNone << 16);
+        };
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          drop(bias_words[c].x, c * 8);
+          drop(bias_words[c].y, c * 8 + 2);
+          drop(bias_words[c].z, c * 8 + 4);
+          drop(bias_words[c].w, c * 8 + 6);
+        }
+      }
       // image rows are queries; this warpgroup's 32 keys are chunks (wg & 1) * 4 .. + 3 of half (wg >> 1)
       const int row_at = (wg >> 1) * 16384 + t * 128 + (((t & 7) ^ ((wg & 1) * 4)) << 4);
       const uint32_t p_row = smem_base + FSmem::ps + row_at;
@@ -1395,7 +1505,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
                     make_uint4(pack16<T>(ds2[0]), pack16<T>(ds2[1]), pack16<T>(ds2[2]), pack16<T>(ds2[3])));
         }
       };
-      if (bits == 0xffffffffu)
+      if (HAS_BIAS || !has_bits || bits == 0xffffffffu)
         step_body(std::false_type{});
       else
         step_body(std::true_type{});
@@ -1414,8 +1524,11 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
         ok = mbar_wait(bar(FSmem::pds_done + ((s - 1) & 1)), ((s - 1) >> 1) & 1, abort_flag);
         if (!ok) break;
         tc_fence_after_sync();
-        store_key_tile(last_item, last_part, last_kt);
-        if (kt == 0) store_query_tiles(last_item, last_first);
+        store_key_tile(last_item, last_part, last_kt, last_tile);
+        if (kt == 0) {
+          store_query_tiles(last_item, last_first);
+          mbar_arrive_warp(bar(FSmem::stat_free + ((w.part & 1) ^ 1)));
+        }
       }
     }
     const int steps = w.s;
@@ -1427,7 +1540,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     if (ok && steps > 0) ok = mbar_wait(bar(FSmem::pds_done + ((steps - 1) & 1)), ((steps - 1) >> 1) & 1, abort_flag);
     if (ok && steps > 0) {
       tc_fence_after_sync();
-      store_key_tile(last_item, last_part, last_kt);
+      store_key_tile(last_item, last_part, last_kt, last_tile);
       store_query_tiles(last_item, last_first);
     }
     if (GROUPS) {
@@ -1500,6 +1613,11 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
     mbar_init(bar(FSmem::sd_free), 16);
     mbar_init(bar(FSmem::dkv_free), 8);
     mbar_init(bar(FSmem::dq_free), 16);
+    for (int i = 0; i < 2 * kFMaxQTiles; ++i) mbar_init(bar(FSmem::stat_full + i), 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar(FSmem::stat_free + i), 16);
+      mbar_init(bar(FSmem::kv_ready + i), 1);
+    }
     fence_barrier_init();
   }
   if (warp == kFScoreWarp) {
@@ -1963,6 +2081,11 @@ uint64_t fused_slot_bytes(const oops_ta_problem& p) {
   return align256(uint64_t(kFSlots) * 2 * fused_slot_keys(p) * kHeadDim * sizeof(float));
 }
 
+// Rows from which the single-pass kernel makes the row dots itself.  Its statistics warp takes some 6000 clocks a query tile for them, which
+// are hidden under the steps where a row has many: 768 columns 1023 + 51 (prepare_kernel) -> 1040 + 5 us, 700 950 + 44 -> 970; 512
+// 329 + 24 -> 350, 256 (two samples) 104 + 11 -> 160.  In rows of several groups the first tiles delay a CTA's start (1024: 2842 + 84 -> 3149).
+constexpr int kOwnDeltaCols = 4 * kTile;
+
 // The single-pass kernel serves calls that want dQ together with dK or dV and no per-row bias gradient, on rows
 // of up to 4096 columns (32 key tiles, one bit each in the words that describe a row's mask).
 bool fused_applies(const oops_ta_problem& p, const oops_ta_grads& g) {
@@ -2029,7 +2152,10 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
 
   // delta = rowsum(O * dO), unless an earlier call has left it, and what the kernels ask about the mask, which they must find
   // whatever the workspace holds (a second call with a mask: 159 -> 169 us at 96 rows of 768 columns, 1165 -> 1168 at 768).
-  const int64_t total = (p.flags & OOPS_TA_FLAG_REUSE_DELTA) != 0 ? 0 : int64_t(p.batch) * p.rows * p.heads * p.cols;
+  const bool fused = fused_applies(p, g);
+  const bool words16 = (reinterpret_cast<uintptr_t>(out.ptr) & 15) == 0 && out.sb % 8 == 0 && out.sr % 8 == 0 && out.sc % 8 == 0 && out.sh % 8 == 0;
+  const bool own_delta = fused && words16 && (p.flags & OOPS_TA_FLAG_REUSE_DELTA) == 0 && p.cols > kOwnDeltaCols && fused_groups(p) == 1;
+  const int64_t total = (p.flags & OOPS_TA_FLAG_REUSE_DELTA) != 0 || own_delta ? 0 : int64_t(p.batch) * p.rows * p.heads * p.cols;
   const int64_t cells = p.heads > 0 ? total / p.heads : 0;
   const unsigned delta_blocks = (unsigned)ceil_div(cells, 64);
   const unsigned mask_blocks = live ? (unsigned)ceil_div(int64_t(p.batch) * p.rows, 8) : 0u;
@@ -2046,7 +2172,6 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
     if (status) return status;
   }
 
-  const bool fused = fused_applies(p, g);
   if (fused) {
     FParams P{};
     status = encode_pair(&P.map_q, p, p.q, kTile, "query");
@@ -2064,6 +2189,9 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
     P.write_dv = g.dv.ptr != nullptr;
     P.lse = lse;
     P.delta = delta;
+    P.out = out;
+    P.dout = dout;
+    P.own_delta = own_delta;
     P.mask = p.mask;
     P.m_sb = p.mask_sb;
     P.m_sr = p.mask_sr;
