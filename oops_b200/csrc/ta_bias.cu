@@ -1,5 +1,5 @@
 // Bias rows for the TMA kernels: a 16-bit bias (batch, group, head, query, key) of any strides copied to contiguous rows of
-// whole 16-byte words, zeros behind the last key.  One launch for what took a permuting copy, a fill and a padding copy.
+// whole 16-byte words, zeros (or another value, up to a longer row) behind the last key.  One launch for what took a permuting copy, a fill and a padding copy.
 //
 // Bound by latency and, for a bias as a linear map over the pair leaves it (heads innermost), by strided reads.  A thread
 // writes one word of eight keys.  Neighbouring threads then take the heads of the same cells where the heads are the
@@ -16,7 +16,8 @@ struct BiasRows {
   int64_t s_b, s_g, s_h, s_q, s_k;
   uint32_t words, heads, cols, groups;  // words of a row
   uint64_t total;
-  int heads_inner;
+  int heads_inner, whole;  // whole: rows of the source are whole 16-byte words
+  uint32_t fill;           // two elements of padding
 };
 
 // I counts words: 32 bits up to 64 GB of them.
@@ -39,11 +40,16 @@ __global__ void __launch_bounds__(256) bias_rows_kernel(const BiasRows p) {
   }
   const uint32_t g = uint32_t(i % p.groups), b = uint32_t(i / p.groups);
   const uint16_t* src = p.src + b * p.s_b + g * p.s_g + h * p.s_h + q * p.s_q;
-  uint32_t packed[4] = {0, 0, 0, 0};
+  uint32_t packed[4] = {p.fill, p.fill, p.fill, p.fill};
+  if (p.whole && word * 8 + 8 <= p.cols) {
+    const uint4 v = *reinterpret_cast<const uint4*>(src + word * 8);
+    packed[0] = v.x; packed[1] = v.y; packed[2] = v.z; packed[3] = v.w;
+  } else {
 #pragma unroll
-  for (uint32_t e = 0; e < 8; ++e) {
-    const uint32_t key = word * 8 + e;
-    if (key < p.cols) packed[e / 2] |= uint32_t(src[int64_t(key) * p.s_k]) << (e % 2 * 16);
+    for (uint32_t e = 0; e < 8; ++e) {
+      const uint32_t key = word * 8 + e;
+      if (key < p.cols) packed[e / 2] = (packed[e / 2] & (0xffff0000u >> (e % 2 * 16))) | uint32_t(src[int64_t(key) * p.s_k]) << (e % 2 * 16);
+    }
   }
   const int64_t row = ((int64_t(b) * p.groups + g) * p.heads + h) * p.cols + q;
   reinterpret_cast<uint4*>(p.dst)[row * p.words + word] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
@@ -51,7 +57,8 @@ __global__ void __launch_bounds__(256) bias_rows_kernel(const BiasRows p) {
 
 }  // namespace
 
-int bias_rows(int batch, int groups, int heads, int cols, const void* src, const int64_t strides[5], void* dst, cudaStream_t stream) {
+int bias_rows(int batch, int groups, int heads, int cols, const void* src, const int64_t strides[5], void* dst, cudaStream_t stream,
+              int row, uint16_t fill) {
   BiasRows p{};
   p.src = reinterpret_cast<const uint16_t*>(src);
   p.dst = reinterpret_cast<uint16_t*>(dst);
@@ -60,7 +67,11 @@ int bias_rows(int batch, int groups, int heads, int cols, const void* src, const
   p.s_h = strides[2];
   p.s_q = strides[3];
   p.s_k = strides[4];
-  p.words = uint32_t(ceil_div(cols, 8));
+  p.words = uint32_t(ceil_div(row > 0 ? row : cols, 8));
+  p.fill = fill * 0x10001u;
+  auto words = [](int64_t stride, int size) { return size == 1 || stride % 8 == 0; };
+  p.whole = strides[4] == 1 && (reinterpret_cast<uintptr_t>(src) & 15) == 0 && words(strides[0], batch) && words(strides[1], groups) &&
+            words(strides[2], heads) && words(strides[3], cols);
   p.heads = uint32_t(heads);
   p.cols = uint32_t(cols);
   p.groups = uint32_t(groups);

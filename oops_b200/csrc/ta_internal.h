@@ -86,7 +86,9 @@ int packed_pair_mask(const uint8_t* tokens, const int64_t* token_offsets, int sa
                      cudaStream_t stream);
 int packed_pair_mask_max_samples();
 // 16-bit bias of any strides (batch, group, head, query, key) to contiguous rows of ceil(cols / 8) 16-byte words.
-int bias_rows(int batch, int groups, int heads, int cols, const void* src, const int64_t strides[5], void* dst, cudaStream_t stream);
+// `row`: the length of a row in elements, a multiple of 8, where it is to be more than that; `fill`: the bits of its padding.
+int bias_rows(int batch, int groups, int heads, int cols, const void* src, const int64_t strides[5], void* dst, cudaStream_t stream,
+              int row = 0, uint16_t fill = 0);
 // Layer normalisation over the last axis of (rows, width) activations (row strides in elements, contiguous rows);
 // weight / bias / gradients of them may be NULL; affine_dtype is the activation dtype or f32.
 uint64_t layer_norm_backward_workspace_bytes(int64_t rows, int width);

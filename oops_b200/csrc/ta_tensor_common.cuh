@@ -119,13 +119,24 @@ int encode_pair(CUtensorMap* map, const oops_ta_problem& p, const oops_ta_pair& 
   return encode_map(map, p.dtype, t.ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B, what);
 }
 
-// Map over a bias viewed as (inner, outer, head, group, batch) with `inner` contiguous; box = 64 x `box_outer`.
+// Map over a bias viewed as (inner, outer, head, group, batch) with `inner` (cols, where not given) contiguous; box = 64 x `box_outer`.
 int encode_bias(CUtensorMap* map, const oops_ta_problem& p, const void* ptr, int64_t s_outer, int64_t sh, int64_t sg,
-                int64_t sb, uint32_t box_outer, const char* what) {
-  const uint64_t dims[5] = {uint64_t(p.cols), uint64_t(p.cols), uint64_t(p.heads), uint64_t(p.bias_groups), uint64_t(p.batch)};
+                int64_t sb, uint32_t box_outer, const char* what, int inner = 0) {
+  const uint64_t dims[5] = {uint64_t(inner > 0 ? inner : p.cols), uint64_t(p.cols), uint64_t(p.heads), uint64_t(p.bias_groups), uint64_t(p.batch)};
   const int64_t strides[4] = {s_outer, sh, sg, sb};
   const uint32_t box[5] = {64, box_outer, 1, 1, 1};
   return encode_map(map, p.dtype, ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, what);
+}
+
+// A row-shared bias in rows of whole key tiles whose padding is minus infinity, in a call's scratch: keys behind the end of a ragged row then
+// have no probability without being told apart (their operands are the zeros of the copies), and the kernels take the walks without tests.
+int closed_row(const oops_ta_problem& p) { return int(ceil_div(p.cols, kTile)) * kTile; }
+uint64_t closed_bias_bytes(const oops_ta_problem& p) { return uint64_t(p.batch) * p.heads * p.cols * closed_row(p) * 2; }
+
+int close_bias(CUtensorMap* map, const oops_ta_problem& p, void* scratch, const char* what, cudaStream_t stream) {
+  const int64_t strides[5] = {p.bias_sb, p.bias_sg, p.bias_sh, p.bias_sq, p.bias_sk}, row = closed_row(p), plane = p.cols * row;
+  const int status = bias_rows(p.batch, 1, p.heads, p.cols, p.bias, strides, scratch, stream, int(row), p.dtype == OOPS_TA_BF16 ? 0xff80 : 0xfc00);
+  return status ? status : encode_bias(map, p, scratch, row, plane, plane * p.heads, plane * p.heads, kTile, what, int(row));
 }
 
 int sm_count() {
