@@ -1068,6 +1068,7 @@ struct FParams {
   int q_tiles, k_tiles, groups, tiles_per_group;
   int write_dq, write_dk, write_dv;
   int closed;  // the bias is minus infinity behind a ragged row's end
+  const uint32_t *prefix, *uniform;  // kept first keys of every row and of every sample's rows, null where nobody has looked
   float scale;
 };
 
@@ -1082,8 +1083,8 @@ struct FWalk {
   int part, item, first;  // part, its item, its first query tile
   int kt, qi, nq;         // key tile, query tile within the part, query tiles of the part
   int s, ktc;             // steps and key tiles walked so far
-  __device__ FWalk(const FParams& P)
-      : tiles_per_group(P.tiles_per_group), q_tiles(P.q_tiles), k_tiles(P.k_tiles), parts(GROUPS ? P.groups : P.items),
+  __device__ FWalk(const FParams& P, int k_tiles)
+      : tiles_per_group(P.tiles_per_group), q_tiles(P.q_tiles), k_tiles(k_tiles), parts(GROUPS ? P.groups : P.items),
         item_step(int(gridDim.x)), part(0), item(int(blockIdx.x)), first(0), kt(0), qi(0), nq(min(P.tiles_per_group, P.q_tiles)),
         s(0), ktc(0) {}
   __device__ bool done() const { return GROUPS ? part >= parts : item >= parts; }
@@ -1110,11 +1111,18 @@ struct FWalk {
 
 // GROUPS: rows of several groups of query tiles.  BITS: some key may be dropped, by the mask or because the last key tile
 // is ragged.
-template <typename T, bool HAS_BIAS, bool GROUPS, bool BITS>
+template <typename T, bool HAS_BIAS, bool GROUPS, bool BITS, bool PREFIX>
 __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base, uint8_t* smem_gen, volatile int* abort_flag,
-                                           uint32_t tmem_base, int tid, int warp, int lane) {
+                                           uint32_t tmem_base, int tid, int warp, int lane, int k_tiles) {
   auto bar = [&](int index) -> uint32_t { return smem_base + FSmem::bars + index * 8; };
   const bool has_mask = BITS && P.mask != nullptr;
+  constexpr bool prefixes = PREFIX;
+  static_assert(!PREFIX || !BITS);
+  // PREFIX: rows keep the first keys of their sample's prefix, or none, in `k_tiles` key tiles; dropped keys are
+  // cleared before a product reads them.
+  auto request_prefix = [&](int item) -> uint32_t {  // every lane's copy; an item ahead of its use
+    return PREFIX && item < P.items ? *reinterpret_cast<const volatile uint32_t*>(P.prefix + item / P.heads) : 0u;
+  };
   constexpr bool has_bits = BITS;
   // tensor-memory columns
   constexpr int kSCol = 0, kDpCol = 128, kDkCol = 256, kDvCol = 288, kDqCol = 320;
@@ -1122,7 +1130,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
   if (warp == kFProducerWarp) {
     if (lane == 0) {
       bool ok = true;
-      for (FWalk<GROUPS> w(P); !w.done() && ok; w.next()) {
+      for (FWalk<GROUPS> w(P, k_tiles); !w.done() && ok; w.next()) {
         const int s = w.s, kt = w.kt, qt = w.qt(), qs = s % 3;
         const int row = w.item / P.heads, h = w.item - row * P.heads, b = row / P.rows, r = row - b * P.rows;
         if (w.qi == 0) {
@@ -1152,10 +1160,10 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     {
       constexpr uint32_t idesc = instr_desc(Half2<T>::kFormat, 0, 0, kTile, kTile);
       bool ok = true;
-      for (FWalk<GROUPS> w(P); !w.done() && ok; w.next()) {
+      for (FWalk<GROUPS> w(P, k_tiles); !w.done() && ok; w.next()) {
         const int s = w.s, qs = s % 3, ks = w.ktc & 1;
         ok = mbar_wait_warp(bar(FSmem::qd_full + qs), (s / 3) & 1, abort_flag);
-        if (ok && w.qi == 0) ok = mbar_wait_warp(bar((has_mask ? FSmem::kv_ready : FSmem::kv_full) + ks), (w.ktc >> 1) & 1, abort_flag);
+        if (ok && w.qi == 0) ok = mbar_wait_warp(bar((has_mask || prefixes ? FSmem::kv_ready : FSmem::kv_full) + ks), (w.ktc >> 1) & 1, abort_flag);
         if (ok && s > 0) ok = mbar_wait_warp(bar(FSmem::sd_free), (s - 1) & 1, abort_flag);
         if (!ok) break;
         tc_fence_after_sync();
@@ -1178,7 +1186,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       constexpr uint32_t idesc_t = instr_desc(fmt, 1, 1, kTile, kHeadDim);  // A = image^T (M = keys), B MN-major
       constexpr uint32_t idesc_q = instr_desc(fmt, 0, 1, kTile, kHeadDim);  // A = image (M = queries), B MN-major
       bool ok = true;
-      for (FWalk<GROUPS> w(P); !w.done() && ok; w.next()) {
+      for (FWalk<GROUPS> w(P, k_tiles); !w.done() && ok; w.next()) {
         const int s = w.s, kt = w.kt, qi = w.qi, qs = s % 3, ks = w.ktc & 1;
         ok = mbar_wait_warp(bar(FSmem::qd_full + qs), (s / 3) & 1, abort_flag);
         if (ok) ok = mbar_wait_warp(bar(FSmem::kv_full + ks), (w.ktc >> 1) & 1, abort_flag);
@@ -1216,7 +1224,13 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     // Statistics of a part's queries, a tile at a time and a part ahead: -log2(e) lse, and -delta, which is rowsum(O * dO) where the
     // caller has not left it.  Four lanes share a query, eight channels each.
     bool ok = true;
-    auto tile_stats = [&](int part, int item, int first, int qi) {
+    // `dead`: no key is kept, every probability, and dS, is zero.  `in_use`: the table holds a part that has to be through first (the words are
+    // under way meanwhile).
+    auto tile_stats = [&](int part, int item, int first, int qi, bool dead, bool in_use) {
+      auto table_free = [&]() {
+        if (in_use) ok = mbar_wait_warp(bar(FSmem::stat_free + (part & 1)), ((part >> 1) - 1) & 1, abort_flag);
+        return ok;
+      };
       const int buffer = part & 1, row = item / P.heads, h = item - row * P.heads, b = row / P.rows, r = row - b * P.rows;
       const int64_t stat = int64_t(item) * P.cols;
       const uint32_t table = smem_base + FSmem::stats + (buffer * kFMaxQTiles + qi) * (kTile * 8);
@@ -1229,9 +1243,11 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
           lse[j] = q < P.cols ? ldg_f32_here(P.lse + stat + q) : INFINITY;
           delta[j] = q < P.cols ? ldg_f32_here(P.delta + stat + q) : 0.f;
         }
+        if (!table_free()) return;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) sts_f2_at(table + (j * 32 + lane) * 8, -lse[j] * kLog2e, -delta[j]);
+        for (int j = 0; j < 4; ++j) sts_f2_at(table + (j * 32 + lane) * 8, dead ? -INFINITY : -lse[j] * kLog2e, dead ? 0.f : -delta[j]);
       } else {
+        if (!table_free()) return;
         const T* po = reinterpret_cast<const T*>(P.out.ptr) + b * P.out.sb + int64_t(r) * P.out.sr + h * P.out.sh + (lane & 3) * 8;
         const T* pd = reinterpret_cast<const T*>(P.dout.ptr) + b * P.dout.sb + int64_t(r) * P.dout.sr + h * P.dout.sh + (lane & 3) * 8;
 #pragma unroll 1
@@ -1258,12 +1274,12 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
             if ((lane >> 3) == i) own = mine;
           }
           if (q < P.cols) P.delta[stat + q] = own;
-          sts_f2_at(table + (j + lane) * 8, -lse * kLog2e, -own);
+          sts_f2_at(table + (j + lane) * 8, dead ? -INFINITY : -lse * kLog2e, dead ? 0.f : -own);
         }
       }
       mbar_arrive_warp(bar(FSmem::stat_full + buffer * kFMaxQTiles + qi));
     };
-    FWalk<GROUPS> w(P);
+    FWalk<GROUPS> w(P, k_tiles);
     uint32_t bytes[4] = {0, 0, 0, 0};  // of the mask, for the key tile to come
     auto fetch_mask = [&](const FWalk<GROUPS>& at) {
       if (!has_mask || at.done()) return;
@@ -1276,10 +1292,37 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       }
     };
     fetch_mask(w);
-    for (; !w.done() && ok; w.next_tile()) {
+    auto clear_key = [&](int slot, int key) {
+      const uint32_t at = slot * kBigTile + key * 64;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        sts_v4_at(smem_base + FSmem::k + at + c * 16, make_uint4(0, 0, 0, 0));
+        sts_v4_at(smem_base + FSmem::v + at + c * 16, make_uint4(0, 0, 0, 0));
+      }
+    };
+    uint32_t item_kept = 0, next_kept = request_prefix(int(blockIdx.x));
+    auto last = w;  // the key tile before
+    // The first tile of all travels with the mask's first bytes.
+    if (!w.done()) tile_stats(0, w.item, w.first, 0, prefixes && __shfl_sync(0xffffffffu, next_kept, 0) == 0, false);
+    for (; !w.done() && ok; last = w, w.next_tile()) {
       const int kt = w.kt;
+      if (prefixes && kt == 0) {
+        item_kept = __shfl_sync(0xffffffffu, next_kept, 0);
+        next_kept = request_prefix(GROUPS ? w.item : w.item + int(gridDim.x));
+      }
+      const int slot = w.ktc & 1;
+      if (prefixes) {
+        // (Every tile passes here, with dropped keys or not: this warp is then neither a phase of a slot behind nor two ahead.)
+        ok = mbar_wait_warp(bar(FSmem::kv_full + slot), (w.ktc >> 1) & 1, abort_flag);
+        if (!ok) break;
+        if (item_kept < uint32_t(min(P.cols, (kt + 1) * kTile))) {
+          for (int key = lane; key < kTile; key += 32)
+            if (kt * kTile + key >= int(item_kept)) clear_key(slot, key);
+          fence_proxy_async_smem();
+        }
+        mbar_arrive_warp(bar(FSmem::kv_ready + slot));
+      }
       if (has_mask) {
-        const int slot = w.ktc & 1;
         uint32_t kept[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) kept[i] = __ballot_sync(0xffffffffu, bytes[i] != 0);
@@ -1293,30 +1336,26 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
           // Dropped keys and values must not reach a product (0 * inf): their rows are cleared.
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            if (((kept[i] >> lane) & 1u) != 0) continue;
-            const uint32_t at = slot * kBigTile + (i * 32 + lane) * 64;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              sts_v4_at(smem_base + FSmem::k + at + c * 16, make_uint4(0, 0, 0, 0));
-              sts_v4_at(smem_base + FSmem::v + at + c * 16, make_uint4(0, 0, 0, 0));
-            }
+            if (((kept[i] >> lane) & 1u) == 0) clear_key(slot, i * 32 + lane);
           }
           fence_proxy_async_smem();
         }
         mbar_arrive_warp(bar(FSmem::kv_ready + slot));
       }
-      // The tiles of the first part, then a tile of the next part for every key tile of this one.
-      FWalk<GROUPS> ahead = w;
-      ahead.kt = P.k_tiles - 1;
-      ahead.next_tile();
-      const bool there = !ahead.done() && kt < ahead.nq;
-      if (there && kt == 0 && ahead.part >= 2) ok = mbar_wait_warp(bar(FSmem::stat_free + (ahead.part & 1)), ((ahead.part >> 1) - 1) & 1, abort_flag);
-      if (!ok) break;
-#pragma unroll 1
-      for (int n = w.ktc == 0 ? -w.nq : 0; n < (there ? 1 : 0); ++n) {
-        const bool own = n < 0;
-        tile_stats(own ? 0 : ahead.part, own ? w.item : ahead.item, own ? w.first : ahead.first, own ? w.nq + n : kt);
+      // The query tiles of the first part, then one of the next part for every key tile of this one (the rest by the last, where keys have
+      // fewer tiles): a key tile late, so that a tile with dropped keys does not wait for the table to be free.
+      auto ahead = last;
+      int from = 1, to = w.nq;
+      if (w.ktc > 0) {
+        ahead.kt = k_tiles - 1;
+        ahead.next_tile();
+        if (ahead.done()) continue;
+        from = last.kt;
+        to = last.kt == k_tiles - 1 ? ahead.nq : min(last.kt + 1, ahead.nq);
       }
+      const bool dead = prefixes && __shfl_sync(0xffffffffu, ahead.part == w.part ? item_kept : next_kept, 0) == 0;
+#pragma unroll 1
+      for (int qi = from; qi < to && ok; ++qi) tile_stats(ahead.part, ahead.item, ahead.first, qi, dead, qi == 0 && ahead.part >= 2);
     }
   } else if (warp < 16) {
     const int wg = warp >> 2;  // 32 of the step's 128 keys
@@ -1344,9 +1383,16 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       tmem_loaded(acc);
       tc_fence_before_sync();
       mbar_arrive_warp(bar(FSmem::dkv_free));
+      const bool wanted = wg == 0 ? P.write_dk != 0 : P.write_dv != 0;
+      if (PREFIX && !GROUPS && wanted && kt == k_tiles - 1) {  // keys that no row of the call keeps
+        const oops_ta_pair& o = wg == 0 ? P.dk : P.dv;
+        uint32_t none[32];
+#pragma unroll
+        for (int n = 0; n < 32; ++n) none[n] = 0u;
+        for (int key = k_tiles * kTile + t; key < P.cols; key += kTile) store_row32<T>(item_row(o, item) + int64_t(key) * o.sc, none, 1.f, pair_vec_ok(o));
+      }
       const int key = kt * kTile + t;
       if (key >= P.cols) return;
-      const bool wanted = wg == 0 ? P.write_dk != 0 : P.write_dv != 0;
       if (!wanted) return;
       if (has_mask && ((lds_u32_at(smem_base + FSmem::kept + (tile & 3) * 16 + (t >> 5) * 4) >> lane) & 1u) == 0) {
 #pragma unroll
@@ -1387,7 +1433,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       tc_fence_before_sync();
       mbar_arrive_warp(bar(FSmem::dq_free));
     };
-    FWalk<GROUPS> w(P);
+    FWalk<GROUPS> w(P, k_tiles);
     uint32_t bits = 0xffffffffu;  // kept keys among this warpgroup's 32
     bool ok = true;
     if (GROUPS && sm_id >= uint32_t(kFSlots)) {  // no scratch slot for this SM id: give up like a wait that ran out
@@ -1557,7 +1603,11 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
           const bool wanted = which == 0 ? P.write_dk != 0 : P.write_dv != 0;
           if (!wanted) continue;
           const float4* slot = reinterpret_cast<const float4*>(P.slots) + (int64_t(sm_id) * 2 + which) * 8 * P.slot_keys + key;
-          const float4 lo = ldcg_f4(slot + (2 * j) * P.slot_keys), hi = ldcg_f4(slot + (2 * j + 1) * P.slot_keys);
+          float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+          if (!PREFIX || key < k_tiles * kTile) {  // (behind them the slot holds what another row has left)
+            lo = ldcg_f4(slot + (2 * j) * P.slot_keys);
+            hi = ldcg_f4(slot + (2 * j + 1) * P.slot_keys);
+          }
           const float f = which == 0 ? scale : 1.f;
           const oops_ta_pair& o = which == 0 ? P.dk : P.dv;
           T* dst = item_row(o, int(blockIdx.x)) + int64_t(key) * o.sc + j * 8;
@@ -1593,32 +1643,15 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   if (device_failed()) return;
-  if (tid == 0) {
-    *abort_flag = 0;
-    for (int i = 0; i < 3; ++i) {
-      mbar_init(bar(FSmem::qd_full + i), 1);
-      mbar_init(bar(FSmem::qd_empty + i), 1);
+  if (warp == 0) {  // a lane each: one thread took half a microsecond for them
+    for (int i = lane; i < FSmem::num_bars; i += 32) {
+      int arrivals = 1;
+      if (i == FSmem::bias_empty || i == FSmem::sd_free || i == FSmem::dq_free) arrivals = 16;
+      if (i == FSmem::pds_full || i == FSmem::pds_full + 1 || i == FSmem::stat_free || i == FSmem::stat_free + 1) arrivals = 16;
+      if (i == FSmem::dkv_free) arrivals = 8;
+      mbar_init(bar(i), arrivals);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(FSmem::pds_full + i), 16);
-      mbar_init(bar(FSmem::pds_done + i), 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(FSmem::kv_full + i), 1);
-      mbar_init(bar(FSmem::kv_empty + i), 1);
-    }
-    mbar_init(bar(FSmem::p_done), 1);
-    mbar_init(bar(FSmem::bias_full), 1);
-    mbar_init(bar(FSmem::bias_empty), 16);
-    mbar_init(bar(FSmem::sd_full), 1);
-    mbar_init(bar(FSmem::sd_free), 16);
-    mbar_init(bar(FSmem::dkv_free), 8);
-    mbar_init(bar(FSmem::dq_free), 16);
-    for (int i = 0; i < 2 * kFMaxQTiles; ++i) mbar_init(bar(FSmem::stat_full + i), 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(FSmem::stat_free + i), 16);
-      mbar_init(bar(FSmem::kv_ready + i), 1);
-    }
+    if (lane == 0) *abort_flag = 0;
     fence_barrier_init();
   }
   if (warp == kFScoreWarp) {
@@ -1631,10 +1664,35 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
   const uint32_t tmem_base = *tmem_slot;
   bool plain = !MASKED;
   if (MASKED && P.mask && (P.cols % kTile == 0 || P.closed)) plain = keeps_all(P.live, P.batch * P.rows, lane);
-  if (plain)
-    fused_walk<T, HAS_BIAS, GROUPS, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane);
-  else if (MASKED)
-    fused_walk<T, HAS_BIAS, GROUPS, true>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane);
+  if (plain) {
+    fused_walk<T, HAS_BIAS, GROUPS, false, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, P.k_tiles);
+  } else if constexpr (MASKED) {
+    uint32_t most = 0;
+    const bool uniform = HAS_BIAS && P.uniform && uniform_prefix(P.uniform, P.batch, lane, most);
+    if (GROUPS && uniform && *reinterpret_cast<const volatile uint32_t*>(P.prefix + blockIdx.x / uint32_t(P.heads)) == 0) {
+      // The CTA's one row keeps no key: zeros.
+      const int row = int(blockIdx.x) / P.heads, b = row / P.rows, r = row - b * P.rows, h = int(blockIdx.x) - row * P.heads;
+      auto zeros = [&](const oops_ta_pair& t) {
+        T* to = reinterpret_cast<T*>(t.ptr) + b * t.sb + int64_t(r) * t.sr + int64_t(h) * t.sh;
+        const bool words = pair_vec_ok(t);
+        for (int at = tid; at < P.cols * 4; at += kFThreads) {
+          T* dst = to + int64_t(at >> 2) * t.sc + (at & 3) * 8;
+          if (words) {
+            *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+          } else {
+            for (int c = 0; c < 8; ++c) dst[c] = T(0.f);
+          }
+        }
+      };
+      if (P.write_dq) zeros(P.dq);
+      if (P.write_dk) zeros(P.dk);
+      if (P.write_dv) zeros(P.dv);
+    } else if (uniform)
+      fused_walk<T, HAS_BIAS, GROUPS, false, HAS_BIAS>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane,
+                                                       __shfl_sync(0xffffffffu, max(1, int(most + kTile - 1) / kTile), 0));
+    else
+      fused_walk<T, HAS_BIAS, GROUPS, true, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, P.k_tiles);
+  }
   teardown(abort_flag, tmem_base, kFScoreWarp);
 }
 
@@ -2096,11 +2154,18 @@ bool fused_applies(const oops_ta_problem& p, const oops_ta_grads& g) {
   return g.dq.ptr != nullptr && (g.dk.ptr != nullptr || g.dv.ptr != nullptr);
 }
 
+// Rows from which a mask is asked whether its rows all keep the same first keys, or none (94 % of the tokens kept: 256 columns 125 -> 121 us and a copy of
+// 3 us, 384 187 -> 177 + 4, 700 1050 -> 959 + 7, 1024 3085 -> 2980 + 8; 80 %: 512 385 -> 358 + 5, 768 1202 -> 947 + 11, 1400 7855 -> 5914 + 15).
+constexpr int kUniformCols = 192;
+
 // Whether the single-pass kernel gets a bias that is closed behind a ragged row's end (300 columns 134 -> 124 us, 500 347 -> 328, 700 962 -> 912; the
 // copy 3 to 5).
 bool closes_bias(const oops_ta_problem& p, const oops_ta_grads& g) {
-  return fused_applies(p, g) && p.bias_groups == 1 && p.cols % kTile != 0 && p.cols >= 192 && p.rows >= 64;
+  return fused_applies(p, g) && p.bias_groups == 1 && (p.cols % kTile != 0 ? p.cols >= 192 : p.mask && p.cols >= kUniformCols) && p.rows >= 64;
 }
+
+// What it takes behind the rest of the scratch: a word per sample, the bias.
+uint64_t closing_bytes(const oops_ta_problem& p) { return align256(uint64_t(p.batch) * 4) + closed_bias_bytes(p); }
 
 struct Layout {
   uint64_t delta, live, bias_t, pair_parts, parts, total;
@@ -2187,9 +2252,15 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
     if (!status) status = encode_pair(&P.map_dout, p, dout, kTile, "upstream gradient");
     if (!status) status = encode_pair(&P.map_k, p, p.k, kTile, "key");
     if (!status) status = encode_pair(&P.map_v, p, p.v, kTile, "value");
-    P.closed = closes_bias(p, g) && p.workspace_bytes >= layout.closed + closed_bias_bytes(p) && ((reinterpret_cast<uintptr_t>(base) + layout.closed) & 15) == 0;
-    if (!status && P.closed)
-      status = close_bias(&P.map_bias, p, base + layout.closed, "bias", stream);
+    P.closed = closes_bias(p, g) && p.workspace_bytes >= layout.closed + closing_bytes(p) && ((reinterpret_cast<uintptr_t>(base) + layout.closed) & 15) == 0;
+    if (!status && P.closed) {
+      if (live && p.batch <= kUniformSamples && p.cols >= kUniformCols) {
+        P.prefix = live + 2 * int64_t(p.batch) * p.rows;
+        P.uniform = reinterpret_cast<uint32_t*>(base + layout.closed);
+      }
+      status = close_bias(&P.map_bias, p, base + layout.closed + align256(uint64_t(p.batch) * 4), "bias", stream, P.prefix,
+                          const_cast<uint32_t*>(P.uniform));
+    }
     else if (!status && has_bias)
       status = encode_bias(&P.map_bias, p, p.bias, p.bias_sq, p.bias_sh, p.bias_sg, p.bias_sb, kTile, "bias");
     if (status) return status;
@@ -2404,7 +2475,7 @@ bool tensor_backward_applies(const oops_ta_problem& p, const oops_ta_grads* g) {
 
 uint64_t tensor_backward_workspace(const oops_ta_problem& p, const oops_ta_grads& g) {
   const Layout layout = workspace_layout(p, g);
-  return closes_bias(p, g) ? layout.closed + closed_bias_bytes(p) : layout.total;
+  return closes_bias(p, g) ? layout.closed + closing_bytes(p) : layout.total;
 }
 
 int tensor_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_ta_pair& dout, const float* lse,

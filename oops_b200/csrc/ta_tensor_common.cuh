@@ -133,10 +133,21 @@ int encode_bias(CUtensorMap* map, const oops_ta_problem& p, const void* ptr, int
 int closed_row(const oops_ta_problem& p) { return int(ceil_div(p.cols, kTile)) * kTile; }
 uint64_t closed_bias_bytes(const oops_ta_problem& p) { return uint64_t(p.batch) * p.heads * p.cols * closed_row(p) * 2; }
 
-int close_bias(CUtensorMap* map, const oops_ta_problem& p, void* scratch, const char* what, cudaStream_t stream) {
+int close_bias(CUtensorMap* map, const oops_ta_problem& p, void* scratch, const char* what, cudaStream_t stream, const uint32_t* prefix = nullptr,
+               uint32_t* uniform = nullptr, bool early = false) {
   const int64_t strides[5] = {p.bias_sb, p.bias_sg, p.bias_sh, p.bias_sq, p.bias_sk}, row = closed_row(p), plane = p.cols * row;
-  const int status = bias_rows(p.batch, 1, p.heads, p.cols, p.bias, strides, scratch, stream, int(row), p.dtype == OOPS_TA_BF16 ? 0xff80 : 0xfc00);
+  const int status = closed_bias(p.batch, p.heads, p.cols, p.bias, strides, scratch, int(row), p.dtype == OOPS_TA_BF16 ? 0xff80 : 0xfc00, prefix,
+                                 p.rows, uniform, early, stream);
   return status ? status : encode_bias(map, p, scratch, row, plane, plane * p.heads, plane * p.heads, kTile, what, int(row));
+}
+
+// A mask whose rows may all keep the same first keys (or none), as masks of tokens do: whether they do is found out on the device, and the bias is
+// closed behind those keys.  `uniform` has a word per sample.
+constexpr int kUniformSamples = 32;
+__device__ __forceinline__ bool uniform_prefix(const uint32_t* uniform, int batch, int lane, uint32_t& most) {
+  const uint32_t v = lane < batch ? *reinterpret_cast<const volatile uint32_t*>(uniform + lane) : 0u;
+  most = __reduce_max_sync(0xffffffffu, v);
+  return most != ~0u;
 }
 
 int sm_count() {

@@ -1,6 +1,6 @@
 """Statistics warp of the single-pass reverse kernel: rows whose dots it makes itself (above 512 columns, one group of query tiles) and rows
 whose dots a launch of their own makes, several items per CTA, ragged ends, outputs off 16-byte words, masks (prefixes, scattered keys,
-rows without a kept key) over dropped keys and values that are not finite.  16-bit bounds as in the parity tests: 2e-2 of the largest value
+the same keys in all rows that keep any, none) over dropped keys and values that are not finite.  16-bit bounds as in the parity tests: 2e-2 of the largest value
 (at least 1); gradients of dropped keys and values are exactly zero."""
 
 import pytest
@@ -17,18 +17,24 @@ def _close(name, got, ref):
     assert error <= 2e-2 * max(1.0, float(ref.abs().max())), (name, error)
 
 
-@pytest.mark.parametrize("kind", ["none", "prefix", "scattered"])
-@pytest.mark.parametrize("dtype,rows,n,heads", [(torch.bfloat16, 80, 129, 4), (torch.float16, 80, 256, 4), (torch.bfloat16, 42, 513, 4),
-                                                (torch.float16, 160, 600, 1), (torch.bfloat16, 40, 768, 4), (torch.bfloat16, 6, 800, 2)])
-def test_gradients(cuda, kind, dtype, rows, n, heads):
+@pytest.mark.parametrize("kind", ["none", "prefix", "scattered", "tokens", "empty"])
+@pytest.mark.parametrize("dtype,batch,rows,n,heads", [(torch.bfloat16, 1, 80, 129, 4), (torch.float16, 2, 80, 256, 2), (torch.bfloat16, 1, 64, 513, 3),
+                                                      (torch.float16, 3, 64, 200, 1), (torch.bfloat16, 1, 64, 768, 3), (torch.bfloat16, 1, 64, 800, 1)])
+def test_gradients(cuda, kind, dtype, batch, rows, n, heads):
     gen = torch.Generator().manual_seed(n)
-    q, k, v, up = (torch.randn(1, rows, n, heads, 32, generator=gen).to(dtype) for _ in range(4))
-    bias = torch.randn(1, 1, heads, n, n, generator=gen).to(dtype)
+    q, k, v, up = (torch.randn(batch, rows, n, heads, 32, generator=gen).to(dtype) for _ in range(4))
+    bias = torch.randn(batch, 1, heads, n, n, generator=gen).to(dtype)
     mask = None
     if kind == "prefix":
-        mask = torch.arange(n)[None, None] < torch.randint(-n // 8, n + 1, (1, rows, 1), generator=gen)
+        mask = torch.arange(n) < torch.randint(-n // 8, n + 1, (batch, rows, 1), generator=gen)
     elif kind == "scattered":
-        mask = torch.rand(1, rows, n, generator=gen) < 0.7
+        mask = torch.rand(batch, rows, n, generator=gen) < 0.7
+    elif kind == "tokens":  # every row of a sample that keeps a key keeps the same ones; whole key tiles are dropped
+        ends = torch.tensor([n - n // 3, n // 2, n])[:batch, None, None]
+        live = (torch.arange(rows) < rows - rows // 5) & (torch.arange(rows) != 3)
+        mask = (torch.arange(n) < ends) & live[None, :, None]
+    elif kind == "empty":
+        mask = torch.zeros(batch, rows, n, dtype=torch.bool)
     want = oracle.forward_backward(q, k, v, mask, bias, up)
     if mask is not None:
         dead = ~mask[..., None, None]
