@@ -151,10 +151,11 @@ int oops_ta_uses_tensor_path(const oops_ta_problem* problem, int backward);
    `result`.  Host only; pointers are not dereferenced. */
 int oops_ta_uses_wide_path(const oops_ta_problem* problem, const oops_ta_pair* result, const oops_ta_grads* grads);
 
-/* Scratch bytes oops_ta_forward needs for this problem (may be 0). */
+/* Scratch bytes oops_ta_forward uses for this problem (may be 0).  A tcgen05 problem is served without them too, more slowly. */
 uint64_t oops_ta_forward_workspace_bytes(const oops_ta_problem* problem);
 
-/* Scratch bytes oops_ta_backward needs for this problem and gradient request. */
+/* Scratch bytes oops_ta_backward uses for this problem and gradient request.  The closed copy of a row-shared bias at their end (heads * cols
+   * cols elements, rounded up to whole tiles of 128 keys, and a word per sample) is done without where there is no room for it. */
 uint64_t oops_ta_backward_workspace_bytes(const oops_ta_problem* problem, const oops_ta_grads* grads);
 
 /*

@@ -124,10 +124,6 @@ __device__ __forceinline__ uint32_t ldg_u8_here(const uint8_t* p) {
   return v;
 }
 
-// ---- dependent launches ------------------------------------------------------------------------
-__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_for_predecessors() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // Four f32 added to global memory without a return value (performed at the L2; nothing to wait for).
 __device__ __forceinline__ void red_add_f4(float4* p, float a, float b, float c, float d) {
   asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");

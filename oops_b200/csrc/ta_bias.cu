@@ -5,7 +5,6 @@
 // writes one word of eight keys.  Neighbouring threads then take the heads of the same cells where the heads are the
 // neighbours in memory, so that a warp's reads share their sectors, and the next words of the row otherwise.
 // N = 100, 4 heads: 3.9 -> 2.1 us and one launch less; attention of N = 499 with a projected bias: 260 -> 244 us.
-#include "sm100_ptx.cuh"
 #include "ta_internal.h"
 
 namespace oops_ta {
@@ -56,45 +55,17 @@ __global__ void __launch_bounds__(256) bias_rows_kernel(const BiasRows p) {
   reinterpret_cast<uint4*>(p.dst)[row * p.words + word] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
 }
 
-// How many keys a row of the mask keeps if they are its first ones, else ~0: a warp a row.
-__global__ void __launch_bounds__(256) mask_prefix_kernel(const uint8_t* mask, int64_t m_sb, int64_t m_sr, int64_t m_sc, int rows, int cols,
-                                                          int num_rows, uint32_t* prefix) {
-  ptx::launch_dependents();
-  const int row = int(blockIdx.x) * 8 + int(threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (row >= num_rows) return;
-  const uint8_t* bytes = mask + row / rows * m_sb + int64_t(row % rows) * m_sr;
-  int count = 0, end = 0;
-  constexpr int kBatch = 16;  // words of 32 keys whose bytes travel together
-  for (int first = 0; first < cols; first += kBatch * 32) {
-    uint32_t kept[kBatch];
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      const int key = first + i * 32 + lane;
-      kept[i] = key < cols ? ptx::ldg_u8_here(bytes + int64_t(key) * m_sc) : 0u;
-    }
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      kept[i] = __ballot_sync(0xffffffffu, kept[i] != 0);
-      count += __popc(kept[i]);
-      if (kept[i] != 0) end = first + i * 32 + 32 - __clz(int(kept[i]));
-    }
-  }
-  if (lane == 0) prefix[row] = count == end ? uint32_t(count) : ~0u;
-}
-
 // A row-shared bias (batch, head, query, key) in rows of `words` 16-byte words whose keys from an end on are minus infinity: the row's, or,
 // where all rows of a sample that keep a key keep the same first ones, the end of those, which uniform[sample] then has (~0 where they do not;
 // 0: no row keeps a key).  One launch for all samples; every CTA looks at all of its sample's rows (L2).
 __global__ void __launch_bounds__(256) closed_bias_kernel(const BiasRows p, const uint32_t* prefix, int rows, uint32_t* uniform) {
-  ptx::launch_dependents();
   __shared__ uint32_t low[8], high[8];
   const uint32_t b = blockIdx.y;
   uint32_t end = p.cols;
   if (prefix) {
-    ptx::wait_for_predecessors();
     uint32_t lo = ~0u, hi = 0u;
     for (int r = threadIdx.x; r < rows; r += 256) {
-      const uint32_t v = *reinterpret_cast<const volatile uint32_t*>(prefix + int64_t(b) * rows + r);
+      const uint32_t v = prefix[int64_t(b) * rows + r];
       if (v != 0) lo = min(lo, v);
       hi = max(hi, v);
     }
@@ -160,40 +131,16 @@ BiasRows describe_rows(int batch, int groups, int heads, int cols, const void* s
   return p;
 }
 
-// A launch that may begin before the one ahead of it in the stream has ended.
-template <typename... Params, typename... Args>
-int launch_early(void (*kernel)(Params...), dim3 grid, cudaStream_t stream, const char* what, Args... args) {
-  cudaLaunchConfig_t config{};
-  config.gridDim = grid;
-  config.blockDim = dim3(256);
-  config.stream = stream;
-  cudaLaunchAttribute attribute{};
-  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute.val.programmaticStreamSerializationAllowed = 1;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
-  cudaLaunchKernelEx(&config, kernel, Params(args)...);
-  count_launch();
-  return check_launch(what);
-}
-
 }  // namespace
 
-int mask_prefixes(const uint8_t* mask, int64_t m_sb, int64_t m_sr, int64_t m_sc, int batch, int rows, int cols, uint32_t* prefix, cudaStream_t stream) {
-  mask_prefix_kernel<<<(unsigned)ceil_div(int64_t(batch) * rows, 8), 256, 0, stream>>>(mask, m_sb, m_sr, m_sc, rows, cols, batch * rows, prefix);
-  count_launch();
-  return check_launch("mask prefixes");
-}
-
 int closed_bias(int batch, int heads, int cols, const void* src, const int64_t strides[5], void* dst, int row, uint16_t fill, const uint32_t* prefix,
-                int rows, uint32_t* uniform, bool early, cudaStream_t stream) {
+                int rows, uint32_t* uniform, cudaStream_t stream) {
   BiasRows p = describe_rows(batch, 1, heads, cols, src, strides, dst, ceil_div(row, 8), fill);
   const int64_t total = int64_t(heads) * cols * p.words;  // of a sample
   if (total == 0 || batch == 0) return OOPS_TA_OK;
   if (total > 0xffffff00ll || batch > 65535) return fail(OOPS_TA_LIMIT_EXCEEDED, "bias of %lld words in %d samples", (long long)total, batch);
   p.total = uint64_t(total);
   const dim3 grid((unsigned)ceil_div(total, 256), (unsigned)batch);
-  if (early) return launch_early(closed_bias_kernel, grid, stream, "closed bias", p, prefix, rows, uniform);
   closed_bias_kernel<<<grid, 256, 0, stream>>>(p, prefix, rows, uniform);
   count_launch();
   return check_launch("closed bias");

@@ -87,13 +87,11 @@ int packed_pair_mask(const uint8_t* tokens, const int64_t* token_offsets, int sa
 int packed_pair_mask_max_samples();
 // 16-bit bias of any strides (batch, group, head, query, key) to contiguous rows of ceil(cols / 8) 16-byte words.
 int bias_rows(int batch, int groups, int heads, int cols, const void* src, const int64_t strides[5], void* dst, cudaStream_t stream);
-// Kept keys of every mask row where they are its first ones, else ~0.
-int mask_prefixes(const uint8_t* mask, int64_t m_sb, int64_t m_sr, int64_t m_sc, int batch, int rows, int cols, uint32_t* prefix, cudaStream_t stream);
 // A row-shared bias in rows of `row` elements (a multiple of 8) that hold `fill` behind the last key, or, where `prefix` is given and all rows of a
-// sample that keep a key keep the same first ones, behind the last of those; uniform[sample] is their number then, else ~0 (0: none keeps any).
-// `early`: may begin under the end of the launch before.
+// sample that keep a key keep the same first ones, behind the last of those; uniform[sample] is their number then, else ~0 (0: none keeps any).  `prefix`: kept keys of every
+// mask row where they are its first ones, else ~0.
 int closed_bias(int batch, int heads, int cols, const void* src, const int64_t strides[5], void* dst, int row, uint16_t fill, const uint32_t* prefix,
-                int rows, uint32_t* uniform, bool early, cudaStream_t stream);
+                int rows, uint32_t* uniform, cudaStream_t stream);
 // Layer normalisation over the last axis of (rows, width) activations (row strides in elements, contiguous rows);
 // weight / bias / gradients of them may be NULL; affine_dtype is the activation dtype or f32.
 uint64_t layer_norm_backward_workspace_bytes(int64_t rows, int width);

@@ -91,6 +91,8 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   return rank;
 }
 // The next launch may set itself up beside this one; it waits, as this one does, for the end of all before it where it first reads or writes memory.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_predecessors() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void named_barrier_arrive(uint32_t id, uint32_t threads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }

@@ -995,9 +995,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) ta_bwd_dkv_kernel(const 
 // A statistics warp of its own puts -log2(e) lse and -delta of a part's queries into a table, a tile at a time and a part ahead, where every
 // thread used to fetch both for every step (N = 768: 1036 -> 1004 us, 1024: 2934 -> 2842, 2048: 22.7 -> 22.0 ms), and makes the row dots where
 // that is hidden (kOwnDeltaCols).  With a mask it also clears the rows of dropped keys and values in shared memory before any
-// product may read them; the element-wise warps give dropped keys a bias of minus infinity (their words are in registers) instead of
-// testing every probability in a second copy of the step's body (N = 384, 360 kept: 187 -> 179 us; 512: 378 -> 357), and the read-out
-// of a key tile stores zeros for them.
+// product may read them.  Where all rows of a sample keep the same first keys (kUniformCols) the bias is minus infinity behind those, key tiles
+// behind them are not walked, and the element-wise warps know of no mask; otherwise they give dropped keys a bias of minus infinity
+// (its words are in registers) instead of testing every probability in a second copy of the step's body, and the read-out of a key
+// tile stores zeros for them.  Rows of up to 190 columns, a tile or two, take 1 to 3 us longer for the warp in their chain (64: 10.7 -> 11.8).
 // Halving the step between two sets of warps that run half a step apart was tried: the single P image couples them, 3 to 10 %
 // slower.
 // Rows of more than 768 columns have several groups.  The CTA walks them in order and carries the f32 sums of dK and
@@ -2154,14 +2155,15 @@ bool fused_applies(const oops_ta_problem& p, const oops_ta_grads& g) {
   return g.dq.ptr != nullptr && (g.dk.ptr != nullptr || g.dv.ptr != nullptr);
 }
 
-// Rows from which a mask is asked whether its rows all keep the same first keys, or none (94 % of the tokens kept: 256 columns 125 -> 121 us and a copy of
-// 3 us, 384 187 -> 177 + 4, 700 1050 -> 959 + 7, 1024 3085 -> 2980 + 8; 80 %: 512 385 -> 358 + 5, 768 1202 -> 947 + 11, 1400 7855 -> 5914 + 15).
+// Rows from which a mask is asked whether its rows all keep the same first keys, or none (94 % of the tokens kept: 256 columns, two samples 124 -> 114 us and
+// a copy of 3, 200, two samples 90 -> 88 + 3, 384 187 -> 174 + 4, 512 379 -> 348 + 4, 1000 3171 -> 2748 + 12; 80 %: 768 1202 -> 980 + 11, 1000 3204 -> 2101 + 12,
+// 1400 7855 -> 4849 + 16).
 constexpr int kUniformCols = 192;
 
 // Whether the single-pass kernel gets a bias that is closed behind a ragged row's end (300 columns 134 -> 124 us, 500 347 -> 328, 700 962 -> 912; the
 // copy 3 to 5).
 bool closes_bias(const oops_ta_problem& p, const oops_ta_grads& g) {
-  return fused_applies(p, g) && p.bias_groups == 1 && (p.cols % kTile != 0 ? p.cols >= 192 : p.mask && p.cols >= kUniformCols) && p.rows >= 64;
+  return fused_applies(p, g) && bias_closes(p) && (p.cols % kTile != 0 ? p.cols >= 192 : p.mask && p.cols >= kUniformCols) && p.rows >= 64;
 }
 
 // What it takes behind the rest of the scratch: a word per sample, the bias.

@@ -131,13 +131,17 @@ int encode_bias(CUtensorMap* map, const oops_ta_problem& p, const void* ptr, int
 // A row-shared bias in rows of whole key tiles whose padding is minus infinity, in a call's scratch: keys behind the end of a ragged row then
 // have no probability without being told apart (their operands are the zeros of the copies), and the kernels take the walks without tests.
 int closed_row(const oops_ta_problem& p) { return int(ceil_div(p.cols, kTile)) * kTile; }
+// (the copy's launch counts a sample's words in 32 bits and has the samples on a grid axis)
+bool bias_closes(const oops_ta_problem& p) {
+  return p.bias_groups == 1 && p.batch <= 65535 && int64_t(p.heads) * p.cols * (closed_row(p) / 8) <= 0x7fffffffll;
+}
 uint64_t closed_bias_bytes(const oops_ta_problem& p) { return uint64_t(p.batch) * p.heads * p.cols * closed_row(p) * 2; }
 
 int close_bias(CUtensorMap* map, const oops_ta_problem& p, void* scratch, const char* what, cudaStream_t stream, const uint32_t* prefix = nullptr,
-               uint32_t* uniform = nullptr, bool early = false) {
+               uint32_t* uniform = nullptr) {
   const int64_t strides[5] = {p.bias_sb, p.bias_sg, p.bias_sh, p.bias_sq, p.bias_sk}, row = closed_row(p), plane = p.cols * row;
   const int status = closed_bias(p.batch, p.heads, p.cols, p.bias, strides, scratch, int(row), p.dtype == OOPS_TA_BF16 ? 0xff80 : 0xfc00, prefix,
-                                 p.rows, uniform, early, stream);
+                                 p.rows, uniform, stream);
   return status ? status : encode_bias(map, p, scratch, row, plane, plane * p.heads, plane * p.heads, kTile, what, int(row));
 }
 

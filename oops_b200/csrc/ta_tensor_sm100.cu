@@ -9,13 +9,19 @@
 //
 // The softmax has no row maximum in its steady state.  The maximum of a row's first step is its reference (that probability
 // is then 1, which 16 bits hold exactly; a reference from fewer columns left every large one rounded, and short rows 2 to 5 %
-// further from the exact result); later steps take 2^(x - reference) as they come, 16 columns at a time, and look at the step's sum only: a
-// sum of 2^10 or more (or a NaN) sends the warp back over the step, which still stands in tensor memory, to raise the
-// reference and rescale the accumulators.  Probabilities therefore stay below 2^10, inside the f32, bf16 and f16 ranges.
+// further from the exact result); later steps take 2^(x - reference) as they come, 16 columns at a time, and look at their sum only: 2^10
+// or more in the first 48 columns (or a NaN), or a logit of 10 or more in the last 16, sends the warp back over the step, which still
+// stands in tensor memory, to raise the reference and rescale the accumulators.  Probabilities therefore stay below 2^10, inside the
+// f32, bf16 and f16 ranges.  With that look the scores are given back before the exponentials of the last 16 columns, and the next
+// score product runs under them (N = 768: 711 -> 681 us, 512: 233 -> 225, 2048: 11.6 -> 11.2 ms; no bit of a result changed).
 // Against a maximum per step this saves the comparisons, and above all the wait: no exponential depended on the last
 // score of a step any more, scores need not be held in registers, and an exponential costs 5 instead of 9.5 issue slots.
-// What bounds it: the element-wise warps' streams, with issue slots (57 %) and the special-function unit (59 %; one ex2 per
-// score at 16 per clock and SM, 0.40 of the 0.73 ms at N = 768) the busiest units.  Hence no tests on kept bits where nothing is dropped: a CTA whose rows keep every key walks a copy
+// What bounds it: the element-wise warps' streams, with the special-function unit (63 %; one ex2 per score at 16 per clock and SM,
+// 0.39 of the 0.68 ms at N = 768) and issue slots (60 %) the busiest units.  Eight softmax warps of an SM alone reach 70 to 80 % of what
+// sixteen do.  Without a bias the kernel takes 0.57 ms; giving the bias another way did not help: as f32 blocks that tcgen05.cp copies
+// into the score accumulators 0.74 ms (a copy of 4 KB holds the tensor queue for some hundred clocks), as f32 in shared memory 0.69;
+// nor did exponentials on the FMA pipe (1/8: 0.71, 1/4: 0.74) or logits computed between the exponentials of the columns before
+// (0.69).  Hence no tests on kept bits where nothing is dropped: a CTA whose rows keep every key walks a copy
 // of the roles without them (N = 768: 757 -> 703 us), and otherwise the steps that every row keeps whole come first, in a
 // loop of their own (the order of the keys is free; N = 1024, 1000 kept: 1659 -> 1618 us), and a step that one of two rows
 // keeps costs the other a row of zeros (N = 1000, rows that keep alternate blocks of 64 keys: 1966 -> 1466 us).
@@ -96,8 +102,9 @@ struct FwdParams {
   int gate_vec16, plain_vec16;
 };
 
-// What sends a step's warp back for a new reference: the sum of the probabilities of the first 48 columns, or a base-2 logit of the last 16.
-constexpr float kStepSumLimit = 1024.f, kLastColumnsLimit = 6.f;
+// What sends a step's warp back for a new reference: the sum of the probabilities of the first 48 columns, or a base-2 logit of the last 16 (whose
+// probabilities are not known yet when the scores are given back).  No probability reaches 2^10 then, no step's sum 2^15.
+constexpr float kStepSumLimit = 1024.f, kLastColumnsLimit = 10.f;
 
 // Where item `idx` lies: query item fastest, then head, row (or pair of rows), batch.
 struct FwdItem {
@@ -733,7 +740,7 @@ bool tensor_forward_applies(const oops_ta_problem& p) {
 
 // A ragged last step costs a call of 1000 columns 4.5 % (1565 us, 1024: 1530), one of 500 5 %; the copy 3 to 6 us.
 uint64_t tensor_forward_workspace(const oops_ta_problem& p) {
-  return p.bias_groups == 1 && p.cols % kKeys != 0 && p.cols >= 384 && p.cols <= 4096 && p.rows >= 128 ? closed_bias_bytes(p) : 0;
+  return bias_closes(p) && p.cols % kKeys != 0 && p.cols >= 384 && p.cols <= 4096 && p.rows >= 128 ? closed_bias_bytes(p) : 0;
 }
 
 namespace {
