@@ -994,11 +994,11 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) ta_bwd_dkv_kernel(const 
 // issuer that acquires it fences once for all of them before its products read (N = 768: 1190 -> 1120 us with both).
 // A statistics warp of its own puts -log2(e) lse and -delta of a part's queries into a table, a tile at a time and a part ahead, where every
 // thread used to fetch both for every step (N = 768: 1036 -> 1004 us, 1024: 2934 -> 2842, 2048: 22.7 -> 22.0 ms), and makes the row dots where
-// that is hidden (kOwnDeltaCols).  With a mask it also clears the rows of dropped keys and values in shared memory before any
-// product may read them.  Where all rows of a sample keep the same first keys (kUniformCols) the bias is minus infinity behind those, key tiles
-// behind them are not walked, and the element-wise warps know of no mask; otherwise they give dropped keys a bias of minus infinity
-// (its words are in registers) instead of testing every probability in a second copy of the step's body, and the read-out of a key
-// tile stores zeros for them.  Rows of up to 190 columns, a tile or two, take 1 to 3 us longer for the warp in their chain (64: 10.7 -> 11.8).
+// that is hidden (kOwnDeltaCols).  Where all rows of a sample keep the same first keys
+// (kUniformCols) the bias is minus infinity behind those, key tiles behind them are not walked, the statistics warp clears dropped keys and
+// values in shared memory before any product may read them, and the element-wise warps know of no mask.  Through other masks they test
+// every probability, in a second copy of the step's body: a tile's way through the statistics warp, or bias words patched in
+// registers instead, cost short rows 10 to 20 %.
 // Halving the step between two sets of warps that run half a step apart was tried: the single P image couples them, 3 to 10 %
 // slower.
 // Rows of more than 768 columns have several groups.  The CTA walks them in order and carries the f32 sums of dK and
@@ -1027,8 +1027,7 @@ struct FSmem {
   static constexpr int dss = ps + kFImage;             // [2] dS image
   static constexpr int bias = dss + 2 * kFImage;       // one staging tile
   static constexpr int stats = bias + kFBias;          // [2][6][128] of two f32: statistics of a part's queries
-  static constexpr int kept = stats + 2 * kFMaxQTiles * kTile * 8;  // [4][4] u32: kept keys of a key tile
-  static constexpr int bars = kept + 64;
+  static constexpr int bars = stats + 2 * kFMaxQTiles * kTile * 8;
   static constexpr int qd_full = 0;                    // [3]
   static constexpr int qd_empty = qd_full + 3;         // [3]
   static constexpr int kv_full = qd_empty + 3;         // [2]
@@ -1044,7 +1043,7 @@ struct FSmem {
   static constexpr int dq_free = dkv_free + 1;         // dQ of a finished group of query tiles has been read out
   static constexpr int stat_full = dq_free + 1;        // [2][6] the statistics of a query tile stand
   static constexpr int stat_free = stat_full + 2 * kFMaxQTiles;  // [2] every warp is done with those of a part
-  static constexpr int kv_ready = stat_free + 2;       // [2] dropped keys have been cleared, and `kept` stands (masks)
+  static constexpr int kv_ready = stat_free + 2;       // [2] dropped keys have been cleared (PREFIX)
   static constexpr int num_bars = kv_ready + 2;
   static constexpr int tmem_slot = bars + num_bars * 8;
   static constexpr int abort_flag = tmem_slot + 4;
@@ -1112,7 +1111,7 @@ struct FWalk {
 
 // GROUPS: rows of several groups of query tiles.  BITS: some key may be dropped, by the mask or because the last key tile
 // is ragged.
-template <typename T, bool HAS_BIAS, bool GROUPS, bool BITS, bool PREFIX>
+template <typename T, bool HAS_BIAS, bool GROUPS, bool BITS, bool PREFIX, bool DIRECT>
 __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base, uint8_t* smem_gen, volatile int* abort_flag,
                                            uint32_t tmem_base, int tid, int warp, int lane, int k_tiles) {
   auto bar = [&](int index) -> uint32_t { return smem_base + FSmem::bars + index * 8; };
@@ -1164,7 +1163,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       for (FWalk<GROUPS> w(P, k_tiles); !w.done() && ok; w.next()) {
         const int s = w.s, qs = s % 3, ks = w.ktc & 1;
         ok = mbar_wait_warp(bar(FSmem::qd_full + qs), (s / 3) & 1, abort_flag);
-        if (ok && w.qi == 0) ok = mbar_wait_warp(bar((has_mask || prefixes ? FSmem::kv_ready : FSmem::kv_full) + ks), (w.ktc >> 1) & 1, abort_flag);
+        if (ok && w.qi == 0) ok = mbar_wait_warp(bar((PREFIX ? FSmem::kv_ready : FSmem::kv_full) + ks), (w.ktc >> 1) & 1, abort_flag);
         if (ok && s > 0) ok = mbar_wait_warp(bar(FSmem::sd_free), (s - 1) & 1, abort_flag);
         if (!ok) break;
         tc_fence_after_sync();
@@ -1221,7 +1220,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
         if (qi == w.nq - 1) mma_commit_warp(bar(FSmem::kv_empty + ks));
       }
     }
-  } else if (warp == kFStatWarp) {
+  } else if (warp == kFStatWarp && !DIRECT) {
     // Statistics of a part's queries, a tile at a time and a part ahead: -log2(e) lse, and -delta, which is rowsum(O * dO) where the
     // caller has not left it.  Four lanes share a query, eight channels each.
     bool ok = true;
@@ -1281,18 +1280,6 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       mbar_arrive_warp(bar(FSmem::stat_full + buffer * kFMaxQTiles + qi));
     };
     FWalk<GROUPS> w(P, k_tiles);
-    uint32_t bytes[4] = {0, 0, 0, 0};  // of the mask, for the key tile to come
-    auto fetch_mask = [&](const FWalk<GROUPS>& at) {
-      if (!has_mask || at.done()) return;
-      const int row = at.item / P.heads, b = row / P.rows;
-      const uint8_t* mask_row = P.mask + b * P.m_sb + int64_t(row - b * P.rows) * P.m_sr;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int key = at.kt * kTile + i * 32 + lane;
-        bytes[i] = key < P.cols ? ldg_u8_here(mask_row + int64_t(key) * P.m_sc) : 0u;
-      }
-    };
-    fetch_mask(w);
     auto clear_key = [&](int slot, int key) {
       const uint32_t at = slot * kBigTile + key * 64;
 #pragma unroll
@@ -1303,7 +1290,6 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     };
     uint32_t item_kept = 0, next_kept = request_prefix(int(blockIdx.x));
     auto last = w;  // the key tile before
-    // The first tile of all travels with the mask's first bytes.
     if (!w.done()) tile_stats(0, w.item, w.first, 0, prefixes && __shfl_sync(0xffffffffu, next_kept, 0) == 0, false);
     for (; !w.done() && ok; last = w, w.next_tile()) {
       const int kt = w.kt;
@@ -1319,26 +1305,6 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
         if (item_kept < uint32_t(min(P.cols, (kt + 1) * kTile))) {
           for (int key = lane; key < kTile; key += 32)
             if (kt * kTile + key >= int(item_kept)) clear_key(slot, key);
-          fence_proxy_async_smem();
-        }
-        mbar_arrive_warp(bar(FSmem::kv_ready + slot));
-      }
-      if (has_mask) {
-        uint32_t kept[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) kept[i] = __ballot_sync(0xffffffffu, bytes[i] != 0);
-        FWalk<GROUPS> next = w;
-        next.next_tile();
-        fetch_mask(next);
-        ok = mbar_wait_warp(bar(FSmem::kv_full + slot), (w.ktc >> 1) & 1, abort_flag);
-        if (!ok) break;
-        if (lane == 0) sts_v4_at(smem_base + FSmem::kept + (w.ktc & 3) * 16, make_uint4(kept[0], kept[1], kept[2], kept[3]));
-        if ((kept[0] & kept[1] & kept[2] & kept[3]) != 0xffffffffu) {
-          // Dropped keys and values must not reach a product (0 * inf): their rows are cleared.
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            if (((kept[i] >> lane) & 1u) == 0) clear_key(slot, i * 32 + lane);
-          }
           fence_proxy_async_smem();
         }
         mbar_arrive_warp(bar(FSmem::kv_ready + slot));
@@ -1365,6 +1331,27 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     const uint32_t lanes_t = tmem_base + lane_field;
     const float scale = P.scale;
     const f32x2 c2 = pack2(scale * kLog2e, scale * kLog2e), log2e2 = pack2(kLog2e, kLog2e);
+    // DIRECT: the statistics of this thread's query in a step's query tile, fetched one step ahead and left untouched till then.
+    auto fetch_stats = [&](const FWalk<GROUPS>& at, float& lse_raw, float& delta_raw) {
+      lse_raw = INFINITY;
+      delta_raw = 0.f;
+      const int q = at.qt() * kTile + t;
+      if (!at.done() && q < P.cols) {
+        const int64_t stat = int64_t(at.item) * P.cols + q;
+        lse_raw = ldg_f32_here(P.lse + stat);
+        delta_raw = ldg_f32_here(P.delta + stat);
+      }
+    };
+    // The kept bit of this lane's key of a key tile (32 keys of this warpgroup), fetched a key tile ahead.
+    auto mask_row_of = [&](int item) -> const uint8_t* {
+      const int row = item / P.heads, b = row / P.rows;
+      return P.mask + b * P.m_sb + int64_t(row - b * P.rows) * P.m_sr;
+    };
+    auto fetch_keep = [&](const uint8_t* row, const FWalk<GROUPS>& at) -> uint32_t {
+      const int key = at.kt * kTile + wg * 32 + lane;
+      if (at.done() || key >= P.cols) return 0;
+      return has_mask ? ldg_u8_here(row + int64_t(key) * P.m_sc) : 1u;
+    };
     const int row0 = int(blockIdx.x) / P.heads, h0 = int(blockIdx.x) - row0 * P.heads, b0 = row0 / P.rows, r0 = row0 - b0 * P.rows;
     auto item_row = [&](const oops_ta_pair& t, int item) -> T* {
       if (GROUPS) return reinterpret_cast<T*>(t.ptr) + b0 * t.sb + int64_t(r0) * t.sr + h0 * t.sh;
@@ -1376,7 +1363,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     // dK (warpgroup 0) and dV (warpgroup 1) of key tile kt, complete for the query tiles of group g: lanes are keys.
     // With several groups the f32 sums travel from group to group through this SM's scratch slot (the same thread
     // owns a key in every group), and the last group stores the 16-bit result.
-    auto store_key_tile = [&](int item, int g, int kt, int tile) {  // `tile` counts key tiles
+    auto store_key_tile = [&](int item, int g, int kt) {
       if (wg > 1) return;
       uint32_t acc[32];
       tmem_ld32(lanes_t + (wg == 0 ? kDkCol : kDvCol), acc);
@@ -1395,10 +1382,6 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       const int key = kt * kTile + t;
       if (key >= P.cols) return;
       if (!wanted) return;
-      if (has_mask && ((lds_u32_at(smem_base + FSmem::kept + (tile & 3) * 16 + (t >> 5) * 4) >> lane) & 1u) == 0) {
-#pragma unroll
-        for (int n = 0; n < 32; ++n) acc[n] = 0u;  // a dropped key, whatever the queries and the upstream gradient hold
-      }
       if (GROUPS) {
         // plane i of the slot holds channels 4i .. 4i+3 of every key, so that a warp's 32 keys are 512 contiguous bytes
         float4* slot = reinterpret_cast<float4*>(P.slots) + (int64_t(sm_id) * 2 + wg) * 8 * P.slot_keys + key;
@@ -1435,7 +1418,10 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       mbar_arrive_warp(bar(FSmem::dq_free));
     };
     FWalk<GROUPS> w(P, k_tiles);
-    uint32_t bits = 0xffffffffu;  // kept keys among this warpgroup's 32
+    float lse_next = 0.f, delta_next = 0.f;
+    if (DIRECT) fetch_stats(w, lse_next, delta_next);
+    const uint8_t* mask_row = has_mask ? mask_row_of(w.item) : nullptr;  // of the key tile to come
+    uint32_t keep_raw = has_bits ? fetch_keep(mask_row, w) : 0u, bits = 0xffffffffu;
     bool ok = true;
     if (GROUPS && sm_id >= uint32_t(kFSlots)) {  // no scratch slot for this SM id: give up like a wait that ran out
       *abort_flag = 1;
@@ -1445,26 +1431,44 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     // bias row of this thread's query in the staging tile: box (wg >> 1), 16-byte chunks (wg & 1) * 4 .. + 3
     const uint8_t* bias_row = smem_gen + FSmem::bias + (wg >> 1) * kBiasStep + t * 128 + (((t & 7) ^ ((wg & 1) * 4)) << 4);
 
-    int last_item = 0, last_part = 0, last_first = 0, last_kt = 0, last_tile = 0;  // of the previous step
-    for (; !w.done() && ok; last_item = w.item, last_part = w.part, last_first = w.first, last_kt = w.kt, last_tile = w.ktc, w.next()) {
+    int last_item = 0, last_part = 0, last_first = 0, last_kt = 0;  // of the previous step
+    for (; !w.done() && ok; last_item = w.item, last_part = w.part, last_first = w.first, last_kt = w.kt, w.next()) {
       const int s = w.s, kt = w.kt, qi = w.qi, buf = s & 1, table = (w.part & 1) * kFMaxQTiles + qi;
+      if (has_bits && qi == 0) {
+        bits = __ballot_sync(0xffffffffu, keep_raw != 0);
+        FWalk<GROUPS> ahead = w;
+        ahead.next_tile();
+        if (!GROUPS && has_mask && ahead.kt == 0 && !ahead.done()) mask_row = mask_row_of(ahead.item);
+        keep_raw = fetch_keep(mask_row, ahead);
+        if (has_mask && bits != 0xffffffffu) {
+          // Key rows of dropped keys must not reach the dQ product (0 * inf): they are cleared in shared memory, eight of
+          // this warpgroup's 32 by each warp.  The scores of these keys are dropped whatever they are.
+          ok = mbar_wait(bar(FSmem::kv_full + (w.ktc & 1)), (w.ktc >> 1) & 1, abort_flag);
+          if (!ok) break;
+          const int key = (warp & 3) * 8 + (lane >> 2);
+          if (((bits >> key) & 1u) == 0)
+            sts_v4_at(smem_base + FSmem::k + (w.ktc & 1) * kBigTile + (wg * 32 + key) * 64 + (lane & 3) * 16, make_uint4(0, 0, 0, 0));
+        }
+      }
       if (s > 0) mbar_arrive_warp(bar(FSmem::pds_full + (buf ^ 1)));  // the images of step s - 1, their stores drained by now
       // The three phases the step needs first are probed together (one round trip to the barrier words); in the steady
       // state, where these warps are the slow side of the pipeline, all three are complete.
       const bool bias_there = HAS_BIAS && mbar_test(bar(FSmem::bias_full), s & 1);
       const bool image_free = s < 2 || mbar_test(bar(FSmem::pds_done + buf), ((s >> 1) - 1) & 1);
       const bool scores_there = mbar_test(bar(FSmem::sd_full), s & 1);
-      const bool stats_there = kt > 0 || mbar_test(bar(FSmem::stat_full + table), (w.part >> 1) & 1);
-      if (has_mask && qi == 0) {
-        const bool kept_there = mbar_test(bar(FSmem::kv_ready + (w.ktc & 1)), (w.ktc >> 1) & 1);
-        ok = mbar_wait_probed(kept_there, bar(FSmem::kv_ready + (w.ktc & 1)), (w.ktc >> 1) & 1, abort_flag);
-        if (!ok) break;
-        bits = lds_u32_at(smem_base + FSmem::kept + (w.ktc & 3) * 16 + wg * 4);
-      }
-      ok = mbar_wait_probed(stats_there, bar(FSmem::stat_full + table), (w.part >> 1) & 1, abort_flag);
-      if (!ok) break;
       float neg_lse2, neg_delta;
-      lds_f2_at(smem_base + FSmem::stats + (table * kTile + t) * 8, neg_lse2, neg_delta);
+      if (DIRECT) {
+        neg_lse2 = -lse_next * kLog2e;
+        neg_delta = -delta_next;
+        FWalk<GROUPS> ahead = w;
+        ahead.next();
+        fetch_stats(ahead, lse_next, delta_next);
+      } else {
+        const bool stats_there = kt > 0 || mbar_test(bar(FSmem::stat_full + table), (w.part >> 1) & 1);
+        ok = mbar_wait_probed(stats_there, bar(FSmem::stat_full + table), (w.part >> 1) & 1, abort_flag);
+        if (!ok) break;
+        lds_f2_at(smem_base + FSmem::stats + (table * kTile + t) * 8, neg_lse2, neg_delta);
+      }
       const f32x2 nl1 = pack2(neg_lse2, neg_lse2), nd1 = pack2(neg_delta, neg_delta);
       // The step's bias words are requested at once; the staging tile is handed back as soon as they have arrived
       // (below, after the first scores have been fetched), so that the next tile's copy runs under this step's arithmetic.
@@ -1480,30 +1484,6 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       if (ok) ok = mbar_wait_probed(scores_there, bar(FSmem::sd_full), s & 1, abort_flag);
       if (!ok) break;
       tc_fence_after_sync();
-      if (has_bits && qi == 0) {
-        if (!has_mask) {
-          const int there = P.cols - kt * kTile - wg * 32;
-          bits = there >= 32 ? 0xffffffffu : there <= 0 ? 0u : (1u << there) - 1;
-        }
-        bits = __shfl_sync(0xffffffffu, bits, 0);
-      }
-      // Keys behind the row's end have zeros for operands and bias: what comes out for them is 2^nl and 2^nl nd, which nobody stores
-      // and which meet zeros in dQ, unless they leave the range of 16 bits.
-      if (HAS_BIAS && has_bits && bits != 0xffffffffu && (has_mask || __any_sync(0xffffffffu, !(neg_lse2 < 10.f && fabsf(neg_delta) < 32.f)))) {
-        // Dropped keys get a bias of minus infinity: no test in the body below.
-        constexpr uint32_t kNone = Half2<T>::kFormat == 1 ? 0xff80u : 0xfc00u;
-        auto drop = [&](uint32_t& word, int key) {
-          if (((bits >> key) & 1u) == 0) word = (word & 0xffff0000u) | kNone;
-          if (((bits >> (key + 1)) & 1u) == 0) word = (word & 0xffffu) | (kNone << 16);
-        };
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          drop(bias_words[c].x, c * 8);
-          drop(bias_words[c].y, c * 8 + 2);
-          drop(bias_words[c].z, c * 8 + 4);
-          drop(bias_words[c].w, c * 8 + 6);
-        }
-      }
       // image rows are queries; this warpgroup's 32 keys are chunks (wg & 1) * 4 .. + 3 of half (wg >> 1)
       const int row_at = (wg >> 1) * 16384 + t * 128 + (((t & 7) ^ ((wg & 1) * 4)) << 4);
       const uint32_t p_row = smem_base + FSmem::ps + row_at;
@@ -1553,7 +1533,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
                     make_uint4(pack16<T>(ds2[0]), pack16<T>(ds2[1]), pack16<T>(ds2[2]), pack16<T>(ds2[3])));
         }
       };
-      if (HAS_BIAS || !has_bits || bits == 0xffffffffu)
+      if (bits == 0xffffffffu)
         step_body(std::false_type{});
       else
         step_body(std::true_type{});
@@ -1572,7 +1552,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
         ok = mbar_wait(bar(FSmem::pds_done + ((s - 1) & 1)), ((s - 1) >> 1) & 1, abort_flag);
         if (!ok) break;
         tc_fence_after_sync();
-        store_key_tile(last_item, last_part, last_kt, last_tile);
+        store_key_tile(last_item, last_part, last_kt);
         if (kt == 0) {
           store_query_tiles(last_item, last_first);
           mbar_arrive_warp(bar(FSmem::stat_free + ((w.part & 1) ^ 1)));
@@ -1588,7 +1568,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     if (ok && steps > 0) ok = mbar_wait(bar(FSmem::pds_done + ((steps - 1) & 1)), ((steps - 1) >> 1) & 1, abort_flag);
     if (ok && steps > 0) {
       tc_fence_after_sync();
-      store_key_tile(last_item, last_part, last_kt, last_tile);
+      store_key_tile(last_item, last_part, last_kt);
       store_query_tiles(last_item, last_first);
     }
     if (GROUPS) {
@@ -1633,7 +1613,9 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
 
 // MASKED: there is a mask or a ragged last key tile.  A mask that keeps everything takes the walk without tests (the
 // tests, and above all what they do to the compiler's schedule, cost 8 %).
-template <typename T, bool HAS_BIAS, bool GROUPS, bool MASKED>
+// DIRECT: rows of one tile, whose statistics every thread fetches itself: one step of an item is too short to hide the way through the table
+// (64 columns 11.8 -> 10.6 us).
+template <typename T, bool HAS_BIAS, bool GROUPS, bool MASKED, bool DIRECT>
 __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid_constant__ FParams P) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -1666,10 +1648,10 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
   bool plain = !MASKED;
   if (MASKED && P.mask && (P.cols % kTile == 0 || P.closed)) plain = keeps_all(P.live, P.batch * P.rows, lane);
   if (plain) {
-    fused_walk<T, HAS_BIAS, GROUPS, false, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, P.k_tiles);
+    fused_walk<T, HAS_BIAS, GROUPS, false, false, DIRECT>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, P.k_tiles);
   } else if constexpr (MASKED) {
     uint32_t most = 0;
-    const bool uniform = HAS_BIAS && P.uniform && uniform_prefix(P.uniform, P.batch, lane, most);
+    const bool uniform = HAS_BIAS && !DIRECT && P.uniform && uniform_prefix(P.uniform, P.batch, lane, most);
     if (GROUPS && uniform && *reinterpret_cast<const volatile uint32_t*>(P.prefix + blockIdx.x / uint32_t(P.heads)) == 0) {
       // The CTA's one row keeps no key: zeros.
       const int row = int(blockIdx.x) / P.heads, b = row / P.rows, r = row - b * P.rows, h = int(blockIdx.x) - row * P.heads;
@@ -1689,10 +1671,10 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
       if (P.write_dk) zeros(P.dk);
       if (P.write_dv) zeros(P.dv);
     } else if (uniform)
-      fused_walk<T, HAS_BIAS, GROUPS, false, HAS_BIAS>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane,
+      fused_walk<T, HAS_BIAS, GROUPS, false, HAS_BIAS, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane,
                                                        __shfl_sync(0xffffffffu, max(1, int(most + kTile - 1) / kTile), 0));
     else
-      fused_walk<T, HAS_BIAS, GROUPS, true, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, P.k_tiles);
+      fused_walk<T, HAS_BIAS, GROUPS, true, false, DIRECT>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, P.k_tiles);
   }
   teardown(abort_flag, tmem_base, kFScoreWarp);
 }
@@ -2310,8 +2292,10 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
     };
     const bool has_bits = p.mask || (p.cols % kTile != 0 && !P.closed);
     auto pick = [&](auto bias, auto groups) {
-      return has_bits ? go(ta_bwd_fused_kernel<T, decltype(bias)::value, decltype(groups)::value, true>)
-                      : go(ta_bwd_fused_kernel<T, decltype(bias)::value, decltype(groups)::value, false>);
+      constexpr bool HAS_BIAS = decltype(bias)::value, GROUPS = decltype(groups)::value;
+      if constexpr (!GROUPS)
+        if (P.q_tiles == 1) return has_bits ? go(ta_bwd_fused_kernel<T, HAS_BIAS, false, true, true>) : go(ta_bwd_fused_kernel<T, HAS_BIAS, false, false, true>);
+      return has_bits ? go(ta_bwd_fused_kernel<T, HAS_BIAS, GROUPS, true, false>) : go(ta_bwd_fused_kernel<T, HAS_BIAS, GROUPS, false, false>);
     };
     using Yes = std::true_type;
     using No = std::false_type;
