@@ -2145,7 +2145,7 @@ constexpr int kUniformCols = 192;
 // Whether the single-pass kernel gets a bias that is closed behind a ragged row's end (300 columns 134 -> 124 us, 500 347 -> 328, 700 962 -> 912; the
 // copy 3 to 5).
 bool closes_bias(const oops_ta_problem& p, const oops_ta_grads& g) {
-  return fused_applies(p, g) && bias_closes(p) && (p.cols % kTile != 0 ? p.cols >= 192 : p.mask && p.cols >= kUniformCols) && p.rows >= 64;
+  return fused_applies(p, g) && bias_closes(p) && (p.cols % kTile != 0 ? p.cols >= 192 : p.mask && p.batch <= kUniformSamples && p.cols >= kUniformCols) && p.rows >= 64;
 }
 
 // What it takes behind the rest of the scratch: a word per sample, the bias.
