@@ -1072,6 +1072,22 @@ struct FParams {
   float scale;
 };
 
+// Zeros for an item's rows from `first` on, by `threads` threads of which this is number `at`.
+template <typename T>
+__device__ __forceinline__ void store_zeros(const oops_ta_pair& t, const FParams& P, int item, int first, int at, int threads) {
+  const int row = item / P.heads, b = row / P.rows;
+  T* to = reinterpret_cast<T*>(t.ptr) + b * t.sb + int64_t(row - b * P.rows) * t.sr + int64_t(item - row * P.heads) * t.sh;
+  const bool words = pair_vec_ok(t);
+  for (int i = first * 4 + at; i < P.cols * 4; i += threads) {
+    T* dst = to + int64_t(i >> 2) * t.sc + (i & 3) * 8;
+    if (words) {
+      *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+    } else {
+      for (int c = 0; c < 8; ++c) dst[c] = T(0.f);
+    }
+  }
+}
+
 // The walk over a CTA's steps, identical in every role of the kernel: parts outermost, then key tiles, then query tiles.
 // A part is a group of query tiles of the CTA's one item, or, where a row is a single group, a whole item of the several
 // that the CTA works through.  Ring slots and barrier phases count steps, key tiles and parts.  (Trip counts come from the
@@ -1308,6 +1324,11 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
           fence_proxy_async_smem();
         }
         mbar_arrive_warp(bar(FSmem::kv_ready + slot));
+        if (!GROUPS && kt == k_tiles - 1) {  // what the element-wise warps leave out of the item
+          if (P.write_dk) store_zeros<T>(P.dk, P, w.item, int(item_kept), lane, 32);
+          if (P.write_dv) store_zeros<T>(P.dv, P, w.item, int(item_kept), lane, 32);
+          if (P.write_dq && item_kept == 0) store_zeros<T>(P.dq, P, w.item, 0, lane, 32);
+        }
       }
       // The query tiles of the first part, then one of the next part for every key tile of this one (the rest by the last, where keys have
       // fewer tiles): a key tile late, so that a tile with dropped keys does not wait for the table to be free.
@@ -1360,6 +1381,9 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     };
     uint32_t sm_id;
     asm volatile("mov.u32 %0, %%smid;" : "=r"(sm_id));
+    // Kept keys of the item that is read out (several groups: at the read-out of the slot).  Nothing is stored for dropped keys and rows that
+    // keep none, whose products a query or upstream gradient that is not finite makes NaN: the statistics warp writes their zeros.
+    uint32_t kept = GROUPS ? 0u : request_prefix(int(blockIdx.x));
     // dK (warpgroup 0) and dV (warpgroup 1) of key tile kt, complete for the query tiles of group g: lanes are keys.
     // With several groups the f32 sums travel from group to group through this SM's scratch slot (the same thread
     // owns a key in every group), and the last group stores the 16-bit result.
@@ -1372,15 +1396,8 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       tc_fence_before_sync();
       mbar_arrive_warp(bar(FSmem::dkv_free));
       const bool wanted = wg == 0 ? P.write_dk != 0 : P.write_dv != 0;
-      if (PREFIX && !GROUPS && wanted && kt == k_tiles - 1) {  // keys that no row of the call keeps
-        const oops_ta_pair& o = wg == 0 ? P.dk : P.dv;
-        uint32_t none[32];
-#pragma unroll
-        for (int n = 0; n < 32; ++n) none[n] = 0u;
-        for (int key = k_tiles * kTile + t; key < P.cols; key += kTile) store_row32<T>(item_row(o, item) + int64_t(key) * o.sc, none, 1.f, pair_vec_ok(o));
-      }
       const int key = kt * kTile + t;
-      if (key >= P.cols) return;
+      if (key >= (PREFIX && !GROUPS ? int(kept) : P.cols)) return;
       if (!wanted) return;
       if (GROUPS) {
         // plane i of the slot holds channels 4i .. 4i+3 of every key, so that a warp's 32 keys are 512 contiguous bytes
@@ -1405,13 +1422,14 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     // warp then reports that the accumulators may be overwritten by the next part
     auto store_query_tiles = [&](int item, int first) {
       const int tiles = min(P.tiles_per_group, P.q_tiles - first);
+      const bool dead = PREFIX && !GROUPS && kept == 0;
       for (int qi = wg; qi < tiles; qi += 4) {
         uint32_t acc[32];
         tmem_ld32(lanes_t + kDqCol + qi * kHeadDim, acc);
         tmem_wait_ld();
         tmem_loaded(acc);
         const int q_index = (first + qi) * kTile + t;
-        if (q_index < P.cols && P.write_dq)
+        if (q_index < P.cols && P.write_dq && !dead)
           store_row32<T>(item_row(P.dq, item) + int64_t(q_index) * P.dq.sc, acc, scale, pair_vec_ok(P.dq));
       }
       tc_fence_before_sync();
@@ -1555,6 +1573,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
         store_key_tile(last_item, last_part, last_kt);
         if (kt == 0) {
           store_query_tiles(last_item, last_first);
+          if (!GROUPS) kept = request_prefix(w.item);  // (it has a key tile's time to arrive)
           mbar_arrive_warp(bar(FSmem::stat_free + ((w.part & 1) ^ 1)));
         }
       }
@@ -1579,13 +1598,14 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       named_barrier_sync(2, 16 * 32);
       if (*abort_flag == 0) {
         const int words = 2 * P.cols * 4;  // (tensor, key, eight channels)
+        const int ends = PREFIX ? int(request_prefix(int(blockIdx.x))) : P.cols;
         for (int at = tid; at < words; at += 16 * 32) {
           const int j = at & 3, key = (at >> 2) % P.cols, which = (at >> 2) / P.cols;
           const bool wanted = which == 0 ? P.write_dk != 0 : P.write_dv != 0;
           if (!wanted) continue;
           const float4* slot = reinterpret_cast<const float4*>(P.slots) + (int64_t(sm_id) * 2 + which) * 8 * P.slot_keys + key;
           float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
-          if (!PREFIX || key < k_tiles * kTile) {  // (behind them the slot holds what another row has left)
+          if (!PREFIX || key < ends) {  // (behind the last key tile that is walked the slot holds what another row has left)
             lo = ldcg_f4(slot + (2 * j) * P.slot_keys);
             hi = ldcg_f4(slot + (2 * j + 1) * P.slot_keys);
           }
@@ -1654,22 +1674,9 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
     const bool uniform = HAS_BIAS && !DIRECT && P.uniform && uniform_prefix(P.uniform, P.batch, lane, most);
     if (GROUPS && uniform && *reinterpret_cast<const volatile uint32_t*>(P.prefix + blockIdx.x / uint32_t(P.heads)) == 0) {
       // The CTA's one row keeps no key: zeros.
-      const int row = int(blockIdx.x) / P.heads, b = row / P.rows, r = row - b * P.rows, h = int(blockIdx.x) - row * P.heads;
-      auto zeros = [&](const oops_ta_pair& t) {
-        T* to = reinterpret_cast<T*>(t.ptr) + b * t.sb + int64_t(r) * t.sr + int64_t(h) * t.sh;
-        const bool words = pair_vec_ok(t);
-        for (int at = tid; at < P.cols * 4; at += kFThreads) {
-          T* dst = to + int64_t(at >> 2) * t.sc + (at & 3) * 8;
-          if (words) {
-            *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
-          } else {
-            for (int c = 0; c < 8; ++c) dst[c] = T(0.f);
-          }
-        }
-      };
-      if (P.write_dq) zeros(P.dq);
-      if (P.write_dk) zeros(P.dk);
-      if (P.write_dv) zeros(P.dv);
+      if (P.write_dq) store_zeros<T>(P.dq, P, int(blockIdx.x), 0, tid, kFThreads);
+      if (P.write_dk) store_zeros<T>(P.dk, P, int(blockIdx.x), 0, tid, kFThreads);
+      if (P.write_dv) store_zeros<T>(P.dv, P, int(blockIdx.x), 0, tid, kFThreads);
     } else if (uniform)
       fused_walk<T, HAS_BIAS, GROUPS, false, HAS_BIAS, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane,
                                                        __shfl_sync(0xffffffffu, max(1, int(most + kTile - 1) / kTile), 0));

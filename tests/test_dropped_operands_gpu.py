@@ -1,0 +1,65 @@
+"""Token masks over operands that are not finite, in the reverse pass: infinities and NaN in the queries, keys, values and upstream gradients
+of rows that keep no key, in dropped keys and values, and in the bias of a sample that keeps nothing, reach no gradient; a query or upstream
+gradient of a row that keeps keys reaches none of its dropped keys.  Rows of one and of several groups of query tiles, with and without a
+ragged key tile.  16-bit bounds as in the parity tests: 2e-2 of the largest value (at least 1)."""
+
+import pytest
+import torch
+
+from oracle import triangle_oracle as oracle
+from oops_b200 import triangle_attention
+
+pytestmark = pytest.mark.gpu
+INF, NAN = float("inf"), float("nan")
+
+
+def _gradients(cuda, q, k, v, mask, bias, up):
+    leaves = [t.to(cuda).requires_grad_(True) for t in (q, k, v, bias)]
+    out = triangle_attention(*leaves[:3], mask.to(cuda), leaves[3])
+    return [t.detach().cpu() for t in (out, *torch.autograd.grad(out, leaves, up.to(cuda)))]
+
+
+@pytest.mark.parametrize("dtype,batch,rows,n", [(torch.bfloat16, 1, 64, 192), (torch.float16, 2, 70, 256), (torch.bfloat16, 1, 64, 700),
+                                                (torch.bfloat16, 1, 64, 800)])
+def test_rows_that_keep_nothing(cuda, dtype, batch, rows, n):
+    gen = torch.Generator().manual_seed(n)
+    q, k, v, up = (torch.randn(batch, rows, n, 2, 32, generator=gen).to(dtype) for _ in range(4))
+    bias = torch.randn(batch, 1, 2, n, n, generator=gen).to(dtype)
+    live = torch.arange(rows) < rows - rows // 4
+    mask = ((torch.arange(n) < n - n // 5) & live[:, None])[None].repeat(batch, 1, 1)
+    if batch > 1:
+        mask[1] = False
+    want = oracle.forward_backward(q, k, v, mask, bias, up)
+    if batch > 1:
+        bias[1, ..., ::3], bias[1, ..., 1::3] = INF, NAN
+    for row in range(rows):
+        for b in range(batch):
+            if not mask[b, row].any():
+                q[b, row, ::2], q[b, row, 1::2] = INF, NAN
+                up[b, row, ::3], up[b, row, 1::3] = NAN, -INF
+    dead = ~mask[..., None, None]
+    got = _gradients(cuda, q, k.masked_fill(dead, INF), v.masked_fill(dead, NAN), mask, bias, up)
+    for name, g, ref in zip(("out", "dq", "dk", "dv", "dbias"), got, want):
+        error = float((g.float() - ref).abs().max())
+        assert error <= 2e-2 * max(1.0, float(ref.abs().max())), (name, error)
+    for g in got[:2]:
+        assert not g[~mask.any(-1)].any()
+    for g in got[2:4]:
+        assert not g[~mask].any()
+
+
+@pytest.mark.parametrize("n", [256, 700, 800])
+def test_dropped_keys_of_other_rows(cuda, n):
+    gen = torch.Generator().manual_seed(n)
+    rows = 64
+    q, k, v, up = (torch.randn(1, rows, n, 1, 32, generator=gen).to(torch.bfloat16) for _ in range(4))
+    bias = torch.randn(1, 1, 1, n, n, generator=gen).to(torch.bfloat16)
+    mask = (torch.arange(n) < n - 70).expand(1, rows, n).contiguous()
+    q[0, 3, 5], q[0, 4, 6, 0, 7], up[0, 5, 7] = NAN, INF, -INF
+    got = _gradients(cuda, q, k, v, mask, bias, up)
+    for g in got[2:4]:
+        assert not g[~mask].any()
+    fine = torch.ones(rows, dtype=torch.bool)
+    fine[3:6] = False
+    for g in got[:4]:
+        assert torch.isfinite(g[0, fine]).all()
