@@ -1061,6 +1061,7 @@ struct FParams {
   float* delta;     // read, or written from `out` and `dout` where own_delta is set
   oops_ta_pair out, dout;
   int own_delta;
+  Logits logits;  // operands of a closed bias
   const uint8_t* mask;
   const uint32_t* live;  // what prepare_kernel has found out about the mask
   int64_t m_sb, m_sr, m_sc;
@@ -1429,8 +1430,16 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
         tmem_wait_ld();
         tmem_loaded(acc);
         const int q_index = (first + qi) * kTile + t;
-        if (q_index < P.cols && P.write_dq && !dead)
-          store_row32<T>(item_row(P.dq, item) + int64_t(q_index) * P.dq.sc, acc, scale, pair_vec_ok(P.dq));
+        if (!(q_index < P.cols && P.write_dq && !dead)) continue;
+        store_row32<T>(item_row(P.dq, item) + int64_t(q_index) * P.dq.sc, acc, scale, pair_vec_ok(P.dq));
+        if (HAS_BIAS && !BITS && !DIRECT && (PREFIX || P.closed) && isnan(__uint_as_float(acc[0]))) {
+          const int row = item / P.heads, b = row / P.rows;
+          if (P.logits.all_minus_infinity<T>(b, row - b * P.rows, item - row * P.heads, q_index, PREFIX ? int(request_prefix(item)) : P.cols)) {
+#pragma unroll
+            for (int n = 0; n < 32; ++n) acc[n] = 0u;
+            store_row32<T>(item_row(P.dq, item) + int64_t(q_index) * P.dq.sc, acc, scale, pair_vec_ok(P.dq));
+          }
+        }
       }
       tc_fence_before_sync();
       mbar_arrive_warp(bar(FSmem::dq_free));
@@ -2249,6 +2258,7 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
         P.prefix = live + 2 * int64_t(p.batch) * p.rows;
         P.uniform = reinterpret_cast<uint32_t*>(base + layout.closed);
       }
+      P.logits = Logits(p);
       status = close_bias(&P.map_bias, p, base + layout.closed + align256(uint64_t(p.batch) * 4), "bias", stream, P.prefix,
                           const_cast<uint32_t*>(P.uniform));
     }

@@ -145,6 +145,31 @@ int close_bias(CUtensorMap* map, const oops_ta_problem& p, void* scratch, const 
   return status ? status : encode_bias(map, p, scratch, row, plane, plane * p.heads, plane * p.heads, kTile, what, int(row));
 }
 
+// What a walk over a closed bias asks about a row that came out as NaN: a query that holds an infinity has NaN for the zeros of the keys that
+// the bias closes, but where its kept logits are minus infinity, all of them, it has no probability (the first keys answer it otherwise).
+struct Logits {
+  oops_ta_pair q, k;
+  const void* bias;  // row-shared, keys contiguous
+  int64_t bias_sb, bias_sh, bias_sq;
+  float scale;
+  Logits() = default;
+  explicit Logits(const oops_ta_problem& p) : q(p.q), k(p.k), bias(p.bias), bias_sb(p.bias_sb), bias_sh(p.bias_sh), bias_sq(p.bias_sq), scale(p.scale) {}
+  template <typename T>
+  __device__ __forceinline__ bool all_minus_infinity(int b, int r, int h, int query, int kept) const {
+    const T* q_at = reinterpret_cast<const T*>(q.ptr) + b * q.sb + int64_t(r) * q.sr + int64_t(query) * q.sc + h * q.sh;
+    const T* k_at = reinterpret_cast<const T*>(k.ptr) + b * k.sb + int64_t(r) * k.sr + h * k.sh;
+    const T* bias_at = reinterpret_cast<const T*>(bias) + b * bias_sb + h * bias_sh + query * bias_sq;
+#pragma unroll 1
+    for (int key = 0; key < kept; ++key, k_at += k.sc) {
+      float dot = 0.f;
+#pragma unroll 4
+      for (int c = 0; c < kHeadDim; ++c) dot = fmaf(float(q_at[c]), float(k_at[c]), dot);
+      if (dot * scale + float(bias_at[key]) != -INFINITY) return false;
+    }
+    return true;
+  }
+};
+
 // A mask whose rows may all keep the same first keys (or none), as masks of tokens do: whether they do is found out on the device, and the bias is
 // closed behind those keys.  `uniform` has a word per sample.
 constexpr int kUniformSamples = 32;

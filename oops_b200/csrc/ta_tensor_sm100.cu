@@ -90,6 +90,7 @@ struct FwdParams {
   int64_t m_sb, m_sr, m_sc;
   int batch, rows, cols, heads, bias_groups;
   int closed;            // the bias is minus infinity behind a ragged row's end
+  Logits logits;         // its operands (a closed bias only)
   int items;             // query items x heads x rows (or pairs of rows) x batch
   int q_items, k_steps;  // query tiles (ROWS) or pairs of query tiles of a row; key steps
   int out_vec16;
@@ -489,6 +490,7 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
     if (PERSIST) at = fwd_item<ROWS>(P, item);  // (not held through the steps)
     const int r = row_of(w), h = at.h, b = at.b, q_index = first_query(w) + t;
     const bool stored = q_index < P.cols && (!PERSIST || !ROWS || at.r0 + w < P.rows);
+    const bool none = PLAIN && HAS_BIAS && P.closed && stored && isnan(l_run) && P.logits.all_minus_infinity<T>(b, r, h, q_index, P.cols);
     // Gated epilogue: the thread's 32 gate logits are requested before the wait for the last product, so that their
     // trip from global memory runs under it (the words are not touched until the output row is ready).
     uint4 gate_words[4] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
@@ -509,6 +511,11 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
         tmem_loaded(acc);
       }
       if (stored) {
+        if (none) {
+          l_run = 0.f;
+#pragma unroll
+          for (int n = 0; n < 32; ++n) acc[n] = 0u;
+        }
         const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
         uint32_t o2[16];
 #pragma unroll
@@ -769,6 +776,7 @@ int launch_forward(const oops_ta_problem& p, const oops_ta_pair& out, float* lse
   if (P.closed) {
     status = close_bias(&P.map_bias, p, p.workspace, "bias", stream);
     if (status) return status;
+    P.logits = Logits(p);
   } else if (has_bias) {
     status = encode_bias(&P.map_bias, p, p.bias, p.bias_sq, p.bias_sh, p.bias_sg, p.bias_sb, kTile, "bias");
     if (status) return status;

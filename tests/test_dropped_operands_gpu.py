@@ -63,3 +63,29 @@ def test_dropped_keys_of_other_rows(cuda, n):
     fine[3:6] = False
     for g in got[:4]:
         assert torch.isfinite(g[0, fine]).all()
+
+
+@pytest.mark.parametrize("rows,n,masked", [(128, 390, False), (128, 447, False), (2, 700, False), (64, 700, False), (64, 1000, False),
+                                           (64, 256, True), (64, 700, True), (64, 800, True)])
+def test_rows_whose_logits_are_minus_infinity(cuda, rows, n, masked):
+    """A query that holds an infinity and whose products with the kept keys are minus infinity, all of them, has no probability: zeros."""
+    gen = torch.Generator().manual_seed(n)
+    q, k, v, up = (torch.randn(1, rows, n, 1, 32, generator=gen).to(torch.bfloat16) for _ in range(4))
+    bias = torch.randn(1, 1, 1, n, n, generator=gen).to(torch.bfloat16)
+    mask = torch.ones(1, rows, n, dtype=torch.bool)
+    if masked:
+        mask[..., n - 70:] = False
+    k[0, 1, :, 0, 9] = -k[0, 1, :, 0, 9].abs() - 1.0
+    empty = [n // 2, n - 1, 3]
+    q[0, 1, empty, 0, 9] = INF
+    q[0, 0, 6, 0, 9] = INF  # (its keys have both signs: NaN)
+    leaves = [t.to(cuda).requires_grad_(True) for t in (q, k, v, bias)]
+    out = triangle_attention(*leaves[:3], mask.to(cuda) if masked else None, leaves[3])
+    dq, dk, dv, _ = torch.autograd.grad(out, leaves, up.to(cuda))
+    for got in (out, dq):
+        assert not got[0, 1, empty].any()
+        assert torch.isnan(got[0, 0, 6]).all()
+        got = got.detach().clone()
+        got[0, 0, 6] = 0
+        assert torch.isfinite(got).all()
+    assert torch.isfinite(dv[0, 1:]).all()
