@@ -64,7 +64,7 @@ struct FwdSmem {
   static constexpr int bias_empty = bias_full + bias_rings * 2;
   static constexpr int s_full = bias_empty + bias_rings * 2;      // [2] S of a step is in tensor memory
   static constexpr int p_full = s_full + 2;                       // [2] P is in tensor memory
-  static constexpr int s_free = p_full + 2;                       // [2] the scores of a step are in registers
+  static constexpr int s_free = p_full + 2;                       // [2] the scores of a step without tests are in registers
   static constexpr int pv_done = s_free + 2;                      // [2] the latest P V product has completed
   static constexpr int q_empty = pv_done + 2;                     // [2] every score product of an item has completed (PERSIST)
   static constexpr int num_bars = q_empty + 2;
@@ -221,6 +221,16 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
         mma_commit(bar(Smem::s_full + w));
         mma_commit(bar(Smem::k_empty + ring + st));
       };
+      // O[128 x 32] += P[128 x 64] V[64 x 32]; V is MN-major (channel contiguous), 64-byte swizzle:
+      // 8-key groups are 512 bytes apart, each 16-key step advances 1024 bytes.
+      auto issue_pv = [&](int st, int i) {
+        const uint64_t vdesc = vdesc0 + uint64_t((st * kKvBytes) >> 4);
+#pragma unroll
+        for (int kk = 0; kk < kKeys / 16; ++kk)
+          mma_ts(o_t, p_t + kk * 8, vdesc + uint64_t(kk * (1024 >> 4)), idesc_pv, (i > 0 || kk > 0) ? 1u : 0u);
+        mma_commit(bar(Smem::pv_done + w));
+        mma_commit(bar(Smem::v_empty + ring + st));
+      };
       bool ok = mbar_wait(bar(Smem::q_full + w), 0, abort_flag);
       if (ok) ok = mbar_wait(bar(Smem::k_full + ring), 0, abort_flag);
       if (ok) {
@@ -228,21 +238,28 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
         issue_qk(0);
         if (PERSIST && KS == 1) mma_commit(bar(Smem::q_empty + w));
       }
-      int st = 0, round = 0, n = 0;
+      int st = 0, round = 0, n = 0, untested = 0;  // steps so far, and those without tests
       for (int item = int(blockIdx.x), turn = 0; ok && item_there(item, turn); item += int(gridDim.x), ++turn) {
         for (int i = 0; i < KS && ok; ++i, ++n) {
           const int next = st + 1 == kStages ? 0 : st + 1, next_round = next == 0 ? round + 1 : round;
-          // The next scores (of this item or the next one) overwrite these as soon as the last columns are in registers.
-          const bool more = i + 1 < KS, turns = PERSIST && !more && item + int(gridDim.x) < P.items;
-          if (turns) ok = mbar_wait(bar(Smem::q_full + w), (turn + 1) & 1, abort_flag);
-          if (ok && (more || turns)) {
-            ok = mbar_wait(bar(Smem::k_full + ring + next), next_round & 1, abort_flag);
-            if (ok) ok = mbar_wait(bar(Smem::s_free + w), n & 1, abort_flag);
-            if (!ok) break;
+          const bool more = i + 1 < KS, turns = PERSIST && !more && item + int(gridDim.x) < P.items, tests = !PLAIN && i >= full_steps;
+          // The next scores (of this item or the next one) overwrite these as soon as the last columns are in registers, or, after a step with
+          // tests, when its probabilities stand.
+          auto issue_next = [&]() {
             tc_fence_after_sync();
             issue_qk(next);
             if (PERSIST && (more ? i + 2 == KS : KS == 1)) mma_commit(bar(Smem::q_empty + w));
+          };
+          if (turns) ok = mbar_wait(bar(Smem::q_full + w), (turn + 1) & 1, abort_flag);
+          if (ok && (more || turns)) {
+            ok = mbar_wait(bar(Smem::k_full + ring + next), next_round & 1, abort_flag);
+            if (!tests) {
+              if (ok) ok = mbar_wait(bar(Smem::s_free + w), (PLAIN ? n : untested) & 1, abort_flag);
+              if (!ok) break;
+              issue_next();
+            }
           }
+          if (!PLAIN && !tests) ++untested;
           if (ok) ok = mbar_wait(bar(Smem::v_full + ring + st), round & 1, abort_flag);
           // a warpgroup signs off the value steps with dropped keys after clearing their rows
           if (ok && signoff && i >= full_steps) {
@@ -252,14 +269,8 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
           if (ok) ok = mbar_wait(bar(Smem::p_full + w), n & 1, abort_flag);
           if (!ok) break;
           tc_fence_after_sync();
-          // O[128 x 32] += P[128 x 64] V[64 x 32]; V is MN-major (channel contiguous), 64-byte swizzle:
-          // 8-key groups are 512 bytes apart, each 16-key step advances 1024 bytes.
-          const uint64_t vdesc = vdesc0 + uint64_t((st * kKvBytes) >> 4);
-#pragma unroll
-          for (int kk = 0; kk < kKeys / 16; ++kk)
-            mma_ts(o_t, p_t + kk * 8, vdesc + uint64_t(kk * (1024 >> 4)), idesc_pv, (i > 0 || kk > 0) ? 1u : 0u);
-          mma_commit(bar(Smem::pv_done + w));
-          mma_commit(bar(Smem::v_empty + ring + st));
+          if (tests && (more || turns)) issue_next();
+          issue_pv(st, i);
           st = next;
           round = next_round;
         }
@@ -379,7 +390,8 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
       // Probabilities of the step into tensor memory; returns their sum.  Before the exponentials of the last columns the
       // scores are given back for the next product, unless the step has to be repeated (`wanted`, only asked where `may_repeat`).
       bool p_free = i == 0;
-      auto step_pass = [&](bool may_repeat, bool& wanted) -> float {
+      bool wanted = ref == -INFINITY, may_repeat = true;
+      auto step_pass = [&]() -> float {
         const float shift = ref == -INFINITY ? 0.f : -ref;
         const f32x2 shift2 = pack2(shift, shift);
         f32x2 totals[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
@@ -437,13 +449,6 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
         }
         float lo, hi;
         unpack2(add2(totals[0], totals[1]), lo, hi);
-        if (kDrops) {  // (in a step with tests the look at the last logits costs more than the lead of the product gives: scattered keys of 768 columns 936 us, without it 923)
-          wanted = may_repeat && !(lo + hi < kStepSumLimit);
-          if (__any_sync(0xffffffffu, wanted)) return 0.f;
-          tc_fence_before_sync();
-          mbar_arrive_warp(bar(Smem::s_free + w));
-          if (HAS_BIAS) mbar_arrive_warp(bar(Smem::bias_empty + bias_slot));
-        }
         return lo + hi;
       };
       float sum = 0.f;
@@ -454,21 +459,20 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
           ok = mbar_wait(bar(Smem::pv_done + w), (at_step - 1) & 1, abort_flag);
           tc_fence_after_sync();
         }
-        mbar_arrive_warp(bar(Smem::s_free + w));
-        if (HAS_BIAS) mbar_arrive_warp(bar(Smem::bias_empty + bias_slot));
         uint32_t zeros[16];
 #pragma unroll
         for (int n = 0; n < 16; ++n) zeros[n] = 0u;
         tmem_st16(p_tmem, zeros);
         tmem_st16(p_tmem + 16, zeros);
       } else {
-        bool wanted = ref == -INFINITY;
 #pragma unroll 1
         for (int attempt = 0; attempt < 2 && ok; ++attempt) {
           if (__any_sync(0xffffffffu, wanted)) ok = raise(wanted);
           else if (attempt > 0) break;
           if (!ok) return;
-          sum = step_pass(attempt == 0, wanted);
+          may_repeat = attempt == 0;
+          sum = step_pass();
+          if (kDrops) wanted = !(sum < kStepSumLimit);
         }
       }
       if (!ok) return;
@@ -476,6 +480,7 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
       tmem_wait_st();
       tc_fence_before_sync();
       mbar_arrive_warp(bar(Smem::p_full + w));
+      if (kDrops && HAS_BIAS) mbar_arrive_warp(bar(Smem::bias_empty + bias_slot));
     };
     for (int item = int(blockIdx.x), turn = 0; ok && item_there(item, turn); item += int(gridDim.x), ++turn, base += KS) {
     if (PERSIST) {
