@@ -1130,7 +1130,7 @@ struct FWalk {
 // is ragged.
 template <typename T, bool HAS_BIAS, bool GROUPS, bool BITS, bool PREFIX, bool DIRECT>
 __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base, uint8_t* smem_gen, volatile int* abort_flag,
-                                           uint32_t tmem_base, int tid, int warp, int lane, int k_tiles) {
+                                           uint32_t tmem_base, int tid, int warp, int lane, int k_tiles, bool& suspects) {
   auto bar = [&](int index) -> uint32_t { return smem_base + FSmem::bars + index * 8; };
   const bool has_mask = BITS && P.mask != nullptr;
   constexpr bool prefixes = PREFIX;
@@ -1262,6 +1262,8 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
         }
         if (!table_free()) return;
 #pragma unroll
+        for (int j = 0; j < 4; ++j) suspects |= lse[j] == 0.f && !dead;
+#pragma unroll
         for (int j = 0; j < 4; ++j) sts_f2_at(table + (j * 32 + lane) * 8, dead ? -INFINITY : -lse[j] * kLog2e, dead ? 0.f : -delta[j]);
       } else {
         if (!table_free()) return;
@@ -1291,6 +1293,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
             if ((lane >> 3) == i) own = mine;
           }
           if (q < P.cols) P.delta[stat + q] = own;
+          suspects |= lse == 0.f && !dead;
           sts_f2_at(table + (j + lane) * 8, dead ? -INFINITY : -lse * kLog2e, dead ? 0.f : -own);
         }
       }
@@ -1430,16 +1433,8 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
         tmem_wait_ld();
         tmem_loaded(acc);
         const int q_index = (first + qi) * kTile + t;
-        if (!(q_index < P.cols && P.write_dq && !dead)) continue;
-        store_row32<T>(item_row(P.dq, item) + int64_t(q_index) * P.dq.sc, acc, scale, pair_vec_ok(P.dq));
-        if (HAS_BIAS && !BITS && !DIRECT && (PREFIX || P.closed) && isnan(__uint_as_float(acc[0]))) {
-          const int row = item / P.heads, b = row / P.rows;
-          if (P.logits.all_minus_infinity<T>(b, row - b * P.rows, item - row * P.heads, q_index, PREFIX ? int(request_prefix(item)) : P.cols)) {
-#pragma unroll
-            for (int n = 0; n < 32; ++n) acc[n] = 0u;
-            store_row32<T>(item_row(P.dq, item) + int64_t(q_index) * P.dq.sc, acc, scale, pair_vec_ok(P.dq));
-          }
-        }
+        if (q_index < P.cols && P.write_dq && !dead)
+          store_row32<T>(item_row(P.dq, item) + int64_t(q_index) * P.dq.sc, acc, scale, pair_vec_ok(P.dq));
       }
       tc_fence_before_sync();
       mbar_arrive_warp(bar(FSmem::dq_free));
@@ -1674,10 +1669,10 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  bool plain = !MASKED;
+  bool plain = !MASKED, suspects = false;  // suspects: rows without a probability, perhaps (statistics warp)
   if (MASKED && P.mask && (P.cols % kTile == 0 || P.closed)) plain = keeps_all(P.live, P.batch * P.rows, lane);
   if (plain) {
-    fused_walk<T, HAS_BIAS, GROUPS, false, false, DIRECT>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, P.k_tiles);
+    fused_walk<T, HAS_BIAS, GROUPS, false, false, DIRECT>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, P.k_tiles, suspects);
   } else if constexpr (MASKED) {
     uint32_t most = 0;
     const bool uniform = HAS_BIAS && !DIRECT && P.uniform && uniform_prefix(P.uniform, P.batch, lane, most);
@@ -1688,11 +1683,24 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
       if (P.write_dv) store_zeros<T>(P.dv, P, int(blockIdx.x), 0, tid, kFThreads);
     } else if (uniform)
       fused_walk<T, HAS_BIAS, GROUPS, false, HAS_BIAS, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane,
-                                                       __shfl_sync(0xffffffffu, max(1, int(most + kTile - 1) / kTile), 0));
+                                                       __shfl_sync(0xffffffffu, max(1, int(most + kTile - 1) / kTile), 0), suspects);
     else
-      fused_walk<T, HAS_BIAS, GROUPS, true, false, DIRECT>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, P.k_tiles);
+      fused_walk<T, HAS_BIAS, GROUPS, true, false, DIRECT>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, P.k_tiles, suspects);
   }
   teardown(abort_flag, tmem_base, kFScoreWarp);
+  if (HAS_BIAS && !DIRECT && P.closed && suspects && P.write_dq) {
+    // A query that holds an infinity has NaN for the zeros of keys that the bias closes.  A row whose kept logits are minus infinity, all of
+    // them, has no probability (the forward pass leaves it a log-sum-exp of 0) and no gradient all the same; its dQ stands by now.
+    for (int item = int(blockIdx.x); item < P.items; item += GROUPS ? P.items : int(gridDim.x)) {
+      const int row = item / P.heads, h = item - row * P.heads, b = row / P.rows, r = row - b * P.rows;
+      const int kept = P.prefix && P.uniform[b] != ~0u ? int(P.prefix[row]) : P.cols;
+      T* dq = reinterpret_cast<T*>(P.dq.ptr) + b * P.dq.sb + int64_t(r) * P.dq.sr + h * P.dq.sh;
+      for (int q = lane; q < P.cols; q += 32) {
+        if (P.lse[int64_t(item) * P.cols + q] != 0.f || !P.logits.all_minus_infinity<T>(b, r, h, q, kept)) continue;
+        for (int c = 0; c < kHeadDim; ++c) dq[q * P.dq.sc + c] = T(0.f);
+      }
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
