@@ -17,8 +17,19 @@ struct BiasRows {
   uint32_t words, heads, cols, groups;  // words of a row
   uint64_t total;
   int heads_inner, whole;  // whole: rows of the source are whole 16-byte words
-  uint32_t fill;           // two elements of padding
 };
+
+// Eight keys of a row from key `word` * 8 on, `fill` (two elements) from key `end` on.
+__device__ __forceinline__ uint4 bias_word(const uint16_t* src, int64_t s_k, bool whole, uint32_t word, uint32_t end, uint32_t fill) {
+  if (whole && word * 8 + 8 <= end) return *reinterpret_cast<const uint4*>(src + word * 8);
+  uint32_t packed[4] = {fill, fill, fill, fill};
+#pragma unroll
+  for (uint32_t e = 0; e < 8; ++e) {
+    const uint32_t key = word * 8 + e;
+    if (key < end) packed[e / 2] = (packed[e / 2] & (0xffff0000u >> (e % 2 * 16))) | uint32_t(src[int64_t(key) * s_k]) << (e % 2 * 16);
+  }
+  return make_uint4(packed[0], packed[1], packed[2], packed[3]);
+}
 
 // I counts words: 32 bits up to 64 GB of them.
 template <typename I>
@@ -40,32 +51,28 @@ __global__ void __launch_bounds__(256) bias_rows_kernel(const BiasRows p) {
   }
   const uint32_t g = uint32_t(i % p.groups), b = uint32_t(i / p.groups);
   const uint16_t* src = p.src + b * p.s_b + g * p.s_g + h * p.s_h + q * p.s_q;
-  uint32_t packed[4] = {p.fill, p.fill, p.fill, p.fill};
-  if (p.whole && word * 8 + 8 <= p.cols) {
-    const uint4 v = *reinterpret_cast<const uint4*>(src + word * 8);
-    packed[0] = v.x; packed[1] = v.y; packed[2] = v.z; packed[3] = v.w;
-  } else {
-#pragma unroll
-    for (uint32_t e = 0; e < 8; ++e) {
-      const uint32_t key = word * 8 + e;
-      if (key < p.cols) packed[e / 2] = (packed[e / 2] & (0xffff0000u >> (e % 2 * 16))) | uint32_t(src[int64_t(key) * p.s_k]) << (e % 2 * 16);
-    }
-  }
   const int64_t row = ((int64_t(b) * p.groups + g) * p.heads + h) * p.cols + q;
-  reinterpret_cast<uint4*>(p.dst)[row * p.words + word] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+  reinterpret_cast<uint4*>(p.dst)[row * p.words + word] = bias_word(src, p.s_k, p.whole, word, p.cols, 0u);
 }
 
-// A row-shared bias (batch, head, query, key) in rows of `words` 16-byte words whose keys from an end on are minus infinity: the row's, or,
-// where all rows of a sample that keep a key keep the same first ones, the end of those, which uniform[sample] then has (~0 where they do not;
-// 0: no row keeps a key).  One launch for all samples; every CTA looks at all of its sample's rows (L2).
-__global__ void __launch_bounds__(256) closed_bias_kernel(const BiasRows p, const uint32_t* prefix, int rows, uint32_t* uniform) {
+// The bias (batch, head, query, key) in rows of `words` 16-byte words whose keys from an end on are `fill`: the row's end, or a token mask's.
+// What no kernel would walk over is not copied.  One launch for all samples; every CTA looks for itself (L2).
+struct ClosedBias {
+  const uint16_t* src;
+  uint16_t* dst;
+  int64_t s_b, s_h, s_q;
+  uint32_t words, cols, total;  // words of a row, words of a sample
+  uint32_t fill;
+  ClosedBiasLook look;
+};
+__global__ void __launch_bounds__(256) closed_bias_kernel(const ClosedBias p) {
   __shared__ uint32_t low[8], high[8];
   const uint32_t b = blockIdx.y;
   uint32_t end = p.cols;
-  if (prefix) {
+  if (p.look.prefix) {
     uint32_t lo = ~0u, hi = 0u;
-    for (int r = threadIdx.x; r < rows; r += 256) {
-      const uint32_t v = prefix[int64_t(b) * rows + r];
+    for (int r = threadIdx.x; r < p.look.rows; r += 256) {
+      const uint32_t v = p.look.prefix[int64_t(b) * p.look.rows + r];
       if (v != 0) lo = min(lo, v);
       hi = max(hi, v);
     }
@@ -82,35 +89,37 @@ __global__ void __launch_bounds__(256) closed_bias_kernel(const BiasRows p, cons
       hi = max(hi, high[i]);
     }
     const bool same = hi == 0 || (lo == hi && hi != ~0u);
+    if (blockIdx.x == 0 && threadIdx.x == 0) p.look.found[b] = same ? hi : ~0u;
     if (same && hi != 0) end = hi;
-    if (blockIdx.x == 0 && threadIdx.x == 0) uniform[b] = same ? hi : ~0u;
-  }
-  uint32_t i = blockIdx.x * 256u + threadIdx.x, h = 0;
-  if (i >= uint32_t(p.total)) return;
-  if (p.heads_inner) {
-    h = i % p.heads;
-    i /= p.heads;
-  }
-  const uint32_t word = i % p.words;
-  i /= p.words;
-  const uint32_t q = i % p.cols;
-  if (!p.heads_inner) h = i / p.cols;
-  const uint16_t* src = p.src + b * p.s_b + h * p.s_h + q * p.s_q;
-  uint32_t packed[4] = {p.fill, p.fill, p.fill, p.fill};
-  if (p.whole && word * 8 + 8 <= end) {
-    const uint4 v = *reinterpret_cast<const uint4*>(src + word * 8);
-    packed[0] = v.x; packed[1] = v.y; packed[2] = v.z; packed[3] = v.w;
-  } else {
-#pragma unroll
-    for (uint32_t e = 0; e < 8; ++e) {
-      const uint32_t key = word * 8 + e;
-      if (key < end) packed[e / 2] = (packed[e / 2] & (0xffff0000u >> (e % 2 * 16))) | uint32_t(src[int64_t(key) * p.s_k]) << (e % 2 * 16);
+    if (p.look.whole && end == p.cols) {  // closed behind a prefix of another sample, or not walked over
+      bool drops = false;
+      const uint32_t words = (gridDim.y * uint32_t(p.look.rows) + 7) / 8;
+      for (uint32_t i = threadIdx.x; i < words; i += 256) drops |= p.look.drops[i] != 0;
+      if (!__syncthreads_or(drops) || !same) return;
     }
   }
-  reinterpret_cast<uint4*>(p.dst)[((int64_t(b) * p.heads + h) * p.cols + q) * p.words + word] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+  const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= p.total) return;
+  const uint32_t row = i / p.words, word = i - row * p.words, h = row / p.cols, q = row - h * p.cols;
+  const uint16_t* src = p.src + b * p.s_b + h * p.s_h + q * p.s_q;
+  reinterpret_cast<uint4*>(p.dst)[int64_t(b) * p.total + i] = bias_word(src, 1, true, word, end, p.fill);
 }
 
-BiasRows describe_rows(int batch, int groups, int heads, int cols, const void* src, const int64_t strides[5], void* dst, int64_t words, uint16_t fill) {
+}  // namespace
+
+int closed_bias(int batch, int heads, int cols, const void* src, int64_t s_b, int64_t s_h, int64_t s_q, void* dst, int row, uint16_t fill,
+                const ClosedBiasLook& look, cudaStream_t stream) {
+  const int64_t total = int64_t(heads) * cols * (row / 8);  // of a sample
+  if (total == 0 || batch == 0) return OOPS_TA_OK;
+  if (total > 0xffffff00ll || batch > 65535) return fail(OOPS_TA_LIMIT_EXCEEDED, "bias of %lld words in %d samples", (long long)total, batch);
+  const ClosedBias p{reinterpret_cast<const uint16_t*>(src), reinterpret_cast<uint16_t*>(dst), s_b, s_h, s_q, uint32_t(row / 8), uint32_t(cols),
+                     uint32_t(total), fill * 0x10001u, look};
+  closed_bias_kernel<<<dim3((unsigned)ceil_div(total, 256), (unsigned)batch), 256, 0, stream>>>(p);
+  count_launch();
+  return check_launch("closed bias");
+}
+
+int bias_rows(int batch, int groups, int heads, int cols, const void* src, const int64_t strides[5], void* dst, cudaStream_t stream) {
   BiasRows p{};
   p.src = reinterpret_cast<const uint16_t*>(src);
   p.dst = reinterpret_cast<uint16_t*>(dst);
@@ -119,8 +128,7 @@ BiasRows describe_rows(int batch, int groups, int heads, int cols, const void* s
   p.s_h = strides[2];
   p.s_q = strides[3];
   p.s_k = strides[4];
-  p.words = uint32_t(words);
-  p.fill = fill * 0x10001u;
+  p.words = uint32_t(ceil_div(cols, 8));
   auto aligned = [](int64_t stride, int size) { return size == 1 || stride % 8 == 0; };
   p.whole = strides[4] == 1 && (reinterpret_cast<uintptr_t>(src) & 15) == 0 && aligned(strides[0], batch) && aligned(strides[1], groups) &&
             aligned(strides[2], heads) && aligned(strides[3], cols);
@@ -128,26 +136,6 @@ BiasRows describe_rows(int batch, int groups, int heads, int cols, const void* s
   p.cols = uint32_t(cols);
   p.groups = uint32_t(groups);
   p.heads_inner = heads > 1 && p.s_h < p.s_k;
-  return p;
-}
-
-}  // namespace
-
-int closed_bias(int batch, int heads, int cols, const void* src, const int64_t strides[5], void* dst, int row, uint16_t fill, const uint32_t* prefix,
-                int rows, uint32_t* uniform, cudaStream_t stream) {
-  BiasRows p = describe_rows(batch, 1, heads, cols, src, strides, dst, ceil_div(row, 8), fill);
-  const int64_t total = int64_t(heads) * cols * p.words;  // of a sample
-  if (total == 0 || batch == 0) return OOPS_TA_OK;
-  if (total > 0xffffff00ll || batch > 65535) return fail(OOPS_TA_LIMIT_EXCEEDED, "bias of %lld words in %d samples", (long long)total, batch);
-  p.total = uint64_t(total);
-  const dim3 grid((unsigned)ceil_div(total, 256), (unsigned)batch);
-  closed_bias_kernel<<<grid, 256, 0, stream>>>(p, prefix, rows, uniform);
-  count_launch();
-  return check_launch("closed bias");
-}
-
-int bias_rows(int batch, int groups, int heads, int cols, const void* src, const int64_t strides[5], void* dst, cudaStream_t stream) {
-  BiasRows p = describe_rows(batch, groups, heads, cols, src, strides, dst, ceil_div(cols, 8), 0);
   const int64_t total = int64_t(batch) * groups * heads * cols * p.words;
   if (total == 0) return OOPS_TA_OK;
   if (ceil_div(total, 256) > 0x7fffffffll) return fail(OOPS_TA_LIMIT_EXCEEDED, "bias of %lld words", (long long)total);

@@ -87,11 +87,18 @@ int packed_pair_mask(const uint8_t* tokens, const int64_t* token_offsets, int sa
 int packed_pair_mask_max_samples();
 // 16-bit bias of any strides (batch, group, head, query, key) to contiguous rows of ceil(cols / 8) 16-byte words.
 int bias_rows(int batch, int groups, int heads, int cols, const void* src, const int64_t strides[5], void* dst, cudaStream_t stream);
-// A row-shared bias in rows of `row` elements (a multiple of 8) that hold `fill` behind the last key, or, where `prefix` is given and all rows of a
-// sample that keep a key keep the same first ones, behind the last of those; uniform[sample] is their number then, else ~0 (0: none keeps any).  `prefix`: kept keys of every
-// mask row where they are its first ones, else ~0.
-int closed_bias(int batch, int heads, int cols, const void* src, const int64_t strides[5], void* dst, int row, uint16_t fill, const uint32_t* prefix,
-                int rows, uint32_t* uniform, cudaStream_t stream);
+// A row-shared bias (rows of whole 16-byte words) in rows of `row` elements (a multiple of 8) that hold `fill` behind the last key.
+// With `prefix` (kept keys of every mask row where they are its first ones, else ~0) the launch looks at a sample's rows first.  Where all that
+// keep a key keep the same first ones, found[sample] is their number (0: none keeps any) and the bias is closed behind those; else it is ~0.
+// Where `whole` (there is nothing to close behind the last key) such a sample is not copied, and none is if no row drops a key: `drops` says
+// that of every eight rows of the call.
+struct ClosedBiasLook {
+  const uint32_t *prefix = nullptr, *drops = nullptr;
+  int rows = 0, whole = 0;
+  uint32_t* found = nullptr;
+};
+int closed_bias(int batch, int heads, int cols, const void* src, int64_t s_b, int64_t s_h, int64_t s_q, void* dst, int row, uint16_t fill,
+                const ClosedBiasLook& look, cudaStream_t stream);
 // Layer normalisation over the last axis of (rows, width) activations (row strides in elements, contiguous rows);
 // weight / bias / gradients of them may be NULL; affine_dtype is the activation dtype or f32.
 uint64_t layer_norm_backward_workspace_bytes(int64_t rows, int width);

@@ -994,9 +994,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) ta_bwd_dkv_kernel(const 
 // issuer that acquires it fences once for all of them before its products read (N = 768: 1190 -> 1120 us with both).
 // A statistics warp of its own puts -log2(e) lse and -delta of a part's queries into a table, a tile at a time and a part ahead, where every
 // thread used to fetch both for every step (N = 768: 1036 -> 1004 us, 1024: 2934 -> 2842, 2048: 22.7 -> 22.0 ms), and makes the row dots where
-// that is hidden (kOwnDeltaCols).  Where all rows of a sample keep the same first keys
-// (kUniformCols) the bias is minus infinity behind those, key tiles behind them are not walked, the statistics warp clears dropped keys and
-// values in shared memory before any product may read them, and the element-wise warps know of no mask.  Through other masks they test
+// that is hidden (kOwnDeltaCols).  Where all rows of a sample keep the same first keys (closes_bias) the bias is minus infinity behind
+// those, key tiles behind them are not walked, the statistics warp clears dropped keys and values in shared memory before any product may
+// read them, and the element-wise warps know of no mask.  The launch that closes the bias looks at the mask first, and copies no sample that no
+// walk needs closed (an all-ones mask of 768 columns: 5.0 -> 3.7 us, 2048: 20.8 -> 14.8).  Through other masks they test
 // every probability, in a second copy of the step's body: a tile's way through the statistics warp, or bias words patched in
 // registers instead, cost short rows 10 to 20 %.
 // Halving the step between two sets of warps that run half a step apart was tried: the single P image couples them, 3 to 10 %
@@ -1053,7 +1054,7 @@ constexpr int kFSmemBytes = FSmem::total + 1024;
 static_assert(kFSmemBytes <= 232448, "fused reverse kernel: shared memory over the per-CTA limit");
 
 struct FParams {
-  CUtensorMap map_q, map_dout, map_k, map_v, map_bias;
+  CUtensorMap map_q, map_dout, map_k, map_v, map_bias, map_closed;
   oops_ta_pair dq, dk, dv;
   float* slots;     // [kFSlots][2][8][slot_keys][4] f32: sums of dK and dV carried from group to group (groups > 1)
   int64_t slot_keys;
@@ -1068,7 +1069,7 @@ struct FParams {
   int batch, rows, cols, heads, bias_groups, items;
   int q_tiles, k_tiles, groups, tiles_per_group;
   int write_dq, write_dk, write_dv;
-  int closed;  // the bias is minus infinity behind a ragged row's end
+  int closed;  // map_closed: the bias, minus infinity behind a ragged row's end or a token mask's, for walks without tests
   const uint32_t *prefix, *uniform;  // kept first keys of every row and of every sample's rows, null where nobody has looked
   float scale;
 };
@@ -1147,6 +1148,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
   if (warp == kFProducerWarp) {
     if (lane == 0) {
       bool ok = true;
+      const CUtensorMap* map_bias = PREFIX || (P.closed && P.cols % kTile != 0) ? &P.map_closed : &P.map_bias;
       for (FWalk<GROUPS> w(P, k_tiles); !w.done() && ok; w.next()) {
         const int s = w.s, kt = w.kt, qt = w.qt(), qs = s % 3;
         const int row = w.item / P.heads, h = w.item - row * P.heads, b = row / P.rows, r = row - b * P.rows;
@@ -1168,7 +1170,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
           if (!ok) break;
           mbar_expect_tx(bar(FSmem::bias_full), kFBias);
           for (int box = 0; box < 2; ++box)
-            tma_load_5d(smem_base + FSmem::bias + box * kBiasStep, &P.map_bias, bar(FSmem::bias_full), kt * kTile + box * 64,
+            tma_load_5d(smem_base + FSmem::bias + box * kBiasStep, map_bias, bar(FSmem::bias_full), kt * kTile + box * 64,
                         qt * kTile, h, P.bias_groups == 1 ? 0 : r, b);
         }
       }
@@ -2161,15 +2163,14 @@ bool fused_applies(const oops_ta_problem& p, const oops_ta_grads& g) {
   return g.dq.ptr != nullptr && (g.dk.ptr != nullptr || g.dv.ptr != nullptr);
 }
 
-// Rows from which a mask is asked whether its rows all keep the same first keys, or none (94 % of the tokens kept: 256 columns, two samples 124 -> 114 us and
-// a copy of 3, 200, two samples 90 -> 88 + 3, 384 187 -> 174 + 4, 512 379 -> 348 + 4, 1000 3171 -> 2748 + 12; 80 %: 768 1202 -> 980 + 11, 1000 3204 -> 2101 + 12,
-// 1400 7855 -> 4849 + 16).
-constexpr int kUniformCols = 192;
-
-// Whether the single-pass kernel gets a bias that is closed behind a ragged row's end (300 columns 134 -> 124 us, 500 347 -> 328, 700 962 -> 912; the
-// copy 3 to 5).
+// Rows and columns from which the single-pass kernel gets a bias that is closed behind a ragged row's end, or a token mask's.  Ragged: 300 columns 134 -> 124 us, 500
+// 347 -> 328, 700 962 -> 912, the copy 3 to 5.  Masks of 94 % of the tokens: 256 columns, two samples 125 -> 113 us and a copy of 3, 200, two samples 91 -> 88 + 3,
+// 384 186 -> 170 + 3, 512 375 -> 338 + 4, 1000 3175 -> 2778 + 7; of 80 %: 768 1202 -> 980 + 11, 1400 7855 -> 4849 + 16.  A copy that only tests walk over
+// is worth its time in ragged rows, whose own pitch is no multiple of a tile's 128 bytes (scattered keys, 500 columns 399 -> 394 + 4 - 2.5).
+constexpr int kClosedCols = 192, kClosedRows = 64;
 bool closes_bias(const oops_ta_problem& p, const oops_ta_grads& g) {
-  return fused_applies(p, g) && bias_closes(p) && (p.cols % kTile != 0 ? p.cols >= 192 : p.mask && p.batch <= kUniformSamples && p.cols >= kUniformCols) && p.rows >= 64;
+  return fused_applies(p, g) && bias_closes(p) && (p.cols % kTile != 0 || (p.mask && p.batch <= kUniformSamples)) && p.cols >= kClosedCols &&
+         p.rows >= kClosedRows;
 }
 
 // What it takes behind the rest of the scratch: a word per sample, the bias.
@@ -2262,15 +2263,18 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
     if (!status) status = encode_pair(&P.map_v, p, p.v, kTile, "value");
     P.closed = closes_bias(p, g) && p.workspace_bytes >= layout.closed + closing_bytes(p) && ((reinterpret_cast<uintptr_t>(base) + layout.closed) & 15) == 0;
     if (!status && P.closed) {
-      if (live && p.batch <= kUniformSamples && p.cols >= kUniformCols) {
-        P.prefix = live + 2 * int64_t(p.batch) * p.rows;
-        P.uniform = reinterpret_cast<uint32_t*>(base + layout.closed);
+      ClosedBiasLook look;
+      if (live && p.batch <= kUniformSamples) {
+        P.prefix = look.prefix = live + 2 * int64_t(p.batch) * p.rows;
+        P.uniform = look.found = reinterpret_cast<uint32_t*>(base + layout.closed);
+        look.drops = live + 3 * int64_t(p.batch) * p.rows;
+        look.rows = p.rows;
+        look.whole = p.cols % kTile == 0;
       }
       P.logits = Logits(p);
-      status = close_bias(&P.map_bias, p, base + layout.closed + align256(uint64_t(p.batch) * 4), "bias", stream, P.prefix,
-                          const_cast<uint32_t*>(P.uniform));
+      status = close_bias(&P.map_closed, p, base + layout.closed + align256(uint64_t(p.batch) * 4), "bias", stream, look);
     }
-    else if (!status && has_bias)
+    if (!status && has_bias && (!P.closed || p.cols % kTile == 0))  // (over ragged rows every walk takes the closed one)
       status = encode_bias(&P.map_bias, p, p.bias, p.bias_sq, p.bias_sh, p.bias_sg, p.bias_sb, kTile, "bias");
     if (status) return status;
     P.dq = g.dq;

@@ -137,11 +137,10 @@ bool bias_closes(const oops_ta_problem& p) {
 }
 uint64_t closed_bias_bytes(const oops_ta_problem& p) { return uint64_t(p.batch) * p.heads * p.cols * closed_row(p) * 2; }
 
-int close_bias(CUtensorMap* map, const oops_ta_problem& p, void* scratch, const char* what, cudaStream_t stream, const uint32_t* prefix = nullptr,
-               uint32_t* uniform = nullptr) {
-  const int64_t strides[5] = {p.bias_sb, p.bias_sg, p.bias_sh, p.bias_sq, p.bias_sk}, row = closed_row(p), plane = p.cols * row;
-  const int status = closed_bias(p.batch, p.heads, p.cols, p.bias, strides, scratch, int(row), p.dtype == OOPS_TA_BF16 ? 0xff80 : 0xfc00, prefix,
-                                 p.rows, uniform, stream);
+int close_bias(CUtensorMap* map, const oops_ta_problem& p, void* scratch, const char* what, cudaStream_t stream, const ClosedBiasLook& look = {}) {
+  const int64_t row = closed_row(p), plane = p.cols * row;
+  const int status = closed_bias(p.batch, p.heads, p.cols, p.bias, p.bias_sb, p.bias_sh, p.bias_sq, scratch, int(row),
+                                 p.dtype == OOPS_TA_BF16 ? 0xff80 : 0xfc00, look, stream);
   return status ? status : encode_bias(map, p, scratch, row, plane, plane * p.heads, plane * p.heads, kTile, what, int(row));
 }
 
@@ -171,7 +170,8 @@ struct Logits {
 };
 
 // A mask whose rows may all keep the same first keys (or none), as masks of tokens do: whether they do is found out on the device, and the bias is
-// closed behind those keys.  `uniform` has a word per sample.
+// closed behind those keys.  `uniform` has a word per sample, `most` is the largest of them.  (A word a lane: a loop over more costs the walks behind it 0.5 %,
+// and one that lanes leave apart has them compiled for divergence, 2 to 7 %.)
 constexpr int kUniformSamples = 32;
 __device__ __forceinline__ bool uniform_prefix(const uint32_t* uniform, int batch, int lane, uint32_t& most) {
   const uint32_t v = lane < batch ? *reinterpret_cast<const volatile uint32_t*>(uniform + lane) : 0u;
