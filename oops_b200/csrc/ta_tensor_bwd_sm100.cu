@@ -2149,10 +2149,11 @@ uint64_t fused_slot_bytes(const oops_ta_problem& p) {
   return align256(uint64_t(kFSlots) * 2 * fused_slot_keys(p) * kHeadDim * sizeof(float));
 }
 
-// Rows from which the single-pass kernel makes the row dots itself.  Its statistics warp takes some 6000 clocks a query tile for them, which
-// are hidden under the steps where a row has many: 768 columns 1023 + 51 (prepare_kernel) -> 1040 + 5 us, 700 950 + 44 -> 970; 512
-// 329 + 24 -> 350, 256 (two samples) 104 + 11 -> 160.  In rows of several groups the first tiles delay a CTA's start (1024: 2842 + 84 -> 3149).
-constexpr int kOwnDeltaCols = 4 * kTile;
+// Columns, and items per CTA, from which the single-pass kernel makes the row dots itself.  Its statistics warp takes some 6000 clocks a query tile for them, which
+// are hidden under the steps where a row has many: 768 columns 1008 + 50 (prepare_kernel) -> 1032 us, 520 505 + 25 -> 520; 512
+// 329 + 24 -> 350, 256 (two samples) 104 + 11 -> 160.  In rows of several groups the first tiles delay a CTA's start (1024: 2842 + 84 -> 3149), and so do
+// those of its first item: 768 columns, 1 item a CTA 52 + 2 -> 63, 4 items 198 + 10 -> 215, 6 293 + 16 -> 311, 8 434 + 22 -> 454; 520, 8 306 + 15 -> 320.
+constexpr int kOwnDeltaCols = 4 * kTile, kOwnDeltaItems = 8;
 
 // The single-pass kernel serves calls that want dQ together with dK or dV and no per-row bias gradient, on rows
 // of up to 4096 columns (32 key tiles, one bit each in the words that describe a row's mask).
@@ -2237,7 +2238,8 @@ int run_backward(const oops_ta_problem& p, const oops_ta_pair& out, const oops_t
   // whatever the workspace holds (a second call with a mask: 159 -> 169 us at 96 rows of 768 columns, 1165 -> 1168 at 768).
   const bool fused = fused_applies(p, g);
   const bool words16 = (reinterpret_cast<uintptr_t>(out.ptr) & 15) == 0 && out.sb % 8 == 0 && out.sr % 8 == 0 && out.sc % 8 == 0 && out.sh % 8 == 0;
-  const bool own_delta = fused && words16 && (p.flags & OOPS_TA_FLAG_REUSE_DELTA) == 0 && p.cols > kOwnDeltaCols && fused_groups(p) == 1;
+  const bool own_delta = fused && words16 && (p.flags & OOPS_TA_FLAG_REUSE_DELTA) == 0 && p.cols > kOwnDeltaCols && fused_groups(p) == 1 &&
+                         int64_t(p.batch) * p.rows * p.heads >= int64_t(kOwnDeltaItems) * sm_count();
   const int64_t total = (p.flags & OOPS_TA_FLAG_REUSE_DELTA) != 0 || own_delta ? 0 : int64_t(p.batch) * p.rows * p.heads * p.cols;
   const int64_t cells = p.heads > 0 ? total / p.heads : 0;
   const unsigned delta_blocks = (unsigned)ceil_div(cells, 64);

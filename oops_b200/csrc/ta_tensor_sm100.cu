@@ -757,9 +757,12 @@ bool tensor_forward_applies(const oops_ta_problem& p) {
   return ctas <= 0x7fffffffll;
 }
 
-// A ragged last step costs a call of 1000 columns 4.5 % (1565 us, 1024: 1530), one of 500 5 %; the copy 3 to 6 us.
+// Rows and columns from which a ragged row's bias is closed: 390 columns 170 -> 162 us with the copy, 500 239 -> 228, 1000 1594 -> 1498; all-ones masks 170 -> 167,
+// 238 -> 234, 1578 -> 1541.  A token mask has no use for the copy and pays it (390 columns 145.4 -> 146.8, 700 541 -> 545, 1000 as before), and scattered keys
+// (214 -> 216); to look at the mask's first row before the copy is made cost them more (148.1, 217).
+constexpr int kClosedCols = 384, kClosedRows = 128, kClosedMaxCols = 4096;
 uint64_t tensor_forward_workspace(const oops_ta_problem& p) {
-  return bias_closes(p) && p.cols % kKeys != 0 && p.cols >= 384 && p.cols <= 4096 && p.rows >= 128 ? closed_bias_bytes(p) : 0;
+  return bias_closes(p) && p.cols % kKeys != 0 && p.cols >= kClosedCols && p.cols <= kClosedMaxCols && p.rows >= kClosedRows ? closed_bias_bytes(p) : 0;
 }
 
 namespace {
