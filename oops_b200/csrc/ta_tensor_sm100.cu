@@ -13,7 +13,9 @@
 // or more in the first 48 columns (or a NaN), or a logit of 10 or more in the last 16, sends the warp back over the step, which still
 // stands in tensor memory, to raise the reference and rescale the accumulators.  Probabilities therefore stay below 2^10, inside the
 // f32, bf16 and f16 ranges.  With that look the scores are given back before the exponentials of the last 16 columns, and the next
-// score product runs under them (N = 768: 711 -> 681 us, 512: 233 -> 225, 2048: 11.6 -> 11.2 ms; no bit of a result changed).
+// score product runs under them (N = 768: 711 -> 683 us, 512: 234 -> 222, 2048: 11.6 -> 11.23 ms; an all-ones mask, 768: 726 -> 702).  A step that
+// tests kept bits looks at the sum of all its columns and gives its scores back with its probabilities: there the look at the last logits costs more
+// than the lead of the product gives (scattered keys of 768 columns 936 us, without it 924), and a report of its own for the scores 1 %.
 // Against a maximum per step this saves the comparisons, and above all the wait: no exponential depended on the last
 // score of a step any more, scores need not be held in registers, and an exponential costs 5 instead of 9.5 issue slots.
 // What bounds it: the element-wise warps' streams, with the special-function unit (63 %; one ex2 per score at 16 per clock and SM,
@@ -70,7 +72,8 @@ struct FwdSmem {
   static constexpr int num_bars = q_empty + 2;
   static constexpr int tmem_slot = bars + num_bars * 8;
   static constexpr int abort_flag = tmem_slot + 4;
-  static constexpr int drop_flags = abort_flag + 4;               // [8] per-warp: the mask drops a key of this row
+  static constexpr int lost_flag = abort_flag + 4;                // a row of a walk over a closed bias came out as NaN
+  static constexpr int drop_flags = lost_flag + 4;               // [8] per-warp: the mask drops a key of this row
   static constexpr int step_count = drop_flags + 32;
   static constexpr int full_count = step_count + 4;
   static constexpr int steps = full_count + 4;                    // [2][256] u16: full steps, other steps with a kept key
@@ -104,7 +107,7 @@ struct FwdParams {
 };
 
 // What sends a step's warp back for a new reference: the sum of the probabilities of the first 48 columns, or a base-2 logit of the last 16 (whose
-// probabilities are not known yet when the scores are given back).  No probability reaches 2^10 then, no step's sum 2^15.
+// probabilities are not known yet when the scores are given back); in a step with tests the sum of all.  No probability reaches 2^10 then, no step's sum 2^15.
 constexpr float kStepSumLimit = 1024.f, kLastColumnsLimit = 10.f;
 
 // Where item `idx` lies: query item fastest, then head, row (or pair of rows), batch.
@@ -495,7 +498,6 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
     if (PERSIST) at = fwd_item<ROWS>(P, item);  // (not held through the steps)
     const int r = row_of(w), h = at.h, b = at.b, q_index = first_query(w) + t;
     const bool stored = q_index < P.cols && (!PERSIST || !ROWS || at.r0 + w < P.rows);
-    const bool none = PLAIN && HAS_BIAS && P.closed && stored && isnan(l_run) && P.logits.all_minus_infinity<T>(b, r, h, q_index, P.cols);
     // Gated epilogue: the thread's 32 gate logits are requested before the wait for the last product, so that their
     // trip from global memory runs under it (the words are not touched until the output row is ready).
     uint4 gate_words[4] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
@@ -516,11 +518,7 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
         tmem_loaded(acc);
       }
       if (stored) {
-        if (none) {
-          l_run = 0.f;
-#pragma unroll
-          for (int n = 0; n < 32; ++n) acc[n] = 0u;
-        }
+        if (PLAIN && HAS_BIAS && P.closed && isnan(l_run)) *reinterpret_cast<volatile int*>(smem_gen + Smem::lost_flag) = 1;
         const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
         uint32_t o2[16];
 #pragma unroll
@@ -577,6 +575,27 @@ __device__ __forceinline__ void fwd_walk(const FwdParams& P, uint32_t smem_base,
   }
 }
 
+// A query that holds an infinity has NaN for the zeros of keys that the bias closes.  A row whose kept logits are minus infinity, all of
+// them, has no probability all the same: zeros (its log-sum-exp is 0 already).  Asked behind a walk in which a row came out as NaN.
+template <typename T, bool GATED, bool ROWS, bool PERSIST>
+__device__ __forceinline__ void clear_lost_rows(const FwdParams& P, int tid, int warp) {
+  const int w = warp >> 2;
+  for (int item = int(blockIdx.x); warp < 8 && item < (PERSIST ? P.items : int(blockIdx.x) + 1); item += int(gridDim.x)) {
+    const FwdItem i = fwd_item<ROWS>(P, item);
+    const int r = ROWS ? i.r0 + w : i.r0, q = (ROWS ? i.q0 : i.q0 + w * kTile) + (tid & (kTile - 1));
+    if (r >= P.rows || q >= P.cols) continue;
+    T* out = reinterpret_cast<T*>(P.out) + i.b * P.o_sb + int64_t(r) * P.o_sr + int64_t(q) * P.o_sc + i.h * P.o_sh;
+    if (!isnan(float(*out)) || !P.logits.all_minus_infinity<T>(i.b, r, i.h, q, P.cols)) continue;
+    const T* gate = reinterpret_cast<const T*>(P.gate) + i.b * P.g_sb + int64_t(r) * P.g_sr + int64_t(q) * P.g_sc + i.h * P.g_sh;
+    T* plain = reinterpret_cast<T*>(P.plain) + i.b * P.p_sb + int64_t(r) * P.p_sr + int64_t(q) * P.p_sc + i.h * P.p_sh;
+#pragma unroll 1
+    for (int c = 0; c < kHeadDim; ++c) {
+      out[c] = GATED && isnan(float(gate[c])) ? gate[c] : T(0.f);
+      if (GATED && P.plain) plain[c] = T(0.f);
+    }
+  }
+}
+
 template <typename T, bool HAS_BIAS, bool GATED, bool ROWS, bool PERSIST>
 __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_constant__ FwdParams P) {
   using Smem = FwdSmem<ROWS>;
@@ -616,7 +635,10 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
       if (i >= Smem::p_full && i < Smem::pv_done) arrivals = kTile / 32;  // (s_free among them)
       mbar_init(bar(i), arrivals);
     }
-    if (lane == 0) *abort_flag = 0;
+    if (lane == 0) {
+      *abort_flag = 0;
+      *reinterpret_cast<volatile int*>(smem_gen + Smem::lost_flag) = 0;
+    }
     fence_barrier_init();
     __syncwarp();
     if (lane == 0) {
@@ -698,11 +720,23 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
   }
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  if (!listed && !ragged)
+  // (Two ends of the kernel, and the question about lost rows behind the walk that asks it: with one end, or the question in the output, what the
+  // compiler makes of the listed walk is 1 to 3 % slower.  A persistent kernel has one end: 300 columns 78.3 -> 77.8 us.)
+  auto any_lost = [&]() { return HAS_BIAS && P.closed && *reinterpret_cast<volatile int*>(smem_gen + Smem::lost_flag) != 0; };
+  if (!listed && !ragged) {
     fwd_walk<T, HAS_BIAS, GATED, ROWS, PERSIST, true>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, at, n_tiles, false);
-  else
+    if constexpr (!PERSIST) {
+      teardown(abort_flag, tmem_base, 9, kFwdTmemCols);
+      if (any_lost()) clear_lost_rows<T, GATED, ROWS, PERSIST>(P, tid, warp);
+    }
+  } else {
     fwd_walk<T, HAS_BIAS, GATED, ROWS, PERSIST, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, at, n_tiles, listed);
-  teardown(abort_flag, tmem_base, 9, kFwdTmemCols);
+    if constexpr (!PERSIST) teardown(abort_flag, tmem_base, 9, kFwdTmemCols);
+  }
+  if constexpr (PERSIST) {
+    teardown(abort_flag, tmem_base, 9, kFwdTmemCols);
+    if (any_lost()) clear_lost_rows<T, GATED, ROWS, PERSIST>(P, tid, warp);
+  }
 }
 
 // Self-test of the bounded wait: one CTA allocates tensor memory and waits, with a one-millisecond limit, on a barrier

@@ -89,3 +89,23 @@ def test_rows_whose_logits_are_minus_infinity(cuda, rows, n, masked):
         got[0, 0, 6] = 0
         assert torch.isfinite(got).all()
     assert torch.isfinite(dv[0, 1:]).all()
+
+
+@pytest.mark.parametrize("rows,n", [(128, 399), (160, 450), (128, 700)])
+def test_gated_rows_whose_logits_are_minus_infinity(cuda, rows, n):
+    """The same through the gated form, whose gate then holds a NaN or none; one item a CTA and several."""
+    from oops_b200 import triangle_attention_gated
+
+    gen = torch.Generator().manual_seed(n)
+    q, k, v, gate = (torch.randn(1, rows, n, 4, 32, generator=gen).to(torch.float16) for _ in range(4))
+    bias = torch.randn(1, 1, 4, n, n, generator=gen).to(torch.float16)
+    k[0, 1, :, 2, 9] = -k[0, 1, :, 2, 9].abs() - 1.0
+    empty = [n // 2, n - 1, 3]
+    q[0, 1, empty, 2, 9] = INF
+    gate[0, 1, 3, 2, 5] = NAN
+    with torch.no_grad():
+        out = triangle_attention_gated(*(t.to(cuda) for t in (q, k, v, gate)), None, bias.to(cuda)).cpu()
+    assert bool(torch.isnan(out[0, 1, 3, 2, 5]))
+    out[0, 1, 3, 2, 5] = 0
+    assert not out[0, 1, empty, 2].any()
+    assert torch.isfinite(out).all()
