@@ -1093,8 +1093,9 @@ __device__ __forceinline__ void store_zeros(const oops_ta_pair& t, const FParams
 // The walk over a CTA's steps, identical in every role of the kernel: parts outermost, then key tiles, then query tiles.
 // A part is a group of query tiles of the CTA's one item, or, where a row is a single group, a whole item of the several
 // that the CTA works through.  Ring slots and barrier phases count steps, key tiles and parts.  (Trip counts come from the
-// launch parameters alone: with counts read from memory the compiler takes the loops for divergent and guards every
-// branch in them, which cost the kernel 8 %.)
+// launch parameters: with counts read from memory the compiler takes the loops for divergent and guards every
+// branch in them, which cost the kernel 8 %.  The key tiles of a token mask are the exception: they come from memory once per CTA, through a shuffle
+// that makes them one value for the warp, and without a loop over lanes before it.)
 template <bool GROUPS>
 struct FWalk {
   int tiles_per_group, q_tiles, k_tiles, parts, item_step;
@@ -1128,20 +1129,17 @@ struct FWalk {
 };
 
 // GROUPS: rows of several groups of query tiles.  BITS: some key may be dropped, by the mask or because the last key tile
-// is ragged.
+// is ragged, and every probability is tested.  PREFIX: rows keep the first keys of their sample's prefix, or none, in `k_tiles` key tiles; dropped
+// keys are cleared before a product reads them.  DIRECT: rows of one tile (below).  `suspects`: rows without a probability, perhaps.
 template <typename T, bool HAS_BIAS, bool GROUPS, bool BITS, bool PREFIX, bool DIRECT>
 __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base, uint8_t* smem_gen, volatile int* abort_flag,
                                            uint32_t tmem_base, int tid, int warp, int lane, int k_tiles, bool& suspects) {
   auto bar = [&](int index) -> uint32_t { return smem_base + FSmem::bars + index * 8; };
   const bool has_mask = BITS && P.mask != nullptr;
-  constexpr bool prefixes = PREFIX;
   static_assert(!PREFIX || !BITS);
-  // PREFIX: rows keep the first keys of their sample's prefix, or none, in `k_tiles` key tiles; dropped keys are
-  // cleared before a product reads them.
   auto request_prefix = [&](int item) -> uint32_t {  // every lane's copy; an item ahead of its use
     return PREFIX && item < P.items ? *reinterpret_cast<const volatile uint32_t*>(P.prefix + item / P.heads) : 0u;
   };
-  constexpr bool has_bits = BITS;
   // tensor-memory columns
   constexpr int kSCol = 0, kDpCol = 128, kDkCol = 256, kDvCol = 288, kDqCol = 320;
 
@@ -1312,15 +1310,15 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     };
     uint32_t item_kept = 0, next_kept = request_prefix(int(blockIdx.x));
     auto last = w;  // the key tile before
-    if (!w.done()) tile_stats(0, w.item, w.first, 0, prefixes && __shfl_sync(0xffffffffu, next_kept, 0) == 0, false);
+    if (!w.done()) tile_stats(0, w.item, w.first, 0, PREFIX && __shfl_sync(0xffffffffu, next_kept, 0) == 0, false);
     for (; !w.done() && ok; last = w, w.next_tile()) {
       const int kt = w.kt;
-      if (prefixes && kt == 0) {
+      if (PREFIX && kt == 0) {
         item_kept = __shfl_sync(0xffffffffu, next_kept, 0);
         next_kept = request_prefix(GROUPS ? w.item : w.item + int(gridDim.x));
       }
       const int slot = w.ktc & 1;
-      if (prefixes) {
+      if (PREFIX) {
         // (Every tile passes here, with dropped keys or not: this warp is then neither a phase of a slot behind nor two ahead.)
         ok = mbar_wait_warp(bar(FSmem::kv_full + slot), (w.ktc >> 1) & 1, abort_flag);
         if (!ok) break;
@@ -1347,7 +1345,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
         from = last.kt;
         to = last.kt == k_tiles - 1 ? ahead.nq : min(last.kt + 1, ahead.nq);
       }
-      const bool dead = prefixes && __shfl_sync(0xffffffffu, ahead.part == w.part ? item_kept : next_kept, 0) == 0;
+      const bool dead = PREFIX && __shfl_sync(0xffffffffu, ahead.part == w.part ? item_kept : next_kept, 0) == 0;
 #pragma unroll 1
       for (int qi = from; qi < to && ok; ++qi) tile_stats(ahead.part, ahead.item, ahead.first, qi, dead, qi == 0 && ahead.part >= 2);
     }
@@ -1445,7 +1443,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     float lse_next = 0.f, delta_next = 0.f;
     if (DIRECT) fetch_stats(w, lse_next, delta_next);
     const uint8_t* mask_row = has_mask ? mask_row_of(w.item) : nullptr;  // of the key tile to come
-    uint32_t keep_raw = has_bits ? fetch_keep(mask_row, w) : 0u, bits = 0xffffffffu;
+    uint32_t keep_raw = BITS ? fetch_keep(mask_row, w) : 0u, bits = 0xffffffffu;
     bool ok = true;
     if (GROUPS && sm_id >= uint32_t(kFSlots)) {  // no scratch slot for this SM id: give up like a wait that ran out
       *abort_flag = 1;
@@ -1458,7 +1456,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     int last_item = 0, last_part = 0, last_first = 0, last_kt = 0;  // of the previous step
     for (; !w.done() && ok; last_item = w.item, last_part = w.part, last_first = w.first, last_kt = w.kt, w.next()) {
       const int s = w.s, kt = w.kt, qi = w.qi, buf = s & 1, table = (w.part & 1) * kFMaxQTiles + qi;
-      if (has_bits && qi == 0) {
+      if (BITS && qi == 0) {
         bits = __ballot_sync(0xffffffffu, keep_raw != 0);
         FWalk<GROUPS> ahead = w;
         ahead.next_tile();
