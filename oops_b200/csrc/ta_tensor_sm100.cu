@@ -666,6 +666,9 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
     bool dropped_any = false;
     if (ring < n_rings) {
       const uint8_t* mask_row = has_mask ? P.mask + b * P.m_sb + int64_t(row_of(ring)) * P.m_sr : nullptr;
+      // (Two turns of bytes under way: with the pair axes exchanged a lane's byte is a sector of its own, and four take 992 columns, 77 % of the tokens
+      // kept, from 1056 to 1084 us; one takes an all-ones mask of 768 from 702 to 720.)
+#pragma unroll 2
       for (int word = ROWS ? warp & 3 : warp; word < P.k_steps * 2; word += ROWS ? 4 : 8) {
         const int key = word * 32 + lane;
         bool keep = key < P.cols;
