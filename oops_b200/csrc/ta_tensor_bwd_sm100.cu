@@ -1048,7 +1048,8 @@ struct FSmem {
   static constexpr int num_bars = kv_ready + 2;
   static constexpr int tmem_slot = bars + num_bars * 8;
   static constexpr int abort_flag = tmem_slot + 4;
-  static constexpr int total = abort_flag + 4;
+  static constexpr int suspects = abort_flag + 4;      // query tiles with a row without a probability, perhaps
+  static constexpr int total = suspects + 4;
 };
 constexpr int kFSmemBytes = FSmem::total + 1024;
 static_assert(kFSmemBytes <= 232448, "fused reverse kernel: shared memory over the per-CTA limit");
@@ -1130,10 +1131,10 @@ struct FWalk {
 
 // GROUPS: rows of several groups of query tiles.  BITS: some key may be dropped, by the mask or because the last key tile
 // is ragged, and every probability is tested.  PREFIX: rows keep the first keys of their sample's prefix, or none, in `k_tiles` key tiles; dropped
-// keys are cleared before a product reads them.  DIRECT: rows of one tile (below).  `suspects`: rows without a probability, perhaps.
+// keys are cleared before a product reads them.  DIRECT: rows of one tile (below).
 template <typename T, bool HAS_BIAS, bool GROUPS, bool BITS, bool PREFIX, bool DIRECT>
 __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base, uint8_t* smem_gen, volatile int* abort_flag,
-                                           uint32_t tmem_base, int tid, int warp, int lane, int k_tiles, bool& suspects) {
+                                           uint32_t tmem_base, int tid, int warp, int lane, int k_tiles) {
   auto bar = [&](int index) -> uint32_t { return smem_base + FSmem::bars + index * 8; };
   const bool has_mask = BITS && P.mask != nullptr;
   static_assert(!PREFIX || !BITS);
@@ -1241,6 +1242,8 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
     // Statistics of a part's queries, a tile at a time and a part ahead: -log2(e) lse, and -delta, which is rowsum(O * dO) where the
     // caller has not left it.  Four lanes share a query, eight channels each.
     bool ok = true;
+    // Query tiles with a row that has no probability, perhaps (the forward pass leaves such a row a log-sum-exp of 0): looked at behind the walk.
+    uint32_t suspects = 0;
     // `dead`: no key is kept, every probability, and dS, is zero.  `in_use`: the table holds a part that has to be through first (the words are
     // under way meanwhile).
     auto tile_stats = [&](int part, int item, int first, int qi, bool dead, bool in_use) {
@@ -1262,7 +1265,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
         }
         if (!table_free()) return;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) suspects |= lse[j] == 0.f && !dead;
+        for (int j = 0; j < 4; ++j) suspects |= lse[j] == 0.f && !dead ? 1u << (first + qi) : 0u;
 #pragma unroll
         for (int j = 0; j < 4; ++j) sts_f2_at(table + (j * 32 + lane) * 8, dead ? -INFINITY : -lse[j] * kLog2e, dead ? 0.f : -delta[j]);
       } else {
@@ -1293,7 +1296,7 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
             if ((lane >> 3) == i) own = mine;
           }
           if (q < P.cols) P.delta[stat + q] = own;
-          suspects |= lse == 0.f && !dead;
+          suspects |= lse == 0.f && !dead ? 1u << (first + qi) : 0u;
           sts_f2_at(table + (j + lane) * 8, dead ? -INFINITY : -lse * kLog2e, dead ? 0.f : -own);
         }
       }
@@ -1348,6 +1351,10 @@ __device__ __forceinline__ void fused_walk(const FParams& P, uint32_t smem_base,
       const bool dead = PREFIX && __shfl_sync(0xffffffffu, ahead.part == w.part ? item_kept : next_kept, 0) == 0;
 #pragma unroll 1
       for (int qi = from; qi < to && ok; ++qi) tile_stats(ahead.part, ahead.item, ahead.first, qi, dead, qi == 0 && ahead.part >= 2);
+    }
+    if (HAS_BIAS && !BITS) {  // (tests drop what is dropped)
+      suspects = __reduce_or_sync(0xffffffffu, suspects);
+      if (lane == 0) *reinterpret_cast<volatile uint32_t*>(smem_gen + FSmem::suspects) = suspects;
     }
   } else if (warp < 16) {
     const int wg = warp >> 2;  // 32 of the step's 128 keys
@@ -1658,7 +1665,10 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
       if (i == FSmem::dkv_free) arrivals = 8;
       mbar_init(bar(i), arrivals);
     }
-    if (lane == 0) *abort_flag = 0;
+    if (lane == 0) {
+      *abort_flag = 0;
+      *reinterpret_cast<volatile uint32_t*>(smem_gen + FSmem::suspects) = 0;
+    }
     fence_barrier_init();
   }
   if (warp == kFScoreWarp) {
@@ -1669,10 +1679,10 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  bool plain = !MASKED, suspects = false;  // suspects: rows without a probability, perhaps (statistics warp)
+  bool plain = !MASKED;
   if (MASKED && P.mask && (P.cols % kTile == 0 || P.closed)) plain = keeps_all(P.live, P.batch * P.rows, lane);
   if (plain) {
-    fused_walk<T, HAS_BIAS, GROUPS, false, false, DIRECT>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, P.k_tiles, suspects);
+    fused_walk<T, HAS_BIAS, GROUPS, false, false, DIRECT>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, P.k_tiles);
   } else if constexpr (MASKED) {
     uint32_t most = 0;
     const bool uniform = HAS_BIAS && !DIRECT && P.uniform && uniform_prefix(P.uniform, P.batch, lane, most);
@@ -1683,22 +1693,27 @@ __global__ void __launch_bounds__(kFThreads, 1) ta_bwd_fused_kernel(const __grid
       if (P.write_dv) store_zeros<T>(P.dv, P, int(blockIdx.x), 0, tid, kFThreads);
     } else if (uniform)
       fused_walk<T, HAS_BIAS, GROUPS, false, HAS_BIAS, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane,
-                                                       __shfl_sync(0xffffffffu, max(1, int(most + kTile - 1) / kTile), 0), suspects);
+                                                       __shfl_sync(0xffffffffu, max(1, int(most + kTile - 1) / kTile), 0));
     else
-      fused_walk<T, HAS_BIAS, GROUPS, true, false, DIRECT>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, P.k_tiles, suspects);
+      fused_walk<T, HAS_BIAS, GROUPS, true, false, DIRECT>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, P.k_tiles);
   }
   teardown(abort_flag, tmem_base, kFScoreWarp);
-  if (HAS_BIAS && !DIRECT && P.closed && suspects && P.write_dq) {
+  if (HAS_BIAS && !DIRECT && P.closed && P.write_dq) {
     // A query that holds an infinity has NaN for the zeros of keys that the bias closes.  A row whose kept logits are minus infinity, all of
-    // them, has no probability (the forward pass leaves it a log-sum-exp of 0) and no gradient all the same; its dQ stands by now.
-    for (int item = int(blockIdx.x); item < P.items; item += GROUPS ? P.items : int(gridDim.x)) {
+    // them, has no probability and no gradient all the same; its dQ stands by now.  A warp takes 32 queries of an item.
+    const uint32_t suspects = *reinterpret_cast<volatile uint32_t*>(smem_gen + FSmem::suspects);
+    const int item_step = GROUPS ? P.items : int(gridDim.x), chunks = (P.cols + 31) / 32;
+    int item = int(blockIdx.x);
+    for (int at = warp; suspects != 0 && item < P.items; at += kFThreads / 32) {
+      for (; at >= chunks && item < P.items; at -= chunks) item += item_step;
+      const int q = at * 32 + lane;
+      if (item >= P.items || (suspects >> (at / 4) & 1u) == 0 || q >= P.cols) continue;
       const int row = item / P.heads, h = item - row * P.heads, b = row / P.rows, r = row - b * P.rows;
+      T* dq = reinterpret_cast<T*>(P.dq.ptr) + b * P.dq.sb + int64_t(r) * P.dq.sr + int64_t(q) * P.dq.sc + h * P.dq.sh;
+      if (P.lse[int64_t(item) * P.cols + q] != 0.f || !isnan(float(*dq))) continue;
       const int kept = P.prefix && P.uniform[b] != ~0u ? int(P.prefix[row]) : P.cols;
-      T* dq = reinterpret_cast<T*>(P.dq.ptr) + b * P.dq.sb + int64_t(r) * P.dq.sr + h * P.dq.sh;
-      for (int q = lane; q < P.cols; q += 32) {
-        if (P.lse[int64_t(item) * P.cols + q] != 0.f || !P.logits.all_minus_infinity<T>(b, r, h, q, kept)) continue;
-        for (int c = 0; c < kHeadDim; ++c) dq[q * P.dq.sc + c] = T(0.f);
-      }
+      if (!P.logits.all_minus_infinity<T>(b, r, h, q, kept)) continue;
+      for (int c = 0; c < kHeadDim; ++c) dq[c] = T(0.f);
     }
   }
 }

@@ -146,6 +146,7 @@ int close_bias(CUtensorMap* map, const oops_ta_problem& p, void* scratch, const 
 
 // What a walk over a closed bias asks about a row that came out as NaN: a query that holds an infinity has NaN for the zeros of the keys that
 // the bias closes, but where its kept logits are minus infinity, all of them, it has no probability (the first keys answer it otherwise).
+// (Only a call with a closed bias has the operands here.)
 struct Logits {
   oops_ta_pair q, k;
   const void* bias;  // row-shared, keys contiguous

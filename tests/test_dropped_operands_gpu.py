@@ -109,3 +109,23 @@ def test_gated_rows_whose_logits_are_minus_infinity(cuda, rows, n):
     out[0, 1, 3, 2, 5] = 0
     assert not out[0, 1, empty, 2].any()
     assert torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("rows,n,pad", [(64, 200, 20), (128, 399, 130), (64, 700, 60), (64, 801, 100)])
+def test_padding_through_the_bias(cuda, rows, n, pad):
+    """Padded queries and keys under a bias of minus infinity, without a mask: what the call without them gives, and zeros."""
+    gen = torch.Generator().manual_seed(n)
+    q, k, v, up = (torch.randn(1, rows, n, 2, 32, generator=gen).to(torch.bfloat16) for _ in range(4))
+    bias = torch.randn(1, 1, 2, n, n, generator=gen).to(torch.bfloat16)
+    kept = n - pad
+    want = oracle.forward_backward(*(t[:, :, :kept] for t in (q, k, v)), None, bias[..., :kept, :kept], up[:, :, :kept])
+    bias[..., kept:, :], bias[..., kept:] = -INF, -INF
+    leaves = [t.to(cuda).requires_grad_(True) for t in (q, k, v, bias)]
+    out = triangle_attention(*leaves[:3], None, leaves[3])
+    got = [t.detach().float().cpu() for t in (out, *torch.autograd.grad(out, leaves, up.to(cuda)))]
+    for name, g, ref in zip(("out", "dq", "dk", "dv"), got, want):
+        error = float((g[:, :, :kept] - ref).abs().max())
+        assert error <= 2e-2 * max(1.0, float(ref.abs().max())), (name, error)
+        assert not g[:, :, kept:].any(), name
+    error = float((got[4][..., :kept, :kept] - want[4]).abs().max())
+    assert error <= 2e-2 * max(1.0, float(want[4].abs().max())), error
