@@ -667,8 +667,8 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
     if (ring < n_rings) {
       const uint8_t* mask_row = has_mask ? P.mask + b * P.m_sb + int64_t(row_of(ring)) * P.m_sr : nullptr;
       // (Two turns of bytes under way: with the pair axes exchanged a lane's byte is a sector of its own, and four take 992 columns, 77 % of the tokens
-      // kept, from 1056 to 1084 us; one takes an all-ones mask of 768 from 702 to 720.)
-#pragma unroll 2
+      // kept, from 1056 to 1084 us; one takes an all-ones mask of 768 from 702 to 720.  Gated: four, 611 columns 409 -> 407, 1000 1543 -> 1532.)
+#pragma unroll(GATED ? 4 : 2)
       for (int word = ROWS ? warp & 3 : warp; word < P.k_steps * 2; word += ROWS ? 4 : 8) {
         const int key = word * 32 + lane;
         bool keep = key < P.cols;
@@ -723,20 +723,22 @@ __global__ void __launch_bounds__(kFwdThreads, 2) ta_fwd_kernel(const __grid_con
   }
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  // (Two ends of the kernel, and the question about lost rows behind the walk that asks it: with one end, or the question in the output, what the
-  // compiler makes of the listed walk is 1 to 3 % slower.  A persistent kernel has one end: 300 columns 78.3 -> 77.8 us.)
+  // Two ends of the kernel, and the question about lost rows behind the walk that asks it: with one end, or the question in the output, what the
+  // compiler makes of the listed walk is 1 to 3 % slower.  One end is better for a persistent kernel (300 columns 78.3 -> 77.8 us) and for
+  // the gated ones (768 columns 711 -> 705).
+  constexpr bool kTwoEnds = !PERSIST && !GATED;
   auto any_lost = [&]() { return HAS_BIAS && P.closed && *reinterpret_cast<volatile int*>(smem_gen + Smem::lost_flag) != 0; };
   if (!listed && !ragged) {
     fwd_walk<T, HAS_BIAS, GATED, ROWS, PERSIST, true>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, at, n_tiles, false);
-    if constexpr (!PERSIST) {
+    if constexpr (kTwoEnds) {
       teardown(abort_flag, tmem_base, 9, kFwdTmemCols);
       if (any_lost()) clear_lost_rows<T, GATED, ROWS, PERSIST>(P, tid, warp);
     }
   } else {
     fwd_walk<T, HAS_BIAS, GATED, ROWS, PERSIST, false>(P, smem_base, smem_gen, abort_flag, tmem_base, tid, warp, lane, at, n_tiles, listed);
-    if constexpr (!PERSIST) teardown(abort_flag, tmem_base, 9, kFwdTmemCols);
+    if constexpr (kTwoEnds) teardown(abort_flag, tmem_base, 9, kFwdTmemCols);
   }
-  if constexpr (PERSIST) {
+  if constexpr (!kTwoEnds) {
     teardown(abort_flag, tmem_base, 9, kFwdTmemCols);
     if (any_lost()) clear_lost_rows<T, GATED, ROWS, PERSIST>(P, tid, warp);
   }
